@@ -1,0 +1,39 @@
+"""The automaton-free ROSA match (lookup by contexts and by run lengths, sets of lags, constant q) against the oracle's
+pushes: lengths around its word, piece and set-width limits, and streams that each of its ways has to take."""
+import numpy as np
+import pytest
+
+from conftest import pack_plane
+
+pytestmark = pytest.mark.gpu
+
+
+def planes(kind, T, C, rng):
+    if kind == "even":
+        return [rng.integers(0, 2, (T, C), dtype=np.uint8) for _ in range(3)]
+    if kind == "biased":        # q and k biased independently: by bits, by runs, or neither
+        p = rng.choice([0.002, 0.03, 0.1, 0.2, 0.5, 0.8, 0.93, 0.99], (3, 1, C))
+        return [(rng.random((T, C)) < p[i]).astype(np.uint8) for i in range(3)]
+    if kind == "repeating":     # long agreements: sets of lags, windows longer than the ring
+        period = rng.integers(2, 100, C)
+        base = rng.integers(0, 2, (2, 100, C), dtype=np.uint8)
+        phase = np.arange(T)[:, None] % period[None, :]
+        q, v = (np.take_along_axis(base[i], phase, 0) for i in range(2))
+        return [q ^ (rng.random((T, C)) < 0.002), q ^ (rng.random((T, C)) < 0.001), v ^ (rng.random((T, C)) < 0.3)]
+    q, k, v = (rng.integers(0, 2, (T, C), dtype=np.uint8) for _ in range(3))
+    q[:] = rng.integers(0, 2, (1, C))                                   # constant q, keys of several densities
+    return [q, (rng.random((T, C)) < rng.choice([0.01, 0.5, 0.99], (1, C))).astype(np.uint8), v]
+
+
+@pytest.mark.parametrize("kind", ["even", "biased", "repeating", "constant_q"])
+@pytest.mark.parametrize("T", [2, 32, 63, 64, 65, 127, 513, 1023, 1025, 2048, 2049, 4097, 8191, 8192])
+def test_match_equals_the_pushes(cuda_rt, oracle, kind, T):
+    C = 96 if T <= 2049 else 32
+    rng = np.random.default_rng([T, len(kind)])
+    q, k, v = (pack_plane(np.asarray(x, np.uint8)) for x in planes(kind, T, C, rng))
+    cuda_rt.kernel_timing(True)
+    idx, _ = cuda_rt.rosa_qkv_1bit_fwd(q, k, v, np.zeros(C, np.uint16), 1, T, C)
+    ran = cuda_rt.kernel_times()
+    cuda_rt.kernel_timing(False)
+    assert "rosa_context" in ran and "rosa_match" in ran
+    assert np.array_equal(idx, oracle.rosa_qkv_batch_packed(q, k, v, 1, T, C))

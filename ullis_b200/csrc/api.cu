@@ -106,6 +106,7 @@ ullis_cuda_runtime* ullis_cuda_runtime::child(size_t i) {
     ullis_cuda_runtime* c = children[i];
     c->mode = mode;
     c->sam_algo = sam_algo;
+    c->sam_automaton = sam_automaton;
     c->sam_coop = sam_coop;
     c->sam_side = sam_side;
     c->sam_lanes = sam_lanes;
@@ -299,6 +300,13 @@ int32_t ullis_cuda_runtime_create(int32_t device, ullis_cuda_runtime** out) {
             const int a = atoi(env) / 10, b = atoi(env) % 10;   // e.g. 32 = 3 stages (one operand), 2 stages (two)
             if (a >= 2 && a <= 4 && b >= 2 && b <= 4) { rt->tc_stages = a; rt->tc_stages2 = b; }
         }
+        // Options of the suffix automaton: it only runs where the match by sets of lags does not reach, so asking for one
+        // of its forms asks for the automaton.
+        for (const char* name : {"ULLIS_CUDA_SAM_COOP", "ULLIS_CUDA_SAM_BUDGET_MB", "ULLIS_CUDA_SAM_SPARSE", "ULLIS_CUDA_SAM_WORDS",
+                                 "ULLIS_CUDA_SAM_WALK_CHUNKED", "ULLIS_CUDA_SAM_SMEM_WAVES", "ULLIS_CUDA_SAM_RELOAD_W",
+                                 "ULLIS_CUDA_SAM_DEFER_CLIMB", "ULLIS_CUDA_SAM_SPLIT", "ULLIS_CUDA_SAM_SIDE",
+                                 "ULLIS_CUDA_SAM_COOP_THREADS", "ULLIS_CUDA_SAM_LANES"})
+            if (getenv(name)) rt->sam_automaton = true;
         if (const char* env = getenv("ULLIS_CUDA_SAM_COOP")) rt->sam_coop = atoi(env) != 0;
         if (const char* env = getenv("ULLIS_CUDA_SAM_BUDGET_MB")) {
             const long mb = atol(env);
@@ -435,7 +443,7 @@ int32_t ullis_cuda_runtime_sam_counts(ullis_cuda_runtime* rt, uint64_t* total, u
             uint32_t host[2] = {0, 0};
             if (r->sam_last_streams) {
                 // the two counters sit behind the automaton list (k::rosa_sam)
-                r->d2h(host, r->sam_list.as<uint32_t>(2 * r->sam_last_streams + 2) + r->sam_last_streams, 8);
+                r->d2h(host, static_cast<uint32_t*>(r->sam_list.get()) + r->sam_last_streams, 8);
                 r->sync();
             }
             sum[0] += r->sam_last_streams;

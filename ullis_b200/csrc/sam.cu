@@ -1,16 +1,26 @@
-// ROSA 1-bit suffix-automaton match on the GPU: one thread per (sequence,
-// channel) stream, automaton state in a per-stream block of global scratch
-// (compact 16-bit state ids whenever 2T+2 <= 65535), bit streams read and idx
-// bits written as stream-major 32-step words.  The per-stream algorithm lives
-// in sam_core.cuh; results equal T pushes of the reference's RosaSam
-// (src/rosa.rs:100-176) for every stream.
+// ROSA 1-bit match on the GPU, bit streams read and idx bits written as
+// stream-major 32-step words; results equal T pushes of the reference's
+// RosaSam (src/rosa.rs:100-176) for every stream.
 //
-// Streams with constant k bits are finished by a closed form first; the rest
-// are processed in waves sized to the scratch budget, so any batch works; all
+// Up to 8192 steps a stream needs no automaton (rosa_match below): every step
+// is looked up by itself (rosa_context.cuh) or in sets of lags
+// (rosa_match.cuh), so no launch lasts as long as a stream's chain of steps.
+// 64 sequences x 512 channels x 2048 steps: 1.8 ms on evenly spread bits where
+// the automaton took 11.3, 0.6 to 1.4 ms against 2.6 on the benchmark model's
+// layers; 1 sequence 0.07 to 0.2 ms against 0.7.
+//
+// Longer streams, and calls that ask for one of its forms, run the suffix
+// automaton: one thread per (sequence, channel) stream, automaton state in a
+// per-stream block of global scratch (compact 16-bit state ids whenever
+// 2T+2 <= 65535).  The per-stream algorithm lives in sam_core.cuh.  Streams
+// with constant k bits are finished by a closed form first; the rest are
+// processed in waves sized to the scratch budget, so any batch works; all
 // waves are enqueued back to back on the runtime stream.
 #include <algorithm>
 
 #include "kernels.hpp"
+#include "rosa_context.cuh"
+#include "rosa_match.cuh"
 #include "sam_coop.cuh"
 #include "sam_core.cuh"
 
@@ -326,6 +336,369 @@ rosa_coop_kernel(uint8_t* __restrict__ scratch, size_t scratch_stride, const uin
     sam::coop_tour_pass2<NT, MODE != 0, MODE == 1>(coop_smem, B, v_sw + s * wps, idx_sw + s * wps, T);
 }
 
+// The listed streams by contexts (rosa_context.cuh), a CTA per stream, CTAs take streams from a counter until they run
+// out.  A stream whose buckets are too large, or whose agreements turn out to be long, goes to `hard` instead.
+// (step, key position in its bucket) pairs per step: up to which a stream is taken by its last bits without looking at
+// the other way, and up to which at all.
+struct ContextLimits {
+    uint32_t easy, by_bits, by_runs;
+    uint32_t deep;   // 32-step comparisons beyond the first, and words gone back, per thread before a stream is given up
+};
+
+struct ContextLayout {   // bytes of shared memory
+    uint32_t hist, nq, start, q, k, q_ends, k_ends, in_word, before, out, entries, steps, total;
+    __host__ __device__ ContextLayout(uint32_t T, uint32_t c, uint32_t warps) {
+        const uint32_t C = 1u << c, words = (T + 31u) / 32u + 1u;
+        entries = 0;                           // Entry [T]
+        hist = entries + T * 8u;               // u16 [warps][C]: counts, then write positions
+        nq = hist + warps * C * 2u;            // u16 [C]: the same for the steps
+        start = nq + C * 2u;                   // u16 [C + 2]
+        q = start + (C + 2u) * 2u;
+        k = q + words * 4u;
+        before = k + words * 4u;               // u32 [2][words]
+        out = before + words * 8u;
+        in_word = out + words * 4u;             // u16 [2][words]
+        q_ends = in_word + words * 4u;         // u16 [words]
+        k_ends = q_ends + words * 2u;
+        steps = k_ends + words * 2u;           // u16 [T]
+        total = (steps + T * 2u + 15u) & ~15u;
+    }
+};
+
+template <int NT>
+__global__ void __launch_bounds__(NT)
+rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restrict__ k_sw, const uint32_t* __restrict__ v_sw,
+                    uint32_t* __restrict__ idx_sw, const uint32_t* __restrict__ list, const uint32_t* __restrict__ count,
+                    uint32_t* __restrict__ next, uint32_t* __restrict__ hard, uint32_t* __restrict__ hard_count, uint32_t T,
+                    size_t wps, uint32_t c, ContextLimits limits) {
+    constexpr uint32_t NW = NT / 32, BRUTE = context::BRUTE;
+    extern __shared__ __align__(16) uint8_t context_mem[];
+    __shared__ uint32_t sh_item, sh_sums[NW], sh_pairs[NW], sh_gone;
+    const uint32_t C = 1u << c, pair_words = C / 2u, words = (T + 31u) / 32u;
+    const ContextLayout L(T, c, NW);
+    uint16_t* hist = reinterpret_cast<uint16_t*>(context_mem + L.hist);
+    uint32_t* hist2 = reinterpret_cast<uint32_t*>(context_mem + L.hist);   // two counts per word
+    uint16_t* nq = reinterpret_cast<uint16_t*>(context_mem + L.nq);
+    uint32_t* nq2 = reinterpret_cast<uint32_t*>(context_mem + L.nq);
+    uint16_t* start = reinterpret_cast<uint16_t*>(context_mem + L.start);
+    uint32_t* Q = reinterpret_cast<uint32_t*>(context_mem + L.q);
+    uint32_t* K = reinterpret_cast<uint32_t*>(context_mem + L.k);
+    uint16_t* q_ends = reinterpret_cast<uint16_t*>(context_mem + L.q_ends);
+    uint16_t* k_ends = reinterpret_cast<uint16_t*>(context_mem + L.k_ends);
+    uint16_t* in_word = reinterpret_cast<uint16_t*>(context_mem + L.in_word);
+    uint32_t* before_word = reinterpret_cast<uint32_t*>(context_mem + L.before);
+    uint32_t* out_s = reinterpret_cast<uint32_t*>(context_mem + L.out);
+    context::Entry* entries = reinterpret_cast<context::Entry*>(context_mem + L.entries);
+    uint16_t* steps = reinterpret_cast<uint16_t*>(context_mem + L.steps);
+    const context::Runs runs{k_ends, in_word, before_word};
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t total = *count;
+    const uint32_t rows_per_warp = (words + NW - 1u) / NW;
+    const uint32_t row0 = min(warp * rows_per_warp, words), row1 = min(row0 + rows_per_warp, words);   // a warp's keys
+    for (;;) {
+        __syncthreads();   // the stream before this one is done with everything below
+        if (threadIdx.x == 0) {
+            sh_item = atomicAdd(next, 1u);
+            sh_gone = 0u;
+        }
+        __syncthreads();
+        if (sh_item >= total) return;
+        const size_t s = list[sh_item];
+        for (uint32_t w = threadIdx.x; w < words; w += NT) {
+            Q[w + 1u] = q_sw[s * wps + w];
+            K[w + 1u] = k_sw[s * wps + w];
+            out_s[w] = 0u;
+        }
+        if (threadIdx.x == 0) Q[0] = K[0] = 0u;
+        bool by_runs = false, taken = false, sorted = false;   // sorted: the steps bucket by bucket too
+        uint32_t pairs_by_bits = 0;
+        auto key_of_key = [&](uint32_t r) {
+            return by_runs ? context::run_key(K, k_ends, r, c) : context::window(K, r) >> (32u - c);
+        };
+        auto key_of_step = [&](uint32_t t) {
+            return by_runs ? context::run_key(Q, q_ends, t, c) : context::window(Q, t) >> (32u - c);
+        };
+        for (int attempt = 0;; ++attempt) {
+            for (uint32_t i = threadIdx.x; i < (NW + 1u) * pair_words; i += NT) hist2[i] = 0u;   // hist and nq
+            __syncthreads();
+            for (uint32_t row = row0; row < row1; ++row) {
+                const uint32_t r = row * 32u + lane;
+                if (r < T) {
+                    const uint32_t ck = key_of_key(r);
+                    atomicAdd(&hist2[warp * pair_words + (ck >> 1)], 1u << ((ck & 1u) * 16u));
+                    if (r >= BRUTE) {
+                        const uint32_t cq = key_of_step(r);
+                        atomicAdd(&nq2[cq >> 1], 1u << ((cq & 1u) * 16u));
+                    }
+                }
+            }
+            __syncthreads();
+            // exclusive sums over the buckets (keys in the low half, steps in the high half), and the number of pairs
+            const uint32_t per = (pair_words + NT - 1u) / NT;
+            const uint32_t j0 = min(threadIdx.x * per, pair_words), j1 = min(j0 + per, pair_words);
+            uint32_t sum = 0, pairs = 0;
+            for (uint32_t j = j0; j < j1; ++j) {
+                uint32_t n = 0;
+                for (uint32_t w = 0; w < NW; ++w) n += hist2[w * pair_words + j];
+                const uint32_t m = nq2[j];
+                pairs += (n & 0xFFFFu) * (m & 0xFFFFu) + (n >> 16) * (m >> 16);
+                sum += (n & 0xFFFFu) + (n >> 16) + (((m & 0xFFFFu) + (m >> 16)) << 16);
+            }
+            uint32_t before = sum;
+#pragma unroll
+            for (uint32_t o = 1; o < 32u; o <<= 1) {
+                const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, before, o);
+                if (lane >= o) before += x;
+            }
+            pairs = __reduce_add_sync(0xFFFFFFFFu, pairs);
+            if (lane == 31u) {
+                sh_sums[warp] = before;
+                sh_pairs[warp] = pairs;
+            }
+            __syncthreads();
+            uint32_t run = before - sum;
+            pairs = 0;
+            for (uint32_t w = 0; w < NW; ++w) {
+                if (w < warp) run += sh_sums[w];
+                pairs += sh_pairs[w];
+            }
+            // By bits when that is easy; otherwise by whichever of the two ways has fewer pairs, if those are few enough.
+            if (attempt == 0) {
+                taken = pairs <= limits.easy * T;
+                pairs_by_bits = pairs;
+            } else if (attempt == 1) {
+                taken = pairs <= pairs_by_bits && pairs <= limits.by_runs * T;
+            } else {
+                taken = true;
+            }
+            if (taken) {
+                uint32_t run_k = run & 0xFFFFu, run_q = run >> 16;
+                for (uint32_t x = 2u * j0; x < 2u * j1; ++x) {
+                    start[x] = (uint16_t)run_k;
+                    for (uint32_t w = 0; w < NW; ++w) {
+                        const uint32_t n = hist[w * C + x];
+                        hist[w * C + x] = (uint16_t)run_k;
+                        run_k += n;
+                    }
+                    const uint32_t m = nq[x];
+                    nq[x] = (uint16_t)run_q;
+                    run_q += m;
+                }
+                if (threadIdx.x == 0) start[C] = (uint16_t)T;
+            }
+            sorted = attempt != 0;
+            if (taken || (attempt == 1 && pairs_by_bits > limits.by_bits * T)) break;
+            by_runs = attempt == 0;
+            if (by_runs) {
+                for (uint32_t w = threadIdx.x; w < words; w += NT) {
+                    q_ends[w] = (uint16_t)context::run_at_end(Q, w);
+                    k_ends[w] = (uint16_t)context::run_at_end(K, w);
+                }
+            }
+        }
+        if (!taken) {
+            if (threadIdx.x == 0) hard[atomicAdd(hard_count, 1u)] = (uint32_t)s;
+            continue;
+        }
+        __syncthreads();
+        // a warp's keys in order: equal contexts of 32 steps take consecutive places
+        for (uint32_t row = row0; row < row1; ++row) {
+            const uint32_t r = row * 32u + lane;
+            const uint32_t ck = r < T ? key_of_key(r) : 0xFFFFFFFFu;
+            const uint32_t same = __match_any_sync(0xFFFFFFFFu, ck);
+            const uint32_t rank = __popc(same & ((1u << lane) - 1u));
+            uint32_t at = 0;
+            if (r < T) {
+                at = hist[warp * C + ck];
+                entries[at + rank] = context::Entry{context::window(K, r), r};
+                if (sorted && r >= BRUTE) {   // in any order within a bucket
+                    const uint32_t cq = key_of_step(r), sh = (cq & 1u) * 16u;
+                    steps[(atomicAdd(&nq2[cq >> 1], 1u << sh) >> sh) & 0xFFFFu] = (uint16_t)r;
+                }
+            }
+            __syncwarp();
+            if (r < T && rank == 0u) hist[warp * C + ck] = (uint16_t)(at + __popc(same));
+            __syncwarp();
+        }
+        if (by_runs) {
+            for (uint32_t i = threadIdx.x; i < 2u * words; i += NT) {
+                const uint32_t b = i >= words, w = i - b * words;
+                const uint32_t x = context::longest_in_word(K, k_ends, w, T, b);
+                before_word[i] = x;
+                in_word[i] = (uint16_t)(x >> 16);
+            }
+            __syncthreads();
+            if (warp < 2u) {   // running maximum over the words, exclusive: a warp per bit
+                uint32_t carry = 0;
+                for (uint32_t w0 = 0; w0 < words; w0 += 32u) {
+                    const uint32_t w = w0 + lane;
+                    uint32_t x = w < words ? before_word[warp * words + w] : 0u;
+#pragma unroll
+                    for (uint32_t o = 1; o < 32u; o <<= 1) {
+                        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+                        if (lane >= o) x = max(x, y);
+                    }
+                    x = max(x, carry);
+                    uint32_t excl = __shfl_up_sync(0xFFFFFFFFu, x, 1);
+                    if (lane == 0) excl = carry;
+                    __syncwarp();
+                    if (w < words) before_word[warp * words + w] = excl;
+                    carry = __shfl_sync(0xFFFFFFFFu, x, 31);
+                }
+            }
+        }
+        __syncthreads();
+        // Easy streams step by step.  On the others the number of positions to look at differs a lot from bucket to bucket:
+        // their steps are taken bucket by bucket, so that the lanes of a warp look through the same ones.
+        const uint32_t* v = v_sw + s * wps;
+        uint32_t* out = idx_sw + s * wps;
+        uint32_t deep = 0;
+        for (uint32_t row = warp; row < words; row += NW) {
+            const uint32_t i = row * 32u + lane, t = sorted && i >= BRUTE && i < T ? steps[i - BRUTE] : i;
+            uint32_t bit = 0;
+            if (i < T) {
+                const uint32_t r1 = by_runs && i >= BRUTE
+                                        ? context::find_by_runs(entries, start, Q, K, q_ends, runs, words, c, t, deep)
+                                        : context::find(entries, start, Q, K, c, !sorted, t, deep);
+                bit = r1 ? (v[r1 >> 5] >> (r1 & 31u)) & 1u : 0u;
+            }
+            if (sorted) {
+                if (bit) atomicOr(&out_s[t >> 5], 1u << (t & 31u));
+            } else {
+                const uint32_t word = __ballot_sync(0xFFFFFFFFu, bit != 0u);
+                if (lane == 0) out[row] = word;
+            }
+            if (__any_sync(0xFFFFFFFFu, deep > limits.deep)) {
+                if (lane == 0) sh_gone = 1u;
+                break;
+            }
+            if (*static_cast<volatile uint32_t*>(&sh_gone)) break;
+        }
+        __syncthreads();
+        if (sh_gone) {
+            if (threadIdx.x == 0) hard[atomicAdd(hard_count, 1u)] = (uint32_t)s;
+        } else if (sorted) {
+            for (uint32_t w = threadIdx.x; w < words; w += NT) out[w] = out_s[w];
+        }
+    }
+}
+
+// The remaining streams by sets of lags (rosa_match.cuh).  A work item is a piece of one stream, a warp takes items
+// from a counter until they run out; the warps of a CTA have nothing to do with one another.
+constexpr int MATCH_WARPS = 4;
+
+// A stream whose query bits are all c: idx follows the longest run of c among the keys so far, the latest of equals
+// (sam_core.cuh run_constant_q), a running maximum over (run length, position).  T <= 65535.
+__device__ __forceinline__ void constant_q_warp(uint32_t c, const uint32_t* __restrict__ k, const uint32_t* __restrict__ v,
+                                                uint32_t* __restrict__ out, uint32_t T) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t run_before = 0, best = 0;   // run length << 16 | position + 1
+    for (uint32_t row = 0; row < (T + 31u) / 32u; ++row) {
+        const uint32_t t = row * 32u + lane, same = c ? k[row] : ~k[row];
+        const uint32_t n = min((uint32_t)__clz((int)~(same << (31u - lane))), lane + 1u);
+        const uint32_t run = n == lane + 1u ? n + run_before : n;
+        uint32_t key = run ? run << 16 | (t + 1u) : 0u;
+#pragma unroll
+        for (uint32_t o = 1; o < 32u; o <<= 1) {
+            const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, key, o);
+            if (lane >= o) key = max(key, x);
+        }
+        uint32_t mine = __shfl_up_sync(0xFFFFFFFFu, key, 1);   // the positions before t
+        mine = lane == 0u ? best : max(mine, best);
+        const uint32_t p = mine & 0xFFFFu;
+        const uint32_t word = __ballot_sync(0xFFFFFFFFu, mine != 0u && t < T && ((v[p >> 5] >> (p & 31u)) & 1u) != 0u);
+        if (lane == 0) out[row] = word;
+        run_before = __shfl_sync(0xFFFFFFFFu, run, 31);
+        best = max(best, __shfl_sync(0xFFFFFFFFu, key, 31));
+    }
+}
+
+template <int NW>
+__global__ void __launch_bounds__(32 * MATCH_WARPS)
+rosa_match_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restrict__ k_sw, const uint32_t* __restrict__ v_sw,
+                  uint32_t* __restrict__ idx_sw, const uint32_t* __restrict__ hard, const uint32_t* __restrict__ hard_count,
+                  const uint32_t* __restrict__ cq_list, const uint32_t* __restrict__ cq_count, uint32_t* __restrict__ next,
+                  uint32_t* __restrict__ kept, uint32_t T, size_t wps, uint32_t ring_words) {
+    extern __shared__ __align__(16) uint32_t match_mem[];
+    const match::Layout L(NW, ring_words);
+    uint32_t* mem = match_mem + (threadIdx.x >> 5) * L.total;
+    kept += (size_t)(blockIdx.x * MATCH_WARPS + (threadIdx.x >> 5)) * (match::CHECKPOINTS * 32u * NW);
+    const uint32_t gap = match::checkpoint_gap(T);
+    const uint32_t total = *hard_count, constant = *cq_count;
+    // Pieces as long as the number of streams allows: a piece costs its set-up and the search for its first window
+    // on top of its steps, but the device wants a few pieces per warp.
+    const uint32_t warps = gridDim.x * MATCH_WARPS;
+    uint32_t piece = 1024u * NW;
+    while (piece > 32u && (uint64_t)total * ((T + piece - 1u) / piece) < 3ull * warps) piece >>= 1;
+    const uint32_t pieces = (T + piece - 1u) / piece;
+    const uint32_t items = total * pieces;   // below 2^32: the host checked it for the shortest pieces
+    for (;;) {
+        uint32_t item = 0;
+        if ((threadIdx.x & 31u) == 0u) item = atomicAdd(next, 1u);
+        item = __shfl_sync(0xFFFFFFFFu, item, 0);
+        if (item >= items + constant) return;
+        if (item >= items) {
+            const size_t s = cq_list[item - items];
+            constant_q_warp(q_sw[s * wps] & 1u, k_sw + s * wps, v_sw + s * wps, idx_sw + s * wps, T);
+            continue;
+        }
+        const uint32_t i = item % total, t0 = (pieces - 1u - item / total) * piece, t1 = min(t0 + piece, T);   // the wide sets first
+        const size_t s = hard[i];
+        const uint32_t *q = q_sw + s * wps, *k = k_sw + s * wps, *v = v_sw + s * wps;
+        uint32_t* out = idx_sw + s * wps;
+        if (NW >= 8 && t1 > 4096u) match::piece<8>(mem, L, ring_words, kept, gap, q, k, v, out, t0, t1);
+        else if (NW >= 4 && t1 > 2048u) match::piece<4>(mem, L, ring_words, kept, gap, q, k, v, out, t0, t1);
+        else if (NW >= 2 && t1 > 1024u) match::piece<2>(mem, L, ring_words, kept, gap, q, k, v, out, t0, t1);
+        else match::piece<1>(mem, L, ring_words, kept, gap, q, k, v, out, t0, t1);
+    }
+}
+
+struct MatchCall {   // the buffers of one call
+    const uint32_t *q, *k, *v;
+    uint32_t *idx, *list, *cq_list, *hard, *counts;   // counts: listed, constant q, hard, next of the contexts, next of the matches
+    size_t streams, wps;
+    uint32_t T;
+};
+constexpr uint32_t MATCH_COUNTS = 5;
+
+template <int NT>
+void launch_context(ullis_cuda_runtime* rt, const MatchCall& m, int slot) {
+    const uint32_t c = context::bits_for(m.T);
+    const size_t smem = ContextLayout(m.T, c, NT / 32).total;
+    if (rt->context_smem[slot] != smem) {
+        int per_sm = 0;
+        ULLIS_CUDA_CHECK(cudaFuncSetAttribute(rosa_context_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        ULLIS_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rosa_context_kernel<NT>, NT, smem));
+        rt->context_ctas[slot] = std::max(1, per_sm) * rt->sm_count;
+        rt->context_smem[slot] = smem;
+    }
+    const unsigned grid = (unsigned)std::min<size_t>(rt->context_ctas[slot], m.streams);
+    // A match kernel step costs about as much as 100 positions here; up to 24 the lanes are even enough without sorting
+    // the steps.  128 long comparisons per stream at most are thrown away when a stream turns out to repeat itself.
+    const ContextLimits limits{24u, 96u, 160u, 256u};
+    rosa_context_kernel<NT><<<grid, NT, smem, rt->stream>>>(m.q, m.k, m.v, m.idx, m.list, m.counts, m.counts + 3, m.hard,
+                                                            m.counts + 2, m.T, m.wps, c, limits);
+    rt->launched("rosa_context");
+}
+
+template <int NW>
+void launch_match(ullis_cuda_runtime* rt, const MatchCall& m, int slot, uint32_t ring_words) {
+    const match::Layout L(NW, ring_words);
+    const size_t smem = (size_t)L.total * 4u * MATCH_WARPS;
+    if (!rt->match_ctas[slot]) {
+        int per_sm = 0;
+        ULLIS_CUDA_CHECK(cudaFuncSetAttribute(rosa_match_kernel<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        ULLIS_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rosa_match_kernel<NW>, 32 * MATCH_WARPS, smem));
+        rt->match_ctas[slot] = std::max(1, per_sm) * rt->sm_count;
+    }
+    const size_t most = (m.streams * m.wps + MATCH_WARPS - 1) / MATCH_WARPS;   // every stream in the shortest pieces
+    const unsigned grid = (unsigned)std::min<size_t>(rt->match_ctas[slot], most);
+    uint32_t* kept = rt->sam_scratch.as<uint32_t>((size_t)grid * MATCH_WARPS * match::CHECKPOINTS * 32u * NW);
+    rosa_match_kernel<NW><<<grid, 32 * MATCH_WARPS, smem, rt->stream>>>(m.q, m.k, m.v, m.idx, m.hard, m.counts + 2, m.cq_list,
+                                                                        m.counts + 1, m.counts + 4, kept, m.T, m.wps, ring_words);
+    rt->launched("rosa_match");
+}
+
 // EAGER keeps the reference's schedule for every stream (no shortcut): list = all streams
 __global__ void rosa_list_all_kernel(uint32_t* __restrict__ list, uint32_t* __restrict__ count, size_t streams) {
     const size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -337,6 +710,34 @@ template <typename Ix>
 size_t stride_for(int algo, size_t T) {
     return algo == ULLIS_CUDA_SAM_EAGER ? sam::EagerLayout<Ix>((uint32_t)T).total
                                         : sam::EulerLayout<Ix>((uint32_t)T).total;
+}
+
+// The whole call without an automaton: classification, the listed streams by contexts, and by sets of lags those that
+// the contexts leave and the ones with a constant q.
+constexpr size_t MATCH_MAX_TIME = 8192;   // 256 words of lags, eight per lane
+void rosa_match(ullis_cuda_runtime* rt, const uint32_t* q_sw, const uint32_t* k_sw, const uint32_t* v_sw, uint32_t* idx_sw,
+                size_t streams, uint32_t T) {
+    MatchCall m;
+    m.q = q_sw; m.k = k_sw; m.v = v_sw; m.idx = idx_sw;
+    m.streams = streams; m.T = T; m.wps = (T + 31u) / 32u;
+    m.list = rt->sam_list.as<uint32_t>(3 * streams + MATCH_COUNTS);
+    m.counts = m.list + streams;
+    m.cq_list = m.counts + MATCH_COUNTS;
+    m.hard = m.cq_list + streams;
+    rt->sam_last_streams = streams;
+    if (!rt->parent) rt->lanes_last = 1;
+    rt->zero(m.counts, MATCH_COUNTS * 4u);
+    rosa_classify_kernel<<<(unsigned)((streams * CLASSIFY_LANES + 127) / 128), 128, 0, rt->stream>>>(
+        q_sw, k_sw, v_sw, idx_sw, streams, T, m.wps, m.list, m.counts, m.cq_list, m.counts + 1);
+    rt->launched("rosa_classify");
+    // few streams: sixteen warps each, so that the last of them is done soon (one sequence of 512 channels: 0.20 ms
+    // against 0.28 with eight); many: eight (1.79 ms for 32 768 streams against 1.98 with sixteen)
+    if (streams <= 1024u) launch_context<512>(rt, m, 1);
+    else launch_context<256>(rt, m, 0);
+    if (T <= 1024u) launch_match<1>(rt, m, 0, 1024);
+    else if (T <= 2048u) launch_match<2>(rt, m, 1, 1024);
+    else if (T <= 4096u) launch_match<4>(rt, m, 2, 2048);
+    else launch_match<8>(rt, m, 3, 4096);
 }
 
 }  // namespace
@@ -351,6 +752,11 @@ void rosa_sam(ullis_cuda_runtime* rt, const uint32_t* q_sw, const uint32_t* k_sw
     if (streams == 0 || time == 0) return;
     if (time > 0x3FFFFFFFu) fail(ULLIS_CUDA_ERR_SHAPE, "ROSA time does not fit 32-bit state ids");
     const int algo = rt->sam_algo;
+    if (streams > 0xFFFFFFFFull) fail(ULLIS_CUDA_ERR_SHAPE, "too many ROSA streams");
+    if (algo == ULLIS_CUDA_SAM_EULER && !rt->sam_automaton && time <= MATCH_MAX_TIME && streams * ((time + 31) / 32) < 0x7FFFFFFFull) {
+        rosa_match(rt, q_sw, k_sw, v_sw, idx_sw, streams, (uint32_t)time);
+        return;
+    }
     const bool narrow = sam::node_capacity((uint32_t)time) <= 0xFFFFu;
     const size_t stride = rosa_sam_scratch_bytes_per_stream(algo, time);
     const size_t wps = (time + 31) / 32;
@@ -369,13 +775,12 @@ void rosa_sam(ullis_cuda_runtime* rt, const uint32_t* q_sw, const uint32_t* k_sw
         if (wave > streams) wave = streams;
     }
     uint8_t* scratch = static_cast<uint8_t*>(rt->sam_scratch.ensure(wave * stride));
-    if (streams > 0xFFFFFFFFull) fail(ULLIS_CUDA_ERR_SHAPE, "too many ROSA streams");
-    uint32_t* list = rt->sam_list.as<uint32_t>(2 * streams + 2);
+    uint32_t* list = rt->sam_list.as<uint32_t>(3 * streams + MATCH_COUNTS);
     rt->sam_last_streams = streams;
     if (!rt->parent) rt->lanes_last = 1;   // a forward that splits its batch raises this after its last layer
     uint32_t* count = list + streams;
     uint32_t* cq_count = count + 1;           // the constant-q streams, settled by a kernel of their own
-    uint32_t* cq_list = count + 2;
+    uint32_t* cq_list = count + 3;
     const unsigned cgrid = (unsigned)((streams + 127) / 128);
     // The number of streams left for the automaton is only known on the device;
     // each wave is sized for the worst case and surplus threads exit at once.
