@@ -71,16 +71,18 @@ __global__ void cast16_kernel(const float* __restrict__ x, uint16_t* __restrict_
 // Time-shift mixes of one LayerNorm output (reference src/model.rs:1291-1298:
 // in = x + (x[t-1]-x[t])*mix, unfused) written as FP16 hi and lo = FP16(in - hi)
 // for up to three mixes, plus the row's sum |in| that scales the sign-bit error
-// band. One warp per row.
+// band. One warp per row.  A sequence of `time` rows takes `pitch` rows of the operands (and of s1): the sign-bit
+// GEMM wants the steps of a sequence in whole words; what is in the rows between is never looked at.
 __global__ void __launch_bounds__(256)
 mix_split_kernel(const float* __restrict__ x, const uint16_t* __restrict__ m0, const uint16_t* __restrict__ m1,
                  const uint16_t* __restrict__ m2, uint16_t* __restrict__ hi0, uint16_t* __restrict__ lo0,
                  uint16_t* __restrict__ hi1, uint16_t* __restrict__ lo1, uint16_t* __restrict__ hi2,
-                 uint16_t* __restrict__ lo2, float* __restrict__ s1, size_t rows, size_t time, size_t C) {
+                 uint16_t* __restrict__ lo2, float* __restrict__ s1, size_t rows, size_t time, size_t pitch, size_t C) {
     const int lane = threadIdx.x & 31;
     const size_t row = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= rows) return;
     const bool first = row % time == 0;
+    const size_t orow = row + row / time * (pitch - time), orows = rows / time * pitch;
     const uint16_t* mix[3] = {m0, m1, m2};
     uint16_t* hi[3] = {hi0, hi1, hi2};
     uint16_t* lo[3] = {lo0, lo1, lo2};
@@ -109,10 +111,10 @@ mix_split_kernel(const float* __restrict__ x, const uint16_t* __restrict__ m0, c
                 lb[e] = __half_as_ushort(__float2half_rn(v - __half2float(h)));
                 sum[k] += fabsf(v);
             }
-            *reinterpret_cast<uint2*>(hi[k] + row * C + c) =
+            *reinterpret_cast<uint2*>(hi[k] + orow * C + c) =
                 make_uint2(hb[0] | ((uint32_t)hb[1] << 16), hb[2] | ((uint32_t)hb[3] << 16));
             if (lo[k])
-                *reinterpret_cast<uint2*>(lo[k] + row * C + c) =
+                *reinterpret_cast<uint2*>(lo[k] + orow * C + c) =
                     make_uint2(lb[0] | ((uint32_t)lb[1] << 16), lb[2] | ((uint32_t)lb[3] << 16));
         }
     }
@@ -121,7 +123,7 @@ mix_split_kernel(const float* __restrict__ x, const uint16_t* __restrict__ m0, c
         for (int k = 0; k < 3; ++k) {
             float s = sum[k];
             for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (lane == 0 && mix[k]) s1[k * rows + row] = s;
+            if (lane == 0 && mix[k]) s1[k * orows + orow] = s;
         }
     }
 }
@@ -137,7 +139,7 @@ ln_mix_split_kernel(const float* __restrict__ x, const uint16_t* __restrict__ lw
                     float* __restrict__ ln_out, const uint16_t* __restrict__ m0, const uint16_t* __restrict__ m1,
                     const uint16_t* __restrict__ m2, uint16_t* __restrict__ hi0, uint16_t* __restrict__ lo0,
                     uint16_t* __restrict__ hi1, uint16_t* __restrict__ lo1, uint16_t* __restrict__ hi2,
-                    uint16_t* __restrict__ lo2, float* __restrict__ s1, size_t rows, size_t time) {
+                    uint16_t* __restrict__ lo2, float* __restrict__ s1, size_t rows, size_t time, size_t pitch) {
     constexpr int C = 128 * VEC;
     const int lane = threadIdx.x & 31;
     // a warp takes ROWS consecutive rows: the LayerNorm of a row is then computed once and handed on as the next
@@ -183,6 +185,7 @@ ln_mix_split_kernel(const float* __restrict__ x, const uint16_t* __restrict__ lw
     const size_t row = row0 + r;
     if (row >= rows) break;
     const bool first = row % time == 0;   // the same for the whole warp
+    const size_t orow = row + row / time * (pitch - time), orows = rows / time * pitch;
     const float4* src = reinterpret_cast<const float4*>(x + row * C);
 #pragma unroll
     for (int i = 0; i < VEC; ++i) cur[i] = src[lane + 32 * i];
@@ -220,10 +223,10 @@ ln_mix_split_kernel(const float* __restrict__ x, const uint16_t* __restrict__ lw
                 lbt[e] = __half_as_ushort(__float2half_rn(v - __half2float(h)));
                 sum[k] += fabsf(v);
             }
-            *reinterpret_cast<uint2*>(hi[k] + row * C + c) =
+            *reinterpret_cast<uint2*>(hi[k] + orow * C + c) =
                 make_uint2(hb[0] | ((uint32_t)hb[1] << 16), hb[2] | ((uint32_t)hb[3] << 16));
             if (lo[k])
-                *reinterpret_cast<uint2*>(lo[k] + row * C + c) =
+                *reinterpret_cast<uint2*>(lo[k] + orow * C + c) =
                     make_uint2(lbt[0] | ((uint32_t)lbt[1] << 16), lbt[2] | ((uint32_t)lbt[3] << 16));
         }
     }
@@ -232,7 +235,7 @@ ln_mix_split_kernel(const float* __restrict__ x, const uint16_t* __restrict__ lw
         for (int k = 0; k < 3; ++k) {
             float s = sum[k];
             for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (lane == 0 && mix[k]) s1[k * rows + row] = s;
+            if (lane == 0 && mix[k]) s1[k * orows + orow] = s;
         }
     }
 #pragma unroll
@@ -776,7 +779,7 @@ GemmParams base_params(ullis_cuda_runtime* rt, size_t M, size_t N, size_t K) {
 bool launch_ln_mix_split(ullis_cuda_runtime* rt, const float* x, const LayerNormWeights& ln, float* ln_out,
                          const uint16_t* m0, const uint16_t* m1, const uint16_t* m2, uint16_t* hi0, uint16_t* lo0,
                          uint16_t* hi1, uint16_t* lo1, uint16_t* hi2, uint16_t* lo2, float* s1, size_t rows, size_t time,
-                         size_t d, const char* what) {
+                         size_t pitch, size_t d, const char* what) {
     if (!rt->tc_fuse_ln || d % 128 != 0 || d > 1024) return false;
     // rows per warp: several once there are enough rows to fill the device with warps anyway
     // (measured at 131 072 rows: the Q/K/V form, bound by its 0.8 GB of stores, is best with two; the one-operand
@@ -787,13 +790,13 @@ bool launch_ln_mix_split(ullis_cuda_runtime* rt, const float* x, const LayerNorm
     do {                                                                                                                 \
         if (per_warp == 4)                                                                                               \
             ln_mix_split_kernel<V, 4><<<grid, 256, 0, rt->stream>>>(x, ln.weight, ln.bias, ln_out, m0, m1, m2, hi0, lo0, \
-                                                                    hi1, lo1, hi2, lo2, s1, rows, time);                 \
+                                                                    hi1, lo1, hi2, lo2, s1, rows, time, pitch);                 \
         else if (per_warp == 2)                                                                                          \
             ln_mix_split_kernel<V, 2><<<grid, 256, 0, rt->stream>>>(x, ln.weight, ln.bias, ln_out, m0, m1, m2, hi0, lo0, \
-                                                                    hi1, lo1, hi2, lo2, s1, rows, time);                 \
+                                                                    hi1, lo1, hi2, lo2, s1, rows, time, pitch);                 \
         else                                                                                                             \
             ln_mix_split_kernel<V, 1><<<grid, 256, 0, rt->stream>>>(x, ln.weight, ln.bias, ln_out, m0, m1, m2, hi0, lo0, \
-                                                                    hi1, lo1, hi2, lo2, s1, rows, time);                 \
+                                                                    hi1, lo1, hi2, lo2, s1, rows, time, pitch);                 \
     } while (0)
     switch (d / 128) {
         case 1: ULLIS_LN_MIX(1); break;
@@ -901,35 +904,38 @@ bool rosa_qkv_bits(ullis_cuda_runtime* rt, const float* ln3_out, const LayerWeig
                    uint32_t* k_sw, uint32_t* v_sw, size_t batch, size_t time, size_t d, const float* x_before_ln,
                    float* ln3_write) {
     const size_t rows = batch * time;
-    if (!usable(rt) || !shape_ok(rows, d, d) || time % 32) return false;
-    const size_t n = rows * d, wps = time / 32, sw = batch * d * wps;
+    // the GEMM's rows: every sequence padded to whole words of 32 steps, so that a warp of its epilogue holds one word
+    const size_t wps = (time + 31) / 32, pitch = 32 * wps, prows = batch * pitch;
+    if (!usable(rt) || !shape_ok(prows, d, d)) return false;
+    const size_t n = prows * d, sw = batch * d * wps;
     uint16_t* op = rt->tc_ws[1].as<uint16_t>(6 * n);   // q/k/v hi, then q/k/v lo
-    float* s1 = rt->tc_ws[2].as<float>(3 * rows);
+    float* s1 = rt->tc_ws[2].as<float>(3 * prows);
     uint32_t* flags = rt->tc_ws[3].as<uint32_t>(3 * sw);
     // x_before_ln: ln3 has not run yet - it is folded into the operand kernel, which leaves its output in ln3_write
     // (= ln3_out) for the exact fix-up below
     if (!(x_before_ln && launch_ln_mix_split(rt, x_before_ln, L.ln3, ln3_write, L.x_q, L.x_k, L.x_v, op, op + 3 * n, op + n,
-                                             op + 4 * n, op + 2 * n, op + 5 * n, s1, rows, time, d, "ln_mix_split"))) {
+                                             op + 4 * n, op + 2 * n, op + 5 * n, s1, rows, time, pitch, d, "ln_mix_split"))) {
         if (x_before_ln) k::layer_norm(rt, x_before_ln, L.ln3.weight, L.ln3.bias, ln3_write, rows, d, false);
         mix_split_kernel<<<blocks_for(rows, 8), 256, 0, rt->stream>>>(ln3_out, L.x_q, L.x_k, L.x_v, op, op + 3 * n, op + n,
-                                                                     op + 4 * n, op + 2 * n, op + 5 * n, s1, rows, time, d);
+                                                                     op + 4 * n, op + 2 * n, op + 5 * n, s1, rows, time, pitch, d);
         rt->launched("mix_split");
     }
     GemmMaps maps;
     memset(&maps, 0, sizeof(maps));
     for (int z = 0; z < 3; ++z) {
-        maps.a[z][0] = make_map(op + z * n, rows, d, false);
-        maps.a[z][1] = make_map(op + (3 + z) * n, rows, d, false);
+        maps.a[z][0] = make_map(op + z * n, prows, d, false);
+        maps.a[z][1] = make_map(op + (3 + z) * n, prows, d, false);
     }
-    GemmParams p = base_params(rt, rows, d, d);
+    GemmParams p = base_params(rt, prows, d, d);
     p.n_a = 2;
     p.stages = rt->tc_stages2;
-    p.time = (uint32_t)time;
+    p.time = (uint32_t)pitch;
+    p.steps = (uint32_t)time;
     p.wps = (uint32_t)wps;
     const PackedWeights* W[3] = {&L.q, &L.k, &L.v};
     uint32_t* outs[3] = {q_sw, k_sw, v_sw};
     for (int z = 0; z < 3; ++z)
-        p.prob[z] = GemmProblem{W[z]->bits, W[z]->scale, W[z]->bias, outs[z], flags + z * sw, s1 + z * rows};
+        p.prob[z] = GemmProblem{W[z]->bits, W[z]->scale, W[z]->bias, outs[z], flags + z * sw, s1 + z * prows};
     launch<EPI_SIGNBITS, true>(rt, maps, p, 3, "gemm_qkv_signbits");
     const unsigned grid = (unsigned)(((wps + FIX_WIN - 1) / FIX_WIN) * batch);   // rows < 2^30, so this fits
     const uint32_t* only_if = nullptr;
@@ -978,10 +984,10 @@ bool cmix_residual(ullis_cuda_runtime* rt, const LayerWeights& L, float* x, size
     uint16_t* a16 = rt->tc_ws[0].as<uint16_t>(rows * d);
     uint16_t* k16 = rt->tc_ws[5].as<uint16_t>(rows * ffn);
     if (!launch_ln_mix_split(rt, x, L.ln2, nullptr, L.ffn_x_k, nullptr, nullptr, a16, nullptr, nullptr, nullptr, nullptr,
-                             nullptr, nullptr, rows, time, d, "ln_mix_f16")) {
+                             nullptr, nullptr, rows, time, time, d, "ln_mix_f16")) {
         k::layer_norm(rt, x, L.ln2.weight, L.ln2.bias, ln, rows, d, false);
         mix_split_kernel<<<blocks_for(rows, 8), 256, 0, rt->stream>>>(ln, L.ffn_x_k, nullptr, nullptr, a16, nullptr,
-                                                                     nullptr, nullptr, nullptr, nullptr, nullptr, rows, time, d);
+                                                                     nullptr, nullptr, nullptr, nullptr, nullptr, rows, time, time, d);
         rt->launched("mix_f16");
     }
     GemmMaps maps;
@@ -1022,7 +1028,7 @@ void wait_selftest(ullis_cuda_runtime* rt, uint32_t polls) {
 }
 
 bool takes_model(ullis_cuda_runtime* rt, size_t rows, size_t time, size_t d, size_t ffn, size_t vocab) {
-    return usable(rt) && shape_ok(rows, d, d) && time % 32 == 0 && d % 4 == 0 && shape_ok(rows, d, ffn) &&
+    return usable(rt) && shape_ok((rows + time - 1) / time * ((time + 31) / 32 * 32), d, d) && d % 4 == 0 && shape_ok(rows, d, ffn) &&
            shape_ok(rows, ffn, d) && shape_ok(rows, d, vocab);
 }
 

@@ -62,7 +62,8 @@ struct GemmParams {
     uint32_t stages;         // shared-memory pipeline depth, 2..MAX_STAGES
     uint32_t a_fmt, b_fmt;   // 0 = f16, 1 = bf16
     uint32_t out_fmt;        // EPI_RELU2: 0 = f16, 1 = bf16
-    uint32_t time, wps;      // EPI_SIGNBITS / EPI_CE: steps per sequence, words per stream
+    uint32_t time, wps;      // EPI_SIGNBITS / EPI_CE: rows per sequence, words per stream
+    uint32_t steps;          // EPI_SIGNBITS: rows of a sequence that are steps (the rest, up to a multiple of 32, is padding)
     const uint32_t* labels;  // EPI_CE
     uint32_t ignore_id;      // EPI_CE
     uint32_t n_tiles;        // EPI_CE: (max, sum exp) partials per row: one per vocabulary tile and epilogue warp group
@@ -92,9 +93,9 @@ template <int EPI, typename SB = float, bool STAGED16 = false>
 __device__ __forceinline__ void epilogue(const GemmParams& p, const GemmProblem& pr, uint32_t taddr, uint32_t m,
                                          uint32_t n0, const SB* s_scale, const SB* s_bias, int lane, uint32_t part,
                                          uint32_t c_begin = 0, uint32_t c_end = BN / 32, float* stage = nullptr) {
-    const bool row_ok = m < p.M;
-    // EPI_SIGNBITS: the 32 rows of this warp are 32 consecutive steps of one sequence (M, time % 32 == 0)
+    // EPI_SIGNBITS: the 32 rows of this warp are 32 consecutive rows of one sequence (M, time % 32 == 0)
     const uint32_t m_warp = m - lane;
+    const bool row_ok = m < p.M && (EPI != EPI_SIGNBITS || m_warp % p.time + lane < p.steps);
     const float s1 = (EPI == EPI_SIGNBITS && row_ok) ? pr.aux[m] : 0.0f;
     // EPI_CE running state
     float run_max = -INFINITY, run_sum = 0.0f;
