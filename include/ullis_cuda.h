@@ -115,6 +115,12 @@ ULLIS_CUDA_API int32_t ullis_cuda_runtime_kernel_names(ullis_cuda_runtime* rt, c
  * No counterpart in the reference, which runs every stream through RosaSam.  Synchronises. */
 ULLIS_CUDA_API int32_t ullis_cuda_runtime_sam_counts(ullis_cuda_runtime* rt, uint64_t* total, uint64_t* automaton,
                                                      uint64_t* constant_q);
+/* Page-locked host memory: a call that reads its inputs from it or writes its results into it copies at the rate of the
+ * link, without the driver's staging.  Any other host memory works too.  Freed with ullis_cuda_host_free, which any
+ * thread may call as long as no call is using the block. */
+ULLIS_CUDA_API int32_t ullis_cuda_host_alloc(ullis_cuda_runtime* rt, size_t bytes, void** out);
+ULLIS_CUDA_API void ullis_cuda_host_free(void* block);
+
 /* Error-path self-test: one small kernel waits - with the bounded mbarrier wait that every tensor-core kernel of
  * the library uses, cut to `polls` polls (1..2^20) - on a barrier nothing ever arrives on, gives up, returns by
  * itself and reports through the device status words.  The expected result is ULLIS_CUDA_ERR_TIMEOUT with

@@ -113,6 +113,8 @@ unsafe extern "C" {
         automaton: *mut u64,
         constant_q: *mut u64,
     ) -> i32;
+    pub fn ullis_cuda_host_alloc(rt: *mut ullis_cuda_runtime, bytes: usize, out: *mut *mut c_void) -> i32;
+    pub fn ullis_cuda_host_free(block: *mut c_void);
     pub fn ullis_cuda_runtime_wait_selftest(rt: *mut ullis_cuda_runtime, polls: u32) -> i32;
     pub fn ullis_cuda_runtime_is_sm100(rt: *const ullis_cuda_runtime) -> i32;
     pub fn ullis_cuda_model_load_safetensors(

@@ -66,6 +66,38 @@ T* stage(ullis_cuda_runtime* rt, int slot, const T* host, size_t count) {
     return dev;
 }
 
+// The inputs of an op-level call.  Small ones are gathered and cross the link in one copy (send()): seventeen copies
+// of a few KB from pageable memory were 80 us of a ROSA block call of 260.  The call synchronises before it returns,
+// so the memory is free again for the next one.
+struct Inputs {
+    ullis_cuda_runtime* rt;
+    explicit Inputs(ullis_cuda_runtime* r) : rt(r) {
+        if (!rt->inputs_host) {
+            void* p = nullptr;
+            ULLIS_CUDA_CHECK(cudaHostAlloc(&p, ullis_cuda_runtime::INPUTS_BYTES, cudaHostAllocDefault));
+            rt->inputs_host = static_cast<uint8_t*>(p);
+            rt->inputs_dev.ensure(ullis_cuda_runtime::INPUTS_BYTES);
+        }
+        // a call that failed half way did not wait for its copy
+        if (rt->inputs_sent && cudaStreamQuery(rt->stream) != cudaSuccess) rt->sync();
+        rt->inputs_used = rt->inputs_sent = 0;
+    }
+    template <typename T>
+    T* add(int slot, const T* host, size_t count) {
+        const size_t bytes = count * sizeof(T), at = (rt->inputs_used + 255) / 256 * 256;
+        if (bytes > ullis_cuda_runtime::SMALL_INPUT || at + bytes > ullis_cuda_runtime::INPUTS_BYTES)
+            return stage(rt, slot, host, count);
+        std::memcpy(rt->inputs_host + at, host, bytes);
+        rt->inputs_used = at + bytes;
+        return reinterpret_cast<T*>(static_cast<uint8_t*>(rt->inputs_dev.get()) + at);
+    }
+    void send() {   // before the first kernel
+        rt->h2d(static_cast<uint8_t*>(rt->inputs_dev.get()) + rt->inputs_sent, rt->inputs_host + rt->inputs_sent,
+                rt->inputs_used - rt->inputs_sent);
+        rt->inputs_sent = rt->inputs_used;
+    }
+};
+
 void packed_linear_dev(ullis_cuda_runtime* rt, const float* x, const uint32_t* bits, const uint16_t* scale,
                        const uint16_t* bias, float* y, size_t rows, size_t K, size_t N) {
     if (rt->mode == ULLIS_CUDA_MODE_EXACT || !tc::binary_linear(rt, x, bits, scale, bias, y, rows, K, N))
@@ -347,6 +379,7 @@ int32_t ullis_cuda_runtime_create(int32_t device, ullis_cuda_runtime** out) {
 void ullis_cuda_runtime_destroy(ullis_cuda_runtime* rt) {
     if (!rt) return;
     cudaSetDevice(rt->device);
+    if (rt->inputs_host) cudaFreeHost(rt->inputs_host);
     for (ullis_cuda_runtime* c : rt->children) {
         c->dev_status = nullptr;    // the parent's
         c->host_status = nullptr;
@@ -454,6 +487,22 @@ int32_t ullis_cuda_runtime_sam_counts(ullis_cuda_runtime* rt, uint64_t* total, u
         if (automaton) *automaton = sum[1];
         if (constant_q) *constant_q = sum[2];
     });
+}
+
+int32_t ullis_cuda_host_alloc(ullis_cuda_runtime* rt, size_t bytes, void** out) {
+    return guard(rt, [&] {
+        need_ptr(out, "out");
+        *out = nullptr;
+        if (cudaHostAlloc(out, bytes ? bytes : 1, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            *out = nullptr;
+            fail(ULLIS_CUDA_ERR_NOMEM, "page-locked host allocation failed");
+        }
+    });
+}
+
+void ullis_cuda_host_free(void* block) {
+    if (block) cudaFreeHost(block);
 }
 
 int32_t ullis_cuda_runtime_wait_selftest(ullis_cuda_runtime* rt, uint32_t polls) {
@@ -830,10 +879,12 @@ int32_t ullis_cuda_layer_norm(ullis_cuda_runtime* rt, const float* x, const uint
         const size_t n = mul_or_fail(rows, channels, "LayerNorm");
         if (n == 0) return;
         need_ptr(x, "x"); need_ptr(weight, "weight"); need_ptr(bias, "bias"); need_ptr(y, "y");
-        float* dx = stage(rt, 0, x, n);
-        uint16_t* dw = stage(rt, 1, weight, channels);
-        uint16_t* db = stage(rt, 2, bias, channels);
+        Inputs in(rt);
+        float* dx = in.add(0, x, n);
+        uint16_t* dw = in.add(1, weight, channels);
+        uint16_t* db = in.add(2, bias, channels);
         float* dy = rt->pool[3].as<float>(n);
+        in.send();
         k::layer_norm(rt, dx, dw, db, dy, rows, channels, rt->mode == ULLIS_CUDA_MODE_EXACT);
         rt->d2h(y, dy, n * 4);
         rt->sync();
@@ -865,11 +916,13 @@ int32_t ullis_cuda_binary_linear(ullis_cuda_runtime* rt, const float* x, const u
         const size_t words = (mul_or_fail(in_features, out_features, "packed linear") + 31) / 32;
         if (rows == 0) return;
         need_ptr(x, "x"); need_ptr(bits, "bits"); need_ptr(scale, "scale"); need_ptr(y, "y");
-        float* dx = stage(rt, 0, x, nx);
-        uint32_t* dbits = stage(rt, 1, bits, words);
-        uint16_t* ds = stage(rt, 2, scale, out_features);
-        uint16_t* db = bias ? stage(rt, 3, bias, out_features) : nullptr;
+        Inputs in(rt);
+        float* dx = in.add(0, x, nx);
+        uint32_t* dbits = in.add(1, bits, words);
+        uint16_t* ds = in.add(2, scale, out_features);
+        uint16_t* db = bias ? in.add(3, bias, out_features) : nullptr;
         float* dy = rt->pool[4].as<float>(ny);
+        in.send();
         rt->clear_status();
         packed_linear_dev(rt, dx, dbits, ds, db, dy, rows, in_features, out_features);
         rt->d2h(y, dy, ny * 4);
@@ -886,9 +939,11 @@ int32_t ullis_cuda_fp16_linear(ullis_cuda_runtime* rt, const float* x, const uin
         const size_t nw = mul_or_fail(in_features, out_features, "FP16 linear");
         if (rows == 0) return;
         need_ptr(x, "x"); need_ptr(weight, "weight"); need_ptr(y, "y");
-        float* dx = stage(rt, 0, x, nx);
-        uint16_t* dw = stage(rt, 1, weight, nw);
+        Inputs in(rt);
+        float* dx = in.add(0, x, nx);
+        uint16_t* dw = in.add(1, weight, nw);
         float* dy = rt->pool[2].as<float>(ny);
+        in.send();
         rt->clear_status();
         dense_linear_dev(rt, dx, dw, dy, rows, in_features, out_features);
         rt->d2h(y, dy, ny * 4);
@@ -943,14 +998,16 @@ int32_t ullis_cuda_rosa_qkv_1bit_fwd(ullis_cuda_runtime* rt, const uint32_t* q_b
         const size_t n = mul_or_fail(mul_or_fail(batch, time, "ROSA"), channels, "ROSA");
         need_ptr(q_bits, "q_bits"); need_ptr(k_bits, "k_bits"); need_ptr(v_bits, "v_bits"); need_ptr(e, "e");
         const size_t words = (n + 31) / 32, wps = (time + 31) / 32, sw = batch * channels * wps;
-        uint32_t* dq = stage(rt, 0, q_bits, words);
-        uint32_t* dk = stage(rt, 1, k_bits, words);
-        uint32_t* dv = stage(rt, 2, v_bits, words);
-        uint16_t* de = stage(rt, 3, e, channels);
+        Inputs in(rt);
+        uint32_t* dq = in.add(0, q_bits, words);
+        uint32_t* dk = in.add(1, k_bits, words);
+        uint32_t* dv = in.add(2, v_bits, words);
+        uint16_t* de = in.add(3, e, channels);
         uint32_t* qs = rt->pool[4].as<uint32_t>(sw);
         uint32_t* ks = rt->pool[5].as<uint32_t>(sw);
         uint32_t* vs = rt->pool[6].as<uint32_t>(sw);
         uint32_t* is = rt->pool[7].as<uint32_t>(sw);
+        in.send();
         k::planes_to_streams(rt, dq, qs, batch, time, channels);
         k::planes_to_streams(rt, dk, ks, batch, time, channels);
         k::planes_to_streams(rt, dv, vs, batch, time, channels);
@@ -982,16 +1039,17 @@ int32_t ullis_cuda_rosa_block_forward(ullis_cuda_runtime* rt, const float* x, co
                              v_bits, v_scale, v_bias, e, o_bits, o_scale, o_bias};
         for (const void* p : req) need_ptr(p, "ROSA block argument");
         LayerWeights L;
-        float* dx = stage(rt, 0, x, n);
-        L.x_q = stage(rt, 1, mix_q, d);
-        L.x_k = stage(rt, 2, mix_k, d);
-        L.x_v = stage(rt, 3, mix_v, d);
-        L.e = stage(rt, 4, e, d);
+        Inputs in(rt);
+        float* dx = in.add(0, x, n);
+        L.x_q = in.add(1, mix_q, d);
+        L.x_k = in.add(2, mix_k, d);
+        L.x_v = in.add(3, mix_v, d);
+        L.e = in.add(4, e, d);
         auto lin = [&](PackedWeights& w, int slot, const uint32_t* b, const uint16_t* s, const uint16_t* bi) {
             w.out = d; w.in = d;
-            w.bits = stage(rt, slot, b, words);
-            w.scale = stage(rt, slot + 1, s, d);
-            w.bias = stage(rt, slot + 2, bi, d);
+            w.bits = in.add(slot, b, words);
+            w.scale = in.add(slot + 1, s, d);
+            w.bias = in.add(slot + 2, bi, d);
         };
         lin(L.q, 5, q_bits, q_scale, q_bias);
         lin(L.k, 8, k_bits, k_scale, k_bias);
@@ -1002,6 +1060,7 @@ int32_t ullis_cuda_rosa_block_forward(ullis_cuda_runtime* rt, const float* x, co
         float *bq = work, *bk = work + n, *bv = work + 2 * n, *w = work + 3 * n, *dout = work + 4 * n;
         uint32_t* sws = rt->pool[18].as<uint32_t>(sw * 4);
         uint32_t *qs = sws, *ks = sws + sw, *vs = sws + 2 * sw, *is = sws + 3 * sw;
+        in.send();
         rt->clear_status();
         const bool exact = rt->mode == ULLIS_CUDA_MODE_EXACT;
         if (exact || !tc::rosa_qkv_bits(rt, dx, L, qs, ks, vs, batch, time, d)) {
@@ -1018,14 +1077,13 @@ int32_t ullis_cuda_rosa_block_forward(ullis_cuda_runtime* rt, const float* x, co
         k::rosa_emit(rt, is, L.e, didx, w, batch, time, d);  // w <- y
         packed_linear_dev(rt, w, L.o.bits, L.o.scale, L.o.bias, dout, rows, d, d);
         const size_t plane_words = (n + 31) / 32;
-        uint32_t* dplane = rt->pool[20].as<uint32_t>(plane_words);
+        uint32_t* dplanes = rt->pool[20].as<uint32_t>(3 * plane_words);
         uint32_t* planes_out[3] = {q_plane, k_plane, v_plane};
         uint32_t* planes_in[3] = {qs, ks, vs};
         for (int i = 0; i < 3; ++i) {
             if (!planes_out[i]) continue;
-            k::streams_to_planes(rt, planes_in[i], dplane, batch, time, d);
-            rt->d2h(planes_out[i], dplane, plane_words * 4);
-            rt->sync();  // dplane is reused
+            k::streams_to_planes(rt, planes_in[i], dplanes + i * plane_words, batch, time, d);
+            rt->d2h(planes_out[i], dplanes + i * plane_words, plane_words * 4);
         }
         if (idx) rt->d2h(idx, didx, n);
         if (y) rt->d2h(y, w, n * 4);
@@ -1046,14 +1104,16 @@ int32_t ullis_cuda_cmix_block_forward(ullis_cuda_runtime* rt, const float* x, co
         const size_t nw = mul_or_fail(d_model, dim_ffn, "CMix");
         need_ptr(x, "x"); need_ptr(mix, "mix"); need_ptr(key_bits, "key_bits"); need_ptr(key_scale, "key_scale");
         need_ptr(value, "value"); need_ptr(out, "out");
-        float* dx = stage(rt, 0, x, n);
-        uint16_t* dm = stage(rt, 1, mix, d_model);
-        uint32_t* dkb = stage(rt, 2, key_bits, (nw + 31) / 32);
-        uint16_t* dks = stage(rt, 3, key_scale, dim_ffn);
-        uint16_t* dv = stage(rt, 4, value, nw);
+        Inputs in(rt);
+        float* dx = in.add(0, x, n);
+        uint16_t* dm = in.add(1, mix, d_model);
+        uint32_t* dkb = in.add(2, key_bits, (nw + 31) / 32);
+        uint16_t* dks = in.add(3, key_scale, dim_ffn);
+        uint16_t* dv = in.add(4, value, nw);
         float* sh = rt->pool[5].as<float>(n);
         float* key = rt->pool[6].as<float>(nf);
         float* dout = rt->pool[7].as<float>(n);
+        in.send();
         rt->clear_status();
         k::shift_mix(rt, dx, dm, nullptr, nullptr, sh, nullptr, nullptr, rows, time, d_model);
         packed_linear_dev(rt, sh, dkb, dks, nullptr, key, rows, d_model, dim_ffn);
@@ -1079,15 +1139,17 @@ int32_t ullis_cuda_streamed_ce(ullis_cuda_runtime* rt, const float* hidden, cons
             return;
         }
         need_ptr(hidden, "hidden"); need_ptr(bits, "bits"); need_ptr(scale, "scale"); need_ptr(labels, "labels");
-        float* dh = stage(rt, 0, hidden, nh);
+        Inputs in(rt);
+        float* dh = in.add(0, hidden, nh);
         PackedWeights head;
         head.out = vocab; head.in = channels;
-        head.bits = stage(rt, 1, bits, words);
-        head.scale = stage(rt, 2, scale, vocab);
-        head.bias = bias ? stage(rt, 3, bias, vocab) : nullptr;
-        uint32_t* dl = stage(rt, 4, labels, rows);
+        head.bits = in.add(1, bits, words);
+        head.scale = in.add(2, scale, vocab);
+        head.bias = bias ? in.add(3, bias, vocab) : nullptr;
+        uint32_t* dl = in.add(4, labels, rows);
         float* rl = rt->pool[5].as<float>(rows);
         uint8_t* res = static_cast<uint8_t*>(rt->pool[6].ensure(16));
+        in.send();
         rt->clear_status();
         if (rt->mode == ULLIS_CUDA_MODE_EXACT ||
             !tc::head_ce(rt, dh, head, dl, ignore_id, rows, time, channels, vocab, rl)) {

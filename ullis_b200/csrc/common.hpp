@@ -129,6 +129,11 @@ struct ullis_cuda_runtime {
     uint32_t* dev_status = nullptr;     // 4 words, device
     uint32_t* host_status = nullptr;    // 4 words, pinned
     ullis::DeviceBuffer pool[24];       // op-level scratch slots
+    // Small inputs of one op-level call, side by side in page-locked memory and copied to the device together.
+    static constexpr size_t INPUTS_BYTES = 1 << 20, SMALL_INPUT = 64 << 10;
+    uint8_t* inputs_host = nullptr;
+    ullis::DeviceBuffer inputs_dev;
+    size_t inputs_used = 0, inputs_sent = 0;
     size_t sam_budget_bytes = (size_t)12 << 30;   // cap of sam_scratch; more streams than fit run in waves
     ullis::DeviceBuffer sam_scratch;    // suffix-automaton state blocks
     ullis::DeviceBuffer sam_list;       // ids of the streams that need the automaton + their count

@@ -18,6 +18,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import threading
 
 import numpy as np
 
@@ -54,7 +55,8 @@ ABI_SYMBOLS = (
     "ullis_cuda_binary_linear", "ullis_cuda_fp16_linear", "ullis_cuda_sign_pack_bits", "ullis_cuda_cmix_relu2",
     "ullis_cuda_residual_add", "ullis_cuda_rosa_qkv_1bit_fwd", "ullis_cuda_rosa_block_forward",
     "ullis_cuda_cmix_block_forward", "ullis_cuda_streamed_ce", "ullis_cuda_rosa_sam_static",
-    "ullis_cuda_runtime_sam_counts", "ullis_cuda_runtime_wait_selftest", "ullis_cuda_model_read_loss_global", "ullis_cuda_dp_rendezvous",
+    "ullis_cuda_runtime_sam_counts", "ullis_cuda_runtime_wait_selftest", "ullis_cuda_host_alloc",
+    "ullis_cuda_host_free", "ullis_cuda_model_read_loss_global", "ullis_cuda_dp_rendezvous",
     "ullis_cuda_dp_unique_id", "ullis_cuda_dp_init",
     "ullis_cuda_dp_allreduce_loss", "ullis_cuda_dp_finalize",
 )
@@ -93,6 +95,8 @@ def load_library() -> C.CDLL:
         lib.ullis_cuda_rosa_pushers_destroy.argtypes = [C.c_void_p]
         lib.ullis_cuda_train_state_destroy.restype = None
         lib.ullis_cuda_train_state_destroy.argtypes = [C.c_void_p]
+        lib.ullis_cuda_host_free.restype = None
+        lib.ullis_cuda_host_free.argtypes = [C.c_void_p]
         lib.ullis_cuda_generate_state_time.restype = C.c_size_t
         lib.ullis_cuda_generate_state_time.argtypes = [C.c_void_p]
         _LIB = lib
@@ -140,6 +144,76 @@ def _z(n):
     return C.c_size_t(int(n))
 
 
+class _ResultBlock:
+    """One page-locked block lent to a numpy array; it goes back to the pool with the last array that looks at it."""
+
+    __slots__ = ("addr", "size", "__array_interface__")
+
+    def __init__(self, addr: int, size: int, nbytes: int):
+        self.addr, self.size = addr, size
+        self.__array_interface__ = {"data": (addr, False), "shape": (nbytes,), "typestr": "|u1", "version": 3}
+
+    def __del__(self):
+        if _RESULTS is not None:             # not while the interpreter shuts down
+            _RESULTS.give_back(self.addr, self.size)
+
+
+class _ResultPool:
+    """Page-locked memory for result arrays.  A fresh numpy array is pageable memory nobody has touched: the copy into
+    it went through the driver's staging buffer and took a page fault every 4 KB (168 MB of ROSA results: 36 ms, now 4).
+    Blocks are reused once the arrays over them are gone.  At most `limit` bytes are page-locked, lent and idle
+    together; beyond that results are ordinary arrays."""
+
+    def __init__(self, limit: int = 1 << 30, smallest: int = 64):
+        self.limit, self.smallest = limit, smallest
+        self._idle = {}                      # block size -> [addresses]
+        self._held = 0                       # bytes page-locked
+        self._lock = threading.RLock()       # a garbage collection inside empty() may give a block back
+
+    @staticmethod
+    def _block_size(nbytes: int) -> int:
+        step = 1 << max(12, nbytes.bit_length() - 3)      # eighths of a power of two
+        return (nbytes + step - 1) // step * step
+
+    def empty(self, rt: "CudaRuntime", shape, dtype) -> np.ndarray:
+        dtype = np.dtype(dtype)
+        nbytes = dtype.itemsize * (int(np.prod(shape)) if isinstance(shape, tuple) else int(shape))
+        if nbytes < self.smallest:
+            return np.empty(shape, dtype)
+        size = self._block_size(nbytes)
+        with self._lock:
+            idle = self._idle.get(size)
+            addr = idle.pop() if idle else self._lock_memory(rt, size)
+        if addr is None:
+            return np.empty(shape, dtype)
+        return np.asarray(_ResultBlock(addr, size, nbytes)).view(dtype).reshape(shape)
+
+    def _lock_memory(self, rt, size):
+        if self._held + size > self.limit:
+            self._drop_idle(self._held + size - self.limit)
+            if self._held + size > self.limit:
+                return None
+        p = C.c_void_p()
+        if rt._lib.ullis_cuda_host_alloc(rt._h, C.c_size_t(size), C.byref(p)) != OK:
+            return None
+        self._held += size
+        return p.value
+
+    def _drop_idle(self, nbytes):
+        for size in sorted(self._idle, reverse=True):
+            while nbytes > 0 and self._idle[size]:
+                _LIB.ullis_cuda_host_free(C.c_void_p(self._idle[size].pop()))
+                self._held -= size
+                nbytes -= size
+
+    def give_back(self, addr, size):
+        with self._lock:
+            self._idle.setdefault(size, []).append(addr)
+
+
+_RESULTS = _ResultPool()
+
+
 class CudaRuntime:
     """One per device per process, used from one thread (like MetalRuntime)."""
 
@@ -169,6 +243,9 @@ class CudaRuntime:
     def _check(self, rc: int):
         if rc != OK:
             raise UllisCudaError(rc, self._lib.ullis_cuda_last_error(self._h).decode())
+
+    def _empty(self, shape, dtype) -> np.ndarray:
+        return _RESULTS.empty(self, shape, dtype)
 
     # ---- options / introspection
     def set_mode(self, mode: int):
@@ -214,13 +291,13 @@ class CudaRuntime:
         x = _arr(x, np.float32, "x", rows * channels)
         w = _arr(weight_bits, np.uint16, "weight", channels)
         b = _arr(bias_bits, np.uint16, "bias", channels)
-        y = np.empty(rows * channels, np.float32)
+        y = self._empty(rows * channels, np.float32)
         self._check(self._lib.ullis_cuda_layer_norm(self._h, _ptr(x), _ptr(w), _ptr(b), _ptr(y), _z(rows), _z(channels)))
         return y
 
     def time_shift_delta(self, x, rows: int, time: int, channels: int) -> np.ndarray:
         x = _arr(x, np.float32, "x", rows * channels)
-        xx = np.empty(rows * channels, np.float32)
+        xx = self._empty(rows * channels, np.float32)
         self._check(self._lib.ullis_cuda_time_shift_delta(self._h, _ptr(x), _ptr(xx), _z(rows), _z(time), _z(channels)))
         return xx
 
@@ -229,7 +306,7 @@ class CudaRuntime:
         bits = _arr(bits, np.uint32, "bits", (in_features * out_features + 31) // 32)
         s = _arr(scale_bits, np.uint16, "scale", out_features)
         b = _arr(bias_bits, np.uint16, "bias", out_features, allow_none=True)
-        y = np.empty(rows * out_features, np.float32)
+        y = self._empty(rows * out_features, np.float32)
         self._check(self._lib.ullis_cuda_binary_linear(self._h, _ptr(x), _ptr(bits), _ptr(s), _ptr(b), _ptr(y),
                                                        _z(rows), _z(in_features), _z(out_features)))
         return y
@@ -237,7 +314,7 @@ class CudaRuntime:
     def fp16_linear(self, x, weight_bits, rows: int, in_features: int, out_features: int) -> np.ndarray:
         x = _arr(x, np.float32, "x", rows * in_features)
         w = _arr(weight_bits, np.uint16, "weight", in_features * out_features)
-        y = np.empty(rows * out_features, np.float32)
+        y = self._empty(rows * out_features, np.float32)
         self._check(self._lib.ullis_cuda_fp16_linear(self._h, _ptr(x), _ptr(w), _ptr(y), _z(rows), _z(in_features),
                                                      _z(out_features)))
         return y
@@ -250,7 +327,7 @@ class CudaRuntime:
 
     def cmix_relu2(self, x) -> np.ndarray:
         x = _arr(x, np.float32, "x")
-        y = np.empty(x.size, np.float32)
+        y = self._empty(x.size, np.float32)
         self._check(self._lib.ullis_cuda_cmix_relu2(self._h, _ptr(x), _ptr(y), _z(x.size)))
         return y
 
@@ -258,7 +335,7 @@ class CudaRuntime:
         w = _arr(parameters, np.uint16, "parameters")
         r = _arr(residual, np.float32, "residual", w.size)
         g = _arr(gradient, np.float32, "gradient", w.size)
-        nw, nr = np.empty(w.size, np.uint16), np.empty(w.size, np.float32)
+        nw, nr = self._empty(w.size, np.uint16), self._empty(w.size, np.float32)
         self._check(fn(self._h, _ptr(w), _ptr(r), _ptr(g), C.c_float(learning_rate), *extra, _z(w.size), _ptr(nw),
                        _ptr(nr)))
         return nw, nr
@@ -276,8 +353,8 @@ class CudaRuntime:
         w = _arr(latent, np.uint16, "latent")
         r = _arr(residual, np.float32, "residual", w.size)
         g = _arr(gradient, np.float32, "gradient", w.size)
-        nw, nr = np.empty(w.size, np.uint16), np.empty(w.size, np.float32)
-        bits = np.empty((w.size + 31) // 32, np.uint32)
+        nw, nr = self._empty(w.size, np.uint16), self._empty(w.size, np.float32)
+        bits = self._empty((w.size + 31) // 32, np.uint32)
         self._check(self._lib.ullis_cuda_apply_latent_sgd(self._h, _ptr(w), _ptr(r), _ptr(g), C.c_float(learning_rate),
                                                           C.c_float(ste_scale), _z(w.size), _ptr(nw), _ptr(nr),
                                                           _ptr(bits)))
@@ -288,7 +365,7 @@ class CudaRuntime:
         n = batch * time * channels
         gy = _arr(output_gradient, np.float32, "output_gradient", n)
         ix = _arr(idx, np.uint8, "idx", n)
-        out = np.empty(channels, np.float32)
+        out = self._empty(channels, np.float32)
         self._check(self._lib.ullis_cuda_rosa_qkv_1bit_bwd_e(self._h, _ptr(gy), _ptr(ix), _z(batch), _z(time),
                                                              _z(channels), _ptr(out)))
         return out
@@ -297,7 +374,7 @@ class CudaRuntime:
         """MetalRuntime::cmix_relu2_backward (src/metal.rs:1546)."""
         x = _arr(input, np.float32, "input")
         g = _arr(output_gradient, np.float32, "output_gradient", x.size)
-        out = np.empty(x.size, np.float32)
+        out = self._empty(x.size, np.float32)
         self._check(self._lib.ullis_cuda_cmix_relu2_backward(self._h, _ptr(x), _ptr(g), _ptr(out), _z(x.size)))
         return out
 
@@ -306,7 +383,7 @@ class CudaRuntime:
         x = _arr(input, np.float32, "input", rows * channels)
         g = _arr(output_gradient, np.float32, "output_gradient", rows * channels)
         w = _arr(weight_bits, np.uint16, "weight", channels)
-        gx, gw, gb = np.empty(x.size, np.float32), np.empty(channels, np.float32), np.empty(channels, np.float32)
+        gx, gw, gb = self._empty(x.size, np.float32), self._empty(channels, np.float32), self._empty(channels, np.float32)
         self._check(self._lib.ullis_cuda_layer_norm_backward(self._h, _ptr(x), _ptr(g), _ptr(w), _z(rows), _z(channels),
                                                              _ptr(gx), _ptr(gw), _ptr(gb)))
         return gx, gw, gb
@@ -314,7 +391,7 @@ class CudaRuntime:
     def residual_add(self, residual, update) -> np.ndarray:
         a = _arr(residual, np.float32, "residual")
         b = _arr(update, np.float32, "update", a.size)
-        out = np.empty(a.size, np.float32)
+        out = self._empty(a.size, np.float32)
         self._check(self._lib.ullis_cuda_residual_add(self._h, _ptr(a), _ptr(b), _ptr(out), _z(a.size)))
         return out
 
@@ -328,8 +405,8 @@ class CudaRuntime:
         k = _arr(k_bits, np.uint32, "k_bits", words)
         v = _arr(v_bits, np.uint32, "v_bits", words)
         e = _arr(e_bits, np.uint16, "e", channels)
-        idx = np.empty(n, np.uint8)
-        out = np.empty(n, np.float32) if want_out else None
+        idx = self._empty(n, np.uint8)
+        out = self._empty(n, np.float32) if want_out else None
         self._check(self._lib.ullis_cuda_rosa_qkv_1bit_fwd(self._h, _ptr(q), _ptr(k), _ptr(v), _ptr(e), _ptr(idx),
                                                            _ptr(out), _z(batch), _z(time), _z(channels)))
         return idx, out
@@ -349,9 +426,9 @@ class CudaRuntime:
         o = [_arr(p["o"]["bits"], np.uint32, "o.bits", (d * d + 31) // 32),
              _arr(p["o"]["scale"], np.uint16, "o.scale", d), _arr(p["o"]["bias"], np.uint16, "o.bias", d)]
         words = (n + 31) // 32
-        r = {"q_plane": np.empty(words, np.uint32), "k_plane": np.empty(words, np.uint32),
-             "v_plane": np.empty(words, np.uint32), "idx": np.empty(n, np.uint8),
-             "y": np.empty(n, np.float32), "out": np.empty(n, np.float32)}
+        r = {"q_plane": self._empty(words, np.uint32), "k_plane": self._empty(words, np.uint32),
+             "v_plane": self._empty(words, np.uint32), "idx": self._empty(n, np.uint8),
+             "y": self._empty(n, np.float32), "out": self._empty(n, np.float32)}
         self._check(self._lib.ullis_cuda_rosa_block_forward(
             self._h, _ptr(x), *[_ptr(a) for a in args], *[_ptr(a) for a in lin], _ptr(e), *[_ptr(a) for a in o],
             _z(batch), _z(time), _z(d), _ptr(r["q_plane"]), _ptr(r["k_plane"]), _ptr(r["v_plane"]), _ptr(r["idx"]),
@@ -366,7 +443,7 @@ class CudaRuntime:
         kb = _arr(key_bits, np.uint32, "key_bits", (d_model * dim_ffn + 31) // 32)
         ks = _arr(key_scale_bits, np.uint16, "key_scale", dim_ffn)
         val = _arr(value_bits, np.uint16, "value", d_model * dim_ffn)
-        out = np.empty(n, np.float32)
+        out = self._empty(n, np.float32)
         self._check(self._lib.ullis_cuda_cmix_block_forward(self._h, _ptr(x), _ptr(mix), _ptr(kb), _ptr(ks),
                                                             _ptr(val), _z(batch), _z(time), _z(d_model),
                                                             _z(dim_ffn), _ptr(out)))
@@ -380,7 +457,7 @@ class CudaRuntime:
         s = _arr(scale_bits, np.uint16, "scale", vocab)
         b = _arr(bias_bits, np.uint16, "bias", vocab, allow_none=True)
         lab = _arr(labels, np.uint32, "labels", rows)
-        row_loss = np.empty(rows, np.float32)
+        row_loss = self._empty(rows, np.float32)
         mean = C.c_float(0)
         n_valid = C.c_uint64(0)
         self._check(self._lib.ullis_cuda_streamed_ce(self._h, _ptr(h), _ptr(bits), _ptr(s), _ptr(b), _ptr(lab),
@@ -482,7 +559,7 @@ class CudaHeron:
         t = _arr(tokens, np.uint32, "tokens", batch * time)
         lab = _arr(labels, np.uint32, "labels", batch * time)
         mean, s, n = C.c_float(0), C.c_double(0), C.c_uint64(0)
-        rl = np.empty(batch * time, np.float32) if want_row_loss else None
+        rl = self.rt._empty(batch * time, np.float32) if want_row_loss else None
         self.rt._check(self._lib.ullis_cuda_model_forward_ce(self._h, _ptr(t), _ptr(lab), C.c_uint32(ignore_id),
                                                              _z(batch), _z(time), C.byref(mean), C.byref(s),
                                                              C.byref(n), _ptr(rl)))
@@ -500,7 +577,7 @@ class CudaHeron:
 
     def read_loss(self, rows: int = 0, want_row_loss: bool = False):
         mean, s, n = C.c_float(0), C.c_double(0), C.c_uint64(0)
-        rl = np.empty(rows, np.float32) if want_row_loss else None
+        rl = self.rt._empty(rows, np.float32) if want_row_loss else None
         self.rt._check(self._lib.ullis_cuda_model_read_loss(self._h, C.byref(mean), C.byref(s), C.byref(n),
                                                             _ptr(rl), _z(rows)))
         out = (float(mean.value), float(s.value), int(n.value))
@@ -515,13 +592,13 @@ class CudaHeron:
 
     def logits(self, tokens, batch: int, time: int) -> np.ndarray:
         t = _arr(tokens, np.uint32, "tokens", batch * time)
-        out = np.empty(batch * time * self.vocab_size, np.float32)
+        out = self.rt._empty(batch * time * self.vocab_size, np.float32)
         self.rt._check(self._lib.ullis_cuda_model_logits(self._h, _ptr(t), _z(batch), _z(time), _ptr(out)))
         return out
 
     def hidden(self, tokens, batch: int, time: int) -> np.ndarray:
         t = _arr(tokens, np.uint32, "tokens", batch * time)
-        out = np.empty(batch * time * self.d_model, np.float32)
+        out = self.rt._empty(batch * time * self.d_model, np.float32)
         self.rt._check(self._lib.ullis_cuda_model_hidden(self._h, _ptr(t), _z(batch), _z(time), _ptr(out)))
         return out
 
@@ -543,7 +620,7 @@ class CudaHeron:
     def tap(self, layer: int, which: str, rows: int) -> np.ndarray:
         code = TAPS[which]
         dtype = np.uint8 if 2 <= code <= 5 else np.float32
-        out = np.empty(rows * self.d_model, dtype)
+        out = self.rt._empty(rows * self.d_model, dtype)
         self.rt._check(self._lib.ullis_cuda_model_tap(self._h, C.c_int32(layer), C.c_int32(code), _ptr(out),
                                                       _z(out.nbytes)))
         return out
@@ -581,7 +658,7 @@ class CudaGenerateState:
 
     def step(self, tokens) -> np.ndarray:
         t = _arr(np.atleast_1d(tokens), np.uint32, "tokens", self.batch)
-        out = np.empty((self.batch, self.model.vocab_size), np.float32)
+        out = self.model.rt._empty((self.batch, self.model.vocab_size), np.float32)
         self.model.rt._check(self._lib.ullis_cuda_generate_step(self._h, _ptr(t), _ptr(out)))
         return out
 
@@ -614,7 +691,7 @@ class CudaRosaPushers:
         q = np.ascontiguousarray(np.atleast_2d(q), np.uint8)
         steps = q.shape[0]
         q, k, v = (_arr(np.atleast_2d(a), np.uint8, n, steps * self.streams) for a, n in ((q, "q"), (k, "k"), (v, "v")))
-        idx = np.empty((steps, self.streams), np.uint8)
+        idx = self.rt._empty((steps, self.streams), np.uint8)
         self.rt._check(self._lib.ullis_cuda_rosa_pushers_push(self._handle.h, _ptr(q), _ptr(k), _ptr(v), _z(steps), _ptr(idx)))
         return idx
 
@@ -678,7 +755,7 @@ class CudaTrainState:
 
     def read(self, name: str, dtype, count: int) -> np.ndarray:
         """Tensor of the trained model or of its carry by checkpoint name (u16 = FP16 bits)."""
-        out = np.empty(count, dtype)
+        out = self.model.rt._empty(count, dtype)
         self.model.rt._check(self._lib.ullis_cuda_train_state_read(self._h, name.encode(), _ptr(out),
                                                                    _z(out.nbytes)))
         return out
