@@ -1,0 +1,173 @@
+// RosaSam::push (src/rosa.rs:100-176) for streams that advance one step per call, without an automaton.
+//
+// rosa_match.cuh says what a push computes: the position r < i whose key history agrees with the query history of
+// step i over the most steps, the latest of equals, and the v bit after it.  While the lag of the step before still
+// matches it stays the answer (the matches of step i are those of step i - 1 that go on), which is one bit to look at;
+// otherwise a warp compares the last 32 query bits with the 32 key bits before every position, 32 positions per
+// handful of instructions, and counts on beyond 32 steps only where all of them agree.  A stream is its three bit
+// histories and a lag: 3 * T / 8 + 16 bytes (at T = 2048 784 instead of the 28.7 KB of an automaton with its
+// chain), and the cost of a step grows with i / 32 and not with the runs of the keys.
+#pragma once
+#include <stdint.h>
+
+namespace ullis {
+namespace push {
+
+// Per stream: the lag of the last step (0: no match), the last 32 query bits (the latest on top), and the words of k
+// and v that are being filled.
+struct alignas(16) Current {
+    uint32_t lag, q, k, v;
+};
+
+// The histories of all streams, stream by stream: words of q, then of k, then of v (whole words only).
+struct Histories {
+    Current* current;
+    uint32_t* words;
+    size_t wps;
+    __device__ const uint32_t* of(size_t stream, int which) const { return words + (stream * 3 + which) * wps; }
+};
+
+// 32 bits that end with bit p of a history whose word `last` is still in a register.
+__device__ __forceinline__ uint32_t window(const uint32_t* words, uint32_t last, uint32_t current, uint32_t p) {
+    const uint32_t w = p >> 5;
+    const uint32_t hi = w == last ? current : words[w], lo = w ? words[w - 1u] : 0u;
+    return __funnelshift_l(lo, hi, 31u - (p & 31u));
+}
+
+// The lag of step i for one stream, by the whole warp; wq: the query bits up to i, k_word: the keys before i.
+__device__ __forceinline__ uint32_t search(const uint32_t* q, const uint32_t* k, uint32_t i, uint32_t wq, uint32_t k_word) {
+    const uint32_t lane = threadIdx.x & 31u, last = i >> 5, q_word = wq >> (31u - (i & 31u));
+    uint32_t best = 0, before = 0;      // agreement << 26 | word of the position, the bit within the word is the lane
+    for (uint32_t w0 = 0; w0 <= last; w0 += 32u) {
+        const uint32_t mine = w0 + lane < last ? k[w0 + lane] : w0 + lane == last ? k_word : 0u;
+        const uint32_t n_words = min(32u, last + 1u - w0);
+        for (uint32_t j = 0; j < n_words; ++j) {
+            const uint32_t w = w0 + j, word = __shfl_sync(0xFFFFFFFFu, mine, (int)j);
+            uint32_t n = (uint32_t)__clz((int)(wq ^ __funnelshift_l(before, word, 31u - lane)));
+            if (w == 0u) n = min(n, lane + 1u);                  // a history has position + 1 steps
+            if (w == last && lane >= (i & 31u)) n = 0u;          // not a key yet
+            best = max(best, n ? n << 26 | w : 0u);
+            before = word;
+        }
+    }
+    const uint32_t most = __reduce_max_sync(0xFFFFFFFFu, best);
+    if (most >> 26 < 32u) {
+        if (most == 0u) return 0u;
+        const uint32_t at = 31u - (uint32_t)__clz((int)__ballot_sync(0xFFFFFFFFu, best == most));
+        return i - (32u * (most & 0x3FFFFFFu) + at);
+    }
+    // whole windows agree: count on from there
+    uint32_t longest = 0, position = 0;
+    for (uint32_t r = lane; r < i; r += 32u) {
+        if (window(k, last, k_word, r) != wq) continue;
+        uint32_t n = 32u;
+        while (n <= r) {
+            const uint32_t same = (uint32_t)__clz((int)(window(q, last, q_word, i - n) ^ window(k, last, k_word, r - n)));
+            n += same;
+            if (same < 32u) break;
+        }
+        n = min(n, r + 1u);
+        if (n >= longest) { longest = n; position = r; }
+    }
+    const uint32_t top = __reduce_max_sync(0xFFFFFFFFu, longest);
+    return i - __reduce_max_sync(0xFFFFFFFFu, longest == top ? position : 0u);
+}
+
+// The same for one stream per lane (open lanes only).  The position is found at once, so it has to fit 26 bits.
+__device__ __forceinline__ uint32_t search_alone(const uint32_t* q, const uint32_t* k, uint32_t i, uint32_t wq, uint32_t k_word) {
+    const uint32_t last = i >> 5, q_word = wq >> (31u - (i & 31u));
+    uint32_t best = 0, before = 0, next = last ? k[0] : k_word;
+    for (uint32_t w = 0; w <= last; ++w) {
+        const uint32_t word = next, n_bits = w == last ? i & 31u : 32u;
+        next = w + 1u < last ? k[w + 1u] : k_word;
+#pragma unroll 8
+        for (uint32_t b = 0; b < n_bits; ++b) {
+            uint32_t n = (uint32_t)__clz((int)(wq ^ __funnelshift_l(before, word, 31u - b)));
+            if (w == 0u) n = min(n, b + 1u);
+            best = max(best, (n << 26) + 32u * w + b);
+        }
+        before = word;
+    }
+    const uint32_t most = best >> 26;
+    if (most < 32u) return most ? i - (best & 0x3FFFFFFu) : 0u;
+    uint32_t longest = 0, position = 0;
+    for (uint32_t r = 31u; r < i; ++r) {
+        if (window(k, last, k_word, r) != wq) continue;
+        uint32_t n = 32u;
+        while (n <= r) {
+            const uint32_t same = (uint32_t)__clz((int)(window(q, last, q_word, i - n) ^ window(k, last, k_word, r - n)));
+            n += same;
+            if (same < 32u) break;
+        }
+        n = min(n, r + 1u);
+        if (n >= longest) { longest = n; position = r; }
+    }
+    return i - position;
+}
+
+// What step i of 32 streams (first + lane; a lane with live = false has none) can know before its bits: whether the lag of
+// the step before goes on if q is 1, and the v bit that it leads to (of the word being filled for lag 1: not known yet).
+struct Ahead {
+    Current c;
+    uint32_t key, value;
+};
+__device__ __forceinline__ Ahead begin(const Histories& H, size_t first, bool live, uint32_t i) {
+    Ahead a{{0u, 0u, 0u, 0u}, 0u, 0u};
+    const size_t s = first + (threadIdx.x & 31u);
+    if (!live || i == 0u) return a;
+    a.c = H.current[s];
+    if ((i & 31u) == 0u) a.c.k = a.c.v = 0u;
+    if (a.c.lag) {
+        const uint32_t p = i - a.c.lag, last = i >> 5;
+        a.key = ((p >> 5 == last ? a.c.k : H.of(s, 1)[p >> 5]) >> (p & 31u)) & 1u;
+        a.value = ((p + 1u) >> 5 == last ? a.c.v : H.of(s, 2)[(p + 1u) >> 5]) >> ((p + 1u) & 31u) & 1u;
+    }
+    return a;
+}
+
+// Step i of the same streams: returns idx of the lane's stream.
+__device__ __forceinline__ bool step(const Histories& H, size_t first, bool live, uint32_t i, Ahead a, uint32_t qb, uint32_t kb, uint32_t vb) {
+    const uint32_t lane = threadIdx.x & 31u, b = i & 31u, last = i >> 5;
+    const size_t s = first + lane;
+    Current c = a.c;
+    c.q = c.q >> 1 | qb << 31;
+    c.v |= vb << b;
+    const bool goes_on = c.lag && a.key == qb;
+    const bool known = !live || goes_on;
+    uint32_t open = __ballot_sync(0xFFFFFFFFu, !known);
+    // One after the other by the whole warp, or side by side with a lane each: by the instructions either takes.
+    if ((uint32_t)__popc(open) * (6u * last + 150u) > 6u * i + 100u && i < (1u << 26)) {
+        if (!known) c.lag = search_alone(H.of(s, 0), H.of(s, 1), i, c.q, c.k);
+        __syncwarp();
+        open = 0u;
+    }
+    while (open) {
+        const int l = __ffs((int)open) - 1;
+        open &= open - 1u;
+        const uint32_t lag = search(H.of(first + l, 0), H.of(first + l, 1), i, __shfl_sync(0xFFFFFFFFu, c.q, l),
+                                    __shfl_sync(0xFFFFFFFFu, c.k, l));
+        if ((int)lane == l) c.lag = lag;
+    }
+    bool bit = false;
+    if (live) {
+        if (goes_on && c.lag > 1u) {
+            bit = a.value != 0u;
+        } else if (c.lag) {
+            const uint32_t p = i - c.lag + 1u;
+            const uint32_t word = p >> 5 == last ? c.v : H.of(s, 2)[p >> 5];
+            bit = ((word >> (p & 31u)) & 1u) != 0u;
+        }
+        c.k |= kb << b;
+        H.current[s] = c;
+        if (b == 31u) {
+            uint32_t* words = H.words + s * 3 * H.wps + last;
+            words[0] = c.q;
+            words[H.wps] = c.k;
+            words[2 * H.wps] = c.v;
+        }
+    }
+    return bit;
+}
+
+}  // namespace push
+}  // namespace ullis

@@ -4,19 +4,14 @@
 // per-block forward_one src/model.rs:2243-2262, ROSA 1320-1352, CMix 1003-1016).
 //
 // A step is a handful of [batch, d_model] row operations, so it runs on the
-// CUDA-core kernels in the reference's summation order: the logits of step t
+// CUDA cores in the reference's summation order: the logits of step t
 // are bit-identical to row t of the one-shot forward in EXACT mode, which is
-// what the reference's own test asserts (src/model.rs:4991-5004).  The automata
-// follow the reference's eager schedule (push stamps the whole suffix-link chain
-// of the new state), because the O(T log T) form needs the whole sequence in
-// advance; the chain is kept as an array and stamped by a warp, 32 states per
-// round, instead of one dependent load per state.  A stream whose key bits have
-// all been equal so far is answered in closed form and its automaton written
-// only when that ends.
-//
-// Nothing in a step depends on the host except the tokens, so after the first
-// use the ~150 small launches of a step are replayed as one CUDA graph (two
+// what the reference's own test asserts (src/model.rs:4991-5004).  The whole
+// step is one cooperative kernel (generate_step.cuh) where the shape allows;
+// otherwise its ~90 small launches are replayed as one CUDA graph (two
 // graphs: before and after the first token, which has no time-shift history).
+// A stream's automaton is not kept: a push is answered from the bit histories
+// (gen_push.cuh).
 #include "generate.hpp"
 
 #include <cuda_fp16.h>
@@ -27,8 +22,8 @@
 #include <string>
 #include <vector>
 
+#include "generate_step.cuh"
 #include "kernels.hpp"
-#include "sam_core.cuh"
 
 namespace ullis {
 namespace {
@@ -36,19 +31,6 @@ namespace {
 inline unsigned blocks_for(size_t n, unsigned per) { return (unsigned)((n + per - 1) / per); }
 
 __device__ __forceinline__ float h2f(uint16_t b) { return __half2float(__ushort_as_half(b)); }
-
-// empty automaton per stream (src/rosa.rs:66-74)
-template <typename Ix>
-__global__ void gen_init_kernel(uint8_t* __restrict__ blocks, size_t stride, sam::WalkerState* __restrict__ ws,
-                                size_t streams, uint32_t T) {
-    const size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= streams) return;
-    // no pushes yet; the automaton is written lazily (sam::gen_push), not even the root is needed
-    sam::WalkerState st;
-    st.u = 1; st.g = 0; st.w = 0; st.gmax = 0; st.gfail = 0; st.h = 0; st.steps = 0; st.pad = 0;
-    ws[s] = st;
-    (void)blocks; (void)stride; (void)T;
-}
 
 // time_shift_one + mixes (src/model.rs:214-228, 1331-1340, 1008-1012): xx = prev - x, or -x before the
 // first token; out_m = x + xx*mix_m, unfused; then x becomes the layer's new time-shift history
@@ -136,41 +118,45 @@ gen_ln_shift_mix_kernel(const float* __restrict__ x, const uint16_t* __restrict_
     }
 }
 
-// one RosaSam::push per (sequence, channel) of one layer and y = (2*idx - 1)*e (src/model.rs:1344-1351).
-// One warp per stream: lane 0 runs the query and the extend, all lanes the stamping of the suffix-link chain
-// (sam::gen_push), which is what a late position costs.
-template <typename Ix>
+// one RosaSam::push per (sequence, channel) of one layer and y = (2*idx - 1)*e (src/model.rs:1344-1351); `per_warp`
+// streams per warp
 __global__ void __launch_bounds__(128)
-gen_push_kernel(uint8_t* __restrict__ blocks, size_t stride, sam::WalkerState* __restrict__ ws,
-                uint32_t* __restrict__ vhist, size_t wps, const float* __restrict__ q, const float* __restrict__ k,
-                const float* __restrict__ v, const uint16_t* __restrict__ e, float* __restrict__ y, size_t streams,
-                size_t C, uint32_t T, uint32_t* __restrict__ status) {
-    const size_t s = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t lane = threadIdx.x & 31u;
-    if (s >= streams) return;   // the whole warp
-    sam::GenLayout<Ix> L(T);
-    uint8_t* blk = blocks + s * stride;
-    sam::WalkerState st = ws[s];
-    const uint32_t i = st.steps;
-    if (i >= T) {  // the host checks the context length first; never write past the state block
-        if (lane == 0 && atomicCAS(status, ULLIS_DEV_OK, ULLIS_DEV_SAM_CAPACITY) == ULLIS_DEV_OK) status[1] = (uint32_t)s;
-        return;
-    }
+gen_push_kernel(push::Histories H, size_t first, const uint32_t* __restrict__ time, uint32_t per_warp, const float* __restrict__ q,
+                const float* __restrict__ k, const float* __restrict__ v, const uint16_t* __restrict__ e, float* __restrict__ y,
+                size_t streams, size_t C) {
+    const size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, s = warp * per_warp + (threadIdx.x & 31u);
+    const bool live = (threadIdx.x & 31u) < per_warp && s < streams;
     // src/rosa.rs:372-374: bit = activation > 0
-    const uint32_t qb = q[s] > 0.0f, kb = k[s] > 0.0f, vb = v[s] > 0.0f;
-    uint32_t* vh = vhist + s * wps;
-    if (lane == 0) {   // only lane 0 reads the v history
-        const uint32_t word = (i & 31u) ? vh[i >> 5] : 0u;   // a new word starts empty
-        vh[i >> 5] = word | (vb << (i & 31u));
-    }
-    // constant key so far: O(1); otherwise RosaSam::push with the chain stamped by the warp
-    const uint32_t idx = sam::gen_push<Ix>(reinterpret_cast<sam::Node<Ix>*>(blk + L.nodes), reinterpret_cast<Ix*>(blk + L.last),
-                                           reinterpret_cast<Ix*>(blk + L.path), vh, &st, qb, kb);
-    if (lane == 0) {
-        ws[s] = st;
+    const size_t f = first + warp * per_warp;
+    const uint32_t i = *time;
+    const bool idx = push::step(H, f, live, i, push::begin(H, f, live, i), live && q[s] > 0.0f, live && k[s] > 0.0f, live && v[s] > 0.0f);
+    if (live) {
         const float ev = h2f(e[s % C]);
         y[s] = idx ? ev : -ev;
     }
+}
+
+// `steps` pushes of every stream, bits as bytes [steps, streams]
+__global__ void __launch_bounds__(128)
+push_steps_kernel(push::Histories H, size_t time, size_t steps, uint32_t per_warp, const uint8_t* __restrict__ q,
+                  const uint8_t* __restrict__ k, const uint8_t* __restrict__ v, uint8_t* __restrict__ idx, size_t streams) {
+    const size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, s = warp * per_warp + (threadIdx.x & 31u);
+    const bool live = (threadIdx.x & 31u) < per_warp && s < streams;
+    for (size_t t = 0; t < steps; ++t) {
+        const size_t at = t * streams + s;
+        const size_t f = warp * per_warp;
+        const uint32_t i = (uint32_t)(time + t);
+        const bool bit = push::step(H, f, live, i, push::begin(H, f, live, i), live && q[at], live && k[at], live && v[at]);
+        if (live) idx[at] = bit;
+        __syncwarp();   // a lane's words are read by the whole warp in the next step
+    }
+}
+
+// Streams per warp: a warp takes its streams' searches one after the other, so no more than keep the device busy.
+uint32_t streams_per_warp(const ullis_cuda_runtime* rt, size_t streams) {
+    uint32_t n = 1;
+    while (n < 32u && streams > (size_t)n * (size_t)rt->sm_count * 32u) n *= 2;
+    return n;
 }
 
 }  // namespace
@@ -180,29 +166,88 @@ using namespace ullis;
 
 ullis_cuda_generate_state::ullis_cuda_generate_state(ullis_cuda_model* m, size_t batch_) : model(m), batch(batch_) {
     if (batch == 0) fail(ULLIS_CUDA_ERR_SHAPE, "generate needs at least one sequence");
-    const uint32_t T = (uint32_t)m->context_len;
-    narrow = sam::node_capacity(T) <= 0xFFFFu;
-    stride = narrow ? sam::GenLayout<uint16_t>(T).total : sam::GenLayout<uint32_t>(T).total;
     wps = (m->context_len + 31) / 32;
     const size_t per_layer = batch * m->d;
     if (per_layer / m->d != batch || m->layers > SIZE_MAX / per_layer) fail(ULLIS_CUDA_ERR_SHAPE, "generate state shape overflow");
     streams = m->layers * per_layer;
-    if (streams > SIZE_MAX / stride) fail(ULLIS_CUDA_ERR_SHAPE, "generate state shape overflow");
-    m->rt->bind();
-    k::rowvec_prepare(m->rt);   // before any step is recorded into a graph
-    blocks.ensure(streams * stride);
-    walkers.ensure(streams * sizeof(sam::WalkerState));
-    vhist.ensure(streams * wps * 4);
-    prev.ensure(m->layers * 2 * per_layer * 4);
-    ids.ensure(batch * 4);
+    if (streams > SIZE_MAX / (wps * 12 + sizeof(push::Current))) fail(ULLIS_CUDA_ERR_SHAPE, "generate state shape overflow");
+    ullis_cuda_runtime* rt = m->rt;
+    rt->bind();
+    k::rowvec_prepare(rt);   // before any step is recorded into a graph
+    words.ensure(streams * wps * 12);
+    current.ensure(streams * sizeof(push::Current));
+    prev.ensure(2 * m->layers * 2 * per_layer * 4);   // read one half, write the other (generate_step.cuh)
+    ids.ensure((batch + 1) * 4);
     for (ullis::DeviceBuffer* buf : {&x, &a, &bq, &bk, &bv}) buf->ensure(per_layer * 4);
     wide.ensure(batch * std::max(m->ffn, 3 * m->d) * 4);
     logits.ensure(batch * m->vocab * 4);
-    ULLIS_CUDA_CHECK(cudaMallocHost(&h_tokens, batch * 4));
+    ULLIS_CUDA_CHECK(cudaMallocHost(&h_tokens, (batch + 1) * 4));
     ULLIS_CUDA_CHECK(cudaMallocHost(&h_logits, batch * m->vocab * 4));
     use_graph = !getenv("ULLIS_CUDA_NO_GRAPH");
     if (const char* env = getenv("ULLIS_CUDA_INJECT_GENERATE_FAILURE")) inject_failure_at = (size_t)std::max(0, atoi(env));
+    prepare_one_kernel();
     reset();
+}
+
+// Whether a step of this shape runs as one kernel, and how it is split over clusters.
+void ullis_cuda_generate_state::prepare_one_kernel() {
+    ullis_cuda_model* m = model;
+    ullis_cuda_runtime* rt = m->rt;
+    if (getenv("ULLIS_CUDA_GEN_UNFUSED") || getenv("ULLIS_CUDA_NO_GRAPH") || m->d % 32 || m->ffn % gen::PIECE || rt->cc_major < 9) return;
+    auto kernel_for = [](uint32_t g) {
+        return g == 1 ? reinterpret_cast<const void*>(gen::gen_step_kernel<1>)
+               : g == 2 ? reinterpret_cast<const void*>(gen::gen_step_kernel<2>) : reinterpret_cast<const void*>(gen::gen_step_kernel<4>);
+    };
+    // One round of clusters if there is a way, with as many CTAs per cluster as have 32 channels each (a CTA's share of the
+    // sums is shortest then) and as few sequences per cluster as the clusters that the device holds at once allow.
+    constexpr size_t MOST_SMEM = 224 * 1024;
+    size_t best_rounds = SIZE_MAX;
+    for (uint32_t c = gen::MAX_CLUSTER; c >= 1 && best_rounds > 1; c /= 2) {
+        if (m->d % (c * 32) || m->ffn % (c * 4)) continue;
+        for (uint32_t g = 1; g <= gen::MAX_GROUP && best_rounds > 1; g *= 2) {
+            const size_t smem = gen::step_smem_bytes(g, m->d, m->ffn, m->d / c), want = (batch + g - 1) / g;
+            if (smem > MOST_SMEM) break;
+            const void* kernel = kernel_for(g);
+            ULLIS_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MOST_SMEM));
+            ULLIS_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            cudaLaunchAttribute attr;
+            const cudaLaunchConfig_t cfg = step_config(&attr, c, c, smem);
+            int clusters = 0;
+            ULLIS_CUDA_CHECK(cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg));
+            if (clusters < 1) break;
+            const size_t rounds = (want + clusters - 1) / clusters;
+            if (rounds >= best_rounds) continue;
+            best_rounds = rounds;
+            cluster = c; group = g; step_kernel = kernel; step_smem = smem;
+            step_grid = (unsigned)(std::min<size_t>(want, (size_t)clusters) * c);
+        }
+    }
+    if (!step_grid) return;
+    std::vector<gen::Layer> layers(m->layers);
+    for (size_t l = 0; l < m->layers; ++l) {
+        const LayerWeights& L = m->blocks[l];
+        auto packed = [](const PackedWeights& w) { return gen::Packed{w.bits, w.scale, w.bias}; };
+        layers[l] = gen::Layer{L.ln3.weight, L.ln3.bias, {L.x_q, L.x_k, L.x_v}, L.e, L.ln2.weight, L.ln2.bias, L.ffn_x_k, L.value,
+                               {packed(L.q), packed(L.k), packed(L.v)}, packed(L.o), gen::Packed{L.key.bits, L.key.scale, nullptr}};
+    }
+    step_layers.ensure(layers.size() * sizeof(gen::Layer) + 16);
+    rt->h2d(step_layers.get(), layers.data(), layers.size() * sizeof(gen::Layer));
+    rt->sync();
+}
+
+cudaLaunchConfig_t ullis_cuda_generate_state::step_config(cudaLaunchAttribute* attr, unsigned grid, unsigned per_cluster, size_t smem) const {
+    cudaLaunchConfig_t cfg;
+    std::memset(&cfg, 0, sizeof(cfg));
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = per_cluster;
+    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(gen::THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = model->rt->stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
 }
 
 ullis_cuda_generate_state::~ullis_cuda_generate_state() {
@@ -212,18 +257,45 @@ ullis_cuda_generate_state::~ullis_cuda_generate_state() {
     if (h_logits) cudaFreeHost(h_logits);
 }
 
+// Empty histories (src/rosa.rs:66-74): a push at position 0 looks at nothing that was there before.
 void ullis_cuda_generate_state::reset() {
     ullis_cuda_runtime* rt = model->rt;
     rt->bind();
-    const uint32_t T = (uint32_t)model->context_len;
-    auto* ws = static_cast<sam::WalkerState*>(walkers.get());
-    auto* blk = static_cast<uint8_t*>(blocks.get());
-    if (narrow) gen_init_kernel<uint16_t><<<blocks_for(streams, 256), 256, 0, rt->stream>>>(blk, stride, ws, streams, T);
-    else gen_init_kernel<uint32_t><<<blocks_for(streams, 256), 256, 0, rt->stream>>>(blk, stride, ws, streams, T);
-    rt->launched("gen_init");
-    rt->sync();
+    if (poisoned) rt->sync();   // whatever failed has left the device before the next step starts
     time = 0;
     poisoned = false;
+}
+
+ullis::push::Histories ullis_cuda_generate_state::histories() {
+    return {static_cast<push::Current*>(current.get()), static_cast<uint32_t*>(words.get()), wps};
+}
+
+// Enqueues a step as one kernel; logits_to: device memory or page-locked host memory.
+void ullis_cuda_generate_state::launch_one_kernel(float* logits_to) {
+    ullis_cuda_model* m = model;
+    ullis_cuda_runtime* rt = m->rt;
+    const size_t half = m->layers * 2 * batch * m->d;
+    float* history = static_cast<float*>(prev.get());
+    gen::Step p{};
+    p.layers = static_cast<const gen::Layer*>(step_layers.get());
+    p.n_layers = (uint32_t)m->layers; p.rows = (uint32_t)batch; p.d = (uint32_t)m->d; p.ffn = (uint32_t)m->ffn;
+    p.vocab = (uint32_t)m->vocab; p.time = (uint32_t)time;
+    p.group = group;
+    p.tokens = h_tokens;
+    p.embedding = m->embedding;
+    p.ln0_w = m->blocks[0].ln0.weight; p.ln0_b = m->blocks[0].ln0.bias;
+    p.ln_out_w = m->ln_out.weight; p.ln_out_b = m->ln_out.bias;
+    p.head = gen::Packed{m->head.bits, m->head.scale, m->head.bias};
+    p.prev_in = history + (time & 1) * half;
+    p.prev_out = history + (~time & 1) * half;
+    p.push = histories();
+    p.logits = logits_to;
+    rt->host_status[0] = ULLIS_DEV_OK;   // this kernel reports nothing
+    void* args[] = {&p};
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = step_config(&attr, step_grid, cluster, step_smem);
+    ULLIS_CUDA_CHECK(cudaLaunchKernelExC(&cfg, step_kernel, args));
+    rt->launched("gen_step");
 }
 
 void ullis_cuda_generate_state::step(const uint32_t* tokens, float* logits_out) {
@@ -239,6 +311,7 @@ void ullis_cuda_generate_state::step(const uint32_t* tokens, float* logits_out) 
     rt->bind();
     if (rt->kernel_timing) rt->mark("(between steps)");
     std::memcpy(h_tokens, tokens, batch * 4);
+    h_tokens[batch] = (uint32_t)time;
     const int has_prev = time != 0;
     // From here on the device-side automata, v history and time-shift inputs may have moved on by one position
     // while `time` has not: a failure below leaves the state out of step with itself, and a retry would push the
@@ -249,7 +322,21 @@ void ullis_cuda_generate_state::step(const uint32_t* tokens, float* logits_out) 
         ~Poison() { if (armed) *flag = true; }
     } poison{&poisoned};
 
-    if (use_graph && !rt->kernel_timing) {
+    // The logits go straight into page-locked memory (what the Python layer passes), else through h_logits.
+    float* to = logits_out;
+    cudaPointerAttributes attr;
+    if (cudaPointerGetAttributes(&attr, logits_out) != cudaSuccess || attr.type != cudaMemoryTypeHost) {
+        cudaGetLastError();
+        to = h_logits;
+    }
+    if (step_grid) {
+        if (batch <= DIRECT_LOGITS) {
+            launch_one_kernel(to);
+        } else {
+            launch_one_kernel(static_cast<float*>(logits.get()));
+            rt->d2h(to, logits.get(), batch * m->vocab * 4);
+        }
+    } else if (use_graph && !rt->kernel_timing) {
         // Replay the step as one graph launch; per-kernel timing needs the plain launches.
         if (!graph[has_prev]) {
             cudaGraph_t captured = nullptr;
@@ -272,8 +359,10 @@ void ullis_cuda_generate_state::step(const uint32_t* tokens, float* logits_out) 
         }
         ULLIS_CUDA_CHECK(cudaGraphLaunch(graph[has_prev], rt->stream));
         rt->launches += graph_launches;
+        to = h_logits;
     } else {
         enqueue(has_prev);
+        to = h_logits;
     }
     rt->sync();
     rt->throw_on_status();
@@ -281,7 +370,7 @@ void ullis_cuda_generate_state::step(const uint32_t* tokens, float* logits_out) 
         inject_failure_at = 0;
         fail(ULLIS_CUDA_ERR_CUDA, "injected failure after the step's kernels ran");
     }
-    std::memcpy(logits_out, h_logits, batch * m->vocab * 4);
+    if (to != logits_out) std::memcpy(logits_out, to, batch * m->vocab * 4);
     time += 1;
     poison.armed = false;
 }
@@ -290,7 +379,6 @@ void ullis_cuda_generate_state::enqueue(int has_prev) {
     ullis_cuda_model* m = model;
     ullis_cuda_runtime* rt = m->rt;
     const size_t d = m->d, ffn = m->ffn, rows = batch, n = rows * d;
-    const uint32_t T = (uint32_t)m->context_len;
     uint32_t* IDS = static_cast<uint32_t*>(ids.get());
     float* X = static_cast<float*>(x.get());
     float* A = static_cast<float*>(a.get());
@@ -300,7 +388,7 @@ void ullis_cuda_generate_state::enqueue(int has_prev) {
     float* W = static_cast<float*>(wide.get());
     float* LG = static_cast<float*>(logits.get());
     rt->clear_status();
-    rt->h2d(IDS, h_tokens, rows * 4);
+    rt->h2d(IDS, h_tokens, (rows + 1) * 4);   // the ids and the position: a recorded graph takes both from here
     k::embed(rt, IDS, m->embedding, X, rows, d, m->vocab);
     const bool fused_ln = d * 4 <= 48 * 1024 && !getenv("ULLIS_CUDA_GEN_UNFUSED");   // a row in shared memory
     for (size_t l = 0; l < m->layers; ++l) {
@@ -336,15 +424,9 @@ void ullis_cuda_generate_state::enqueue(int has_prev) {
             }
         }
         {
-            auto* ws = static_cast<sam::WalkerState*>(walkers.get()) + s0;
-            uint8_t* blk = static_cast<uint8_t*>(blocks.get()) + s0 * stride;
-            uint32_t* vh = static_cast<uint32_t*>(vhist.get()) + s0 * wps;
-            if (narrow)
-                gen_push_kernel<uint16_t><<<blocks_for(n * 32, 128), 128, 0, rt->stream>>>(blk, stride, ws, vh, wps, W, W + n, W + 2 * n,
-                                                                                     L.e, A, n, d, T, rt->dev_status);
-            else
-                gen_push_kernel<uint32_t><<<blocks_for(n * 32, 128), 128, 0, rt->stream>>>(blk, stride, ws, vh, wps, W, W + n, W + 2 * n,
-                                                                                     L.e, A, n, d, T, rt->dev_status);
+            const uint32_t per = streams_per_warp(rt, n);
+            gen_push_kernel<<<blocks_for((n + per - 1) / per * 32, 128), 128, 0, rt->stream>>>(
+                histories(), s0, IDS + batch, per, W, W + n, W + 2 * n, L.e, A, n, d);
             rt->launched("gen_push");
         }
         k::binary_linear_exact(rt, A, L.o.bits, L.o.scale, L.o.bias, X, rows, d, d, true);  // h += rosa out
@@ -386,27 +468,14 @@ ullis_cuda_rosa_pushers::ullis_cuda_rosa_pushers(ullis_cuda_runtime* rt_, size_t
     : rt(rt_), streams(streams_), capacity(capacity_) {
     if (streams == 0 || capacity == 0) fail(ULLIS_CUDA_ERR_SHAPE, "ROSA pushers need at least one stream and one position");
     if (capacity > 0x7FFFFFF0u) fail(ULLIS_CUDA_ERR_SHAPE, "ROSA pushers: capacity too large");
-    const uint32_t T = (uint32_t)capacity;
-    narrow = sam::node_capacity(T) <= 0xFFFFu;
-    stride = narrow ? sam::GenLayout<uint16_t>(T).total : sam::GenLayout<uint32_t>(T).total;
     wps = (capacity + 31) / 32;
-    if (streams > SIZE_MAX / stride) fail(ULLIS_CUDA_ERR_SHAPE, "ROSA pushers: shape overflow");
+    if (streams > SIZE_MAX / (wps * 12 + sizeof(push::Current))) fail(ULLIS_CUDA_ERR_SHAPE, "ROSA pushers: shape overflow");
     rt->bind();
-    blocks.ensure(streams * stride);
-    walkers.ensure(streams * sizeof(sam::WalkerState));
-    vhist.ensure(streams * wps * 4);
-    reset();
+    words.ensure(streams * wps * 12);
+    current.ensure(streams * sizeof(push::Current));
 }
 
-void ullis_cuda_rosa_pushers::reset() {
-    rt->bind();
-    auto* ws = static_cast<sam::WalkerState*>(walkers.get());
-    auto* blk = static_cast<uint8_t*>(blocks.get());
-    gen_init_kernel<uint16_t><<<blocks_for(streams, 256), 256, 0, rt->stream>>>(blk, stride, ws, streams, (uint32_t)capacity);
-    rt->launched("gen_init");
-    rt->sync();
-    time = 0;
-}
+void ullis_cuda_rosa_pushers::reset() { time = 0; }   // a push at position 0 looks at nothing that was there before
 
 void ullis_cuda_rosa_pushers::push(const uint8_t* q, const uint8_t* k, const uint8_t* v, size_t steps, uint8_t* idx) {
     // RosaSam has no capacity (src/rosa.rs:55-64 grows its vectors); here it is fixed when the state is made
@@ -415,40 +484,16 @@ void ullis_cuda_rosa_pushers::push(const uint8_t* q, const uint8_t* k, const uin
     if (steps > SIZE_MAX / streams / 20) fail(ULLIS_CUDA_ERR_SHAPE, "ROSA pushers: shape overflow");
     rt->bind();
     const size_t n = steps * streams;
-    // the generation kernel takes activations (bit = x > 0) and writes (2*idx - 1)*e: feed it +-1 and e = 1
-    std::vector<float> h(3 * n);
-    for (size_t i = 0; i < n; ++i) {
-        h[i] = q[i] ? 1.0f : -1.0f;
-        h[n + i] = k[i] ? 1.0f : -1.0f;
-        h[2 * n + i] = v[i] ? 1.0f : -1.0f;
-    }
-    io.ensure(4 * n * 4 + 16);
-    float* d = static_cast<float*>(io.get());
-    uint16_t* one = reinterpret_cast<uint16_t*>(d + 4 * n);
-    const uint16_t h_one = 0x3C00u;   // FP16 1.0
-    rt->clear_status();
-    rt->h2d(d, h.data(), 3 * n * 4);
-    rt->h2d(one, &h_one, 2);
-    auto* ws = static_cast<sam::WalkerState*>(walkers.get());
-    auto* blk = static_cast<uint8_t*>(blocks.get());
-    uint32_t* vh = static_cast<uint32_t*>(vhist.get());
-    for (size_t t = 0; t < steps; ++t) {
-        const float* row = d + t * streams;
-        if (narrow)
-            gen_push_kernel<uint16_t><<<blocks_for(streams * 32, 128), 128, 0, rt->stream>>>(
-                blk, stride, ws, vh, wps, row, row + n, row + 2 * n, one, d + 3 * n + t * streams, streams, 1, (uint32_t)capacity,
-                rt->dev_status);
-        else
-            gen_push_kernel<uint32_t><<<blocks_for(streams * 32, 128), 128, 0, rt->stream>>>(
-                blk, stride, ws, vh, wps, row, row + n, row + 2 * n, one, d + 3 * n + t * streams, streams, 1, (uint32_t)capacity,
-                rt->dev_status);
-        rt->launched("gen_push");
-    }
-    std::vector<float> y(n);
-    rt->d2h(y.data(), d + 3 * n, n * 4);
-    rt->d2h(rt->host_status, rt->dev_status, 16);
+    uint8_t* d = io.as<uint8_t>(4 * n);
+    rt->h2d(d, q, n);
+    rt->h2d(d + n, k, n);
+    rt->h2d(d + 2 * n, v, n);
+    const push::Histories H{static_cast<push::Current*>(current.get()), static_cast<uint32_t*>(words.get()), wps};
+    const uint32_t per = streams_per_warp(rt, streams);
+    push_steps_kernel<<<blocks_for((streams + per - 1) / per * 32, 128), 128, 0, rt->stream>>>(H, time, steps, per, d, d + n, d + 2 * n,
+                                                                                              d + 3 * n, streams);
+    rt->launched("gen_push");
+    rt->d2h(idx, d + 3 * n, n);
     rt->sync();
-    time += steps;   // the automata have moved on whatever the status says
-    rt->throw_on_status();
-    for (size_t i = 0; i < n; ++i) idx[i] = y[i] > 0.0f;
+    time += steps;
 }

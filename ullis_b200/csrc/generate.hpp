@@ -1,17 +1,24 @@
 // Device-resident state of incremental generation (reference HeronGenerateState,
-// src/model.rs:2433-2454): per layer one suffix automaton per (sequence,
-// channel) and the two time-shift inputs; `batch` independent sequences advance
-// in lock step.
+// src/model.rs:2433-2454): per layer the bit histories of one ROSA stream per
+// (sequence, channel) and the two time-shift inputs; `batch` independent
+// sequences advance in lock step.
 #pragma once
+#include "gen_push.cuh"
 #include "model.hpp"
 
 struct ullis_cuda_generate_state {
     ullis_cuda_model* model = nullptr;
     size_t batch = 0, time = 0;
-    bool narrow = true;          // 16-bit state ids (context_len <= 32766)
-    size_t stride = 0, wps = 0;  // bytes of one automaton block, v-history words per stream
+    size_t wps = 0;              // history words per stream and bit
     size_t streams = 0;          // layers * batch * d_model
-    ullis::DeviceBuffer blocks, walkers, vhist, prev;
+    ullis::DeviceBuffer words, current, prev;
+    // The step as one kernel (generate_step.cuh); step_grid = 0: a shape it does not take.
+    static constexpr size_t DIRECT_LOGITS = 8;   // sequences up to which the kernel stores the logits over the link itself
+    unsigned step_grid = 0;
+    size_t step_smem = 0;
+    const void* step_kernel = nullptr;
+    uint32_t group = 1, cluster = 1;             // sequences of a cluster, CTAs of a cluster
+    ullis::DeviceBuffer step_layers;
     // activations of one step (owned here, so that a captured graph's pointers stay valid)
     ullis::DeviceBuffer ids, x, a, bq, bk, bv, wide, logits;
     uint32_t* h_tokens = nullptr;   // pinned staging of the step's inputs / outputs
@@ -32,19 +39,22 @@ struct ullis_cuda_generate_state {
     ullis_cuda_generate_state(const ullis_cuda_generate_state&) = delete;
     ullis_cuda_generate_state& operator=(const ullis_cuda_generate_state&) = delete;
     void reset();
+    void prepare_one_kernel();
+    cudaLaunchConfig_t step_config(cudaLaunchAttribute* attr, unsigned grid, unsigned per_cluster, size_t smem) const;
+    void launch_one_kernel(float* logits_to);
+    ullis::push::Histories histories();
     void enqueue(int has_prev);   // copies in, every kernel of one step, copies out; no synchronisation
     // tokens [batch] (host) -> logits [batch, vocab] (host); advances time by one
     void step(const uint32_t* tokens, float* logits);
 };
 
-// `streams` independent RosaSam automata (src/rosa.rs:55-176) kept on the device between calls: the op-level form
+// `streams` independent RosaSam states (src/rosa.rs:55-176) kept on the device between calls: the op-level form
 // of what a generate state holds per layer.  push() advances every stream by `steps` positions.
 struct ullis_cuda_rosa_pushers {
     ullis_cuda_runtime* rt = nullptr;
     size_t streams = 0, capacity = 0, time = 0;
-    bool narrow = true;
-    size_t stride = 0, wps = 0;
-    ullis::DeviceBuffer blocks, walkers, vhist, io;
+    size_t wps = 0;
+    ullis::DeviceBuffer words, current, io;
 
     ullis_cuda_rosa_pushers(ullis_cuda_runtime* rt, size_t streams, size_t capacity);
     void reset();

@@ -147,15 +147,14 @@ def _z(n):
 class _ResultBlock:
     """One page-locked block lent to a numpy array; it goes back to the pool with the last array that looks at it."""
 
-    __slots__ = ("addr", "size", "__array_interface__")
+    __slots__ = ("pool", "addr", "size", "__array_interface__")
 
-    def __init__(self, addr: int, size: int, nbytes: int):
-        self.addr, self.size = addr, size
+    def __init__(self, pool: "_ResultPool", addr: int, size: int, nbytes: int):
+        self.pool, self.addr, self.size = pool, addr, size
         self.__array_interface__ = {"data": (addr, False), "shape": (nbytes,), "typestr": "|u1", "version": 3}
 
     def __del__(self):
-        if _RESULTS is not None:             # not while the interpreter shuts down
-            _RESULTS.give_back(self.addr, self.size)
+        self.pool.give_back(self.addr, self.size)
 
 
 class _ResultPool:
@@ -186,7 +185,7 @@ class _ResultPool:
             addr = idle.pop() if idle else self._lock_memory(rt, size)
         if addr is None:
             return np.empty(shape, dtype)
-        return np.asarray(_ResultBlock(addr, size, nbytes)).view(dtype).reshape(shape)
+        return np.asarray(_ResultBlock(self, addr, size, nbytes)).view(dtype).reshape(shape)
 
     def _lock_memory(self, rt, size):
         if self._held + size > self.limit:
