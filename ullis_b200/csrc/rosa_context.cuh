@@ -115,25 +115,26 @@ RC_HD uint32_t longest_in_word(const uint32_t* W, const uint16_t* ends, uint32_t
     return best;
 }
 
-// find() below on buckets by run_key.
-RC_HD uint32_t find_by_runs(const Entry* entries, const uint16_t* start, const uint32_t* Q, const uint32_t* K,
-                            const uint16_t* q_ends, const Runs& R, uint32_t words, uint32_t c, uint32_t t, uint32_t& deep) {
-    const uint32_t half = 1u << (c - 1u), run = run_at(Q, q_ends, t), bit = bit_at(Q, t);
-    const uint32_t key = bit * half + (run & (half - 1u));
-    uint32_t best = 0, at = 0;
-    if (run <= t) {                                            // beyond the run there is more of the query history
-        const uint32_t wq = window(Q, t - run);
-        for (uint32_t b = start[key], e = start[key + 1u]; b < e; ++b) {
-            const uint32_t r = entries[b].r;
-            if (r >= t) break;
-            if (r < run || run_at(K, R.ends, r) != run) continue;
-            const uint32_t n = agreement(Q, K, t - run, r - run, wq ^ window(K, r - run), deep);   // at least 1
-            if (n >= best) { best = n; at = r + 1u; }
-        }
-        if (best) return at;
+// Of the positions among entries [b, e), every step-th, that lie before t and have the query's run length: the longest
+// agreement beyond the run, packed as agreement << 16 | position + 1 with the latest of equals (0: none).
+RC_HD uint32_t scan_runs(const Entry* entries, uint32_t b, uint32_t e, uint32_t step, const uint32_t* Q, const uint32_t* K, const Runs& R, uint32_t run,
+                         uint32_t t, uint32_t& deep) {
+    uint32_t best = 0;
+    if (run > t) return 0u;                                    // beyond the run there is no more of the query history
+    const uint32_t wq = window(Q, t - run);
+    for (; b < e; b += step) {
+        const uint32_t r = entries[b].r;
+        if (r >= t) break;
+        if (r < run || run_at(K, R.ends, r) != run) continue;
+        const uint32_t v = agreement(Q, K, t - run, r - run, wq ^ window(K, r - run), deep) << 16 | (r + 1u);   // at least 1
+        best = v > best ? v : best;
     }
-    // The latest position before t whose run of this bit reaches `run`, else the latest of the longest runs.
-    uint32_t w = t >> 5;
+    return best;
+}
+// Without such a position: the latest one before t whose run of this bit reaches `run`, else the latest of the longest
+// runs, as r + 1.
+RC_HD uint32_t find_inside_run(const uint32_t* K, const Runs& R, uint32_t words, uint32_t bit, uint32_t run, uint32_t t, uint32_t& deep) {
+    uint32_t best = 0, at = 0, w = t >> 5;
     for (uint32_t i = t; i > 32u * w;) {                       // the positions in the word of t
         const uint32_t n = run_at(K, R.ends, i - 1u);
         if (bit_at(K, i - 1u) == bit) {
@@ -177,6 +178,13 @@ RC_HD int32_t scan(const Entry* entries, const uint16_t* start, uint32_t first, 
     }
     return best;
 }
+// One position of them.
+RC_HD int32_t scan_one(Entry a, uint32_t t, uint32_t wq, int32_t best) {
+    if (a.r >= t) return best;
+    const int32_t top = 31 - (int32_t)leading(wq ^ a.key), least = 30 - (int32_t)a.r;
+    const int32_t v = (top > least ? top : least) * 65536 - (int32_t)a.r;
+    return v < best ? v : best;
+}
 // The same where the positions of a bucket are known to agree in equally many bits: the latest one of each counts, found
 // by bisection (a bucket beside the query's own can be as large as the stream).
 RC_HD int32_t scan_latest(const Entry* entries, const uint16_t* start, uint32_t first, uint32_t n, uint32_t t, uint32_t wq,
@@ -202,39 +210,59 @@ RC_HD int32_t scan_latest(const Entry* entries, const uint16_t* start, uint32_t 
 RC_HD uint32_t scan_position(int32_t best) { return (uint32_t)-best & 0xFFFFu; }
 RC_HD int32_t scan_agreement(int32_t best) { return 31 - ((best + (int32_t)scan_position(best)) >> 16); }   // -1: no position
 
-// r + 1 for step t, 0 without a match.  entries / start: the positions sorted by context, first entry of each of the
-// 2^c + 1 buckets.  The search begins with `wide` sets of as many context bits as leave 4 to 8 positions before t on
-// evenly spread keys, otherwise with all c bits; whatever has not been looked at when it ends agrees in fewer bits than
-// the best.  (A position with a history shorter than a context lies in the bucket of that history filled up with zeros,
-// which agrees with the query in no fewer bits than the history itself.)
-RC_HD uint32_t find(const Entry* entries, const uint16_t* start, const uint32_t* Q, const uint32_t* K, uint32_t c, bool wide,
-                    uint32_t t, uint32_t& deep) {
-    const uint32_t wq = window(Q, t), ctx = wq >> (32u - c);
-    if (t < BRUTE) {
-        uint32_t best = 0, at = 0;
-        for (uint32_t r = 0; r < t; ++r) {
-            const uint32_t n = agreement(Q, K, t, r, wq ^ window(K, r), deep);
-            if (n && n >= best) { best = n; at = r + 1u; }
-        }
-        return at;
+constexpr int32_t SCAN_NOTHING = 32 * 65536;
+RC_HD bool scan_full(int32_t best) { return best <= -65536; }   // a whole window agrees
+
+// Where the search for step t begins: with `wide` sets of as many context bits as leave 4 to 8 positions before t on
+// evenly spread keys, otherwise with all c bits - the buckets [first, first + n).
+struct Query {
+    uint32_t wq, ctx, l, first, n;
+};
+RC_HD Query query(const uint32_t* Q, uint32_t c, bool wide, uint32_t t) {
+    Query z;
+    z.wq = window(Q, t);
+    z.ctx = z.wq >> (32u - c);
+    z.l = c;
+    if (wide && 29u - leading(t) < c) z.l = 29u - leading(t);  // floor(log2 t) - 2
+    z.first = z.ctx >> (c - z.l) << (c - z.l);
+    z.n = 1u << (c - z.l);
+    return z;
+}
+
+// Agreements counted on beyond the windows: of the positions before t among entries [b, e), every step-th, whose window is
+// wq; packed as in scan_runs.
+RC_HD uint32_t scan_deep(const Entry* entries, uint32_t b, uint32_t e, uint32_t step, const uint32_t* Q, const uint32_t* K, uint32_t wq, uint32_t t,
+                         uint32_t& deep) {
+    uint32_t best = 0;
+    for (; b < e; b += step) {
+        const Entry a = entries[b];
+        if (a.r >= t || wq != a.key) continue;
+        const uint32_t v = agreement(Q, K, t, a.r, 0u, deep) << 16 | (a.r + 1u);
+        best = v > best ? v : best;
     }
-    uint32_t l = c;
-    if (wide && 29u - leading(t) < c) l = 29u - leading(t);    // floor(log2 t) - 2
-    const uint32_t first = ctx >> (c - l) << (c - l), n_first = 1u << (c - l);
-    int32_t best = scan(entries, start, first, n_first, t, wq, 32 * 65536);
-    if (best <= -65536) {                                      // a whole window agrees: count on beyond the windows
-        uint32_t most = 0, at = 0;
-        for (uint32_t b = start[first], e = start[first + n_first]; b < e; ++b) {
-            const uint32_t r = entries[b].r;
-            if (r >= t || wq != entries[b].key) continue;
-            const uint32_t n = agreement(Q, K, t, r, 0u, deep);
-            if (n > most || (n == most && r + 1u > at)) { most = n; at = r + 1u; }
-        }
-        return at;
+    return best;
+}
+
+// r + 1 for a step below BRUTE, 0 without a match.
+RC_HD uint32_t find_brute(const uint32_t* Q, const uint32_t* K, uint32_t t, uint32_t& deep) {
+    const uint32_t wq = window(Q, t);
+    uint32_t best = 0;
+    for (uint32_t r = 0; r < t; ++r) {
+        const uint32_t n = agreement(Q, K, t, r, wq ^ window(K, r), deep), v = n << 16 | (r + 1u);
+        best = n && v > best ? v : best;
     }
+    return best & 0xFFFFu;
+}
+
+// r + 1 for step t >= BRUTE, 0 without a match; best: what scan() found in the query's own buckets, not scan_full().
+// Whatever has not been looked at when the search ends agrees in fewer bits than the best.  (A position with a history
+// shorter than a context lies in the bucket of that history filled up with zeros, which agrees with the query in no fewer
+// bits than the history itself.)
+RC_HD uint32_t find_shorter(const Entry* entries, const uint16_t* start, uint32_t c, const Query& z, uint32_t t, int32_t best) {
+    uint32_t l = z.l;
     while (scan_agreement(best) < (int32_t)l && --l > 0u) {    // the buckets that agree in l bits and differ in the next
         const uint32_t sh = c - 1u - l;
-        best = scan_latest(entries, start, ((ctx >> sh) ^ 1u) << sh, 1u << sh, t, wq, best);
+        best = scan_latest(entries, start, ((z.ctx >> sh) ^ 1u) << sh, 1u << sh, t, z.wq, best);
     }
     return scan_agreement(best) > 0 ? scan_position(best) + 1u : 0u;
 }

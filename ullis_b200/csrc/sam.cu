@@ -345,6 +345,8 @@ struct ContextLimits {
     uint32_t deep;   // 32-step comparisons beyond the first, and words gone back, per thread before a stream is given up
 };
 
+constexpr uint32_t CONTEXT_LARGE = 48;   // positions before a step in its buckets from which on the whole warp looks through them
+
 struct ContextLayout {   // bytes of shared memory
     uint32_t hist, nq, start, q, k, q_ends, k_ends, in_word, before, out, entries, steps, total;
     __host__ __device__ ContextLayout(uint32_t T, uint32_t c, uint32_t warps) {
@@ -366,12 +368,15 @@ struct ContextLayout {   // bytes of shared memory
 };
 
 template <int NT>
-__global__ void __launch_bounds__(NT)
+__global__ void __launch_bounds__(NT, NT > 256 ? 2 : 5)
 rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restrict__ k_sw, const uint32_t* __restrict__ v_sw,
                     uint32_t* __restrict__ idx_sw, const uint32_t* __restrict__ list, const uint32_t* __restrict__ count,
                     uint32_t* __restrict__ next, uint32_t* __restrict__ hard, uint32_t* __restrict__ hard_count, uint32_t T,
                     size_t wps, uint32_t c, ContextLimits limits) {
     constexpr uint32_t NW = NT / 32, BRUTE = context::BRUTE;
+    // Large buckets by the whole warp: for few streams, where a launch lasts as long as its slowest row (one sequence 3.9 ->
+    // 3.6 ms); with many the ballots cost more than they save (16 sequences 12.5 -> 12.9 ms).
+    constexpr bool TOGETHER = NT > 256;
     extern __shared__ __align__(16) uint8_t context_mem[];
     __shared__ uint32_t sh_item, sh_sums[NW], sh_pairs[NW], sh_gone;
     const uint32_t C = 1u << c, pair_words = C / 2u, words = (T + 31u) / 32u;
@@ -555,13 +560,56 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
         uint32_t deep = 0;
         for (uint32_t row = warp; row < words; row += NW) {
             const uint32_t i = row * 32u + lane, t = sorted && i >= BRUTE && i < T ? steps[i - BRUTE] : i;
-            uint32_t bit = 0;
-            if (i < T) {
-                const uint32_t r1 = by_runs && i >= BRUTE
-                                        ? context::find_by_runs(entries, start, Q, K, q_ends, runs, words, c, t, deep)
-                                        : context::find(entries, start, Q, K, c, !sorted, t, deep);
-                bit = r1 ? (v[r1 >> 5] >> (r1 & 31u)) & 1u : 0u;
+            uint32_t r1 = 0;
+            if (row * 32u < BRUTE) {
+                if (i < T) r1 = context::find_brute(Q, K, t, deep);
+            } else {
+                // The step's bucket, or buckets; large ones are looked through by the whole warp, one step after the other
+                // (a lane alone with a bucket of 1 900 positions held up its warp for all of them).
+                uint32_t b = 0, e = 0, run = 0, found = 0;
+                context::Query z{};
+                int32_t best = context::SCAN_NOTHING;
+                if (i < T && by_runs) {
+                    const uint32_t key = context::run_key(Q, q_ends, t, c);
+                    run = context::run_at(Q, q_ends, t);
+                    b = start[key];
+                    e = start[key + 1u];
+                } else if (i < T) {
+                    z = context::query(Q, c, !sorted, t);
+                    b = start[z.first];
+                    e = start[z.first + z.n];
+                }
+                const bool large = TOGETHER && (e - b) * t > CONTEXT_LARGE * T;   // about so many of them lie before t
+                for (uint32_t open = TOGETHER ? __ballot_sync(0xFFFFFFFFu, large) : 0u; open; open &= open - 1u) {
+                    const int l = __ffs((int)open) - 1;
+                    const uint32_t lb = __shfl_sync(0xFFFFFFFFu, b, l) + lane, le = __shfl_sync(0xFFFFFFFFu, e, l);
+                    const uint32_t lt = __shfl_sync(0xFFFFFFFFu, t, l);
+                    uint32_t v = 0;
+                    if (by_runs) {
+                        const uint32_t lr = __shfl_sync(0xFFFFFFFFu, run, l);
+                        v = __reduce_max_sync(0xFFFFFFFFu, context::scan_runs(entries, lb, le, 32u, Q, K, runs, lr, lt, deep));
+                    } else {
+                        const uint32_t lw = __shfl_sync(0xFFFFFFFFu, z.wq, l);
+                        int32_t mine = context::SCAN_NOTHING;
+                        for (uint32_t k = lb; k < le; k += 32u) mine = context::scan_one(entries[k], lt, lw, mine);
+                        mine = __reduce_min_sync(0xFFFFFFFFu, mine);
+                        if (context::scan_full(mine)) v = __reduce_max_sync(0xFFFFFFFFu, context::scan_deep(entries, lb, le, 32u, Q, K, lw, lt, deep));
+                        else if ((int)lane == l) best = mine;
+                    }
+                    if ((int)lane == l) found = v;
+                }
+                if (i < T && by_runs) {
+                    if (!large) found = context::scan_runs(entries, b, e, 1u, Q, K, runs, run, t, deep);
+                    r1 = found ? found & 0xFFFFu : context::find_inside_run(K, runs, words, context::bit_at(Q, t), run, t, deep);
+                } else if (i < T) {
+                    if (!large) {
+                        best = context::scan(entries, start, z.first, z.n, t, z.wq, best);
+                        if (context::scan_full(best)) found = context::scan_deep(entries, b, e, 1u, Q, K, z.wq, t, deep);
+                    }
+                    r1 = found ? found & 0xFFFFu : context::find_shorter(entries, start, c, z, t, best);
+                }
             }
+            const uint32_t bit = r1 ? (v[r1 >> 5] >> (r1 & 31u)) & 1u : 0u;
             if (sorted) {
                 if (bit) atomicOr(&out_s[t >> 5], 1u << (t & 31u));
             } else {
