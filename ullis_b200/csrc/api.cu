@@ -475,8 +475,7 @@ int32_t ullis_cuda_runtime_sam_counts(ullis_cuda_runtime* rt, uint64_t* total, u
             ullis_cuda_runtime* r = lane == 0 ? rt : rt->children.at(lane - 1);
             uint32_t host[2] = {0, 0};
             if (r->sam_last_streams) {
-                // the two counters sit behind the automaton list (k::rosa_sam)
-                r->d2h(host, static_cast<uint32_t*>(r->sam_list.get()) + r->sam_last_streams, 8);
+                r->d2h(host, r->sam_last_counts, 8);
                 r->sync();
             }
             sum[0] += r->sam_last_streams;

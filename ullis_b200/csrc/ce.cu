@@ -53,6 +53,7 @@ __global__ void __launch_bounds__(1024)
 ce_reduce_kernel(const float* __restrict__ row_loss, const uint32_t* __restrict__ labels, uint32_t ignore_id,
                  size_t rows, size_t time, double* __restrict__ loss_sum, unsigned long long* __restrict__ n_valid,
                  double* __restrict__ pair) {
+    chain_entry();
     __shared__ double s_sum[1024];
     __shared__ unsigned long long s_cnt[1024];
     double acc = 0.0;
@@ -96,7 +97,7 @@ void ce_rows_from_logits(ullis_cuda_runtime* rt, const float* logits, const uint
 
 void ce_reduce(ullis_cuda_runtime* rt, const float* row_loss, const uint32_t* labels, uint32_t ignore_id,
                size_t rows, size_t time, double* loss_sum, unsigned long long* n_valid, double* pair) {
-    ce_reduce_kernel<<<1, 1024, 0, rt->stream>>>(row_loss, labels, ignore_id, rows, time, loss_sum, n_valid, pair);
+    rt->chain(ce_reduce_kernel, 1, 1024, 0, row_loss, labels, ignore_id, rows, time, loss_sum, n_valid, pair);
     rt->launched("ce_reduce");
 }
 

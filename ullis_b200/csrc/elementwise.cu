@@ -20,6 +20,7 @@ inline unsigned blocks_for(size_t n, unsigned per_block) { return (unsigned)((n 
 // reference src/model.rs:2660-2669
 __global__ void embed_kernel(const uint32_t* __restrict__ ids, const uint16_t* __restrict__ emb,
                              float* __restrict__ x, size_t rows, size_t d, size_t vocab, uint32_t* status) {
+    chain_entry();
     size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= rows * d) return;
     size_t row = e / d, c = e % d;
@@ -98,6 +99,7 @@ template <int VEC_PER_LANE>
 __global__ void __launch_bounds__(256)
 ln_warp_kernel(const float* __restrict__ x, const uint16_t* __restrict__ w, const uint16_t* __restrict__ b,
                float* __restrict__ y, size_t rows, int C) {
+    chain_entry();
     const int lane = threadIdx.x & 31;
     const size_t row = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= rows) return;
@@ -139,6 +141,7 @@ ln_warp_kernel(const float* __restrict__ x, const uint16_t* __restrict__ w, cons
 __global__ void __launch_bounds__(256)
 ln_warp_generic_kernel(const float* __restrict__ x, const uint16_t* __restrict__ w,
                        const uint16_t* __restrict__ b, float* __restrict__ y, size_t rows, size_t C) {
+    chain_entry();
     const int lane = threadIdx.x & 31;
     const size_t row = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= rows) return;
@@ -209,6 +212,7 @@ sign_pack_streams_kernel(const float* __restrict__ x, uint32_t* __restrict__ sw,
 // flat [B,T,C] plane words -> stream-major words (any T, C)
 __global__ void planes_to_streams_kernel(const uint32_t* __restrict__ plane, uint32_t* __restrict__ sw, size_t B,
                                          size_t T, size_t C, size_t wps) {
+    chain_entry();
     size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= B * C * wps) return;
     size_t s = e / wps, wd = e % wps, b = s / C, c = s % C;
@@ -231,6 +235,7 @@ constexpr int P2S_BLOCKS = 8;
 __global__ void __launch_bounds__(512)
 planes_to_streams_words_kernel(const uint32_t* __restrict__ plane, uint32_t* __restrict__ sw, size_t T, size_t C,
                                size_t wps) {
+    chain_entry();
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, cwords = (uint32_t)(C >> 5);
     const size_t b = blockIdx.z, tb0 = (size_t)blockIdx.x * P2S_BLOCKS;
     const uint32_t cw = blockIdx.y * (blockDim.x >> 5) + warp;
@@ -256,6 +261,7 @@ planes_to_streams_words_kernel(const uint32_t* __restrict__ plane, uint32_t* __r
 
 __global__ void streams_to_planes_kernel(const uint32_t* __restrict__ sw, uint32_t* __restrict__ plane, size_t B,
                                          size_t T, size_t C, size_t wps) {
+    chain_entry();
     size_t wd = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t n = B * T * C;
     if (wd >= (n + 31) / 32) return;
@@ -287,6 +293,7 @@ __global__ void residual_add_kernel(const float* __restrict__ a, const float* __
 __global__ void __launch_bounds__(1024)
 rosa_emit_kernel(const uint32_t* __restrict__ idx_sw, const uint16_t* __restrict__ e, uint8_t* __restrict__ idx,
                  float* __restrict__ y, size_t T, size_t C, size_t wps) {
+    chain_entry();
     __shared__ uint32_t wsm[32];
     const size_t b = blockIdx.z, t0 = (size_t)blockIdx.x * 32, c0 = (size_t)blockIdx.y * 32;
     const int tx = threadIdx.x, ty = threadIdx.y;
@@ -307,7 +314,7 @@ rosa_emit_kernel(const uint32_t* __restrict__ idx_sw, const uint16_t* __restrict
 void embed(ullis_cuda_runtime* rt, const uint32_t* ids, const uint16_t* emb, float* x, size_t rows, size_t d,
            size_t vocab) {
     if (rows * d == 0) return;
-    embed_kernel<<<blocks_for(rows * d, 256), 256, 0, rt->stream>>>(ids, emb, x, rows, d, vocab, rt->dev_status);
+    rt->chain(embed_kernel, blocks_for(rows * d, 256), 256, 0, ids, emb, x, rows, d, vocab, rt->dev_status);
     rt->launched("embed");
 }
 
@@ -325,17 +332,17 @@ void layer_norm(ullis_cuda_runtime* rt, const float* x, const uint16_t* w, const
                      (reinterpret_cast<uintptr_t>(w) % 8 == 0) && (reinterpret_cast<uintptr_t>(b) % 8 == 0);
     if (vec) {
         switch (channels / 128) {
-            case 1: ln_warp_kernel<1><<<grid, 256, 0, rt->stream>>>(x, w, b, y, rows, (int)channels); break;
-            case 2: ln_warp_kernel<2><<<grid, 256, 0, rt->stream>>>(x, w, b, y, rows, (int)channels); break;
-            case 3: ln_warp_kernel<3><<<grid, 256, 0, rt->stream>>>(x, w, b, y, rows, (int)channels); break;
-            case 4: ln_warp_kernel<4><<<grid, 256, 0, rt->stream>>>(x, w, b, y, rows, (int)channels); break;
-            case 5: ln_warp_kernel<5><<<grid, 256, 0, rt->stream>>>(x, w, b, y, rows, (int)channels); break;
-            case 6: ln_warp_kernel<6><<<grid, 256, 0, rt->stream>>>(x, w, b, y, rows, (int)channels); break;
-            case 7: ln_warp_kernel<7><<<grid, 256, 0, rt->stream>>>(x, w, b, y, rows, (int)channels); break;
-            default: ln_warp_kernel<8><<<grid, 256, 0, rt->stream>>>(x, w, b, y, rows, (int)channels); break;
+            case 1: rt->chain_small(ln_warp_kernel<1>, grid, 256, 0, x, w, b, y, rows, (int)channels); break;
+            case 2: rt->chain_small(ln_warp_kernel<2>, grid, 256, 0, x, w, b, y, rows, (int)channels); break;
+            case 3: rt->chain_small(ln_warp_kernel<3>, grid, 256, 0, x, w, b, y, rows, (int)channels); break;
+            case 4: rt->chain_small(ln_warp_kernel<4>, grid, 256, 0, x, w, b, y, rows, (int)channels); break;
+            case 5: rt->chain_small(ln_warp_kernel<5>, grid, 256, 0, x, w, b, y, rows, (int)channels); break;
+            case 6: rt->chain_small(ln_warp_kernel<6>, grid, 256, 0, x, w, b, y, rows, (int)channels); break;
+            case 7: rt->chain_small(ln_warp_kernel<7>, grid, 256, 0, x, w, b, y, rows, (int)channels); break;
+            default: rt->chain_small(ln_warp_kernel<8>, grid, 256, 0, x, w, b, y, rows, (int)channels); break;
         }
     } else {
-        ln_warp_generic_kernel<<<grid, 256, 0, rt->stream>>>(x, w, b, y, rows, channels);
+        rt->chain_small(ln_warp_generic_kernel, grid, 256, 0, x, w, b, y, rows, channels);
     }
     rt->launched("ln_warp");
 }
@@ -378,11 +385,11 @@ void planes_to_streams(ullis_cuda_runtime* rt, const uint32_t* plane, uint32_t* 
     if (channels % 32 == 0 && batch <= 65535) {
         const unsigned cwords = (unsigned)(channels / 32), warps = cwords < 16 ? cwords : 16;
         dim3 grid((unsigned)((wps + P2S_BLOCKS - 1) / P2S_BLOCKS), (cwords + warps - 1) / warps, (unsigned)batch);
-        planes_to_streams_words_kernel<<<grid, warps * 32, 0, rt->stream>>>(plane, sw, time, channels, wps);
+        rt->chain(planes_to_streams_words_kernel, grid, warps * 32, 0, plane, sw, time, channels, wps);
         rt->launched("planes_to_streams");
         return;
     }
-    planes_to_streams_kernel<<<blocks_for(n, 256), 256, 0, rt->stream>>>(plane, sw, batch, time, channels, wps);
+    rt->chain(planes_to_streams_kernel, blocks_for(n, 256), 256, 0, plane, sw, batch, time, channels, wps);
     rt->launched("planes_to_streams");
 }
 
@@ -390,7 +397,7 @@ void streams_to_planes(ullis_cuda_runtime* rt, const uint32_t* sw, uint32_t* pla
                        size_t channels) {
     const size_t wps = (time + 31) / 32, n = (batch * time * channels + 31) / 32;
     if (!n) return;
-    streams_to_planes_kernel<<<blocks_for(n, 256), 256, 0, rt->stream>>>(sw, plane, batch, time, channels, wps);
+    rt->chain(streams_to_planes_kernel, blocks_for(n, 256), 256, 0, sw, plane, batch, time, channels, wps);
     rt->launched("streams_to_planes");
 }
 
@@ -411,7 +418,7 @@ void rosa_emit(ullis_cuda_runtime* rt, const uint32_t* idx_sw, const uint16_t* e
     if (batch * time * channels == 0) return;
     const size_t wps = (time + 31) / 32;
     dim3 grid((unsigned)wps, (unsigned)((channels + 31) / 32), (unsigned)batch);
-    rosa_emit_kernel<<<grid, dim3(32, 32), 0, rt->stream>>>(idx_sw, e, idx, y, time, channels, wps);
+    rt->chain(rosa_emit_kernel, grid, dim3(32, 32), 0, idx_sw, e, idx, y, time, channels, wps);
     rt->launched("rosa_emit");
 }
 

@@ -55,6 +55,7 @@ __device__ __forceinline__ float h2f(uint16_t b) { return __half2float(__ushort_
 // (FP16 ends at 65504: a larger finite input is reported through the status word, not turned into inf)
 __global__ void cast16_kernel(const float* __restrict__ x, uint16_t* __restrict__ y, size_t n, int bf16, size_t K,
                               uint32_t* __restrict__ status) {
+    chain_entry();
     size_t e = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (e >= n) return;
     float v[4];
@@ -78,6 +79,7 @@ mix_split_kernel(const float* __restrict__ x, const uint16_t* __restrict__ m0, c
                  const uint16_t* __restrict__ m2, uint16_t* __restrict__ hi0, uint16_t* __restrict__ lo0,
                  uint16_t* __restrict__ hi1, uint16_t* __restrict__ lo1, uint16_t* __restrict__ hi2,
                  uint16_t* __restrict__ lo2, float* __restrict__ s1, size_t rows, size_t time, size_t pitch, size_t C) {
+    chain_entry();
     const int lane = threadIdx.x & 31;
     const size_t row = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= rows) return;
@@ -140,6 +142,7 @@ ln_mix_split_kernel(const float* __restrict__ x, const uint16_t* __restrict__ lw
                     const uint16_t* __restrict__ m2, uint16_t* __restrict__ hi0, uint16_t* __restrict__ lo0,
                     uint16_t* __restrict__ hi1, uint16_t* __restrict__ lo1, uint16_t* __restrict__ hi2,
                     uint16_t* __restrict__ lo2, float* __restrict__ s1, size_t rows, size_t time, size_t pitch) {
+    chain_entry();
     constexpr int C = 128 * VEC;
     const int lane = threadIdx.x & 31;
     // a warp takes ROWS consecutive rows: the LayerNorm of a row is then computed once and handed on as the next
@@ -248,6 +251,7 @@ ln_mix_split_kernel(const float* __restrict__ x, const uint16_t* __restrict__ lw
 __global__ void __launch_bounds__(256)
 emit_f16_kernel(const uint32_t* __restrict__ idx_sw, const uint16_t* __restrict__ e, uint16_t* __restrict__ y,
                 size_t T, size_t C, size_t wps) {
+    chain_entry();
     __shared__ __align__(16) uint32_t wsm[256];
     const size_t b = blockIdx.z, t0 = (size_t)blockIdx.x * 32, c0 = (size_t)blockIdx.y * 256;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -321,6 +325,7 @@ constexpr int FIXQ_MAX_WORDS = 32;
 __global__ void __launch_bounds__(256)
 fix_collect_kernel(const uint32_t* __restrict__ flags, size_t sw, size_t batch, size_t C, size_t wps,
                    uint32_t* __restrict__ list, uint32_t cap, uint32_t* __restrict__ ctrl) {
+    chain_entry();
     const int lane = threadIdx.x & 31;
     const size_t warps = ((size_t)gridDim.x * blockDim.x) >> 5;
     const size_t buckets = batch * wps * 3;
@@ -378,6 +383,7 @@ fix_apply_kernel(const float* __restrict__ x, const uint16_t* __restrict__ mq, c
                  uint32_t* __restrict__ bq, uint32_t* __restrict__ bk, uint32_t* __restrict__ bv,
                  const uint32_t* __restrict__ list, uint32_t cap, const uint32_t* __restrict__ ctrl, size_t sw, size_t T,
                  size_t C, size_t wps) {
+    chain_entry();
     __shared__ float terms[FIXQ_WARPS][32 * FIXQ_PITCH];
     // what the whole warp needs to know about entry e, written by lane e once per task
     __shared__ const float* e_row[FIXQ_WARPS][32];
@@ -474,7 +480,10 @@ sign_fixup_kernel(const float* __restrict__ x, const uint16_t* __restrict__ mq, 
                   const uint16_t* __restrict__ mv, PackedWeights wq, PackedWeights wk, PackedWeights wv,
                   uint32_t* __restrict__ bq, uint32_t* __restrict__ bk, uint32_t* __restrict__ bv,
                   const uint32_t* __restrict__ fq, const uint32_t* __restrict__ fk, const uint32_t* __restrict__ fv,
-                  size_t batch, size_t T, size_t C, size_t wps, const uint32_t* __restrict__ only_if) {
+                  size_t batch, size_t T, size_t C, size_t wps, const uint32_t* __restrict__ only_if,
+                  uint32_t* __restrict__ clear) {
+    chain_entry();
+    if (clear && blockIdx.x == 0 && threadIdx.x < 2) clear[threadIdx.x] = 0u;   // the counters of the next call
     if (only_if && *only_if == 0u) return;   // the compact list took every flag: nothing left for the windows
     extern __shared__ uint32_t fix_queue[];  // entries: matrix << 28 | channel << 8 | word in window << 5 | bit
     __shared__ uint32_t q_count, announced;   // entries queued; flag bits announced so far (never reset)
@@ -562,6 +571,7 @@ sign_fixup_kernel(const float* __restrict__ x, const uint16_t* __restrict__ mq, 
 __global__ void ce_finish_kernel(const float2* __restrict__ part, const float* __restrict__ target_logit,
                                  const uint32_t* __restrict__ labels, uint32_t ignore_id, size_t rows, size_t time,
                                  size_t vocab, uint32_t n_tiles, float* __restrict__ row_loss, uint32_t* status) {
+    chain_entry();
     const size_t m = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= rows) return;
     const bool valid = time != 0 && (m % time) + 1 < time && m + 1 < rows && labels[m + 1] != ignore_id;
@@ -595,16 +605,18 @@ template <int EPI, bool RESIDENT_W = true>
 int ws2_resident_clusters(ullis_cuda_runtime* rt) {
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 2;
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 1;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // as ullis_cuda_runtime::chain
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.gridDim = dim3(2u * (unsigned)rt->sm_count);
     cfg.blockDim = dim3(WS2_THREADS);
     cfg.dynamicSmemBytes = WS_SMEM_LIMIT;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, gemm_ws2_kernel<EPI, RESIDENT_W>, &cfg) != cudaSuccess) {
         cudaGetLastError();
@@ -698,17 +710,19 @@ void launch_ws2(ullis_cuda_runtime* rt, const GemmMaps& maps, const GemmParams& 
     if (members > m_tiles) members = m_tiles;
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 2;
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 1;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // as ullis_cuda_runtime::chain
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.gridDim = dim3(2u * pairs * members);
     cfg.blockDim = dim3(WS2_THREADS);
     cfg.dynamicSmemBytes = shape.smem;
     cfg.stream = rt->stream;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
     if (rt->kernel_timing) rt->mark("(cta_pair)");   // a zero-length entry in the timing table: which form ran
     ULLIS_CUDA_CHECK(cudaLaunchKernelEx(&cfg, gemm_ws2_kernel<EPI, RESIDENT_W>, maps, q, pairs));
     rt->launched(what);
@@ -730,7 +744,7 @@ void launch(ullis_cuda_runtime* rt, const GemmMaps& maps, const GemmParams& p, u
             uint32_t members = (uint32_t)rt->sm_count / pairs;
             if (members < 1) members = 1;
             if (members > m_tiles) members = m_tiles;
-            gemm_ws_kernel<EPI><<<pairs * members, WS_THREADS, shape.smem, rt->stream>>>(maps, q, pairs);
+            rt->chain(gemm_ws_kernel<EPI>, pairs * members, WS_THREADS, shape.smem, maps, q, pairs);
             rt->launched(what);
             return;
         }
@@ -752,13 +766,13 @@ void launch(ullis_cuda_runtime* rt, const GemmMaps& maps, const GemmParams& p, u
             uint32_t members = (uint32_t)rt->sm_count / pairs;
             if (members < 1) members = 1;
             if (members > m_tiles) members = m_tiles;
-            gemm_ws_kernel<EPI, false><<<pairs * members, WS_THREADS, shape.smem, rt->stream>>>(maps, q, pairs);
+            rt->chain(gemm_ws_kernel<EPI, false>, pairs * members, WS_THREADS, shape.smem, maps, q, pairs);
             rt->launched(what);
             return;
         }
     }
     dim3 grid((p.N + BN - 1) / BN, (p.M + BM - 1) / BM, n_prob);
-    gemm_kernel<EPI, PACKED><<<grid, GEMM_THREADS, gemm_smem_bytes(p.n_a, p.stages), rt->stream>>>(maps, p);
+    rt->chain(gemm_kernel<EPI, PACKED>, grid, GEMM_THREADS, gemm_smem_bytes(p.n_a, p.stages), maps, p);
     rt->launched(what);
 }
 
@@ -789,13 +803,13 @@ bool launch_ln_mix_split(ullis_cuda_runtime* rt, const float* x, const LayerNorm
 #define ULLIS_LN_MIX(V)                                                                                                  \
     do {                                                                                                                 \
         if (per_warp == 4)                                                                                               \
-            ln_mix_split_kernel<V, 4><<<grid, 256, 0, rt->stream>>>(x, ln.weight, ln.bias, ln_out, m0, m1, m2, hi0, lo0, \
+            rt->chain_small(ln_mix_split_kernel<V, 4>, grid, 256, 0, x, ln.weight, ln.bias, ln_out, m0, m1, m2, hi0, lo0, \
                                                                     hi1, lo1, hi2, lo2, s1, rows, time, pitch);                 \
         else if (per_warp == 2)                                                                                          \
-            ln_mix_split_kernel<V, 2><<<grid, 256, 0, rt->stream>>>(x, ln.weight, ln.bias, ln_out, m0, m1, m2, hi0, lo0, \
+            rt->chain_small(ln_mix_split_kernel<V, 2>, grid, 256, 0, x, ln.weight, ln.bias, ln_out, m0, m1, m2, hi0, lo0, \
                                                                     hi1, lo1, hi2, lo2, s1, rows, time, pitch);                 \
         else                                                                                                             \
-            ln_mix_split_kernel<V, 1><<<grid, 256, 0, rt->stream>>>(x, ln.weight, ln.bias, ln_out, m0, m1, m2, hi0, lo0, \
+            rt->chain_small(ln_mix_split_kernel<V, 1>, grid, 256, 0, x, ln.weight, ln.bias, ln_out, m0, m1, m2, hi0, lo0, \
                                                                     hi1, lo1, hi2, lo2, s1, rows, time, pitch);                 \
     } while (0)
     switch (d / 128) {
@@ -816,7 +830,7 @@ bool launch_ln_mix_split(ullis_cuda_runtime* rt, const float* x, const LayerNorm
 // x [rows, K] f32 -> 16-bit operand
 void cast16(ullis_cuda_runtime* rt, const float* x, uint16_t* y, size_t rows, size_t K, bool bf16) {
     const size_t n = rows * K;
-    cast16_kernel<<<blocks_for((n + 3) / 4, 256), 256, 0, rt->stream>>>(x, y, n, bf16 ? 1 : 0, K, rt->dev_status);
+    rt->chain(cast16_kernel, blocks_for((n + 3) / 4, 256), 256, 0, x, y, n, bf16 ? 1 : 0, K, rt->dev_status);
     rt->launched("cast16");
 }
 
@@ -888,7 +902,7 @@ bool dense_nt(ullis_cuda_runtime* rt, const uint16_t* a16, const uint16_t* b16, 
             p.split_k = splits;
             p.prob[0].out = part;
             dim3 grid((unsigned)((N + BN - 1) / BN), (unsigned)((M + BM - 1) / BM), splits);
-            gemm_kernel<EPI_STORE, false><<<grid, GEMM_THREADS, gemm_smem_bytes(p.n_a, p.stages), rt->stream>>>(maps, p);
+            rt->chain(gemm_kernel<EPI_STORE, false>, grid, GEMM_THREADS, gemm_smem_bytes(p.n_a, p.stages), maps, p);
             rt->launched("gemm_dense_nt_splitk");
             const size_t n = M * N;
             splitk_reduce_kernel<<<blocks_for((n + 3) / 4, 256), 256, 0, rt->stream>>>(part, y, splits, n);
@@ -916,7 +930,7 @@ bool rosa_qkv_bits(ullis_cuda_runtime* rt, const float* ln3_out, const LayerWeig
     if (!(x_before_ln && launch_ln_mix_split(rt, x_before_ln, L.ln3, ln3_write, L.x_q, L.x_k, L.x_v, op, op + 3 * n, op + n,
                                              op + 4 * n, op + 2 * n, op + 5 * n, s1, rows, time, pitch, d, "ln_mix_split"))) {
         if (x_before_ln) k::layer_norm(rt, x_before_ln, L.ln3.weight, L.ln3.bias, ln3_write, rows, d, false);
-        mix_split_kernel<<<blocks_for(rows, 8), 256, 0, rt->stream>>>(ln3_out, L.x_q, L.x_k, L.x_v, op, op + 3 * n, op + n,
+        rt->chain_small(mix_split_kernel, blocks_for(rows, 8), 256, 0, ln3_out, L.x_q, L.x_k, L.x_v, op, op + 3 * n, op + n,
                                                                      op + 4 * n, op + 2 * n, op + 5 * n, s1, rows, time, pitch, d);
         rt->launched("mix_split");
     }
@@ -939,22 +953,23 @@ bool rosa_qkv_bits(ullis_cuda_runtime* rt, const float* ln3_out, const LayerWeig
     launch<EPI_SIGNBITS, true>(rt, maps, p, 3, "gemm_qkv_signbits");
     const unsigned grid = (unsigned)(((wps + FIX_WIN - 1) / FIX_WIN) * batch);   // rows < 2^30, so this fits
     const uint32_t* only_if = nullptr;
+    uint32_t* clear = nullptr;
     if (rt->tc_fix_list && 3 * sw < ((size_t)1 << 27) && d % FIXQ_COLS == 0 && d <= 32 * FIXQ_MAX_WORDS) {
         // one thread per flagged output, from a compact list; room for one output in 64
         const size_t cap = std::max<size_t>(65536, 3 * sw * 32 / 64);
-        uint32_t* ctrl = rt->tc_ws[9].as<uint32_t>(2 + cap);
-        uint32_t* list = ctrl + 2;
-        rt->zero(ctrl, 8);
-        fix_collect_kernel<<<4 * (unsigned)rt->sm_count, 256, 0, rt->stream>>>(flags, sw, batch, d, wps, list, (uint32_t)cap, ctrl);
+        uint32_t* list = rt->tc_ws[9].as<uint32_t>(cap);
+        uint32_t* ctrl = nullptr;
+        rt->counters(rt->fix_counters, 2, &ctrl, &clear);
+        rt->chain(fix_collect_kernel, 4 * (unsigned)rt->sm_count, 256, 0, flags, sw, batch, d, wps, list, (uint32_t)cap, ctrl);
         rt->launched("fix_collect");
-        fix_apply_kernel<<<12 * (unsigned)rt->sm_count, FIXQ_WARPS * 32, 0, rt->stream>>>(
-            ln3_out, L.x_q, L.x_k, L.x_v, L.q, L.k, L.v, q_sw, k_sw, v_sw, list, (uint32_t)cap, ctrl, sw, time, d, wps);
+        rt->chain(fix_apply_kernel, 12 * (unsigned)rt->sm_count, FIXQ_WARPS * 32, 0, ln3_out, L.x_q, L.x_k, L.x_v, L.q, L.k, L.v, q_sw, k_sw, v_sw, list, (uint32_t)cap, ctrl, sw, time, d, wps);
         rt->launched("fix_apply");
         only_if = ctrl + 1;
     }
-    sign_fixup_kernel<<<grid, FIX_THREADS, FIX_QUEUE * 4, rt->stream>>>(ln3_out, L.x_q, L.x_k, L.x_v, L.q, L.k, L.v, q_sw, k_sw, v_sw, flags,
-                                                   flags + sw, flags + 2 * sw, batch, time, d, wps, only_if);
+    rt->chain(sign_fixup_kernel, grid, FIX_THREADS, FIX_QUEUE * 4, ln3_out, L.x_q, L.x_k, L.x_v, L.q, L.k, L.v, q_sw, k_sw, v_sw, flags,
+                                                   flags + sw, flags + 2 * sw, batch, time, d, wps, only_if, clear);
     rt->launched("sign_fixup");
+    if (clear) rt->counters_cleared(rt->fix_counters);
     return true;
 }
 
@@ -965,7 +980,7 @@ bool rosa_out_residual(ullis_cuda_runtime* rt, const uint32_t* idx_sw, const Lay
     uint16_t* y16 = rt->tc_ws[0].as<uint16_t>(rows * d);
     const size_t wps = (time + 31) / 32;
     dim3 grid((unsigned)wps, (unsigned)((d + 255) / 256), (unsigned)batch);
-    emit_f16_kernel<<<grid, 256, 0, rt->stream>>>(idx_sw, L.e, y16, time, d, wps);
+    rt->chain(emit_f16_kernel, grid, 256, 0, idx_sw, L.e, y16, time, d, wps);
     rt->launched("emit_f16");
     GemmMaps maps;
     memset(&maps, 0, sizeof(maps));
@@ -986,7 +1001,7 @@ bool cmix_residual(ullis_cuda_runtime* rt, const LayerWeights& L, float* x, size
     if (!launch_ln_mix_split(rt, x, L.ln2, nullptr, L.ffn_x_k, nullptr, nullptr, a16, nullptr, nullptr, nullptr, nullptr,
                              nullptr, nullptr, rows, time, time, d, "ln_mix_f16")) {
         k::layer_norm(rt, x, L.ln2.weight, L.ln2.bias, ln, rows, d, false);
-        mix_split_kernel<<<blocks_for(rows, 8), 256, 0, rt->stream>>>(ln, L.ffn_x_k, nullptr, nullptr, a16, nullptr,
+        rt->chain_small(mix_split_kernel, blocks_for(rows, 8), 256, 0, ln, L.ffn_x_k, nullptr, nullptr, a16, nullptr,
                                                                      nullptr, nullptr, nullptr, nullptr, nullptr, rows, time, time, d);
         rt->launched("mix_f16");
     }
@@ -1051,7 +1066,7 @@ bool head_ce(ullis_cuda_runtime* rt, const float* hidden, const PackedWeights& h
     p.time = (uint32_t)time;
     p.prob[0] = GemmProblem{head.bits, head.scale, head.bias, part, tl, nullptr};
     launch<EPI_CE, true>(rt, maps, p, 1, "gemm_head_ce");
-    ce_finish_kernel<<<blocks_for(rows, 256), 256, 0, rt->stream>>>(part, tl, labels, ignore_id, rows, time, vocab, n_tiles,
+    rt->chain(ce_finish_kernel, blocks_for(rows, 256), 256, 0, part, tl, labels, ignore_id, rows, time, vocab, n_tiles,
                                                                   row_loss, rt->dev_status);
     rt->launched("ce_finish");
     return true;

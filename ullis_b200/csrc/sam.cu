@@ -43,6 +43,7 @@ rosa_classify_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restri
                      const uint32_t* __restrict__ v_sw, uint32_t* __restrict__ idx_sw, size_t streams, uint32_t T,
                      size_t wps, uint32_t* __restrict__ list, uint32_t* __restrict__ count,
                      uint32_t* __restrict__ cq_list, uint32_t* __restrict__ cq_count) {
+    chain_entry();
     constexpr uint32_t G = CLASSIFY_LANES;
     const size_t s = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
     if (s >= streams) return;   // a whole group
@@ -373,6 +374,7 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
                     uint32_t* __restrict__ idx_sw, const uint32_t* __restrict__ list, const uint32_t* __restrict__ count,
                     uint32_t* __restrict__ next, uint32_t* __restrict__ hard, uint32_t* __restrict__ hard_count, uint32_t T,
                     size_t wps, uint32_t c, ContextLimits limits) {
+    chain_entry();
     constexpr uint32_t NW = NT / 32, BRUTE = context::BRUTE;
     // Large buckets by the whole warp: for few streams, where a launch lasts as long as its slowest row (one sequence 3.9 ->
     // 3.6 ms); with many the ballots cost more than they save (16 sequences 12.5 -> 12.9 ms).
@@ -634,6 +636,7 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
 // The remaining streams by sets of lags (rosa_match.cuh).  A work item is a piece of one stream, a warp takes items
 // from a counter until they run out; the warps of a CTA have nothing to do with one another.
 constexpr int MATCH_WARPS = 4;
+constexpr uint32_t MATCH_COUNTS = 5;   // of MatchCall
 
 // A stream whose query bits are all c: idx follows the longest run of c among the keys so far, the latest of equals
 // (sam_core.cuh run_constant_q), a running maximum over (run length, position).  T <= 65535.
@@ -666,7 +669,9 @@ __global__ void __launch_bounds__(32 * MATCH_WARPS)
 rosa_match_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restrict__ k_sw, const uint32_t* __restrict__ v_sw,
                   uint32_t* __restrict__ idx_sw, const uint32_t* __restrict__ hard, const uint32_t* __restrict__ hard_count,
                   const uint32_t* __restrict__ cq_list, const uint32_t* __restrict__ cq_count, uint32_t* __restrict__ next,
-                  uint32_t* __restrict__ kept, uint32_t T, size_t wps, uint32_t ring_words) {
+                  uint32_t* __restrict__ clear, uint32_t* __restrict__ kept, uint32_t T, size_t wps, uint32_t ring_words) {
+    chain_entry();
+    if (blockIdx.x == 0 && threadIdx.x < MATCH_COUNTS) clear[threadIdx.x] = 0u;   // the counters of the next call
     extern __shared__ __align__(16) uint32_t match_mem[];
     const match::Layout L(NW, ring_words);
     uint32_t* mem = match_mem + (threadIdx.x >> 5) * L.total;
@@ -703,11 +708,10 @@ rosa_match_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restrict_
 
 struct MatchCall {   // the buffers of one call
     const uint32_t *q, *k, *v;
-    uint32_t *idx, *list, *cq_list, *hard, *counts;   // counts: listed, constant q, hard, next of the contexts, next of the matches
+    uint32_t *idx, *list, *cq_list, *hard, *clear, *counts;   // counts: listed, constant q, hard, next of the contexts, next of the matches
     size_t streams, wps;
     uint32_t T;
 };
-constexpr uint32_t MATCH_COUNTS = 5;
 
 template <int NT>
 void launch_context(ullis_cuda_runtime* rt, const MatchCall& m, int slot) {
@@ -724,7 +728,7 @@ void launch_context(ullis_cuda_runtime* rt, const MatchCall& m, int slot) {
     // A match kernel step costs about as much as 100 positions here; up to 24 the lanes are even enough without sorting
     // the steps.  128 long comparisons per stream at most are thrown away when a stream turns out to repeat itself.
     const ContextLimits limits{24u, 96u, 160u, 256u};
-    rosa_context_kernel<NT><<<grid, NT, smem, rt->stream>>>(m.q, m.k, m.v, m.idx, m.list, m.counts, m.counts + 3, m.hard,
+    rt->chain(rosa_context_kernel<NT>, grid, NT, smem, m.q, m.k, m.v, m.idx, m.list, m.counts, m.counts + 3, m.hard,
                                                             m.counts + 2, m.T, m.wps, c, limits);
     rt->launched("rosa_context");
 }
@@ -742,8 +746,8 @@ void launch_match(ullis_cuda_runtime* rt, const MatchCall& m, int slot, uint32_t
     const size_t most = (m.streams * m.wps + MATCH_WARPS - 1) / MATCH_WARPS;   // every stream in the shortest pieces
     const unsigned grid = (unsigned)std::min<size_t>(rt->match_ctas[slot], most);
     uint32_t* kept = rt->sam_scratch.as<uint32_t>((size_t)grid * MATCH_WARPS * match::CHECKPOINTS * 32u * NW);
-    rosa_match_kernel<NW><<<grid, 32 * MATCH_WARPS, smem, rt->stream>>>(m.q, m.k, m.v, m.idx, m.hard, m.counts + 2, m.cq_list,
-                                                                        m.counts + 1, m.counts + 4, kept, m.T, m.wps, ring_words);
+    rt->chain(rosa_match_kernel<NW>, grid, 32 * MATCH_WARPS, smem, m.q, m.k, m.v, m.idx, m.hard, m.counts + 2, m.cq_list,
+                                                                        m.counts + 1, m.counts + 4, m.clear, kept, m.T, m.wps, ring_words);
     rt->launched("rosa_match");
 }
 
@@ -768,15 +772,14 @@ void rosa_match(ullis_cuda_runtime* rt, const uint32_t* q_sw, const uint32_t* k_
     MatchCall m;
     m.q = q_sw; m.k = k_sw; m.v = v_sw; m.idx = idx_sw;
     m.streams = streams; m.T = T; m.wps = (T + 31u) / 32u;
-    m.list = rt->sam_list.as<uint32_t>(3 * streams + MATCH_COUNTS);
-    m.counts = m.list + streams;
-    m.cq_list = m.counts + MATCH_COUNTS;
+    m.list = rt->sam_list.as<uint32_t>(3 * streams);
+    m.cq_list = m.list + streams;
     m.hard = m.cq_list + streams;
+    rt->counters(rt->match_counters, MATCH_COUNTS, &m.counts, &m.clear);
+    rt->sam_last_counts = m.counts;
     rt->sam_last_streams = streams;
     if (!rt->parent) rt->lanes_last = 1;
-    rt->zero(m.counts, MATCH_COUNTS * 4u);
-    rosa_classify_kernel<<<(unsigned)((streams * CLASSIFY_LANES + 127) / 128), 128, 0, rt->stream>>>(
-        q_sw, k_sw, v_sw, idx_sw, streams, T, m.wps, m.list, m.counts, m.cq_list, m.counts + 1);
+    rt->chain(rosa_classify_kernel, (unsigned)((streams * CLASSIFY_LANES + 127) / 128), 128, 0, q_sw, k_sw, v_sw, idx_sw, streams, T, m.wps, m.list, m.counts, m.cq_list, m.counts + 1);
     rt->launched("rosa_classify");
     // few streams: sixteen warps each, so that the last of them is done soon (one sequence of 512 channels: 0.20 ms
     // against 0.28 with eight); many: eight (1.79 ms for 32 768 streams against 1.98 with sixteen)
@@ -786,6 +789,7 @@ void rosa_match(ullis_cuda_runtime* rt, const uint32_t* q_sw, const uint32_t* k_
     else if (T <= 2048u) launch_match<2>(rt, m, 1, 1024);
     else if (T <= 4096u) launch_match<4>(rt, m, 2, 2048);
     else launch_match<8>(rt, m, 3, 4096);
+    rt->counters_cleared(rt->match_counters);
 }
 
 }  // namespace
@@ -823,10 +827,11 @@ void rosa_sam(ullis_cuda_runtime* rt, const uint32_t* q_sw, const uint32_t* k_sw
         if (wave > streams) wave = streams;
     }
     uint8_t* scratch = static_cast<uint8_t*>(rt->sam_scratch.ensure(wave * stride));
-    uint32_t* list = rt->sam_list.as<uint32_t>(3 * streams + MATCH_COUNTS);
+    uint32_t* list = rt->sam_list.as<uint32_t>(2 * streams + 3);
     rt->sam_last_streams = streams;
     if (!rt->parent) rt->lanes_last = 1;   // a forward that splits its batch raises this after its last layer
     uint32_t* count = list + streams;
+    rt->sam_last_counts = count;
     uint32_t* cq_count = count + 1;           // the constant-q streams, settled by a kernel of their own
     uint32_t* cq_list = count + 3;
     const unsigned cgrid = (unsigned)((streams + 127) / 128);
@@ -851,7 +856,7 @@ void rosa_sam(ullis_cuda_runtime* rt, const uint32_t* q_sw, const uint32_t* k_sw
     } else {
         rt->zero(count, 8);   // both counters
         const unsigned classify_grid = (unsigned)((streams * CLASSIFY_LANES + 127) / 128);
-        rosa_classify_kernel<<<classify_grid, 128, 0, rt->stream>>>(q_sw, k_sw, v_sw, idx_sw, streams, (uint32_t)time, wps, list,
+        rt->chain(rosa_classify_kernel, classify_grid, 128, 0, q_sw, k_sw, v_sw, idx_sw, streams, (uint32_t)time, wps, list,
                                                              count, cq_list, cq_count);
         rt->launched("rosa_classify");
         // The constant-q scan is a long serial loop for a few thousand threads; it depends on nothing but the

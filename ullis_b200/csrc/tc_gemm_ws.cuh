@@ -61,6 +61,7 @@ __device__ __forceinline__ bool ws_wait(uint64_t* bar, uint32_t parity, volatile
 template <int EPI, bool RESIDENT_W = true>
 __global__ void __launch_bounds__(WS_THREADS, 1)
 gemm_ws_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p, const uint32_t pairs) {
+    chain_entry();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const uint32_t KB = p.K / BK;
