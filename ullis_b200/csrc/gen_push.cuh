@@ -34,9 +34,66 @@ __device__ __forceinline__ uint32_t window(const uint32_t* words, uint32_t last,
     return __funnelshift_l(lo, hi, 31u - (p & 31u));
 }
 
+// Steps on which the histories that end at step i of the queries and at position r of the keys agree, from n on.
+__device__ __forceinline__ uint32_t agreement(const uint32_t* q, const uint32_t* k, uint32_t last, uint32_t q_word,
+                                              uint32_t k_word, uint32_t i, uint32_t r, uint32_t n) {
+    while (n <= r) {
+        const uint32_t same = (uint32_t)__clz((int)(window(q, last, q_word, i - n) ^ window(k, last, k_word, r - n)));
+        n += same;
+        if (same < 32u) break;
+    }
+    return min(n, r + 1u);
+}
+
+// The lag of step i by the whole warp where the last 32 query bits are equal (c); 0: fewer than 32 steps agree anywhere.
+// Streams that hardly ever change come here at almost every step, with whole windows of equal bits at most positions, so
+// these are not compared one by one but as runs: with n the run of c at step i, a position at the end of a shorter run of
+// c among the keys agrees on just that run, one with a longer run on n, and only one whose run is n long on more.  A lane
+// has a word; a run of 32 or more that ends in it covers its lowest bits, and the words before say how much goes before
+// them.  (64 sequences of the default model with nearly constant channels, position 2 000: 69 ms a step position by
+// position, by the runs of the keys 1.8 ms.)
+__device__ __forceinline__ uint32_t search_runs(const uint32_t* q, const uint32_t* k, uint32_t i, uint32_t wq, uint32_t k_word) {
+    const uint32_t lane = threadIdx.x & 31u, last = i >> 5, q_word = wq >> (31u - (i & 31u));
+    uint32_t n_run = (i & 31u) + 1u;
+    for (uint32_t w1 = last;; w1 -= 32u) {                       // words of c below w1
+        const uint32_t y = lane < w1 ? q[w1 - 1u - lane] ^ ~wq : 0u, full = __ballot_sync(0xFFFFFFFFu, y == ~0u);
+        if (full == ~0u) { n_run += 1024u; continue; }
+        const uint32_t l = (uint32_t)__ffs((int)~full) - 1u;
+        n_run += 32u * l + (uint32_t)__clz((int)~__shfl_sync(0xFFFFFFFFu, y, (int)l));
+        break;
+    }
+    uint32_t longest = 0, position = 0, before = 0;              // before: run of c that ends at the last word so far
+    for (uint32_t w0 = 0; w0 <= last; w0 += 32u) {
+        const uint32_t w = w0 + lane;
+        const uint32_t x = w < last ? k[w] ^ ~wq : w == last ? (k_word ^ ~wq) & ((1u << (i & 31u)) - 1u) : 0u;
+        const uint32_t full = __ballot_sync(0xFFFFFFFFu, x == ~0u), upper = (uint32_t)__clz((int)~x);
+        const uint32_t lower = x == ~0u ? 32u : (uint32_t)__ffs((int)~x) - 1u;
+        const uint32_t z = lane ? min((uint32_t)__clz((int)(~full << (32u - lane))), lane) : 0u;   // words of c right below
+        const uint32_t there = __shfl_sync(0xFFFFFFFFu, upper, (int)(z < lane ? lane - 1u - z : 0u));
+        const uint32_t carry = 32u * z + (z < lane ? there : before), run = carry + lower;
+        if (run >= 32u && lower) {
+            if (carry < n_run && n_run <= run) {
+                const uint32_t r = 32u * w + n_run - carry - 1u, n = agreement(q, k, last, q_word, k_word, i, r, n_run);
+                if (n >= longest) { longest = n; position = r; }
+            }
+            if (run != n_run && min(run, n_run) >= longest) { longest = min(run, n_run); position = 32u * w + lower - 1u; }
+        }
+        const uint32_t h = 31u - (uint32_t)__clz((int)~full);   // full == ~0: h = -1
+        const uint32_t top = __shfl_sync(0xFFFFFFFFu, upper, (int)(full == ~0u ? 0u : h));
+        before = full == ~0u ? before + 1024u : 32u * (31u - h) + top;
+    }
+    const uint32_t top = __reduce_max_sync(0xFFFFFFFFu, longest);
+    if (top < 32u) return 0u;
+    return i - __reduce_max_sync(0xFFFFFFFFu, longest == top ? position : 0u);
+}
+
 // The lag of step i for one stream, by the whole warp; wq: the query bits up to i, k_word: the keys before i.
 __device__ __forceinline__ uint32_t search(const uint32_t* q, const uint32_t* k, uint32_t i, uint32_t wq, uint32_t k_word) {
     const uint32_t lane = threadIdx.x & 31u, last = i >> 5, q_word = wq >> (31u - (i & 31u));
+    if (i >= 32u && (wq == 0u || wq == ~0u)) {
+        const uint32_t lag = search_runs(q, k, i, wq, k_word);
+        if (lag) return lag;
+    }
     uint32_t best = 0, before = 0;      // agreement << 26 | word of the position, the bit within the word is the lane
     for (uint32_t w0 = 0; w0 <= last; w0 += 32u) {
         const uint32_t mine = w0 + lane < last ? k[w0 + lane] : w0 + lane == last ? k_word : 0u;
@@ -60,22 +117,18 @@ __device__ __forceinline__ uint32_t search(const uint32_t* q, const uint32_t* k,
     uint32_t longest = 0, position = 0;
     for (uint32_t r = lane; r < i; r += 32u) {
         if (window(k, last, k_word, r) != wq) continue;
-        uint32_t n = 32u;
-        while (n <= r) {
-            const uint32_t same = (uint32_t)__clz((int)(window(q, last, q_word, i - n) ^ window(k, last, k_word, r - n)));
-            n += same;
-            if (same < 32u) break;
-        }
-        n = min(n, r + 1u);
+        const uint32_t n = agreement(q, k, last, q_word, k_word, i, r, 32u);
         if (n >= longest) { longest = n; position = r; }
     }
     const uint32_t top = __reduce_max_sync(0xFFFFFFFFu, longest);
     return i - __reduce_max_sync(0xFFFFFFFFu, longest == top ? position : 0u);
 }
 
-// The same for one stream per lane (open lanes only).  The position is found at once, so it has to fit 26 bits.
-__device__ __forceinline__ uint32_t search_alone(const uint32_t* q, const uint32_t* k, uint32_t i, uint32_t wq, uint32_t k_word) {
-    const uint32_t last = i >> 5, q_word = wq >> (31u - (i & 31u));
+// The same for one stream per lane (open lanes only); DEEP where whole windows agree, which is left to search().  The
+// position is found at once, so it has to fit 26 bits.
+constexpr uint32_t DEEP = ~0u;
+__device__ __forceinline__ uint32_t search_alone(const uint32_t* k, uint32_t i, uint32_t wq, uint32_t k_word) {
+    const uint32_t last = i >> 5;
     uint32_t best = 0, before = 0, next = last ? k[0] : k_word;
     for (uint32_t w = 0; w <= last; ++w) {
         const uint32_t word = next, n_bits = w == last ? i & 31u : 32u;
@@ -89,20 +142,7 @@ __device__ __forceinline__ uint32_t search_alone(const uint32_t* q, const uint32
         before = word;
     }
     const uint32_t most = best >> 26;
-    if (most < 32u) return most ? i - (best & 0x3FFFFFFu) : 0u;
-    uint32_t longest = 0, position = 0;
-    for (uint32_t r = 31u; r < i; ++r) {
-        if (window(k, last, k_word, r) != wq) continue;
-        uint32_t n = 32u;
-        while (n <= r) {
-            const uint32_t same = (uint32_t)__clz((int)(window(q, last, q_word, i - n) ^ window(k, last, k_word, r - n)));
-            n += same;
-            if (same < 32u) break;
-        }
-        n = min(n, r + 1u);
-        if (n >= longest) { longest = n; position = r; }
-    }
-    return i - position;
+    return most == 32u ? DEEP : most ? i - (best & 0x3FFFFFFu) : 0u;
 }
 
 // What step i of 32 streams (first + lane; a lane with live = false has none) can know before its bits: whether the lag of
@@ -137,9 +177,8 @@ __device__ __forceinline__ bool step(const Histories& H, size_t first, bool live
     uint32_t open = __ballot_sync(0xFFFFFFFFu, !known);
     // One after the other by the whole warp, or side by side with a lane each: by the instructions either takes.
     if ((uint32_t)__popc(open) * (6u * last + 150u) > 6u * i + 100u && i < (1u << 26)) {
-        if (!known) c.lag = search_alone(H.of(s, 0), H.of(s, 1), i, c.q, c.k);
-        __syncwarp();
-        open = 0u;
+        if (!known) c.lag = search_alone(H.of(s, 1), i, c.q, c.k);
+        open = __ballot_sync(0xFFFFFFFFu, !known && c.lag == DEEP);
     }
     while (open) {
         const int l = __ffs((int)open) - 1;
