@@ -484,8 +484,8 @@ def run_cuda(args):
         # dominant kernel = the one with the largest share of device time in the instrumented pass
         kernel_ms = {k: v for k, v in kernel_ms.items() if not k.startswith("(")}   # drop the between-steps bracket
         top = sorted(kernel_ms.items(), key=lambda kv: -kv[1][0])
-        # (on every supported shape that is one of the suffix-automaton kernels; should a GEMM
-        # ever lead, the line still reports the leading automaton kernel and names the leader)
+        # (usually one of the ROSA match kernels; should a GEMM lead, the line still reports the
+        # leading ROSA kernel and names the leader)
         leader = top[0][0]
         dominant, (dom_total, dom_launches) = next((kv for kv in top if kv[0].startswith("rosa_")), top[0])
         dom_ms = dom_total / max(dom_launches, 1)
@@ -503,7 +503,7 @@ def run_cuda(args):
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": n_warm, "ms_per_step": ms_total / args.steps, "higher_is_better": True,
             "scaling": args.scaling, "vs_baseline": None,
-            "dtype": "f32" if args.mode == "exact" else "fp16 tensor-core operands, f32 accumulate; u16 automaton state",
+            "dtype": "f32" if args.mode == "exact" else "fp16 tensor-core operands, f32 accumulate; packed bit streams",
             "data": "synthetic", "config": workload_config(args, shape, time_, world),
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(2 * rows * 4),
                     "d2h_bytes_per_step": 16 if world > 1 else 32},
@@ -669,8 +669,8 @@ def run_op_loop(args, rt, stream, torch):
         ms, launches = rt.kernel_times().get("gen_push", (0.0, 0))
         rt.kernel_timing(False)
         print(json.dumps({"workload": "pushers", "streams": n, "position": T - steps, "pushes_timed": steps,
-                          "gen_push_ms_per_push": ms / max(launches, 1), "launches": launches,
-                          "stream_pushes_per_s": n * launches / (ms * 1e-3) if ms else None,
+                          "gen_push_ms_per_push": ms / steps, "launches": launches,
+                          "stream_pushes_per_s": n * steps / (ms * 1e-3) if ms else None,
                           "ms_per_call_host_timed": dt * 1e3}))
         pushers.close()
     elif args.workload == "rosa":
