@@ -861,8 +861,8 @@ int32_t ullis_cuda_layer_norm_backward(ullis_cuda_runtime* rt, const float* inpu
             float* dgy = stage(rt, 1, output_gradient, n);
             uint16_t* dw = stage(rt, 2, weight, channels);
             float* dgx = rt->pool[3].as<float>(n);
-            float* dxh = rt->pool[4].as<float>(n);
-            k::layer_norm_backward(rt, dx, dgy, dw, dgx, dxh, dsmall, dsmall + channels, rows, channels, rt->pool[6]);
+            float2* stats = rt->pool[4].as<float2>(rows);
+            k::layer_norm_backward(rt, dx, dgy, dw, dgx, stats, dsmall, rows, channels, rt->pool[6]);
             rt->d2h(gx, dgx, n * 4);
         }
         rt->d2h(gw, dsmall, channels * 4);

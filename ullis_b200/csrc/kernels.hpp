@@ -82,7 +82,7 @@ void rosa_e_grad(ullis_cuda_runtime* rt, const float* gy, const uint8_t* idx, fl
 void relu2_backward(ullis_cuda_runtime* rt, const float* input, float* g, size_t n);
 // LayerNorm::backward (src/model.rs:270-315); xhat is scratch of the input's size.
 void layer_norm_backward(ullis_cuda_runtime* rt, const float* x, const float* gy, const uint16_t* w, float* gx,
-                         float* xhat, float* gw, float* gb, size_t rows, size_t channels, DeviceBuffer& scratch);
+                         float2* stats, float* gw_gb, size_t rows, size_t channels, ullis::DeviceBuffer& scratch);
 
 }  // namespace k
 }  // namespace ullis

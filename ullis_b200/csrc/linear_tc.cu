@@ -870,6 +870,7 @@ bool fp16_linear(ullis_cuda_runtime* rt, const float* x, const uint16_t* w, floa
 namespace {
 // y = sum of the split-K partials, in split order
 __global__ void splitk_reduce_kernel(const float* __restrict__ part, float* __restrict__ y, uint32_t splits, size_t n) {
+    chain_entry();
     const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (i >= n) return;   // n % 4 == 0 (N % 8 == 0)
     float4 acc = *reinterpret_cast<const float4*>(part + i);
@@ -905,7 +906,7 @@ bool dense_nt(ullis_cuda_runtime* rt, const uint16_t* a16, const uint16_t* b16, 
             rt->chain(gemm_kernel<EPI_STORE, false>, grid, GEMM_THREADS, gemm_smem_bytes(p.n_a, p.stages), maps, p);
             rt->launched("gemm_dense_nt_splitk");
             const size_t n = M * N;
-            splitk_reduce_kernel<<<blocks_for((n + 3) / 4, 256), 256, 0, rt->stream>>>(part, y, splits, n);
+            rt->chain(splitk_reduce_kernel, blocks_for((n + 3) / 4, 256), 256, 0, part, y, splits, n);
             rt->launched("splitk_reduce");
             return true;
         }
@@ -960,14 +961,16 @@ bool rosa_qkv_bits(ullis_cuda_runtime* rt, const float* ln3_out, const LayerWeig
         uint32_t* list = rt->tc_ws[9].as<uint32_t>(cap);
         uint32_t* ctrl = nullptr;
         rt->counters(rt->fix_counters, 2, &ctrl, &clear);
-        rt->chain(fix_collect_kernel, 4 * (unsigned)rt->sm_count, 256, 0, flags, sw, batch, d, wps, list, (uint32_t)cap, ctrl);
+        rt->chain(fix_collect_kernel, 4 * (unsigned)rt->sm_count, 256, 0, flags, sw, batch, d, wps, list,
+                  (uint32_t)cap, ctrl);
         rt->launched("fix_collect");
-        rt->chain(fix_apply_kernel, 12 * (unsigned)rt->sm_count, FIXQ_WARPS * 32, 0, ln3_out, L.x_q, L.x_k, L.x_v, L.q, L.k, L.v, q_sw, k_sw, v_sw, list, (uint32_t)cap, ctrl, sw, time, d, wps);
+        rt->chain(fix_apply_kernel, 12 * (unsigned)rt->sm_count, FIXQ_WARPS * 32, 0, ln3_out, L.x_q, L.x_k, L.x_v, L.q, L.k, L.v,
+                  q_sw, k_sw, v_sw, list, (uint32_t)cap, ctrl, sw, time, d, wps);
         rt->launched("fix_apply");
         only_if = ctrl + 1;
     }
-    rt->chain(sign_fixup_kernel, grid, FIX_THREADS, FIX_QUEUE * 4, ln3_out, L.x_q, L.x_k, L.x_v, L.q, L.k, L.v, q_sw, k_sw, v_sw, flags,
-                                                   flags + sw, flags + 2 * sw, batch, time, d, wps, only_if, clear);
+    rt->chain(sign_fixup_kernel, grid, FIX_THREADS, FIX_QUEUE * 4, ln3_out, L.x_q, L.x_k, L.x_v, L.q, L.k, L.v, q_sw, k_sw,
+              v_sw, flags, flags + sw, flags + 2 * sw, batch, time, d, wps, only_if, clear);
     rt->launched("sign_fixup");
     if (clear) rt->counters_cleared(rt->fix_counters);
     return true;

@@ -708,7 +708,8 @@ rosa_match_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restrict_
 
 struct MatchCall {   // the buffers of one call
     const uint32_t *q, *k, *v;
-    uint32_t *idx, *list, *cq_list, *hard, *clear, *counts;   // counts: listed, constant q, hard, next of the contexts, next of the matches
+    uint32_t *idx, *list, *cq_list, *hard;
+    uint32_t *counts, *clear;   // listed, constant q, hard, next of the contexts, next of the matches; those of the next call
     size_t streams, wps;
     uint32_t T;
 };
@@ -728,8 +729,8 @@ void launch_context(ullis_cuda_runtime* rt, const MatchCall& m, int slot) {
     // A match kernel step costs about as much as 100 positions here; up to 24 the lanes are even enough without sorting
     // the steps.  128 long comparisons per stream at most are thrown away when a stream turns out to repeat itself.
     const ContextLimits limits{24u, 96u, 160u, 256u};
-    rt->chain(rosa_context_kernel<NT>, grid, NT, smem, m.q, m.k, m.v, m.idx, m.list, m.counts, m.counts + 3, m.hard,
-                                                            m.counts + 2, m.T, m.wps, c, limits);
+    rt->chain(rosa_context_kernel<NT>, grid, NT, smem, m.q, m.k, m.v, m.idx, m.list, m.counts, m.counts + 3,
+              m.hard, m.counts + 2, m.T, m.wps, c, limits);
     rt->launched("rosa_context");
 }
 
@@ -746,8 +747,8 @@ void launch_match(ullis_cuda_runtime* rt, const MatchCall& m, int slot, uint32_t
     const size_t most = (m.streams * m.wps + MATCH_WARPS - 1) / MATCH_WARPS;   // every stream in the shortest pieces
     const unsigned grid = (unsigned)std::min<size_t>(rt->match_ctas[slot], most);
     uint32_t* kept = rt->sam_scratch.as<uint32_t>((size_t)grid * MATCH_WARPS * match::CHECKPOINTS * 32u * NW);
-    rt->chain(rosa_match_kernel<NW>, grid, 32 * MATCH_WARPS, smem, m.q, m.k, m.v, m.idx, m.hard, m.counts + 2, m.cq_list,
-                                                                        m.counts + 1, m.counts + 4, m.clear, kept, m.T, m.wps, ring_words);
+    rt->chain(rosa_match_kernel<NW>, grid, 32 * MATCH_WARPS, smem, m.q, m.k, m.v, m.idx, m.hard, m.counts + 2,
+              m.cq_list, m.counts + 1, m.counts + 4, m.clear, kept, m.T, m.wps, ring_words);
     rt->launched("rosa_match");
 }
 
@@ -779,7 +780,8 @@ void rosa_match(ullis_cuda_runtime* rt, const uint32_t* q_sw, const uint32_t* k_
     rt->sam_last_counts = m.counts;
     rt->sam_last_streams = streams;
     if (!rt->parent) rt->lanes_last = 1;
-    rt->chain(rosa_classify_kernel, (unsigned)((streams * CLASSIFY_LANES + 127) / 128), 128, 0, q_sw, k_sw, v_sw, idx_sw, streams, T, m.wps, m.list, m.counts, m.cq_list, m.counts + 1);
+    rt->chain(rosa_classify_kernel, (unsigned)((streams * CLASSIFY_LANES + 127) / 128), 128, 0, q_sw, k_sw, v_sw, idx_sw,
+              streams, T, m.wps, m.list, m.counts, m.cq_list, m.counts + 1);
     rt->launched("rosa_classify");
     // few streams: sixteen warps each, so that the last of them is done soon (one sequence of 512 channels: 0.20 ms
     // against 0.28 with eight); many: eight (1.79 ms for 32 768 streams against 1.98 with sixteen)

@@ -50,90 +50,87 @@ inline unsigned blocks_for(size_t n, unsigned per) { return (unsigned)((n + per 
 inline size_t pad64(size_t n) { return (n + 63) / 64 * 64; }
 
 // ------------------------------------------------------------ GEMM operands
-// the same for C == Cp, C % 4 == 0: four elements per thread
-__global__ void cast_rows4_kernel(const float* __restrict__ x, const uint16_t* __restrict__ colscale,
-                                  uint16_t* __restrict__ out, size_t R, size_t C, uint32_t* status) {
-    const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
-    if (i >= R * C) return;
-    const size_t r = i / C, c = i % C;
-    const float4 v = *reinterpret_cast<const float4*>(x + i);
-    float f[4] = {v.x, v.y, v.z, v.w};
-    if (colscale) {
-        const uint2 sw = *reinterpret_cast<const uint2*>(colscale + c);
-        f[0] = __fmul_rn(f[0], h2f((uint16_t)(sw.x & 0xFFFFu)));
-        f[1] = __fmul_rn(f[1], h2f((uint16_t)(sw.x >> 16)));
-        f[2] = __fmul_rn(f[2], h2f((uint16_t)(sw.y & 0xFFFFu)));
-        f[3] = __fmul_rn(f[3], h2f((uint16_t)(sw.y >> 16)));
-    }
-    const uint32_t lo = to_f16(f[0], status, r) | ((uint32_t)to_f16(f[1], status, r) << 16);
-    const uint32_t hi = to_f16(f[2], status, r) | ((uint32_t)to_f16(f[3], status, r) << 16);
-    *reinterpret_cast<uint2*>(out + i) = make_uint2(lo, hi);
-}
-
-// out [R, Cp] = FP16(x [R, C] * colscale[c]), columns C..Cp zero
-__global__ void cast_rows_kernel(const float* __restrict__ x, const uint16_t* __restrict__ colscale,
-                                 uint16_t* __restrict__ out, size_t R, size_t C, size_t Cp, uint32_t* status) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= R * Cp) return;
-    const size_t r = i / Cp, c = i % Cp;
-    float v = 0.0f;
-    if (c < C) {
-        v = x[r * C + c];
-        if (colscale) v = __fmul_rn(v, h2f(colscale[c]));
-    }
-    out[i] = to_f16(v, status, r);
-}
-
-// out [C, Rp] = FP16(op(x [R, C]))^T, columns R..Rp zero (Rp % 64 == 0).  op 1: relu(x)^2
-// A CTA moves 64 rows x 64 columns: 16-byte loads along a row, 16-byte stores of eight consecutive
-// rows of one column.
+// FP16 operands of the gradient products from x [R, C], both ways in one pass over it:
+//   rows_out [R, Cp] = FP16(x * colscale[c]), columns C..Cp zero (null: not wanted)
+//   t_out    [C, Rp] = FP16(x)^T, columns R..Rp zero
+// CMIX: x is g_relu2 and `key` the pre-activation; x becomes g_key = key > 0 ? 2 * key * x : 0 (relu2_bwd_on,
+// src/model.rs:1189-1204) first, and relu2_t [C, Rp] = FP16(relu(key)^2)^T leaves as well.
+// Bound by memory: a CTA moves 64 rows x 64 columns, 16-byte loads along a row, 16-byte stores of eight rows of a column.
+// As relu^2 backward, cast and two transposes one after the other the CMix part moved 1.0 GB per layer at 16 384 rows of
+// 2 048, in one pass 0.47 GB.
+template <bool CMIX>
 __global__ void __launch_bounds__(256)
-transpose_cast_kernel(const float* __restrict__ x, uint16_t* __restrict__ out, size_t R, size_t C, size_t Rp, int op,
-                      uint32_t* status) {
-    __shared__ float tile[64][65];
+operands_kernel(const float* __restrict__ x, const float* __restrict__ key, const uint16_t* __restrict__ colscale,
+                uint16_t* __restrict__ rows_out, uint16_t* __restrict__ t_out, uint16_t* __restrict__ relu2_t, size_t R,
+                size_t C, size_t Cp, size_t Rp, uint32_t* status) {
+    chain_entry();
+    __shared__ uint16_t tile[CMIX ? 2 : 1][64][66];
     const size_t r0 = (size_t)blockIdx.x * 64, c0 = (size_t)blockIdx.y * 64;
     const bool vec = (C & 3) == 0;
+    const auto load = [&](const float* from, size_t r, size_t c, float* v) {
+        if (vec && c + 3 < C) {
+            const float4 t = *reinterpret_cast<const float4*>(from + r * C + c);
+            v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+        } else {
+            for (int e = 0; e < 4; ++e) v[e] = c + e < C ? from[r * C + c + e] : 0.0f;
+        }
+    };
+    float v[4][4] = {}, kv[CMIX ? 4 : 1][4] = {};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {   // 64 rows x 16 groups of four columns
+        const size_t r = r0 + ((threadIdx.x + k * 256) >> 4), c = c0 + (threadIdx.x & 15) * 4;
+        if (r < R) load(x, r, c, v[k]);
+        if (CMIX && r < R) load(key, r, c, kv[CMIX ? k : 0]);
+    }
+    const int q = (threadIdx.x & 15) * 4;
+    float scale[4] = {1.0f, 1.0f, 1.0f, 1.0f};
+    if (rows_out && colscale)
+        for (int e = 0; e < 4; ++e) if (c0 + q + e < C) scale[e] = h2f(colscale[c0 + q + e]);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const int slot = threadIdx.x + k * 256;      // 64 rows x 16 groups of four columns
-        const int j = slot >> 4, q = (slot & 15) * 4;
-        const size_t r = r0 + j, c = c0 + q;
-        float v[4] = {0.f, 0.f, 0.f, 0.f};
-        if (r < R) {
-            if (vec && c + 3 < C) {
-                const float4 t = *reinterpret_cast<const float4*>(x + r * C + c);
-                v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
-            } else {
-                for (int e = 0; e < 4; ++e) if (c + e < C) v[e] = x[r * C + c + e];
-            }
-        }
+        const int j = (threadIdx.x + k * 256) >> 4;
+        uint16_t row[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            float t = v[e];
-            if (op == 1) { t = fmaxf(t, 0.0f); t *= t; }
-            tile[j][q + e] = t;
+            float t = v[k][e];
+            if (CMIX) {
+                const float y = kv[CMIX ? k : 0][e];
+                t = y > 0.0f ? 2.0f * y * t : 0.0f;
+                const float relu = fmaxf(y, 0.0f);
+                tile[CMIX ? 1 : 0][j][q + e] = to_f16(relu * relu, status, r0 + j);
+            }
+            tile[0][j][q + e] = to_f16(t, status, r0 + j);
+            row[e] = to_f16(colscale ? __fmul_rn(t, scale[e]) : t, status, r0 + j);
         }
+        if (rows_out && r0 + j < R)
+            *reinterpret_cast<uint2*>(rows_out + (r0 + j) * Cp + c0 + q) =
+                make_uint2(row[0] | (uint32_t)row[1] << 16, row[2] | (uint32_t)row[3] << 16);
     }
     __syncthreads();
     const int cl = threadIdx.x >> 2, seg = (threadIdx.x & 3) * 16;   // column, first of its sixteen rows
     const size_t c = c0 + cl;
     if (c >= C) return;
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        uint32_t w[4];
+    for (int which = 0; which < (CMIX ? 2 : 1); ++which) {
+        uint16_t* out = which ? relu2_t : t_out;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int j = seg + h * 8 + e * 2;
-            w[e] = (uint32_t)to_f16(tile[j][cl], status, r0 + j) | ((uint32_t)to_f16(tile[j + 1][cl], status, r0 + j + 1) << 16);
+        for (int h = 0; h < 2; ++h) {
+            uint32_t w[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int j = seg + h * 8 + e * 2;
+                w[e] = tile[which][j][cl] | (uint32_t)tile[which][j + 1][cl] << 16;
+            }
+            // r0 + seg + 8h + 7 < Rp: Rp is a multiple of 64
+            *reinterpret_cast<uint4*>(out + c * Rp + r0 + seg + h * 8) = make_uint4(w[0], w[1], w[2], w[3]);
         }
-        // r0 + seg + 8h + 7 < Rp: Rp is a multiple of 64
-        *reinterpret_cast<uint4*>(out + c * Rp + r0 + seg + h * 8) = make_uint4(w[0], w[1], w[2], w[3]);
     }
 }
 
 // packed signs [out, in] -> FP16 +/-1 [in, outp], columns out..outp zero
 __global__ void unpack_transpose_kernel(const uint32_t* __restrict__ bits, uint16_t* __restrict__ b16, size_t out_f,
                                         size_t in_f, size_t outp) {
+    chain_entry();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= in_f * outp) return;
     const size_t k = i / outp, o = i % outp;
@@ -145,13 +142,23 @@ __global__ void unpack_transpose_kernel(const uint32_t* __restrict__ bits, uint1
     b16[i] = v;
 }
 
-// w [R, C] FP16 -> [C, Rp], columns R..Rp zero
-__global__ void transpose16_kernel(const uint16_t* __restrict__ w, uint16_t* __restrict__ out, size_t R, size_t C,
-                                   size_t Rp) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= C * Rp) return;
-    const size_t c = i / Rp, r = i % Rp;
-    out[i] = r < R ? w[r * C + c] : (uint16_t)0;
+// w [R, C] FP16 -> [C, Rp], columns R..Rp zero; a CTA has 64 rows x 64 columns
+__global__ void __launch_bounds__(256)
+transpose16_kernel(const uint16_t* __restrict__ w, uint16_t* __restrict__ out, size_t R, size_t C, size_t Rp) {
+    chain_entry();
+    __shared__ uint16_t tile[64][66];
+    const size_t r0 = (size_t)blockIdx.x * 64, c0 = (size_t)blockIdx.y * 64;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+        const int j = (threadIdx.x >> 6) + k * 4, q = threadIdx.x & 63;
+        tile[j][q] = r0 + j < R && c0 + q < C ? w[(r0 + j) * C + c0 + q] : (uint16_t)0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+        const int j = threadIdx.x & 63, q = (threadIdx.x >> 6) + k * 4;
+        if (c0 + q < C) out[(c0 + q) * Rp + r0 + j] = tile[j][q];   // r0 + j < Rp: Rp is a multiple of 64
+    }
 }
 
 // y [M, N] = a [M, K] . b [N, K]^T, f32 accumulation of the same FP16 operands the
@@ -181,6 +188,7 @@ __global__ void __launch_bounds__(256)
 ce_grad_kernel(float* __restrict__ logits, const uint32_t* __restrict__ labels, uint32_t ignore_id, size_t rows,
                size_t time, size_t vocab, float loss_scale, float P, float* __restrict__ row_loss,
                uint32_t* status) {
+    chain_entry();
     __shared__ float red[8];
     __shared__ float bcast;
     const size_t m = blockIdx.x;
@@ -231,71 +239,202 @@ ce_grad_kernel(float* __restrict__ logits, const uint32_t* __restrict__ labels, 
 }
 
 // ------------------------------------------------------------ reductions over rows
-// part[chunk, c] = sum over the chunk's 256 rows of f(a, b); mode 0: a, 1: a*b (b f32), 2: a*(2*b-1) (b u8)
+// part[chunk, c] = sum over the chunk's 256 rows of f(a, b):
+//   COL_SUM    a
+//   COL_LN     a * (b - mean) / deviation, by the row's statistics, and a in a second part behind the first
+//   COL_SHIFT  a * (b of the row before - b), 0 before the first row of a sequence
+//   COL_SIGN   b ? a : -a                                   b u8 [R, C]
+//   COL_BITS   the same, b stream-major bits
+// The sum of a column is a serial chain, but its terms are not: a CTA of eight warps brings 128 rows of 32 columns to shared
+// memory, 16 rows per warp with all their loads in flight, and one warp adds them up, a column per lane.  As one thread per
+// column that also did the loads, one per addition, 16 384 rows of 512 took 44 us, with the loads of 64 rows ahead of
+// their additions 12 (COL_SUM) to 54; so 10 to 23.
+enum ColMode { COL_SUM, COL_LN, COL_SHIFT, COL_SIGN, COL_BITS };
+constexpr int COL_ROWS = 256, COL_STEP = 128, COL_WARP_ROWS = COL_STEP / 8;
+template <ColMode MODE>
 __global__ void __launch_bounds__(256)
-col_partial_kernel(const float* __restrict__ a, const void* __restrict__ b, float* __restrict__ part, size_t R,
-                   size_t C, int mode) {
-    const size_t c = (size_t)blockIdx.x * 256 + threadIdx.x;
-    if (c >= C) return;
-    const size_t r0 = (size_t)blockIdx.y * 256, r1 = min(r0 + 256, R);
+col_partial_kernel(const float* __restrict__ a, const void* __restrict__ b, const float2* __restrict__ stats,
+                   float* __restrict__ part, uint32_t R, uint32_t C, uint32_t time) {
+    chain_entry();
+    constexpr bool PRODUCT = MODE == COL_LN || MODE == COL_SHIFT;
+    __shared__ float sa[COL_STEP][32], sb[PRODUCT ? COL_STEP : 1][32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, c = blockIdx.x * 32u + lane;
+    const uint32_t r0 = blockIdx.y * COL_ROWS, r1 = min(r0 + COL_ROWS, R);
+    const float* b32 = static_cast<const float*>(b);
     float acc = 0.0f;
-    for (size_t r = r0; r < r1; ++r) {
-        const float av = a[r * C + c];
-        if (mode == 0) acc += av;
-        else if (mode == 1) acc += av * static_cast<const float*>(b)[r * C + c];
-        else acc += static_cast<const uint8_t*>(b)[r * C + c] ? av : -av;
+    for (uint32_t h = r0; h < r1; h += COL_STEP) {
+        const uint32_t rw = h + warp * COL_WARP_ROWS;
+        float av[COL_WARP_ROWS] = {}, bv[COL_WARP_ROWS] = {};
+        if (c < C) {
+            if (rw + COL_WARP_ROWS <= r1) {
+#pragma unroll
+                for (int i = 0; i < COL_WARP_ROWS; ++i) {
+                    av[i] = a[(size_t)(rw + i) * C + c];
+                    if (PRODUCT) bv[i] = b32[(size_t)(rw + i) * C + c];
+                    if (MODE == COL_SIGN) bv[i] = static_cast<const uint8_t*>(b)[(size_t)(rw + i) * C + c];
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < COL_WARP_ROWS; ++i)
+                    if (rw + i < r1) {
+                        av[i] = a[(size_t)(rw + i) * C + c];
+                        if (PRODUCT) bv[i] = b32[(size_t)(rw + i) * C + c];
+                        if (MODE == COL_SIGN) bv[i] = static_cast<const uint8_t*>(b)[(size_t)(rw + i) * C + c];
+                    }
+            }
+            if (MODE == COL_LN) {
+#pragma unroll
+                for (int i = 0; i < COL_WARP_ROWS; ++i)
+                    if (rw + i < r1) {
+                        const float2 st = stats[rw + i];
+                        bv[i] = (bv[i] - st.x) * st.y;
+                    }
+            }
+            if (MODE == COL_SHIFT && rw < r1) {
+                uint32_t t = rw % time;
+                float before = t ? b32[(size_t)(rw - 1) * C + c] : 0.0f;
+#pragma unroll
+                for (int i = 0; i < COL_WARP_ROWS; ++i) {
+                    const float now = bv[i];
+                    bv[i] = t ? __fsub_rn(before, now) : -now;
+                    before = now;
+                    t = t + 1 == time ? 0 : t + 1;
+                }
+            }
+            if (MODE == COL_BITS && rw < r1) {
+                const uint32_t wps = (time + 31u) / 32u;
+                uint32_t seq = rw / time, t = rw - seq * time, word = 0;
+                for (int i = 0; i < COL_WARP_ROWS; ++i) {
+                    if (i == 0 || (t & 31u) == 0u)
+                        word = rw + i < r1 ? static_cast<const uint32_t*>(b)[((size_t)seq * C + c) * wps + (t >> 5)] : 0u;
+                    bv[i] = (float)((word >> (t & 31u)) & 1u);
+                    if (++t == time) { t = 0; ++seq; }
+                }
+            }
+        }
+        if (h != r0) __syncthreads();                        // the rows before have been added up
+#pragma unroll
+        for (int i = 0; i < COL_WARP_ROWS; ++i) {
+            const bool negative = (MODE == COL_SIGN || MODE == COL_BITS) && bv[i] == 0.0f;
+            sa[warp * COL_WARP_ROWS + i][lane] = negative ? -av[i] : av[i];
+            if (PRODUCT) sb[PRODUCT ? warp * COL_WARP_ROWS + i : 0][lane] = bv[i];
+        }
+        __syncthreads();
+        const uint32_t n = min((uint32_t)COL_STEP, r1 - h);
+        if (warp == 0) {
+#pragma unroll 16
+            for (uint32_t j = 0; j < n; ++j) {
+                if (PRODUCT) acc += sa[j][lane] * sb[PRODUCT ? j : 0][lane];
+                else acc += sa[j][lane];
+            }
+        } else if (MODE == COL_LN && warp == 1) {
+#pragma unroll 16
+            for (uint32_t j = 0; j < n; ++j) acc += sa[j][lane];
+        }
     }
-    part[(size_t)blockIdx.y * C + c] = acc;
+    if (c < C && warp < (MODE == COL_LN ? 2u : 1u)) part[((size_t)warp * gridDim.y + blockIdx.y) * C + c] = acc;
 }
 
-__global__ void col_final_kernel(const float* __restrict__ part, float* __restrict__ out, size_t chunks, size_t C) {
-    const size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+// out[y, c] = sum over the chunks of part[y, chunk, c]
+__global__ void __launch_bounds__(64)
+col_final_kernel(const float* __restrict__ part, float* __restrict__ out, size_t chunks, size_t C) {
+    chain_entry();
+    const size_t c = (size_t)blockIdx.x * 64 + threadIdx.x;
     if (c >= C) return;
+    part += blockIdx.y * chunks * C + c;
     float acc = 0.0f;
-    for (size_t k = 0; k < chunks; ++k) acc += part[k * C + c];
-    out[c] = acc;
+    size_t k = 0;
+    for (; k + 16 <= chunks; k += 16) {
+        float v[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = part[(k + i) * C];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc += v[i];
+    }
+    for (; k < chunks; ++k) acc += part[k * C];
+    out[blockIdx.y * C + c] = acc;
 }
 
 // ------------------------------------------------------------ LayerNorm backward
-// gx (+)= d/dx, xhat out (for g_w = sum gy*xhat); one warp per row (src/model.rs:270-315)
+// gx (+)= d/dx, and the row's mean and 1 / deviation (for g_w = sum gy * xhat); one warp per row (src/model.rs:270-315).
+// N > 0: C = 32 * N, the row, its gradient and the old gx in registers (all loads in flight together, each read once); N = 0:
+// any C.  16 384 rows of 512 added to gx: 47 -> 20 us (an f32 row per column sum was written besides before).
+template <int N>
 __global__ void __launch_bounds__(256)
 ln_backward_kernel(const float* __restrict__ x, const float* __restrict__ gy, const uint16_t* __restrict__ w,
-                   float* __restrict__ gx, float* __restrict__ xhat_out, size_t rows, size_t C, int accumulate) {
+                   float* __restrict__ gx, float2* __restrict__ stats, size_t rows, size_t C, int accumulate) {
+    chain_entry();
     const int lane = threadIdx.x & 31;
     const size_t row = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (row >= rows) return;
     const float* xr = x + row * C;
     const float* gr = gy + row * C;
+    float xs[N ? N : 1], gs[N ? N : 1], old[N ? N : 1];
+    if constexpr (N > 0) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) xs[i] = xr[lane + 32 * i];
+#pragma unroll
+        for (int i = 0; i < N; ++i) gs[i] = gr[lane + 32 * i];
+#pragma unroll
+        for (int i = 0; i < N; ++i) old[i] = accumulate ? gx[row * C + lane + 32 * i] : 0.0f;
+    }
+    const auto each = [&](auto f) {   // f(column, x, gy)
+        if constexpr (N > 0) {
+#pragma unroll
+            for (int i = 0; i < N; ++i) f((size_t)(lane + 32 * i), xs[i], gs[i]);
+        } else {
+            for (size_t c = lane; c < C; c += 32) f(c, xr[c], gr[c]);
+        }
+    };
     float s = 0.0f;
-    for (size_t c = lane; c < C; c += 32) s += xr[c];
+    each([&](size_t, float xv, float) { s += xv; });
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     const float mean = s / (float)C;
     float v = 0.0f;
-    for (size_t c = lane; c < C; c += 32) { const float dlt = xr[c] - mean; v += dlt * dlt; }
+    each([&](size_t, float xv, float) { const float dlt = xv - mean; v += dlt * dlt; });
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     const float inv = 1.0f / sqrtf(v / (float)C + LN_EPS);
     float s1 = 0.0f, s2 = 0.0f;
-    for (size_t c = lane; c < C; c += 32) {
-        const float xh = (xr[c] - mean) * inv, dx = gr[c] * h2f(w[c]);
+    each([&](size_t c, float xv, float gv) {
+        const float xh = (xv - mean) * inv, dx = gv * h2f(w[c]);
         s1 += dx;
         s2 += dx * xh;
-    }
+    });
     for (int o = 16; o > 0; o >>= 1) {
         s1 += __shfl_xor_sync(0xffffffffu, s1, o);
         s2 += __shfl_xor_sync(0xffffffffu, s2, o);
     }
     const float inv_n = inv / (float)C;
-    for (size_t c = lane; c < C; c += 32) {
-        const float xh = (xr[c] - mean) * inv, dx = gr[c] * h2f(w[c]);
-        const float g = inv_n * ((float)C * dx - s1 - xh * s2);
-        xhat_out[row * C + c] = xh;
-        gx[row * C + c] = accumulate ? gx[row * C + c] + g : g;
+    if (lane == 0) stats[row] = make_float2(mean, inv);
+    if constexpr (N > 0) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const float xh = (xs[i] - mean) * inv, dx = gs[i] * h2f(w[lane + 32 * i]);
+            const float g = inv_n * ((float)C * dx - s1 - xh * s2);
+            gx[row * C + lane + 32 * i] = accumulate ? old[i] + g : g;
+        }
+    } else {
+        for (size_t c = lane; c < C; c += 32) {
+            const float xh = (xr[c] - mean) * inv, dx = gr[c] * h2f(w[c]);
+            const float g = inv_n * ((float)C * dx - s1 - xh * s2);
+            gx[row * C + c] = accumulate ? gx[row * C + c] + g : g;
+        }
     }
+}
+
+void ln_backward_launch(ullis_cuda_runtime* rt, const float* x, const float* gy, const uint16_t* w, float* gx, float2* stats,
+                        size_t rows, size_t C, int accumulate) {
+    const unsigned grid = blocks_for(rows, 8);
+    if (C == 256) rt->chain(ln_backward_kernel<8>, grid, 256, 0, x, gy, w, gx, stats, rows, C, accumulate);
+    else if (C == 512) rt->chain(ln_backward_kernel<16>, grid, 256, 0, x, gy, w, gx, stats, rows, C, accumulate);
+    else rt->chain(ln_backward_kernel<0>, grid, 256, 0, x, gy, w, gx, stats, rows, C, accumulate);
+    rt->launched("ln_backward");
 }
 
 // ------------------------------------------------------------ CMix pieces
 // g <- key > 0 ? 2*key*g : 0   (relu2_bwd_on, src/model.rs:1189-1204)
 __global__ void relu2_bwd_kernel(const float* __restrict__ key, float* __restrict__ g, size_t n) {
+    chain_entry();
     const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (i >= n) return;
     if (i + 4 <= n) {
@@ -311,16 +450,53 @@ __global__ void relu2_bwd_kernel(const float* __restrict__ key, float* __restric
     for (size_t j = i; j < n; ++j) g[j] = key[j] > 0.0f ? 2.0f * key[j] * g[j] : 0.0f;
 }
 
-// lerp_shift_backward (src/model.rs:1206-1240): out[t] = (g[t] - g[t]*mix) + g[t+1]*mix
+// lerp_shift_backward (src/model.rs:1206-1240): out[t] = (g[t] - g[t]*mix) + g[t+1]*mix.  Four columns per thread
+// (C % 4 == 0), or one.
+template <int N>
 __global__ void lerp_bwd_kernel(const float* __restrict__ g, const uint16_t* __restrict__ mix, float* __restrict__ out,
-                                size_t rows, size_t time, size_t C) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= rows * C) return;
-    const size_t row = i / C, c = i % C;
-    const float mv = h2f(mix[c]);
-    float v = __fsub_rn(g[i], __fmul_rn(g[i], mv));
-    if (row % time + 1 < time) v = __fadd_rn(v, __fmul_rn(g[i + C], mv));
-    out[i] = v;
+                                uint32_t rows, uint32_t time, uint32_t C) {
+    chain_entry();
+    const uint32_t per_row = C / N, i = blockIdx.x * blockDim.x + threadIdx.x, row = i / per_row;
+    if (row >= rows) return;
+    const uint32_t c = (i - row * per_row) * N;
+    const size_t at = (size_t)row * C + c;
+    const bool more = row % time + 1u < time;
+    float now[N], next[N], res[N];
+    if constexpr (N == 4) {
+        const float4 a = *reinterpret_cast<const float4*>(g + at), b = more ? *reinterpret_cast<const float4*>(g + at + C) : a;
+        now[0] = a.x; now[1] = a.y; now[2] = a.z; now[3] = a.w;
+        next[0] = b.x; next[1] = b.y; next[2] = b.z; next[3] = b.w;
+    } else {
+        now[0] = g[at];
+        next[0] = more ? g[at + C] : 0.0f;
+    }
+#pragma unroll
+    for (int e = 0; e < N; ++e) {
+        const float mv = h2f(mix[c + e]);
+        res[e] = __fsub_rn(now[e], __fmul_rn(now[e], mv));
+        if (more) res[e] = __fadd_rn(res[e], __fmul_rn(next[e], mv));
+    }
+    if constexpr (N == 4) *reinterpret_cast<float4*>(out + at) = make_float4(res[0], res[1], res[2], res[3]);
+    else out[at] = res[0];
+}
+
+// out [C, Rp] = FP16(+/-e)^T by the idx bits of stream-major words, rows R..Rp zero: the ROSA output (src/model.rs:1313) as
+// the operand of a weight gradient.  A thread has eight rows of a column; blockIdx.y is the column.
+__global__ void emit_transposed_kernel(const uint32_t* __restrict__ idx_sw, const uint16_t* __restrict__ e,
+                                       uint16_t* __restrict__ out, uint32_t R, uint32_t C, uint32_t Rp, uint32_t time) {
+    chain_entry();
+    const uint32_t r0 = (blockIdx.x * blockDim.x + threadIdx.x) * 8u, c = blockIdx.y, wps = (time + 31u) / 32u;
+    if (r0 >= Rp) return;
+    uint32_t seq = r0 / time, t = r0 - seq * time, h[8];
+    const uint32_t plus = e[c];
+#pragma unroll
+    for (uint32_t k = 0; k < 8u; ++k) {
+        h[k] = 0u;
+        if (r0 + k < R) h[k] = (idx_sw[((size_t)seq * C + c) * wps + (t >> 5)] >> (t & 31u)) & 1u ? plus : plus ^ 0x8000u;
+        if (++t == time) { t = 0u; ++seq; }
+    }
+    *reinterpret_cast<uint4*>(out + (size_t)c * Rp + r0) =
+        make_uint4(h[0] | h[1] << 16, h[2] | h[3] << 16, h[4] | h[5] << 16, h[6] | h[7] << 16);
 }
 
 // ------------------------------------------------------------ optimiser
@@ -334,47 +510,85 @@ __device__ __forceinline__ void clipped_step(uint16_t& w, float& residual, float
     w = rounded;
 }
 
-__global__ void clipped_sgd_kernel(uint16_t* __restrict__ w, float* __restrict__ residual, const float* __restrict__ g,
-                                   float gmul, float lr, size_t n) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    uint16_t wb = w[i];
-    float r = residual[i];
-    clipped_step(wb, r, __fmul_rn(g[i], gmul), lr);
-    w[i] = wb;
-    residual[i] = r;
+// A CTA has 1024 elements, four per thread, their loads in flight together.
+__global__ void __launch_bounds__(256)
+clipped_sgd_kernel(uint16_t* __restrict__ w, float* __restrict__ residual, const float* __restrict__ g, float gmul, float lr,
+                   size_t n) {
+    chain_entry();
+    const size_t i0 = (size_t)blockIdx.x * 1024 + threadIdx.x;
+    uint16_t wb[4];
+    float r[4], gv[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const size_t i = i0 + k * 256;
+        if (i < n) { wb[k] = w[i]; r[k] = residual[i]; gv[k] = g[i]; }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const size_t i = i0 + k * 256;
+        if (i >= n) break;
+        clipped_step(wb[k], r[k], __fmul_rn(gv[k], gmul), lr);
+        w[i] = wb[k];
+        residual[i] = r[k];
+    }
 }
 
 // Latent step of a packed matrix (apply_binaryconnect_sgd, src/precision.rs:124-134, on
 // g_w = scale[o] * G[o,i] * gmul * ste_scale), re-packing of the sign bits (rebinarize,
-// src/model.rs:878-884) and the count of bits that changed.  One warp per 32-bit word.
+// src/model.rs:878-884) and the count of bits that changed.  A warp has LATENT_WORDS words of 32 elements, their loads
+// in flight together; a CTA adds its count of changed bits once (an addition per word was up to 32 768 on one address:
+// 38 us for a matrix of 1 M elements).
+constexpr int LATENT_WORDS = 4;
 __global__ void __launch_bounds__(256)
 latent_sgd_kernel(uint16_t* __restrict__ latent, float* __restrict__ residual, const float* __restrict__ G,
                   const uint16_t* __restrict__ scale, uint32_t* __restrict__ bits, size_t out_f, size_t in_f,
                   float gmul, float ste_scale, float lr, unsigned long long* flips) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t n = out_f * in_f;
-    bool plus = false;
-    if (i < n) {
-        const float g = __fmul_rn(__fmul_rn(__fmul_rn(scale ? h2f(scale[i / in_f]) : 1.0f, G[i]), gmul), ste_scale);
-        uint16_t lb = latent[i];
-        if (g != 0.0f && fabsf(g) <= 3.4028234e38f) {
-            const float current = h2f(lb);
-            const float update = __fmul_rn(lr, fminf(fmaxf(g, -1.0f), 1.0f));
-            const float desired = fminf(fmaxf(__fadd_rn(__fsub_rn(current, update), residual[i]), -1.0f), 1.0f);
-            lb = __half_as_ushort(__float2half_rn(desired));
-            residual[i] = __fsub_rn(desired, h2f(lb));
-            latent[i] = lb;
+    chain_entry();
+    const int lane = threadIdx.x & 31;
+    const size_t n = out_f * in_f, i0 = ((size_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * (32 * LATENT_WORDS) + lane;
+    float g[LATENT_WORDS], carry[LATENT_WORDS];
+    uint16_t lb[LATENT_WORDS];
+    uint32_t old[LATENT_WORDS];
+#pragma unroll
+    for (int j = 0; j < LATENT_WORDS; ++j) {
+        const size_t i = i0 + 32 * j;
+        if (i < n) {
+            const size_t o = n >> 32 ? i / in_f : (uint32_t)i / (uint32_t)in_f;
+            g[j] = __fmul_rn(__fmul_rn(__fmul_rn(scale ? h2f(scale[o]) : 1.0f, G[i]), gmul), ste_scale);
+            lb[j] = latent[i];
+            carry[j] = residual[i];
+            old[j] = bits ? bits[i >> 5] : 0u;
         }
-        plus = h2f(lb) >= 0.0f;
     }
-    const uint32_t word = __ballot_sync(0xffffffffu, plus);
-    if (bits && (threadIdx.x & 31) == 0 && i < n) {
-        const uint32_t old = bits[i >> 5];
-        bits[i >> 5] = word;
-        const uint32_t diff = __popc(old ^ word);
-        if (diff && flips) atomicAdd(flips, (unsigned long long)diff);
+    uint32_t changed = 0;
+#pragma unroll
+    for (int j = 0; j < LATENT_WORDS; ++j) {
+        const size_t i = i0 + 32 * j;
+        bool plus = false;
+        if (i < n) {
+            if (g[j] != 0.0f && fabsf(g[j]) <= 3.4028234e38f) {
+                const float current = h2f(lb[j]);
+                const float update = __fmul_rn(lr, fminf(fmaxf(g[j], -1.0f), 1.0f));
+                const float desired = fminf(fmaxf(__fadd_rn(__fsub_rn(current, update), carry[j]), -1.0f), 1.0f);
+                lb[j] = __half_as_ushort(__float2half_rn(desired));
+                residual[i] = __fsub_rn(desired, h2f(lb[j]));
+                latent[i] = lb[j];
+            }
+            plus = h2f(lb[j]) >= 0.0f;
+        }
+        const uint32_t word = __ballot_sync(0xffffffffu, plus);
+        if (bits && lane == 0 && i < n) {
+            bits[i >> 5] = word;
+            changed += __popc(old[j] ^ word);
+        }
     }
+    if (!flips) return;
+    __shared__ uint32_t total;
+    if (threadIdx.x == 0) total = 0;
+    __syncthreads();
+    if (changed) atomicAdd(&total, changed);
+    __syncthreads();
+    if (threadIdx.x == 0 && total) atomicAdd(flips, (unsigned long long)total);
 }
 
 // g_scale[o] = sum_i sign[o,i] * G[o,i]   (g_scale of backward_ste, src/model.rs:784-790, with the
@@ -382,6 +596,7 @@ latent_sgd_kernel(uint16_t* __restrict__ latent, float* __restrict__ residual, c
 __global__ void __launch_bounds__(256)
 g_scale_kernel(const float* __restrict__ G, const uint32_t* __restrict__ bits, float* __restrict__ out, size_t out_f,
                size_t in_f) {
+    chain_entry();
     const int lane = threadIdx.x & 31;
     const size_t o = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (o >= out_f) return;
@@ -400,6 +615,7 @@ g_scale_kernel(const float* __restrict__ G, const uint32_t* __restrict__ bits, f
 __global__ void embed_sgd_kernel(uint16_t* __restrict__ emb, float* __restrict__ residual, const float* __restrict__ gx,
                                  const uint32_t* __restrict__ toks, const uint32_t* __restrict__ starts,
                                  const uint32_t* __restrict__ order, size_t d, float gmul, float lr) {
+    chain_entry();
     const uint32_t tok = toks[blockIdx.x], r0 = starts[blockIdx.x], r1 = starts[blockIdx.x + 1];
     const size_t c = (size_t)blockIdx.y * blockDim.x + threadIdx.x;
     if (c >= d) return;
@@ -423,14 +639,25 @@ __global__ void init_latent_kernel(const uint32_t* __restrict__ bits, uint16_t* 
     latent[i] = (bits[i >> 5] >> (i & 31)) & 1u ? LATENT_PLUS : (uint16_t)(LATENT_PLUS | 0x8000u);
 }
 
-void col_reduce_launch(ullis_cuda_runtime* rt, const float* a, const void* b, float* out, size_t R, size_t C, int mode,
-                       DeviceBuffer& scratch) {
-    const size_t chunks = (R + 255) / 256;
-    float* part = scratch.as<float>(chunks * C);
-    dim3 grid(blocks_for(C, 256), (unsigned)chunks);
-    col_partial_kernel<<<grid, 256, 0, rt->stream>>>(a, b, part, R, C, mode);
+// out [C] (COL_LN: two of them)
+void col_reduce_launch(ullis_cuda_runtime* rt, const float* a, const void* b, float* out, size_t R, size_t C, ColMode mode,
+                       DeviceBuffer& scratch, size_t time = 0, const float2* stats = nullptr) {
+    const size_t chunks = (R + COL_ROWS - 1) / COL_ROWS;
+    const unsigned outs = mode == COL_LN ? 2 : 1;
+    float* part = scratch.as<float>(outs * chunks * C);
+    const dim3 grid(blocks_for(C, 32), (unsigned)chunks);
+    const auto run = [&](auto kernel) {
+        rt->chain(kernel, grid, 256, 0, a, b, stats, part, (uint32_t)R, (uint32_t)C, (uint32_t)time);
+    };
+    switch (mode) {
+        case COL_SUM: run(col_partial_kernel<COL_SUM>); break;
+        case COL_LN: run(col_partial_kernel<COL_LN>); break;
+        case COL_SHIFT: run(col_partial_kernel<COL_SHIFT>); break;
+        case COL_SIGN: run(col_partial_kernel<COL_SIGN>); break;
+        case COL_BITS: run(col_partial_kernel<COL_BITS>); break;
+    }
     rt->launched("col_partial");
-    col_final_kernel<<<blocks_for(C, 256), 256, 0, rt->stream>>>(part, out, chunks, C);
+    rt->chain(col_final_kernel, dim3(blocks_for(C, 64), outs), 64, 0, part, out, chunks, C);
     rt->launched("col_final");
 }
 
@@ -447,38 +674,38 @@ struct Step {
         gemm_nt_plain_kernel<<<grid, block, 0, rt->stream>>>(a, b, y, M, K, N);
         rt->launched("gemm_nt_plain");
     }
-    void cast_rows(const float* x, const uint16_t* colscale, uint16_t* out, size_t R, size_t C, size_t Cp) {
-        if (C == Cp && C % 4 == 0 && (reinterpret_cast<uintptr_t>(colscale) & 7) == 0)
-            cast_rows4_kernel<<<blocks_for(R * C / 4, 256), 256, 0, rt->stream>>>(x, colscale, out, R, C, rt->dev_status);
-        else
-            cast_rows_kernel<<<blocks_for(R * Cp, 256), 256, 0, rt->stream>>>(x, colscale, out, R, C, Cp, rt->dev_status);
-        rt->launched("cast_rows");
+    // rows_out [R, pad64(C)] (or null) and t_out [C, Rp] of x [R, C]
+    void operands(const float* x, const uint16_t* colscale, uint16_t* rows_out, uint16_t* t_out, size_t R, size_t C, size_t Rp) {
+        const dim3 grid(blocks_for(Rp, 64), blocks_for(C, 64));
+        rt->chain(operands_kernel<false>, grid, 256, 0, x, nullptr, colscale, rows_out, t_out, nullptr, R, C, pad64(C), Rp,
+                  rt->dev_status);
+        rt->launched("operands");
     }
-    void transpose_cast(const float* x, uint16_t* out, size_t R, size_t C, size_t Rp, int op = 0) {
-        dim3 grid(blocks_for(Rp, 64), blocks_for(C, 64));
-        transpose_cast_kernel<<<grid, 256, 0, rt->stream>>>(x, out, R, C, Rp, op, rt->dev_status);
-        rt->launched("transpose_cast");
+    void operands_cmix(const float* g_relu2, const float* key, const uint16_t* colscale, uint16_t* rows_out, uint16_t* t_out,
+                       uint16_t* relu2_t, size_t R, size_t C, size_t Rp) {
+        const dim3 grid(blocks_for(Rp, 64), blocks_for(C, 64));
+        rt->chain(operands_kernel<true>, grid, 256, 0, g_relu2, key, colscale, rows_out, t_out, relu2_t, R, C, pad64(C), Rp,
+                  rt->dev_status);
+        rt->launched("operands_cmix");
     }
     void unpack_transpose(const uint32_t* bits, uint16_t* out, size_t out_f, size_t in_f, size_t outp) {
-        unpack_transpose_kernel<<<blocks_for(in_f * outp, 256), 256, 0, rt->stream>>>(bits, out, out_f, in_f, outp);
+        rt->chain(unpack_transpose_kernel, blocks_for(in_f * outp, 256), 256, 0, bits, out, out_f, in_f, outp);
         rt->launched("unpack_transpose");
     }
     // out[c] = sum_r f(a[r,c], b[r,c])
-    void col_reduce(const float* a, const void* b, float* out, size_t R, size_t C, int mode) {
-        col_reduce_launch(rt, a, b, out, R, C, mode, st->part);
+    void col_reduce(const float* a, const void* b, float* out, size_t R, size_t C, ColMode mode, size_t time = 0) {
+        col_reduce_launch(rt, a, b, out, R, C, mode, st->part, time);
     }
     void sgd(const Fp16Param& p, const float* g, float rate) {
-        clipped_sgd_kernel<<<blocks_for(p.n, 256), 256, 0, rt->stream>>>(p.w, p.residual, g, gmul, rate, p.n);
+        rt->chain(clipped_sgd_kernel, blocks_for(p.n, 1024), 256, 0, p.w, p.residual, g, gmul, rate, p.n);
         rt->launched("clipped_sgd");
     }
     // gx_out (+)= LN backward of (x, gy); steps the LayerNorm's weight and bias
     void ln_backward(const float* x, const float* gy, const Fp16Param& w, const Fp16Param& b, float* gx_out,
-                     bool accumulate, float* xhat, float* small, size_t rows, size_t d) {
-        ln_backward_kernel<<<blocks_for(rows, 8), 256, 0, rt->stream>>>(x, gy, w.w, gx_out, xhat, rows, d,
-                                                                       accumulate ? 1 : 0);
-        rt->launched("ln_backward");
-        col_reduce(gy, xhat, small, rows, d, 1);
-        col_reduce(gy, nullptr, small + d, rows, d, 0);
+                     bool accumulate, float* small, size_t rows, size_t d) {
+        float2* stats = st->ln_stats.as<float2>(rows);
+        ln_backward_launch(rt, x, gy, w.w, gx_out, stats, rows, d, accumulate ? 1 : 0);
+        col_reduce_launch(rt, gy, x, small, rows, d, COL_LN, st->part, 0, stats);   // g_weight, then g_bias
         sgd(w, small, lr);
         sgd(b, small + d, lr);
     }
@@ -489,10 +716,9 @@ struct Step {
         const size_t out_f = p.weights->out, in_f = p.weights->in;
         float* G = st->gmat.as<float>(out_f * in_f);
         gemm(gy16t, x16t, G, out_f, rows_p, in_f);
-        g_scale_kernel<<<blocks_for(out_f, 8), 256, 0, rt->stream>>>(G, p.weights->bits, small, out_f, in_f);
+        rt->chain(g_scale_kernel, blocks_for(out_f, 8), 256, 0, G, p.weights->bits, small, out_f, in_f);
         rt->launched("g_scale");
-        latent_sgd_kernel<<<blocks_for((out_f * in_f + 31) / 32 * 32, 256), 256, 0, rt->stream>>>(
-            p.latent, p.latent_residual, G, p.scale.w, const_cast<uint32_t*>(p.weights->bits), out_f, in_f, gmul, ste,
+        rt->chain(latent_sgd_kernel, blocks_for(out_f * in_f, 256 * LATENT_WORDS), 256, 0, p.latent, p.latent_residual, G, p.scale.w, const_cast<uint32_t*>(p.weights->bits), out_f, in_f, gmul, ste,
             lr, flips);
         rt->launched("latent_sgd");
         sgd(p.scale, small, lr);
@@ -507,33 +733,31 @@ namespace ullis {
 namespace k {
 
 void clipped_sgd(ullis_cuda_runtime* rt, uint16_t* w, float* residual, const float* g, float lr, size_t n) {
-    clipped_sgd_kernel<<<blocks_for(n, 256), 256, 0, rt->stream>>>(w, residual, g, 1.0f, lr, n);
+    rt->chain(clipped_sgd_kernel, blocks_for(n, 1024), 256, 0, w, residual, g, 1.0f, lr, n);
     rt->launched("clipped_sgd");
 }
 
 void latent_sgd(ullis_cuda_runtime* rt, uint16_t* latent, float* residual, const float* g, float lr, float ste_scale,
                 uint32_t* bits, size_t n) {
-    latent_sgd_kernel<<<blocks_for((n + 31) / 32 * 32, 256), 256, 0, rt->stream>>>(latent, residual, g, nullptr, bits, 1,
+    rt->chain(latent_sgd_kernel, blocks_for(n, 256 * LATENT_WORDS), 256, 0, latent, residual, g, nullptr, bits, 1,
                                                                                   n, 1.0f, ste_scale, lr, nullptr);
     rt->launched("latent_sgd");
 }
 
 void rosa_e_grad(ullis_cuda_runtime* rt, const float* gy, const uint8_t* idx, float* g_e, size_t rows, size_t channels,
                  DeviceBuffer& scratch) {
-    col_reduce_launch(rt, gy, idx, g_e, rows, channels, 2, scratch);
+    col_reduce_launch(rt, gy, idx, g_e, rows, channels, COL_SIGN, scratch);
 }
 
 void relu2_backward(ullis_cuda_runtime* rt, const float* input, float* g, size_t n) {
-    relu2_bwd_kernel<<<blocks_for((n + 3) / 4, 256), 256, 0, rt->stream>>>(input, g, n);
+    rt->chain(relu2_bwd_kernel, blocks_for((n + 3) / 4, 256), 256, 0, input, g, n);
     rt->launched("relu2_bwd");
 }
 
 void layer_norm_backward(ullis_cuda_runtime* rt, const float* x, const float* gy, const uint16_t* w, float* gx,
-                         float* xhat, float* gw, float* gb, size_t rows, size_t channels, DeviceBuffer& scratch) {
-    ln_backward_kernel<<<blocks_for(rows, 8), 256, 0, rt->stream>>>(x, gy, w, gx, xhat, rows, channels, 0);
-    rt->launched("ln_backward");
-    col_reduce_launch(rt, gy, xhat, gw, rows, channels, 1, scratch);
-    col_reduce_launch(rt, gy, nullptr, gb, rows, channels, 0, scratch);
+                         float2* stats, float* gw_gb, size_t rows, size_t channels, DeviceBuffer& scratch) {
+    ln_backward_launch(rt, x, gy, w, gx, stats, rows, channels, 0);
+    col_reduce_launch(rt, gy, x, gw_gb, rows, channels, COL_LN, scratch, 0, stats);
 }
 
 }  // namespace k
@@ -722,8 +946,9 @@ void ullis_cuda_train_state::step(const uint32_t* tokens, const uint32_t* labels
     float* W2 = wide2.as<float>(rows * f);
     float* LG = logits.as<float>(rows * vocab);
     const size_t widest = std::max({f_p, vocab_p, d_p});
-    uint16_t* A16 = a16.as<uint16_t>(std::max(rows * widest, std::max({f, vocab, d}) * rows_p));
-    uint16_t* B16 = b16.as<uint16_t>(std::max(std::max(f, d) * rows_p, widest * std::max(f, d)));
+    uint16_t* A16 = a16.as<uint16_t>(rows * widest);
+    uint16_t* B16 = b16.as<uint16_t>(std::max(d * rows_p, widest * std::max(f, d)));
+    uint16_t* T16 = t16.as<uint16_t>(std::max(vocab, d + 2 * f) * rows_p);
     float* SM = small.as<float>(4 * std::max({f, vocab, d}));
     unsigned long long* CNT = counters.as<unsigned long long>(3);
     const uint32_t* lab = m->labels.as<uint32_t>(rows);
@@ -731,27 +956,26 @@ void ullis_cuda_train_state::step(const uint32_t* tokens, const uint32_t* labels
     uint8_t* res = static_cast<uint8_t*>(m->result.ensure(16));
     rt->zero(CNT, 24);
     gmat.as<float>(std::max({d * f, vocab * d, d * d}));                        // sized once: no growth mid-step
-    part.as<float>((rows + 255) / 256 * std::max({f, vocab, d}));
+    part.as<float>((rows + 255) / 256 * std::max({f, vocab, 2 * d}));
 
     // ---- head: logits, loss, gy (src/model.rs:3204-3257)
     if (!tc::binary_linear(rt, H, m->head.bits, m->head.scale, m->head.bias, LG, rows, d, vocab))
         k::binary_linear_exact(rt, H, m->head.bits, m->head.scale, m->head.bias, LG, rows, d, vocab, false);
-    ce_grad_kernel<<<(unsigned)rows, 256, 0, rt->stream>>>(LG, lab, ignore_id, rows, time, vocab,
+    rt->chain(ce_grad_kernel, (unsigned)rows, 256, 0, LG, lab, ignore_id, rows, time, vocab,
                                                           1.0f / (float)(time - 1), P, RL, rt->dev_status);
     rt->launched("ce_grad");
     k::ce_reduce(rt, RL, lab, ignore_id, rows, time, reinterpret_cast<double*>(res),
                  reinterpret_cast<unsigned long long*>(res + 8));
     m->have_result = true;
-    s.col_reduce(LG, nullptr, SM + 2 * vocab, rows, vocab, 0);                      // g_bias
-    s.cast_rows(LG, m->head.scale, A16, rows, vocab, vocab_p);                      // (gy*scale) [rows, V]
+    s.col_reduce(LG, nullptr, SM + 2 * vocab, rows, vocab, COL_SUM);                // g_bias
+    s.operands(LG, m->head.scale, A16, T16, rows, vocab, rows_p);                   // (gy*scale) [rows, V], gy^T [V, rows]
     s.unpack_transpose(m->head.bits, B16, vocab, d, vocab_p);                       // S^T [d, V]
     s.gemm(A16, B16, GX, rows, vocab_p, d);                                         // g_hidden
-    s.transpose_cast(LG, A16, rows, vocab, rows_p);                                 // gy^T [V, rows]
-    s.transpose_cast(H, B16, rows, d, rows_p);                                      // hidden^T [d, rows]
-    s.packed_update(head, A16, B16, rows_p, SM + 2 * vocab, learning_rate * HEAD_BIAS_LR_MULT, CNT + 0, SM);
+    s.operands(H, nullptr, nullptr, B16, rows, d, rows_p);                          // hidden^T [d, rows]
+    s.packed_update(head, T16, B16, rows_p, SM + 2 * vocab, learning_rate * HEAD_BIAS_LR_MULT, CNT + 0, SM);
 
     // ---- ln_out
-    s.ln_backward(X, GX, ln_out_w, ln_out_b, T1, false, T2, SM, rows, d);
+    s.ln_backward(X, GX, ln_out_w, ln_out_b, T1, false, SM, rows, d);
     std::swap(GX, T1);
 
     for (size_t li = m->layers; li-- > 0;) {
@@ -764,58 +988,54 @@ void ullis_cuda_train_state::step(const uint32_t* tokens, const uint32_t* labels
         if (!tc::binary_linear(rt, T2, L.key.bits, L.key.scale, nullptr, W1, rows, d, f))
             k::binary_linear_exact(rt, T2, L.key.bits, L.key.scale, nullptr, W1, rows, d, f, false);  // key
         // value: g_relu2 = gy . W (before W is stepped), g_W = gy^T . relu2 (src/model.rs:1138-1140)
-        s.cast_rows(GX, nullptr, A16, rows, d, d_p);
-        {
-            uint16_t* wt = B16;
-            transpose16_kernel<<<blocks_for(f * d_p, 256), 256, 0, rt->stream>>>(L.value, wt, d, f, d_p);
-            rt->launched("transpose16");
-            s.gemm(A16, wt, W2, rows, d_p, f);                                                        // g_relu2
-        }
-        s.transpose_cast(GX, A16, rows, d, rows_p);                                                   // gy^T
-        s.transpose_cast(W1, B16, rows, f, rows_p, 1);                                                // relu2^T
+        uint16_t *key_t = T16 + d * rows_p, *relu2_t = key_t + f * rows_p;
+        s.operands(GX, nullptr, A16, T16, rows, d, rows_p);                                           // gy, gy^T
+        rt->chain(transpose16_kernel, dim3(blocks_for(d_p, 64), blocks_for(f, 64)), 256, 0, L.value, B16, d, f, d_p);
+        rt->launched("transpose16");
+        s.gemm(A16, B16, W2, rows, d_p, f);                                                           // g_relu2
+        s.operands_cmix(W2, W1, L.key.scale, A16, key_t, relu2_t, rows, f, rows_p);
         {
             float* G = gmat.as<float>(d * f);
-            s.gemm(A16, B16, G, d, rows_p, f);
+            s.gemm(T16, relu2_t, G, d, rows_p, f);
             s.sgd(T.value, G, learning_rate);
         }
-        relu2_bwd_kernel<<<blocks_for((rows * f + 3) / 4, 256), 256, 0, rt->stream>>>(W1, W2, rows * f);        // g_key
-        rt->launched("relu2_bwd");
         // key (src/model.rs:1141-1163)
-        s.cast_rows(W2, L.key.scale, A16, rows, f, f_p);
         s.unpack_transpose(L.key.bits, B16, f, d, f_p);
         s.gemm(A16, B16, T3, rows, f_p, d);                                                           // g_shifted
-        s.transpose_cast(W2, A16, rows, f, rows_p);
-        s.transpose_cast(T2, B16, rows, d, rows_p);
-        s.packed_update(T.key, A16, B16, rows_p, nullptr, 0.0f, CNT + 1, SM);
+        s.operands(T2, nullptr, nullptr, B16, rows, d, rows_p);
+        s.packed_update(T.key, key_t, B16, rows_p, nullptr, 0.0f, CNT + 1, SM);
         // time-shift mix (src/model.rs:1164-1176)
-        k::time_shift_delta(rt, T1, T2, rows, time, d);                                               // xx
-        s.col_reduce(T3, T2, SM, rows, d, 1);                                                         // g_mix
-        lerp_bwd_kernel<<<blocks_for(n, 256), 256, 0, rt->stream>>>(T3, L.ffn_x_k, T1, rows, time, d);
+        s.col_reduce(T3, T1, SM, rows, d, COL_SHIFT, time);                                                     // g_mix
+        if (d % 4 == 0)
+            rt->chain(lerp_bwd_kernel<4>, blocks_for(n / 4, 256), 256, 0, T3, L.ffn_x_k, T1, (uint32_t)rows, (uint32_t)time,
+                      (uint32_t)d);
+        else
+            rt->chain(lerp_bwd_kernel<1>, blocks_for(n, 256), 256, 0, T3, L.ffn_x_k, T1, (uint32_t)rows, (uint32_t)time, (uint32_t)d);
         rt->launched("lerp_bwd");
         s.sgd(T.x_k, SM, learning_rate);                                                              // after its last use
-        s.ln_backward(AR, T1, T.ln2_w, T.ln2_b, GX, true, T2, SM, rows, d);
+        s.ln_backward(AR, T1, T.ln2_w, T.ln2_b, GX, true, SM, rows, d);
 
         // ---- ROSA: gradients stop at the q/k/v bits (src/model.rs:1494-1521)
-        uint8_t* IDX = reinterpret_cast<uint8_t*>(T3);
-        k::rosa_emit(rt, m->tape_idx[li].as<uint32_t>(1), L.e, IDX, T1, batch, time, d);               // idx, y = +/-e
-        s.col_reduce(GX, nullptr, SM + 2 * d, rows, d, 0);                                            // g_bias
-        s.cast_rows(GX, L.o.scale, A16, rows, d, d_p);
+        const uint32_t* idx = m->tape_idx[li].as<uint32_t>(1);
+        s.col_reduce(GX, nullptr, SM + 2 * d, rows, d, COL_SUM);                                      // g_bias
+        s.operands(GX, L.o.scale, A16, T16, rows, d, rows_p);
         s.unpack_transpose(L.o.bits, B16, d, d, d_p);
         s.gemm(A16, B16, T2, rows, d_p, d);                                                           // g_y
-        s.col_reduce(T2, IDX, SM + 3 * d, rows, d, 2);                                                // g_e
-        s.transpose_cast(GX, A16, rows, d, rows_p);
-        s.transpose_cast(T1, B16, rows, d, rows_p);
-        s.packed_update(T.o, A16, B16, rows_p, SM + 2 * d, learning_rate, CNT + 2, SM);
+        s.col_reduce(T2, idx, SM + 3 * d, rows, d, COL_BITS, time);                                   // g_e
+        rt->chain(emit_transposed_kernel, dim3(blocks_for(rows_p, 8 * 128), (unsigned)d), 128, 0, idx, L.e, B16, (uint32_t)rows,
+                  (uint32_t)d, (uint32_t)rows_p, (uint32_t)time);                                      // y = +/-e
+        rt->launched("emit_transposed");
+        s.packed_update(T.o, T16, B16, rows_p, SM + 2 * d, learning_rate, CNT + 2, SM);
         s.sgd(T.e, SM + 3 * d, learning_rate);
 
         if (li == 0) {   // ln0 replaced x on layer 0: its input is the embedded rows (src/model.rs:2972-2977)
             k::embed(rt, m->ids.as<uint32_t>(rows), m->embedding, T1, rows, d, vocab);
-            s.ln_backward(T1, GX, T.ln0_w, T.ln0_b, T2, false, T3, SM, rows, d);
+            s.ln_backward(T1, GX, T.ln0_w, T.ln0_b, T2, false, SM, rows, d);
             std::swap(GX, T2);
         }
     }
     // ---- embedding rows (src/model.rs:2980-2987)
-    embed_sgd_kernel<<<dim3((unsigned)h_toks.size(), blocks_for(d, 128)), 128, 0, rt->stream>>>(embedding.w, embedding.residual, GX,
+    rt->chain(embed_sgd_kernel, dim3((unsigned)h_toks.size(), blocks_for(d, 128)), 128, 0, embedding.w, embedding.residual, GX,
                                                                       toks.as<uint32_t>(1), starts.as<uint32_t>(1),
                                                                       order.as<uint32_t>(1), d, s.gmul, learning_rate);
     rt->launched("embed_sgd");

@@ -42,7 +42,7 @@ struct ullis_cuda_train_state {
     std::map<std::string, Named> named;   // every tensor a caller may read back, by checkpoint name
 
     // step scratch (grow-only)
-    ullis::DeviceBuffer gx, t1, t2, t3, wide1, wide2, logits, a16, b16, gmat, part, small, counters, order, starts,
+    ullis::DeviceBuffer gx, t1, t2, t3, wide1, wide2, logits, a16, b16, t16, gmat, part, ln_stats, small, counters, order, starts,
         toks;
     uint64_t steps = 0;
 
