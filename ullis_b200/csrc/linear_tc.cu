@@ -631,7 +631,7 @@ bool usable(ullis_cuda_runtime* rt) {
         rt->tc_ready = -1;
         if (rt->cc_major == 10 && !getenv("ULLIS_CUDA_NO_TC")) {
             encode_fn();
-            const int smem = (int)gemm_smem_bytes(2, MAX_STAGES);
+            const int smem = (int)WS_SMEM_LIMIT;
 #define ULLIS_SET_SMEM(EPI, PACKED) \
     ULLIS_CUDA_CHECK(cudaFuncSetAttribute(gemm_kernel<EPI, PACKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem))
             ULLIS_SET_SMEM(EPI_STORE, true);
@@ -704,7 +704,7 @@ void launch_ws2(ullis_cuda_runtime* rt, const GemmMaps& maps, const GemmParams& 
     const WsShape shape = ws2_shape(p.K, p.n_a, EPI, RESIDENT_W);
     GemmParams q = p;
     q.stages = shape.stages;
-    const uint32_t pairs = n_prob * (p.N / WS2_BN), m_tiles = (p.M + WS2_BM - 1) / WS2_BM;
+    const uint32_t pairs = n_prob * (p.N / WS2_BN) * std::max(p.split_k, 1u), m_tiles = (p.M + WS2_BM - 1) / WS2_BM;
     uint32_t members = (uint32_t)resident / pairs;
     if (members < 1) members = 1;
     if (members > m_tiles) members = m_tiles;
@@ -726,6 +726,27 @@ void launch_ws2(ullis_cuda_runtime* rt, const GemmMaps& maps, const GemmParams& 
     if (rt->kernel_timing) rt->mark("(cta_pair)");   // a zero-length entry in the timing table: which form ran
     ULLIS_CUDA_CHECK(cudaLaunchKernelEx(&cfg, gemm_ws2_kernel<EPI, RESIDENT_W>, maps, q, pairs));
     rt->launched(what);
+}
+
+// Pipeline depth of gemm_kernel: shallow where three CTAs share an SM (one's epilogue runs under another's MMAs), as deep as
+// the shared memory of one or two CTAs allows where the grid leaves no more than that to an SM: a CTA by itself with two
+// stages waits for memory at every k-block (K = 2 048, 2 048 rows of 512: 28 -> 25 us).
+uint32_t stages_for(const ullis_cuda_runtime* rt, const GemmParams& p, size_t ctas) {
+    const size_t per_sm = (ctas + rt->sm_count - 1) / rt->sm_count;
+    if (per_sm > 2) return p.stages;
+    const size_t room = WS_SMEM_LIMIT / per_sm - 1024 * (per_sm - 1), fixed = gemm_smem_bytes(p.n_a, 0);
+    const uint32_t fit = (uint32_t)((room - fixed) / ((p.n_a + 1) * TILE_BYTES));
+    return std::max(p.stages, std::min({fit, (uint32_t)MAX_STAGES, p.K / BK}));
+}
+
+// Whether the pair kernel takes dense weights.  It needs half of the pairs at work, or the smaller tiles of gemm_kernel
+// spread the rows better (K = 2 048, 16 384 rows of 512, 128 tiles on 74 pairs: 65 -> 43 us; 7 680 rows, 60: 34 -> 31).
+template <int EPI>
+bool takes_ws2_dense(const ullis_cuda_runtime* rt, const GemmParams& p, unsigned n_prob) {
+    const size_t tiles = (size_t)n_prob * ((p.M + WS2_BM - 1) / WS2_BM) * (p.N / WS2_BN);
+    return rt->tc_ws2_kernel && p.N % WS2_BN == 0 && rt->tc_ws2_dense_clusters[EPI] >= 8 &&
+           2 * tiles * std::max(p.split_k, 1u) >= (size_t)rt->tc_ws2_dense_clusters[EPI] &&
+           ws2_shape(p.K, p.n_a, EPI, false).stages >= 2;
 }
 
 template <int EPI, bool PACKED>
@@ -753,9 +774,7 @@ void launch(ullis_cuda_runtime* rt, const GemmMaps& maps, const GemmParams& p, u
         // dense weights: the persistent kernel with the weight tile in the ring (large M only: a CTA needs
         // several row tiles to amortise its set-up)
         const uint32_t m_tiles = (p.M + BM - 1) / BM, pairs = n_prob * ((p.N + BN - 1) / BN);
-        if (rt->tc_ws2_kernel && m_tiles * pairs >= 4u * (uint32_t)rt->sm_count && p.N % WS2_BN == 0 &&
-            p.M >= rt->tc_ws2_min_rows && rt->tc_ws2_dense_clusters[EPI] >= 8 &&
-            ws2_shape(p.K, p.n_a, EPI, false).stages >= 2) {
+        if (p.M >= rt->tc_ws2_min_rows && takes_ws2_dense<EPI>(rt, p, n_prob)) {
             launch_ws2<EPI, false>(rt, maps, p, n_prob, rt->tc_ws2_dense_clusters[EPI], what);
             return;
         }
@@ -772,7 +791,9 @@ void launch(ullis_cuda_runtime* rt, const GemmMaps& maps, const GemmParams& p, u
         }
     }
     dim3 grid((p.N + BN - 1) / BN, (p.M + BM - 1) / BM, n_prob);
-    rt->chain(gemm_kernel<EPI, PACKED>, grid, GEMM_THREADS, gemm_smem_bytes(p.n_a, p.stages), maps, p);
+    GemmParams q = p;
+    q.stages = stages_for(rt, p, (size_t)grid.x * grid.y * grid.z);
+    rt->chain(gemm_kernel<EPI, PACKED>, grid, GEMM_THREADS, gemm_smem_bytes(q.n_a, q.stages), maps, q);
     rt->launched(what);
 }
 
@@ -891,8 +912,29 @@ bool dense_nt(ullis_cuda_runtime* rt, const uint16_t* a16, const uint16_t* b16, 
     maps.b[0] = make_map(b16, N, K, false);
     GemmParams p = base_params(rt, M, N, K);
     p.prob[0] = GemmProblem{nullptr, nullptr, nullptr, y, nullptr, nullptr};
-    // A long K under a few output tiles (a weight gradient: K = rows of the batch) is split over
-    // blockIdx.z so that the whole GPU works on it; the partials are then summed in split order.
+    // A long K under a few output tiles (a weight gradient: K = rows of the batch) is split so that the whole GPU works on
+    // it; the partials are then summed in split order.  By CTA pairs where the columns allow (512 x 2 048 of 16 384 rows:
+    // 48 -> 37 us).
+    const auto reduce = [&](float* part, uint32_t splits) {
+        const size_t n = M * N;
+        rt->chain(splitk_reduce_kernel, blocks_for((n + 3) / 4, 256), 256, 0, part, y, splits, n);
+        rt->launched("splitk_reduce");
+    };
+    if (N % WS2_BN == 0 && K / BK >= 32) {
+        const uint32_t pair_tiles = (uint32_t)((M + WS2_BM - 1) / WS2_BM * (N / WS2_BN)), blocks = (uint32_t)(K / BK);
+        uint32_t want = std::min((uint32_t)rt->tc_ws2_dense_clusters[EPI_STORE] / pair_tiles, blocks / 8);
+        const uint32_t per = want > 1 ? (blocks + want - 1) / want : blocks, splits = (blocks + per - 1) / per;
+        GemmParams q = p;
+        q.split_k = splits > 1 ? splits : 0;
+        if (takes_ws2_dense<EPI_STORE>(rt, q, 1)) {
+            float* part = splits > 1 ? rt->tc_ws[8].as<float>((size_t)splits * M * N) : y;
+            q.prob[0].out = part;
+            launch_ws2<EPI_STORE, false>(rt, maps, q, 1, rt->tc_ws2_dense_clusters[EPI_STORE],
+                                         splits > 1 ? "gemm_dense_nt_splitk" : "gemm_dense_nt");
+            if (splits > 1) reduce(part, splits);
+            return true;
+        }
+    }
     const uint32_t tiles = (uint32_t)(((M + BM - 1) / BM) * ((N + BN - 1) / BN)), kb = (uint32_t)(K / BK);
     if (tiles < (uint32_t)rt->sm_count && kb >= 32) {
         uint32_t want = (2u * (uint32_t)rt->sm_count + tiles - 1) / tiles;
@@ -905,9 +947,7 @@ bool dense_nt(ullis_cuda_runtime* rt, const uint16_t* a16, const uint16_t* b16, 
             dim3 grid((unsigned)((N + BN - 1) / BN), (unsigned)((M + BM - 1) / BM), splits);
             rt->chain(gemm_kernel<EPI_STORE, false>, grid, GEMM_THREADS, gemm_smem_bytes(p.n_a, p.stages), maps, p);
             rt->launched("gemm_dense_nt_splitk");
-            const size_t n = M * N;
-            rt->chain(splitk_reduce_kernel, blocks_for((n + 3) / 4, 256), 256, 0, part, y, splits, n);
-            rt->launched("splitk_reduce");
+            reduce(part, splits);
             return true;
         }
     }

@@ -35,7 +35,7 @@ namespace tc {
 
 enum { EPI_STORE = 0, EPI_RESIDUAL = 1, EPI_RELU2 = 2, EPI_SIGNBITS = 3, EPI_CE = 4 };
 
-constexpr int BM = 128, BN = 128, BK = 64, MAX_STAGES = 4;
+constexpr int BM = 128, BN = 128, BK = 64, MAX_STAGES = 6;
 constexpr int TILE_BYTES = BM * BK * 2;  // 16 KiB, also the B tile (BN == BM)
 constexpr int GEMM_THREADS = 192;
 constexpr int STAGE_STRIDE = 20;                         // floats per row of an epilogue warp's 32 x 16 transposition buffer
@@ -67,7 +67,7 @@ struct GemmParams {
     const uint32_t* labels;  // EPI_CE
     uint32_t ignore_id;      // EPI_CE
     uint32_t n_tiles;        // EPI_CE: (max, sum exp) partials per row: one per vocabulary tile and epilogue warp group
-    uint32_t split_k;        // > 1 (gemm_kernel, one problem): blockIdx.z owns a K range and writes its own [M,N] partial
+    uint32_t split_k;        // > 1 (dense weights, one problem): a share of the grid owns a K range and writes its own [M,N] partial
     uint32_t* status;
 };
 

@@ -42,14 +42,15 @@ inline WsShape ws2_shape(uint32_t K, uint32_t n_a, int epi, bool resident_w = tr
 }
 
 // RESIDENT_W = false: dense 16-bit weights of any K; each CTA fetches the 128 weight rows of its half of the
-// pair's 256 columns by TMA into the same ring stage as its activations (nothing stays resident).
+// pair's 256 columns by TMA into the same ring stage as its activations (nothing stays resident).  With split_k a pair
+// owns one range of K as well (counted in `pairs`).
 template <int EPI, bool RESIDENT_W = true>
 __global__ void __launch_bounds__(WS2_THREADS, 1)
 gemm_ws2_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p, const uint32_t pairs) {
     chain_entry();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const uint32_t KB = p.K / BK;
+    uint32_t KB = p.K / BK, kb0 = 0;
     const uint32_t STAGES = p.stages;
     const uint32_t stage_bytes = (p.n_a + (RESIDENT_W ? 0u : 1u)) * TILE_BYTES;
     uint8_t* w_tiles = smem;                               // [KB] this CTA's 128 weight rows
@@ -74,11 +75,18 @@ gemm_ws2_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p, const
     const uint32_t owner = cluster % pairs, member = cluster / pairs;
     const uint32_t members = (clusters - owner + pairs - 1) / pairs;
     const uint32_t n_tiles = (p.N + WS2_BN - 1) / WS2_BN;
-    const uint32_t z = owner / n_tiles, n_tile = owner % n_tiles;
+    const uint32_t per_split = !RESIDENT_W && p.split_k > 1 ? pairs / p.split_k : pairs;
+    const uint32_t z = owner % per_split / n_tiles, n_tile = owner % n_tiles;   // n_tiles divides per_split
     const uint32_t n0 = n_tile * WS2_BN;
     const uint32_t m_tiles = (p.M + WS2_BM - 1) / WS2_BM;
     const uint32_t my_tiles = member < m_tiles ? (m_tiles - member + members - 1) / members : 0;
-    const GemmProblem& pr = p.prob[z];
+    GemmProblem pr = p.prob[z];
+    if (!RESIDENT_W && p.split_k > 1) {   // the host leaves every split at least one k-block
+        const uint32_t per = (KB + p.split_k - 1) / p.split_k, split = owner / per_split;
+        kb0 = split * per;
+        KB = min(per, KB - kb0);
+        pr.out = static_cast<float*>(pr.out) + (size_t)split * p.M * p.N;
+    }
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < STAGES; ++s) {
@@ -156,12 +164,12 @@ gemm_ws2_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p, const
                     }
                     uint8_t* st = a_ring + s * stage_bytes;
                     if (rank == 0) ptx::mbar_arrive_expect_tx(&full[s], 2 * stage_bytes);
-                    ptx::tma_load_2d_pair(st, &maps.a[z][0], full_even + 8 * s, (int32_t)(kb * BK), (int32_t)m0);
+                    ptx::tma_load_2d_pair(st, &maps.a[z][0], full_even + 8 * s, (int32_t)((kb0 + kb) * BK), (int32_t)m0);
                     if (p.n_a == 2)
                         ptx::tma_load_2d_pair(st + TILE_BYTES, &maps.a[z][1], full_even + 8 * s, (int32_t)(kb * BK),
                                               (int32_t)m0);
                     if (!RESIDENT_W)
-                        ptx::tma_load_2d_pair(st + p.n_a * TILE_BYTES, &maps.b[z], full_even + 8 * s, (int32_t)(kb * BK),
+                        ptx::tma_load_2d_pair(st + p.n_a * TILE_BYTES, &maps.b[z], full_even + 8 * s, (int32_t)((kb0 + kb) * BK),
                                               (int32_t)(n0 + rank * BN));
                 }
             }
