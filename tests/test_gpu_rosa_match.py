@@ -37,3 +37,16 @@ def test_match_equals_the_pushes(cuda_rt, oracle, kind, T):
     cuda_rt.kernel_timing(False)
     assert "rosa_context" in ran and "rosa_match" in ran
     assert np.array_equal(idx, oracle.rosa_qkv_batch_packed(q, k, v, 1, T, C))
+
+
+@pytest.mark.parametrize("T,B,C,left", [(1024, 1, 96, 0.3), (8192, 1, 32, 0.4), (300, 9, 128, 0.2), (700, 9, 128, 0.3), (700, 9, 128, 0.9),
+                                        (1100, 5, 256, 0.2), (1100, 5, 256, 0.8), (1030, 9, 256, 0.3)])
+def test_each_split_of_the_contexts(cuda_rt, oracle, T, B, C, left):
+    """Few or most streams without a closed form, in few and in many streams: every shape of the context kernel."""
+    rng = np.random.default_rng([T, B])
+    q, k, v = planes("biased", T, B * C, rng)
+    q, k, v = (x.reshape(T, B, C).transpose(1, 0, 2).copy() for x in (q, k, v))
+    k[:, :, rng.random(C) >= left] = 1          # the others: constant keys
+    q, k, v = (pack_plane(x.reshape(B * T, C)) for x in (q, k, v))
+    idx, _ = cuda_rt.rosa_qkv_1bit_fwd(q, k, v, np.zeros(C, np.uint16), B, T, C)
+    assert np.array_equal(idx, oracle.rosa_qkv_batch_packed(q, k, v, B, T, C))

@@ -368,19 +368,18 @@ struct ContextLayout {   // bytes of shared memory
     }
 };
 
-template <int NT>
-__global__ void __launch_bounds__(NT, NT > 256 ? 2 : 5)
+// TOGETHER: large buckets by a whole warp, one step after the other.  Runs where the number of listed streams is in
+// [from, to).
+template <int NT, bool TOGETHER>
+__global__ void __launch_bounds__(NT, NT > 512 ? 1 : NT > 256 ? 2 : 5)
 rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restrict__ k_sw, const uint32_t* __restrict__ v_sw,
                     uint32_t* __restrict__ idx_sw, const uint32_t* __restrict__ list, const uint32_t* __restrict__ count,
                     uint32_t* __restrict__ next, uint32_t* __restrict__ hard, uint32_t* __restrict__ hard_count, uint32_t T,
-                    size_t wps, uint32_t c, ContextLimits limits) {
+                    size_t wps, uint32_t c, ContextLimits limits, uint32_t from, uint32_t to) {
     chain_entry();
     constexpr uint32_t NW = NT / 32, BRUTE = context::BRUTE;
-    // Large buckets by the whole warp: for few streams, where a launch lasts as long as its slowest row (one sequence 3.9 ->
-    // 3.6 ms); with many the ballots cost more than they save (16 sequences 12.5 -> 12.9 ms).
-    constexpr bool TOGETHER = NT > 256;
     extern __shared__ __align__(16) uint8_t context_mem[];
-    __shared__ uint32_t sh_item, sh_sums[NW], sh_pairs[NW], sh_gone;
+    __shared__ uint32_t sh_item, sh_sums[NW], sh_pairs[NW], sh_gone, sh_large;
     const uint32_t C = 1u << c, pair_words = C / 2u, words = (T + 31u) / 32u;
     const ContextLayout L(T, c, NW);
     uint16_t* hist = reinterpret_cast<uint16_t*>(context_mem + L.hist);
@@ -397,9 +396,11 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
     uint32_t* out_s = reinterpret_cast<uint32_t*>(context_mem + L.out);
     context::Entry* entries = reinterpret_cast<context::Entry*>(context_mem + L.entries);
     uint16_t* steps = reinterpret_cast<uint16_t*>(context_mem + L.steps);
+    uint16_t* large_steps = hist;   // after the sort; NW * C > T entries for the 16 warps of TOGETHER
     const context::Runs runs{k_ends, in_word, before_word};
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t total = *count;
+    if (total < from || total >= to) return;
     const uint32_t rows_per_warp = (words + NW - 1u) / NW;
     const uint32_t row0 = min(warp * rows_per_warp, words), row1 = min(row0 + rows_per_warp, words);   // a warp's keys
     for (;;) {
@@ -407,6 +408,7 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
         if (threadIdx.x == 0) {
             sh_item = atomicAdd(next, 1u);
             sh_gone = 0u;
+            sh_large = 0u;
         }
         __syncthreads();
         if (sh_item >= total) return;
@@ -560,74 +562,118 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
         const uint32_t* v = v_sw + s * wps;
         uint32_t* out = idx_sw + s * wps;
         uint32_t deep = 0;
-        for (uint32_t row = warp; row < words; row += NW) {
+        // Where a step's bucket lies, its best position within it (by the lanes of a warp where `together`: entries b + lane,
+        // b + lane + 32, ...), and the answer.
+        struct Step {
+            uint32_t b, e, run;
+            context::Query z;
+        };
+        auto find_bucket = [&](uint32_t t) {
+            Step x;
+            if (by_runs) {
+                const uint32_t key = context::run_key(Q, q_ends, t, c);
+                x.run = context::run_at(Q, q_ends, t);
+                x.z.wq = context::window(Q, t);
+                x.z.first = key;
+                x.z.n = 1u;
+            } else {
+                x.run = 0u;
+                x.z = context::query(Q, c, !sorted, t);
+            }
+            x.b = start[x.z.first];
+            x.e = start[x.z.first + x.z.n];
+            return x;
+        };
+        auto finish = [&](const Step& x, uint32_t t, uint32_t found, int32_t best) -> uint32_t {
+            if (found) return found & 0xFFFFu;
+            if (!by_runs) return context::find_shorter(entries, start, c, x.z, t, best);
+            if (context::scan_agreement(best) > (int32_t)x.run) return context::scan_position(best) + 1u;
+            return context::find_inside_run(K, runs, words, context::bit_at(Q, t), x.run, t, deep);
+        };
+        auto v_bit = [&](uint32_t r1) { return r1 ? (v[r1 >> 5] >> (r1 & 31u)) & 1u : 0u; };
+        auto gone = [&] {
+            if (__any_sync(0xFFFFFFFFu, deep > limits.deep)) {
+                if (lane == 0) sh_gone = 1u;
+                return true;
+            }
+            return *static_cast<volatile uint32_t*>(&sh_gone) != 0u;
+        };
+        if (TOGETHER) {   // the steps below BRUTE by a warp each
+            for (uint32_t t = warp; t < min(BRUTE, T); t += NW) {
+                const uint32_t wq = context::window(Q, t);
+                uint32_t best = 0;
+                for (uint32_t r = lane; r < t; r += 32u) {
+                    const uint32_t n = context::agreement(Q, K, t, r, wq ^ context::window(K, r), deep);
+                    if (n) best = max(best, n << 16 | (r + 1u));
+                }
+                best = __reduce_max_sync(0xFFFFFFFFu, best);
+                if (lane == 0 && v_bit(best & 0xFFFFu)) atomicOr(&out_s[t >> 5], 1u << (t & 31u));
+            }
+        }
+        for (uint32_t row = warp + (TOGETHER ? BRUTE / 32u : 0u); row < words; row += NW) {
             const uint32_t i = row * 32u + lane, t = sorted && i >= BRUTE && i < T ? steps[i - BRUTE] : i;
             uint32_t r1 = 0;
+            bool large = false;
             if (row * 32u < BRUTE) {
                 if (i < T) r1 = context::find_brute(Q, K, t, deep);
-            } else {
-                // The step's bucket, or buckets; large ones are looked through by the whole warp, one step after the other
-                // (a lane alone with a bucket of 1 900 positions held up its warp for all of them).
-                uint32_t b = 0, e = 0, run = 0, found = 0;
-                context::Query z{};
-                int32_t best = context::SCAN_NOTHING;
-                if (i < T && by_runs) {
-                    const uint32_t key = context::run_key(Q, q_ends, t, c);
-                    run = context::run_at(Q, q_ends, t);
-                    b = start[key];
-                    e = start[key + 1u];
-                } else if (i < T) {
-                    z = context::query(Q, c, !sorted, t);
-                    b = start[z.first];
-                    e = start[z.first + z.n];
-                }
-                const bool large = TOGETHER && (e - b) * t > CONTEXT_LARGE * T;   // about so many of them lie before t
-                for (uint32_t open = TOGETHER ? __ballot_sync(0xFFFFFFFFu, large) : 0u; open; open &= open - 1u) {
-                    const int l = __ffs((int)open) - 1;
-                    const uint32_t lb = __shfl_sync(0xFFFFFFFFu, b, l) + lane, le = __shfl_sync(0xFFFFFFFFu, e, l);
-                    const uint32_t lt = __shfl_sync(0xFFFFFFFFu, t, l);
-                    uint32_t v = 0;
-                    if (by_runs) {
-                        const uint32_t lr = __shfl_sync(0xFFFFFFFFu, run, l);
-                        v = __reduce_max_sync(0xFFFFFFFFu, context::scan_runs(entries, lb, le, 32u, Q, K, runs, lr, lt, deep));
+            } else if (i < T) {
+                const Step x = find_bucket(t);
+                large = TOGETHER && (x.e - x.b) * t > CONTEXT_LARGE * T;   // about so many of them lie before t
+                if (!large) {
+                    uint32_t found = 0;
+                    int32_t best = context::SCAN_NOTHING;
+                    if (by_runs && x.run >= 32u) {
+                        found = context::scan_runs(entries, x.b, x.e, 1u, Q, K, runs, x.run, t, deep);
                     } else {
-                        const uint32_t lw = __shfl_sync(0xFFFFFFFFu, z.wq, l);
-                        int32_t mine = context::SCAN_NOTHING;
-                        for (uint32_t k = lb; k < le; k += 32u) mine = context::scan_one(entries[k], lt, lw, mine);
-                        mine = __reduce_min_sync(0xFFFFFFFFu, mine);
-                        if (context::scan_full(mine)) v = __reduce_max_sync(0xFFFFFFFFu, context::scan_deep(entries, lb, le, 32u, Q, K, lw, lt, deep));
-                        else if ((int)lane == l) best = mine;
+                        best = context::scan(entries, start, x.z.first, x.z.n, t, x.z.wq, best);
+                        if (context::scan_full(best)) found = context::scan_deep(entries, x.b, x.e, 1u, Q, K, x.z.wq, t, deep);
                     }
-                    if ((int)lane == l) found = v;
-                }
-                if (i < T && by_runs) {
-                    if (!large) found = context::scan_runs(entries, b, e, 1u, Q, K, runs, run, t, deep);
-                    r1 = found ? found & 0xFFFFu : context::find_inside_run(K, runs, words, context::bit_at(Q, t), run, t, deep);
-                } else if (i < T) {
-                    if (!large) {
-                        best = context::scan(entries, start, z.first, z.n, t, z.wq, best);
-                        if (context::scan_full(best)) found = context::scan_deep(entries, b, e, 1u, Q, K, z.wq, t, deep);
-                    }
-                    r1 = found ? found & 0xFFFFu : context::find_shorter(entries, start, c, z, t, best);
+                    r1 = finish(x, t, found, best);
                 }
             }
-            const uint32_t bit = r1 ? (v[r1 >> 5] >> (r1 & 31u)) & 1u : 0u;
-            if (sorted) {
+            const uint32_t bit = v_bit(r1);
+            if (sorted || TOGETHER) {
                 if (bit) atomicOr(&out_s[t >> 5], 1u << (t & 31u));
             } else {
                 const uint32_t word = __ballot_sync(0xFFFFFFFFu, bit != 0u);
                 if (lane == 0) out[row] = word;
             }
-            if (__any_sync(0xFFFFFFFFu, deep > limits.deep)) {
-                if (lane == 0) sh_gone = 1u;
-                break;
+            if (TOGETHER) {
+                const uint32_t these = __ballot_sync(0xFFFFFFFFu, large);
+                uint32_t at = 0;
+                if (these && lane == 0) at = atomicAdd(&sh_large, (uint32_t)__popc(these));
+                at = __shfl_sync(0xFFFFFFFFu, at, 0) + __popc(these & ((1u << lane) - 1u));
+                if (large) large_steps[at] = (uint16_t)t;
             }
-            if (*static_cast<volatile uint32_t*>(&sh_gone)) break;
+            if (gone()) break;
+        }
+        if (TOGETHER) {
+            // Large buckets a step per warp.  They lie side by side, so without this list they fell to a few warps (one
+            // sequence of the default model: a row of 32 such steps took 100 000 cycles, the whole stream 300 000).
+            __syncthreads();
+            const uint32_t n_large = sh_large;
+            for (uint32_t j = warp; j < n_large; j += NW) {
+                const uint32_t t = large_steps[j];
+                const Step x = find_bucket(t);
+                uint32_t found = 0;
+                int32_t best = context::SCAN_NOTHING;
+                if (by_runs && x.run >= 32u) {
+                    found = __reduce_max_sync(0xFFFFFFFFu, context::scan_runs(entries, x.b + lane, x.e, 32u, Q, K, runs, x.run, t, deep));
+                } else {
+                    for (uint32_t k = x.b + lane; k < x.e; k += 32u) best = context::scan_one(entries[k], t, x.z.wq, best);
+                    best = __reduce_min_sync(0xFFFFFFFFu, best);
+                    if (context::scan_full(best))
+                        found = __reduce_max_sync(0xFFFFFFFFu, context::scan_deep(entries, x.b + lane, x.e, 32u, Q, K, x.z.wq, t, deep));
+                }
+                const uint32_t bit = v_bit(finish(x, t, found, best));
+                if (lane == 0 && bit) atomicOr(&out_s[t >> 5], 1u << (t & 31u));
+                if (gone()) break;
+            }
         }
         __syncthreads();
         if (sh_gone) {
             if (threadIdx.x == 0) hard[atomicAdd(hard_count, 1u)] = (uint32_t)s;
-        } else if (sorted) {
+        } else if (sorted || TOGETHER) {
             for (uint32_t w = threadIdx.x; w < words; w += NT) out[w] = out_s[w];
         }
     }
@@ -714,14 +760,15 @@ struct MatchCall {   // the buffers of one call
     uint32_t T;
 };
 
-template <int NT>
-void launch_context(ullis_cuda_runtime* rt, const MatchCall& m, int slot) {
+template <int NT, bool TOGETHER>
+void launch_context(ullis_cuda_runtime* rt, const MatchCall& m, int slot, uint32_t from, uint32_t to) {
+    const auto kernel = rosa_context_kernel<NT, TOGETHER>;
     const uint32_t c = context::bits_for(m.T);
     const size_t smem = ContextLayout(m.T, c, NT / 32).total;
     if (rt->context_smem[slot] != smem) {
         int per_sm = 0;
-        ULLIS_CUDA_CHECK(cudaFuncSetAttribute(rosa_context_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        ULLIS_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rosa_context_kernel<NT>, NT, smem));
+        ULLIS_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        ULLIS_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, NT, smem));
         rt->context_ctas[slot] = std::max(1, per_sm) * rt->sm_count;
         rt->context_smem[slot] = smem;
     }
@@ -729,8 +776,8 @@ void launch_context(ullis_cuda_runtime* rt, const MatchCall& m, int slot) {
     // A match kernel step costs about as much as 100 positions here; up to 24 the lanes are even enough without sorting
     // the steps.  128 long comparisons per stream at most are thrown away when a stream turns out to repeat itself.
     const ContextLimits limits{24u, 96u, 160u, 256u};
-    rt->chain(rosa_context_kernel<NT>, grid, NT, smem, m.q, m.k, m.v, m.idx, m.list, m.counts, m.counts + 3,
-              m.hard, m.counts + 2, m.T, m.wps, c, limits);
+    rt->chain(kernel, grid, NT, smem, m.q, m.k, m.v, m.idx, m.list, m.counts, m.counts + 3, m.hard, m.counts + 2, m.T, m.wps, c,
+              limits, from, to);
     rt->launched("rosa_context");
 }
 
@@ -783,10 +830,22 @@ void rosa_match(ullis_cuda_runtime* rt, const uint32_t* q_sw, const uint32_t* k_
     rt->chain(rosa_classify_kernel, (unsigned)((streams * CLASSIFY_LANES + 127) / 128), 128, 0, q_sw, k_sw, v_sw, idx_sw,
               streams, T, m.wps, m.list, m.counts, m.cq_list, m.counts + 1);
     rt->launched("rosa_classify");
-    // few streams: sixteen warps each, so that the last of them is done soon (one sequence of 512 channels: 0.20 ms
-    // against 0.28 with eight); many: eight (1.79 ms for 32 768 streams against 1.98 with sixteen)
-    if (streams <= 1024u) launch_context<512>(rt, m, 1);
-    else launch_context<256>(rt, m, 0);
+    // Two ways, one of which has nothing to do: how many streams are left is known on the device only.  Where most had a
+    // closed form the others are uneven too, and large buckets and many warps per stream pay; where hardly any had, few warps
+    // do, unless the streams are so few that a launch lasts as long as one of them.  Default model, ms: gain N(0, 0.02), of
+    // whose streams 12 % are left, with 1024 threads together / 512 together / 256: one sequence 2.5 / 2.8 / 4.3, four 3.7 /
+    // 4.0 / 5.9, 16 9.7 / 9.2 / 11.1, 64 32.2 / 29.8 / 31.2; gain 1 + N(0, 0.02), all left: one sequence 2.5 / 2.3 / 2.5, four
+    // 5.6 / 4.7 / 4.4, 16 18.7 / 14.8 / 12.7.
+    const uint32_t half = (uint32_t)(streams / 2) + 1u, all = ~0u;
+    // Short streams by the thousand have too few steps for many warps (64 times 300 steps 5.2 with 256 threads alone, 5.7).
+    if (streams > 1024u && (T < 512u || (T < 1024u && streams > 8192u))) {
+        launch_context<256, false>(rt, m, 2, 0u, all);
+    } else {
+        if (streams <= 2048u && T >= 1024u) launch_context<1024, true>(rt, m, 0, 0u, half);
+        else launch_context<512, true>(rt, m, 1, 0u, streams <= 1024u ? all : half);
+        if (streams > 1024u) launch_context<256, false>(rt, m, 2, half, all);
+        else if (T >= 1024u) launch_context<512, true>(rt, m, 1, half, all);
+    }
     if (T <= 1024u) launch_match<1>(rt, m, 0, 1024);
     else if (T <= 2048u) launch_match<2>(rt, m, 1, 1024);
     else if (T <= 4096u) launch_match<4>(rt, m, 2, 2048);
