@@ -761,7 +761,8 @@ struct MatchCall {   // the buffers of one call
 };
 
 template <int NT, bool TOGETHER>
-void launch_context(ullis_cuda_runtime* rt, const MatchCall& m, int slot, uint32_t from, uint32_t to) {
+void launch_context(ullis_cuda_runtime* rt, const MatchCall& m, int slot, uint32_t from, uint32_t to,
+                    const char* what = "rosa_context") {
     const auto kernel = rosa_context_kernel<NT, TOGETHER>;
     const uint32_t c = context::bits_for(m.T);
     const size_t smem = ContextLayout(m.T, c, NT / 32).total;
@@ -778,7 +779,7 @@ void launch_context(ullis_cuda_runtime* rt, const MatchCall& m, int slot, uint32
     const ContextLimits limits{24u, 96u, 160u, 256u};
     rt->chain(kernel, grid, NT, smem, m.q, m.k, m.v, m.idx, m.list, m.counts, m.counts + 3, m.hard, m.counts + 2, m.T, m.wps, c,
               limits, from, to);
-    rt->launched("rosa_context");
+    rt->launched(what);
 }
 
 template <int NW>
@@ -843,8 +844,8 @@ void rosa_match(ullis_cuda_runtime* rt, const uint32_t* q_sw, const uint32_t* k_
     } else {
         if (streams <= 2048u && T >= 1024u) launch_context<1024, true>(rt, m, 0, 0u, half);
         else launch_context<512, true>(rt, m, 1, 0u, streams <= 1024u ? all : half);
-        if (streams > 1024u) launch_context<256, false>(rt, m, 2, half, all);
-        else if (T >= 1024u) launch_context<512, true>(rt, m, 1, half, all);
+        if (streams > 1024u) launch_context<256, false>(rt, m, 2, half, all, "rosa_context_even");
+        else if (T >= 1024u) launch_context<512, true>(rt, m, 1, half, all, "rosa_context_even");
     }
     if (T <= 1024u) launch_match<1>(rt, m, 0, 1024);
     else if (T <= 2048u) launch_match<2>(rt, m, 1, 1024);
