@@ -688,25 +688,41 @@ constexpr uint32_t MATCH_COUNTS = 5;   // of MatchCall
 // (sam_core.cuh run_constant_q), a running maximum over (run length, position).  T <= 65535.
 __device__ __forceinline__ void constant_q_warp(uint32_t c, const uint32_t* __restrict__ k, const uint32_t* __restrict__ v,
                                                 uint32_t* __restrict__ out, uint32_t T) {
-    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t lane = threadIdx.x & 31u, words = (T + 31u) / 32u;
     uint32_t run_before = 0, best = 0;   // run length << 16 | position + 1
-    for (uint32_t row = 0; row < (T + 31u) / 32u; ++row) {
-        const uint32_t t = row * 32u + lane, same = c ? k[row] : ~k[row];
-        const uint32_t n = min((uint32_t)__clz((int)~(same << (31u - lane))), lane + 1u);
-        const uint32_t run = n == lane + 1u ? n + run_before : n;
-        uint32_t key = run ? run << 16 | (t + 1u) : 0u;
+    for (uint32_t row0 = 0; row0 < words; row0 += 32u) {
+        const uint32_t keys = row0 + lane < words ? k[row0 + lane] : 0u;
+        for (uint32_t row4 = row0; row4 < min(row0 + 32u, words); row4 += 4u) {   // four words, their v bits in flight together
+            uint32_t mine[4], bit[4];
 #pragma unroll
-        for (uint32_t o = 1; o < 32u; o <<= 1) {
-            const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, key, o);
-            if (lane >= o) key = max(key, x);
+            for (uint32_t u = 0; u < 4u; ++u) {
+                const uint32_t row = row4 + u, t = row * 32u + lane, word = __shfl_sync(0xFFFFFFFFu, keys, (int)(row - row0));
+                const uint32_t same = c ? word : ~word;
+                const uint32_t n = min((uint32_t)__clz((int)~(same << (31u - lane))), lane + 1u);
+                const uint32_t run = n == lane + 1u ? n + run_before : n;
+                uint32_t key = run ? run << 16 | (t + 1u) : 0u;
+#pragma unroll
+                for (uint32_t o = 1; o < 32u; o <<= 1) {
+                    const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, key, o);
+                    if (lane >= o) key = max(key, x);
+                }
+                mine[u] = __shfl_up_sync(0xFFFFFFFFu, key, 1);   // the positions before t
+                mine[u] = lane == 0u ? best : max(mine[u], best);
+                if (t >= T) mine[u] = 0u;
+                run_before = __shfl_sync(0xFFFFFFFFu, run, 31);
+                best = max(best, __shfl_sync(0xFFFFFFFFu, key, 31));
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < 4u; ++u) {
+                const uint32_t p = mine[u] & 0xFFFFu;
+                bit[u] = mine[u] ? (v[p >> 5] >> (p & 31u)) & 1u : 0u;
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < 4u; ++u) {
+                const uint32_t word = __ballot_sync(0xFFFFFFFFu, bit[u] != 0u);
+                if (lane == 0 && row4 + u < words) out[row4 + u] = word;
+            }
         }
-        uint32_t mine = __shfl_up_sync(0xFFFFFFFFu, key, 1);   // the positions before t
-        mine = lane == 0u ? best : max(mine, best);
-        const uint32_t p = mine & 0xFFFFu;
-        const uint32_t word = __ballot_sync(0xFFFFFFFFu, mine != 0u && t < T && ((v[p >> 5] >> (p & 31u)) & 1u) != 0u);
-        if (lane == 0) out[row] = word;
-        run_before = __shfl_sync(0xFFFFFFFFu, run, 31);
-        best = max(best, __shfl_sync(0xFFFFFFFFu, key, 31));
     }
 }
 
@@ -731,11 +747,9 @@ rosa_match_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restrict_
     while (piece > 32u && (uint64_t)total * ((T + piece - 1u) / piece) < 3ull * warps) piece >>= 1;
     const uint32_t pieces = (T + piece - 1u) / piece;
     const uint32_t items = total * pieces;   // below 2^32: the host checked it for the shortest pieces
-    for (;;) {
-        uint32_t item = 0;
-        if ((threadIdx.x & 31u) == 0u) item = atomicAdd(next, 1u);
-        item = __shfl_sync(0xFFFFFFFFu, item, 0);
-        if (item >= items + constant) return;
+    // The first item of a warp is its own number, so that the many without one leave without a word to anybody.
+    for (uint32_t item = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; item < items + constant;
+         item = warps + __shfl_sync(0xFFFFFFFFu, (threadIdx.x & 31u) == 0u ? atomicAdd(next, 1u) : 0u, 0)) {
         if (item >= items) {
             const size_t s = cq_list[item - items];
             constant_q_warp(q_sw[s * wps] & 1u, k_sw + s * wps, v_sw + s * wps, idx_sw + s * wps, T);
