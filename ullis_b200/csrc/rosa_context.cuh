@@ -230,11 +230,11 @@ RC_HD Query query(const uint32_t* Q, uint32_t c, bool wide, uint32_t t) {
 }
 
 // Agreements counted on beyond the windows: of the positions before t among entries [b, e), every step-th, whose window is
-// wq; packed as in scan_runs.
+// wq; packed as in scan_runs.  Ends when `deep` passes `most`: the stream is given up then, whatever the answer.
 RC_HD uint32_t scan_deep(const Entry* entries, uint32_t b, uint32_t e, uint32_t step, const uint32_t* Q, const uint32_t* K, uint32_t wq, uint32_t t,
-                         uint32_t& deep) {
+                         uint32_t& deep, uint32_t most) {
     uint32_t best = 0;
-    for (; b < e; b += step) {
+    for (; b < e && deep <= most; b += step) {
         const Entry a = entries[b];
         if (a.r >= t || wq != a.key) continue;
         const uint32_t v = agreement(Q, K, t, a.r, 0u, deep) << 16 | (a.r + 1u);

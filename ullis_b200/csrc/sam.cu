@@ -626,7 +626,7 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
                         found = context::scan_runs(entries, x.b, x.e, 1u, Q, K, runs, x.run, t, deep);
                     } else {
                         best = context::scan(entries, start, x.z.first, x.z.n, t, x.z.wq, best);
-                        if (context::scan_full(best)) found = context::scan_deep(entries, x.b, x.e, 1u, Q, K, x.z.wq, t, deep);
+                        if (context::scan_full(best)) found = context::scan_deep(entries, x.b, x.e, 1u, Q, K, x.z.wq, t, deep, limits.deep);
                     }
                     r1 = finish(x, t, found, best);
                 }
@@ -663,7 +663,7 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
                     for (uint32_t k = x.b + lane; k < x.e; k += 32u) best = context::scan_one(entries[k], t, x.z.wq, best);
                     best = __reduce_min_sync(0xFFFFFFFFu, best);
                     if (context::scan_full(best))
-                        found = __reduce_max_sync(0xFFFFFFFFu, context::scan_deep(entries, x.b + lane, x.e, 32u, Q, K, x.z.wq, t, deep));
+                        found = __reduce_max_sync(0xFFFFFFFFu, context::scan_deep(entries, x.b + lane, x.e, 32u, Q, K, x.z.wq, t, deep, limits.deep));
                 }
                 const uint32_t bit = v_bit(finish(x, t, found, best));
                 if (lane == 0 && bit) atomicOr(&out_s[t >> 5], 1u << (t & 31u));
