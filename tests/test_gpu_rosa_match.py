@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 from conftest import pack_plane
+from ullis_b200 import cuda
 
 pytestmark = pytest.mark.gpu
 
@@ -50,3 +51,17 @@ def test_each_split_of_the_contexts(cuda_rt, oracle, T, B, C, left):
     q, k, v = (pack_plane(x.reshape(B * T, C)) for x in (q, k, v))
     idx, _ = cuda_rt.rosa_qkv_1bit_fwd(q, k, v, np.zeros(C, np.uint16), B, T, C)
     assert np.array_equal(idx, oracle.rosa_qkv_batch_packed(q, k, v, B, T, C))
+
+
+def test_two_runtimes_of_one_device_at_lengths_of_their_own(oracle):
+    """Shared memory of the context kernel grows with the length, its limit belongs to the function: a runtime at a short
+    length takes nothing away from one at a long length."""
+    runtimes = [cuda.CudaRuntime(0) for _ in range(2)]
+    try:
+        for which, T, C in ((0, 8192, 32), (1, 64, 32), (0, 8192, 32), (1, 512, 64), (1, 8192, 32), (0, 4096, 32), (1, 8192, 32)):
+            q, k, v = (pack_plane(x) for x in planes("even", T, C, np.random.default_rng([T, which])))
+            idx, _ = runtimes[which].rosa_qkv_1bit_fwd(q, k, v, np.zeros(C, np.uint16), 1, T, C)
+            assert np.array_equal(idx, oracle.rosa_qkv_batch_packed(q, k, v, 1, T, C)), (which, T)
+    finally:
+        for rt in runtimes:
+            rt.close()

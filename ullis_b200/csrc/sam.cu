@@ -766,6 +766,8 @@ rosa_match_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restrict_
     }
 }
 
+constexpr size_t MATCH_MAX_TIME = 8192;   // 256 words of lags, eight per lane
+
 struct MatchCall {   // the buffers of one call
     const uint32_t *q, *k, *v;
     uint32_t *idx, *list, *cq_list, *hard;
@@ -780,9 +782,12 @@ void launch_context(ullis_cuda_runtime* rt, const MatchCall& m, int slot, uint32
     const auto kernel = rosa_context_kernel<NT, TOGETHER>;
     const uint32_t c = context::bits_for(m.T);
     const size_t smem = ContextLayout(m.T, c, NT / 32).total;
+    if (!rt->context_smem[slot]) {   // the attribute belongs to the function, not to this runtime: always the same value
+        const size_t most = ContextLayout((uint32_t)MATCH_MAX_TIME, context::bits_for((uint32_t)MATCH_MAX_TIME), NT / 32).total;
+        ULLIS_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+    }
     if (rt->context_smem[slot] != smem) {
         int per_sm = 0;
-        ULLIS_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         ULLIS_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, NT, smem));
         rt->context_ctas[slot] = std::max(1, per_sm) * rt->sm_count;
         rt->context_smem[slot] = smem;
@@ -829,7 +834,6 @@ size_t stride_for(int algo, size_t T) {
 
 // The whole call without an automaton: classification, the listed streams by contexts, and by sets of lags those that
 // the contexts leave and the ones with a constant q.
-constexpr size_t MATCH_MAX_TIME = 8192;   // 256 words of lags, eight per lane
 void rosa_match(ullis_cuda_runtime* rt, const uint32_t* q_sw, const uint32_t* k_sw, const uint32_t* v_sw, uint32_t* idx_sw,
                 size_t streams, uint32_t T) {
     MatchCall m;
