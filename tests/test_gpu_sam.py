@@ -186,3 +186,37 @@ def test_both_forms_of_the_serial_pass_give_the_same_idx(oracle, monkeypatch, wa
         assert ("rosa_pass1_smem" in ran) == (waves != "0") and ("rosa_pass1" in ran) == (waves != "1000")
     finally:
         rt.close()
+
+
+@pytest.mark.parametrize("budget_mb", ["16", "17"])
+def test_waves_at_a_length_that_takes_the_automaton_by_itself(oracle, monkeypatch, budget_mb):
+    """8 200 steps are beyond the match without an automaton, 297 344 bytes of states per stream: 56 and 59 streams per wave."""
+    monkeypatch.setenv("ULLIS_CUDA_SAM_BUDGET_MB", budget_mb)
+    rt = cuda.CudaRuntime(0)
+    try:
+        rt.kernel_timing(True)
+        B, T, C = 2, 8200, 96
+        for gen, seed in ((synth.rosa_bits_iid, 33), (synth.rosa_bits_periodic, 34)):
+            run_both(rt, oracle, *gen(seed, B, T, C), B, T, C, algos=(cuda.SAM_EULER,))
+        assert rt.kernel_times()["rosa_pass1"][1] == 2 * -(-B * C // (56 if budget_mb == "16" else 59))
+    finally:
+        rt.close()
+
+
+@pytest.mark.parametrize("T", [2048, 8192])
+def test_a_cap_on_scratch_memory_does_not_ask_for_the_automaton(oracle, monkeypatch, T):
+    """With 1 MiB for the sets of lags the match runs in fewer CTAs: same kernels, same idx."""
+    monkeypatch.setenv("ULLIS_CUDA_SAM_BUDGET_MB", "1")
+    rt = cuda.CudaRuntime(0)
+    try:
+        rng = np.random.default_rng(T)
+        C = 64                                                    # streams that repeat themselves: left to the sets of lags
+        base, phase = rng.integers(0, 2, (100, C), dtype=np.uint8), np.arange(T)[:, None] % rng.integers(2, 100, C)[None, :]
+        q = np.take_along_axis(base, phase, 0)
+        k, v = q ^ (rng.random((T, C)) < 0.001), rng.integers(0, 2, (T, C), dtype=np.uint8)
+        rt.kernel_timing(True)
+        run_both(rt, oracle, *(pack_plane(np.asarray(x, np.uint8)) for x in (q, k, v)), 1, T, C, algos=(cuda.SAM_EULER,))
+        ran = rt.kernel_times()
+        assert "rosa_context" in ran and "rosa_match" in ran and "rosa_pass1" not in ran
+    finally:
+        rt.close()

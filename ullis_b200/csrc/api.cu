@@ -332,12 +332,11 @@ int32_t ullis_cuda_runtime_create(int32_t device, ullis_cuda_runtime** out) {
             const int a = atoi(env) / 10, b = atoi(env) % 10;   // e.g. 32 = 3 stages (one operand), 2 stages (two)
             if (a >= 2 && a <= 4 && b >= 2 && b <= 4) { rt->tc_stages = a; rt->tc_stages2 = b; }
         }
-        // Options of the suffix automaton: it only runs where the match by sets of lags does not reach, so asking for one
-        // of its forms asks for the automaton.
-        for (const char* name : {"ULLIS_CUDA_SAM_COOP", "ULLIS_CUDA_SAM_BUDGET_MB", "ULLIS_CUDA_SAM_SPARSE", "ULLIS_CUDA_SAM_WORDS",
-                                 "ULLIS_CUDA_SAM_WALK_CHUNKED", "ULLIS_CUDA_SAM_SMEM_WAVES", "ULLIS_CUDA_SAM_RELOAD_W",
-                                 "ULLIS_CUDA_SAM_DEFER_CLIMB", "ULLIS_CUDA_SAM_SPLIT", "ULLIS_CUDA_SAM_SIDE",
-                                 "ULLIS_CUDA_SAM_COOP_THREADS", "ULLIS_CUDA_SAM_LANES"})
+        // Options that choose a form of the suffix automaton: it only runs where the match without one does not reach, so
+        // asking for a form asks for the automaton.  The cap on scratch memory is no such option: either way keeps to it.
+        for (const char* name : {"ULLIS_CUDA_SAM_COOP", "ULLIS_CUDA_SAM_SPARSE", "ULLIS_CUDA_SAM_WORDS", "ULLIS_CUDA_SAM_WALK_CHUNKED",
+                                 "ULLIS_CUDA_SAM_SMEM_WAVES", "ULLIS_CUDA_SAM_RELOAD_W", "ULLIS_CUDA_SAM_DEFER_CLIMB",
+                                 "ULLIS_CUDA_SAM_SPLIT", "ULLIS_CUDA_SAM_SIDE", "ULLIS_CUDA_SAM_COOP_THREADS", "ULLIS_CUDA_SAM_LANES"})
             if (getenv(name)) rt->sam_automaton = true;
         if (const char* env = getenv("ULLIS_CUDA_SAM_COOP")) rt->sam_coop = atoi(env) != 0;
         if (const char* env = getenv("ULLIS_CUDA_SAM_BUDGET_MB")) {

@@ -144,8 +144,8 @@ struct ullis_cuda_runtime {
     uint8_t* inputs_host = nullptr;
     ullis::DeviceBuffer inputs_dev;
     size_t inputs_used = 0, inputs_sent = 0;
-    size_t sam_budget_bytes = (size_t)12 << 30;   // cap of sam_scratch; more streams than fit run in waves
-    ullis::DeviceBuffer sam_scratch;    // suffix-automaton state blocks
+    size_t sam_budget_bytes = (size_t)12 << 30;   // cap of sam_scratch; more streams than fit run in waves, the match takes fewer CTAs
+    ullis::DeviceBuffer sam_scratch;    // suffix-automaton state blocks, or the sets that the match keeps
     ullis::DeviceBuffer sam_list;       // ids of the streams that need the automaton + their count
     size_t sam_last_streams = 0;        // streams of the last suffix-automaton call ...
     const uint32_t* sam_last_counts = nullptr;   // ... and its counters: listed, constant q

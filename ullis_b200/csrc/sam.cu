@@ -812,8 +812,11 @@ void launch_match(ullis_cuda_runtime* rt, const MatchCall& m, int slot, uint32_t
         rt->match_ctas[slot] = std::max(1, per_sm) * rt->sm_count;
     }
     const size_t most = (m.streams * m.wps + MATCH_WARPS - 1) / MATCH_WARPS;   // every stream in the shortest pieces
-    const unsigned grid = (unsigned)std::min<size_t>(rt->match_ctas[slot], most);
-    uint32_t* kept = rt->sam_scratch.as<uint32_t>((size_t)grid * MATCH_WARPS * match::CHECKPOINTS * 32u * NW);
+    // the kept sets count against the same cap on scratch memory as the automaton's states (32 KB * NW per CTA)
+    const size_t kept_words = (size_t)MATCH_WARPS * match::CHECKPOINTS * 32u * NW;
+    const size_t allowed = std::max<size_t>(1, rt->sam_budget_bytes / (kept_words * 4));
+    const unsigned grid = (unsigned)std::min({(size_t)rt->match_ctas[slot], most, allowed});
+    uint32_t* kept = rt->sam_scratch.as<uint32_t>((size_t)grid * kept_words);
     rt->chain(rosa_match_kernel<NW>, grid, 32 * MATCH_WARPS, smem, m.q, m.k, m.v, m.idx, m.hard, m.counts + 2,
               m.cq_list, m.counts + 1, m.counts + 4, m.clear, kept, m.T, m.wps, ring_words);
     rt->launched("rosa_match");
