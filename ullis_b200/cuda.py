@@ -145,34 +145,57 @@ def _z(n):
 
 
 class _ResultBlock:
-    """One page-locked block lent to a numpy array; it goes back to the pool with the last array that looks at it."""
+    """The memory under one numpy array; it goes back to the pool with the last array that looks at it.  `own`: an ordinary
+    array it keeps alive, where the memory is not page-locked."""
 
-    __slots__ = ("pool", "addr", "size", "__array_interface__")
+    __slots__ = ("pool", "addr", "size", "own", "__array_interface__")
 
-    def __init__(self, pool: "_ResultPool", addr: int, size: int, nbytes: int):
-        self.pool, self.addr, self.size = pool, addr, size
+    def __init__(self, pool: "_ResultPool", addr: int, size: int, nbytes: int, own=None):
+        self.pool, self.addr, self.size, self.own = pool, addr, size, own
         self.__array_interface__ = {"data": (addr, False), "shape": (nbytes,), "typestr": "|u1", "version": 3}
 
     def __del__(self):
-        self.pool.give_back(self.addr, self.size)
+        self.pool.give_back(None if self.own is not None else self.addr, self.size)
 
 
 class _ResultPool:
     """Page-locked memory for result arrays.  A fresh numpy array is pageable memory nobody has touched: the copy into
-    it went through the driver's staging buffer and took a page fault every 4 KB (168 MB of ROSA results: 36 ms, now 4).
-    Blocks are reused once the arrays over them are gone.  At most `limit` bytes are page-locked, lent and idle
-    together; beyond that results are ordinary arrays."""
+    it goes through the driver's staging buffer and takes a page fault every 4 KB.  Blocks are reused once the arrays over
+    them are gone.  At most `limit` bytes are page-locked, lent and idle together; beyond that results are ordinary arrays.
 
-    def __init__(self, limit: int = 1 << 30, smallest: int = 64):
-        self.limit, self.smallest = limit, smallest
+    Page-locking costs more than the first copy gains, and only reuse brings it back.  Microseconds for a result of 16 / 64
+    / 160 MiB: into an ordinary array 5 800 / 22 800 / 57 600, into a block page-locked for it 7 600 / 31 000 / 89 200, into
+    a reused block 1 200 / 7 300 / 18 500.  So there are at most as many blocks of a size as ordinary arrays of that size have
+    been dropped, each of which would have left a block to reuse: a first result and those of a caller that keeps them are
+    ordinary arrays.  Up to `at_once` bytes (2 to 5 us to lock) every result is page-locked."""
+
+    def __init__(self, limit: int = 1 << 30, smallest: int = 64, at_once: int = 1 << 18):
+        self.limit, self.smallest, self.at_once = limit, smallest, at_once
         self._idle = {}                      # block size -> [addresses]
+        self._blocks = {}                    # block size -> page-locked blocks, lent and idle
+        self._dropped = {}                   # block size -> ordinary arrays that are gone
         self._held = 0                       # bytes page-locked
+        self._users = 0                      # open runtimes
+        self._retired = False                # the last one was closed: what comes back is freed
+        self._free = None
         self._lock = threading.RLock()       # a garbage collection inside empty() may give a block back
 
     @staticmethod
     def _block_size(nbytes: int) -> int:
         step = 1 << max(12, nbytes.bit_length() - 3)      # eighths of a power of two
         return (nbytes + step - 1) // step * step
+
+    def attach(self):
+        with self._lock:
+            self._users += 1
+            self._retired = False
+
+    def detach(self):
+        with self._lock:
+            self._users -= 1
+            if self._users == 0:
+                self._retired = True
+                self.release()
 
     def empty(self, rt: "CudaRuntime", shape, dtype) -> np.ndarray:
         dtype = np.dtype(dtype)
@@ -183,11 +206,16 @@ class _ResultPool:
         with self._lock:
             idle = self._idle.get(size)
             addr = idle.pop() if idle else self._lock_memory(rt, size)
-        if addr is None:
-            return np.empty(shape, dtype)
-        return np.asarray(_ResultBlock(self, addr, size, nbytes)).view(dtype).reshape(shape)
+        if addr is not None:
+            block = _ResultBlock(self, addr, size, nbytes)
+        else:
+            own = np.empty(nbytes, np.uint8)
+            block = _ResultBlock(self, own.ctypes.data, size, nbytes, own)
+        return np.asarray(block).view(dtype).reshape(shape)
 
     def _lock_memory(self, rt, size):
+        if size > self.limit or (size > self.at_once and self._blocks.get(size, 0) >= self._dropped.get(size, 0)):
+            return None
         if self._held + size > self.limit:
             self._drop_idle(self._held + size - self.limit)
             if self._held + size > self.limit:
@@ -195,22 +223,46 @@ class _ResultPool:
         p = C.c_void_p()
         if rt._lib.ullis_cuda_host_alloc(rt._h, C.c_size_t(size), C.byref(p)) != OK:
             return None
+        self._free = rt._lib.ullis_cuda_host_free
         self._held += size
+        self._blocks[size] = self._blocks.get(size, 0) + 1
         return p.value
+
+    def _unlock_memory(self, addr, size):
+        self._free(C.c_void_p(addr))
+        self._held -= size
+        self._blocks[size] -= 1
+        self._dropped[size] = self._dropped.get(size, 0) - 1   # its size has to show again that it is worth it
 
     def _drop_idle(self, nbytes):
         for size in sorted(self._idle, reverse=True):
             while nbytes > 0 and self._idle[size]:
-                _LIB.ullis_cuda_host_free(C.c_void_p(self._idle[size].pop()))
-                self._held -= size
+                self._unlock_memory(self._idle[size].pop(), size)
                 nbytes -= size
+
+    def release(self):
+        """Gives the idle blocks back to the system; those under a live array follow when they are idle and this is called
+        again, or when the array is dropped after the last runtime was closed."""
+        with self._lock:
+            self._drop_idle(self._held)
 
     def give_back(self, addr, size):
         with self._lock:
-            self._idle.setdefault(size, []).append(addr)
+            if addr is None:
+                self._dropped[size] = self._dropped.get(size, 0) + 1
+            elif self._retired:
+                self._unlock_memory(addr, size)
+            else:
+                self._idle.setdefault(size, []).append(addr)
 
 
 _RESULTS = _ResultPool()
+
+
+def release_result_memory() -> None:
+    """Returns the page-locked memory of results that were dropped (kept for the next result of their size, at most 1 GiB
+    in all) to the system.  Closing the last runtime does the same."""
+    _RESULTS.release()
 
 
 class CudaRuntime:
@@ -224,14 +276,16 @@ class CudaRuntime:
             raise UllisCudaError(rc, self._lib.ullis_cuda_last_error(None).decode())
         self._handle = _Handle(h, self._lib.ullis_cuda_runtime_destroy)
         self.device = device
+        _RESULTS.attach()
 
     @property
     def _h(self):
         return self._handle.h
 
     def close(self):
-        if getattr(self, "_handle", None):
+        if getattr(self, "_handle", None) and self._handle.h:
             self._handle.close()
+            _RESULTS.detach()
 
     def __del__(self):
         try:
