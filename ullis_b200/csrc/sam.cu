@@ -591,12 +591,10 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
             return context::find_inside_run(K, runs, words, context::bit_at(Q, t), x.run, t, deep);
         };
         auto v_bit = [&](uint32_t r1) { return r1 ? (v[r1 >> 5] >> (r1 & 31u)) & 1u : 0u; };
-        auto gone = [&] {
-            if (__any_sync(0xFFFFFFFFu, deep > limits.deep)) {
-                if (lane == 0) sh_gone = 1u;
-                return true;
-            }
-            return *static_cast<volatile uint32_t*>(&sh_gone) != 0u;
+        auto gone = [&] {   // by vote: lanes that read the flag apart from one another could disagree, and part for good
+            if (!__any_sync(0xFFFFFFFFu, deep > limits.deep || *static_cast<volatile uint32_t*>(&sh_gone) != 0u)) return false;
+            if (lane == 0) sh_gone = 1u;
+            return true;
         };
         if (TOGETHER) {   // the steps below BRUTE by a warp each
             for (uint32_t t = warp; t < min(BRUTE, T); t += NW) {
