@@ -33,33 +33,34 @@ def lib():
     return Library()
 
 
-def test_kept_results_lock_nothing_and_dropped_ones_lock_once(lib):
-    pool = cuda._ResultPool()
+def test_kept_results_lock_little_and_dropped_ones_are_reused(lib):
+    pool = cuda._ResultPool(unproven=3 * BIG)
     kept = [pool.empty(lib, BIG, np.uint8) for _ in range(20)]
-    assert lib.locks == 0
+    assert lib.locks == 3
     for i, a in enumerate(kept):
         a[:] = i
     assert all((a == i).all() for i, a in enumerate(kept))
     del kept[5:], a
     for _ in range(50):
         pool.empty(lib, BIG, np.uint8)
-    assert lib.locks == 1
+    assert lib.locks == 4                                              # the three are under live arrays
     kept += [pool.empty(lib, BIG, np.uint8) for _ in range(100)]       # as many blocks as results came back before, no more
-    assert lib.locks <= 16 and pool._held == lib.locks * pool._block_size(BIG)
+    assert lib.locks <= 3 + 15 and pool._held == lib.locks * pool._block_size(BIG)
 
 
 def test_results_that_live_in_batches_are_all_reused(lib):
-    pool = cuda._ResultPool()
+    pool = cuda._ResultPool(unproven=BIG)
     for _ in range(4):
         batch = [pool.empty(lib, (2, BIG // 8), np.float32) for _ in range(10)]
         del batch
     assert lib.locks == 10
 
 
-def test_small_results_are_page_locked_at_once(lib):
-    pool = cuda._ResultPool()
-    kept = [pool.empty(lib, 1000, np.float32) for _ in range(5)]
-    assert lib.locks == 5 and len(kept) == 5
+def test_one_result_larger_than_the_trial_is_locked_the_second_time(lib):
+    pool = cuda._ResultPool(unproven=BIG)
+    for locks in (0, 1, 1):
+        pool.empty(lib, 2 * BIG, np.uint8)
+        assert lib.locks == locks
 
 
 def test_idle_memory_is_given_back_on_request_and_with_the_last_runtime(lib):
@@ -82,13 +83,15 @@ def test_idle_memory_is_given_back_on_request_and_with_the_last_runtime(lib):
     assert not lib.blocks and pool._held == 0
 
 
-def test_two_sizes_that_do_not_fit_together_do_not_take_turns_at_every_call(lib):
-    pool = cuda._ResultPool(limit=3 * BIG, at_once=0)
+@pytest.mark.parametrize("unproven", [0, 1 << 28])
+def test_sizes_that_do_not_fit_together_do_not_take_turns_at_every_call(lib, unproven):
+    pool = cuda._ResultPool(limit=3 * BIG, unproven=unproven)
     for _ in range(10):
         pool.empty(lib, 2 * BIG, np.uint8)
         pool.empty(lib, 2 * BIG + BIG // 2, np.uint8)
-    assert lib.locks <= 12 and pool._held <= pool.limit
-    assert pool.empty(lib, 4 * BIG, np.uint8).size == 4 * BIG          # never fits: nothing idle is dropped for it
+    assert lib.locks <= 12 and pool._held <= pool.limit                # of 20 calls
+    held = pool._held
+    assert pool.empty(lib, 4 * BIG, np.uint8).size == 4 * BIG and pool._held == held   # never fits: nothing goes for it
 
 
 def test_threads_share_the_pool(lib):

@@ -165,16 +165,18 @@ class _ResultPool:
 
     Page-locking costs more than the first copy gains, and only reuse brings it back.  Microseconds for a result of 16 / 64
     / 160 MiB: into an ordinary array 5 800 / 22 800 / 57 600, into a block page-locked for it 7 600 / 31 000 / 89 200, into
-    a reused block 1 200 / 7 300 / 18 500.  So there are at most as many blocks of a size as ordinary arrays of that size have
-    been dropped, each of which would have left a block to reuse: a first result and those of a caller that keeps them are
-    ordinary arrays.  Up to `at_once` bytes (2 to 5 us to lock) every result is page-locked."""
+    a reused block 1 200 / 7 300 / 18 500.  So at most `unproven` bytes lie in blocks that have never come back: a caller
+    that keeps its results loses no more than those (256 MiB: 50 ms, once) and gets ordinary arrays then.  An ordinary array
+    that is dropped shows that a block would have come back, and one more of its size may be locked."""
 
-    def __init__(self, limit: int = 1 << 30, smallest: int = 64, at_once: int = 1 << 18):
-        self.limit, self.smallest, self.at_once = limit, smallest, at_once
+    def __init__(self, limit: int = 1 << 30, smallest: int = 64, unproven: int = 1 << 28):
+        self.limit, self.smallest, self.unproven = limit, smallest, unproven
         self._idle = {}                      # block size -> [addresses]
         self._blocks = {}                    # block size -> page-locked blocks, lent and idle
         self._dropped = {}                   # block size -> ordinary arrays that are gone
         self._held = 0                       # bytes page-locked
+        self._new = set()                    # addresses of the blocks that have not come back yet ...
+        self._new_bytes = 0                  # ... and their bytes
         self._users = 0                      # open runtimes
         self._retired = False                # the last one was closed: what comes back is freed
         self._free = None
@@ -214,9 +216,12 @@ class _ResultPool:
         return np.asarray(block).view(dtype).reshape(shape)
 
     def _lock_memory(self, rt, size):
-        if size > self.limit or (size > self.at_once and self._blocks.get(size, 0) >= self._dropped.get(size, 0)):
+        proven = self._blocks.get(size, 0) < self._dropped.get(size, 0)
+        if size > self.limit or not (proven or self._new_bytes + size <= self.unproven):
             return None
         if self._held + size > self.limit:
+            if not proven:                   # no block of another size goes for a trial
+                return None
             self._drop_idle(self._held + size - self.limit)
             if self._held + size > self.limit:
                 return None
@@ -226,6 +231,8 @@ class _ResultPool:
         self._free = rt._lib.ullis_cuda_host_free
         self._held += size
         self._blocks[size] = self._blocks.get(size, 0) + 1
+        self._new.add(p.value)
+        self._new_bytes += size
         return p.value
 
     def _unlock_memory(self, addr, size):
@@ -248,6 +255,9 @@ class _ResultPool:
 
     def give_back(self, addr, size):
         with self._lock:
+            if addr in self._new:
+                self._new.discard(addr)
+                self._new_bytes -= size
             if addr is None:
                 self._dropped[size] = self._dropped.get(size, 0) + 1
             elif self._retired:
