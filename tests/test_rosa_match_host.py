@@ -76,3 +76,24 @@ def test_long_streams(oracle, rosa_host, kind, T, n):
         if way == 32 and T > 2081:
             continue
         assert np.array_equal(rosa_host(way, q, k, v, n, T), ref), (kind, way)
+
+
+@pytest.mark.parametrize("flips", [0, 1, 3])
+@pytest.mark.parametrize("T", [97, 1000, 1024, 2047, 4100])
+def test_streams_that_repeat_themselves_but_for_a_few_flips(oracle, rosa_host, T, flips):
+    """Windows that reach back to the first key, and ones that stop doing so in the middle of a piece; the queries repeat
+    the keys at once or a few steps later."""
+    n = 24 if T <= 2047 else 6
+    rng = np.random.default_rng([T, flips])
+    base = rng.integers(0, 2, (n, 100), dtype=np.uint8)
+    shift, period = rng.integers(0, 5, (n, 1)), rng.integers(2, 100, (n, 1))
+    steps = np.arange(T)[None, :]
+    q, k = (np.take_along_axis(base, (steps + s) % period, 1) for s in (shift, 0 * shift))
+    for x in (q, k):
+        for _ in range(flips):
+            x[np.arange(n), rng.integers(0, T, n)] ^= 1
+    v = rng.integers(0, 2, (n, T), dtype=np.uint8)
+    q, k, v = (pack_streams(x) for x in (q, k, v))
+    ref = oracle.rosa_qkv_streams(q, k, v, n, T)
+    for way in (32, 64, 512, 8192):
+        assert np.array_equal(rosa_host(way, q, k, v, n, T), ref), way
