@@ -343,7 +343,8 @@ rosa_coop_kernel(uint8_t* __restrict__ scratch, size_t scratch_stride, const uin
 // the other way, and up to which at all.
 struct ContextLimits {
     uint32_t easy, by_bits, by_runs;
-    uint32_t deep;   // 32-step comparisons beyond the first, and words gone back, per thread before a stream is given up
+    // 32-step comparisons beyond the first, and words gone back, per thread before a stream is given up
+    uint32_t deep_by_bits, deep_by_runs;
 };
 
 constexpr uint32_t CONTEXT_LARGE = 48;   // positions before a step in its buckets from which on the whole warp looks through them
@@ -562,6 +563,7 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
         const uint32_t* v = v_sw + s * wps;
         uint32_t* out = idx_sw + s * wps;
         uint32_t deep = 0;
+        const uint32_t most_deep = by_runs ? limits.deep_by_runs : limits.deep_by_bits;
         // Where a step's bucket lies, its best position within it (by the lanes of a warp where `together`: entries b + lane,
         // b + lane + 32, ...), and the answer.
         struct Step {
@@ -592,7 +594,7 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
         };
         auto v_bit = [&](uint32_t r1) { return r1 ? (v[r1 >> 5] >> (r1 & 31u)) & 1u : 0u; };
         auto gone = [&] {   // by vote: lanes that read the flag apart from one another could disagree, and part for good
-            if (!__any_sync(0xFFFFFFFFu, deep > limits.deep || *static_cast<volatile uint32_t*>(&sh_gone) != 0u)) return false;
+            if (!__any_sync(0xFFFFFFFFu, deep > most_deep || *static_cast<volatile uint32_t*>(&sh_gone) != 0u)) return false;
             if (lane == 0) sh_gone = 1u;
             return true;
         };
@@ -608,7 +610,10 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
                 if (lane == 0 && v_bit(best & 0xFFFFu)) atomicOr(&out_s[t >> 5], 1u << (t & 31u));
             }
         }
-        for (uint32_t row = warp + (TOGETHER ? BRUTE / 32u : 0u); row < words; row += NW) {
+        // The last rows first: they have the most keys to agree with, so a stream that has to be given up is at once.
+        const uint32_t first_row = min(TOGETHER ? BRUTE / 32u : 0u, words);
+        const uint32_t next_row = sorted ? NW : 0u - NW;
+        for (uint32_t row = sorted ? first_row + warp : words - 1u - warp; row - first_row < words - first_row; row += next_row) {
             const uint32_t i = row * 32u + lane, t = sorted && i >= BRUTE && i < T ? steps[i - BRUTE] : i;
             uint32_t r1 = 0;
             bool large = false;
@@ -624,7 +629,7 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
                         found = context::scan_runs(entries, x.b, x.e, 1u, Q, K, runs, x.run, t, deep);
                     } else {
                         best = context::scan(entries, start, x.z.first, x.z.n, t, x.z.wq, best);
-                        if (context::scan_full(best)) found = context::scan_deep(entries, x.b, x.e, 1u, Q, K, x.z.wq, t, deep, limits.deep);
+                        if (context::scan_full(best)) found = context::scan_deep(entries, x.b, x.e, 1u, Q, K, x.z.wq, t, deep, most_deep);
                     }
                     r1 = finish(x, t, found, best);
                 }
@@ -661,7 +666,7 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
                     for (uint32_t k = x.b + lane; k < x.e; k += 32u) best = context::scan_one(entries[k], t, x.z.wq, best);
                     best = __reduce_min_sync(0xFFFFFFFFu, best);
                     if (context::scan_full(best))
-                        found = __reduce_max_sync(0xFFFFFFFFu, context::scan_deep(entries, x.b + lane, x.e, 32u, Q, K, x.z.wq, t, deep, limits.deep));
+                        found = __reduce_max_sync(0xFFFFFFFFu, context::scan_deep(entries, x.b + lane, x.e, 32u, Q, K, x.z.wq, t, deep, most_deep));
                 }
                 const uint32_t bit = v_bit(finish(x, t, found, best));
                 if (lane == 0 && bit) atomicOr(&out_s[t >> 5], 1u << (t & 31u));
@@ -792,8 +797,11 @@ void launch_context(ullis_cuda_runtime* rt, const MatchCall& m, int slot, uint32
     }
     const unsigned grid = (unsigned)std::min<size_t>(rt->context_ctas[slot], m.streams);
     // A match kernel step costs about as much as 100 positions here; up to 24 the lanes are even enough without sorting
-    // the steps.  128 long comparisons per stream at most are thrown away when a stream turns out to repeat itself.
-    const ContextLimits limits{24u, 96u, 160u, 256u};
+    // the steps.  What a thread has compared when its stream turns out to repeat itself is thrown away: by bits 64 long
+    // comparisons tell (streams of clean periods 16 to 256, 2048 steps, 512 / 8192 of them: contexts 0.37 / 2.12 ms with
+    // 256, now 0.13 / 0.67), by runs 256 (with 64, 64 sequences of the default model 33.3 ms, not 29.8: streams that hardly
+    // ever change went to the match kernel).
+    const ContextLimits limits{24u, 96u, 160u, 64u, 256u};
     rt->chain(kernel, grid, NT, smem, m.q, m.k, m.v, m.idx, m.list, m.counts, m.counts + 3, m.hard, m.counts + 2, m.T, m.wps, c,
               limits, from, to);
     rt->launched(what);
