@@ -104,6 +104,11 @@ def test_layer_norm_backward(cuda_rt, rows, c):
     assert np.allclose(gb, wb, rtol=1e-4, atol=1e-4 * np.sqrt(rows))
 
 
+@pytest.mark.parametrize("c", [31, 32, 33, 64, 96, 128, 160, 256, 288, 384, 640, 768, 896, 992, 1024, 1056])
+def test_layer_norm_backward_at_every_width_in_registers(cuda_rt, c):
+    test_layer_norm_backward(cuda_rt, 11, c)
+
+
 def test_head_unigram_prior_matches_the_restatement(cuda_rt, oracle):
     d, vocab = 64, 260
     cfg = synth.train_config(d, 1, vocab, 40, 2, 96)

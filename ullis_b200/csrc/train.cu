@@ -358,7 +358,8 @@ col_final_kernel(const float* __restrict__ part, float* __restrict__ out, size_t
 // ------------------------------------------------------------ LayerNorm backward
 // gx (+)= d/dx, and the row's mean and 1 / deviation (for g_w = sum gy * xhat); one warp per row (src/model.rs:270-315).
 // N > 0: C = 32 * N, the row, its gradient and the old gx in registers (all loads in flight together, each read once); N = 0:
-// any C.  16 384 rows of 512 added to gx: 47 -> 20 us (an f32 row per column sum was written besides before).
+// any C, the same sums in the same order.  16 384 rows of 512 added to gx: 47 -> 20 us (an f32 row per column sum was
+// written besides before).
 template <int N>
 __global__ void __launch_bounds__(256)
 ln_backward_kernel(const float* __restrict__ x, const float* __restrict__ gy, const uint16_t* __restrict__ w,
@@ -422,12 +423,22 @@ ln_backward_kernel(const float* __restrict__ x, const float* __restrict__ gy, co
     }
 }
 
+// Widths of up to 1024 that a warp can take into registers whole, in steps of 32 up to 128 and of 128 above (as far as
+// LayerNorm goes forward); the others loop over the row.  us for 16 384 rows, loop / registers: 64 columns 12.0 / 6.3, 128
+// 12.1 / 8.0, 256 17.7 / 10.3, 384 23.0 / 13.6, 512 31.3 / 17.0, 640 37.2 / 23.3, 768 45.7 / 25.0, 896 52.5 / 28.2, 1024
+// 64.4 / 31.9; for 1000 rows 5.4 / 3.6 to 23.7 / 5.4.
 void ln_backward_launch(ullis_cuda_runtime* rt, const float* x, const float* gy, const uint16_t* w, float* gx, float2* stats,
                         size_t rows, size_t C, int accumulate) {
     const unsigned grid = blocks_for(rows, 8);
-    if (C == 256) rt->chain(ln_backward_kernel<8>, grid, 256, 0, x, gy, w, gx, stats, rows, C, accumulate);
-    else if (C == 512) rt->chain(ln_backward_kernel<16>, grid, 256, 0, x, gy, w, gx, stats, rows, C, accumulate);
-    else rt->chain(ln_backward_kernel<0>, grid, 256, 0, x, gy, w, gx, stats, rows, C, accumulate);
+    switch (C % 32 == 0 ? C / 32 : 0) {
+#define ULLIS_LN_BACKWARD(N) \
+    case N: rt->chain(ln_backward_kernel<N>, grid, 256, 0, x, gy, w, gx, stats, rows, C, accumulate); break
+        ULLIS_LN_BACKWARD(1); ULLIS_LN_BACKWARD(2); ULLIS_LN_BACKWARD(3); ULLIS_LN_BACKWARD(4);
+        ULLIS_LN_BACKWARD(8); ULLIS_LN_BACKWARD(12); ULLIS_LN_BACKWARD(16); ULLIS_LN_BACKWARD(20);
+        ULLIS_LN_BACKWARD(24); ULLIS_LN_BACKWARD(28); ULLIS_LN_BACKWARD(32);
+#undef ULLIS_LN_BACKWARD
+        default: rt->chain(ln_backward_kernel<0>, grid, 256, 0, x, gy, w, gx, stats, rows, C, accumulate);
+    }
     rt->launched("ln_backward");
 }
 
