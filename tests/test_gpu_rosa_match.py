@@ -53,6 +53,15 @@ def test_each_split_of_the_contexts(cuda_rt, oracle, T, B, C, left):
     assert np.array_equal(idx, oracle.rosa_qkv_batch_packed(q, k, v, B, T, C))
 
 
+# Beside those: fewer streams than SMs, the steps and streams where a shape changes, and lengths that leave an SM two or
+# one block of 256 threads (512 or 1024 threads take every stream there).
+@pytest.mark.parametrize("T,B,C,left", [(511, 2, 64, 0.9), (512, 2, 64, 0.9), (513, 1, 148, 0.9), (513, 1, 149, 0.9), (511, 3, 256, 0.9), (1023, 3, 256, 0.3),
+                                        (1023, 3, 256, 0.9), (2048, 1, 148, 0.2), (2048, 9, 256, 0.2), (2048, 9, 256, 0.9), (6000, 5, 64, 0.2), (6000, 5, 64, 0.9),
+                                        (7000, 5, 256, 0.9), (7000, 9, 256, 0.04), (8192, 3, 64, 0.9), (8192, 9, 256, 0.04)])
+def test_each_choice_of_shape(cuda_rt, oracle, T, B, C, left):
+    test_each_split_of_the_contexts(cuda_rt, oracle, T, B, C, left)
+
+
 def test_two_runtimes_of_one_device_at_lengths_of_their_own(oracle):
     """Shared memory of the context kernel grows with the length, its limit belongs to the function: a runtime at a short
     length takes nothing away from one at a long length."""

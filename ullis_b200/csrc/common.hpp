@@ -107,7 +107,7 @@ struct ullis_cuda_runtime {
     int sam_algo = ULLIS_CUDA_SAM_EULER;
     bool sam_automaton = false;         // the suffix automaton for every length (an option that names one of its forms was given)
     int match_ctas[4] = {0, 0, 0, 0};   // CTAs of the match kernel the device holds at once, per width of its sets
-    int context_ctas[3] = {};       // the same for the context kernel, for the shared memory it was last asked for
+    int context_ctas[3] = {};       // the same for the context kernel, per shape, for the shared memory it was last asked for
     size_t context_smem[3] = {};
     bool sam_coop = true;               // warp-cooperative tour / pass 2 when the stream fits shared memory
     bool sam_coop_ready = false;

@@ -779,31 +779,36 @@ struct MatchCall {   // the buffers of one call
     uint32_t T;
 };
 
+// The shapes of the context kernel: threads per stream, and whether a warp takes a large bucket together.
+enum ContextShape { CONTEXT_256, CONTEXT_512, CONTEXT_1024, CONTEXT_SHAPES };
+
 template <int NT, bool TOGETHER>
-void launch_context(ullis_cuda_runtime* rt, const MatchCall& m, int slot, uint32_t from, uint32_t to,
-                    const char* what = "rosa_context") {
+void prepare_context(ullis_cuda_runtime* rt, uint32_t T, int shape) {
     const auto kernel = rosa_context_kernel<NT, TOGETHER>;
-    const uint32_t c = context::bits_for(m.T);
-    const size_t smem = ContextLayout(m.T, c, NT / 32).total;
-    if (!rt->context_smem[slot]) {   // the attribute belongs to the function, not to this runtime: always the same value
+    const size_t smem = ContextLayout(T, context::bits_for(T), NT / 32).total;
+    if (!rt->context_smem[shape]) {   // the attribute belongs to the function, not to this runtime: always the same value
         const size_t most = ContextLayout((uint32_t)MATCH_MAX_TIME, context::bits_for((uint32_t)MATCH_MAX_TIME), NT / 32).total;
         ULLIS_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
     }
-    if (rt->context_smem[slot] != smem) {
+    if (rt->context_smem[shape] != smem) {
         int per_sm = 0;
         ULLIS_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, NT, smem));
-        rt->context_ctas[slot] = std::max(1, per_sm) * rt->sm_count;
-        rt->context_smem[slot] = smem;
+        rt->context_ctas[shape] = std::max(1, per_sm) * rt->sm_count;
+        rt->context_smem[shape] = smem;
     }
-    const unsigned grid = (unsigned)std::min<size_t>(rt->context_ctas[slot], m.streams);
+}
+
+template <int NT, bool TOGETHER>
+void launch_context(ullis_cuda_runtime* rt, const MatchCall& m, int shape, uint32_t from, uint32_t to, const char* what) {
+    const unsigned grid = (unsigned)std::min<size_t>(rt->context_ctas[shape], m.streams);
     // A match kernel step costs about as much as 100 positions here; up to 24 the lanes are even enough without sorting
     // the steps.  What a thread has compared when its stream turns out to repeat itself is thrown away: by bits 64 long
     // comparisons tell (streams of clean periods 16 to 256, 2048 steps, 512 / 8192 of them: contexts 0.37 / 2.12 ms with
     // 256, now 0.13 / 0.67), by runs 256 (with 64, 64 sequences of the default model 33.3 ms, not 29.8: streams that hardly
     // ever change went to the match kernel).
     const ContextLimits limits{24u, 96u, 160u, 64u, 256u};
-    rt->chain(kernel, grid, NT, smem, m.q, m.k, m.v, m.idx, m.list, m.counts, m.counts + 3, m.hard, m.counts + 2, m.T, m.wps, c,
-              limits, from, to);
+    rt->chain(rosa_context_kernel<NT, TOGETHER>, grid, NT, rt->context_smem[shape], m.q, m.k, m.v, m.idx, m.list, m.counts,
+              m.counts + 3, m.hard, m.counts + 2, m.T, m.wps, context::bits_for(m.T), limits, from, to);
     rt->launched(what);
 }
 
@@ -841,6 +846,57 @@ size_t stride_for(int algo, size_t T) {
                                         : sam::EulerLayout<Ix>((uint32_t)T).total;
 }
 
+// The listed streams by contexts, in the shapes that suit how many there are.  That number is known on the device only,
+// where a launch whose range it misses leaves at once: one launch for the calls where most streams had a closed form, whose
+// others are uneven (large buckets), one for the rest - a single one where both are of the same shape.
+//
+// Many streams: the shape with the most warps per SM, which shared memory decides - up to T = 4096 256 threads, for 8192
+// steps (110 KB of shared memory at 256 threads, 160 at 1024) 1024.  Fewer streams than SMs: a launch lasts as long as one
+// stream, so 1024 threads.  Between them larger blocks pay the more the fewer and the more uneven the streams are.  Context
+// kernels in us, 256 / 512 / 1024 threads, all streams listed, i.i.d. bits and bits of probabilities 0.002 to 0.99:
+//
+//     streams        128                  512                    1024                     4096
+//     T = 300     17 / 14 / 16         17 / 21 / 38           28 / 34 / 61            70 / 102 / 219
+//                 29 / 31 / 35         32 / 42 / 62           41 / 54 / 91            93 / 149 / 300
+//     T = 2048    39 / 33 / 33         53 / 58 / 79           74 / 91 / 124          216 / 298 / 453
+//                191 / 117 / 81       356 / 176 / 175        324 / 275 / 299         754 / 825 / 1016
+//     T = 6000    92 / 69 / 63        163 / 128 / 161        235 / 214 / 258         728 / 725 / 961
+//                967 / 516 / 324     1035 / 629 / 559       1382 / 947 / 904        3316 / 2691 / 2937
+//     T = 8192   112 / 78 / 69        226 / 249 / 211        426 / 451 / 388        1440 / 1681 / 1422
+//               1544 / 725 / 460     1764 / 1115 / 863      2625 / 2021 / 1358       6785 / 6422 / 4486
+//
+// One stream in eight listed, the others constant, 512 / 1024 threads: 512 listed of 4096, T = 2048 181 / 172, 1024 of 8192
+// 283 / 304, 2048 of 16 384 462 / 546; on the layers of the default model with gain N(0, 0.02) one sequence 2.8 / 2.5 ms in
+// all, four 4.0 / 3.7, 16 9.2 / 9.7, 64 29.8 / 32.2.
+void contexts(ullis_cuda_runtime* rt, const MatchCall& m) {
+    prepare_context<256, false>(rt, m.T, CONTEXT_256);
+    prepare_context<512, true>(rt, m.T, CONTEXT_512);
+    prepare_context<1024, true>(rt, m.T, CONTEXT_1024);
+    const size_t sms = (size_t)rt->sm_count;
+    int many = CONTEXT_256;
+    for (int shape = CONTEXT_512; shape < CONTEXT_SHAPES; ++shape)
+        if (rt->context_ctas[shape] << shape > rt->context_ctas[many] << many) many = shape;
+    int uneven, rest;
+    if (m.T < 512u) {   // too few steps for many warps
+        uneven = rest = m.streams <= (size_t)rt->context_ctas[CONTEXT_512] ? (int)CONTEXT_512 : many;
+    } else if (m.streams <= sms) {
+        uneven = rest = CONTEXT_1024;
+    } else if (m.T < 1024u && m.streams > 56u * sms) {   // 64 times 300 steps of the default model 5.2 ms with 256 threads alone, 5.7
+        uneven = rest = many;
+    } else {
+        uneven = std::max<int>(many, m.T >= 1024u && m.streams <= 14u * sms ? CONTEXT_1024 : CONTEXT_512);
+        rest = std::max<int>(many, m.streams <= 7u * sms ? CONTEXT_512 : CONTEXT_256);
+    }
+    const uint32_t all = ~0u, half = uneven == rest ? all : (uint32_t)(m.streams / 2) + 1u;
+    auto launch = [&](int shape, uint32_t from, uint32_t to, const char* what) {
+        if (shape == CONTEXT_256) launch_context<256, false>(rt, m, shape, from, to, what);
+        else if (shape == CONTEXT_512) launch_context<512, true>(rt, m, shape, from, to, what);
+        else launch_context<1024, true>(rt, m, shape, from, to, what);
+    };
+    launch(uneven, 0u, half, "rosa_context");
+    if (half != all) launch(rest, half, all, "rosa_context_even");
+}
+
 // The whole call without an automaton: classification, the listed streams by contexts, and by sets of lags those that
 // the contexts leave and the ones with a constant q.
 void rosa_match(ullis_cuda_runtime* rt, const uint32_t* q_sw, const uint32_t* k_sw, const uint32_t* v_sw, uint32_t* idx_sw,
@@ -858,22 +914,7 @@ void rosa_match(ullis_cuda_runtime* rt, const uint32_t* q_sw, const uint32_t* k_
     rt->chain(rosa_classify_kernel, (unsigned)((streams * CLASSIFY_LANES + 127) / 128), 128, 0, q_sw, k_sw, v_sw, idx_sw,
               streams, T, m.wps, m.list, m.counts, m.cq_list, m.counts + 1);
     rt->launched("rosa_classify");
-    // Two ways, one of which has nothing to do: how many streams are left is known on the device only.  Where most had a
-    // closed form the others are uneven too, and large buckets and many warps per stream pay; where hardly any had, few warps
-    // do, unless the streams are so few that a launch lasts as long as one of them.  Default model, ms: gain N(0, 0.02), of
-    // whose streams 12 % are left, with 1024 threads together / 512 together / 256: one sequence 2.5 / 2.8 / 4.3, four 3.7 /
-    // 4.0 / 5.9, 16 9.7 / 9.2 / 11.1, 64 32.2 / 29.8 / 31.2; gain 1 + N(0, 0.02), all left: one sequence 2.5 / 2.3 / 2.5, four
-    // 5.6 / 4.7 / 4.4, 16 18.7 / 14.8 / 12.7.
-    const uint32_t half = (uint32_t)(streams / 2) + 1u, all = ~0u;
-    // Short streams by the thousand have too few steps for many warps (64 times 300 steps 5.2 with 256 threads alone, 5.7).
-    if (streams > 1024u && (T < 512u || (T < 1024u && streams > 8192u))) {
-        launch_context<256, false>(rt, m, 2, 0u, all);
-    } else {
-        if (streams <= 2048u && T >= 1024u) launch_context<1024, true>(rt, m, 0, 0u, half);
-        else launch_context<512, true>(rt, m, 1, 0u, streams <= 1024u ? all : half);
-        if (streams > 1024u) launch_context<256, false>(rt, m, 2, half, all, "rosa_context_even");
-        else if (T >= 1024u) launch_context<512, true>(rt, m, 1, half, all, "rosa_context_even");
-    }
+    contexts(rt, m);
     if (T <= 1024u) launch_match<1>(rt, m, 0, 1024);
     else if (T <= 2048u) launch_match<2>(rt, m, 1, 1024);
     else if (T <= 4096u) launch_match<4>(rt, m, 2, 2048);
