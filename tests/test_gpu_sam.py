@@ -220,3 +220,24 @@ def test_a_cap_on_scratch_memory_does_not_ask_for_the_automaton(oracle, monkeypa
         assert "rosa_context" in ran and "rosa_match" in ran and "rosa_pass1" not in ran
     finally:
         rt.close()
+
+
+@pytest.mark.parametrize("T,C", [(8193, 48), (8193, 160), (9276, 48), (9277, 48), (9277, 160)])
+def test_lengths_beyond_the_match_without_an_automaton(oracle, T, C):
+    """One step more than the match takes, and the last and first lengths on either side of what the tour kernel's shared
+    memory holds, with no option set: few streams (their states in shared memory from the second call on) and more than
+    one round of resident CTAs."""
+    rng = np.random.default_rng([T, C])
+    pr = rng.choice([0.02, 0.3, 0.5, 0.9], (1, C))
+    q, k, v = (pack_plane((rng.random((T, C)) < pr).astype(np.uint8)) for _ in range(3))
+    rt = cuda.CudaRuntime(0)   # of its own: how many streams the last call had decides where the states go
+    try:
+        rt.kernel_timing(True)
+        for _ in range(2):
+            run_both(rt, oracle, q, k, v, 1, T, C, algos=(cuda.SAM_EULER,))
+        ran = rt.kernel_times()
+    finally:
+        rt.close()
+    assert "rosa_context" not in ran and "rosa_match" not in ran
+    assert ("rosa_coop" in ran) == (T <= 9276) and ("rosa_sam" in ran) == (T > 9276)
+    assert ("rosa_pass1_smem" in ran) == (T <= 9276 and C == 48)
