@@ -514,6 +514,9 @@ def run_cuda(args):
                          "peak_source": peak_kind, "launch_ms": dom_ms, "leading_kernel": leader,
                          "algorithmic_bytes_per_launch": alg_bytes,
                          "rosa_kernels_ms_per_layer": rosa_ms,
+                         "limited_by": "instruction issue (the kernel reads each stream once and works in shared memory; "
+                                       "`frac` sets the op's interface bytes against the copy bandwidth)"
+                         if dominant.startswith("rosa_context") else "see bound",
                          "achieved_all_rosa_kernels": alg_bytes / (rosa_ms * 1e-3) / 1e9 if rosa_ms > 0 else 0.0},
             "tensor_core": {"flop_per_token": flops_per_token, "tflops_whole_step": flops_per_token * value / world / 1e12,
                             "frac_of_sustained_peak": flops_per_token * value / world / 1e12 /

@@ -62,8 +62,9 @@ enum {
  *         backend (validation mode, much slower). */
 enum { ULLIS_CUDA_MODE_FAST = 0, ULLIS_CUDA_MODE_EXACT = 1 };
 
-/* Suffix-automaton schedule. Both give identical idx.
- * EULER : O(T log T) per stream for any input (default).
+/* Schedule of the ROSA match. Both give identical idx.
+ * EULER : without an automaton up to T = 8192, a suffix automaton in
+ *         O(T log T) per stream beyond (default).
  * EAGER : the reference's per-step chain stamping, O(T^2) on constant streams. */
 enum { ULLIS_CUDA_SAM_EULER = 0, ULLIS_CUDA_SAM_EAGER = 1 };
 
@@ -109,9 +110,9 @@ ULLIS_CUDA_API int32_t ullis_cuda_runtime_kernel_timing(ullis_cuda_runtime* rt, 
 ULLIS_CUDA_API int32_t ullis_cuda_runtime_kernel_time(ullis_cuda_runtime* rt, const char* name, float* total_ms,
                                                       uint32_t* launches);
 ULLIS_CUDA_API int32_t ullis_cuda_runtime_kernel_names(ullis_cuda_runtime* rt, char* buf, size_t len, size_t* needed);
-/* How the last suffix-automaton call on `rt` (op-level or inside a model forward: the last layer's) split its
- * streams: `automaton` streams went through the automaton kernels, `constant_q` were settled by the
- * constant-query closed form, and the rest of `total` by the other closed forms (constant key or value bits).
+/* How the last ROSA match on `rt` (op-level or inside a model forward: the last layer's) split its streams:
+ * `automaton` streams had no closed form (they went through the context, match or automaton kernels), `constant_q` were
+ * settled by the constant-query one, and the rest of `total` by the other closed forms (constant key or value bits).
  * No counterpart in the reference, which runs every stream through RosaSam.  Synchronises. */
 ULLIS_CUDA_API int32_t ullis_cuda_runtime_sam_counts(ullis_cuda_runtime* rt, uint64_t* total, uint64_t* automaton,
                                                      uint64_t* constant_q);
@@ -189,14 +190,14 @@ ULLIS_CUDA_API int32_t ullis_cuda_model_phase_ms(ullis_cuda_model* model, float 
 
 /* ----------------------------------------------------------------- generate
  * Incremental generation with the state on the device (HeronGenerateState,
- * src/model.rs:2433-2454): per layer one suffix automaton per (sequence,
- * channel) plus the ROSA and CMix time-shift inputs.  The reference generates
+ * src/model.rs:2433-2454): per layer the bit histories of one RosaSam per
+ * (sequence, channel) plus the ROSA and CMix time-shift inputs.  The reference generates
  * one sequence; here `batch` independent sequences advance in lock step.
  * Arithmetic is the reference's (CUDA cores, its summation order), whatever
  * the runtime's mode: the logits of step t are bit-identical to row t of
  * ullis_cuda_model_logits in ULLIS_CUDA_MODE_EXACT (src/model.rs:4991-5004). */
 
-/* UllisHeron::generate_state (src/model.rs:2691-2715): empty automata sized for
+/* UllisHeron::generate_state (src/model.rs:2691-2715): empty histories sized for
  * the model's context_len, no time-shift history, time 0.  The state borrows
  * `model`; destroy it before the model. */
 ULLIS_CUDA_API int32_t ullis_cuda_generate_state_create(ullis_cuda_model* model, size_t batch,

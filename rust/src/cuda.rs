@@ -878,7 +878,7 @@ impl Drop for CudaHeron<'_> {
     }
 }
 
-/// `HeronGenerateState` (`src/model.rs:2433-2454`) with the automata on the device.
+/// `HeronGenerateState` (`src/model.rs:2433-2454`) with its histories on the device.
 #[derive(Debug)]
 pub struct CudaGenerateState<'m, 'rt> {
     raw: *mut sys::ullis_cuda_generate_state,
@@ -922,7 +922,7 @@ impl Drop for CudaGenerateState<'_, '_> {
     }
 }
 
-/// `streams` independent `RosaSam` automata (`src/rosa.rs:55-176`) kept on the device between calls: the
+/// `streams` independent `RosaSam` states (`src/rosa.rs:55-176`) kept on the device between calls: the
 /// per-layer state of a generate state at op level.
 #[derive(Debug)]
 pub struct CudaRosaPushers<'rt> {

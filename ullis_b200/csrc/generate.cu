@@ -1,15 +1,16 @@
-// Incremental generation: one token per sequence and call, with the automata
-// of every (sequence, layer, channel) kept on the device between calls
-// (reference UllisHeron::generate_state / generate_step, src/model.rs:2691-2753;
+// Incremental generation: one token per sequence and call, with the bit
+// histories of every (sequence, layer, channel) kept on the device between
+// calls (reference UllisHeron::generate_state / generate_step, src/model.rs:2691-2753;
 // per-block forward_one src/model.rs:2243-2262, ROSA 1320-1352, CMix 1003-1016).
 //
 // A step is a handful of [batch, d_model] row operations, so it runs on the
 // CUDA cores in the reference's summation order: the logits of step t
 // are bit-identical to row t of the one-shot forward in EXACT mode, which is
 // what the reference's own test asserts (src/model.rs:4991-5004).  The whole
-// step is one cooperative kernel (generate_step.cuh) where the shape allows;
-// otherwise its ~90 small launches are replayed as one CUDA graph (two
-// graphs: before and after the first token, which has no time-shift history).
+// step is one kernel of thread-block clusters (generate_step.cuh) where the
+// shape allows; otherwise its ~90 small launches are replayed as one CUDA graph
+// (two graphs: before and after the first token, which has no time-shift
+// history).
 // A stream's automaton is not kept: a push is answered from the bit histories
 // (gen_push.cuh).
 #include "generate.hpp"
@@ -313,7 +314,7 @@ void ullis_cuda_generate_state::step(const uint32_t* tokens, float* logits_out) 
     std::memcpy(h_tokens, tokens, batch * 4);
     h_tokens[batch] = (uint32_t)time;
     const int has_prev = time != 0;
-    // From here on the device-side automata, v history and time-shift inputs may have moved on by one position
+    // From here on the device-side histories and time-shift inputs may have moved on by one position
     // while `time` has not: a failure below leaves the state out of step with itself, and a retry would push the
     // same position twice.  The state stays refused until reset() (which rebuilds it from scratch).
     struct Poison {

@@ -5,9 +5,9 @@
 // Up to 8192 steps a stream needs no automaton (rosa_match below): every step
 // is looked up by itself (rosa_context.cuh) or in sets of lags
 // (rosa_match.cuh), so no launch lasts as long as a stream's chain of steps.
-// 64 sequences x 512 channels x 2048 steps: 1.8 ms on evenly spread bits where
-// the automaton took 11.3, 0.6 to 1.4 ms against 2.6 on the benchmark model's
-// layers; 1 sequence 0.07 to 0.2 ms against 0.7.
+// 64 sequences x 512 channels x 2048 steps: 1.5 ms on evenly spread bits where
+// the automaton took 11.3, 0.79 against 2.10 per layer of the benchmark model;
+// 1 sequence 0.105 against 0.62.
 //
 // Longer streams, and calls that ask for one of its forms, run the suffix
 // automaton: one thread per (sequence, channel) stream, automaton state in a

@@ -553,7 +553,7 @@ class CudaRuntime:
         self._check(self._lib.ullis_cuda_runtime_wait_selftest(self._h, C.c_uint32(polls)))
 
     def sam_counts(self) -> dict:
-        """Streams of the last suffix-automaton call: total, through the automaton, through the constant-q form."""
+        """Streams of the last ROSA match: total, without a closed form, through the constant-q form."""
         t, a, q = C.c_uint64(0), C.c_uint64(0), C.c_uint64(0)
         self._check(self._lib.ullis_cuda_runtime_sam_counts(self._h, C.byref(t), C.byref(a), C.byref(q)))
         return {"total": int(t.value), "automaton": int(a.value), "constant_q": int(q.value)}
@@ -698,7 +698,7 @@ class CudaHeron:
 
 
 class CudaGenerateState:
-    """HeronGenerateState (src/model.rs:2433-2454) on the device: one automaton per
+    """HeronGenerateState (src/model.rs:2433-2454) on the device: the bit histories of one RosaSam per
     (sequence, layer, channel) and the time-shift inputs; borrowed model."""
 
     def __init__(self, model: CudaHeron, batch: int = 1):
@@ -737,7 +737,7 @@ class CudaGenerateState:
 
 
 class CudaRosaPushers:
-    """`streams` RosaSam automata (src/rosa.rs:55-176) on the device; push() is RosaSam::push for every stream,
+    """`streams` RosaSam states (src/rosa.rs:55-176) on the device; push() is RosaSam::push for every stream,
     once per row of q / k / v ([steps, streams] of 0 / 1), and returns idx in the same shape."""
 
     def __init__(self, rt: CudaRuntime, streams: int, capacity: int):
