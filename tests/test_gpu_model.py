@@ -183,3 +183,22 @@ def test_per_kernel_device_times(cuda_rt, case):
     assert cuda_rt.kernel_times() == {}
     cuda_rt.kernel_timing(False)
     m.close()
+
+
+def test_a_call_that_fails_leaves_nothing_in_flight(cuda_rt):
+    """Copies of a failed call may touch page-locked memory that its caller has back: the error comes when the stream is idle,
+    here behind a forward that was only enqueued."""
+    import torch
+    m = cuda.CudaHeron(cuda_rt, synth.heron_checkpoint("default", batch_size=16))
+    tokens = synth.zipf_tokens(5, 16 * 2048, m.vocab_size)
+    m.upload_tokens(tokens, tokens, 16, 2048)
+    m.enqueue_forward_ce(cuda.CE_NO_IGNORE, 16, 2048)
+    m.read_loss()
+    stream = torch.cuda.ExternalStream(cuda_rt.stream)
+    m.enqueue_forward_ce(cuda.CE_NO_IGNORE, 16, 2048)
+    assert not stream.query()                                    # 9 ms of kernels, enqueued in about one
+    with pytest.raises(cuda.UllisCudaError):
+        cuda_rt.layer_norm(np.zeros(0, np.float32), np.zeros(0, np.uint16), np.zeros(0, np.uint16), 1, 0)
+    assert stream.query()
+    m.read_loss()
+    m.close()

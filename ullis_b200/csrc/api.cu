@@ -25,19 +25,23 @@ int32_t guard(ullis_cuda_runtime* rt, F&& body) {
         set_global_error("runtime handle is null");
         return ULLIS_CUDA_ERR_ARG;
     }
+    // Nothing of a call that fails stays in flight: its copies may run between page-locked memory of the caller, which is
+    // the caller's again, and the library's buffers.
+    const auto failed = [&](int32_t code, const char* msg) {
+        rt->last_error = msg;
+        if (rt->stream) cudaStreamSynchronize(rt->stream);
+        return code;
+    };
     try {
         rt->bind();
         body();
         return ULLIS_CUDA_OK;
     } catch (const Error& e) {
-        rt->last_error = e.msg;
-        return e.code;
+        return failed(e.code, e.msg.c_str());
     } catch (const std::bad_alloc&) {
-        rt->last_error = "host allocation failed";
-        return ULLIS_CUDA_ERR_NOMEM;
+        return failed(ULLIS_CUDA_ERR_NOMEM, "host allocation failed");
     } catch (const std::exception& e) {
-        rt->last_error = e.what();
-        return ULLIS_CUDA_ERR_ARG;
+        return failed(ULLIS_CUDA_ERR_ARG, e.what());
     }
 }
 
@@ -67,8 +71,8 @@ T* stage(ullis_cuda_runtime* rt, int slot, const T* host, size_t count) {
 }
 
 // The inputs of an op-level call.  Small ones are gathered and cross the link in one copy (send()): seventeen copies
-// of a few KB from pageable memory were 80 us of a ROSA block call of 260.  The call synchronises before it returns,
-// so the memory is free again for the next one.
+// of a few KB from pageable memory were 80 us of a ROSA block call of 260.  The call synchronises before it returns
+// (guard() where it fails), so the memory is free again for the next one.
 struct Inputs {
     ullis_cuda_runtime* rt;
     explicit Inputs(ullis_cuda_runtime* r) : rt(r) {
@@ -78,8 +82,6 @@ struct Inputs {
             rt->inputs_host = static_cast<uint8_t*>(p);
             rt->inputs_dev.ensure(ullis_cuda_runtime::INPUTS_BYTES);
         }
-        // a call that failed half way did not wait for its copy
-        if (rt->inputs_sent && cudaStreamQuery(rt->stream) != cudaSuccess) rt->sync();
         rt->inputs_used = rt->inputs_sent = 0;
     }
     template <typename T>
@@ -378,7 +380,6 @@ int32_t ullis_cuda_runtime_create(int32_t device, ullis_cuda_runtime** out) {
 void ullis_cuda_runtime_destroy(ullis_cuda_runtime* rt) {
     if (!rt) return;
     cudaSetDevice(rt->device);
-    if (rt->inputs_host) cudaFreeHost(rt->inputs_host);
     for (ullis_cuda_runtime* c : rt->children) {
         c->dev_status = nullptr;    // the parent's
         c->host_status = nullptr;
@@ -395,6 +396,7 @@ void ullis_cuda_runtime_destroy(ullis_cuda_runtime* rt) {
         cudaStreamSynchronize(rt->side_stream);
         cudaStreamDestroy(rt->side_stream);
     }
+    if (rt->inputs_host) cudaFreeHost(rt->inputs_host);   // behind the wait
     if (rt->side_fork) cudaEventDestroy(rt->side_fork);
     if (rt->side_join) cudaEventDestroy(rt->side_join);
     if (rt->dev_status) cudaFree(rt->dev_status);
