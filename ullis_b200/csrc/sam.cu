@@ -855,7 +855,7 @@ size_t stride_for(int algo, size_t T) {
 // stream, so 1024 threads.  Between them larger blocks pay the more the fewer and the more uneven the streams are.  Context
 // kernels in us, 256 / 512 / 1024 threads, all streams listed, i.i.d. bits and bits of probabilities 0.002 to 0.99:
 //
-//     streams        128                  512                    1024                     4096
+//     streams         96 *                512                    1024                     4096           (* T = 6000: 128)
 //     T = 300     17 / 14 / 16         17 / 21 / 38           28 / 34 / 61            70 / 102 / 219
 //                 29 / 31 / 35         32 / 42 / 62           41 / 54 / 91            93 / 149 / 300
 //     T = 2048    39 / 33 / 33         53 / 58 / 79           74 / 91 / 124          216 / 298 / 453
