@@ -37,6 +37,7 @@ __device__ __forceinline__ uint32_t window(const uint32_t* words, uint32_t last,
 // Steps on which the histories that end at step i of the queries and at position r of the keys agree, from n on.
 __device__ __forceinline__ uint32_t agreement(const uint32_t* q, const uint32_t* k, uint32_t last, uint32_t q_word,
                                               uint32_t k_word, uint32_t i, uint32_t r, uint32_t n) {
+#pragma unroll 1
     while (n <= r) {
         const uint32_t same = (uint32_t)__clz((int)(window(q, last, q_word, i - n) ^ window(k, last, k_word, r - n)));
         n += same;
@@ -55,6 +56,7 @@ __device__ __forceinline__ uint32_t agreement(const uint32_t* q, const uint32_t*
 __device__ __forceinline__ uint32_t search_runs(const uint32_t* q, const uint32_t* k, uint32_t i, uint32_t wq, uint32_t k_word) {
     const uint32_t lane = threadIdx.x & 31u, last = i >> 5, q_word = wq >> (31u - (i & 31u));
     uint32_t n_run = (i & 31u) + 1u;
+#pragma unroll 1
     for (uint32_t w1 = last;; w1 -= 32u) {                       // words of c below w1
         const uint32_t y = lane < w1 ? q[w1 - 1u - lane] ^ ~wq : 0u, full = __ballot_sync(0xFFFFFFFFu, y == ~0u);
         if (full == ~0u) { n_run += 1024u; continue; }
@@ -63,6 +65,7 @@ __device__ __forceinline__ uint32_t search_runs(const uint32_t* q, const uint32_
         break;
     }
     uint32_t longest = 0, position = 0, before = 0;              // before: run of c that ends at the last word so far
+#pragma unroll 1
     for (uint32_t w0 = 0; w0 <= last; w0 += 32u) {
         const uint32_t w = w0 + lane;
         const uint32_t x = w < last ? k[w] ^ ~wq : w == last ? (k_word ^ ~wq) & ((1u << (i & 31u)) - 1u) : 0u;
@@ -95,9 +98,11 @@ __device__ __forceinline__ uint32_t search(const uint32_t* q, const uint32_t* k,
         if (lag) return lag;
     }
     uint32_t best = 0, before = 0;      // agreement << 26 | word of the position, the bit within the word is the lane
+#pragma unroll 1
     for (uint32_t w0 = 0; w0 <= last; w0 += 32u) {
         const uint32_t mine = w0 + lane < last ? k[w0 + lane] : w0 + lane == last ? k_word : 0u;
         const uint32_t n_words = min(32u, last + 1u - w0);
+#pragma unroll 2
         for (uint32_t j = 0; j < n_words; ++j) {
             const uint32_t w = w0 + j, word = __shfl_sync(0xFFFFFFFFu, mine, (int)j);
             uint32_t n = (uint32_t)__clz((int)(wq ^ __funnelshift_l(before, word, 31u - lane)));
@@ -115,6 +120,7 @@ __device__ __forceinline__ uint32_t search(const uint32_t* q, const uint32_t* k,
     }
     // whole windows agree: count on from there
     uint32_t longest = 0, position = 0;
+#pragma unroll 1
     for (uint32_t r = lane; r < i; r += 32u) {
         if (window(k, last, k_word, r) != wq) continue;
         const uint32_t n = agreement(q, k, last, q_word, k_word, i, r, 32u);
@@ -130,6 +136,7 @@ constexpr uint32_t DEEP = ~0u;
 __device__ __forceinline__ uint32_t search_alone(const uint32_t* k, uint32_t i, uint32_t wq, uint32_t k_word) {
     const uint32_t last = i >> 5;
     uint32_t best = 0, before = 0, next = last ? k[0] : k_word;
+#pragma unroll 1
     for (uint32_t w = 0; w <= last; ++w) {
         const uint32_t word = next, n_bits = w == last ? i & 31u : 32u;
         next = w + 1u < last ? k[w + 1u] : k_word;

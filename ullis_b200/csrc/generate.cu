@@ -25,6 +25,7 @@
 
 #include "generate_step.cuh"
 #include "kernels.hpp"
+#include "linear_tc.hpp"
 
 namespace ullis {
 namespace {
@@ -206,8 +207,15 @@ void ullis_cuda_generate_state::prepare_one_kernel() {
     for (uint32_t c = gen::MAX_CLUSTER; c >= 1 && best_rounds > 1; c /= 2) {
         if (m->d % (c * 32) || m->ffn % (c * 4)) continue;
         for (uint32_t g = 1; g <= gen::MAX_GROUP && best_rounds > 1; g *= 2) {
-            const size_t smem = gen::step_smem_bytes(g, m->d, m->ffn, m->d / c), want = (batch + g - 1) / g;
-            if (smem > MOST_SMEM) break;
+            // packed weights stay where they are if there is no room for them beside the ring
+            bool staged = true;
+            uint32_t stages = gen::ring_stages(g, (uint32_t)m->d, (uint32_t)m->ffn, c, true, MOST_SMEM);
+            if (gen::Layout(g, (uint32_t)m->d, (uint32_t)m->ffn, c, stages, true).total > MOST_SMEM) {
+                staged = false;
+                stages = gen::ring_stages(g, (uint32_t)m->d, (uint32_t)m->ffn, c, false, MOST_SMEM);
+            }
+            const size_t smem = gen::Layout(g, (uint32_t)m->d, (uint32_t)m->ffn, c, stages, staged).total, want = (batch + g - 1) / g;
+            if (smem > MOST_SMEM || stages > gen::MAX_STAGES) break;
             const void* kernel = kernel_for(g);
             ULLIS_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MOST_SMEM));
             ULLIS_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
@@ -219,7 +227,7 @@ void ullis_cuda_generate_state::prepare_one_kernel() {
             const size_t rounds = (want + clusters - 1) / clusters;
             if (rounds >= best_rounds) continue;
             best_rounds = rounds;
-            cluster = c; group = g; step_kernel = kernel; step_smem = smem;
+            cluster = c; group = g; step_stages = stages; step_staged = staged; step_kernel = kernel; step_smem = smem;
             step_grid = (unsigned)(std::min<size_t>(want, (size_t)clusters) * c);
         }
     }
@@ -228,11 +236,16 @@ void ullis_cuda_generate_state::prepare_one_kernel() {
     for (size_t l = 0; l < m->layers; ++l) {
         const LayerWeights& L = m->blocks[l];
         auto packed = [](const PackedWeights& w) { return gen::Packed{w.bits, w.scale, w.bias}; };
-        layers[l] = gen::Layer{L.ln3.weight, L.ln3.bias, {L.x_q, L.x_k, L.x_v}, L.e, L.ln2.weight, L.ln2.bias, L.ffn_x_k, L.value,
+        layers[l] = gen::Layer{L.ln3.weight, L.ln3.bias, {L.x_q, L.x_k, L.x_v}, L.e, L.ln2.weight, L.ln2.bias, L.ffn_x_k,
                                {packed(L.q), packed(L.k), packed(L.v)}, packed(L.o), gen::Packed{L.key.bits, L.key.scale, nullptr}};
     }
+    std::vector<CUtensorMap> values;
+    const uint32_t own = (uint32_t)m->d / cluster, slabs = group * own == gen::VALUE_OUT ? (uint32_t)m->ffn / gen::SLAB : own <= gen::MAX_BOX ? gen::PIECE / gen::SLAB : 1u;
+    for (size_t l = 0; l < m->layers; ++l) values.push_back(tc::slab_map(m->blocks[l].value, m->d, m->ffn, std::min(own, gen::MAX_BOX), slabs));
     step_layers.ensure(layers.size() * sizeof(gen::Layer) + 16);
+    step_values.ensure(values.size() * sizeof(CUtensorMap));
     rt->h2d(step_layers.get(), layers.data(), layers.size() * sizeof(gen::Layer));
+    rt->h2d(step_values.get(), values.data(), values.size() * sizeof(CUtensorMap));
     rt->sync();
 }
 
@@ -279,9 +292,13 @@ void ullis_cuda_generate_state::launch_one_kernel(float* logits_to) {
     float* history = static_cast<float*>(prev.get());
     gen::Step p{};
     p.layers = static_cast<const gen::Layer*>(step_layers.get());
+    p.values = static_cast<const CUtensorMap*>(step_values.get());
+    p.staged = step_staged;
+    p.status = rt->host_status;
     p.n_layers = (uint32_t)m->layers; p.rows = (uint32_t)batch; p.d = (uint32_t)m->d; p.ffn = (uint32_t)m->ffn;
     p.vocab = (uint32_t)m->vocab; p.time = (uint32_t)time;
-    p.group = group;
+    p.stages = step_stages;
+    p.minus_zero = -0.0f;
     p.tokens = h_tokens;
     p.embedding = m->embedding;
     p.ln0_w = m->blocks[0].ln0.weight; p.ln0_b = m->blocks[0].ln0.bias;
@@ -291,7 +308,7 @@ void ullis_cuda_generate_state::launch_one_kernel(float* logits_to) {
     p.prev_out = history + (~time & 1) * half;
     p.push = histories();
     p.logits = logits_to;
-    rt->host_status[0] = ULLIS_DEV_OK;   // this kernel reports nothing
+    rt->host_status[0] = ULLIS_DEV_OK;   // the kernel writes there itself
     void* args[] = {&p};
     cudaLaunchAttribute attr;
     const cudaLaunchConfig_t cfg = step_config(&attr, step_grid, cluster, step_smem);

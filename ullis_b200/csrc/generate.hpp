@@ -17,8 +17,9 @@ struct ullis_cuda_generate_state {
     unsigned step_grid = 0;
     size_t step_smem = 0;
     const void* step_kernel = nullptr;
-    uint32_t group = 1, cluster = 1;             // sequences of a cluster, CTAs of a cluster
-    ullis::DeviceBuffer step_layers;
+    uint32_t group = 1, cluster = 1, step_stages = 0;   // sequences of a cluster, CTAs of a cluster, pieces of the value weights in flight
+    bool step_staged = false;                    // packed weights through shared memory
+    ullis::DeviceBuffer step_layers, step_values;
     // activations of one step (owned here, so that a captured graph's pointers stay valid)
     ullis::DeviceBuffer ids, x, a, bq, bk, bv, wide, logits;
     uint32_t* h_tokens = nullptr;   // pinned staging of the step's inputs / outputs

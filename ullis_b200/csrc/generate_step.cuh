@@ -1,12 +1,12 @@
 // One generation step - every layer, the head - as ONE kernel, a thread-block cluster per handful of sequences.
 //
-// A step is a chain of short stages, each bound by the latency of one f32 sum that the reference adds in order
-// (LayerNorm: 2 d additions, Q / K / V, O and key: d, CMix value: dim_ffn).  As 88 kernels it took 6.5 us per kernel, two
-// thirds of that launch, ramp and the first loads; as one kernel over the whole device with grid barriers a hand-over
-// (barrier, then the row from L2) still cost 4 600 cycles, more than most of the sums.  Sequences are independent, so
-// they need no device-wide hand-over: the CTAs of a cluster split the channels of their sequences, keep the residual rows,
-// the ROSA output and the CMix hidden in shared memory, all of it in every CTA, and write their share into all of them
-// (st.shared::cluster) before a cluster barrier.  Four barriers per layer:
+// A step is a chain of short stages, each bound by f32 sums that the reference adds in order (LayerNorm: 2 d additions,
+// Q / K / V, O and key: d, CMix value: dim_ffn).  As 88 kernels it took 6.5 us per kernel, two thirds of that launch, ramp
+// and the first loads; as one kernel over the whole device with grid barriers a hand-over (barrier, then the row from L2)
+// still cost 4 600 cycles, more than most of the sums.  Sequences are independent, so they need no device-wide hand-over:
+// the CTAs of a cluster split the channels of their sequences, keep the residual rows, the ROSA output and the CMix hidden
+// in shared memory, all of it in every CTA, and write their share into all of them (st.shared::cluster) before a cluster
+// barrier.  Four barriers per layer:
 //
 //   A  LayerNorm, mixes, Q / K / V and the ROSA push of a CTA's channels
 //   B  O, added to the residual rows
@@ -14,9 +14,19 @@
 //   D  value, added to the residual rows
 //
 // A LayerNorm is redone by every CTA (a chain costs the same once or sixteen times over).  What a stage reads from global
-// memory does not depend on the step's values; it is asked for a stage ahead (weights of D into a shared-memory ring, the
-// rest into L1), because one trip to L2 takes as long as 400 additions.
-// All sums are the reference's, one thread per output, so the logits are those of the kernels one by one, bit for bit.
+// memory does not depend on the step's values: the weights are copied to shared memory a stage ahead by the copy engine (with
+// cp.async the issuing threads stood still for 4 500 cycles per layer), and LayerNorm's vectors and the time-shift history go
+// to registers before its sums.
+//
+// With one row per thread and output a sum takes 4.4 to 5 cycles per term, the latency of the addition; with more rows and
+// outputs in a cluster it is issue slots and shared-memory reads that count.  Therefore the rows of a cluster lie side by side
+// per channel, a thread adds up all of them for J outputs at once, and two rows take one fma.f32x2 (512 inputs, 1024 sums of
+// a CTA: one output and two scalar rows per thread 22 000 cycles, four outputs and a pair of rows 11 000).
+// All layers run the same code, and what of it does not fit the instruction cache of an SM is fetched again in every one (with
+// a copy of the sums per stage, 160 KB in all, 1 000 misses per layer).  So A, B and C are three turns of one loop, and loops are
+// unrolled only as far as a sum needs it; a function that is not inlined costs more (550 cycles per call).
+// All sums are the reference's, so the logits are those of the kernels one by one, bit for bit: x * +-1 is exact, so
+// fma(x, +-1, sum) rounds what sum +- x does.
 // The time-shift history is double-buffered, since every CTA reads a row of it that one of them writes anew.
 #pragma once
 #include <cuda_fp16.h>
@@ -24,6 +34,7 @@
 
 #include "common.hpp"
 #include "gen_push.cuh"
+#include "tc_ptx.cuh"
 
 namespace ullis {
 namespace gen {
@@ -33,13 +44,16 @@ struct Packed {
     const uint16_t *scale, *bias;
 };
 struct Layer {
-    const uint16_t *ln3_w, *ln3_b, *mix[3], *e, *ln2_w, *ln2_b, *ffn_mix, *value;
+    const uint16_t *ln3_w, *ln3_b, *mix[3], *e, *ln2_w, *ln2_b, *ffn_mix;
     Packed qkv[3], o, key;
 };
 struct Step {   // kernel arguments
     const Layer* layers;
+    const CUtensorMap* values;                              // of the layers' value matrices by slabs (tc::slab_map)
     uint32_t n_layers, rows, d, ffn, vocab, time;
-    uint32_t group;                                         // sequences of a cluster
+    uint32_t stages;                                        // of the ring of D
+    uint32_t staged;                                        // packed weights go through shared memory
+    float minus_zero;                                       // -0.0f, unknown to the compiler (value_piece)
     const uint32_t* tokens;                                 // page-locked host memory
     const uint16_t *embedding, *ln0_w, *ln0_b, *ln_out_w, *ln_out_b;
     Packed head;
@@ -47,43 +61,79 @@ struct Step {   // kernel arguments
     float* prev_out;
     push::Histories push;
     float* logits;
+    uint32_t* status;                                       // page-locked host memory
 };
 
-constexpr uint32_t THREADS = 256, WARPS = THREADS / 32, MAX_GROUP = 4, MAX_CLUSTER = 16, TURN = 128;
-// D: 32 outputs of a warp; a row of a piece is 16 bytes longer than its values, so that the lanes (an output each) meet no
-// bank conflict
-constexpr uint32_t VALUE_OUT = 32, PIECE = 128, PIECE_PITCH = PIECE * 2 + 16, PRODUCTS = 256, PRODUCT_PITCH = PRODUCTS + 4;
+constexpr uint32_t THREADS = 256, WARPS = THREADS / 32, MAX_GROUP = 4, MAX_CLUSTER = 16;
+// D: 32 outputs of a warp.  Weights come in pieces of 128 inputs of all of a CTA's outputs: slab by slab of 64 inputs, output by
+// output, and 16-byte granule g of output o lies at g ^ (o % 8) (the copy engine's 128-byte swizzle: the lanes, an output each,
+// meet no bank conflict).  A piece is one copy, since each of them holds the asking warp, and the shared memory it works on, up.  A CTA with 32 sums in all has one warp add what the others have multiplied, PRODUCTS inputs at a time.
+constexpr uint32_t VALUE_OUT = 32, PIECE = 128, SLAB = 64, BOX_BYTES = SLAB * VALUE_OUT * 2, PRODUCTS = PIECE, PRODUCT_PITCH = PRODUCTS + 4, PRODUCT_SLOTS = 3;
+constexpr uint32_t VALUE_BODY = 8;   // granules of the loop body of D
+constexpr uint32_t MAX_STAGES = 32;
 
-// Pieces of PIECE inputs in flight in D, by the bytes of one (the weights of `own` outputs); a CTA with one sum has them all.
-__host__ __device__ inline uint32_t ring_stages(uint32_t group, uint32_t own, uint32_t ffn) {
-    return group * own == VALUE_OUT ? ffn / PIECE : own <= 32 ? 8 : own <= 64 ? 6 : 4;
-}
-// Shared memory: ring | x [group][d] | y [group][d] | in [3][group][d] | act [group][ffn] | products [2][32][pitch]
-inline size_t step_smem_bytes(size_t group, size_t d, size_t ffn, size_t own) {
-    return ring_stages((uint32_t)group, (uint32_t)own, (uint32_t)ffn) * own * PIECE_PITCH + group * (5 * d + ffn) * 4 +
-           (group * own == VALUE_OUT ? 2 * VALUE_OUT * PRODUCT_PITCH * 4 : 0);
+__host__ __device__ inline uint32_t most(uint32_t a, uint32_t b) { return a > b ? a : b; }
+// Floats of a row: the residual row, the first input (where the squares of LayerNorm lie before it), and one region for the
+// CMix hidden (C, D), the ROSA output (A, B) and the other two inputs (A).
+__host__ __device__ inline uint32_t row_floats(uint32_t d, uint32_t ffn) { return 2u * d + most(ffn, 3u * d); }
+
+// How a CTA's shared memory is laid out: ring | products | rows | bits of q, k and v | Q/K/V or key weights | O weights.
+struct Layout {
+    uint32_t ring, products, rows, bits, wide, o, total;   // byte offsets
+    __host__ __device__ Layout(uint32_t group, uint32_t d, uint32_t ffn, uint32_t ctas, uint32_t stages, bool staged) {
+        const uint32_t own = d / ctas;
+        ring = 0;
+        products = ring + stages * own * (PIECE * 2u);
+        rows = products + (group * own == VALUE_OUT ? PRODUCT_SLOTS * VALUE_OUT * PRODUCT_PITCH * 4u : 0u);
+        bits = rows + group * row_floats(d, ffn) * 4u;
+        wide = bits + 3u * group * own;
+        o = wide + (staged ? most(3u * own, ffn / ctas) * (d / 8u) : 0u);
+        total = o + (staged ? own * (d / 8u) : 0u) + 1024u;   // the ring starts on a border of 1024 bytes
+    }
+};
+// Pieces of D's weights in flight: as many as fit, up to 8; a CTA with one sum per lane of a warp has them all.
+inline uint32_t ring_stages(uint32_t group, uint32_t d, uint32_t ffn, uint32_t ctas, bool staged, size_t limit) {
+    if (group * d / ctas == VALUE_OUT) return ffn / PIECE;
+    for (uint32_t s : {8u, 6u, 4u, 3u})
+        if (Layout(group, d, ffn, ctas, s, staged).total <= limit) return s;
+    return 2u;
 }
 
 __device__ __forceinline__ float h2f(uint16_t b) { return __half2float(__ushort_as_half(b)); }
 
 __device__ __forceinline__ uint32_t cluster_size() { uint32_t n; asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(n)); return n; }
 __device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
-__device__ __forceinline__ void cluster_barrier() {   // every thread of the cluster; orders the shared-memory writes
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+// Every thread of the cluster; orders the shared-memory writes.  What lies between the two halves must not touch memory that
+// another CTA writes in this stage or reads in the next.
+__device__ __forceinline__ void cluster_arrive() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 }
-// n floats (a multiple of 4) of each of `rows` rows, `pitch` apart, from this CTA's shared memory to the same place in
-// every CTA of the cluster
+__device__ __forceinline__ void cluster_wait() {
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// n floats (a multiple of 4) of each of `rows` rows, `pitch` apart, from this CTA's shared memory to the same place in every
+// other CTA of the cluster, a CTA per warp at a time.
 __device__ __forceinline__ void share_with_cluster(const float* from, uint32_t rows, uint32_t pitch, uint32_t n) {
-    const uint32_t quads = n / 4u, per_cta = rows * quads, ctas = cluster_size();
-    for (uint32_t i = threadIdx.x; i < per_cta * ctas; i += THREADS) {
-        const uint32_t cta = i / per_cta, q = i % per_cta;
-        const float* src = from + (q / quads) * pitch + q % quads * 4u;
-        const float4 v = *reinterpret_cast<const float4*>(src);
-        uint32_t to;
-        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"((uint32_t)__cvta_generic_to_shared(src)), "r"(cta));
-        if (cta != cluster_rank())
-            asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+    const uint32_t ctas = cluster_size(), me = cluster_rank(), lane = threadIdx.x & 31u;
+#pragma unroll 1
+    for (uint32_t cta = threadIdx.x >> 5; cta < ctas; cta += WARPS) {
+        if (cta == me) continue;
+#pragma unroll 1
+        for (uint32_t r = 0; r < rows; ++r)
+#pragma unroll 1
+            for (uint32_t q = 4u * lane; q < n; q += 128u) {
+                const float* src = from + r * pitch + q;
+                const float4 v = *reinterpret_cast<const float4*>(src);
+                asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(ptx::cluster_map(src, cta)), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+            }
     }
+}
+// `bytes` (a multiple of 16, like both addresses) to shared memory by the copy engine, counted on `bar`.
+__device__ __forceinline__ void copy_bytes(void* to, const void* from, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(ptx::smem_u32(to)), "l"(from), "r"(bytes),
+                 "r"(ptx::smem_u32(bar)) : "memory");
 }
 // Asks for `bytes` from p on to be in L1 by the time they are read.  (Loads whose result nobody waits for: with
 // prefetch.global.L1 the later loads took as long as without.)
@@ -91,14 +141,10 @@ __device__ __forceinline__ void warm_line(uintptr_t p) {
     uint32_t unused;
     asm volatile("ld.global.ca.u32 %0, [%1];" : "=r"(unused) : "l"(p & ~(uintptr_t)3));
 }
-__device__ __forceinline__ void warm(const void* p, size_t bytes, uint32_t me, uint32_t threads) {
-    const uintptr_t from = reinterpret_cast<uintptr_t>(p) / 128u * 128u, to = reinterpret_cast<uintptr_t>(p) + bytes;
-    for (uintptr_t i = from + me * 128u; i < to; i += threads * 128u) warm_line(i < reinterpret_cast<uintptr_t>(p) ? reinterpret_cast<uintptr_t>(p) : i);
-}
-__device__ __forceinline__ void warm_packed(const Packed& W, uint32_t o0, uint32_t n, uint32_t K, uint32_t me, uint32_t threads) {
-    warm(W.bits + ((size_t)o0 * K >> 5), (size_t)n * K / 8u, me, threads);
-    warm(W.scale + o0, n * 2u, me, threads);
-    if (W.bias) warm(W.bias + o0, n * 2u, me, threads);
+__device__ __forceinline__ void warm(const void* p, uint32_t bytes) {
+    const uintptr_t to = reinterpret_cast<uintptr_t>(p) + bytes;
+#pragma unroll 1
+    for (uintptr_t i = reinterpret_cast<uintptr_t>(p); i < to; i = i / 128u * 128u + 128u) warm_line(i);
 }
 
 // acc + v[0] + v[1] + ... + v[C - 1] in this order, by one thread; the next sixteen values are fetched while sixteen are added.
@@ -124,358 +170,683 @@ __device__ __forceinline__ float sum_in_order(const float* v, uint32_t C, float 
     return acc;
 }
 
-// n rows in shared memory, normalised in place (src/model.rs:259-276); `squares` is room for as much again.  Both sums of
-// a row are one thread's, in order; the squares in between are everybody's.  The warps without a row do `meanwhile` (of
-// thread me of so many) under the first sum.
-template <typename F>
-__device__ __forceinline__ void layer_norm(float* rows, float* squares, uint32_t n, uint32_t C, const uint16_t* w, const uint16_t* b, F meanwhile) {
-    __shared__ float s_mean[MAX_GROUP], s_inv[MAX_GROUP];
-    const uint32_t r = threadIdx.x >> 5;
-    __syncthreads();
-    if (r >= n) meanwhile(threadIdx.x - n * 32u, THREADS - n * 32u);
-    else if ((threadIdx.x & 31u) == 0u) s_mean[r] = __fdiv_rn(sum_in_order(rows + r * C, C), (float)C);
-    __syncthreads();
-    for (uint32_t k = 0; k < n; ++k) {
-        const float mean = s_mean[k];
-        for (uint32_t c = threadIdx.x; c < C; c += THREADS) {
-            const float x = __fsub_rn(rows[k * C + c], mean);
-            squares[k * C + c] = __fmul_rn(x, x);
+// Mean and 1 / sqrt(variance + eps) of a row (src/model.rs:259-276) by a warp, in its first lane: both sums in order by one lane,
+// the squares in between by all of them, into `squares`.
+__device__ __forceinline__ float2 row_statistics(const float* row, float* squares, uint32_t C) {
+    const uint32_t lane = threadIdx.x & 31u;
+    float mean = 0.0f;
+#pragma unroll 1
+    for (int pass = 0;; ++pass) {
+        float average = 0.0f;
+        if (lane == 0u) average = __fdiv_rn(sum_in_order(pass ? squares : row, C), (float)C);
+        if (pass) return make_float2(mean, __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(average, 1e-5f))));
+        mean = __shfl_sync(0xFFFFFFFFu, average, 0);
+#pragma unroll 1
+        for (uint32_t c = 4u * lane; c < C; c += 128u) {
+            float4 x = *reinterpret_cast<const float4*>(row + c);
+            x.x = __fsub_rn(x.x, mean); x.y = __fsub_rn(x.y, mean); x.z = __fsub_rn(x.z, mean); x.w = __fsub_rn(x.w, mean);
+            *reinterpret_cast<float4*>(squares + c) = make_float4(__fmul_rn(x.x, x.x), __fmul_rn(x.y, x.y), __fmul_rn(x.z, x.z), __fmul_rn(x.w, x.w));
         }
+        __syncwarp();
     }
-    __syncthreads();
-    if ((threadIdx.x & 31u) == 0u && r < n)
-        s_inv[r] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(sum_in_order(squares + r * C, C), (float)C), 1e-5f)));
-    __syncthreads();
-    for (uint32_t c = threadIdx.x; c < C; c += THREADS) {
-        const float wc = h2f(w[c]), bc = h2f(b[c]);
-        for (uint32_t k = 0; k < n; ++k)
-            rows[k * C + c] = __fadd_rn(__fmul_rn(__fmul_rn(__fsub_rn(rows[k * C + c], s_mean[k]), s_inv[k]), wc), bc);
-    }
+}
+__device__ __forceinline__ float normalised(float x, float mean, float inv, float w, float b) {
+    return __fadd_rn(__fmul_rn(__fmul_rn(__fsub_rn(x, mean), inv), w), b);
 }
 
-// One packed output of N rows by one thread: the sums of +/- in[i] for i ascending (src/model.rs:724-742).  The rows are
-// `pitch` apart; K is a multiple of 32.
-template <int N>
-__device__ __forceinline__ void packed_sums(const float* in, uint32_t pitch, const uint32_t* w, uint32_t K, float (&sum)[N]) {
-    constexpr int CH = 8 / N;   // 16-byte pieces of a row at a time; the next ones are on their way while these are added
-    float4 x[2][N][CH];
-    auto load = [&](int which, uint32_t i) {
-#pragma unroll
-        for (int n = 0; n < N; ++n)
-#pragma unroll
-            for (int u = 0; u < CH; ++u) x[which][n][u] = *reinterpret_cast<const float4*>(in + n * pitch + i + 4 * u);
-    };
-    uint32_t minus = ~w[0];
-#pragma unroll
-    for (int n = 0; n < N; ++n) sum[n] = 0.0f;
-    load(0, 0);
-    for (uint32_t i0 = 0; i0 < K; i0 += 64) {   // two words, so that the buffers are named at compile time
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const uint32_t i1 = i0 + 32 * half;
-            if (half && i1 >= K) break;
-            const uint32_t next = i1 + 32 < K ? ~w[(i1 >> 5) + 1] : 0u;
-#pragma unroll
-            for (int c = 0; c < N; ++c) {
-                const uint32_t after = i1 + 4 * CH * (c + 1);
-                load((half * N + c + 1) & 1, after < K ? after : 0u);
-#pragma unroll
-                for (int u = 0; u < CH; ++u) {
-                    const int bit = 4 * (c * CH + u);
-#pragma unroll
-                    for (int n = 0; n < N; ++n) {
-                        const float4 v = x[(half * N + c) & 1][n][u];
-                        auto add = [&](float f, int b) {
-                            sum[n] = __fadd_rn(sum[n], __uint_as_float(__float_as_uint(f) ^ (minus << (31 - b) & 0x80000000u)));
-                        };
-                        add(v.x, bit); add(v.y, bit + 1); add(v.z, bit + 2); add(v.w, bit + 3);
-                    }
-                }
-            }
-            minus = next;
-        }
-    }
+__device__ __forceinline__ uint32_t load_ahead(const void* p) {   // issued here, not where the value is needed
+    uint32_t v;
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
 }
-__device__ __forceinline__ float scaled(const Packed& p, uint32_t o, float sum) {
-    return __fadd_rn(p.bias ? h2f(p.bias[o]) : 0.0f, __fmul_rn(h2f(p.scale[o]), sum));
+__device__ __forceinline__ uint32_t load_half_ahead(const uint16_t* p) {
+    uint32_t v;
+    asm volatile("ld.global.u16 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
 }
-
-// LayerNorm and time-shift mixes of the cluster's rows (src/model.rs:214-228, 1331-1340, 1008-1012): in[z][n][d] from
-// x[n][d]; half: 0 for the ROSA history, 1 for the CMix history.  The new history of a CTA's channels [o0, o0 + own) is its own
-// to write.
-template <int Z, typename F>
-__device__ __forceinline__ void mixed_inputs(const Step& p, uint32_t layer, uint32_t half, uint32_t row, uint32_t n, uint32_t o0, uint32_t own,
-                                             const uint16_t* ln_w, const uint16_t* ln_b, const uint16_t* const (&mix)[Z], const float* x, float* in,
-                                             F meanwhile) {
-    const uint32_t d = p.d;
-    const size_t at = (((size_t)layer * 2 + half) * p.rows + row) * d;
-    float* xs = in;   // normalised in the place of the first input, squares in that of the second (or behind the first)
-    __syncthreads();
-    for (uint32_t c = threadIdx.x; c < n * d; c += THREADS) xs[c] = x[c];
-    layer_norm(xs, in + p.group * d, n, d, ln_w, ln_b, meanwhile);
-    for (uint32_t i = threadIdx.x; i < d; i += THREADS) {   // the same thread normalised these
-        float m[Z];
-#pragma unroll
-        for (int z = 0; z < Z; ++z) m[z] = h2f(mix[z][i]);
-        for (uint32_t k = 0; k < n; ++k) {
-            const uint32_t c = k * d + i;
-            const float xt = xs[c], xx = p.time ? __fsub_rn(p.prev_in[at + c], xt) : -xt;
-            if (i - o0 < own) p.prev_out[at + c] = xt;
-#pragma unroll
-            for (int z = Z - 1; z >= 0; --z) in[z * p.group * d + c] = __fadd_rn(xt, __fmul_rn(xx, m[z]));
-        }
-    }
-    __syncthreads();
-}
-// `own` outputs from o0 on of a packed linear over n rows in shared memory, N rows per thread; out(row, output, value).
-template <int N, typename F>
-__device__ __forceinline__ void packed_outputs(const Packed& W, const float* in, uint32_t n, uint32_t K, uint32_t o0, uint32_t own, F out) {
-    const uint32_t row_sets = (n + N - 1u) / N;
-    for (uint32_t i = threadIdx.x; i < own * row_sets; i += THREADS) {
-        const uint32_t o = o0 + i % own, r = i / own * N;
-        float sum[N];
-        packed_sums<N>(in + r * K, K, W.bits + ((size_t)o * K >> 5), K, sum);
-#pragma unroll
-        for (int k = 0; k < N; ++k)
-            if (r + k < n) out(r + k, o, scaled(W, o, sum[k]));
-    }
-}
-
-// Piece `piece` of the weights of the CTA's value outputs into a stage of the ring, by threads [0, threads) of which this one
-// is `me`.  (One bulk copy per row of a piece was slower: 32 copies of 512 bytes took 2 400 cycles.)
-__device__ __forceinline__ void fetch_value(uint8_t* stage, const uint16_t* value, uint32_t o0, uint32_t own, uint32_t ffn, uint32_t piece, uint32_t me,
-                                            uint32_t threads) {
-    const uint32_t to = (uint32_t)__cvta_generic_to_shared(stage);
-    for (uint32_t i = me; i < own * (PIECE / 8u); i += threads) {
-        const uint32_t o = i / (PIECE / 8u), g = i % (PIECE / 8u);
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + o * PIECE_PITCH + g * 16u),
-                     "l"(value + (size_t)(o0 + o) * ffn + piece * PIECE + g * 8u) : "memory");
-    }
-}
-__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-
 __device__ __forceinline__ float low_half(uint32_t w) { return h2f((uint16_t)(w & 0xFFFFu)); }
 __device__ __forceinline__ float high_half(uint32_t w) { return h2f((uint16_t)(w >> 16)); }
 
-// The products of PRODUCTS inputs of one row by `producers` warps (this one is number `me`), a granule of eight inputs at a
-// time, lane = output; the weights are two pieces side by side.  The sums have to be added one after the other; multiplied
-// they are beforehand.
-__device__ __forceinline__ void value_products(const uint8_t* pieces, uint32_t piece_bytes, const float* a, uint32_t n, uint32_t me, uint32_t producers,
-                                               float* products) {
+// The statistics of the rows x[r * d] by a warp each; true for the threads that have none to do.
+struct Statistics {
+    float mean[MAX_GROUP], inv[MAX_GROUP];
+};
+__device__ __forceinline__ bool rows_statistics(const float* x, float* squares, uint32_t n, uint32_t d, Statistics& s) {
+    const uint32_t r = threadIdx.x >> 5;
+    if (r >= n) return true;
+    const float2 v = row_statistics(x + r * d, squares + r * d, d);
+    if ((threadIdx.x & 31u) == 0u) { s.mean[r] = v.x; s.inv[r] = v.y; }
+    return false;
+}
+
+// LayerNorm and time-shift mixes of the cluster's rows (src/model.rs:214-228, 1331-1340, 1008-1012): input z of row r and channel c
+// to in[z * apart + c * G + r] from x[r * d + c].  half: 0 for ROSA (three inputs, its history), 1 for the CMix (one).  The new
+// history of a CTA's channels [o0, o0 + own) is its own to write.  A thread has two channels side by side at a time; what it reads
+// from global memory for the first ones is asked for before the sums.
+template <int G>
+__device__ __forceinline__ void mixed_inputs(const Step& p, const Layer& L, uint32_t layer, uint32_t half, uint32_t row, uint32_t n, uint32_t o0, uint32_t own,
+                                          const float* x, float* in, uint32_t apart) {
+    __shared__ Statistics stats;
+    const uint32_t d = p.d, inputs = half ? 1u : 3u;
+    const size_t at = (((size_t)layer * 2 + half) * p.rows + row) * d;
+    const uint16_t *ln_w = half ? L.ln2_w : L.ln3_w, *ln_b = half ? L.ln2_b : L.ln3_b, *mix0 = half ? L.ffn_mix : L.mix[0];
+    uint32_t w, b, m[3];
+    float2 before[G];
+    auto ask = [&](uint32_t c) {
+        w = load_ahead(ln_w + c);
+        b = load_ahead(ln_b + c);
+        m[0] = load_ahead(mix0 + c);
+        if (inputs > 1u) {
+            m[1] = load_ahead(L.mix[1] + c);
+            m[2] = load_ahead(L.mix[2] + c);
+        }
+#pragma unroll
+        for (int r = 0; r < G; ++r)
+            if (p.time && r < n)
+                asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(before[r].x), "=f"(before[r].y) : "l"(p.prev_in + at + (size_t)r * d + c));
+    };
+    uint32_t c = 2u * threadIdx.x;
+    if (c < d) ask(c);
+    __syncthreads();
+    if (rows_statistics(x, in, n, d, stats) && !half) {
+        // the keys of this CTA's streams, for a search
+        const uint32_t threads = THREADS - n * 32u;
+#pragma unroll 1
+        for (uint32_t i = threadIdx.x - n * 32u; i < n * own; i += threads)
+            warm(p.push.of(((size_t)layer * p.rows + row + i / own) * d + o0 + i % own, 1), (p.time / 32u + 1u) * 4u);
+    }
+    __syncthreads();
+#pragma unroll 1
+    while (c < d) {
+#pragma unroll
+        for (int r = 0; r < G; ++r) {
+            if (r >= n) break;
+            const float2 v = *reinterpret_cast<const float2*>(x + r * d + c);
+            const float a = normalised(v.x, stats.mean[r], stats.inv[r], low_half(w), low_half(b));
+            const float e = normalised(v.y, stats.mean[r], stats.inv[r], high_half(w), high_half(b));
+            const float da = p.time ? __fsub_rn(before[r].x, a) : -a, de = p.time ? __fsub_rn(before[r].y, e) : -e;
+            if (c - o0 < own) *reinterpret_cast<float2*>(p.prev_out + at + (size_t)r * d + c) = make_float2(a, e);
+#pragma unroll
+            for (int z = 0; z < 3; ++z) {
+                if (z >= inputs) break;
+                in[z * apart + c * G + r] = __fadd_rn(a, __fmul_rn(da, low_half(m[z])));
+                in[z * apart + (c + 1u) * G + r] = __fadd_rn(e, __fmul_rn(de, high_half(m[z])));
+            }
+        }
+        c += 2u * THREADS;
+        if (c < d) ask(c);
+    }
+}
+
+__device__ __forceinline__ float2 fma_pair(float2 a, float2 b, float2 c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(*reinterpret_cast<uint64_t*>(&a)), "l"(*reinterpret_cast<uint64_t*>(&b)), "l"(*reinterpret_cast<uint64_t*>(&c)));
+    return *reinterpret_cast<float2*>(&r);
+}
+__device__ __forceinline__ float2 add_pair(float2 a, float2 b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(*reinterpret_cast<uint64_t*>(&a)), "l"(*reinterpret_cast<uint64_t*>(&b)));
+    return *reinterpret_cast<float2*>(&r);
+}
+// The sign of x turned unless the top bit of `bits` is set, and 1.0 with that sign, as one instruction each.
+__device__ __forceinline__ uint32_t flip_unless(uint32_t bits, uint32_t x) {
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0xA6;" : "=r"(r) : "r"(bits), "r"(0x80000000u), "r"(x));   // (~a & b) ^ c
+    return r;
+}
+__device__ __forceinline__ uint32_t minus_unless(uint32_t bits) {
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0xAE;" : "=r"(r) : "r"(bits), "r"(0x80000000u), "r"(0x3F800000u));   // (~a & b) | c
+    return r;
+}
+__device__ __forceinline__ float& lane_of(float4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
+
+// Four words of a packed row, of which `left` are there.
+__device__ __forceinline__ uint4 four_words(const uint32_t* w, uint32_t left, bool quads) {
+    if (quads) return *reinterpret_cast<const uint4*>(w);
+    return make_uint4(w[0], left > 1u ? w[1] : 0u, left > 2u ? w[2] : 0u, left > 3u ? w[3] : 0u);
+}
+// The sums of +/- in[i] for i ascending (src/model.rs:724-742) of G rows side by side (input i of row r at i * G + r) for J
+// outputs; output j takes its inputs from in + j * apart and their signs from w + j * w_apart, in shared or global memory.  K is a
+// multiple of 32.  The inputs of the next CH terms and the next four words are on their way while these are added.
+template <int G, int J, bool APART>
+__device__ __forceinline__ void packed_sums(const float* in, uint32_t apart, const uint32_t* w, uint32_t w_apart, uint32_t K, float (&sum)[J][G]) {
+    constexpr int S = APART ? J : 1, BODY = G * J == 1 ? 64 : 32, CH = G * J == 1 ? 16 : G == 1 ? 8 : (G * S > 4 || J * G > 8) ? 4 : 8, Q = CH * G / 4;
+    const uint32_t words = K / 32u;
+    const bool quads = words % 4u == 0u;
+    float4 x[2][S][Q];
+    float total[J][G];
+    uint4 now[J], next[J];
+    auto load = [&](int which, uint32_t i) {
+#pragma unroll
+        for (int s = 0; s < S; ++s)
+#pragma unroll
+            for (int q = 0; q < Q; ++q) x[which][s][q] = *reinterpret_cast<const float4*>(in + s * apart + i * G + 4 * q);
+    };
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+        next[j] = four_words(w + j * w_apart, words, quads);
+#pragma unroll
+        for (int r = 0; r < G; ++r) total[j][r] = 0.0f;
+    }
+    load(0, 0u);
+#pragma unroll 1
+    for (uint32_t i = 0; i < K; i += BODY) {
+        if (i % 128u == 0u) {
+            const uint32_t then = i + 128u < K ? i / 32u + 4u : 0u;
+#pragma unroll
+            for (int j = 0; j < J; ++j) {
+                now[j] = next[j];
+                next[j] = four_words(w + j * w_apart + then, words - then, quads);
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < BODY / CH; ++c) {
+            if (BODY == 64 && c == 32 / CH && i + 32u >= K) break;   // K an odd number of words
+            const uint32_t after = i + CH * (c + 1);
+            load((c & 1) ^ 1, after < K ? after : 0u);
+#pragma unroll
+            for (int e = 0; e < CH; ++e)
+#pragma unroll
+                for (int j = 0; j < J; ++j) {
+                    const uint32_t up = (c * CH + e < 32 ? now[j].x : now[j].y) << (31 - (c * CH + e) % 32);   // the sign on top: 1 is +
+                    if (G == 1) {
+                        const float v = lane_of(x[c & 1][APART ? j : 0][e / 4], e % 4);
+                        total[j][0] = __fadd_rn(total[j][0], __uint_as_float(flip_unless(up, __float_as_uint(v))));
+                    } else {
+                        const float sign = __uint_as_float(minus_unless(up));
+#pragma unroll
+                        for (int r = 0; r < G; r += 2) {
+                            const int q = e * G + r, r1 = r + 1 < G ? r + 1 : 0;
+                            const float2 v = make_float2(lane_of(x[c & 1][APART ? j : 0][q / 4], q % 4), lane_of(x[c & 1][APART ? j : 0][q / 4], (q + 1) % 4));
+                            const float2 s = fma_pair(v, make_float2(sign, sign), make_float2(total[j][r], total[j][r1]));
+                            total[j][r] = s.x;
+                            total[j][r1] = s.y;
+                        }
+                    }
+                }
+        }
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            if (BODY == 32) {
+                now[j].x = now[j].y; now[j].y = now[j].z; now[j].z = now[j].w;
+            } else {
+                now[j].x = now[j].z; now[j].y = now[j].w;
+            }
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < J; ++j)
+#pragma unroll
+        for (int r = 0; r < G; ++r) sum[j][r] = total[j][r];
+}
+
+// n_out outputs of a packed linear over G rows, J per thread (n_out a multiple of J); `first`: where they begin in scale and bias;
+// emit(output, row, value) with the output counted from 0.
+template <int G, int J, typename F>
+__device__ __forceinline__ void packed_outputs(const Packed& P, const uint32_t* w, const float* in, uint32_t n, uint32_t K, uint32_t first, uint32_t n_out,
+                                               F emit) {
+    const uint32_t apart = n_out / J;
+#pragma unroll 1
+    for (uint32_t o = threadIdx.x; o < apart; o += THREADS) {
+        uint32_t scale[J], bias[J];
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            scale[j] = load_half_ahead(P.scale + first + o + j * apart);
+            bias[j] = P.bias ? load_half_ahead(P.bias + first + o + j * apart) : 0u;
+        }
+        float sum[J][G];
+        packed_sums<G, J, false>(in, 0u, w + (size_t)o * (K / 32u), apart * (K / 32u), K, sum);
+#pragma unroll
+        for (int j = 0; j < J; ++j)
+#pragma unroll
+            for (int r = 0; r < G; ++r)
+                if (r < n) emit(o + j * apart, (uint32_t)r, __fadd_rn(low_half(bias[j]), __fmul_rn(low_half(scale[j]), sum[j][r])));
+    }
+}
+
+// The copies of a CTA, issued by one thread, and the waits for them.  gave_up: a wait ran out; nobody waits any more then, and
+// the step reports it.
+constexpr uint32_t BARS = 2 * MAX_STAGES + 3, MAX_BOX = 256;
+struct Copies {
+    uint64_t ring[BARS];   // mbarriers: a stage of the ring is full, is empty, and one for each set of packed weights
+    __device__ uint64_t* empty() { return ring + MAX_STAGES; }
+    __device__ uint64_t* qkv_o() { return ring + 2 * MAX_STAGES; }
+    __device__ uint64_t* key() { return ring + 2 * MAX_STAGES + 1; }
+    __device__ uint64_t* head() { return ring + 2 * MAX_STAGES + 2; }
+    uint32_t gave_up;
+};
+__device__ __forceinline__ void copies_wait(Copies& copies, uint64_t* bar, uint32_t phase, uint32_t* status, uint32_t site) {
+    if (*static_cast<volatile uint32_t*>(&copies.gave_up)) return;
+#pragma unroll 1
+    for (uint32_t polls = 0; polls < 1u << 22; ++polls)
+        if (ptx::mbar_try_wait(bar, phase & 1u)) return;
+    *static_cast<volatile uint32_t*>(&copies.gave_up) = 1u;
+    *static_cast<volatile uint32_t*>(status) = ULLIS_DEV_WAIT_TIMEOUT;
+    *static_cast<volatile uint32_t*>(status + 1) = site;
+}
+// `slabs` slabs (as many as the map's box has) from slab `slab` on of the weights of the value outputs [o0, o0 + own), by one thread.
+__device__ __forceinline__ void fetch_value(uint8_t* to, const CUtensorMap* map, uint32_t o0, uint32_t own, uint32_t slab, uint32_t slabs, uint64_t* bar) {
+    ptx::mbar_arrive_expect_tx(bar, slabs * own * (SLAB * 2u));
+    const uint32_t rows = min(own, MAX_BOX);
+    if (rows == own) {
+        ptx::tma_load_3d(to, map, bar, 0, (int32_t)o0, (int32_t)slab);
+    } else {   // the box is one slab of MAX_BOX outputs
+#pragma unroll 1
+        for (uint32_t b = 0; b < slabs * (own / rows); ++b)
+            ptx::tma_load_3d(to + b * rows * (SLAB * 2u), map, bar, 0, (int32_t)(o0 + b % (own / rows) * rows), (int32_t)(slab + b / (own / rows)));
+    }
+}
+// Where the lane's output of a tile has its granules in the box of a slab (shared address): granule g (eight inputs) at
+// granules ^ 16 g.
+__device__ __forceinline__ uint32_t lane_granules(const uint8_t* box) {
     const uint32_t lane = threadIdx.x & 31u;
-#pragma unroll 2
-    for (uint32_t g = me; g < n / 8u; g += producers) {
-        const uint4 w8 = *reinterpret_cast<const uint4*>(pieces + g / (PIECE / 8u) * piece_bytes + lane * PIECE_PITCH + g % (PIECE / 8u) * 16u);
+    return ptx::smem_u32(box) + lane * 128u + (lane & 7u) * 16u;
+}
+__device__ __forceinline__ uint4 granule(uint32_t granules, uint32_t g) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(granules ^ 16u * g));
+    return v;
+}
+
+__device__ __forceinline__ void barrier_arrive(uint32_t id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(THREADS) : "memory"); }
+__device__ __forceinline__ void barrier_sync(uint32_t id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(THREADS) : "memory"); }
+
+// The products of PRODUCTS inputs of one row by `producers` warps (this one is number `me`), a granule of eight inputs at a
+// time, lane = output.  The sums have to be added one after the other; multiplied they are beforehand.
+__device__ __forceinline__ void value_products(const uint8_t* piece, const float* a, uint32_t me, uint32_t producers, float* products) {
+    const uint32_t lane = threadIdx.x & 31u;
+#pragma unroll 3
+    for (uint32_t g = me; g < PRODUCTS / 8u; g += producers) {
+        const uint4 w8 = granule(lane_granules(piece + g / 8u * BOX_BYTES), g % 8u);
         const float4 xa = *reinterpret_cast<const float4*>(a + g * 8u), xb = *reinterpret_cast<const float4*>(a + g * 8u + 4u);
         float4* to = reinterpret_cast<float4*>(products + lane * PRODUCT_PITCH + g * 8u);
         to[0] = make_float4(__fmul_rn(low_half(w8.x), xa.x), __fmul_rn(high_half(w8.x), xa.y), __fmul_rn(low_half(w8.y), xa.z), __fmul_rn(high_half(w8.y), xa.w));
         to[1] = make_float4(__fmul_rn(low_half(w8.z), xb.x), __fmul_rn(high_half(w8.z), xb.y), __fmul_rn(low_half(w8.w), xb.z), __fmul_rn(high_half(w8.w), xb.w));
     }
 }
-// sum + w[0] a[0] + w[1] a[1] + ... of one piece in this order, lane = output; the next granule is on its way while one is
-// added.
-__device__ __forceinline__ float value_piece(float sum, const uint8_t* tile, const float* a) {
-    const uint4* t = reinterpret_cast<const uint4*>(tile + (threadIdx.x & 31u) * PIECE_PITCH);
-    uint4 w = t[0];
-    float4 xa = *reinterpret_cast<const float4*>(a), xb = *reinterpret_cast<const float4*>(a + 4);
-#pragma unroll 8
-    for (uint32_t g = 0; g < PIECE / 8u; ++g) {
-        const uint32_t h = g + 1u < PIECE / 8u ? g + 1u : 0u;
-        const uint4 w_next = t[h];
-        const float4 xa_next = *reinterpret_cast<const float4*>(a + h * 8u), xb_next = *reinterpret_cast<const float4*>(a + h * 8u + 4u);
-        const float p[8] = {__fmul_rn(low_half(w.x), xa.x), __fmul_rn(high_half(w.x), xa.y), __fmul_rn(low_half(w.y), xa.z), __fmul_rn(high_half(w.y), xa.w),
-                            __fmul_rn(low_half(w.z), xb.x), __fmul_rn(high_half(w.z), xb.y), __fmul_rn(low_half(w.w), xb.z), __fmul_rn(high_half(w.w), xb.w)};
+// The 32 sums of a CTA that has no more (src/model.rs:419-436): warp 0 adds, the others multiply for it into PRODUCT_SLOTS
+// slots, handed over by named barriers (1 + slot: full, 4 + slot: empty).  Returns the sum of the lane's output in warp 0.
+__device__ __forceinline__ float value_alone(const uint8_t* ring, Copies& copies, uint32_t phase, const float* act, uint32_t pieces, float* products, uint32_t* status) {
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    constexpr uint32_t FULL = 1u, EMPTY = FULL + PRODUCT_SLOTS, SLOT = VALUE_OUT * PRODUCT_PITCH;
+    float sum = 0.0f;
+    uint32_t slot = 0;
+    copies_wait(copies, copies.ring, phase, status, 0x601u);
+    if (warp != 0u) {
+#pragma unroll 1
+        for (uint32_t k = 0; k < pieces; ++k) {
+            if (k >= PRODUCT_SLOTS) barrier_sync(EMPTY + slot);
+            value_products(ring + k * (VALUE_OUT * PIECE * 2u), act + k * PIECE, warp - 1u, WARPS - 1u, products + slot * SLOT);
+            barrier_arrive(FULL + slot);
+            slot = slot + 1u < PRODUCT_SLOTS ? slot + 1u : 0u;
+        }
+        return sum;
+    }
+    // CH products are fetched while CH are added, by turns (a batch of loads would hold the additions up); the barrier of a slot is
+    // passed before the last ones of the slot before are added.
+    constexpr int CH = 32;
+    float4 v[2][CH / 4];
+    uint32_t at = ptx::smem_u32(products) + lane * (PRODUCT_PITCH * 4u);
+    auto load = [&](float4& to, int q) {
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(to.x), "=f"(to.y), "=f"(to.z), "=f"(to.w) : "r"(at + 16u * q) : "memory");
+    };
+    auto load_and_add = [&](int from) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) sum = __fadd_rn(sum, p[e]);
-        w = w_next; xa = xa_next; xb = xb_next;
+        for (int q = 0; q < CH / 4; ++q) {
+            load(v[from ^ 1][q], q);
+            sum = __fadd_rn(sum, v[from][q].x);
+            sum = __fadd_rn(sum, v[from][q].y);
+            sum = __fadd_rn(sum, v[from][q].z);
+            sum = __fadd_rn(sum, v[from][q].w);
+        }
+    };
+    barrier_sync(FULL);
+#pragma unroll
+    for (int q = 0; q < CH / 4; ++q) load(v[0][q], q);
+#pragma unroll 1
+    for (uint32_t k = 0; k < pieces; ++k) {
+        at += CH * 4u;
+        load_and_add(0);
+        at += CH * 4u;
+        load_and_add(1);
+        at += CH * 4u;
+        load_and_add(0);
+        const uint32_t before = slot;
+        slot = slot + 1u < PRODUCT_SLOTS ? slot + 1u : 0u;
+        at = ptx::smem_u32(products + slot * SLOT) + lane * (PRODUCT_PITCH * 4u);
+        if (k + 1u < pieces) barrier_sync(FULL + slot);
+        if (k + PRODUCT_SLOTS < pieces) barrier_arrive(EMPTY + before);
+        load_and_add(1);   // the last one fetches whatever lies there
     }
     return sum;
 }
+// The sums of N rows side by side (input i of row r at a[i * G + r]) over one piece, lane = output: sum + w[0] a[0] + ... in
+// this order, every product and every sum rounded; the next granule of eight inputs is on its way while one is added.
+// (mul.rn.f32x2 and add.rn.f32x2 were contracted to one fma.f32x2; a product as fma(x, y, -0.0) rounds the same and cannot be,
+// if the compiler does not know the -0.0.)
+template <int G, int N>
+__device__ __forceinline__ void value_piece(float (&sum)[N], const uint8_t* piece, uint32_t tiles, uint32_t tile, const float* a, float minus_zero) {
+    constexpr uint32_t GRANULES = PIECE / 8u;
+    const uint32_t first = lane_granules(piece + tile * BOX_BYTES), second = first + tiles * BOX_BYTES;
+    uint4 w[2];
+    float x[2][8 * N];
+    auto load = [&](int which, uint32_t g) {
+        w[which] = granule(g < GRANULES / 2u ? first : second, g % 8u);
+        const float* at = a + g * 8u * G;
+        if (G == N) {
+#pragma unroll
+            for (int q = 0; q < 2 * N; ++q) {
+                const float4 v = *reinterpret_cast<const float4*>(at + 4 * q);
+                x[which][4 * q] = v.x; x[which][4 * q + 1] = v.y; x[which][4 * q + 2] = v.z; x[which][4 * q + 3] = v.w;
+            }
+        } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const float2 v = *reinterpret_cast<const float2*>(at + e * G);
+                x[which][N * e] = v.x; x[which][N * e + N - 1] = v.y;
+            }
+        }
+    };
+    auto add = [&](int b) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const uint32_t pair = e < 2 ? w[b].x : e < 4 ? w[b].y : e < 6 ? w[b].z : w[b].w;
+            const float f = e & 1 ? high_half(pair) : low_half(pair);
+            if (N == 1) {
+                sum[0] = __fadd_rn(sum[0], __fmul_rn(f, x[b][e]));
+            } else {
+                const float2 s = add_pair(make_float2(sum[0], sum[N - 1]), fma_pair(make_float2(f, f), make_float2(x[b][N * e], x[b][N * e + N - 1]), make_float2(minus_zero, minus_zero)));
+                sum[0] = s.x;
+                sum[N - 1] = s.y;
+            }
+        }
+    };
+    load(0, 0u);
+#pragma unroll 1
+    for (uint32_t g = 0; g < GRANULES; g += VALUE_BODY) {
+#pragma unroll
+        for (uint32_t k = 0; k < VALUE_BODY; ++k) {
+            load((k & 1u) ^ 1u, (g + k + 1u) % GRANULES);
+            add(k & 1u);
+        }
+    }
+}
 
-// N: rows of a thread in A, C and the head
-template <int N>
+// G: sequences of a cluster.
+template <int G>
 __global__ void __launch_bounds__(THREADS, 1)
 gen_step_kernel(const Step p) {
     extern __shared__ __align__(16) uint8_t step_smem[];
-    __shared__ uint8_t bits[3 * MAX_GROUP * TURN];
     __shared__ Layer layers[2];
-    const uint32_t d = p.d, ffn = p.ffn, G = p.group, ctas = cluster_size(), rank = cluster_rank();
+    __shared__ Statistics stats;
+    const uint32_t d = p.d, ffn = p.ffn, ctas = cluster_size(), rank = cluster_rank(), words = d / 32u;
     const uint32_t own = d / ctas, o0 = rank * own;                                  // channels of this CTA
     const uint32_t f_own = ffn / ctas, f0 = rank * f_own;                            // CMix hidden units
     const uint32_t v_own = (p.vocab + ctas - 1u) / ctas, v0 = min(rank * v_own, p.vocab), v_n = min(v_own, p.vocab - v0);
-    uint8_t* ring = step_smem;
-    const uint32_t pieces = ffn / PIECE, tiles = own / VALUE_OUT, stages = ring_stages(G, own, ffn), stage_bytes = own * PIECE_PITCH;
-    const bool alone = G * own == VALUE_OUT;   // D: one sum per CTA
-    float* x = reinterpret_cast<float*>(step_smem + stages * stage_bytes);
-    float* y = x + G * d;
-    float* in = y + G * d;
-    float* act = in + 3 * G * d;
-    float* products = act + G * ffn;
+    const uint32_t pieces = ffn / PIECE, tiles = own / VALUE_OUT, stages = p.stages, stage_bytes = own * (PIECE * 2u);
+    const bool staged = p.staged;                 // packed weights in shared memory
+    const Layout at(G, d, ffn, ctas, stages, staged);
+    constexpr int N = G < 2 ? 1 : 2;              // rows of a thread in D
+    const bool alone = G * own == VALUE_OUT;      // D: one sum per lane of a warp
+    uint8_t* const base = step_smem + (0u - ptx::smem_u32(step_smem)) % 1024u;   // the same in every CTA of the cluster
+    uint8_t* ring = base + at.ring;
+    float* products = reinterpret_cast<float*>(base + at.products);
+    float* x = reinterpret_cast<float*>(base + at.rows);   // [G][d]
+    float* in0 = x + G * d;                                     // [d][G]
+    float* act = in0 + G * d;                                   // [ffn][G] in C and D
+    float* in1 = act;                                           // [d][G], and the third input behind it, in A
+    float* y = act + 2u * G * d;                                // [d][G] in A and B
+    uint8_t* bits = base + at.bits;                             // [3][G][own]
+    uint32_t* w_wide = reinterpret_cast<uint32_t*>(base + at.wide);
+    uint32_t* w_o = reinterpret_cast<uint32_t*>(base + at.o);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    __shared__ Copies copies;
+    const bool copier = warp == WARPS - 1u, issuer = copier && lane == 0u;   // its first lane asks for copies
+    uint32_t layers_done = 0, heads_done = 0;     // phases of the barriers of the packed weights
+    uint32_t slot = 0, lap = 0;                   // of the ring: the piece that is used next
+    uint32_t fetch_slot = 0;                      // the piece that is fetched next
+    if (issuer) {
+#pragma unroll 1
+        for (uint32_t b = 0; b < BARS; ++b) ptx::mbar_init(copies.ring + b, b - MAX_STAGES < MAX_STAGES ? WARPS : 1u);
+        ptx::fence_mbar_init();
+        copies.gave_up = 0u;
+    }
+    __syncthreads();
     auto load_layer = [&](uint32_t l) {
         const uint32_t* from = reinterpret_cast<const uint32_t*>(p.layers + l);
         uint32_t* to = reinterpret_cast<uint32_t*>(&layers[l & 1u]);
+#pragma unroll 1
         for (uint32_t i = threadIdx.x; i < sizeof(Layer) / 4u; i += THREADS) to[i] = from[i];
     };
-    auto nothing = [](uint32_t, uint32_t) {};
+    const uint32_t own_bytes = own * words * 4u;
+    auto fetch_qkv_o = [&](const Layer& L) {
+        if (!issuer || !staged || copies.gave_up) return;
+        ptx::mbar_arrive_expect_tx(copies.qkv_o(), 4u * own_bytes);
+        for (uint32_t z = 0; z < 3u; ++z) copy_bytes(w_wide + z * own * words, L.qkv[z].bits + (size_t)o0 * words, own_bytes, copies.qkv_o());
+        copy_bytes(w_o, L.o.bits + (size_t)o0 * words, own_bytes, copies.qkv_o());
+    };
+    // D takes its weights `passes` times: a warp has 32 outputs of N rows per pass
+    auto fetch_piece = [&](uint32_t l, uint32_t i) {
+        if (!issuer || copies.gave_up) return;
+        fetch_value(ring + fetch_slot * stage_bytes, p.values + l, o0, own, i % pieces * (PIECE / SLAB), PIECE / SLAB, copies.ring + fetch_slot);
+        fetch_slot = fetch_slot + 1u < stages ? fetch_slot + 1u : 0u;
+    };
     const uint32_t clusters = gridDim.x / ctas;
     for (uint32_t row = blockIdx.x / ctas * G; row < p.rows; row += clusters * G) {
-        const uint32_t n = min(G, p.rows - row);
+        const uint32_t n = min((uint32_t)G, p.rows - row);
         load_layer(0);
-        for (uint32_t r = 0; r < n; ++r) {   // embedding and ln0, which replaces it
-            const uint16_t* e = p.embedding + (size_t)p.tokens[row + r] * d;
+#pragma unroll 1
+        for (uint32_t r = 0; r < G; ++r) {   // embedding and ln0, which replaces it
+            const uint16_t* e = p.embedding + (size_t)p.tokens[row + min(r, n - 1u)] * d;
+#pragma unroll 1
             for (uint32_t c = threadIdx.x; c < d; c += THREADS) x[r * d + c] = h2f(e[c]);
         }
-        layer_norm(x, in, n, d, p.ln0_w, p.ln0_b, nothing);
-        // the pushes of a turn of at most 128 channels: `per` channels side by side of one row for a warp at a time
-        const uint32_t turn = min(TURN, own);
+        __syncthreads();
+        rows_statistics(x, in0, n, d, stats);
+        __syncthreads();
+        fetch_qkv_o(layers[0]);
+#pragma unroll 1
+        for (uint32_t c = threadIdx.x; c < d; c += THREADS) {
+            const float w = h2f(p.ln0_w[c]), b = h2f(p.ln0_b[c]);
+#pragma unroll 1
+            for (uint32_t r = 0; r < n; ++r) x[r * d + c] = normalised(x[r * d + c], stats.mean[r], stats.inv[r], w, b);
+        }
+        // the pushes: `per` channels side by side of one row for a warp at a time
         uint32_t per = 1u;
-        while (per < 32u && 2u * per <= n * turn / WARPS) per *= 2u;   // turn is a multiple of 32
-        auto push_set = [&](uint32_t l, uint32_t c0, uint32_t j, size_t& stream, uint32_t& r, uint32_t& c) {
-            r = j / (turn / per);
-            c = j % (turn / per) * per + lane;
-            stream = ((size_t)l * p.rows + row + r) * d + o0 + c0 + c - lane;
-            return lane < per && r < n && c0 + c < own;
+        while (per < 32u && 2u * per <= n * min(own, 128u) / WARPS) per *= 2u;   // own is a multiple of 32
+        const uint32_t sets = n * (own / per);
+        auto push_set = [&](uint32_t l, uint32_t j, size_t& stream, uint32_t& r, uint32_t& c) {
+            r = j / (own / per);
+            c = j % (own / per) * per + lane;
+            stream = ((size_t)l * p.rows + row + r) * d + o0 + c - lane;
+            return lane < per && r < n;
         };
         auto push_begin = [&](uint32_t l) {   // of this warp's first set: asked for while something else is waited for
             size_t stream;
             uint32_t r, c;
-            const bool live = push_set(l, 0u, warp, stream, r, c);
+            const bool live = push_set(l, warp, stream, r, c);
             return push::begin(p.push, stream, live, p.time);
         };
         push::Ahead ahead = push_begin(0u);
+        const uint32_t sums = (n + N - 1u) / N * tiles, passes = (sums + WARPS - 1u) / WARPS, items = passes * pieces;   // of D
+#pragma unroll 1
         for (uint32_t l = 0; l < p.n_layers; ++l) {
-            __syncthreads();   // the layer's pointers; the ring is free
-            const Layer& L = layers[l & 1u];
-            // ---- A
-            mixed_inputs<3>(p, l, 0u, row, n, o0, own, L.ln3_w, L.ln3_b, L.mix, x, in, [&](uint32_t me, uint32_t threads) {
-                // what A, B and C read from global memory
-                const size_t at = ((size_t)l * 2 * p.rows + row) * d;
-                auto all = [&](const void* from, size_t bytes) { warm(from, bytes, me, threads); };
-                all(L.ln3_w, d * 2u); all(L.ln3_b, d * 2u);
-                if (p.time) all(p.prev_in + at, (size_t)n * d * 4u);
-                for (int z = 0; z < 3; ++z) {
-                    all(L.mix[z], d * 2u);
-                    warm_packed(L.qkv[z], o0, own, d, me, threads);
-                }
-                all(L.e + o0, own * 2u);
-                for (uint32_t i = me; i < n * own; i += threads)   // the keys of this CTA's streams, for a search
-                    warm(p.push.of(((size_t)l * p.rows + row + i / own) * d + o0 + i % own, 1), (p.time / 32u + 1u) * 4u, 0u, 1u);
-                warm_packed(L.o, o0, own, d, me, threads);
-                all(L.ln2_w, d * 2u); all(L.ln2_b, d * 2u); all(L.ffn_mix, d * 2u);
-                if (p.time) all(p.prev_in + at + (size_t)p.rows * d, (size_t)n * d * 4u);
-                warm_packed(L.key, f0, f_own, d, me, threads);
-            });
-            for (uint32_t c0 = 0; c0 < own; c0 += turn) {
-                const uint32_t nc = min(turn, own - c0), row_sets = (n + N - 1u) / N;
-                for (uint32_t i = threadIdx.x; i < 3u * nc * row_sets; i += THREADS) {
-                    const uint32_t z = i / nc % 3u, c = i % nc, r = i / (3u * nc) * N, o = o0 + c0 + c;
-                    const Packed& W = L.qkv[z];
-                    float sum[N];
-                    packed_sums<N>(in + (z * G + r) * d, d, W.bits + ((size_t)o * d >> 5), d, sum);
-#pragma unroll
-                    for (int k = 0; k < N; ++k)
-                        if (r + k < n) bits[(z * MAX_GROUP + r + k) * TURN + c] = scaled(W, o, sum[k]) > 0.0f;   // src/rosa.rs:372-374
+            const Layer& L = layers[l & 1u];   // everybody's since a barrier ago
+#pragma unroll 1
+            for (uint32_t stage = 0; stage < 3u; ++stage) {   // A, B, C
+                const uint32_t n_out = stage == 0u ? 3u * own : stage == 1u ? own : f_own;
+                if (stage != 1u) {
+                    mixed_inputs<G>(p, L, l, stage / 2u, row, n, o0, own, x, in0, G * d);
+                    if (staged) copies_wait(copies, stage ? copies.key() : copies.qkv_o(), layers_done, p.status, 0x602u);
                 }
                 __syncthreads();
-                for (uint32_t j = warp; j < n * (turn / per); j += WARPS) {
-                    size_t stream;
-                    uint32_t r, c;
-                    const bool live = push_set(l, c0, j, stream, r, c);
-                    if (j != warp || c0) ahead = push::begin(p.push, stream, live, p.time);
-                    const uint32_t at = r * TURN + c;
-                    const bool idx = push::step(p.push, stream, live, p.time, ahead, live ? bits[at] : 0u, live ? bits[MAX_GROUP * TURN + at] : 0u,
-                                                live ? bits[2 * MAX_GROUP * TURN + at] : 0u);
-                    if (live) {   // src/model.rs:1344-1351
-                        const float ev = h2f(L.e[o0 + c0 + c]);
-                        y[r * d + o0 + c0 + c] = idx ? ev : -ev;
+                auto emit = [&](uint32_t o, uint32_t r, float v) {
+                    if (stage == 0u) {
+                        const uint32_t z = o / own, c = o - z * own;
+                        bits[(z * G + r) * own + c] = v > 0.0f;   // src/rosa.rs:372-374
+                    } else if (stage == 1u) {
+                        x[r * d + o0 + o] = __fadd_rn(x[r * d + o0 + o], v);
+                    } else {
+                        const float m = fmaxf(v, 0.0f);           // src/model.rs:999
+                        act[(f0 + o) * G + r] = __fmul_rn(m, m);
+                    }
+                };
+                // As many outputs per thread as leave a warp for every scheduler.
+                if (G > 1 && stage == 0u && staged && own >= THREADS / 2u) {   // q, k and v of a channel
+#pragma unroll 1
+                    for (uint32_t c = threadIdx.x; c < own; c += THREADS) {
+                        uint32_t scale[3], bias[3];
+#pragma unroll
+                        for (int z = 0; z < 3; ++z) {
+                            scale[z] = load_half_ahead(L.qkv[z].scale + o0 + c);
+                            bias[z] = load_half_ahead(L.qkv[z].bias + o0 + c);
+                        }
+                        float sum[3][G];
+                        packed_sums<G, 3, true>(in0, G * d, w_wide + c * words, own * words, d, sum);
+#pragma unroll
+                        for (int z = 0; z < 3; ++z)
+#pragma unroll
+                            for (int r = 0; r < G; ++r)
+                                if (r < n) emit(z * own + c, r, __fadd_rn(low_half(bias[z]), __fmul_rn(low_half(scale[z]), sum[z][r])));
+                    }
+                } else if (stage == 2u && n_out >= 2u * THREADS) {
+                    packed_outputs<G, 4>(L.key, staged ? w_wide : L.key.bits + (size_t)f0 * words, in0, n, d, f0, n_out, emit);
+                } else if (stage == 2u && n_out >= THREADS && n_out % 2u == 0u) {
+                    packed_outputs<G, 2>(L.key, staged ? w_wide : L.key.bits + (size_t)f0 * words, in0, n, d, f0, n_out, emit);
+                } else {
+#pragma unroll 1
+                    for (uint32_t o = threadIdx.x; o < n_out; o += THREADS) {
+                        const uint32_t z = stage == 0u ? o / own : 0u, first = stage == 2u ? f0 : o0, k = o - z * own;
+                        const Packed& P = stage == 0u ? L.qkv[z] : stage == 1u ? L.o : L.key;
+                        const uint32_t scale = load_half_ahead(P.scale + first + k), bias = P.bias ? load_half_ahead(P.bias + first + k) : 0u;
+                        const uint32_t* w = staged ? (stage == 1u ? w_o : w_wide) + (size_t)o * words : P.bits + (size_t)(first + k) * words;
+                        float sum[1][G];
+                        packed_sums<G, 1, false>(stage == 1u ? y : in0 + z * (G * d), 0u, w, 0u, d, sum);
+#pragma unroll
+                        for (int r = 0; r < G; ++r)
+                            if (r < n) emit(o, r, __fadd_rn(low_half(bias), __fmul_rn(low_half(scale), sum[0][r])));
                     }
                 }
                 __syncthreads();
-            }
-            share_with_cluster(y + o0, n, d, own);
-            cluster_barrier();
-            // ---- B
-            // The first pieces of D's weights, by the threads that have no output here if there are enough of them.  (A thread
-            // waits for its own copies; one that took no part has none to wait for.)
-            const uint32_t busy = min((n * own + 31u) / 32u * 32u, THREADS / 2u), first = alone ? pieces : stages - 1u;
-            if (threadIdx.x >= busy)
-                for (uint32_t k = 0; k < first; ++k) {
-                    if (k < pieces) fetch_value(ring + k * stage_bytes, L.value, o0, own, ffn, k, threadIdx.x - busy, THREADS - busy);
-                    copies_commit();
+                if (stage == 0u) {
+#pragma unroll 1
+                    for (uint32_t j = warp; j < sets; j += WARPS) {
+                        size_t stream;
+                        uint32_t r, c;
+                        const bool live = push_set(l, j, stream, r, c);
+                        uint32_t e = 0;
+                        if (live) e = load_half_ahead(L.e + o0 + c);
+                        if (j != warp) ahead = push::begin(p.push, stream, live, p.time);
+                        const uint8_t* b = bits + r * own + c;
+                        const bool idx = push::step(p.push, stream, live, p.time, ahead, live ? b[0] : 0u, live ? b[G * own] : 0u, live ? b[2 * G * own] : 0u);
+                        if (live) y[(o0 + c) * G + r] = idx ? low_half(e) : -low_half(e);   // src/model.rs:1344-1351
+                    }
+                    __syncthreads();
                 }
-            packed_outputs<1>(L.o, y, n, d, o0, own, [&](uint32_t r, uint32_t o, float v) { x[r * d + o] = __fadd_rn(x[r * d + o], v); });
-            __syncthreads();
-            share_with_cluster(x + o0, n, d, own);
-            cluster_barrier();
-            // ---- C
-            const uint16_t* const ffn_mix[1] = {L.ffn_mix};
-            mixed_inputs<1>(p, l, 1u, row, n, o0, own, L.ln2_w, L.ln2_b, ffn_mix, x, in, nothing);
-            packed_outputs<N>(L.key, in, n, d, f0, f_own, [&](uint32_t r, uint32_t o, float v) {
-                const float m = fmaxf(v, 0.0f);   // src/model.rs:999
-                act[r * ffn + o] = __fmul_rn(m, m);
-            });
-            __syncthreads();
-            share_with_cluster(act + f0, n, ffn, f_own);
-            if (l + 1u < p.n_layers) load_layer(l + 1u);
-            cluster_barrier();
+                const float* shared_out = stage == 0u ? y + o0 * G : stage == 1u ? x + o0 : act + f0 * G;
+                share_with_cluster(shared_out, stage == 1u ? n : 1u, d, stage == 0u ? own * G : stage == 1u ? own : f_own * G);
+                cluster_arrive();
+                if (stage == 0u) {
+                    // the key weights, in place of Q, K and V, and the first pieces of D
+                    if (issuer && staged && !copies.gave_up) {
+                        ptx::mbar_arrive_expect_tx(copies.key(), f_own * words * 4u);
+                        copy_bytes(w_wide, L.key.bits + (size_t)f0 * words, f_own * words * 4u, copies.key());
+                    }
+                    if (!alone) {
+#pragma unroll 1
+                        for (uint32_t i = 0; i < min(items, stages - 1u); ++i) fetch_piece(l, i);
+                    } else if (issuer && !copies.gave_up) {
+                        fetch_value(ring, p.values + l, o0, own, 0u, ffn / SLAB, copies.ring);
+                    }
+                } else if (stage == 2u && l + 1u < p.n_layers) {
+                    load_layer(l + 1u);
+                }
+                cluster_wait();
+            }
             // ---- D
             if (alone) {
-                // One warp adds, the others multiply for it, PRODUCTS inputs ahead: it is then as fast as its chain of additions.
-                asm volatile("cp.async.wait_all;" ::: "memory");
-                float sum = 0.0f;
-                for (uint32_t k = 0; k < ffn + PRODUCTS; k += PRODUCTS) {
-                    float* of = products + (k / PRODUCTS & 1u) * VALUE_OUT * PRODUCT_PITCH;
-                    const float* before = products + (~(k / PRODUCTS) & 1u) * VALUE_OUT * PRODUCT_PITCH;
-                    __syncthreads();
-                    if (warp != 0u) {
-                        if (k < ffn) value_products(ring + k / PIECE * stage_bytes, stage_bytes, act + k, min(PRODUCTS, ffn - k), warp - 1u, WARPS - 1u, of);
-                    } else if (k) {
-                        sum = sum_in_order(before + lane * PRODUCT_PITCH, min(PRODUCTS, ffn - (k - PRODUCTS)), sum);   // src/model.rs:419-436
-                    }
-                }
+                const float sum = value_alone(ring, copies, lap, act, pieces, products, p.status);
                 if (warp == 0u) x[o0 + lane] = __fadd_rn(x[o0 + lane], sum);
-            }
-            // A warp adds up 32 outputs of a row.
-            const uint32_t sums = n * tiles;
-            for (uint32_t k0 = 0; k0 < sums && !alone; k0 += WARPS) {
-                if (k0) {   // more sums than warps: the weights once more
-                    __syncthreads();
-                    for (uint32_t k = 0; k < stages - 1u; ++k) {
-                        if (k < pieces) fetch_value(ring + k * stage_bytes, L.value, o0, own, ffn, k, threadIdx.x, THREADS);
-                        copies_commit();
+                ++lap;
+            } else {
+#pragma unroll 1
+                for (uint32_t pass = 0, i = 0; pass < passes; ++pass) {
+                    const uint32_t mine = pass * WARPS + warp, tile = mine % tiles, pair = mine / tiles;
+                    float sum[N];
+#pragma unroll
+                    for (int r = 0; r < N; ++r) sum[r] = 0.0f;
+#pragma unroll 1
+                    for (uint32_t k = 0; k < pieces; ++k, ++i) {
+                        if (copier && i + stages - 1u < items) {   // into the place of the piece before this one
+                            if (i) copies_wait(copies, copies.empty() + (slot ? slot : stages) - 1u, slot ? lap : lap - 1u, p.status, 0x606u);
+                            fetch_piece(l, i + stages - 1u);
+                        }
+                        copies_wait(copies, copies.ring + slot, lap, p.status, 0x604u);
+                        if (mine < sums) value_piece<G, N>(sum, ring + slot * stage_bytes, tiles, tile, act + k * PIECE * G + pair * N, p.minus_zero);
+                        __syncwarp();
+                        if (lane == 0u) ptx::mbar_arrive(copies.empty() + slot);
+                        if (++slot == stages) { slot = 0; ++lap; }
+                    }
+                    if (mine < sums) {
+#pragma unroll
+                        for (int r = 0; r < N; ++r)
+                            if (pair * N + r < n) {
+                                float* to = x + (pair * N + r) * d + o0 + tile * VALUE_OUT + lane;
+                                *to = __fadd_rn(*to, sum[r]);
+                            }
                     }
                 }
-                const uint32_t mine = k0 + warp, tile = mine % tiles, r = mine / tiles;
-                float sum = 0.0f;
-                uint32_t at = 0;   // piece k lies in stage k % stages
-                for (uint32_t k = 0; k < pieces; ++k) {
-                    // one group is committed per piece, so all but the newest stages - 2 having landed means piece k has
-                    if (stages == 8u) asm volatile("cp.async.wait_group 6;" ::: "memory");
-                    else if (stages == 6u) asm volatile("cp.async.wait_group 4;" ::: "memory");
-                    else asm volatile("cp.async.wait_group 2;" ::: "memory");
-                    __syncthreads();   // piece k is everybody's; piece k - 1 is done with
-                    if (k + stages - 1u < pieces)
-                        fetch_value(ring + (at ? at - 1u : stages - 1u) * stage_bytes, L.value, o0, own, ffn, k + stages - 1u, threadIdx.x, THREADS);
-                    copies_commit();
-                    if (mine < sums) sum = value_piece(sum, ring + at * stage_bytes + tile * VALUE_OUT * PIECE_PITCH, act + r * ffn + k * PIECE);
-                    at = at + 1u < stages ? at + 1u : 0u;
-                }
-                if (mine < sums) {
-                    float* to = x + r * d + o0 + tile * VALUE_OUT + lane;
-                    *to = __fadd_rn(*to, sum);
-                }
             }
+            ++layers_done;
             __syncthreads();
             share_with_cluster(x + o0, n, d, own);
-            if (l + 1u < p.n_layers) ahead = push_begin(l + 1u);
-            cluster_barrier();
+            cluster_arrive();
+            if (l + 1u < p.n_layers) {
+                fetch_qkv_o(layers[(l + 1u) & 1u]);
+                ahead = push_begin(l + 1u);
+            }
+            cluster_wait();
         }
-        layer_norm(x, in, n, d, p.ln_out_w, p.ln_out_b, [&](uint32_t me, uint32_t threads) { warm_packed(p.head, v0, v_n, d, me, threads); });
+        // The head: its weights by as many outputs at a time as the ring has room for, where they lie on 16-byte borders.
+        const bool head_staged = staged && v_own * words % 4u == 0u && v_n * words % 4u == 0u;
+        const uint32_t chunk = head_staged ? max(stages * stage_bytes / (words * 4u) / 4u * 4u, 4u) : max(v_n, 1u);
+        auto fetch_head = [&](uint32_t from) {
+            if (!issuer || !head_staged || copies.gave_up) return;
+            const uint32_t bytes = min(chunk, v_n - from) * words * 4u;
+            ptx::mbar_arrive_expect_tx(copies.head(), bytes);
+            copy_bytes(ring, p.head.bits + (size_t)(v0 + from) * words, bytes, copies.head());
+        };
+        if (v_n) fetch_head(0u);
+        rows_statistics(x, in0, n, d, stats);
         __syncthreads();
-        packed_outputs<N>(p.head, x, n, d, v0, v_n, [&](uint32_t r, uint32_t o, float v) { p.logits[(size_t)(row + r) * p.vocab + o] = v; });
-        cluster_barrier();   // the rows are written anew only when nobody reads them
+#pragma unroll 1
+        for (uint32_t c = threadIdx.x; c < d; c += THREADS) {
+            const float w = h2f(p.ln_out_w[c]), b = h2f(p.ln_out_b[c]);
+            for (uint32_t r = 0; r < G; ++r) in1[c * G + r] = r < n ? normalised(x[r * d + c], stats.mean[r], stats.inv[r], w, b) : 0.0f;
+        }
+        auto emit = [&](uint32_t o, uint32_t r, float v) { p.logits[(size_t)(row + r) * p.vocab + v0 + o] = v; };
+#pragma unroll 1
+        for (uint32_t from = 0; from < v_n; from += chunk) {
+            if (from) {
+                __syncthreads();
+                fetch_head(from);
+            }
+            if (head_staged) copies_wait(copies, copies.head(), heads_done++, p.status, 0x605u);
+            __syncthreads();
+            const uint32_t* w = head_staged ? reinterpret_cast<const uint32_t*>(ring) : p.head.bits + (size_t)v0 * words;
+            const uint32_t outputs = min(chunk, v_n - from);
+            auto out = [&](uint32_t o, uint32_t r, float v) { emit(from + o, r, v); };
+            if (outputs % 4u == 0u) packed_outputs<G, 4>(p.head, w, in1, n, d, v0 + from, outputs, out);
+            else packed_outputs<G, 1>(p.head, w, in1, n, d, v0 + from, outputs, out);
+        }
+        cluster_arrive();
+        cluster_wait();   // the rows are written anew only when nobody reads them
     }
+    // After a wait that gave up, copies may still be on their way into this CTA's shared memory.
+    if (copies.gave_up && issuer)
+        for (uint32_t b = 0; b < 2u * BARS; ++b) ptx::mbar_wait(copies.ring + b / 2u, b & 1u, 1u << 16);
+    __syncthreads();
 }
 
 }  // namespace gen

@@ -861,6 +861,19 @@ void cast16(ullis_cuda_runtime* rt, const float* x, uint16_t* y, size_t rows, si
 
 }  // namespace
 
+CUtensorMap slab_map(const void* ptr, size_t rows, size_t K, unsigned box_rows, unsigned box_slabs) {
+    CUtensorMap m;
+    cuuint64_t dims[3] = {64, rows, K / 64};
+    cuuint64_t strides[2] = {K * 2, 128};
+    cuuint32_t box[3] = {64, box_rows, box_slabs};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = encode_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr,
+                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) fail(ULLIS_CUDA_ERR_CUDA, "cuTensorMapEncodeTiled failed with code " + std::to_string((int)r));
+    return m;
+}
+
 bool binary_linear(ullis_cuda_runtime* rt, const float* x, const uint32_t* bits, const uint16_t* scale,
                    const uint16_t* bias, float* y, size_t rows, size_t in_features, size_t out_features) {
     if (!usable(rt) || !shape_ok(rows, in_features, out_features) || out_features % 4) return false;

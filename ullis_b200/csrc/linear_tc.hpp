@@ -3,6 +3,8 @@
 // (validation mode, or a shape outside its tiling), in which case the caller
 // runs the CUDA-core kernels instead; nothing here ever computes on the host.
 #pragma once
+#include <cuda.h>
+
 #include "model.hpp"
 
 namespace ullis {
@@ -32,6 +34,10 @@ bool cmix_residual(ullis_cuda_runtime* rt, const LayerWeights& L, float* x, size
 // row_loss from hidden without materialising logits.
 bool head_ce(ullis_cuda_runtime* rt, const float* hidden, const PackedWeights& head, const uint32_t* labels,
              uint32_t ignore_id, size_t rows, size_t time, size_t d, size_t vocab, float* row_loss);
+
+// TMA descriptor of a [rows, K] FP16 row-major matrix by slabs of 64 columns (column in the slab, row, slab): boxes of box_slabs
+// slabs x box_rows rows, slab by slab, 128-byte swizzle.
+CUtensorMap slab_map(const void* ptr, size_t rows, size_t K, unsigned box_rows, unsigned box_slabs);
 
 // Makes a bounded device wait run out on purpose (a barrier nothing arrives on, `polls` polls): the kernel
 // returns by itself and leaves ULLIS_DEV_WAIT_TIMEOUT in the runtime's status words.
