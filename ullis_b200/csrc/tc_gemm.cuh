@@ -276,7 +276,6 @@ __device__ __forceinline__ void epilogue(const GemmParams& p, const GemmProblem&
 template <int EPI, bool PACKED>
 __global__ void __launch_bounds__(GEMM_THREADS, 3)
 gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p) {
-    chain_entry();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const uint32_t stage_bytes = (p.n_a + 1) * TILE_BYTES;
@@ -340,6 +339,7 @@ gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p) {
         ptx::tmem_alloc(tmem_slot, 128);
         ptx::tmem_relinquish();
     }
+    chain_entry();   // scale and bias are weights, which the kernel directly before never writes
     ptx::tc_fence_before_sync();
     __syncthreads();
     ptx::tc_fence_after_sync();

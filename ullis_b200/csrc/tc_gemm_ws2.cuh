@@ -47,7 +47,6 @@ inline WsShape ws2_shape(uint32_t K, uint32_t n_a, int epi, bool resident_w = tr
 template <int EPI, bool RESIDENT_W = true>
 __global__ void __launch_bounds__(WS2_THREADS, 1)
 gemm_ws2_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p, const uint32_t pairs) {
-    chain_entry();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint32_t KB = p.K / BK, kb0 = 0;
@@ -141,6 +140,7 @@ gemm_ws2_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p, const
         }
     }
     ptx::fence_proxy_async_smem();  // generic-proxy stores -> visible to the MMA's async reads
+    chain_entry();                  // as in gemm_ws_kernel: what was read so far are weights
     ptx::tc_fence_before_sync();
     __syncthreads();                // the table is dead, the ring may be filled
     ptx::cluster_sync_all();        // both CTAs: barriers initialised, weights expanded, TMEM allocated
