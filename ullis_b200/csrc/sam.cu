@@ -388,6 +388,7 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
     uint16_t* nq = reinterpret_cast<uint16_t*>(context_mem + L.nq);
     uint32_t* nq2 = reinterpret_cast<uint32_t*>(context_mem + L.nq);
     uint16_t* start = reinterpret_cast<uint16_t*>(context_mem + L.start);
+    uint32_t* start2 = reinterpret_cast<uint32_t*>(context_mem + L.start);
     uint32_t* Q = reinterpret_cast<uint32_t*>(context_mem + L.q);
     uint32_t* K = reinterpret_cast<uint32_t*>(context_mem + L.k);
     uint16_t* q_ends = reinterpret_cast<uint16_t*>(context_mem + L.q_ends);
@@ -449,7 +450,9 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
             uint32_t sum = 0, pairs = 0;
             for (uint32_t j = j0; j < j1; ++j) {
                 uint32_t n = 0;
+#pragma unroll 8
                 for (uint32_t w = 0; w < NW; ++w) n += hist2[w * pair_words + j];
+                start2[j] = n;
                 const uint32_t m = nq2[j];
                 pairs += (n & 0xFFFFu) * (m & 0xFFFFu) + (n >> 16) * (m >> 16);
                 sum += (n & 0xFFFFu) + (n >> 16) + (((m & 0xFFFFu) + (m >> 16)) << 16);
@@ -482,17 +485,25 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
                 taken = true;
             }
             if (taken) {
+                // two buckets side by side, eight counts in flight (one after the other they were 64 trips for 32 warps)
                 uint32_t run_k = run & 0xFFFFu, run_q = run >> 16;
-                for (uint32_t x = 2u * j0; x < 2u * j1; ++x) {
-                    start[x] = (uint16_t)run_k;
-                    for (uint32_t w = 0; w < NW; ++w) {
-                        const uint32_t n = hist[w * C + x];
-                        hist[w * C + x] = (uint16_t)run_k;
-                        run_k += n;
+                for (uint32_t j = j0; j < j1; ++j) {
+                    const uint32_t n = start2[j], m = nq2[j];
+                    uint32_t at = run_k | (run_k + (n & 0xFFFFu)) << 16;
+                    start2[j] = at;
+                    for (uint32_t w0 = 0; w0 < NW; w0 += 8u) {
+                        uint32_t counts[8];
+#pragma unroll
+                        for (uint32_t u = 0; u < 8u; ++u) counts[u] = hist2[(w0 + u) * pair_words + j];
+#pragma unroll
+                        for (uint32_t u = 0; u < 8u; ++u) {
+                            hist2[(w0 + u) * pair_words + j] = at;
+                            at += counts[u];
+                        }
                     }
-                    const uint32_t m = nq[x];
-                    nq[x] = (uint16_t)run_q;
-                    run_q += m;
+                    nq2[j] = run_q | (run_q + (m & 0xFFFFu)) << 16;
+                    run_k += (n & 0xFFFFu) + (n >> 16);
+                    run_q += (m & 0xFFFFu) + (m >> 16);
                 }
                 if (threadIdx.x == 0) start[C] = (uint16_t)T;
             }
