@@ -214,8 +214,9 @@ RC_HD int32_t scan_agreement(int32_t best) { return 31 - ((best + (int32_t)scan_
 constexpr int32_t SCAN_NOTHING = 32 * 65536;
 RC_HD bool scan_full(int32_t best) { return best <= -65536; }   // a whole window agrees
 
-// Where the search for step t begins: with `wide` sets of as many context bits as leave 4 to 8 positions before t on
-// evenly spread keys, otherwise with all c bits - the buckets [first, first + n).
+// Where the search for step t begins: with `wide` sets of as many context bits as leave 2 to 4 positions before t on
+// evenly spread keys (4 to 8: contexts of 16 sequences in training 6.07 ms, not 5.80), otherwise with all c bits - the
+// buckets [first, first + n).
 struct Query {
     uint32_t wq, ctx, l, first, n;
 };
@@ -224,7 +225,7 @@ RC_HD Query query(const uint32_t* Q, uint32_t c, bool wide, uint32_t t) {
     z.wq = window(Q, t);
     z.ctx = z.wq >> (32u - c);
     z.l = c;
-    if (wide && 29u - leading(t) < c) z.l = 29u - leading(t);  // floor(log2 t) - 2
+    if (wide && 30u - leading(t) < c) z.l = 30u - leading(t);  // floor(log2 t) - 1
     z.first = z.ctx >> (c - z.l) << (c - z.l);
     z.n = 1u << (c - z.l);
     return z;
