@@ -29,7 +29,8 @@ int32_t guard(ullis_cuda_runtime* rt, F&& body) {
     // the caller's again, and the library's buffers.
     const auto failed = [&](int32_t code, const char* msg) {
         rt->last_error = msg;
-        if (rt->stream) cudaStreamSynchronize(rt->stream);
+        for (cudaStream_t s : {rt->stream, rt->copy_in, rt->copy_out})
+            if (s) cudaStreamSynchronize(s);
         return code;
     };
     try {
@@ -100,6 +101,50 @@ struct Inputs {
     }
 };
 
+// An op-level call in shares: the inputs of a share are copied while the one before it is computed, its results while the
+// next one is; the link carries both directions at once.  A copy to or from ordinary (pageable) memory holds the host up, so
+// results that do not go to page-locked memory are asked for only when everything else is enqueued.  copy_in(share, stream)
+// copies, compute(share) enqueues kernels on rt->stream, copy_out(share, stream) copies.
+template <typename In, typename Compute, typename Out>
+void in_shares(ullis_cuda_runtime* rt, size_t shares, bool results_locked, In copy_in, Compute compute, Out copy_out) {
+    if (shares <= 1) {
+        copy_in(0, rt->stream);
+        compute(0);
+        copy_out(0, rt->stream);
+        return;
+    }
+    rt->copy_streams();
+    for (size_t s = 0; s < shares; ++s) {
+        copy_in(s, s ? rt->copy_in : rt->stream);
+        if (s) {
+            ULLIS_CUDA_CHECK(cudaEventRecord(rt->share_in[s], rt->copy_in));
+            ULLIS_CUDA_CHECK(cudaStreamWaitEvent(rt->stream, rt->share_in[s], 0));
+        }
+        compute(s);
+        ULLIS_CUDA_CHECK(cudaEventRecord(rt->share_out[s], rt->stream));
+        ULLIS_CUDA_CHECK(cudaStreamWaitEvent(rt->copy_out, rt->share_out[s], 0));
+        if (results_locked) copy_out(s, rt->copy_out);
+    }
+    for (size_t s = 0; s < shares && !results_locked; ++s) copy_out(s, rt->copy_out);
+    ULLIS_CUDA_CHECK(cudaEventRecord(rt->copies_done, rt->copy_out));
+    ULLIS_CUDA_CHECK(cudaStreamWaitEvent(rt->stream, rt->copies_done, 0));
+}
+// Shares of a call: each with results of 4 MiB at least (about 80 us on the link, where a share costs its launches) and `least` of
+// the `items` that it is cut by.
+size_t shares_for(size_t result_bytes, size_t items, size_t least) {
+    return std::max<size_t>(1, std::min({ullis_cuda_runtime::MAX_SHARES, result_bytes >> 22, items / std::max<size_t>(least, 1)}));
+}
+bool page_locked(const void* p) {
+    cudaPointerAttributes attr;
+    if (p && cudaPointerGetAttributes(&attr, p) == cudaSuccess) return attr.type == cudaMemoryTypeHost;
+    cudaGetLastError();
+    return false;
+}
+template <typename T>
+void copy_async(T* dst, const T* src, size_t count, cudaMemcpyKind kind, cudaStream_t stream) {
+    if (count) ULLIS_CUDA_CHECK(cudaMemcpyAsync(dst, src, count * sizeof(T), kind, stream));
+}
+
 void packed_linear_dev(ullis_cuda_runtime* rt, const float* x, const uint32_t* bits, const uint16_t* scale,
                        const uint16_t* bias, float* y, size_t rows, size_t K, size_t N) {
     if (rt->mode == ULLIS_CUDA_MODE_EXACT || !tc::binary_linear(rt, x, bits, scale, bias, y, rows, K, N))
@@ -119,6 +164,16 @@ void set_global_error(const char* msg) {
     snprintf(g_global_error, sizeof(g_global_error), "%s", msg ? msg : "");
 }
 }  // namespace ullis
+
+void ullis_cuda_runtime::copy_streams() {
+    if (copies_done) return;
+    for (cudaStream_t* s : {&copy_in, &copy_out})
+        if (!*s) ULLIS_CUDA_CHECK(cudaStreamCreateWithFlags(s, cudaStreamNonBlocking));
+    for (size_t i = 0; i < MAX_SHARES; ++i)
+        for (cudaEvent_t* e : {&share_in[i], &share_out[i]})
+            if (!*e) ULLIS_CUDA_CHECK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+    ULLIS_CUDA_CHECK(cudaEventCreateWithFlags(&copies_done, cudaEventDisableTiming));   // last: all of them are there
+}
 
 // Child runtime i of a lane-splitting forward: a stream, scratch and timing marks of its own; everything that
 // configures kernels is copied from the parent on every request, and the status words are the parent's.
@@ -396,6 +451,15 @@ void ullis_cuda_runtime_destroy(ullis_cuda_runtime* rt) {
         cudaStreamSynchronize(rt->side_stream);
         cudaStreamDestroy(rt->side_stream);
     }
+    for (cudaStream_t s : {rt->copy_in, rt->copy_out})
+        if (s) {
+            cudaStreamSynchronize(s);
+            cudaStreamDestroy(s);
+        }
+    for (size_t i = 0; i < ullis_cuda_runtime::MAX_SHARES; ++i)
+        for (cudaEvent_t e : {rt->share_in[i], rt->share_out[i]})
+            if (e) cudaEventDestroy(e);
+    if (rt->copies_done) cudaEventDestroy(rt->copies_done);
     if (rt->inputs_host) cudaFreeHost(rt->inputs_host);   // behind the wait
     if (rt->side_fork) cudaEventDestroy(rt->side_fork);
     if (rt->side_join) cudaEventDestroy(rt->side_join);
@@ -475,13 +539,19 @@ int32_t ullis_cuda_runtime_sam_counts(ullis_cuda_runtime* rt, uint64_t* total, u
         for (size_t lane = 0; lane < rt->lanes_last; ++lane) {
             ullis_cuda_runtime* r = lane == 0 ? rt : rt->children.at(lane - 1);
             uint32_t host[2] = {0, 0};
+            uint32_t shares[2 * ullis_cuda_runtime::MAX_SHARES] = {};
             if (r->sam_last_streams) {
-                r->d2h(host, r->sam_last_counts, 8);
+                if (r->sam_shares > 1) r->d2h(shares, r->sam_share_counts.get(), 8 * r->sam_shares);
+                else r->d2h(host, r->sam_last_counts, 8);
                 r->sync();
             }
             sum[0] += r->sam_last_streams;
             sum[1] += host[0];
             sum[2] += host[1];
+            for (size_t s = 0; s < r->sam_shares && r->sam_shares > 1; ++s) {
+                sum[1] += shares[2 * s];
+                sum[2] += shares[2 * s + 1];
+            }
         }
         if (total) *total = sum[0];
         if (automaton) *automaton = sum[1];
@@ -916,16 +986,30 @@ int32_t ullis_cuda_binary_linear(ullis_cuda_runtime* rt, const float* x, const u
         const size_t words = (mul_or_fail(in_features, out_features, "packed linear") + 31) / 32;
         if (rows == 0) return;
         need_ptr(x, "x"); need_ptr(bits, "bits"); need_ptr(scale, "scale"); need_ptr(y, "y");
+        // whole 256-row tiles in every share but the last
+        const size_t shares = shares_for(ny * 4, rows, 256), share_rows = ((rows + shares - 1) / shares + 255) / 256 * 256;
         Inputs in(rt);
-        float* dx = in.add(0, x, nx);
+        float* dx = shares > 1 ? rt->pool[0].as<float>(nx) : in.add(0, x, nx);
         uint32_t* dbits = in.add(1, bits, words);
         uint16_t* ds = in.add(2, scale, out_features);
         uint16_t* db = bias ? in.add(3, bias, out_features) : nullptr;
         float* dy = rt->pool[4].as<float>(ny);
         in.send();
         rt->clear_status();
-        packed_linear_dev(rt, dx, dbits, ds, db, dy, rows, in_features, out_features);
-        rt->d2h(y, dy, ny * 4);
+        const auto first = [&](size_t s) { return std::min(rows, s * share_rows); };
+        const auto count = [&](size_t s) { return first(s + 1) - first(s); };
+        in_shares(rt, shares, shares > 1 && page_locked(y),
+            [&](size_t s, cudaStream_t stream) {
+                if (shares > 1) copy_async(dx + first(s) * in_features, x + first(s) * in_features, count(s) * in_features, cudaMemcpyHostToDevice, stream);
+            },
+            [&](size_t s) {
+                const size_t r = shares > 1 ? first(s) : 0, n = shares > 1 ? count(s) : rows;
+                if (n) packed_linear_dev(rt, dx + r * in_features, dbits, ds, db, dy + r * out_features, n, in_features, out_features);
+            },
+            [&](size_t s, cudaStream_t stream) {
+                const size_t r = shares > 1 ? first(s) : 0, n = shares > 1 ? count(s) : rows;
+                copy_async(y + r * out_features, dy + r * out_features, n * out_features, cudaMemcpyDeviceToHost, stream);
+            });
         rt->check_status();
     });
 }
@@ -998,26 +1082,43 @@ int32_t ullis_cuda_rosa_qkv_1bit_fwd(ullis_cuda_runtime* rt, const uint32_t* q_b
         const size_t n = mul_or_fail(mul_or_fail(batch, time, "ROSA"), channels, "ROSA");
         need_ptr(q_bits, "q_bits"); need_ptr(k_bits, "k_bits"); need_ptr(v_bits, "v_bits"); need_ptr(e, "e");
         const size_t words = (n + 31) / 32, wps = (time + 31) / 32, sw = batch * channels * wps;
+        // Shares of whole sequences, whose planes begin on a word; 1 024 streams keep the device busy (not in the automaton, whose
+        // launches last as long as a stream).
+        const size_t result_bytes = (idx ? n : 0) + (out ? n * 4 : 0);
+        const size_t shares = time * channels % 32 || !k::rosa_without_automaton(rt, batch * channels, time) ? 1 : shares_for(result_bytes, batch, (1023 + channels) / channels);
         Inputs in(rt);
-        uint32_t* dq = in.add(0, q_bits, words);
-        uint32_t* dk = in.add(1, k_bits, words);
-        uint32_t* dv = in.add(2, v_bits, words);
+        uint32_t* planes[3];
+        const uint32_t* const host[3] = {q_bits, k_bits, v_bits};
+        for (int a = 0; a < 3; ++a) planes[a] = shares > 1 ? rt->pool[a].as<uint32_t>(words) : in.add(a, host[a], words);
         uint16_t* de = in.add(3, e, channels);
-        uint32_t* qs = rt->pool[4].as<uint32_t>(sw);
-        uint32_t* ks = rt->pool[5].as<uint32_t>(sw);
-        uint32_t* vs = rt->pool[6].as<uint32_t>(sw);
+        uint32_t* streams[3];
+        for (int a = 0; a < 3; ++a) streams[a] = rt->pool[4 + a].as<uint32_t>(sw);
         uint32_t* is = rt->pool[7].as<uint32_t>(sw);
-        in.send();
-        k::planes_to_streams(rt, dq, qs, batch, time, channels);
-        k::planes_to_streams(rt, dk, ks, batch, time, channels);
-        k::planes_to_streams(rt, dv, vs, batch, time, channels);
-        rt->clear_status();
-        k::rosa_sam(rt, qs, ks, vs, is, batch * channels, time);
         uint8_t* didx = idx ? rt->pool[8].as<uint8_t>(n) : nullptr;
         float* dout = out ? rt->pool[9].as<float>(n) : nullptr;
-        if (idx || out) k::rosa_emit(rt, is, de, didx, dout, batch, time, channels);
-        if (idx) rt->d2h(idx, didx, n);
-        if (out) rt->d2h(out, dout, n * 4);
+        uint32_t* counts = shares > 1 ? rt->sam_share_counts.as<uint32_t>(2 * ullis_cuda_runtime::MAX_SHARES) : nullptr;
+        in.send();
+        rt->clear_status();
+        const auto first = [&](size_t s) { return batch * s / shares; };
+        in_shares(rt, shares, shares > 1 && page_locked(out ? static_cast<const void*>(out) : idx),
+            [&](size_t s, cudaStream_t stream) {
+                const size_t w0 = first(s) * time * channels / 32, w1 = first(s + 1) * time * channels / 32;
+                for (int a = 0; a < 3 && shares > 1; ++a) copy_async(planes[a] + w0, host[a] + w0, w1 - w0, cudaMemcpyHostToDevice, stream);
+            },
+            [&](size_t s) {
+                const size_t b0 = first(s), b = first(s + 1) - b0, at = b0 * time * channels;
+                for (int a = 0; a < 3; ++a) k::planes_to_streams(rt, planes[a] + at / 32, streams[a], b, time, channels);
+                k::rosa_sam(rt, streams[0], streams[1], streams[2], is, b * channels, time);
+                if (shares > 1) ULLIS_CUDA_CHECK(cudaMemcpyAsync(counts + 2 * s, rt->sam_last_counts, 8, cudaMemcpyDeviceToDevice, rt->stream));
+                if (idx || out) k::rosa_emit(rt, is, de, idx ? didx + at : nullptr, out ? dout + at : nullptr, b, time, channels);
+            },
+            [&](size_t s, cudaStream_t stream) {
+                const size_t at = first(s) * time * channels, count = first(s + 1) * time * channels - at;
+                if (idx) copy_async(idx + at, didx + at, count, cudaMemcpyDeviceToHost, stream);
+                if (out) copy_async(out + at, dout + at, count, cudaMemcpyDeviceToHost, stream);
+            });
+        rt->sam_shares = shares;
+        rt->sam_last_streams = batch * channels;
         rt->check_status();
     });
 }

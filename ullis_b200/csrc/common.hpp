@@ -149,6 +149,14 @@ struct ullis_cuda_runtime {
     ullis::DeviceBuffer sam_list;       // ids of the streams that need the automaton + their count
     size_t sam_last_streams = 0;        // streams of the last suffix-automaton call ...
     const uint32_t* sam_last_counts = nullptr;   // ... and its counters: listed, constant q
+    // Copies beside kernels: an op-level call with large results runs in shares, whose inputs and results travel on streams of
+    // their own while `stream` computes.  Created on first use; idle whenever no call is running.
+    static constexpr size_t MAX_SHARES = 4;
+    cudaStream_t copy_in = nullptr, copy_out = nullptr;
+    cudaEvent_t share_in[MAX_SHARES] = {}, share_out[MAX_SHARES] = {}, copies_done = nullptr;
+    void copy_streams();
+    size_t sam_shares = 1;                       // of the last suffix-automaton call; if more than one, the counters of each:
+    ullis::DeviceBuffer sam_share_counts;
     ullis::DeviceBuffer tc_ws[16];      // 16-bit operands / partials of the tensor-core stages
     int tc_stages = 2, tc_stages2 = 2;  // GEMM pipeline depth with one / two activation operands
     bool tc_ws_kernel = true;           // weight-stationary persistent kernel for packed weights with K <= 512

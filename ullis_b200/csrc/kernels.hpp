@@ -50,6 +50,8 @@ bool binary_rowvec_multi(ullis_cuda_runtime* rt, int count, const float* const* 
 // is about to record them into a CUDA graph does it beforehand.
 void rowvec_prepare(ullis_cuda_runtime* rt);
 
+// Whether rosa_sam() answers a call of this shape without the automaton.
+bool rosa_without_automaton(const ullis_cuda_runtime* rt, size_t streams, size_t time);
 // ---- sam.cu
 // idx_sw <- suffix-automaton match of each stream; uses rt->sam_scratch.  `site` names the caller's call site (a
 // model passes its layer): calls of one site are expected to send a similar number of streams to the automaton,

@@ -940,13 +940,18 @@ size_t rosa_sam_scratch_bytes_per_stream(int algo, size_t time) {
     return narrow ? stride_for<uint16_t>(algo, time) : stride_for<uint32_t>(algo, time);
 }
 
+bool rosa_without_automaton(const ullis_cuda_runtime* rt, size_t streams, size_t time) {
+    return rt->sam_algo == ULLIS_CUDA_SAM_EULER && !rt->sam_automaton && time <= MATCH_MAX_TIME && streams * ((time + 31) / 32) < 0x7FFFFFFFull;
+}
+
 void rosa_sam(ullis_cuda_runtime* rt, const uint32_t* q_sw, const uint32_t* k_sw, const uint32_t* v_sw,
               uint32_t* idx_sw, size_t streams, size_t time, int site) {
     if (streams == 0 || time == 0) return;
     if (time > 0x3FFFFFFFu) fail(ULLIS_CUDA_ERR_SHAPE, "ROSA time does not fit 32-bit state ids");
     const int algo = rt->sam_algo;
     if (streams > 0xFFFFFFFFull) fail(ULLIS_CUDA_ERR_SHAPE, "too many ROSA streams");
-    if (algo == ULLIS_CUDA_SAM_EULER && !rt->sam_automaton && time <= MATCH_MAX_TIME && streams * ((time + 31) / 32) < 0x7FFFFFFFull) {
+    rt->sam_shares = 1;
+    if (rosa_without_automaton(rt, streams, time)) {
         rosa_match(rt, q_sw, k_sw, v_sw, idx_sw, streams, (uint32_t)time);
         return;
     }
