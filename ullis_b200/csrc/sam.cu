@@ -793,10 +793,15 @@ struct MatchCall {   // the buffers of one call
 // The shapes of the context kernel: threads per stream, and whether a warp takes a large bucket together.
 enum ContextShape { CONTEXT_256, CONTEXT_512, CONTEXT_1024, CONTEXT_SHAPES };
 
+// Context bits of a launch.  One more for uneven streams, where shared memory has room for it: their large buckets halve (default
+// model, contexts of 64 sequences 7.44 -> 7.14 ms, of one 0.89 -> 0.85); evenly spread ones pay more for the sort than they save
+// (16 in training 6.1 -> 7.6 ms; 8192 steps, where one shape takes both, 2.47 -> 2.69).
+uint32_t context_bits(uint32_t T, bool uneven) { return context::bits_for(T) + (uneven && T <= 4096u ? 1u : 0u); }
+
 template <int NT, bool TOGETHER>
 void prepare_context(ullis_cuda_runtime* rt, uint32_t T, int shape) {
     const auto kernel = rosa_context_kernel<NT, TOGETHER>;
-    const size_t smem = ContextLayout(T, context::bits_for(T), NT / 32).total;
+    const size_t smem = ContextLayout(T, context_bits(T, TOGETHER), NT / 32).total;
     if (!rt->context_smem[shape]) {   // the attribute belongs to the function, not to this runtime: always the same value
         const size_t most = ContextLayout((uint32_t)MATCH_MAX_TIME, context::bits_for((uint32_t)MATCH_MAX_TIME), NT / 32).total;
         ULLIS_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
@@ -819,7 +824,7 @@ void launch_context(ullis_cuda_runtime* rt, const MatchCall& m, int shape, uint3
     // ever change went to the match kernel).
     const ContextLimits limits{24u, 96u, 160u, 64u, 256u};
     rt->chain(rosa_context_kernel<NT, TOGETHER>, grid, NT, rt->context_smem[shape], m.q, m.k, m.v, m.idx, m.list, m.counts,
-              m.counts + 3, m.hard, m.counts + 2, m.T, m.wps, context::bits_for(m.T), limits, from, to);
+              m.counts + 3, m.hard, m.counts + 2, m.T, m.wps, context_bits(m.T, TOGETHER && from == 0u), limits, from, to);
     rt->launched(what);
 }
 
