@@ -135,24 +135,52 @@ mix_split_kernel(const float* __restrict__ x, const uint16_t* __restrict__ m0, c
 // values), forms the mixes and writes the 16-bit operands; the LayerNorm output itself is only written when
 // something downstream reads it as f32 (`ln_out`: the exact sign fix-up).  Saves the round trip of the
 // LayerNorm output through HBM.  C = 128 * VEC channels, VEC <= 8.
-template <int VEC, int ROWS>
-__global__ void __launch_bounds__(256)
+// A warp takes one row, or (SEVERAL) `per_warp` consecutive ones: the LayerNorm of a row is then computed once and handed
+// on as the next row's "row before" (with one every row is normalised twice, by its own warp and by its successor's).
+// MIXES = 1: one operand in 16 bits alone (m0 -> hi0; no lo, s1, ln_out).
+// Bound by memory for many rows and by a warp's chain of load, two reductions and store for few: everything the rows
+// share is loaded with the first row, and a row's loads go out before the row before it is worked on.
+template <int VEC, bool SEVERAL, int MIXES>
+__global__ void __launch_bounds__(256, VEC <= 4 ? 2 : 1)
 ln_mix_split_kernel(const float* __restrict__ x, const uint16_t* __restrict__ lw, const uint16_t* __restrict__ lb,
                     float* __restrict__ ln_out, const uint16_t* __restrict__ m0, const uint16_t* __restrict__ m1,
                     const uint16_t* __restrict__ m2, uint16_t* __restrict__ hi0, uint16_t* __restrict__ lo0,
                     uint16_t* __restrict__ hi1, uint16_t* __restrict__ lo1, uint16_t* __restrict__ hi2,
-                    uint16_t* __restrict__ lo2, float* __restrict__ s1, size_t rows, size_t time, size_t pitch) {
+                    uint16_t* __restrict__ lo2, float* __restrict__ s1, uint32_t rows, uint32_t time, uint32_t pitch,
+                    uint32_t per_warp) {
     chain_entry();
     constexpr int C = 128 * VEC;
-    const int lane = threadIdx.x & 31;
-    // a warp takes ROWS consecutive rows: the LayerNorm of a row is then computed once and handed on as the next
-    // row's "row before" (with ROWS = 1 every row is normalised twice, by its own warp and by its successor's)
-    const size_t row0 = ((size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * ROWS;
+    // as far as the registers go
+    constexpr bool AHEAD = SEVERAL && VEC <= 4, MIX_FIRST = VEC <= 4 && (MIXES == 1 || !SEVERAL);
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t row0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (SEVERAL ? per_warp : 1u);
     if (row0 >= rows) return;
-    const uint2* w4 = reinterpret_cast<const uint2*>(lw);
-    const uint2* b4 = reinterpret_cast<const uint2*>(lb);
+    const uint32_t last = SEVERAL ? min(row0 + per_warp, rows) : row0 + 1;
+    const uint16_t* mix[3] = {m0, m1, m2};
+    uint16_t* hi[3] = {hi0, hi1, hi2};
+    uint16_t* lo[3] = {lo0, lo1, lo2};
+    uint32_t seq = row0 / time, step = row0 - seq * time;
+    float4 cur[VEC], prev[VEC], next[VEC];
+    uint2 w[VEC], b[VEC], m[MIXES][VEC];
+    const auto load_row = [&](float4 (&v)[VEC], uint32_t row) {
+        const float4* src = reinterpret_cast<const float4*>(x + (size_t)row * C) + lane;
+#pragma unroll
+        for (int i = 0; i < VEC; ++i) v[i] = src[32 * i];
+    };
+    load_row(cur, row0);
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) prev[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (step) load_row(prev, row0 - 1);
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) {
+        w[i] = reinterpret_cast<const uint2*>(lw)[lane + 32 * i];
+        b[i] = reinterpret_cast<const uint2*>(lb)[lane + 32 * i];
+#pragma unroll
+        for (int k = 0; k < MIXES; ++k)
+            if (MIX_FIRST) m[k][i] = reinterpret_cast<const uint2*>(mix[k])[lane + 32 * i];
+    }
     // normalised values of one row, in place
-    auto layer_norm_row = [&](float4 (&v)[VEC]) {
+    const auto layer_norm_row = [&](float4 (&v)[VEC]) {
         float sum = 0.0f;
 #pragma unroll
         for (int i = 0; i < VEC; ++i) sum += (v[i].x + v[i].y) + (v[i].z + v[i].w);
@@ -170,79 +198,73 @@ ln_mix_split_kernel(const float* __restrict__ x, const uint16_t* __restrict__ lw
         const float inv = 1.0f / sqrtf(sq / (float)C + 1e-5f);
 #pragma unroll
         for (int i = 0; i < VEC; ++i) {
-            const uint2 wb = w4[lane + 32 * i], bb = b4[lane + 32 * i];
-            v[i].x = (v[i].x - mean) * inv * h2f((uint16_t)(wb.x & 0xffff)) + h2f((uint16_t)(bb.x & 0xffff));
-            v[i].y = (v[i].y - mean) * inv * h2f((uint16_t)(wb.x >> 16)) + h2f((uint16_t)(bb.x >> 16));
-            v[i].z = (v[i].z - mean) * inv * h2f((uint16_t)(wb.y & 0xffff)) + h2f((uint16_t)(bb.y & 0xffff));
-            v[i].w = (v[i].w - mean) * inv * h2f((uint16_t)(wb.y >> 16)) + h2f((uint16_t)(bb.y >> 16));
+            v[i].x = (v[i].x - mean) * inv * h2f((uint16_t)(w[i].x & 0xffff)) + h2f((uint16_t)(b[i].x & 0xffff));
+            v[i].y = (v[i].y - mean) * inv * h2f((uint16_t)(w[i].x >> 16)) + h2f((uint16_t)(b[i].x >> 16));
+            v[i].z = (v[i].z - mean) * inv * h2f((uint16_t)(w[i].y & 0xffff)) + h2f((uint16_t)(b[i].y & 0xffff));
+            v[i].w = (v[i].w - mean) * inv * h2f((uint16_t)(w[i].y >> 16)) + h2f((uint16_t)(b[i].y >> 16));
         }
     };
-    float4 cur[VEC], prev[VEC];
-#pragma unroll
-    for (int i = 0; i < VEC; ++i) prev[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    const uint16_t* mix[3] = {m0, m1, m2};
-    uint16_t* hi[3] = {hi0, hi1, hi2};
-    uint16_t* lo[3] = {lo0, lo1, lo2};
+    layer_norm_row(prev);   // of a sequence's first step: not used
 #pragma unroll 1
-    for (int r = 0; r < ROWS; ++r) {
-    const size_t row = row0 + r;
-    if (row >= rows) break;
-    const bool first = row % time == 0;   // the same for the whole warp
-    const size_t orow = row + row / time * (pitch - time), orows = rows / time * pitch;
-    const float4* src = reinterpret_cast<const float4*>(x + row * C);
+    for (uint32_t row = row0; row < last; ++row) {
+        if (AHEAD && row + 1 < last) load_row(next, row + 1);
+        const bool first = step == 0;   // the same for the whole warp
+        const size_t orow = (size_t)seq * pitch + step;
+        layer_norm_row(cur);
+        if (MIXES > 1 && ln_out) {
+            float4* dst = reinterpret_cast<float4*>(ln_out + (size_t)row * C) + lane;
 #pragma unroll
-    for (int i = 0; i < VEC; ++i) cur[i] = src[lane + 32 * i];
-    if (r == 0 && !first) {
+            for (int i = 0; i < VEC; ++i) dst[32 * i] = cur[i];
+        }
+        float sum[MIXES] = {};
 #pragma unroll
-        for (int i = 0; i < VEC; ++i) prev[i] = (src - C / 4)[lane + 32 * i];
-        layer_norm_row(prev);
-    }
-    layer_norm_row(cur);
-    if (ln_out) {
-        float4* dst = reinterpret_cast<float4*>(ln_out + row * C);
+        for (int i = 0; i < VEC; ++i) {
+            const float xt[4] = {cur[i].x, cur[i].y, cur[i].z, cur[i].w};
+            const float pt[4] = {prev[i].x, prev[i].y, prev[i].z, prev[i].w};
+            float xx[4];
 #pragma unroll
-        for (int i = 0; i < VEC; ++i) dst[lane + 32 * i] = cur[i];
-    }
-    float sum[3] = {0.0f, 0.0f, 0.0f};
+            for (int e = 0; e < 4; ++e) xx[e] = first ? -xt[e] : __fsub_rn(pt[e], xt[e]);
 #pragma unroll
-    for (int i = 0; i < VEC; ++i) {
-        const size_t c = (size_t)(lane + 32 * i) * 4;
-        const float xt[4] = {cur[i].x, cur[i].y, cur[i].z, cur[i].w}, pt[4] = {prev[i].x, prev[i].y, prev[i].z, prev[i].w};
-        float xx[4];
+            for (int k = 0; k < MIXES; ++k) {
+                if (!MIX_FIRST) m[k][i] = reinterpret_cast<const uint2*>(mix[k])[lane + 32 * i];
+                const uint32_t mb[4] = {m[k][i].x & 0xFFFFu, m[k][i].x >> 16, m[k][i].y & 0xFFFFu, m[k][i].y >> 16};
+                float v[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) xx[e] = first ? -xt[e] : __fsub_rn(pt[e], xt[e]);
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            if (!mix[k]) continue;
-            const uint2 mw = *reinterpret_cast<const uint2*>(mix[k] + c);
-            const uint16_t mb[4] = {(uint16_t)(mw.x & 0xFFFFu), (uint16_t)(mw.x >> 16), (uint16_t)(mw.y & 0xFFFFu),
-                                    (uint16_t)(mw.y >> 16)};
-            uint16_t hb[4], lbt[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float v = __fadd_rn(xt[e], __fmul_rn(xx[e], h2f(mb[e])));
-                const __half h = __float2half_rn(v);
-                hb[e] = __half_as_ushort(h);
-                lbt[e] = __half_as_ushort(__float2half_rn(v - __half2float(h)));
-                sum[k] += fabsf(v);
+                for (int e = 0; e < 4; ++e) {
+                    v[e] = __fadd_rn(xt[e], __fmul_rn(xx[e], h2f((uint16_t)mb[e])));
+                    if (MIXES > 1) sum[k] += fabsf(v[e]);
+                }
+                const size_t at = orow * C + (lane + 32 * i) * 4;
+                const __half2 h01 = __floats2half2_rn(v[0], v[1]), h23 = __floats2half2_rn(v[2], v[3]);
+                *reinterpret_cast<uint2*>(hi[k] + at) =
+                    make_uint2(*reinterpret_cast<const uint32_t*>(&h01), *reinterpret_cast<const uint32_t*>(&h23));
+                if (MIXES > 1) {
+                    const float2 f01 = __half22float2(h01), f23 = __half22float2(h23);
+                    const __half2 l01 = __floats2half2_rn(v[0] - f01.x, v[1] - f01.y);
+                    const __half2 l23 = __floats2half2_rn(v[2] - f23.x, v[3] - f23.y);
+                    *reinterpret_cast<uint2*>(lo[k] + at) =
+                        make_uint2(*reinterpret_cast<const uint32_t*>(&l01), *reinterpret_cast<const uint32_t*>(&l23));
+                }
             }
-            *reinterpret_cast<uint2*>(hi[k] + orow * C + c) =
-                make_uint2(hb[0] | ((uint32_t)hb[1] << 16), hb[2] | ((uint32_t)hb[3] << 16));
-            if (lo[k])
-                *reinterpret_cast<uint2*>(lo[k] + orow * C + c) =
-                    make_uint2(lbt[0] | ((uint32_t)lbt[1] << 16), lbt[2] | ((uint32_t)lbt[3] << 16));
         }
-    }
-    if (s1) {
+        if (MIXES > 1) {
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            float s = sum[k];
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (lane == 0 && mix[k]) s1[k * orows + orow] = s;
+            for (int k = 0; k < MIXES; ++k) {
+                float s = sum[k];
+                for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+                if (lane == 0) s1[(size_t)k * (rows / time * pitch) + orow] = s;
+            }
         }
-    }
 #pragma unroll
-    for (int i = 0; i < VEC; ++i) prev[i] = cur[i];
+        for (int i = 0; i < VEC; ++i) {
+            prev[i] = cur[i];
+            if (AHEAD) cur[i] = next[i];
+        }
+        if (SEVERAL && !AHEAD && row + 1 < last) load_row(cur, row + 1);
+        if (++step == time) {
+            step = 0;
+            ++seq;
+        }
     }
 }
 
@@ -831,22 +853,22 @@ bool launch_ln_mix_split(ullis_cuda_runtime* rt, const float* x, const LayerNorm
                          uint16_t* hi1, uint16_t* lo1, uint16_t* hi2, uint16_t* lo2, float* s1, size_t rows, size_t time,
                          size_t pitch, size_t d, const char* what) {
     if (!rt->tc_fuse_ln || d % 128 != 0 || d > 1024) return false;
-    // rows per warp: several once there are enough rows to fill the device with warps anyway
-    // (measured at 131 072 rows: the Q/K/V form, bound by its 0.8 GB of stores, is best with two; the one-operand
-    // form, bound by instruction issue, with four)
-    const int per_warp = rt->tc_ln_rows > 0 ? rt->tc_ln_rows : rows < 32768 ? 1 : m1 ? 2 : 4;
-    const unsigned grid = blocks_for(rows, 8 * (per_warp == 4 ? 4 : per_warp == 2 ? 2 : 1));
-#define ULLIS_LN_MIX(V)                                                                                                  \
-    do {                                                                                                                 \
-        if (per_warp == 4)                                                                                               \
-            rt->chain_small(ln_mix_split_kernel<V, 4>, grid, 256, 0, x, ln.weight, ln.bias, ln_out, m0, m1, m2, hi0, lo0, \
-                                                                    hi1, lo1, hi2, lo2, s1, rows, time, pitch);                 \
-        else if (per_warp == 2)                                                                                          \
-            rt->chain_small(ln_mix_split_kernel<V, 2>, grid, 256, 0, x, ln.weight, ln.bias, ln_out, m0, m1, m2, hi0, lo0, \
-                                                                    hi1, lo1, hi2, lo2, s1, rows, time, pitch);                 \
-        else                                                                                                             \
-            rt->chain_small(ln_mix_split_kernel<V, 1>, grid, 256, 0, x, ln.weight, ln.bias, ln_out, m0, m1, m2, hi0, lo0, \
-                                                                    hi1, lo1, hi2, lo2, s1, rows, time, pitch);                 \
+    // Rows per warp: one while the rows are too few to fill the device with warps that take more, and no more than help:
+    // us at 512 channels with 1 / 4 / 8, one operand: 4096 rows 9 / 8 / 10, 8192 12.8 / 10.2 / 11.7, 16 384 18 / 14 / 13,
+    // 131 072 128 / 88 / 82 (floor 61); Q/K/V: 4096 rows 16 / 18 / 25, 8192 25 / 23 / 26, 131 072 293 / 266 / 274 (floor
+    // 205).  Without the loads ahead of the row before, every row's weights in front of its sums and single conversions,
+    // 131 072 rows took 131 and 281.
+    const uint32_t per_warp = rt->tc_ln_rows > 0 ? (uint32_t)rt->tc_ln_rows : rows < 8192 ? 1 : m1 || rows < 16384 ? 4 : 8;
+    const unsigned grid = blocks_for(rows, 8 * per_warp);
+#define ULLIS_LN_MIX_FORM(V, SEVERAL, MIXES)                                                                             \
+    rt->chain_small(ln_mix_split_kernel<V, SEVERAL, MIXES>, grid, 256, 0, x, ln.weight, ln.bias, ln_out, m0, m1, m2, hi0, \
+                    lo0, hi1, lo1, hi2, lo2, s1, (uint32_t)rows, (uint32_t)time, (uint32_t)pitch, per_warp)
+#define ULLIS_LN_MIX(V)                                                                \
+    do {                                                                               \
+        if (per_warp > 1 && m1) ULLIS_LN_MIX_FORM(V, true, 3);                         \
+        else if (per_warp > 1) ULLIS_LN_MIX_FORM(V, true, 1);                          \
+        else if (m1) ULLIS_LN_MIX_FORM(V, false, 3);                                   \
+        else ULLIS_LN_MIX_FORM(V, false, 1);                                           \
     } while (0)
     switch (d / 128) {
         case 1: ULLIS_LN_MIX(1); break;
@@ -859,6 +881,7 @@ bool launch_ln_mix_split(ullis_cuda_runtime* rt, const float* x, const LayerNorm
         default: ULLIS_LN_MIX(8); break;
     }
 #undef ULLIS_LN_MIX
+#undef ULLIS_LN_MIX_FORM
     rt->launched(what);
     return true;
 }
