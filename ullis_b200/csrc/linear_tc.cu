@@ -955,8 +955,9 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ part, float* __re
 }  // namespace
 
 bool dense_nt(ullis_cuda_runtime* rt, const uint16_t* a16, const uint16_t* b16, float* y, size_t M, size_t K,
-              size_t N) {
+              size_t N, Partials* partials) {
     if (!usable(rt) || !shape_ok(M, K, N)) return false;
+    if (partials) *partials = Partials{y, 1};
     GemmMaps maps;
     memset(&maps, 0, sizeof(maps));
     maps.a[0][0] = make_map(a16, M, K, false);
@@ -967,6 +968,10 @@ bool dense_nt(ullis_cuda_runtime* rt, const uint16_t* a16, const uint16_t* b16, 
     // it; the partials are then summed in split order.  By CTA pairs where the columns allow (512 x 2 048 of 16 384 rows:
     // 48 -> 37 us).
     const auto reduce = [&](float* part, uint32_t splits) {
+        if (partials) {
+            *partials = Partials{part, splits};
+            return;
+        }
         const size_t n = M * N;
         rt->chain(splitk_reduce_kernel, blocks_for((n + 3) / 4, 256), 256, 0, part, y, splits, n);
         rt->launched("splitk_reduce");

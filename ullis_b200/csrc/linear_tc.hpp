@@ -16,9 +16,14 @@ bool binary_linear(ullis_cuda_runtime* rt, const float* x, const uint32_t* bits,
 // y = x . W^T, W FP16 [out,in].
 bool fp16_linear(ullis_cuda_runtime* rt, const float* x, const uint16_t* w, float* y, size_t rows,
                  size_t in_features, size_t out_features);
-// y [M,N] f32 = a . b^T with both operands already FP16: a [M,K], b [N,K] (K a multiple of 64).
+// y [M,N] f32 = a . b^T with both operands already FP16: a [M,K], b [N,K] (K a multiple of 64).  With `partials` a long K
+// may be left as `count` sums [M,N] one behind the other at `sums`, to be added in that order; they stay until the next call.
+struct Partials {
+    const float* sums;
+    uint32_t count;
+};
 bool dense_nt(ullis_cuda_runtime* rt, const uint16_t* a16, const uint16_t* b16, float* y, size_t M, size_t K,
-              size_t N);
+              size_t N, Partials* partials = nullptr);
 // ln3 output -> time-shift mixes -> packed Q,K,V -> stream-major sign bits.  With `x_before_ln` the LayerNorm
 // itself is part of the call (L.ln3 over x_before_ln, folded into the operand kernel where the width allows) and
 // its output is left in `ln3_write`, which must be the buffer `ln3_out` names.

@@ -521,10 +521,11 @@ __device__ __forceinline__ void clipped_step(uint16_t& w, float& residual, float
     w = rounded;
 }
 
-// A CTA has 1024 elements, four per thread, their loads in flight together.
+// A CTA has 1024 elements, four per thread, their loads in flight together.  The gradient is the sum of `sums` arrays of n
+// elements, in their order (the shares of a split product).
 __global__ void __launch_bounds__(256)
-clipped_sgd_kernel(uint16_t* __restrict__ w, float* __restrict__ residual, const float* __restrict__ g, float gmul, float lr,
-                   size_t n) {
+clipped_sgd_kernel(uint16_t* __restrict__ w, float* __restrict__ residual, const float* __restrict__ g, uint32_t sums, float gmul,
+                   float lr, size_t n) {
     chain_entry();
     const size_t i0 = (size_t)blockIdx.x * 1024 + threadIdx.x;
     uint16_t wb[4];
@@ -534,6 +535,12 @@ clipped_sgd_kernel(uint16_t* __restrict__ w, float* __restrict__ residual, const
         const size_t i = i0 + k * 256;
         if (i < n) { wb[k] = w[i]; r[k] = residual[i]; gv[k] = g[i]; }
     }
+    for (uint32_t s = 1; s < sums; ++s) {
+        g += n;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (i0 + k * 256 < n) gv[k] += g[i0 + k * 256];
+    }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         const size_t i = i0 + k * 256;
@@ -542,6 +549,16 @@ clipped_sgd_kernel(uint16_t* __restrict__ w, float* __restrict__ residual, const
         w[i] = wb[k];
         residual[i] = r[k];
     }
+}
+
+// One latent (apply_binaryconnect_sgd, src/precision.rs:124-134); g not finite or zero: it stays.  True: something changed.
+__device__ __forceinline__ bool latent_step(uint16_t& latent, float& residual, float g, float lr) {
+    if (!(g != 0.0f && fabsf(g) <= 3.4028234e38f)) return false;
+    const float update = __fmul_rn(lr, fminf(fmaxf(g, -1.0f), 1.0f));
+    const float desired = fminf(fmaxf(__fadd_rn(__fsub_rn(h2f(latent), update), residual), -1.0f), 1.0f);
+    latent = __half_as_ushort(__float2half_rn(desired));
+    residual = __fsub_rn(desired, h2f(latent));
+    return true;
 }
 
 // Latent step of a packed matrix (apply_binaryconnect_sgd, src/precision.rs:124-134, on
@@ -577,12 +594,8 @@ latent_sgd_kernel(uint16_t* __restrict__ latent, float* __restrict__ residual, c
         const size_t i = i0 + 32 * j;
         bool plus = false;
         if (i < n) {
-            if (g[j] != 0.0f && fabsf(g[j]) <= 3.4028234e38f) {
-                const float current = h2f(lb[j]);
-                const float update = __fmul_rn(lr, fminf(fmaxf(g[j], -1.0f), 1.0f));
-                const float desired = fminf(fmaxf(__fadd_rn(__fsub_rn(current, update), carry[j]), -1.0f), 1.0f);
-                lb[j] = __half_as_ushort(__float2half_rn(desired));
-                residual[i] = __fsub_rn(desired, h2f(lb[j]));
+            if (latent_step(lb[j], carry[j], g[j], lr)) {
+                residual[i] = carry[j];
                 latent[i] = lb[j];
             }
             plus = h2f(lb[j]) >= 0.0f;
@@ -600,6 +613,77 @@ latent_sgd_kernel(uint16_t* __restrict__ latent, float* __restrict__ residual, c
     if (changed) atomicAdd(&total, changed);
     __syncthreads();
     if (threadIdx.x == 0 && total) atomicAdd(flips, (unsigned long long)total);
+}
+
+// All of a packed matrix's step after its gradient product: the sum of the product's shares (in their order), the latents
+// as latent_sgd_kernel steps them (with the scale from before its own step), the signs, the count of those that changed, the
+// gradient of the row's scale as g_scale_kernel sums it and the clipped step of that scale.  in_f is a multiple of 32.  A CTA
+// has a row, each of its warps PACKED_WORDS words of it at a time; the first warp then adds up what they left, since the sum
+// of a scale keeps its order (a lane's elements are 32 apart).  The loads of a share are in flight together.  On average
+// over a step at 16 384 rows (512 x 512, 2048 x 512 and one 8192 x 512) as four kernels, G and the signs read twice and the
+// sum of the shares written in between, 32 us, with a warp for a row 23, so 12.5.
+constexpr int PACKED_WORDS = 4, PACKED_WARPS = 4;
+__global__ void __launch_bounds__(32 * PACKED_WARPS)
+packed_step_kernel(uint16_t* __restrict__ latent, float* __restrict__ residual, const float* __restrict__ G, uint32_t sums,
+                   uint16_t* __restrict__ scale, float* __restrict__ scale_residual, uint32_t* __restrict__ bits, size_t n,
+                   uint32_t in_f, float gmul, float ste_scale, float lr, unsigned long long* flips) {
+    chain_entry();
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, o = blockIdx.x;
+    __shared__ float terms[PACKED_WARPS * PACKED_WORDS][32];
+    __shared__ uint32_t changed[PACKED_WARPS];
+    uint16_t sw = scale[o];
+    float sr = scale_residual[o], acc = 0.0f;
+    const float s = h2f(sw);
+    uint32_t flipped = 0;
+    for (uint32_t i0 = 0; i0 < in_f; i0 += 32 * PACKED_WARPS * PACKED_WORDS) {
+        const uint32_t here = min(PACKED_WARPS * PACKED_WORDS, (in_f - i0) >> 5);   // words of this round
+        const size_t at = (size_t)o * in_f + i0 + warp * (32 * PACKED_WORDS) + lane;
+        float g[PACKED_WORDS], carry[PACKED_WORDS];
+        uint16_t lb[PACKED_WORDS];
+        uint32_t old[PACKED_WORDS];
+#pragma unroll
+        for (int j = 0; j < PACKED_WORDS; ++j)
+            if (warp * PACKED_WORDS + j < here) {
+                g[j] = G[at + 32 * j];
+                lb[j] = latent[at + 32 * j];
+                carry[j] = residual[at + 32 * j];
+                old[j] = bits[(at >> 5) + j];
+            }
+#pragma unroll 8
+        for (uint32_t k = 1; k < sums; ++k) {
+#pragma unroll
+            for (int j = 0; j < PACKED_WORDS; ++j)
+                if (warp * PACKED_WORDS + j < here) g[j] += G[k * n + at + 32 * j];
+        }
+#pragma unroll
+        for (int j = 0; j < PACKED_WORDS; ++j) {
+            if (warp * PACKED_WORDS + j >= here) break;
+            terms[warp * PACKED_WORDS + j][lane] = (old[j] >> lane) & 1u ? g[j] : -g[j];
+            if (latent_step(lb[j], carry[j], __fmul_rn(__fmul_rn(__fmul_rn(s, g[j]), gmul), ste_scale), lr)) {
+                residual[at + 32 * j] = carry[j];
+                latent[at + 32 * j] = lb[j];
+            }
+            const uint32_t word = __ballot_sync(0xffffffffu, h2f(lb[j]) >= 0.0f);
+            if (lane == 0) bits[(at >> 5) + j] = word;
+            flipped += __popc(old[j] ^ word);
+        }
+        __syncthreads();
+        if (warp == 0)
+            for (uint32_t j = 0; j < here; ++j) acc += terms[j][lane];
+        __syncthreads();
+    }
+    if (lane == 0) changed[warp] = flipped;
+    __syncthreads();
+    if (warp) return;
+    for (int k = 16; k > 0; k >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, k);
+    if (lane == 0) {
+        clipped_step(sw, sr, __fmul_rn(acc, gmul), lr);
+        scale[o] = sw;
+        scale_residual[o] = sr;
+        uint32_t total = 0;
+        for (int w = 0; w < PACKED_WARPS; ++w) total += changed[w];
+        if (total) atomicAdd(flips, (unsigned long long)total);
+    }
 }
 
 // g_scale[o] = sum_i sign[o,i] * G[o,i]   (g_scale of backward_ste, src/model.rs:784-790, with the
@@ -723,8 +807,10 @@ struct Step {
     float gmul, lr, ste;
 
     // y [M,N] = a16 [M,K] . b16 [N,K]^T
-    void gemm(const uint16_t* a, const uint16_t* b, float* y, size_t M, size_t K, size_t N) {
-        if (tc::dense_nt(rt, a, b, y, M, K, N)) return;
+    // (partials: or the shares that sum to it)
+    void gemm(const uint16_t* a, const uint16_t* b, float* y, size_t M, size_t K, size_t N, tc::Partials* partials = nullptr) {
+        if (tc::dense_nt(rt, a, b, y, M, K, N, partials)) return;
+        if (partials) *partials = tc::Partials{y, 1};
         dim3 grid(blocks_for(N, 16), blocks_for(M, 16)), block(16, 16);
         gemm_nt_plain_kernel<<<grid, block, 0, rt->stream>>>(a, b, y, M, K, N);
         rt->launched("gemm_nt_plain");
@@ -751,8 +837,8 @@ struct Step {
     void col_reduce(const float* a, const void* b, float* out, size_t R, size_t C, ColMode mode, size_t time = 0) {
         col_reduce_launch(rt, a, b, out, R, C, mode, st->part, time);
     }
-    void sgd(const Fp16Param& p, const float* g, float rate) {
-        rt->chain(clipped_sgd_kernel, blocks_for(p.n, 1024), 256, 0, p.w, p.residual, g, gmul, rate, p.n);
+    void sgd(const Fp16Param& p, const float* g, float rate, uint32_t sums = 1) {
+        rt->chain(clipped_sgd_kernel, blocks_for(p.n, 1024), 256, 0, p.w, p.residual, g, sums, gmul, rate, p.n);
         rt->launched("clipped_sgd");
     }
     // gx_out (+)= LN backward of (x, gy); steps the LayerNorm's weight and bias
@@ -770,13 +856,22 @@ struct Step {
                        float bias_lr, unsigned long long* flips, float* small) {
         const size_t out_f = p.weights->out, in_f = p.weights->in;
         float* G = st->gmat.as<float>(out_f * in_f);
-        gemm(gy16t, x16t, G, out_f, rows_p, in_f);
-        rt->chain(g_scale_kernel, blocks_for(out_f, 8), 256, 0, G, p.weights->bits, small, out_f, in_f);
-        rt->launched("g_scale");
-        rt->chain(latent_sgd_kernel, blocks_for(out_f * in_f, 256 * LATENT_WORDS), 256, 0, p.latent, p.latent_residual, G, p.scale.w, const_cast<uint32_t*>(p.weights->bits), out_f, in_f, gmul, ste,
-            lr, flips);
-        rt->launched("latent_sgd");
-        sgd(p.scale, small, lr);
+        uint32_t* bits = const_cast<uint32_t*>(p.weights->bits);
+        if (in_f % 32 == 0 && out_f < ((size_t)1 << 31)) {
+            tc::Partials g{};
+            gemm(gy16t, x16t, G, out_f, rows_p, in_f, &g);
+            rt->chain(packed_step_kernel, (unsigned)out_f, 32 * PACKED_WARPS, 0, p.latent, p.latent_residual, g.sums, g.count,
+                      p.scale.w, p.scale.residual, bits, out_f * in_f, (uint32_t)in_f, gmul, ste, lr, flips);
+            rt->launched("packed_step");
+        } else {   // a word has bits of two rows
+            gemm(gy16t, x16t, G, out_f, rows_p, in_f);
+            rt->chain(g_scale_kernel, blocks_for(out_f, 8), 256, 0, G, bits, small, out_f, in_f);
+            rt->launched("g_scale");
+            rt->chain(latent_sgd_kernel, blocks_for(out_f * in_f, 256 * LATENT_WORDS), 256, 0, p.latent, p.latent_residual, G,
+                      p.scale.w, bits, out_f, in_f, gmul, ste, lr, flips);
+            rt->launched("latent_sgd");
+            sgd(p.scale, small, lr);
+        }
         if (p.bias.w && g_bias) sgd(p.bias, g_bias, bias_lr);
     }
 };
@@ -788,7 +883,7 @@ namespace ullis {
 namespace k {
 
 void clipped_sgd(ullis_cuda_runtime* rt, uint16_t* w, float* residual, const float* g, float lr, size_t n) {
-    rt->chain(clipped_sgd_kernel, blocks_for(n, 1024), 256, 0, w, residual, g, 1.0f, lr, n);
+    rt->chain(clipped_sgd_kernel, blocks_for(n, 1024), 256, 0, w, residual, g, 1u, 1.0f, lr, n);
     rt->launched("clipped_sgd");
 }
 
@@ -1051,8 +1146,9 @@ void ullis_cuda_train_state::step(const uint32_t* tokens, const uint32_t* labels
         s.operands_cmix(W2, W1, L.key.scale, A16, key_t, relu2_t, rows, f, rows_p);
         {
             float* G = gmat.as<float>(d * f);
-            s.gemm(T16, relu2_t, G, d, rows_p, f);
-            s.sgd(T.value, G, learning_rate);
+            tc::Partials g{};
+            s.gemm(T16, relu2_t, G, d, rows_p, f, &g);
+            s.sgd(T.value, g.sums, learning_rate, g.count);
         }
         // key (src/model.rs:1141-1163)
         s.unpack_transpose(L.key.bits, B16, f, d, f_p);
