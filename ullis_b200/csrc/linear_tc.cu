@@ -706,6 +706,8 @@ bool usable(ullis_cuda_runtime* rt) {
                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WS_SMEM_LIMIT));
             ULLIS_CUDA_CHECK(cudaFuncSetAttribute(gemm_ws2_kernel<EPI_RESIDUAL, false>,
                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WS_SMEM_LIMIT));
+            ULLIS_CUDA_CHECK(cudaFuncSetAttribute(gemm_ws2_kernel<EPI_CMIX_GRAD, false>,
+                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WS_SMEM_LIMIT));
             rt->tc_ws2_dense_clusters[0] = ws2_resident_clusters<EPI_STORE, false>(rt);
             rt->tc_ws2_dense_clusters[1] = ws2_resident_clusters<EPI_RESIDUAL, false>(rt);
             rt->tc_ws2_kernel = rt->tc_ws_kernel && !getenv("ULLIS_CUDA_NO_WS2");
@@ -781,8 +783,9 @@ uint32_t stages_for(const ullis_cuda_runtime* rt, const GemmParams& p, size_t ct
 template <int EPI>
 bool takes_ws2_dense(const ullis_cuda_runtime* rt, const GemmParams& p, unsigned n_prob) {
     const size_t tiles = (size_t)n_prob * ((p.M + WS2_BM - 1) / WS2_BM) * (p.N / WS2_BN);
-    return rt->tc_ws2_kernel && p.N % WS2_BN == 0 && rt->tc_ws2_dense_clusters[EPI] >= 8 &&
-           2 * tiles * std::max(p.split_k, 1u) >= (size_t)rt->tc_ws2_dense_clusters[EPI] &&
+    const int resident = rt->tc_ws2_dense_clusters[EPI == EPI_RESIDUAL];
+    return rt->tc_ws2_kernel && p.N % WS2_BN == 0 && resident >= 8 &&
+           2 * tiles * std::max(p.split_k, 1u) >= (size_t)resident &&
            ws2_shape(p.K, p.n_a, EPI, false).stages >= 2;
 }
 
@@ -1008,6 +1011,23 @@ bool dense_nt(ullis_cuda_runtime* rt, const uint16_t* a16, const uint16_t* b16, 
         }
     }
     launch<EPI_STORE, false>(rt, maps, p, 1, "gemm_dense_nt");
+    return true;
+}
+
+// Bound by the epilogue (14 bytes moved and some 30 operations per element).  16 384 rows, K = 512, N = 2048: the product and
+// operands_kernel<true> one after the other 60 + 89 us, together 112 (floor 53, 0.34 GB; without stores and key 63, without the
+// arithmetic as well 47).  With too few tiles for the pairs, or fewer rows than they take, the two kernels.
+bool cmix_grad_operands(ullis_cuda_runtime* rt, const uint16_t* gy16, const uint16_t* w16, const float* key, const uint16_t* scale,
+                        uint16_t* rows_out, uint16_t* grad_t, uint16_t* relu2_t, size_t M, size_t K, size_t N, size_t pitch) {
+    if (!usable(rt) || !shape_ok(M, K, N) || M < rt->tc_ws2_min_rows) return false;
+    GemmParams p = base_params(rt, M, N, K);
+    if (!takes_ws2_dense<EPI_CMIX_GRAD>(rt, p, 1)) return false;
+    GemmMaps maps;
+    memset(&maps, 0, sizeof(maps));
+    maps.a[0][0] = make_map(gy16, M, K, false);
+    maps.b[0] = make_map(w16, N, K, false);
+    p.prob[0] = GemmProblem{nullptr, scale, nullptr, rows_out, grad_t, key, relu2_t, (uint32_t)pitch};
+    launch_ws2<EPI_CMIX_GRAD, false>(rt, maps, p, 1, rt->tc_ws2_dense_clusters[EPI_STORE], "gemm_cmix_grad");
     return true;
 }
 

@@ -24,6 +24,11 @@ struct Partials {
 };
 bool dense_nt(ullis_cuda_runtime* rt, const uint16_t* a16, const uint16_t* b16, float* y, size_t M, size_t K,
               size_t N, Partials* partials = nullptr);
+// g = gy . w^T (gy [M,K], w [N,K] FP16, K a multiple of 64), the gradient of relu(key)^2, never leaves the chip: with
+// t = key > 0 ? 2 * key * g : 0, rows_out [M,N] = FP16(t * scale), grad_t [N,pitch] = FP16(t)^T, relu2_t [N,pitch] =
+// FP16(relu(key)^2)^T, pitch = M rounded up to a multiple of 64, the columns from M on 0.
+bool cmix_grad_operands(ullis_cuda_runtime* rt, const uint16_t* gy16, const uint16_t* w16, const float* key, const uint16_t* scale,
+                        uint16_t* rows_out, uint16_t* grad_t, uint16_t* relu2_t, size_t M, size_t K, size_t N, size_t pitch);
 // ln3 output -> time-shift mixes -> packed Q,K,V -> stream-major sign bits.  With `x_before_ln` the LayerNorm
 // itself is part of the call (L.ln3 over x_before_ln, folded into the operand kernel where the width allows) and
 // its output is left in `ln3_write`, which must be the buffer `ln3_out` names.

@@ -33,7 +33,7 @@
 namespace ullis {
 namespace tc {
 
-enum { EPI_STORE = 0, EPI_RESIDUAL = 1, EPI_RELU2 = 2, EPI_SIGNBITS = 3, EPI_CE = 4 };
+enum { EPI_STORE = 0, EPI_RESIDUAL = 1, EPI_RELU2 = 2, EPI_SIGNBITS = 3, EPI_CE = 4, EPI_CMIX_GRAD = 5 };
 
 constexpr int BM = 128, BN = 128, BK = 64, MAX_STAGES = 6;
 constexpr int TILE_BYTES = BM * BK * 2;  // 16 KiB, also the B tile (BN == BM)
@@ -41,13 +41,24 @@ constexpr int GEMM_THREADS = 192;
 constexpr int STAGE_STRIDE = 20;                         // floats per row of an epilogue warp's 32 x 16 transposition buffer
 constexpr int STAGE_BYTES = 32 * STAGE_STRIDE * 4;       // per epilogue warp
 
+// EPI_CMIX_GRAD, per epilogue warp: 32 x 32 floats, and 32 rows of two times 16 columns of 16 bits
+constexpr int GRAD_CHUNK = 32 * 32, GRAD_SECOND = 16 * 64, GRAD_STAGE_BYTES = GRAD_CHUNK * 4 + 2 * GRAD_SECOND;
+// where their pieces lie so that neither side meets a bank conflict: 16 bytes (four columns) of a row, in floats; 8 bytes (four
+// rows) of a column, in bytes
+__device__ __forceinline__ uint32_t grad_chunk_at(uint32_t row, uint32_t piece) { return row * 32 + ((piece ^ (row & 7)) << 2); }
+__device__ __forceinline__ uint32_t grad_turned_at(uint32_t column, uint32_t piece) {
+    return (column >> 1) * 128 + ((((column & 1) << 3 | piece) ^ (column >> 2 << 2)) << 3);
+}
+
 struct GemmProblem {
     const uint32_t* bits;   // packed weights (PACKED kernels)
     const uint16_t* scale;  // FP16 [N] or null (= 1)
     const uint16_t* bias;   // FP16 [N] or null (= 0)
     void* out;
     void* out2;
-    const float* aux;       // EPI_SIGNBITS: per-row sum |a| ; EPI_CE: unused
+    const float* aux;       // EPI_SIGNBITS: per-row sum |a| ; EPI_CMIX_GRAD: key [M,N]
+    void* out3;             // EPI_CMIX_GRAD
+    uint32_t pitch;         // EPI_CMIX_GRAD: of the transposed outputs, M rounded up to a multiple of 64
 };
 
 struct GemmMaps {
@@ -157,6 +168,117 @@ __device__ __forceinline__ void epilogue(const GemmParams& p, const GemmProblem&
                             v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
                         }
                         *dst = v;
+                    }
+                }
+                __syncwarp();
+            }
+        } else if (EPI == EPI_CMIX_GRAD) {
+            // acc is the gradient of relu(key)^2.  t = key > 0 ? 2 * key * acc : 0 leaves as FP16(t * scale) by rows and
+            // FP16(t) by columns, FP16(relu(key)^2) by columns (N is a multiple of the tile's columns).  Through the buffer
+            // into four rows x four columns per lane, which is also how the key is read and the rows leave, 16 columns at a
+            // time, and through the buffer again, now 16 bits, into 64 bytes of a column per four lanes.  The whole chunk
+            // goes to the buffer first: with half of it in registers the kernel spilled, and beside 227 KB of shared memory
+            // a spilled register is read back from L2.
+            uint16_t* rows_out = static_cast<uint16_t*>(pr.out);
+            uint8_t* const turned = reinterpret_cast<uint8_t*>(stage + GRAD_CHUNK);
+            const uint32_t r4 = (lane >> 2) * 4, c4 = (lane & 3) * 4;
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+                *reinterpret_cast<uint4*>(stage + grad_chunk_at(lane, q)) = make_uint4(r[q * 4], r[q * 4 + 1], r[q * 4 + 2], r[q * 4 + 3]);
+            float4 key[4];
+            const auto load_key = [&](int h) {   // rows past M read 0, which becomes the padding of the transposes
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const uint32_t gm = m_warp + r4 + i;
+                    key[i] = gm < p.M ? *reinterpret_cast<const float4*>(pr.aux + (size_t)gm * p.N + nc + h * 16 + c4)
+                                      : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+            };
+            load_key(0);
+            __syncwarp();
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h) {
+                float4 g[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) g[i] = *reinterpret_cast<const float4*>(stage + grad_chunk_at(r4 + i, h * 4 + (lane & 3)));
+                float sc[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) sc[e] = sb_load(s_scale, c * 32 + h * 16 + c4 + e);
+                uint32_t by_row[4][2], grad[4][2], relu2[4][2];   // pairs: of a row's columns; of a column's rows
+                __half2 top = __float2half2_rn(0.0f);
+                const auto pair = [&](float a, float b) {
+                    const __half2 x = __floats2half2_rn(a, b);
+                    top = __hmax2(top, __habs2(x));
+                    return *reinterpret_cast<const uint32_t*>(&x);
+                };
+#pragma unroll
+                for (int i = 0; i < 4; i += 2) {
+                    const float gv[2][4] = {{g[i].x, g[i].y, g[i].z, g[i].w}, {g[i + 1].x, g[i + 1].y, g[i + 1].z, g[i + 1].w}};
+                    const float kv[2][4] = {{key[i].x, key[i].y, key[i].z, key[i].w},
+                                            {key[i + 1].x, key[i + 1].y, key[i + 1].z, key[i + 1].w}};
+                    float t[2][4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        float sq[2];
+#pragma unroll
+                        for (int u = 0; u < 2; ++u) {
+                            t[u][e] = kv[u][e] > 0.0f ? 2.0f * kv[u][e] * gv[u][e] : 0.0f;
+                            const float relu = fmaxf(kv[u][e], 0.0f);
+                            sq[u] = relu * relu;
+                        }
+                        grad[e][i / 2] = pair(t[0][e], t[1][e]);
+                        relu2[e][i / 2] = pair(sq[0], sq[1]);
+                    }
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        by_row[i + u][0] = pair(__fmul_rn(t[u][0], sc[0]), __fmul_rn(t[u][1], sc[1]));
+                        by_row[i + u][1] = pair(__fmul_rn(t[u][2], sc[2]), __fmul_rn(t[u][3], sc[3]));
+                    }
+                }
+                if (h == 0) load_key(1);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (m_warp + r4 + i < p.M)
+                        *reinterpret_cast<uint2*>(rows_out + (size_t)(m_warp + r4 + i) * p.N + nc + h * 16 + c4) =
+                            make_uint2(by_row[i][0], by_row[i][1]);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    uint8_t* at = turned + grad_turned_at(c4 + e, lane >> 2);
+                    *reinterpret_cast<uint2*>(at) = make_uint2(grad[e][0], grad[e][1]);
+                    *reinterpret_cast<uint2*>(at + GRAD_SECOND) = make_uint2(relu2[e][0], relu2[e][1]);
+                }
+                if (fmaxf(__low2float(top), __high2float(top)) >= 65504.0f) {
+                    // At the end of FP16's range or past it (hardly ever): this lane's values once more, one by one and from
+                    // memory, a finite one kept in range and reported.
+                    const auto in_range = [&](float v, uint32_t row) {
+                        if (fabsf(v) > 65504.0f && fabsf(v) <= 3.4028234e38f) {
+                            if (atomicCAS(p.status, ULLIS_DEV_OK, ULLIS_DEV_FP16_RANGE) == ULLIS_DEV_OK) p.status[1] = row;
+                            v = copysignf(65504.0f, v);
+                        }
+                        return __half_as_ushort(__float2half_rn(v));
+                    };
+#pragma unroll 1
+                    for (uint32_t k = 0; k < 16; ++k) {
+                        const uint32_t i = k >> 2, e = k & 3, row = m_warp + r4 + i, col = h * 16 + c4 + e;
+                        if (row >= p.M) break;
+                        const float kv = pr.aux[(size_t)row * p.N + nc + col], relu = fmaxf(kv, 0.0f);
+                        const float t = kv > 0.0f ? 2.0f * kv * stage[grad_chunk_at(r4 + i, col >> 2) + e] : 0.0f;
+                        uint16_t* at = reinterpret_cast<uint16_t*>(turned + grad_turned_at(c4 + e, lane >> 2)) + i;
+                        rows_out[(size_t)row * p.N + nc + col] = in_range(__fmul_rn(t, sb_load(s_scale, c * 32 + col)), row);
+                        at[0] = in_range(t, row);
+                        at[GRAD_SECOND / 2] = in_range(relu * relu, row);
+                    }
+                }
+                __syncwarp();
+                const uint32_t row = m_warp + (lane & 3) * 8;   // two pieces of four rows lie side by side
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    const uint32_t column = k * 8 + (lane >> 2);
+                    const uint8_t* at = turned + grad_turned_at(column, (lane & 3) * 2);
+                    const size_t to = (size_t)(nc + h * 16 + column) * pr.pitch + row;
+                    if (row < pr.pitch) {
+                        *reinterpret_cast<uint4*>(static_cast<uint16_t*>(pr.out2) + to) = *reinterpret_cast<const uint4*>(at);
+                        *reinterpret_cast<uint4*>(static_cast<uint16_t*>(pr.out3) + to) = *reinterpret_cast<const uint4*>(at + GRAD_SECOND);
                     }
                 }
                 __syncwarp();

@@ -28,7 +28,7 @@ constexpr uint32_t WS2_STAGE16_BYTES = 32 * 64;   // per epilogue warp: 32 rows 
 
 // bytes of store-staging buffer per epilogue warp
 inline uint32_t ws2_staging(int epi) {
-    return (epi == EPI_STORE || epi == EPI_RESIDUAL) ? (uint32_t)STAGE_BYTES : epi == EPI_RELU2 ? WS2_STAGE16_BYTES : 0u;
+    return epi == EPI_CMIX_GRAD ? (uint32_t)GRAD_STAGE_BYTES : (epi == EPI_STORE || epi == EPI_RESIDUAL) ? (uint32_t)STAGE_BYTES : epi == EPI_RELU2 ? WS2_STAGE16_BYTES : 0u;
 }
 
 inline WsShape ws2_shape(uint32_t K, uint32_t n_a, int epi, bool resident_w = true) {
@@ -259,7 +259,8 @@ gemm_ws2_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p, const
             const uint32_t taddr = tmem_base + buf * WS2_BN + group * 64 + ((quarter * 32) << 16);
             epilogue<EPI, __half, EPI == EPI_RELU2>(
                 p, pr, taddr, m, n0 + group * 64, s_scale + group * 64, s_bias + group * 64, lane, n_tile * 4 + group, 0, 2,
-                stage_base + (warp - 2) * ((EPI == EPI_RELU2 ? WS2_STAGE16_BYTES : (uint32_t)STAGE_BYTES) / 4));
+                stage_base + (warp - 2) * ((EPI == EPI_RELU2 ? WS2_STAGE16_BYTES : EPI == EPI_CMIX_GRAD ? (uint32_t)GRAD_STAGE_BYTES
+                                                                                                    : (uint32_t)STAGE_BYTES) / 4));
             ptx::tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive_cluster(drained_even + 8 * buf);

@@ -1142,8 +1142,13 @@ void ullis_cuda_train_state::step(const uint32_t* tokens, const uint32_t* labels
         s.operands(GX, nullptr, A16, T16, rows, d, rows_p);                                           // gy, gy^T
         rt->chain(transpose16_kernel, dim3(blocks_for(d_p, 64), blocks_for(f, 64)), 256, 0, L.value, B16, d, f, d_p);
         rt->launched("transpose16");
-        s.gemm(A16, B16, W2, rows, d_p, f);                                                           // g_relu2
-        s.operands_cmix(W2, W1, L.key.scale, A16, key_t, relu2_t, rows, f, rows_p);
+        // g_relu2 and what the products of the key take of it: in one kernel where that goes, which reads A16 while it writes
+        uint16_t* KEY16 = reinterpret_cast<uint16_t*>(W2);
+        if (!tc::cmix_grad_operands(rt, A16, B16, W1, L.key.scale, KEY16, key_t, relu2_t, rows, d_p, f, rows_p)) {
+            KEY16 = A16;
+            s.gemm(A16, B16, W2, rows, d_p, f);
+            s.operands_cmix(W2, W1, L.key.scale, KEY16, key_t, relu2_t, rows, f, rows_p);
+        }
         {
             float* G = gmat.as<float>(d * f);
             tc::Partials g{};
@@ -1152,7 +1157,7 @@ void ullis_cuda_train_state::step(const uint32_t* tokens, const uint32_t* labels
         }
         // key (src/model.rs:1141-1163)
         s.unpack_transpose(L.key.bits, B16, f, d, f_p);
-        s.gemm(A16, B16, T3, rows, f_p, d);                                                           // g_shifted
+        s.gemm(KEY16, B16, T3, rows, f_p, d);                                                         // g_shifted
         s.operands(T2, nullptr, nullptr, B16, rows, d, rows_p);
         s.packed_update(T.key, key_t, B16, rows_p, nullptr, 0.0f, CNT + 1, SM);
         // time-shift mix (src/model.rs:1164-1176)
