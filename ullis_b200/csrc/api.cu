@@ -210,7 +210,7 @@ ullis_cuda_runtime* ullis_cuda_runtime::child(size_t i) {
     c->tc_ln_rows = tc_ln_rows;
     c->sam_walk_chunked = sam_walk_chunked;
     c->sam_budget_bytes = sam_budget_bytes / (children.size() + 1);
-    c->tc_fix_list = tc_fix_list;
+    c->tc_fix_blocks = tc_fix_blocks;
     c->tc_fuse_ln = tc_fuse_ln;
     c->tc_stages = tc_stages;
     c->tc_stages2 = tc_stages2;
@@ -403,7 +403,7 @@ int32_t ullis_cuda_runtime_create(int32_t device, ullis_cuda_runtime** out) {
         if (const char* env = getenv("ULLIS_CUDA_SAM_SPARSE")) rt->sam_sparse_per_sm = (uint32_t)std::max(0, atoi(env));
         if (const char* env = getenv("ULLIS_CUDA_SAM_WORDS")) rt->sam_words = atoi(env) != 0;
         if (const char* env = getenv("ULLIS_CUDA_FUSE_LN")) rt->tc_fuse_ln = atoi(env) != 0;
-        if (const char* env = getenv("ULLIS_CUDA_FIX_LIST")) rt->tc_fix_list = atoi(env) != 0;
+        if (const char* env = getenv("ULLIS_CUDA_FIX_LIST")) rt->tc_fix_blocks = atoi(env) != 0;
         if (const char* env = getenv("ULLIS_CUDA_SAM_WALK_CHUNKED")) rt->sam_walk_chunked = atoi(env) != 0;
         if (const char* env = getenv("ULLIS_CUDA_LN_ROWS")) rt->tc_ln_rows = atoi(env);
         if (const char* env = getenv("ULLIS_CUDA_SAM_SMEM_WAVES")) rt->sam_smem_waves = std::max(0, atoi(env));

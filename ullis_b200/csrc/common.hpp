@@ -165,7 +165,7 @@ struct ullis_cuda_runtime {
     int tc_ws2_dense_clusters[2] = {0, 0};      // the same for dense weights (store, residual)
     int tc_ws2_clusters[5] = {0, 0, 0, 0, 0};   // CTA pairs of that kernel the device holds at once, per epilogue
     bool tc_fuse_ln = true;             // LayerNorm folded into the kernel that writes the 16-bit operands of the next GEMM
-    bool tc_fix_list = true;            // exact sign recomputation from a compact list of the flagged outputs (one thread each)
+    bool tc_fix_blocks = true;          // exact sign recomputation by blocks of 32 steps with their rows in shared memory; false: the window form
     int tc_ready = 0;                   // 0 = not probed, 1 = usable, -1 = unusable on this device
     ullis::NcclState* nccl = nullptr;
 
@@ -250,7 +250,7 @@ struct ullis_cuda_runtime {
         uint32_t turn = 0;
         bool clean = false;   // the set of the next call is zero
     };
-    Counters fix_counters, match_counters;
+    Counters match_counters;
     // The two sets of `n` counters: this call's, and the next one's, which the call has to clear (counters_cleared()).
     void counters(Counters& c, size_t n_, uint32_t** mine, uint32_t** next) {
         if (!c.clean || c.n != n_) {

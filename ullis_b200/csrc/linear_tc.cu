@@ -335,158 +335,157 @@ __device__ __forceinline__ bool exact_mixed_sign(const float* __restrict__ xr, b
     return __fadd_rn(bias, __fmul_rn(scale, sum)) > 0.0f;
 }
 
-// The flagged outputs of one Q/K/V launch as a compact list, so that the exact recomputation runs over the whole
-// device instead of a few busy threads per window.  An entry names the sign bit to redo: (index of its word among
-// the 3 * sw stream-major bit words of the launch) * 32 + bit.  A warp takes one (sequence, block of 32 steps, matrix) at
-// a time, reads that block's flag word of every channel and appends all the bits it found with ONE addition to the
-// list's counter (an addition per word would queue a hundred thousand of them on one address).  Entries of a
-// block lie together in the list and read the same 33 rows of x.  More flags than the list holds (never on
-// realistic inputs: the list takes one output in 64) raise `ctrl[1]`, and the window kernel below then redoes the
-// whole launch.  C <= 32 * FIXQ_MAX_WORDS channels.
-constexpr int FIXQ_MAX_WORDS = 32;
-__global__ void __launch_bounds__(256)
-fix_collect_kernel(const uint32_t* __restrict__ flags, size_t sw, size_t batch, size_t C, size_t wps,
-                   uint32_t* __restrict__ list, uint32_t cap, uint32_t* __restrict__ ctrl) {
-    chain_entry();
-    const int lane = threadIdx.x & 31;
-    const size_t warps = ((size_t)gridDim.x * blockDim.x) >> 5;
-    const size_t buckets = batch * wps * 3;
-    const int rounds = (int)((C + 31) / 32);
-    for (size_t bk = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; bk < buckets; bk += warps) {
-        const size_t m = bk % 3, word = (bk / 3) % wps, b = bk / (3 * wps);
-        const size_t base = m * sw + b * C * wps + word;     // bit word of channel ch: base + ch * wps (stream-major)
-        const uint32_t* fl = flags + m * sw + (b * wps + word) * C;   // its flag word: fl[ch] (channels side by side)
-        uint32_t f[FIXQ_MAX_WORDS];
-        uint32_t mine = 0;
-#pragma unroll
-        for (int r = 0; r < FIXQ_MAX_WORDS; ++r) {
-            const size_t ch = (size_t)r * 32 + lane;
-            f[r] = (r < rounds && ch < C) ? fl[ch] : 0u;
-            mine += __popc(f[r]);
-        }
-        uint32_t incl = mine;                                  // inclusive prefix sum over the lanes
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t up = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += up;
-        }
-        const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-        if (total == 0) continue;
-        uint32_t at = 0;
-        if (lane == 31) at = atomicAdd(&ctrl[0], total);
-        at = __shfl_sync(0xffffffffu, at, 31);
-        if (at + total > cap) {
-            if (lane == 0) ctrl[1] = 1u;
-            continue;
-        }
-        at += incl - mine;
-#pragma unroll
-        for (int r = 0; r < FIXQ_MAX_WORDS; ++r) {
-            uint32_t g = f[r];
-            while (g) {
-                const uint32_t tt = __ffs(g) - 1;
-                g &= g - 1;
-                list[at++] = (uint32_t)(base + ((size_t)r * 32 + lane) * wps) * 32u + tt;
-            }
-        }
-    }
-}
+// The exact recomputation of the flagged outputs of a Q/K/V launch, a CTA per (sequence, block of 32 steps) or per `steps` of
+// one (4, 8, 16): the sequential f32 sum of the reference (src/model.rs:724-742) is a chain that only one thread can run, and all
+// entries of a block (about 50 with 512 channels) read the same 33 rows of x.  So the rows come to shared memory once, 64 columns
+// at a time with the next 64 on their way, and a thread has an entry.  Entries are sorted by step, so that eight lanes side by side
+// read few rows that follow on each other, and 16 bytes of each meet no bank conflict.  Where a sequence begins the row before is
+// 0, since 0 - x is -x up to the sign of a zero, which the sum with x does away with.
+// Bound by issue slots, about seven instructions per term (unsorted, with 4-byte copies and reads, 17 000 per warp and 56 us for
+// the blocks of one sequence); with few blocks by the chain.  64 sequences of the default model, us per layer: a kernel that
+// listed the entries, one that read both rows of each anew for its warp, 4 KB per entry through L2, and one that left at once 179,
+// so 110.  The whole call: 64 sequences 26 860 -> 26 080, 16 in training 11 540 -> 11 370, 5 x 1531 3 697 -> 3 607, one
+// 2 215 -> 2 183.
+// Any number of flags: what the queue does not hold waits in its finder's registers.
+constexpr uint32_t FIXB_COLS = 64, FIXB_PITCH = FIXB_COLS + 4, FIXB_ROWS = 33, FIXB_QUEUE = 512, FIXB_WORDS = 8, FIXB_MAX_THREADS = 160;
+// Threads per CTA: a third more than there are entries on average, so that hardly a block needs a second round; at most
+// FIXB_WORDS flag words of a matrix for each.
+inline unsigned fix_block_threads(size_t C) { return 32u * (unsigned)((C + 32 * FIXB_WORDS - 1) / (32 * FIXB_WORDS) + 1); }
+inline size_t fix_block_smem(size_t C) { return 4 * (3 * (C + 4) + 2 * FIXB_ROWS * FIXB_PITCH + FIXB_QUEUE); }
 
-// The exact recomputation of the listed outputs, a warp for up to 32 entries at a time.  The terms +/- in_i of an
-// output have to be added one after the other in f32 (that order is what makes the sign exact), which only a
-// single thread can do; everything before it is shared: for 128 input columns at a time the whole warp loads the
-// rows of one entry after the other side by side (512 bytes per request instead of 32 requests into 32 rows),
-// forms the signed terms and leaves them in shared memory, and then lane e adds up the 128 terms of entry e.
-constexpr int FIXQ_WARPS = 2, FIXQ_COLS = 128, FIXQ_PITCH = FIXQ_COLS + 1, FIXQ_BATCH = 8;
-
-__global__ void __launch_bounds__(FIXQ_WARPS * 32)
-fix_apply_kernel(const float* __restrict__ x, const uint16_t* __restrict__ mq, const uint16_t* __restrict__ mk,
+__global__ void __launch_bounds__(FIXB_MAX_THREADS)
+fix_block_kernel(const float* __restrict__ x, const uint16_t* __restrict__ mq, const uint16_t* __restrict__ mk,
                  const uint16_t* __restrict__ mv, PackedWeights wq, PackedWeights wk, PackedWeights wv,
                  uint32_t* __restrict__ bq, uint32_t* __restrict__ bk, uint32_t* __restrict__ bv,
-                 const uint32_t* __restrict__ list, uint32_t cap, const uint32_t* __restrict__ ctrl, size_t sw, size_t T,
-                 size_t C, size_t wps) {
-    chain_entry();
-    __shared__ float terms[FIXQ_WARPS][32 * FIXQ_PITCH];
-    // what the whole warp needs to know about entry e, written by lane e once per task
-    __shared__ const float* e_row[FIXQ_WARPS][32];
-    __shared__ const uint32_t* e_w[FIXQ_WARPS][32];
-    __shared__ const uint16_t* e_mix[FIXQ_WARPS][32];
-    __shared__ uint32_t e_flags[FIXQ_WARPS][32];   // 1: first step of its sequence (no row before it)
-    if (ctrl[1]) return;   // the list overflowed: the window kernel redoes everything
-    const uint32_t count = min(ctrl[0], cap);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float* mine = terms[warp];
-    // A task is the loads of `per` entries, eight at a time, for every 128 columns and then their sums: where the entries do
-    // not go round, fewer of them each (one sequence of the default model, 3 100 entries: 22 -> 14 us).
-    const uint32_t at_once = gridDim.x * FIXQ_WARPS / 2u;   // about the warps that the device holds
-    const uint32_t per = count <= 8u * at_once ? 8u : count <= 16u * at_once ? 16u : 32u;
-    const uint32_t tasks = (count + per - 1u) / per;
-    for (uint32_t task = blockIdx.x * FIXQ_WARPS + warp; task < tasks; task += gridDim.x * FIXQ_WARPS) {
-        const uint32_t i = task * per + lane;
-        const bool live = lane < (int)per && i < count;
-        const uint32_t entry = live ? list[i] : 0u, tt = entry & 31u;
-        const size_t wi = entry >> 5, m = wi / sw, rem = wi % sw;
-        const size_t s = rem / wps, word = rem % wps, b = s / C, ch = s % C, t = word * 32 + tt;
-        const PackedWeights& W = m == 0 ? wq : m == 1 ? wk : wv;
-        // a lane without an entry (the tail of the list) stands in with row 0 of x: every load below is then
-        // unconditional, and only the final write looks at `live`
-        e_row[warp][lane] = live ? x + (b * T + t) * C : x;
-        e_w[warp][lane] = W.bits + (ch * C >> 5);               // C % 32 == 0 on this path
-        e_mix[warp][lane] = m == 0 ? mq : m == 1 ? mk : mv;
-        e_flags[warp][lane] = (t == 0 || !live) ? 1u : 0u;     // 1: no row before it
-        __syncwarp();
-        float sum = 0.0f;
-        for (size_t i0 = 0; i0 < C; i0 += FIXQ_COLS) {
-            const size_t c = i0 + 4 * lane;
-            // FIXQ_BATCH entries at a time: first every load of the batch (they do not depend on each other, and the
-            // compiler will not move a load above a store to shared memory by itself), then the arithmetic
-            for (int e0 = 0; e0 < (int)per; e0 += FIXQ_BATCH) {
-                float4 cur[FIXQ_BATCH], prev[FIXQ_BATCH];
-                uint2 mw[FIXQ_BATCH];
-                uint32_t ww[FIXQ_BATCH], fl[FIXQ_BATCH];
+                 const uint32_t* __restrict__ flags, size_t sw, uint32_t T, uint32_t C, uint32_t wps, uint32_t steps) {
+    extern __shared__ __align__(16) float fix_mem[];
+    float* mixes = fix_mem;                                     // [3][C + 4]
+    float* rows = mixes + 3 * (C + 4);                          // [2][FIXB_ROWS][FIXB_PITCH]
+    uint32_t* queue = reinterpret_cast<uint32_t*>(rows + 2 * FIXB_ROWS * FIXB_PITCH);
+    __shared__ uint32_t places[32], found;   // per step: entries, then where the next one goes
+    const uint32_t tid = threadIdx.x, nt = blockDim.x;
+    for (uint32_t c = tid; c < C; c += nt) {
+        mixes[c] = h2f(mq[c]);
+        mixes[C + 4 + c] = h2f(mk[c]);
+        mixes[2 * (C + 4) + c] = h2f(mv[c]);
+    }
+    if (tid < 32) places[tid] = 0;
+    chain_entry();   // the mixes are weights, which the kernel directly before never writes
+    const uint32_t of = blockIdx.x * steps / 32u, b = of / wps, word = of - b * wps, s0 = blockIdx.x * steps % 32u, t0 = word * 32u + s0;
+    const uint32_t have = t0 < T ? min(steps, T - t0) : 0u, mask = (~0u >> (32u - steps)) << s0;   // no flags past T
+    const float* block = x + ((size_t)b * T + t0) * C;
+    const uint32_t* of_block = flags + (size_t)of * C;   // channels side by side, a matrix every sw words
+    uint32_t f[3][FIXB_WORDS];
 #pragma unroll
-                for (int u = 0; u < FIXQ_BATCH; ++u) {
-                    const int e = e0 + u;
-                    fl[u] = e_flags[warp][e];
-                    const float* row = e_row[warp][e];
-                    cur[u] = *reinterpret_cast<const float4*>(row + c);
-                    // the row before it, or (first step of a sequence) the row itself: its value is not used then
-                    prev[u] = *reinterpret_cast<const float4*>((fl[u] & 1u) ? row + c : row - C + c);
-                    mw[u] = *reinterpret_cast<const uint2*>(e_mix[warp][e] + c);
-                    ww[u] = e_w[warp][e][c >> 5] >> (c & 31);
+    for (int m = 0; m < 3; ++m)
+#pragma unroll
+        for (uint32_t u = 0; u < FIXB_WORDS; ++u) f[m][u] = u * nt + tid < C ? of_block[m * sw + u * nt + tid] & mask : 0u;
+    const auto fetch = [&](uint32_t chunk) {
+        float* to = rows + (chunk & 1u) * (FIXB_ROWS * FIXB_PITCH);
+        const float* from = block + chunk * FIXB_COLS;
+        for (uint32_t i = tid; i < (steps + 1u) * (FIXB_COLS / 4); i += nt) {
+            const uint32_t r = i / (FIXB_COLS / 4), c = i % (FIXB_COLS / 4) * 4;   // row r is step t0 + r - 1
+            float* slot = to + r * FIXB_PITCH + c;
+            if (r ? r <= have : t0 != 0u)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(slot)),
+                             "l"(from + (ptrdiff_t)r * C - C + c) : "memory");
+            else
+                *reinterpret_cast<float4*>(slot) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const uint32_t chunks = C / FIXB_COLS;
+    const auto drain = [&](uint32_t count) {
+        for (uint32_t e0 = 0; e0 < count; e0 += nt) {
+            const bool live = e0 + tid < count;
+            const uint32_t entry = live ? queue[e0 + tid] : s0, tt = entry & 31u, ch = (entry >> 5) & 0x7FFFFFu, m = entry >> 28;
+            const uint32_t* w = (m == 0u ? wq.bits : m == 1u ? wk.bits : wv.bits) + ((size_t)ch * C >> 5);   // C % 64 == 0
+            uint32_t signs[2] = {w[0], w[1]};
+            const float* mix = mixes + m * (C + 4);
+            float sum = 0.0f;
+            fetch(0);
+#pragma unroll 1
+            for (uint32_t k = 0; k < chunks; ++k) {
+                uint32_t ahead[2] = {0u, 0u};
+                if (k + 1 < chunks) {
+                    fetch(k + 1);
+                    ahead[0] = w[2 * k + 2];
+                    ahead[1] = w[2 * k + 3];
+                    asm volatile("cp.async.wait_group 1;" ::: "memory");
+                } else {
+                    asm volatile("cp.async.wait_group 0;" ::: "memory");
                 }
+                __syncthreads();
+                const float* prev = rows + (k & 1u) * (FIXB_ROWS * FIXB_PITCH) + (tt - s0) * FIXB_PITCH;
+                if (live) {
 #pragma unroll
-                for (int u = 0; u < FIXQ_BATCH; ++u) {
-                    const int e = e0 + u;
-                    const bool first_step = (fl[u] & 1u) != 0;
-                    const float xs[4] = {cur[u].x, cur[u].y, cur[u].z, cur[u].w};
-                    const float ps[4] = {prev[u].x, prev[u].y, prev[u].z, prev[u].w};
-                    const uint16_t mb[4] = {(uint16_t)(mw[u].x & 0xFFFFu), (uint16_t)(mw[u].x >> 16),
-                                            (uint16_t)(mw[u].y & 0xFFFFu), (uint16_t)(mw[u].y >> 16)};
+                    for (int h = 0; h < 2; ++h) {
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const float xx = first_step ? -xs[k] : __fsub_rn(ps[k], xs[k]);
-                        const float in = __fadd_rn(xs[k], __fmul_rn(xx, h2f(mb[k])));
-                        // column 4 * lane + k of the chunk is kept at k * 32 + lane: no bank conflict here (lanes side
-                        // by side) nor in the sums below (rows 129 words apart)
-                        mine[e * FIXQ_PITCH + k * 32 + lane] = ((ww[u] >> k) & 1u) ? in : -in;
+                        for (int j = 0; j < 32; j += 4) {   // i ascending
+                            const float4 mw = *reinterpret_cast<const float4*>(mix + k * FIXB_COLS + 32 * h + j);
+                            const float4 before = *reinterpret_cast<const float4*>(prev + 32 * h + j);
+                            const float4 at = *reinterpret_cast<const float4*>(prev + FIXB_PITCH + 32 * h + j);
+                            const float mv4[4] = {mw.x, mw.y, mw.z, mw.w}, ps[4] = {before.x, before.y, before.z, before.w};
+                            const float xs[4] = {at.x, at.y, at.z, at.w};
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                const float in = __fadd_rn(xs[e], __fmul_rn(__fsub_rn(ps[e], xs[e]), mv4[e]));
+                                const uint32_t flip = (~signs[h] << (31 - j - e)) & 0x80000000u;   // bit set: +
+                                sum = __fadd_rn(sum, __uint_as_float(__float_as_uint(in) ^ flip));
+                            }
+                        }
                     }
                 }
+                signs[0] = ahead[0];
+                signs[1] = ahead[1];
+                __syncthreads();   // this half of `rows` is filled anew two chunks on
             }
-            __syncwarp();
             if (live) {
-#pragma unroll 8
-                for (int k = 0; k < FIXQ_COLS; ++k)   // i ascending
-                    sum = __fadd_rn(sum, mine[lane * FIXQ_PITCH + (k & 3) * 32 + (k >> 2)]);
+                const uint16_t* scale = m == 0u ? wq.scale : m == 1u ? wk.scale : wv.scale;
+                const uint16_t* bias = m == 0u ? wq.bias : m == 1u ? wk.bias : wv.bias;
+                const float y = __fadd_rn(bias ? h2f(bias[ch]) : 0.0f, __fmul_rn(h2f(scale[ch]), sum));
+                uint32_t* at = (m == 0u ? bq : m == 1u ? bk : bv) + ((size_t)b * C + ch) * wps + word;
+                if (y > 0.0f) atomicOr(at, 1u << tt); else atomicAnd(at, ~(1u << tt));
             }
-            __syncwarp();
         }
-        if (live) {
-            const float y = __fadd_rn(W.bias ? h2f(W.bias[ch]) : 0.0f, __fmul_rn(h2f(W.scale[ch]), sum));
-            uint32_t* bits = m == 0 ? bq : m == 1 ? bk : bv;
-            if (y > 0.0f) atomicOr(&bits[rem], 1u << tt); else atomicAnd(&bits[rem], ~(1u << tt));
+    };
+    __syncthreads();   // `places` are 0
+    for (;;) {
+#pragma unroll
+        for (int m = 0; m < 3; ++m)
+#pragma unroll
+            for (uint32_t u = 0; u < FIXB_WORDS; ++u)
+                for (uint32_t g = f[m][u]; g; g &= g - 1u) atomicAdd(&places[__ffs(g) - 1], 1u);
+        __syncthreads();
+        if (tid < 32) {
+            const uint32_t n = places[tid];
+            uint32_t up_to = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t other = __shfl_up_sync(0xFFFFFFFFu, up_to, o);
+                if (tid >= (uint32_t)o) up_to += other;
+            }
+            places[tid] = up_to - n;
+            if (tid == 31) found = up_to;
         }
-        __syncwarp();   // the entry table is rewritten by the next task
+        __syncthreads();
+#pragma unroll
+        for (int m = 0; m < 3; ++m)
+#pragma unroll
+            for (uint32_t u = 0; u < FIXB_WORDS; ++u)
+                for (uint32_t g = f[m][u]; g; g &= g - 1u) {
+                    const uint32_t step = __ffs(g) - 1, at = atomicAdd(&places[step], 1u);
+                    if (at >= FIXB_QUEUE) continue;
+                    queue[at] = (uint32_t)m << 28 | (u * nt + tid) << 5 | step;
+                    f[m][u] &= ~(1u << step);
+                }
+        const uint32_t n = found;
+        __syncthreads();
+        drain(min(n, FIXB_QUEUE));
+        if (n <= FIXB_QUEUE) return;
+        __syncthreads();
+        if (tid < 32) places[tid] = 0;
+        __syncthreads();
     }
 }
 
@@ -506,11 +505,8 @@ sign_fixup_kernel(const float* __restrict__ x, const uint16_t* __restrict__ mq, 
                   const uint16_t* __restrict__ mv, PackedWeights wq, PackedWeights wk, PackedWeights wv,
                   uint32_t* __restrict__ bq, uint32_t* __restrict__ bk, uint32_t* __restrict__ bv,
                   const uint32_t* __restrict__ fq, const uint32_t* __restrict__ fk, const uint32_t* __restrict__ fv,
-                  size_t batch, size_t T, size_t C, size_t wps, const uint32_t* __restrict__ only_if,
-                  uint32_t* __restrict__ clear) {
+                  size_t batch, size_t T, size_t C, size_t wps) {
     chain_entry();
-    if (clear && blockIdx.x == 0 && threadIdx.x < 2) clear[threadIdx.x] = 0u;   // the counters of the next call
-    if (only_if && *only_if == 0u) return;   // the compact list took every flag: nothing left for the windows
     extern __shared__ uint32_t fix_queue[];  // entries: matrix << 28 | channel << 8 | word in window << 5 | bit
     __shared__ uint32_t q_count, announced;   // entries queued; flag bits announced so far (never reset)
     const size_t windows = (wps + FIX_WIN - 1) / FIX_WIN;
@@ -1068,27 +1064,23 @@ bool rosa_qkv_bits(ullis_cuda_runtime* rt, const float* ln3_out, const LayerWeig
     for (int z = 0; z < 3; ++z)
         p.prob[z] = GemmProblem{W[z]->bits, W[z]->scale, W[z]->bias, outs[z], flags + z * sw, s1 + z * prows};
     launch<EPI_SIGNBITS, true>(rt, maps, p, 3, "gemm_qkv_signbits");
-    const unsigned grid = (unsigned)(((wps + FIX_WIN - 1) / FIX_WIN) * batch);   // rows < 2^30, so this fits
-    const uint32_t* only_if = nullptr;
-    uint32_t* clear = nullptr;
-    if (rt->tc_fix_list && 3 * sw < ((size_t)1 << 27) && d % FIXQ_COLS == 0 && d <= 32 * FIXQ_MAX_WORDS) {
-        // one thread per flagged output, from a compact list; room for one output in 64
-        const size_t cap = std::max<size_t>(65536, 3 * sw * 32 / 64);
-        uint32_t* list = rt->tc_ws[9].as<uint32_t>(cap);
-        uint32_t* ctrl = nullptr;
-        rt->counters(rt->fix_counters, 2, &ctrl, &clear);
-        rt->chain(fix_collect_kernel, 4 * (unsigned)rt->sm_count, 256, 0, flags, sw, batch, d, wps, list,
-                  (uint32_t)cap, ctrl);
-        rt->launched("fix_collect");
-        rt->chain(fix_apply_kernel, 12 * (unsigned)rt->sm_count, FIXQ_WARPS * 32, 0, ln3_out, L.x_q, L.x_k, L.x_v, L.q, L.k, L.v,
-                  q_sw, k_sw, v_sw, list, (uint32_t)cap, ctrl, sw, time, d, wps);
-        rt->launched("fix_apply");
-        only_if = ctrl + 1;
+    // rows < 2^30, so both grids fit
+    if (rt->tc_fix_blocks && fix_block_threads(d) <= FIXB_MAX_THREADS) {   // d % 64 == 0 (shape_ok)
+        // A part of a block for each CTA while that makes no more than the device holds at once: with few blocks the chain of one
+        // CTA is what lasts, with many the rows that are read twice count.  us of a whole call with 32 / 16 / 8 / 4 steps, 64 blocks:
+        // 2 359 / 2 252 / 2 198 / 2 183, 240: 3 928 / 3 672 / 3 607 / 3 703, 512: 6 581 / 6 334 / 6 424 / 6 650, 1024: 8 076 /
+        // 8 143 / 8 339 / 8 803.
+        const size_t blocks = wps * batch;
+        uint32_t steps = 4;
+        while (steps < 32 && blocks * (32 / steps) > 8 * (size_t)rt->sm_count) steps *= 2;
+        rt->chain(fix_block_kernel, (unsigned)(blocks * (32 / steps)), fix_block_threads(d), fix_block_smem(d), ln3_out, L.x_q, L.x_k,
+                  L.x_v, L.q, L.k, L.v, q_sw, k_sw, v_sw, flags, sw, (uint32_t)time, (uint32_t)d, (uint32_t)wps, steps);
+        rt->launched("fix_block");
+    } else {
+        rt->chain(sign_fixup_kernel, (unsigned)(((wps + FIX_WIN - 1) / FIX_WIN) * batch), FIX_THREADS, FIX_QUEUE * 4, ln3_out, L.x_q,
+                  L.x_k, L.x_v, L.q, L.k, L.v, q_sw, k_sw, v_sw, flags, flags + sw, flags + 2 * sw, batch, time, d, wps);
+        rt->launched("sign_fixup");
     }
-    rt->chain(sign_fixup_kernel, grid, FIX_THREADS, FIX_QUEUE * 4, ln3_out, L.x_q, L.x_k, L.x_v, L.q, L.k, L.v, q_sw, k_sw,
-              v_sw, flags, flags + sw, flags + 2 * sw, batch, time, d, wps, only_if, clear);
-    rt->launched("sign_fixup");
-    if (clear) rt->counters_cleared(rt->fix_counters);
     return true;
 }
 
