@@ -341,8 +341,9 @@ __device__ __forceinline__ bool exact_mixed_sign(const float* __restrict__ xr, b
 // at a time with the next 64 on their way, and a thread has an entry.  Entries are sorted by step, so that eight lanes side by side
 // read few rows that follow on each other, and 16 bytes of each meet no bank conflict.  Where a sequence begins the row before is
 // 0, since 0 - x is -x up to the sign of a zero, which the sum with x does away with.
-// Bound by issue slots, about seven instructions per term (unsorted, with 4-byte copies and reads, 17 000 per warp and 56 us for
-// the blocks of one sequence); with few blocks by the chain.  64 sequences of the default model, us per layer: a kernel that
+// With few blocks bound by the chain, with many by the waits for rows and at the barriers: issue slots 39 % used at 16 sequences, 30 %
+// of the warps there (a third buffer 110 -> 128 us, fewer blocks per SM; one barrier per 64 columns instead of two 110 -> 115).
+// Unsorted, with 4-byte copies and reads, a warp issued three times as much.  64 sequences of the default model, us per layer: a kernel that
 // listed the entries, one that read both rows of each anew for its warp, 4 KB per entry through L2, and one that left at once 179,
 // so 110.  The whole call: 64 sequences 26 860 -> 26 080, 16 in training 11 540 -> 11 370, 5 x 1531 3 697 -> 3 607, one
 // 2 215 -> 2 183.
