@@ -187,6 +187,7 @@ ullis_cuda_generate_state::ullis_cuda_generate_state(ullis_cuda_model* m, size_t
     ULLIS_CUDA_CHECK(cudaMallocHost(&h_logits, batch * m->vocab * 4));
     use_graph = !getenv("ULLIS_CUDA_NO_GRAPH");
     if (const char* env = getenv("ULLIS_CUDA_INJECT_GENERATE_FAILURE")) inject_failure_at = (size_t)std::max(0, atoi(env));
+    if (const char* env = getenv("ULLIS_CUDA_GEN_WAIT_POLLS")) wait_polls = (uint32_t)std::min(std::max(0, atoi(env)), 1 << 18);
     prepare_one_kernel();
     reset();
 }
@@ -294,6 +295,7 @@ void ullis_cuda_generate_state::launch_one_kernel(float* logits_to) {
     p.layers = static_cast<const gen::Layer*>(step_layers.get());
     p.values = static_cast<const CUtensorMap*>(step_values.get());
     p.staged = step_staged;
+    p.polls = wait_polls;
     p.status = rt->host_status;
     p.n_layers = (uint32_t)m->layers; p.rows = (uint32_t)batch; p.d = (uint32_t)m->d; p.ffn = (uint32_t)m->ffn;
     p.vocab = (uint32_t)m->vocab; p.time = (uint32_t)time;

@@ -34,6 +34,9 @@ struct ullis_cuda_generate_state {
     // Test hook (ULLIS_CUDA_INJECT_GENERATE_FAILURE=n when the state is created): step n fails on the host after
     // its kernels have run, the way a CUDA error reported at the synchronisation would.
     size_t inject_failure_at = 0;
+    // Polls of a wait of the one kernel before it gives up, 4 us each: about a second.  A test hook too
+    // (ULLIS_CUDA_GEN_WAIT_POLLS=n when the state is created: with 0 every step runs out of its first wait).
+    uint32_t wait_polls = 1u << 18;
 
     ullis_cuda_generate_state(ullis_cuda_model* m, size_t batch);
     ~ullis_cuda_generate_state();

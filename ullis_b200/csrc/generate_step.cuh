@@ -55,6 +55,7 @@ struct Step {   // kernel arguments
     uint32_t n_layers, rows, d, ffn, vocab, time;
     uint32_t stages;                                        // of the ring of D
     uint32_t staged;                                        // packed weights go through shared memory
+    uint32_t polls;                                         // of a wait, before it gives up
     float minus_zero;                                       // -0.0f, unknown to the compiler (value_piece)
     const uint32_t* tokens;                                 // page-locked host memory
     const uint16_t *embedding, *ln0_w, *ln0_b, *ln_out_w, *ln_out_b;
@@ -114,11 +115,43 @@ __device__ __forceinline__ void cluster_wait() {
     __syncwarp();
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// The copies of a CTA, issued by one thread, and the waits for them.  gave_up: a wait of this CTA or of another one of its cluster
+// ran out.  Nobody waits, asks for copies or sends any more then: an mbarrier whose phase is not over must not be told to expect
+// the next one.  The stages run to their end on what lies in shared memory, which decides no address and no loop, so that everybody
+// passes the same barriers; the step reports the failure.
+constexpr uint32_t BARS = 2 * MAX_STAGES + 7, MAX_BOX = 256;
+struct Copies {
+    uint64_t ring[BARS];   // mbarriers: a stage of the ring is full, is empty, one for each set of packed weights, for each exchange
+    __device__ uint64_t* empty() { return ring + MAX_STAGES; }
+    __device__ uint64_t* qkv_o() { return ring + 2 * MAX_STAGES; }
+    __device__ uint64_t* key() { return ring + 2 * MAX_STAGES + 1; }
+    __device__ uint64_t* head() { return ring + 2 * MAX_STAGES + 2; }
+    __device__ uint64_t* exchange(uint32_t stage) { return ring + 2 * MAX_STAGES + 3 + stage; }   // after A, B, C, D
+    uint32_t gave_up;
+};
+__device__ __forceinline__ bool has_given_up(const Copies& copies) { return *static_cast<const volatile uint32_t*>(&copies.gave_up) != 0u; }
+__device__ __forceinline__ void copies_wait(Copies& copies, uint64_t* bar, uint32_t phase, const Step& p, uint32_t site) {
+    uint32_t polls = 0;
+#pragma unroll 1
+    do {
+        if (polls < p.polls && ptx::mbar_try_wait(bar, phase & 1u)) return;
+        if (has_given_up(copies)) return;
+    } while (polls++ < p.polls);
+    *static_cast<volatile uint32_t*>(&copies.gave_up) = 1u;
+    *static_cast<volatile uint32_t*>(p.status) = ULLIS_DEV_WAIT_TIMEOUT;
+    *static_cast<volatile uint32_t*>(p.status + 1) = site;
+}
 // n floats (a multiple of 4) of each of `rows` rows, `pitch` apart, from this CTA's shared memory to the same place in every
 // other CTA of the cluster, a CTA per warp at a time, counted on the receiver's barrier `bar`.  One thread says what this CTA's own
-// barrier has to wait for.
-__device__ __forceinline__ void send_to_cluster(const float* from, uint32_t rows, uint32_t pitch, uint32_t n, uint64_t* bar) {
+// barrier has to wait for.  After a give-up the others are sent word of it in place of the share, and the result is false.
+__device__ __forceinline__ bool send_to_cluster(const float* from, uint32_t rows, uint32_t pitch, uint32_t n, Copies& copies, uint64_t* bar) {
     const uint32_t ctas = cluster_size(), me = cluster_rank(), lane = threadIdx.x & 31u;
+    if (has_given_up(copies)) {
+#pragma unroll 1
+        for (uint32_t cta = threadIdx.x; cta < ctas; cta += THREADS)
+            asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], %1;" ::"r"(ptx::cluster_map(&copies.gave_up, cta)), "r"(1u) : "memory");
+        return false;
+    }
     if (threadIdx.x == 0u) ptx::mbar_arrive_expect_tx(bar, (ctas - 1u) * rows * n * 4u);
 #pragma unroll 1
     for (uint32_t cta = threadIdx.x >> 5; cta < ctas; cta += WARPS) {
@@ -133,6 +166,7 @@ __device__ __forceinline__ void send_to_cluster(const float* from, uint32_t rows
                              "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(counted) : "memory");
             }
     }
+    return true;
 }
 // `bytes` (a multiple of 16, like both addresses) to shared memory by the copy engine, counted on `bar`.
 __device__ __forceinline__ void copy_bytes(void* to, const void* from, uint32_t bytes, uint64_t* bar) {
@@ -409,27 +443,6 @@ __device__ __forceinline__ void packed_outputs(const Packed& P, const uint32_t* 
     }
 }
 
-// The copies of a CTA, issued by one thread, and the waits for them.  gave_up: a wait ran out; nobody waits any more then, and
-// the step reports it.
-constexpr uint32_t BARS = 2 * MAX_STAGES + 7, MAX_BOX = 256;
-struct Copies {
-    uint64_t ring[BARS];   // mbarriers: a stage of the ring is full, is empty, one for each set of packed weights, for each exchange
-    __device__ uint64_t* empty() { return ring + MAX_STAGES; }
-    __device__ uint64_t* qkv_o() { return ring + 2 * MAX_STAGES; }
-    __device__ uint64_t* key() { return ring + 2 * MAX_STAGES + 1; }
-    __device__ uint64_t* head() { return ring + 2 * MAX_STAGES + 2; }
-    __device__ uint64_t* exchange(uint32_t stage) { return ring + 2 * MAX_STAGES + 3 + stage; }   // after A, B, C, D
-    uint32_t gave_up;
-};
-__device__ __forceinline__ void copies_wait(Copies& copies, uint64_t* bar, uint32_t phase, uint32_t* status, uint32_t site) {
-    if (*static_cast<volatile uint32_t*>(&copies.gave_up)) return;
-#pragma unroll 1
-    for (uint32_t polls = 0; polls < 1u << 22; ++polls)
-        if (ptx::mbar_try_wait(bar, phase & 1u)) return;
-    *static_cast<volatile uint32_t*>(&copies.gave_up) = 1u;
-    *static_cast<volatile uint32_t*>(status) = ULLIS_DEV_WAIT_TIMEOUT;
-    *static_cast<volatile uint32_t*>(status + 1) = site;
-}
 // `slabs` slabs (as many as the map's box has) from slab `slab` on of the weights of the value outputs [o0, o0 + own), by one thread.
 __device__ __forceinline__ void fetch_value(uint8_t* to, const CUtensorMap* map, uint32_t o0, uint32_t own, uint32_t slab, uint32_t slabs, uint64_t* bar) {
     ptx::mbar_arrive_expect_tx(bar, slabs * own * (SLAB * 2u));
@@ -472,12 +485,12 @@ __device__ __forceinline__ void value_products(const uint8_t* piece, const float
 }
 // The 32 sums of a CTA that has no more (src/model.rs:419-436): warp 0 adds, the others multiply for it into PRODUCT_SLOTS
 // slots, handed over by named barriers (1 + slot: full, 4 + slot: empty).  Returns the sum of the lane's output in warp 0.
-__device__ __forceinline__ float value_alone(const uint8_t* ring, Copies& copies, uint32_t phase, const float* act, uint32_t pieces, float* products, uint32_t* status) {
+__device__ __forceinline__ float value_alone(const uint8_t* ring, Copies& copies, uint32_t phase, const float* act, uint32_t pieces, float* products, const Step& p) {
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     constexpr uint32_t FULL = 1u, EMPTY = FULL + PRODUCT_SLOTS, SLOT = VALUE_OUT * PRODUCT_PITCH;
     float sum = 0.0f;
     uint32_t slot = 0;
-    copies_wait(copies, copies.ring, phase, status, 0x601u);
+    copies_wait(copies, copies.ring, phase, p, 0x601u);
     if (warp != 0u) {
 #pragma unroll 1
         for (uint32_t k = 0; k < pieces; ++k) {
@@ -611,6 +624,9 @@ gen_step_kernel(const Step p) {
     uint32_t layers_done = 0, heads_done = 0;     // phases of the barriers of the packed weights
     uint32_t slot = 0, lap = 0;                   // of the ring: the piece that is used next
     uint32_t fetch_slot = 0;                      // the piece that is fetched next
+    // whether a barrier was told to expect something an odd number of times: of the ring and of the packed weights (by the issuer), of
+    // the exchanges (by thread 0)
+    uint32_t ring_odd = 0, packed_odd = 0, exchange_odd = 0;
     if (issuer) {
 #pragma unroll 1
         for (uint32_t b = 0; b < BARS; ++b) ptx::mbar_init(copies.ring + b, b - MAX_STAGES < MAX_STAGES ? WARPS : 1u);
@@ -627,14 +643,16 @@ gen_step_kernel(const Step p) {
     };
     const uint32_t own_bytes = own * words * 4u;
     auto fetch_qkv_o = [&](const Layer& L) {
-        if (!issuer || !staged || copies.gave_up) return;
+        if (!issuer || !staged || has_given_up(copies)) return;
+        packed_odd ^= 1u;
         ptx::mbar_arrive_expect_tx(copies.qkv_o(), 4u * own_bytes);
         for (uint32_t z = 0; z < 3u; ++z) copy_bytes(w_wide + z * own * words, L.qkv[z].bits + (size_t)o0 * words, own_bytes, copies.qkv_o());
         copy_bytes(w_o, L.o.bits + (size_t)o0 * words, own_bytes, copies.qkv_o());
     };
     // D takes its weights `passes` times: a warp has 32 outputs of N rows per pass
     auto fetch_piece = [&](uint32_t l, uint32_t i) {
-        if (!issuer || copies.gave_up) return;
+        if (!issuer || has_given_up(copies)) return;
+        ring_odd ^= 1u << fetch_slot;
         fetch_value(ring + fetch_slot * stage_bytes, p.values + l, o0, own, i % pieces * (PIECE / SLAB), PIECE / SLAB, copies.ring + fetch_slot);
         fetch_slot = fetch_slot + 1u < stages ? fetch_slot + 1u : 0u;
     };
@@ -688,7 +706,7 @@ gen_step_kernel(const Step p) {
                 const uint32_t n_out = stage == 0u ? 3u * own : stage == 1u ? own : f_own;
                 if (stage != 1u) {
                     mixed_inputs<G>(p, L, l, stage / 2u, row, n, o0, own, x, in0, G * d);
-                    if (staged) copies_wait(copies, stage ? copies.key() : copies.qkv_o(), layers_done, p.status, 0x602u);
+                    if (staged) copies_wait(copies, stage ? copies.key() : copies.qkv_o(), layers_done, p, 0x602u);
                 }
                 __syncthreads();
                 auto emit = [&](uint32_t o, uint32_t r, float v) {
@@ -755,27 +773,30 @@ gen_step_kernel(const Step p) {
                     __syncthreads();
                 }
                 const float* shared_out = stage == 0u ? y + o0 * G : stage == 1u ? x + o0 : act + f0 * G;
-                send_to_cluster(shared_out, stage == 1u ? n : 1u, d, stage == 0u ? own * G : stage == 1u ? own : f_own * G, copies.exchange(stage));
+                const bool sent = send_to_cluster(shared_out, stage == 1u ? n : 1u, d, stage == 0u ? own * G : stage == 1u ? own : f_own * G, copies, copies.exchange(stage));
+                if (sent) exchange_odd ^= 1u << stage;
                 if (stage == 0u) {
                     // the key weights, in place of Q, K and V, and the first pieces of D
-                    if (issuer && staged && !copies.gave_up) {
+                    if (issuer && staged && !has_given_up(copies)) {
+                        packed_odd ^= 2u;
                         ptx::mbar_arrive_expect_tx(copies.key(), f_own * words * 4u);
                         copy_bytes(w_wide, L.key.bits + (size_t)f0 * words, f_own * words * 4u, copies.key());
                     }
                     if (!alone) {
 #pragma unroll 1
                         for (uint32_t i = 0; i < min(items, stages - 1u); ++i) fetch_piece(l, i);
-                    } else if (issuer && !copies.gave_up) {
+                    } else if (issuer && !has_given_up(copies)) {
+                        ring_odd ^= 1u;
                         fetch_value(ring, p.values + l, o0, own, 0u, ffn / SLAB, copies.ring);
                     }
                 } else if (stage == 2u && l + 1u < p.n_layers) {
                     load_layer(l + 1u);
                 }
-                copies_wait(copies, copies.exchange(stage), layers_done, p.status, 0x607u);
+                copies_wait(copies, copies.exchange(stage), layers_done, p, 0x607u);
             }
             // ---- D
             if (alone) {
-                const float sum = value_alone(ring, copies, lap, act, pieces, products, p.status);
+                const float sum = value_alone(ring, copies, lap, act, pieces, products, p);
                 if (warp == 0u) x[o0 + lane] = __fadd_rn(x[o0 + lane], sum);
                 ++lap;
             } else {
@@ -788,10 +809,10 @@ gen_step_kernel(const Step p) {
 #pragma unroll 1
                     for (uint32_t k = 0; k < pieces; ++k, ++i) {
                         if (copier && i + stages - 1u < items) {   // into the place of the piece before this one
-                            if (i) copies_wait(copies, copies.empty() + (slot ? slot : stages) - 1u, slot ? lap : lap - 1u, p.status, 0x606u);
+                            if (i) copies_wait(copies, copies.empty() + (slot ? slot : stages) - 1u, slot ? lap : lap - 1u, p, 0x606u);
                             fetch_piece(l, i + stages - 1u);
                         }
-                        copies_wait(copies, copies.ring + slot, lap, p.status, 0x604u);
+                        copies_wait(copies, copies.ring + slot, lap, p, 0x604u);
                         if (mine < sums) value_piece<G, N>(sum, ring + slot * stage_bytes, tiles, tile, act + k * PIECE * G + pair * N, p.minus_zero);
                         __syncwarp();
                         if (lane == 0u) ptx::mbar_arrive(copies.empty() + slot);
@@ -809,18 +830,19 @@ gen_step_kernel(const Step p) {
             }
             ++layers_done;
             __syncthreads();
-            send_to_cluster(x + o0, n, d, own, copies.exchange(3u));
+            if (send_to_cluster(x + o0, n, d, own, copies, copies.exchange(3u))) exchange_odd ^= 8u;
             if (l + 1u < p.n_layers) {
                 fetch_qkv_o(layers[(l + 1u) & 1u]);
                 ahead = push_begin(l + 1u);
             }
-            copies_wait(copies, copies.exchange(3u), layers_done - 1u, p.status, 0x608u);
+            copies_wait(copies, copies.exchange(3u), layers_done - 1u, p, 0x608u);
         }
         // The head: its weights by as many outputs at a time as the ring has room for, where they lie on 16-byte borders.
         const bool head_staged = staged && v_own * words % 4u == 0u && v_n * words % 4u == 0u;
         const uint32_t chunk = head_staged ? max(stages * stage_bytes / (words * 4u) / 4u * 4u, 4u) : max(v_n, 1u);
         auto fetch_head = [&](uint32_t from) {
-            if (!issuer || !head_staged || copies.gave_up) return;
+            if (!issuer || !head_staged || has_given_up(copies)) return;
+            packed_odd ^= 4u;
             const uint32_t bytes = min(chunk, v_n - from) * words * 4u;
             ptx::mbar_arrive_expect_tx(copies.head(), bytes);
             copy_bytes(ring, p.head.bits + (size_t)(v0 + from) * words, bytes, copies.head());
@@ -840,7 +862,7 @@ gen_step_kernel(const Step p) {
                 __syncthreads();
                 fetch_head(from);
             }
-            if (head_staged) copies_wait(copies, copies.head(), heads_done++, p.status, 0x605u);
+            if (head_staged) copies_wait(copies, copies.head(), heads_done++, p, 0x605u);
             __syncthreads();
             const uint32_t* w = head_staged ? reinterpret_cast<const uint32_t*>(ring) : p.head.bits + (size_t)v0 * words;
             const uint32_t outputs = min(chunk, v_n - from);
@@ -851,9 +873,23 @@ gen_step_kernel(const Step p) {
         cluster_arrive();
         cluster_wait();   // the rows are written anew only when nobody reads them
     }
-    // After a wait that gave up, copies may still be on their way into this CTA's shared memory.
-    if (copies.gave_up && issuer)
-        for (uint32_t b = 0; b < 2u * BARS; ++b) ptx::mbar_wait(copies.ring + b / 2u, b & 1u, 1u << 16);
+    // After a give-up, copies and shares may still be on their way into this CTA's shared memory: it waits for those that its
+    // barriers expect (a phase that is over is passed at once), and a while for shares that came without being expected.
+    if (has_given_up(copies)) {
+        constexpr uint32_t DRAIN = 1u << 12;
+        if (issuer) {
+#pragma unroll 1
+            for (uint32_t b = 0; b < stages; ++b) ptx::mbar_wait(copies.ring + b, ~(ring_odd >> b) & 1u, DRAIN);
+#pragma unroll 1
+            for (uint32_t b = 0; b < 3u; ++b) ptx::mbar_wait(copies.qkv_o() + b, ~(packed_odd >> b) & 1u, DRAIN);
+        }
+        if (threadIdx.x == 0u) {
+#pragma unroll 1
+            for (uint32_t b = 0; b < 4u; ++b) ptx::mbar_wait(copies.exchange(b), ~(exchange_odd >> b) & 1u, DRAIN);
+#pragma unroll 1
+            for (uint32_t i = 0; i < 64u; ++i) __nanosleep(1000);
+        }
+    }
     __syncthreads();
 }
 
