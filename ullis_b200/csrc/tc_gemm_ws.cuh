@@ -45,7 +45,7 @@ inline WsShape ws_shape(uint32_t K, uint32_t n_a, bool staged_stores, bool resid
 
 // bounded wait that also gives up when another role of the CTA has failed
 __device__ __forceinline__ bool ws_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* s_error) {
-    for (uint32_t spin = 0; spin < (1u << 24); ++spin) {
+    for (uint32_t spin = 0; spin < ptx::WAIT_POLLS; ++spin) {
         if (ptx::mbar_try_wait(bar, parity)) return true;
         if (spin > 64) {
             __nanosleep(spin > 4096 ? 256 : 32);

@@ -54,8 +54,11 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// Bounded wait (~ a second at worst with the default number of polls); false = gave up.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t polls = 1u << 24) {
+// Polls of a bounded wait.  One that finds nothing takes 4 us (the instruction holds the thread up by itself; 16 000 polls 65 ms),
+// so this is about 4 s: far above any wait of a kernel whose copies arrive, or that was launched while the one before it runs.
+constexpr uint32_t WAIT_POLLS = 1u << 20;
+// Bounded wait; false = gave up.
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t polls = WAIT_POLLS) {
     for (uint32_t spin = 0; spin < polls; ++spin) {
         if (mbar_try_wait(bar, parity)) return true;
         if (spin > 64) __nanosleep(spin > 4096 ? 256 : 32);
