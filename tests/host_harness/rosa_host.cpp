@@ -35,11 +35,11 @@ bool by_lags(const uint32_t* q, const uint32_t* k, const uint32_t* v, uint32_t T
     return true;
 }
 
-// One stream by contexts: by the last bits (wide: few positions before a step, as the easy streams are searched), or by
-// the lengths of the runs.
-void by_contexts(const uint32_t* q, const uint32_t* k, const uint32_t* v, uint32_t T, bool by_runs, bool wide, uint32_t* out) {
+// One stream by contexts of c bits: by the last bits (wide: few positions before a step, as the easy streams are searched),
+// or by the lengths of the runs.
+void by_contexts(const uint32_t* q, const uint32_t* k, const uint32_t* v, uint32_t T, uint32_t c, bool by_runs, bool wide, uint32_t* out) {
     using namespace context;
-    const uint32_t c = bits_for(T), C = 1u << c, words = (T + 31u) / 32u;
+    const uint32_t C = 1u << c, words = (T + 31u) / 32u;
     std::vector<uint32_t> Q(words + 1u, 0u), K(words + 1u, 0u);
     std::memcpy(Q.data() + 1, q, words * 4u);
     std::memcpy(K.data() + 1, k, words * 4u);
@@ -106,14 +106,14 @@ void by_contexts(const uint32_t* q, const uint32_t* k, const uint32_t* v, uint32
 
 }  // namespace
 
-// way: 0 = contexts by the last bits, 1 = the same with every bit of a context, 2 = by the lengths of the runs, else the
-// sets of lags in pieces of `way` steps (a multiple of 32)
+// way: 0 = contexts by the last bits, 1 = the same with every bit of a context, 2 = by the lengths of the runs, 3 and 4 = as 1
+// and 2 with the bits of uneven streams, else the sets of lags in pieces of `way` steps (a multiple of 32)
 extern "C" int rosa_host_batch(uint32_t way, const uint32_t* q, const uint32_t* k, const uint32_t* v, size_t n_streams,
                                uint32_t T, uint32_t* out) {
     const size_t wps = (T + 31u) / 32u;
     for (size_t s = 0; s < n_streams; ++s) {
         const size_t at = s * wps;
-        if (way <= 2u) by_contexts(q + at, k + at, v + at, T, way == 2u, way == 0u, out + at);
+        if (way <= 4u) by_contexts(q + at, k + at, v + at, T, way > 2u ? context::bits_for_uneven(T) : context::bits_for(T), way == 2u || way == 4u, way == 0u, out + at);
         else if (!by_lags(q + at, k + at, v + at, T, way, out + at)) return 1;
     }
     return 0;

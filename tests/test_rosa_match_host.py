@@ -12,6 +12,7 @@ from conftest import ROOT, pack_streams
 from test_sam_core_host import _streams
 
 BY_BITS, BY_ALL_BITS, BY_RUNS = 0, 1, 2      # otherwise: sets of lags in pieces of so many steps
+UNEVEN_BY_BITS, UNEVEN_BY_RUNS = 3, 4        # BY_ALL_BITS and BY_RUNS with the wider buckets of uneven streams
 
 
 @pytest.fixture(scope="module")
@@ -59,7 +60,7 @@ def test_every_history_of_ten_steps_behind_a_prefix(oracle, rosa_host, tail):
     v[:] = np.random.default_rng(tail).integers(0, 2, T)
     q, k, v = (pack_streams(x) for x in (q, k, v))
     ref = oracle.rosa_qkv_streams(q, k, v, n, T)
-    for way in (BY_BITS, BY_ALL_BITS, BY_RUNS, 32, 64):
+    for way in (BY_BITS, BY_ALL_BITS, BY_RUNS, UNEVEN_BY_BITS, UNEVEN_BY_RUNS, 32, 64):
         assert np.array_equal(rosa_host(way, q, k, v, n, T), ref), way
 
 
@@ -72,7 +73,7 @@ def test_long_streams(oracle, rosa_host, kind, T, n):
     rng = np.random.default_rng([T, n])
     q, k, v = (pack_streams(np.asarray(b, np.uint8)) for b in _streams(kind, n, T, rng))
     ref = oracle.rosa_qkv_streams(q, k, v, n, T)
-    for way in (BY_BITS, BY_ALL_BITS, BY_RUNS, 32, 256, 1024, 8192):
+    for way in (BY_BITS, BY_ALL_BITS, BY_RUNS, UNEVEN_BY_BITS, UNEVEN_BY_RUNS, 32, 256, 1024, 8192):
         if way == 32 and T > 2081:
             continue
         assert np.array_equal(rosa_host(way, q, k, v, n, T), ref), (kind, way)

@@ -37,6 +37,13 @@ inline uint32_t bits_for(uint32_t T) {
     return c < 2u ? 2u : c > 12u ? 12u : c;
 }
 
+// The same for a stream whose steps find many positions in their buckets: one bit more, so that the large ones halve.  Above 4096
+// steps (6000, biased streams) the sort takes what that saves.
+#if defined(__CUDACC__)
+__host__ __device__
+#endif
+inline uint32_t bits_for_uneven(uint32_t T) { return bits_for(T) + (T <= 4096u ? 1u : 0u); }
+
 constexpr uint32_t BRUTE = 64;      // steps below this compare with every earlier position
 
 struct alignas(8) Entry {           // a position and the 32 key bits that end there

@@ -350,7 +350,7 @@ struct ContextLimits {
 constexpr uint32_t CONTEXT_LARGE = 48;   // positions before a step in its buckets from which on the whole warp looks through them
 
 struct ContextLayout {   // bytes of shared memory
-    uint32_t hist, nq, start, q, k, q_ends, k_ends, in_word, before, out, entries, steps, total;
+    uint32_t hist, nq, start, q, k, q_ends, k_ends, in_word, before, out, entries, steps, total;   // for up to c bits
     __host__ __device__ ContextLayout(uint32_t T, uint32_t c, uint32_t warps) {
         const uint32_t C = 1u << c, words = (T + 31u) / 32u + 1u;
         entries = 0;                           // Entry [T]
@@ -369,20 +369,25 @@ struct ContextLayout {   // bytes of shared memory
     }
 };
 
-// TOGETHER: large buckets by a whole warp, one step after the other.  Runs where the number of listed streams is in
-// [from, to).
+// Bits of the longest contexts of a shape.
+__host__ __device__ inline uint32_t context_bits(uint32_t T, bool together) { return together ? context::bits_for_uneven(T) : context::bits_for(T); }
+
+// TOGETHER: large buckets by a whole warp, one step after the other, and one bit more for the streams that are not easy (a stream
+// at a time: default model with gain N(0, 0.02), contexts of 64 sequences 7.49 -> 6.97 ms, of one at 1000 steps 0.65 -> 0.54; with
+// the bit for every stream of a launch even ones paid, 148 of 2048 steps 26 -> 34 us, of 4096 41 -> 55).  Runs where the
+// number of listed streams is in [from, to).
 template <int NT, bool TOGETHER>
 __global__ void __launch_bounds__(NT, NT > 512 ? 1 : NT > 256 ? 2 : 5)
 rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restrict__ k_sw, const uint32_t* __restrict__ v_sw,
                     uint32_t* __restrict__ idx_sw, const uint32_t* __restrict__ list, const uint32_t* __restrict__ count,
                     uint32_t* __restrict__ next, uint32_t* __restrict__ hard, uint32_t* __restrict__ hard_count, uint32_t T,
-                    size_t wps, uint32_t c, ContextLimits limits, uint32_t from, uint32_t to) {
+                    size_t wps, uint32_t easy_bits, ContextLimits limits, uint32_t from, uint32_t to) {
     chain_entry();
     constexpr uint32_t NW = NT / 32, BRUTE = context::BRUTE;
     extern __shared__ __align__(16) uint8_t context_mem[];
     __shared__ uint32_t sh_item, sh_sums[NW], sh_pairs[NW], sh_gone, sh_large;
-    const uint32_t C = 1u << c, pair_words = C / 2u, words = (T + 31u) / 32u;
-    const ContextLayout L(T, c, NW);
+    const uint32_t words = (T + 31u) / 32u, uneven_bits = TOGETHER ? context::bits_for_uneven(T) : easy_bits;
+    const ContextLayout L(T, uneven_bits, NW);
     uint16_t* hist = reinterpret_cast<uint16_t*>(context_mem + L.hist);
     uint32_t* hist2 = reinterpret_cast<uint32_t*>(context_mem + L.hist);   // two counts per word
     uint16_t* nq = reinterpret_cast<uint16_t*>(context_mem + L.nq);
@@ -422,6 +427,7 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
         }
         if (threadIdx.x == 0) Q[0] = K[0] = 0u;
         bool by_runs = false, taken = false, sorted = false;   // sorted: the steps bucket by bucket too
+        uint32_t c = easy_bits, C = 1u << c, pair_words = C / 2u;
         uint32_t pairs_by_bits = 0;
         auto key_of_key = [&](uint32_t r) {
             return by_runs ? context::run_key(K, k_ends, r, c) : context::window(K, r) >> (32u - c);
@@ -430,7 +436,13 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
             return by_runs ? context::run_key(Q, q_ends, t, c) : context::window(Q, t) >> (32u - c);
         };
         for (int attempt = 0;; ++attempt) {
-            for (uint32_t i = threadIdx.x; i < (NW + 1u) * pair_words; i += NT) hist2[i] = 0u;   // hist and nq
+            if (TOGETHER && attempt == 1) {
+                c = uneven_bits;
+                C = 1u << c;
+                pair_words = C / 2u;
+            }
+            for (uint32_t i = threadIdx.x; i < NW * pair_words; i += NT) hist2[i] = 0u;
+            for (uint32_t i = threadIdx.x; i < pair_words; i += NT) nq2[i] = 0u;
             __syncthreads();
             for (uint32_t row = row0; row < row1; ++row) {
                 const uint32_t r = row * 32u + lane;
@@ -793,11 +805,6 @@ struct MatchCall {   // the buffers of one call
 // The shapes of the context kernel: threads per stream, and whether a warp takes a large bucket together.
 enum ContextShape { CONTEXT_256, CONTEXT_512, CONTEXT_1024, CONTEXT_SHAPES };
 
-// Context bits of a launch.  One more for uneven streams, where shared memory has room for it: their large buckets halve (default
-// model, contexts of 64 sequences 7.44 -> 7.14 ms, of one 0.89 -> 0.85); evenly spread ones pay more for the sort than they save
-// (16 in training 6.1 -> 7.6 ms; 8192 steps, where one shape takes both, 2.47 -> 2.69).
-uint32_t context_bits(uint32_t T, bool uneven) { return context::bits_for(T) + (uneven && T <= 4096u ? 1u : 0u); }
-
 template <int NT, bool TOGETHER>
 void prepare_context(ullis_cuda_runtime* rt, uint32_t T, int shape) {
     const auto kernel = rosa_context_kernel<NT, TOGETHER>;
@@ -824,7 +831,7 @@ void launch_context(ullis_cuda_runtime* rt, const MatchCall& m, int shape, uint3
     // ever change went to the match kernel).
     const ContextLimits limits{24u, 96u, 160u, 64u, 256u};
     rt->chain(rosa_context_kernel<NT, TOGETHER>, grid, NT, rt->context_smem[shape], m.q, m.k, m.v, m.idx, m.list, m.counts,
-              m.counts + 3, m.hard, m.counts + 2, m.T, m.wps, context_bits(m.T, TOGETHER && from == 0u), limits, from, to);
+              m.counts + 3, m.hard, m.counts + 2, m.T, m.wps, context::bits_for(m.T), limits, from, to);
     rt->launched(what);
 }
 
