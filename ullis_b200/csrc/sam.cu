@@ -879,18 +879,23 @@ size_t stride_for(int algo, size_t T) {
 // kernels in us, 256 / 512 / 1024 threads, all streams listed, i.i.d. bits and bits of probabilities 0.002 to 0.99:
 //
 //     streams         96 *                512                    1024                     4096           (* T = 6000: 128)
-//     T = 300     17 / 14 / 16         17 / 21 / 38           28 / 34 / 61            70 / 102 / 219
-//                 29 / 31 / 35         32 / 42 / 62           41 / 54 / 91            93 / 149 / 300
-//     T = 2048    39 / 33 / 33         53 / 58 / 79           74 / 91 / 124          216 / 298 / 453
-//                191 / 117 / 81       356 / 176 / 175        324 / 275 / 299         754 / 825 / 1016
-//     T = 6000    92 / 69 / 63        163 / 128 / 161        235 / 214 / 258         728 / 725 / 961
-//                967 / 516 / 324     1035 / 629 / 559       1382 / 947 / 904        3316 / 2691 / 2937
-//     T = 8192   112 / 78 / 69        226 / 249 / 211        426 / 451 / 388        1440 / 1681 / 1422
-//               1544 / 725 / 460     1764 / 1115 / 863      2625 / 2021 / 1358       6785 / 6422 / 4486
+//     T = 300     15 / 13 / 14         16 / 20 / 33           27 / 33 / 53            67 / 98 / 186
+//                 26 / 29 / 29         31 / 35 / 47           38 / 49 / 74            82 / 127 / 231
+//     T = 700     18 / 16 / 16         21 / 29 / 37           33 / 47 / 62            89 / 145 / 221
+//                 61 / 39 / 33         57 / 53 / 61           88 / 86 / 106          193 / 234 / 334
+//     T = 2048    33 / 27 / 25         46 / 51 / 66           74 / 90 / 121          205 / 291 / 414
+//                158 / 119 / 76       205 / 154 / 145        268 / 225 / 225         596 / 686 / 788
+//     T = 6000    90 / 72 / 61        158 / 123 / 139        229 / 219 / 256         698 / 715 / 907
+//                586 / 512 / 293      811 / 592 / 430        895 / 766 / 643        2080 / 1972 / 1997
+//     T = 8192   109 / 80 / 68        248 / 250 / 201        414 / 453 / 363        1352 / 1649 / 1337
+//                670 / 487 / 375     1077 / 745 / 573       1147 / 1120 / 754       3067 / 3227 / 2364
 //
-// One stream in eight listed, the others constant, 512 / 1024 threads: 512 listed of 4096, T = 2048 181 / 172, 1024 of 8192
-// 283 / 304, 2048 of 16 384 462 / 546; on the layers of the default model with gain N(0, 0.02) one sequence 2.8 / 2.5 ms in
-// all, four 4.0 / 3.7, 16 9.2 / 9.7, 64 29.8 / 32.2.
+// Most streams listed: 512 threads up to 6 streams per SM (layers of the default model with gain 1 + N(0, 0.02), 2048 steps:
+// one sequence 0.89 / 0.80 ms in all layers, two 1.22 / 1.31, three 1.54 / 1.81).
+// Few listed: 1024 threads the longer the more streams there are.  One stream in eight listed, the others constant, 512 / 1024
+// threads: T = 1024, 2048 streams 47 / 49, 4096 68 / 70, 8192 100 / 121; T = 1531, 4096 112 / 109, 6144 129 / 144; T = 2048,
+// 4096 152 / 137, 6144 199 / 190, 8192 233 / 238; T = 4096, 8192 539 / 451.  Layers of the default model with gain N(0, 0.02),
+// 2048 steps: one sequence 1.20 / 0.79 ms, 4 1.41 / 1.00, 8 1.63 / 1.48, 12 1.99 / 1.96, 16 2.33 / 2.43, 64 6.94 / 8.31.
 void contexts(ullis_cuda_runtime* rt, const MatchCall& m) {
     prepare_context<256, false>(rt, m.T, CONTEXT_256);
     prepare_context<512, true>(rt, m.T, CONTEXT_512);
@@ -904,11 +909,11 @@ void contexts(ullis_cuda_runtime* rt, const MatchCall& m) {
         uneven = rest = m.streams <= (size_t)rt->context_ctas[CONTEXT_512] ? (int)CONTEXT_512 : many;
     } else if (m.streams <= sms) {
         uneven = rest = CONTEXT_1024;
-    } else if (m.T < 1024u && m.streams > 56u * sms) {   // 64 times 300 steps of the default model 5.2 ms with 256 threads alone, 5.7
+    } else if (m.T < 1024u && m.streams > 56u * sms) {   // 64 times 300 steps of the default model 4.7 ms with 256 threads alone, 5.1
         uneven = rest = many;
     } else {
-        uneven = std::max<int>(many, m.T >= 1024u && m.streams <= 14u * sms ? CONTEXT_1024 : CONTEXT_512);
-        rest = std::max<int>(many, m.streams <= 7u * sms ? CONTEXT_512 : CONTEXT_256);
+        uneven = std::max<int>(many, m.T >= 1024u && m.streams * 50u <= m.T * sms ? CONTEXT_1024 : CONTEXT_512);
+        rest = std::max<int>(many, m.streams <= 6u * sms ? CONTEXT_512 : CONTEXT_256);
     }
     const uint32_t all = ~0u, half = uneven == rest ? all : (uint32_t)(m.streams / 2) + 1u;
     auto launch = [&](int shape, uint32_t from, uint32_t to, const char* what) {
