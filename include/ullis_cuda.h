@@ -103,7 +103,8 @@ ULLIS_CUDA_API uint64_t ullis_cuda_runtime_launch_count(const ullis_cuda_runtime
  * recorded behind every launch of this runtime; `kernel_time` synchronises the
  * stream and returns the total milliseconds and the number of launches recorded
  * under `name` since timing was enabled (all kernels when `name` is NULL or
- * empty).  `kernel_names` writes the distinct names, newline-separated and
+ * empty).  While it is on, an op-level call runs in one piece, not in shares with
+ * copies beside them.  `kernel_names` writes the distinct names, newline-separated and
  * NUL-terminated, into `buf` (truncated to `len`) and the size needed into
  * `*needed`. */
 ULLIS_CUDA_API int32_t ullis_cuda_runtime_kernel_timing(ullis_cuda_runtime* rt, int32_t enabled);

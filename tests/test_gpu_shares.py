@@ -41,3 +41,19 @@ def test_rosa_in_shares(cuda_rt, B, T, C):
         assert counts["total"] == B * C and counts["automaton"] == listed
     kept, _ = cuda_rt.rosa_qkv_1bit_fwd(*planes, e, B, T, C, want_out=False)
     assert np.array_equal(kept, idx)
+
+
+def test_a_call_whose_kernels_are_timed_goes_in_one_piece(cuda_rt):
+    """The times are then those of the kernels, not of waits for a share's copies."""
+    rows, K, N = 2048, 512, 2048
+    rng = np.random.default_rng(5)
+    x = rng.standard_normal(rows * K, np.float32)
+    bits = rng.integers(0, 1 << 32, K * N // 32, dtype=np.uint32)
+    scale = synth.f16_bits(rng.uniform(0.01, 0.02, N))
+    shared = cuda_rt.binary_linear(x, bits, scale, scale, rows, K, N)
+    cuda_rt.kernel_timing(True)
+    whole = cuda_rt.binary_linear(x, bits, scale, scale, rows, K, N)
+    times = cuda_rt.kernel_times()
+    cuda_rt.kernel_timing(False)
+    assert [n for name, (_, n) in times.items() if name.startswith("gemm_")] == [1]
+    assert np.array_equal(whole, shared)

@@ -130,8 +130,10 @@ void in_shares(ullis_cuda_runtime* rt, size_t shares, bool results_locked, In co
     ULLIS_CUDA_CHECK(cudaStreamWaitEvent(rt->stream, rt->copies_done, 0));
 }
 // Shares of a call: each with results of 4 MiB at least (about 80 us on the link, where a share costs its launches) and `least` of
-// the `items` that it is cut by.
-size_t shares_for(size_t result_bytes, size_t items, size_t least) {
+// the `items` that it is cut by.  A call whose kernels are timed goes in one piece: a bracket of events around a share's kernel
+// would hold the wait for its input, and the copies beside it.
+size_t shares_for(const ullis_cuda_runtime* rt, size_t result_bytes, size_t items, size_t least) {
+    if (rt->kernel_timing) return 1;
     return std::max<size_t>(1, std::min({ullis_cuda_runtime::MAX_SHARES, result_bytes >> 22, items / std::max<size_t>(least, 1)}));
 }
 bool page_locked(const void* p) {
@@ -987,7 +989,7 @@ int32_t ullis_cuda_binary_linear(ullis_cuda_runtime* rt, const float* x, const u
         if (rows == 0) return;
         need_ptr(x, "x"); need_ptr(bits, "bits"); need_ptr(scale, "scale"); need_ptr(y, "y");
         // whole 256-row tiles in every share but the last
-        const size_t shares = shares_for(ny * 4, rows, 256), share_rows = ((rows + shares - 1) / shares + 255) / 256 * 256;
+        const size_t shares = shares_for(rt, ny * 4, rows, 256), share_rows = ((rows + shares - 1) / shares + 255) / 256 * 256;
         Inputs in(rt);
         float* dx = shares > 1 ? rt->pool[0].as<float>(nx) : in.add(0, x, nx);
         uint32_t* dbits = in.add(1, bits, words);
@@ -1085,7 +1087,7 @@ int32_t ullis_cuda_rosa_qkv_1bit_fwd(ullis_cuda_runtime* rt, const uint32_t* q_b
         // Shares of whole sequences, whose planes begin on a word; 1 024 streams keep the device busy (not in the automaton, whose
         // launches last as long as a stream).
         const size_t result_bytes = (idx ? n : 0) + (out ? n * 4 : 0);
-        const size_t shares = time * channels % 32 || !k::rosa_without_automaton(rt, batch * channels, time) ? 1 : shares_for(result_bytes, batch, (1023 + channels) / channels);
+        const size_t shares = time * channels % 32 || !k::rosa_without_automaton(rt, batch * channels, time) ? 1 : shares_for(rt, result_bytes, batch, (1023 + channels) / channels);
         Inputs in(rt);
         uint32_t* planes[3];
         const uint32_t* const host[3] = {q_bits, k_bits, v_bits};
