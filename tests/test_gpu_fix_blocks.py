@@ -38,3 +38,17 @@ def test_flagged_signs_are_those_of_the_oracle(oracle, B, T, d, small):
     for m in "qkv":
         assert np.array_equal(unpack_plane(got[m + "_plane"], B * T * d), want[m + "_bits"]), m
     assert np.array_equal(got["idx"], want["idx"])
+
+
+@pytest.mark.parametrize("name", ["ULLIS_CUDA_FIX_BLOCKS", "ULLIS_CUDA_FIX_LIST"])
+def test_the_switch_by_either_name(monkeypatch, name):
+    monkeypatch.setenv(name, "0")
+    rt = cuda.CudaRuntime(0)
+    try:
+        x = np.random.default_rng(3).standard_normal((66, 64)).astype(np.float32)
+        rt.kernel_timing(True)
+        rt.rosa_block_forward(x.ravel(), _rosa_params(np.random.default_rng(4), 64), 2, 33, 64)
+        ran = rt.kernel_times()
+        assert "sign_fixup" in ran and "fix_block" not in ran
+    finally:
+        rt.close()

@@ -405,7 +405,8 @@ int32_t ullis_cuda_runtime_create(int32_t device, ullis_cuda_runtime** out) {
         if (const char* env = getenv("ULLIS_CUDA_SAM_SPARSE")) rt->sam_sparse_per_sm = (uint32_t)std::max(0, atoi(env));
         if (const char* env = getenv("ULLIS_CUDA_SAM_WORDS")) rt->sam_words = atoi(env) != 0;
         if (const char* env = getenv("ULLIS_CUDA_FUSE_LN")) rt->tc_fuse_ln = atoi(env) != 0;
-        if (const char* env = getenv("ULLIS_CUDA_FIX_LIST")) rt->tc_fix_blocks = atoi(env) != 0;
+        for (const char* name : {"ULLIS_CUDA_FIX_LIST", "ULLIS_CUDA_FIX_BLOCKS"})   // the first: its name when there was a list
+            if (const char* env = getenv(name)) rt->tc_fix_blocks = atoi(env) != 0;
         if (const char* env = getenv("ULLIS_CUDA_SAM_WALK_CHUNKED")) rt->sam_walk_chunked = atoi(env) != 0;
         if (const char* env = getenv("ULLIS_CUDA_LN_ROWS")) rt->tc_ln_rows = atoi(env);
         if (const char* env = getenv("ULLIS_CUDA_SAM_SMEM_WAVES")) rt->sam_smem_waves = std::max(0, atoi(env));
