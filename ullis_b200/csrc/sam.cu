@@ -350,13 +350,12 @@ struct ContextLimits {
 constexpr uint32_t CONTEXT_LARGE = 48;   // positions before a step in its buckets from which on the whole warp looks through them
 
 struct ContextLayout {   // bytes of shared memory
-    uint32_t hist, nq, start, q, k, q_ends, k_ends, in_word, before, out, entries, steps, total;   // for up to c bits
+    uint32_t hist, start, q, k, q_ends, k_ends, in_word, before, out, entries, steps, total;   // for up to c bits
     __host__ __device__ ContextLayout(uint32_t T, uint32_t c, uint32_t warps) {
         const uint32_t C = 1u << c, words = (T + 31u) / 32u + 1u;
         entries = 0;                           // Entry [T]
-        hist = entries + T * 8u;               // u16 [warps][C]: counts, then write positions
-        nq = hist + warps * C * 2u;            // u16 [C]: the same for the steps
-        start = nq + C * 2u;                   // u16 [C + 2]
+        hist = entries + T * 8u;               // u16 [warps][C]: counts, then write positions; behind them [C] for the steps
+        start = hist + (warps + 1u) * C * 2u;  // u16 [C + 2]
         q = start + (C + 2u) * 2u;
         k = q + words * 4u;
         before = k + words * 4u;               // u32 [2][words]
@@ -390,8 +389,6 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
     const ContextLayout L(T, uneven_bits, NW);
     uint16_t* hist = reinterpret_cast<uint16_t*>(context_mem + L.hist);
     uint32_t* hist2 = reinterpret_cast<uint32_t*>(context_mem + L.hist);   // two counts per word
-    uint16_t* nq = reinterpret_cast<uint16_t*>(context_mem + L.nq);
-    uint32_t* nq2 = reinterpret_cast<uint32_t*>(context_mem + L.nq);
     uint16_t* start = reinterpret_cast<uint16_t*>(context_mem + L.start);
     uint32_t* start2 = reinterpret_cast<uint32_t*>(context_mem + L.start);
     uint32_t* Q = reinterpret_cast<uint32_t*>(context_mem + L.q);
@@ -428,6 +425,7 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
         if (threadIdx.x == 0) Q[0] = K[0] = 0u;
         bool by_runs = false, taken = false, sorted = false;   // sorted: the steps bucket by bucket too
         uint32_t c = easy_bits, C = 1u << c, pair_words = C / 2u;
+        uint32_t* nq2 = hist2 + NW * pair_words;   // the same counts of the steps
         uint32_t pairs_by_bits = 0;
         auto key_of_key = [&](uint32_t r) {
             return by_runs ? context::run_key(K, k_ends, r, c) : context::window(K, r) >> (32u - c);
@@ -440,9 +438,9 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
                 c = uneven_bits;
                 C = 1u << c;
                 pair_words = C / 2u;
+                nq2 = hist2 + NW * pair_words;
             }
-            for (uint32_t i = threadIdx.x; i < NW * pair_words; i += NT) hist2[i] = 0u;
-            for (uint32_t i = threadIdx.x; i < pair_words; i += NT) nq2[i] = 0u;
+            for (uint32_t i = threadIdx.x; i < (NW + 1u) * pair_words; i += NT) hist2[i] = 0u;   // hist and nq
             __syncthreads();
             for (uint32_t row = row0; row < row1; ++row) {
                 const uint32_t r = row * 32u + lane;
