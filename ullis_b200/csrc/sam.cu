@@ -889,7 +889,8 @@ size_t stride_for(int algo, size_t T) {
 //                670 / 487 / 375     1077 / 745 / 573       1147 / 1120 / 754       3067 / 3227 / 2364
 //
 // Most streams listed: 512 threads up to 6 streams per SM (layers of the default model with gain 1 + N(0, 0.02), 2048 steps:
-// one sequence 0.89 / 0.80 ms in all layers, two 1.22 / 1.31, three 1.54 / 1.81).
+// one sequence 0.89 / 0.80 ms in all layers, two 1.22 / 1.31, three 1.54 / 1.81); below 1024 steps up to 7, where one launch then
+// takes both kinds (small model, gain N(0, 0.02), 4 times 512 steps 0.17 ms, with a launch for each 0.20).
 // Few listed: 1024 threads the longer the more streams there are.  One stream in eight listed, the others constant, 512 / 1024
 // threads: T = 1024, 2048 streams 47 / 49, 4096 68 / 70, 8192 100 / 121; T = 1531, 4096 112 / 109, 6144 129 / 144; T = 2048,
 // 4096 152 / 137, 6144 199 / 190, 8192 233 / 238; T = 4096, 8192 539 / 451.  Layers of the default model with gain N(0, 0.02),
@@ -911,7 +912,7 @@ void contexts(ullis_cuda_runtime* rt, const MatchCall& m) {
         uneven = rest = many;
     } else {
         uneven = std::max<int>(many, m.T >= 1024u && m.streams * 50u <= m.T * sms ? CONTEXT_1024 : CONTEXT_512);
-        rest = std::max<int>(many, m.streams <= 6u * sms ? CONTEXT_512 : CONTEXT_256);
+        rest = std::max<int>(many, m.streams <= (m.T < 1024u ? 7u : 6u) * sms ? CONTEXT_512 : CONTEXT_256);
     }
     const uint32_t all = ~0u, half = uneven == rest ? all : (uint32_t)(m.streams / 2) + 1u;
     auto launch = [&](int shape, uint32_t from, uint32_t to, const char* what) {
