@@ -115,10 +115,10 @@ __device__ __forceinline__ void cluster_wait() {
     __syncwarp();
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// The copies of a CTA, issued by one thread, and the waits for them.  gave_up: a wait of this CTA or of another one of its cluster
-// ran out.  Nobody waits, asks for copies or sends any more then: an mbarrier whose phase is not over must not be told to expect
-// the next one.  The stages run to their end on what lies in shared memory, which decides no address and no loop, so that everybody
-// passes the same barriers; the step reports the failure.
+// The copies of a CTA, issued by one thread, and the waits for them.  gave_up: where a wait of this CTA, or of another one of its
+// cluster, ran out.  Nobody waits, asks for copies or sends any more then: an mbarrier whose phase is not over must not be told to
+// expect the next one.  The stages run to their end on what lies in shared memory, which decides no address and no loop, so that
+// everybody passes the same barriers; the step reports the failure.
 constexpr uint32_t BARS = 2 * MAX_STAGES + 7, MAX_BOX = 256;
 struct Copies {
     uint64_t ring[BARS];   // mbarriers: a stage of the ring is full, is empty, one for each set of packed weights, for each exchange
@@ -137,21 +137,14 @@ __device__ __forceinline__ void copies_wait(Copies& copies, uint64_t* bar, uint3
         if (polls < p.polls && ptx::mbar_try_wait(bar, phase & 1u)) return;
         if (has_given_up(copies)) return;
     } while (polls++ < p.polls);
-    *static_cast<volatile uint32_t*>(&copies.gave_up) = 1u;
-    *static_cast<volatile uint32_t*>(p.status) = ULLIS_DEV_WAIT_TIMEOUT;
-    *static_cast<volatile uint32_t*>(p.status + 1) = site;
+    *static_cast<volatile uint32_t*>(&copies.gave_up) = site;
 }
 // n floats (a multiple of 4) of each of `rows` rows, `pitch` apart, from this CTA's shared memory to the same place in every
 // other CTA of the cluster, a CTA per warp at a time, counted on the receiver's barrier `bar`.  One thread says what this CTA's own
-// barrier has to wait for.  After a give-up the others are sent word of it in place of the share, and the result is false.
+// barrier has to wait for.  false: nothing was sent, after a give-up.
 __device__ __forceinline__ bool send_to_cluster(const float* from, uint32_t rows, uint32_t pitch, uint32_t n, Copies& copies, uint64_t* bar) {
     const uint32_t ctas = cluster_size(), me = cluster_rank(), lane = threadIdx.x & 31u;
-    if (has_given_up(copies)) {
-#pragma unroll 1
-        for (uint32_t cta = threadIdx.x; cta < ctas; cta += THREADS)
-            asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], %1;" ::"r"(ptx::cluster_map(&copies.gave_up, cta)), "r"(1u) : "memory");
-        return false;
-    }
+    if (has_given_up(copies)) return false;
     if (threadIdx.x == 0u) ptx::mbar_arrive_expect_tx(bar, (ctas - 1u) * rows * n * 4u);
 #pragma unroll 1
     for (uint32_t cta = threadIdx.x >> 5; cta < ctas; cta += WARPS) {
@@ -830,7 +823,12 @@ gen_step_kernel(const Step p) {
             }
             ++layers_done;
             __syncthreads();
-            if (send_to_cluster(x + o0, n, d, own, copies, copies.exchange(3u))) exchange_odd ^= 8u;
+            if (send_to_cluster(x + o0, n, d, own, copies, copies.exchange(3u))) {
+                exchange_odd ^= 8u;
+            } else if (threadIdx.x < ctas) {   // the others need not wait for what is not sent
+                asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], %1;" ::"r"(ptx::cluster_map(&copies.gave_up, threadIdx.x)),
+                             "r"(*static_cast<volatile uint32_t*>(&copies.gave_up)) : "memory");
+            }
             if (l + 1u < p.n_layers) {
                 fetch_qkv_o(layers[(l + 1u) & 1u]);
                 ahead = push_begin(l + 1u);
@@ -884,6 +882,8 @@ gen_step_kernel(const Step p) {
             for (uint32_t b = 0; b < 3u; ++b) ptx::mbar_wait(copies.qkv_o() + b, ~(packed_odd >> b) & 1u, DRAIN);
         }
         if (threadIdx.x == 0u) {
+            *static_cast<volatile uint32_t*>(p.status) = ULLIS_DEV_WAIT_TIMEOUT;
+            *static_cast<volatile uint32_t*>(p.status + 1) = copies.gave_up;
 #pragma unroll 1
             for (uint32_t b = 0; b < 4u; ++b) ptx::mbar_wait(copies.exchange(b), ~(exchange_odd >> b) & 1u, DRAIN);
 #pragma unroll 1
