@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "../../ullis_b200/csrc/rosa_context.cuh"
+#include "../../ullis_b200/csrc/rosa_heads.cuh"
 #include "../../ullis_b200/csrc/rosa_match.cuh"
 
 using namespace ullis;
@@ -104,17 +105,71 @@ void by_contexts(const uint32_t* q, const uint32_t* k, const uint32_t* v, uint32
     }
 }
 
+// One stream by the latest positions of its contexts, the rows of a warp lane by lane; the keys of the rows before row0 are put
+// in without answers.
+void by_heads(const uint32_t* q, const uint32_t* k, const uint32_t* v, uint32_t T, uint32_t row0, uint32_t* out) {
+    const uint32_t words = (T + 31u) / 32u;
+    std::vector<uint32_t> Q(words + 1u, 0u), K(words + 1u, 0u), latest_7(heads::LATEST_7, 0u), latest_3(heads::LATEST_3, 0u);
+    std::memcpy(Q.data() + 1, q, words * 4u);
+    std::memcpy(K.data() + 1, k, words * 4u);
+    std::vector<uint16_t> latest_11(heads::LATEST_11, 0), link(32u * words + 2u, 0);
+    for (uint32_t row = 0; row < words; ++row) {
+        uint32_t found[32], wk[32], wq[32];
+        for (uint32_t l = 0; l < 32u; ++l) {
+            wk[l] = context::window(K.data(), 32u * row + l);
+            wq[l] = context::window(Q.data(), 32u * row + l);
+            found[l] = heads::probe_11(latest_11.data(), wq[l]);
+            if (!found[l]) found[l] = heads::probe(latest_7.data(), wq[l], 7u);
+            if (!found[l]) found[l] = heads::probe(latest_3.data(), wq[l], 3u);
+        }
+        for (uint32_t l = 0; l < 32u; ++l) {   // in order, so that the last lane of a context counts
+            const uint32_t r1 = 32u * row + l + 1u;
+            link[r1] = latest_11[wk[l] >> 21];
+            latest_11[wk[l] >> 21] = (uint16_t)r1;
+            latest_7[wk[l] >> 25] = latest_3[wk[l] >> 29] = r1;
+        }
+        if (row < row0) continue;
+        out[row] = 0u;
+        for (uint32_t l = 0; l < 32u && 32u * row + l < T; ++l) {
+            const uint32_t t = 32u * row + l, below = (1u << l) - 1u;
+            const uint32_t in_row = row ? heads::agreeing<false>(K[row], K[row + 1u], below, wq[l]) : heads::agreeing<true>(0u, K[1], below, wq[l]);
+            if (in_row) {
+                const uint32_t near = heads::latest(row, in_row);
+                uint32_t bits = context::leading(wq[l] ^ wk[(near - 1u) & 31u]);
+                bits = bits < heads::DEPTH ? bits : heads::DEPTH;
+                bits = bits < near ? bits : near;
+                if (bits >= found[l] >> 16) found[l] = bits << 16 | near;
+            }
+            uint32_t r1 = found[l] & 0xFFFFu, best = 0, work = 0;
+            for (uint32_t p = found[l] >> 16 == heads::DEPTH ? r1 : 0u; p; p = link[p]) {
+                uint32_t n = context::leading(wq[l] ^ heads::window_before(K.data(), p));
+                if (n > p) n = p;
+                if (n == 32u) n = context::agreement(Q.data(), K.data(), t, p - 1u, 0u, work);
+                if (n > best) {
+                    best = n;
+                    r1 = p;
+                }
+            }
+            if (r1 && ((v[r1 >> 5] >> (r1 & 31u)) & 1u)) out[row] |= 1u << l;
+        }
+    }
+}
+
 }  // namespace
 
 // way: 0 = contexts by the last bits, 1 = the same with every bit of a context, 2 = by the lengths of the runs, 3 and 4 = as 1
-// and 2 with the bits of uneven streams, else the sets of lags in pieces of `way` steps (a multiple of 32)
+// and 2 with the bits of uneven streams, 5 = the latest positions of the contexts, else the sets of lags in pieces of `way` steps (a multiple of 32)
 extern "C" int rosa_host_batch(uint32_t way, const uint32_t* q, const uint32_t* k, const uint32_t* v, size_t n_streams,
                                uint32_t T, uint32_t* out) {
     const size_t wps = (T + 31u) / 32u;
     for (size_t s = 0; s < n_streams; ++s) {
         const size_t at = s * wps;
         if (way <= 4u) by_contexts(q + at, k + at, v + at, T, way > 2u ? context::bits_for_uneven(T) : context::bits_for(T), way == 2u || way == 4u, way == 0u, out + at);
-        else if (!by_lags(q + at, k + at, v + at, T, way, out + at)) return 1;
+        else if (way == 5u) {
+            const uint32_t half = (uint32_t)wps / 2u;   // in two pieces
+            if (half) by_heads(q + at, k + at, v + at, 32u * half, 0u, out + at);
+            by_heads(q + at, k + at, v + at, T, half, out + at);
+        } else if (!by_lags(q + at, k + at, v + at, T, way, out + at)) return 1;
     }
     return 0;
 }

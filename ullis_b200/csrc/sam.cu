@@ -3,7 +3,7 @@
 // RosaSam (src/rosa.rs:100-176) for every stream.
 //
 // Up to 8192 steps a stream needs no automaton (rosa_match below): every step
-// is looked up by itself (rosa_context.cuh) or in sets of lags
+// is looked up by itself (rosa_heads.cuh, rosa_context.cuh) or in sets of lags
 // (rosa_match.cuh), so no launch lasts as long as a stream's chain of steps.
 // 64 sequences x 512 channels x 2048 steps: 1.5 ms on evenly spread bits where
 // the automaton took 11.3, 0.79 against 2.10 per layer of the benchmark model;
@@ -20,6 +20,7 @@
 
 #include "kernels.hpp"
 #include "rosa_context.cuh"
+#include "rosa_heads.cuh"
 #include "rosa_match.cuh"
 #include "sam_coop.cuh"
 #include "sam_core.cuh"
@@ -42,11 +43,12 @@ __global__ void __launch_bounds__(128)
 rosa_classify_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restrict__ k_sw,
                      const uint32_t* __restrict__ v_sw, uint32_t* __restrict__ idx_sw, size_t streams, uint32_t T,
                      size_t wps, uint32_t* __restrict__ list, uint32_t* __restrict__ count,
-                     uint32_t* __restrict__ cq_list, uint32_t* __restrict__ cq_count) {
+                     uint32_t* __restrict__ cq_list, uint32_t* __restrict__ cq_count, uint32_t* __restrict__ given_up) {
     chain_entry();
     constexpr uint32_t G = CLASSIFY_LANES;
     const size_t s = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
     if (s >= streams) return;   // a whole group
+    if (given_up && threadIdx.x % G == 0) given_up[s] = 0u;
     const uint32_t sub = threadIdx.x % G, lane = threadIdx.x & 31u;
     const uint32_t group = ((1u << G) - 1u) << (lane & ~(G - 1u));
     const uint32_t* qw = q_sw + s * wps;
@@ -374,13 +376,14 @@ __host__ __device__ inline uint32_t context_bits(uint32_t T, bool together) { re
 // TOGETHER: large buckets by a whole warp, one step after the other, and one bit more for the streams that are not easy (a stream
 // at a time: default model with gain N(0, 0.02), contexts of 64 sequences 7.49 -> 6.97 ms, of one at 1000 steps 0.65 -> 0.54; with
 // the bit for every stream of a launch even ones paid, 148 of 2048 steps 26 -> 34 us, of 4096 41 -> 55).  Runs where the
-// number of listed streams is in [from, to).
+// number of listed streams is in [from, to); with `left` for that list where there are more.
 template <int NT, bool TOGETHER>
 __global__ void __launch_bounds__(NT, NT > 512 ? 1 : NT > 256 ? 2 : 5)
 rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restrict__ k_sw, const uint32_t* __restrict__ v_sw,
                     uint32_t* __restrict__ idx_sw, const uint32_t* __restrict__ list, const uint32_t* __restrict__ count,
-                    uint32_t* __restrict__ next, uint32_t* __restrict__ hard, uint32_t* __restrict__ hard_count, uint32_t T,
-                    size_t wps, uint32_t easy_bits, ContextLimits limits, uint32_t from, uint32_t to) {
+                    const uint32_t* __restrict__ left, const uint32_t* __restrict__ left_count, uint32_t* __restrict__ next,
+                    uint32_t* __restrict__ hard, uint32_t* __restrict__ hard_count, uint32_t T, size_t wps, uint32_t easy_bits,
+                    ContextLimits limits, uint32_t from, uint32_t to) {
     chain_entry();
     constexpr uint32_t NW = NT / 32, BRUTE = context::BRUTE;
     extern __shared__ __align__(16) uint8_t context_mem[];
@@ -403,8 +406,13 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
     uint16_t* large_steps = hist;   // after the sort; NW * C > T entries for the 16 warps of TOGETHER
     const context::Runs runs{k_ends, in_word, before_word};
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t total = *count;
-    if (total < from || total >= to) return;
+    uint32_t total = *count;
+    if (left && total >= to) {
+        list = left;
+        total = *left_count;
+    } else if (total < from || total >= to) {
+        return;
+    }
     const uint32_t rows_per_warp = (words + NW - 1u) / NW;
     const uint32_t row0 = min(warp * rows_per_warp, words), row1 = min(row0 + rows_per_warp, words);   // a warp's keys
     for (;;) {
@@ -703,10 +711,136 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
     }
 }
 
+// The streams whose keys are spread evenly (rosa_heads.cuh).  A stream is cut into `pieces`, a warp takes one: it puts the keys
+// of the rows before into tables of its own and goes on from there.  The other streams go to `left`, once: a stream is given up
+// as soon as the walks of a piece, the longest of each row, have come to more than `base` + `per_row` positions per row so far, 32
+// steps beyond the first window counted as a position.  given_up: a word per stream, zero before.
+// Warps per CTA: they have nothing to do with one another, but at 2048 steps two CTAs of 12 leave less shared memory idle than five of
+// four (20 warps per SM, not 24: 16 sequences in all layers 3.85 / 3.56 ms; 8 times 300 steps 0.39 / 0.42).
+constexpr int HEAD_WARPS = 12;
+
+struct HeadsLayout {   // bytes of shared memory of a warp
+    uint32_t latest_7, latest_3, link, q, k, v, total;   // latest_11 is at 0
+    __host__ __device__ explicit HeadsLayout(uint32_t T) {
+        const uint32_t words = (T + 31u) / 32u;
+        latest_7 = heads::LATEST_11 * 2u;
+        latest_3 = latest_7 + heads::LATEST_7 * 4u;
+        link = latest_3 + heads::LATEST_3 * 4u;   // u16 [32 * words + 2]: by position + 1, the latest one before it with its context
+        q = link + (32u * words + 2u) * 2u;       // u32 [words + 1]
+        k = q + (words + 1u) * 4u;
+        v = k + (words + 1u) * 4u;                // u32 [words]
+        total = (v + words * 4u + 15u) & ~15u;
+    }
+};
+
+struct HeadsLimits {
+    uint32_t base, per_row;
+};
+
+// Bound by the integer pipe: per row of 32 steps of the model's streams (2048 steps) about 350 warp instructions, 215 of them on
+// that pipe, which takes one every second cycle - the refinement of the masks 100, the look-ups 70, the walk over the
+// chains 70, the keys 40.  rosa_context_kernel sorts each stream first and compares what lies in a bucket: 750 per row.  Both kernels
+// in all layers, gain 1 + N(0, 0.02), contexts alone before: default model 64 times 2048 steps 21.5 -> 12.8 ms, 16 5.8 -> 4.3, 8 3.2 -> 2.6,
+// 64 times 512 6.5 -> 2.7, 16 times 700 2.4 -> 1.3.
+__global__ void __launch_bounds__(32 * HEAD_WARPS)
+rosa_heads_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restrict__ k_sw, const uint32_t* __restrict__ v_sw,
+                  uint32_t* __restrict__ idx_sw, const uint32_t* __restrict__ list, const uint32_t* __restrict__ count,
+                  uint32_t* __restrict__ next, uint32_t* __restrict__ left, uint32_t* __restrict__ left_count,
+                  uint32_t* __restrict__ given_up, uint32_t T, size_t wps, uint32_t pieces, uint32_t from, HeadsLimits limits) {
+    chain_entry();
+    constexpr uint32_t ALL = 0xFFFFFFFFu;
+    extern __shared__ __align__(16) uint8_t heads_mem[];
+    const uint32_t words = (T + 31u) / 32u, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const HeadsLayout L(T);
+    uint8_t* mem = heads_mem + warp * L.total;
+    uint16_t* latest_11 = reinterpret_cast<uint16_t*>(mem);
+    uint32_t* latest_7 = reinterpret_cast<uint32_t*>(mem + L.latest_7);
+    uint32_t* latest_3 = reinterpret_cast<uint32_t*>(mem + L.latest_3);
+    uint16_t* link = reinterpret_cast<uint16_t*>(mem + L.link);
+    uint32_t* Q = reinterpret_cast<uint32_t*>(mem + L.q);
+    uint32_t* K = reinterpret_cast<uint32_t*>(mem + L.k);
+    uint32_t* V = reinterpret_cast<uint32_t*>(mem + L.v);
+    const uint32_t total = *count >= from ? *count : 0u, warps = gridDim.x * HEAD_WARPS, above = ALL << lane << 1, below = (1u << lane) - 1u;
+    const uint32_t piece_rows = (words + pieces - 1u) / pieces;
+    auto keys_in = [&](uint32_t row, uint32_t wk) {
+        const uint32_t r1 = 32u * row + lane + 1u, ctx = wk >> 21;
+        uint32_t before = latest_11[ctx];
+        atomicMax(&latest_7[wk >> 25], r1);
+        atomicMax(&latest_3[wk >> 29], r1);
+        __syncwarp();   // the tables have been read
+        latest_11[ctx] = (uint16_t)r1;
+        __syncwarp();
+        if (__any_sync(ALL, latest_11[ctx] != (uint16_t)r1)) {   // a context twice in the row: its last lane counts
+            const uint32_t same = __match_any_sync(ALL, ctx);
+            if (!(same & above)) latest_11[ctx] = (uint16_t)r1;
+            if (same & below) before = heads::latest(row, same & below);
+        }
+        link[r1] = (uint16_t)before;
+        __syncwarp();
+    };
+    // The last pieces first, which have the most keys to put in.
+    for (uint32_t item = warp * gridDim.x + blockIdx.x; item < total * pieces;
+         item = warps + __shfl_sync(ALL, lane == 0u ? atomicAdd(next, 1u) : 0u, 0)) {
+        const uint32_t piece = pieces - 1u - item / total;
+        const size_t s = list[item % total], at = s * wps;
+        const uint32_t row0 = min(piece * piece_rows, words), row1 = min(row0 + piece_rows, words);
+        __syncwarp();
+        for (uint32_t w = lane; w < row1; w += 32u) {
+            Q[w + 1u] = q_sw[at + w];
+            K[w + 1u] = k_sw[at + w];
+            V[w] = v_sw[at + w];
+        }
+        if (lane == 0u) Q[0] = K[0] = 0u;
+        for (uint32_t i = lane; i < L.link / 16u; i += 32u) reinterpret_cast<uint4*>(mem)[i] = uint4{0u, 0u, 0u, 0u};
+        __syncwarp();
+        uint32_t k0 = 0u, q0 = Q[row0], work = 0;
+        for (uint32_t row = 0; row < row0; ++row) {
+            const uint32_t k1 = K[row + 1u];
+            keys_in(row, __funnelshift_l(k0, k1, 31u - lane));
+            k0 = k1;
+        }
+        bool gone = false;
+        for (uint32_t row = row0; row < row1 && !gone; ++row) {
+            const uint32_t k1 = K[row + 1u], q1 = Q[row + 1u], t = 32u * row + lane;
+            const uint32_t wk = __funnelshift_l(k0, k1, 31u - lane), wq = __funnelshift_l(q0, q1, 31u - lane);
+            uint32_t found = heads::probe_11(latest_11, wq);
+            if (!found) found = heads::probe(latest_7, wq, 7u);
+            if (!found) found = heads::probe(latest_3, wq, 3u);
+            const uint32_t in_row = row ? heads::agreeing<false>(k0, k1, below, wq) : heads::agreeing<true>(k0, k1, below, wq);
+            k0 = k1;
+            q0 = q1;
+            __syncwarp();
+            keys_in(row, wk);
+            // the latest lane of those that agree longest, and in how many bits
+            const uint32_t near = heads::latest(row, in_row), near_key = __shfl_sync(ALL, wk, (near - 1u) & 31u);
+            const uint32_t near_bits = min(min(context::leading(wq ^ near_key), heads::DEPTH), near);
+            if (in_row && near_bits >= found >> 16) found = near_bits << 16 | near;
+            const uint32_t most = limits.base + limits.per_row * (row - row0) - work;   // not below 0: the stream would be gone
+            uint32_t r1 = found & 0xFFFFu, best = 0, walked = 0, p = found >> 16 == heads::DEPTH && t < T ? r1 : 0u;
+            while (p && walked <= most) {
+                uint32_t n = min(context::leading(wq ^ heads::window_before(K, p)), p);
+                if (n == 32u) n = context::agreement(Q, K, t, p - 1u, 0u, walked);
+                if (n > best) {
+                    best = n;
+                    r1 = p;
+                }
+                p = link[p];
+                ++walked;
+            }
+            walked = __reduce_max_sync(ALL, walked);
+            work += walked;
+            gone = walked > most;
+            const uint32_t word = __ballot_sync(ALL, r1 && t < T && (V[r1 >> 5] >> (r1 & 31u) & 1u));
+            if (lane == 0u) idx_sw[at + row] = word;
+        }
+        if (gone && lane == 0u && atomicExch(&given_up[s], 1u) == 0u) left[atomicAdd(left_count, 1u)] = (uint32_t)s;
+    }
+}
+
 // The remaining streams by sets of lags (rosa_match.cuh).  A work item is a piece of one stream, a warp takes items
 // from a counter until they run out; the warps of a CTA have nothing to do with one another.
 constexpr int MATCH_WARPS = 4;
-constexpr uint32_t MATCH_COUNTS = 5;   // of MatchCall
+constexpr uint32_t MATCH_COUNTS = 7;   // of MatchCall
 
 // A stream whose query bits are all c: idx follows the longest run of c among the keys so far, the latest of equals
 // (sam_core.cuh run_constant_q), a running maximum over (run length, position).  T <= 65535.
@@ -791,11 +925,14 @@ rosa_match_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restrict_
 }
 
 constexpr size_t MATCH_MAX_TIME = 8192;   // 256 words of lags, eight per lane
+constexpr uint32_t HEADS_MAX_TIME = 2048;
 
 struct MatchCall {   // the buffers of one call
     const uint32_t *q, *k, *v;
-    uint32_t *idx, *list, *cq_list, *hard;
-    uint32_t *counts, *clear;   // listed, constant q, hard, next of the contexts, next of the matches; those of the next call
+    uint32_t *idx, *list, *cq_list, *hard, *left, *given_up;
+    // listed, constant q, hard, next of the contexts, next of the matches, left by the latest positions, their next; those of the
+    // next call
+    uint32_t *counts, *clear;
     size_t streams, wps;
     uint32_t T;
 };
@@ -820,7 +957,7 @@ void prepare_context(ullis_cuda_runtime* rt, uint32_t T, int shape) {
 }
 
 template <int NT, bool TOGETHER>
-void launch_context(ullis_cuda_runtime* rt, const MatchCall& m, int shape, uint32_t from, uint32_t to, const char* what) {
+void launch_context(ullis_cuda_runtime* rt, const MatchCall& m, int shape, const uint32_t* left, uint32_t from, uint32_t to, const char* what) {
     const unsigned grid = (unsigned)std::min<size_t>(rt->context_ctas[shape], m.streams);
     // A match kernel step costs about as much as 100 positions here; up to 24 the lanes are even enough without sorting
     // the steps.  What a thread has compared when its stream turns out to repeat itself is thrown away: by bits 64 long
@@ -829,8 +966,37 @@ void launch_context(ullis_cuda_runtime* rt, const MatchCall& m, int shape, uint3
     // ever change went to the match kernel).
     const ContextLimits limits{24u, 96u, 160u, 64u, 256u};
     rt->chain(rosa_context_kernel<NT, TOGETHER>, grid, NT, rt->context_smem[shape], m.q, m.k, m.v, m.idx, m.list, m.counts,
-              m.counts + 3, m.hard, m.counts + 2, m.T, m.wps, context::bits_for(m.T), limits, from, to);
+              left, m.counts + 5, m.counts + 3, m.hard, m.counts + 2, m.T, m.wps, context::bits_for(m.T), limits, from, to);
     rt->launched(what);
+}
+
+// Where at least `from` streams are listed.
+void launch_heads(ullis_cuda_runtime* rt, const MatchCall& m, uint32_t from) {
+    const size_t smem = (size_t)HeadsLayout(m.T).total * HEAD_WARPS;
+    if (!rt->heads_smem) {
+        const size_t most = (size_t)HeadsLayout(HEADS_MAX_TIME).total * HEAD_WARPS;
+        ULLIS_CUDA_CHECK(cudaFuncSetAttribute(rosa_heads_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+    }
+    if (rt->heads_smem != smem) {
+        int per_sm = 0;
+        ULLIS_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rosa_heads_kernel, 32 * HEAD_WARPS, smem));
+        rt->heads_ctas = std::max(1, per_sm) * rt->sm_count;
+        rt->heads_smem = smem;
+    }
+    const size_t warps = (size_t)rt->heads_ctas * HEAD_WARPS;
+    // More pieces make a launch of few streams shorter and one of many longer, since their warps put in the same keys again.  Below
+    // 1024 steps a piece costs more than it saves unless warps would be idle (gain 1 + N(0, 0.02), ROSA kernels in all layers with four
+    // warps per CTA, 1 / 2 / 4 pieces: 16 times 700 steps of the default model 1.51 / 1.66 / 1.81 ms, 3 times 333 of the small one 0.255 / 0.235 /
+    // 0.236; 2048 steps of the default model: 4 sequences 2.90 / 2.45 / 2.10, 8 3.71 / 3.11 / 2.99, 16 5.09 / 4.75 / 4.97, 64 14.0 / 14.4 / 16.7).
+    const uint32_t pieces = m.T < 1024u ? (m.streams * 4u <= warps ? 4u : 1u) : m.streams * 2u < 3u * warps ? 4u : m.streams < 8u * warps ? 2u : 1u;
+    const unsigned grid = (unsigned)std::min<size_t>(rt->heads_ctas, (m.streams * pieces + HEAD_WARPS - 1) / HEAD_WARPS);
+    // A row whose walks are 29 positions long takes as many instructions as in rosa_context_kernel.  Less than 16 leaves it streams that
+    // are cheaper here (8 times 2048 steps 12 / 16 / 24 / 32 per row 3.12 / 3.03 / 2.94 / 2.95 ms, 16 times 1100 2.43 / 2.46 / 2.44 / 2.41),
+    // and a base too small all that are short (twice 700 steps, base 32 / 64 / 128: 0.75 / 0.62 / 0.61).
+    const HeadsLimits limits{128u, 24u};
+    rt->chain(rosa_heads_kernel, grid, 32 * HEAD_WARPS, smem, m.q, m.k, m.v, m.idx, m.list, m.counts, m.counts + 6, m.left, m.counts + 5,
+              m.given_up, m.T, m.wps, pieces, from, limits);
+    rt->launched("rosa_heads");
 }
 
 template <int NW>
@@ -867,7 +1033,7 @@ size_t stride_for(int algo, size_t T) {
                                         : sam::EulerLayout<Ix>((uint32_t)T).total;
 }
 
-// The listed streams by contexts, in the shapes that suit how many there are.  That number is known on the device only,
+// The listed streams by the latest positions or by contexts, in the shapes that suit how many there are.  That number is known on the device only,
 // where a launch whose range it misses leaves at once: one launch for the calls where most streams had a closed form, whose
 // others are uneven (large buckets), one for the rest - a single one where both are of the same shape.
 //
@@ -914,14 +1080,22 @@ void contexts(ullis_cuda_runtime* rt, const MatchCall& m) {
         uneven = std::max<int>(many, m.T >= 1024u && m.streams * 50u <= m.T * sms ? CONTEXT_1024 : CONTEXT_512);
         rest = std::max<int>(many, m.streams <= (m.T < 1024u ? 7u : 6u) * sms ? CONTEXT_512 : CONTEXT_256);
     }
-    const uint32_t all = ~0u, half = uneven == rest ? all : (uint32_t)(m.streams / 2) + 1u;
+    // The latest positions, where most streams are listed: one warp per stream or piece, so there have to be enough of them (all layers,
+    // gain 1 + N(0, 0.02), contexts / latest positions, ms; 2048 steps: two sequences of the default model 1.57 / 1.73, three 1.83 / 1.93, four
+    // 2.18 / 2.05, eight 3.49 / 2.82, 64 21.7 / 13.1; 1100 steps: two 1.01 / 1.06, four 1.39 / 1.25; 700: one 0.58 / 0.69, two 0.81 / 0.62, 16 2.57 / 1.49;
+    // 300: two 0.51 / 0.45, 64 5.88 / 1.98).  Where few are listed those are uneven, and their chains long: 64 times 2048 steps with gain
+    // N(0, 0.02) 7.7 / 9.3.  Beyond 2048 steps chains and tables grow (8192 steps of bits of probability 0.25 to 0.6: 1.09 / 1.63).
+    const bool by_heads = m.T <= HEADS_MAX_TIME && m.streams > (m.T < 512u ? 4u : m.T < 1024u ? 5u : 12u) * sms;
+    const uint32_t all = ~0u, half = uneven == rest && !by_heads ? all : (uint32_t)(m.streams / 2) + 1u;
     auto launch = [&](int shape, uint32_t from, uint32_t to, const char* what) {
-        if (shape == CONTEXT_256) launch_context<256, false>(rt, m, shape, from, to, what);
-        else if (shape == CONTEXT_512) launch_context<512, true>(rt, m, shape, from, to, what);
-        else launch_context<1024, true>(rt, m, shape, from, to, what);
+        const uint32_t* left = by_heads ? m.left : nullptr;
+        if (shape == CONTEXT_256) launch_context<256, false>(rt, m, shape, left, from, to, what);
+        else if (shape == CONTEXT_512) launch_context<512, true>(rt, m, shape, left, from, to, what);
+        else launch_context<1024, true>(rt, m, shape, left, from, to, what);
     };
+    if (by_heads) launch_heads(rt, m, half);
     launch(uneven, 0u, half, "rosa_context");
-    if (half != all) launch(rest, half, all, "rosa_context_even");
+    if (!by_heads && half != all) launch(rest, half, all, "rosa_context_even");
 }
 
 // The whole call without an automaton: classification, the listed streams by contexts, and by sets of lags those that
@@ -931,15 +1105,17 @@ void rosa_match(ullis_cuda_runtime* rt, const uint32_t* q_sw, const uint32_t* k_
     MatchCall m;
     m.q = q_sw; m.k = k_sw; m.v = v_sw; m.idx = idx_sw;
     m.streams = streams; m.T = T; m.wps = (T + 31u) / 32u;
-    m.list = rt->sam_list.as<uint32_t>(3 * streams);
+    m.list = rt->sam_list.as<uint32_t>(5 * streams);
     m.cq_list = m.list + streams;
     m.hard = m.cq_list + streams;
+    m.left = m.hard + streams;
+    m.given_up = m.left + streams;
     rt->counters(rt->match_counters, MATCH_COUNTS, &m.counts, &m.clear);
     rt->sam_last_counts = m.counts;
     rt->sam_last_streams = streams;
     if (!rt->parent) rt->lanes_last = 1;
     rt->chain(rosa_classify_kernel, (unsigned)((streams * CLASSIFY_LANES + 127) / 128), 128, 0, q_sw, k_sw, v_sw, idx_sw,
-              streams, T, m.wps, m.list, m.counts, m.cq_list, m.counts + 1);
+              streams, T, m.wps, m.list, m.counts, m.cq_list, m.counts + 1, m.given_up);
     rt->launched("rosa_classify");
     contexts(rt, m);
     if (T <= 1024u) launch_match<1>(rt, m, 0, 1024);
@@ -1019,7 +1195,7 @@ void rosa_sam(ullis_cuda_runtime* rt, const uint32_t* q_sw, const uint32_t* k_sw
         rt->zero(count, 8);   // both counters
         const unsigned classify_grid = (unsigned)((streams * CLASSIFY_LANES + 127) / 128);
         rt->chain(rosa_classify_kernel, classify_grid, 128, 0, q_sw, k_sw, v_sw, idx_sw, streams, (uint32_t)time, wps, list,
-                                                             count, cq_list, cq_count);
+                                                             count, cq_list, cq_count, nullptr);
         rt->launched("rosa_classify");
         // The constant-q scan is a long serial loop for a few thousand threads; it depends on nothing but the
         // classification and writes idx words no other kernel of this call touches, so it runs on the side stream
