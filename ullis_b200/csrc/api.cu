@@ -5,6 +5,8 @@
 #include <cstdio>
 #include <cstring>
 #include <exception>
+#include <map>
+#include <mutex>
 #include <new>
 
 #include "kernels.hpp"
@@ -99,6 +101,52 @@ struct Inputs {
                 rt->inputs_used - rt->inputs_sent);
         rt->inputs_sent = rt->inputs_used;
     }
+};
+
+// The blocks of ullis_cuda_host_alloc: what lies in one can be written by kernels of any device.
+struct HostBlocks {
+    std::mutex lock;
+    std::map<uintptr_t, size_t> sizes;
+    bool hold(const void* p, size_t bytes) {
+        std::lock_guard<std::mutex> held(lock);
+        const uintptr_t at = reinterpret_cast<uintptr_t>(p);
+        auto it = sizes.upper_bound(at);
+        return it != sizes.begin() && (--it, at - it->first + bytes <= it->second);
+    }
+};
+HostBlocks& host_blocks() {
+    static HostBlocks* blocks = new HostBlocks;   // never gone: blocks may be freed while the process ends
+    return *blocks;
+}
+
+// The results of an op-level call and its status: by one kernel if they are small and go to blocks of ullis_cuda_host_alloc, else by
+// a copy each.  256 KB: beyond that the copy engine moves them faster than a few blocks' stores.
+struct Results {
+    ullis_cuda_runtime* rt;
+    k::HostCopy copies[k::MAX_HOST_COPIES];
+    uint32_t n = 0;
+    size_t bytes = 0;
+    explicit Results(ullis_cuda_runtime* r) : rt(r) {}
+    void add(void* to, const void* from, size_t size) {   // fewer than MAX_HOST_COPIES
+        if (!to || !size) return;
+        copies[n++] = k::HostCopy{to, from, (uint32_t)std::min<size_t>(size, ~0u)};
+        bytes += size;
+        sizes[n - 1] = size;
+    }
+    void finish() {
+        bool small = bytes <= (256u << 10);
+        for (uint32_t i = 0; i < n && small; ++i) small = host_blocks().hold(copies[i].to, sizes[i]);
+        if (!small) {
+            for (uint32_t i = 0; i < n; ++i) rt->d2h(copies[i].to, copies[i].from, sizes[i]);
+            rt->check_status();
+            return;
+        }
+        copies[n] = k::HostCopy{rt->host_status, rt->dev_status, 16u};
+        k::copies_to_host(rt, copies, n + 1);
+        rt->sync();
+        rt->throw_on_status();
+    }
+    size_t sizes[k::MAX_HOST_COPIES];
 };
 
 // An op-level call in shares: the inputs of a share are copied while the one before it is computed, its results while the
@@ -571,11 +619,18 @@ int32_t ullis_cuda_host_alloc(ullis_cuda_runtime* rt, size_t bytes, void** out) 
             *out = nullptr;
             fail(ULLIS_CUDA_ERR_NOMEM, "page-locked host allocation failed");
         }
+        std::lock_guard<std::mutex> held(host_blocks().lock);
+        host_blocks().sizes[reinterpret_cast<uintptr_t>(*out)] = bytes ? bytes : 1;
     });
 }
 
 void ullis_cuda_host_free(void* block) {
-    if (block) cudaFreeHost(block);
+    if (!block) return;
+    {
+        std::lock_guard<std::mutex> held(host_blocks().lock);
+        host_blocks().sizes.erase(reinterpret_cast<uintptr_t>(block));
+    }
+    cudaFreeHost(block);
 }
 
 int32_t ullis_cuda_runtime_wait_selftest(ullis_cuda_runtime* rt, uint32_t polls) {
@@ -1183,16 +1238,21 @@ int32_t ullis_cuda_rosa_block_forward(ullis_cuda_runtime* rt, const float* x, co
         const size_t plane_words = (n + 31) / 32;
         uint32_t* dplanes = rt->pool[20].as<uint32_t>(3 * plane_words);
         uint32_t* planes_out[3] = {q_plane, k_plane, v_plane};
-        uint32_t* planes_in[3] = {qs, ks, vs};
+        const uint32_t* planes_in[3] = {qs, ks, vs};
+        const uint32_t* from[3];
+        uint32_t *to[3], asked = 0;
+        Results results(rt);
         for (int i = 0; i < 3; ++i) {
             if (!planes_out[i]) continue;
-            k::streams_to_planes(rt, planes_in[i], dplanes + i * plane_words, batch, time, d);
-            rt->d2h(planes_out[i], dplanes + i * plane_words, plane_words * 4);
+            from[asked] = planes_in[i];
+            to[asked++] = dplanes + i * plane_words;
+            results.add(planes_out[i], dplanes + i * plane_words, plane_words * 4);
         }
-        if (idx) rt->d2h(idx, didx, n);
-        if (y) rt->d2h(y, w, n * 4);
-        if (out) rt->d2h(out, dout, n * 4);
-        rt->check_status();
+        k::streams_to_planes(rt, from, to, asked, batch, time, d);
+        results.add(idx, didx, n);
+        results.add(y, w, n * 4);
+        results.add(out, dout, n * 4);
+        results.finish();
     });
 }
 

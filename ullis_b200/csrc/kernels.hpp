@@ -26,8 +26,17 @@ void sign_pack_streams(ullis_cuda_runtime* rt, const float* x, uint32_t* sw, siz
                        size_t channels);
 void planes_to_streams(ullis_cuda_runtime* rt, const uint32_t* plane, uint32_t* sw, size_t batch, size_t time,
                        size_t channels);
-void streams_to_planes(ullis_cuda_runtime* rt, const uint32_t* sw, uint32_t* plane, size_t batch, size_t time,
-                       size_t channels);
+// ... of up to three sets of streams
+void streams_to_planes(ullis_cuda_runtime* rt, const uint32_t* const* sw, uint32_t* const* plane, uint32_t n_sets, size_t batch,
+                       size_t time, size_t channels);
+// Up to MAX_HOST_COPIES results, `to` page-locked.
+constexpr uint32_t MAX_HOST_COPIES = 8;
+struct HostCopy {
+    void* to;
+    const void* from;
+    uint32_t bytes;
+};
+void copies_to_host(ullis_cuda_runtime* rt, const HostCopy* copies, uint32_t n);
 void relu2(ullis_cuda_runtime* rt, const float* x, float* y, size_t n);
 void residual_add(ullis_cuda_runtime* rt, const float* a, const float* b, float* out, size_t n);
 // From stream-major idx bits: idx u8 [B,T,C] (nullable) and y = (2*idx-1)*e f32 (nullable).
