@@ -10,8 +10,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("T,B,C,odd", [(1, 9, 256, 0.0), (12, 9, 256, 0.2), (33, 3, 256, 0.2), (64, 40, 512, 0.1), (127, 3, 256, 0.3), (511, 3, 256, 0.3),
-                                       (513, 3, 256, 0.3), (700, 16, 512, 0.1), (1023, 3, 256, 0.3), (1024, 4, 512, 0.2), (1025, 15, 512, 0.02),
-                                       (1100, 4, 512, 0.4), (1531, 8, 256, 0.2), (2047, 4, 512, 0.2), (2048, 8, 256, 0.3), (1024, 72, 512, 0.0)])
+                                       (513, 3, 256, 0.3), (700, 16, 512, 0.1), (1023, 3, 256, 0.3), (1024, 5, 512, 0.2), (1025, 15, 512, 0.02),
+                                       (1100, 5, 512, 0.4), (1531, 9, 256, 0.2), (2047, 5, 512, 0.2), (2048, 9, 256, 0.3), (1024, 72, 512, 0.0)])
 def test_even_streams_beside_others(cuda_rt, oracle, T, B, C, odd):
     rng = np.random.default_rng([T, B, C])
     kinds = ["even", "biased", "repeating", "constant_q"]

@@ -109,8 +109,6 @@ struct ullis_cuda_runtime {
     int match_ctas[4] = {0, 0, 0, 0};   // CTAs of the match kernel the device holds at once, per width of its sets
     int context_ctas[3] = {};       // the same for the context kernel, per shape, for the shared memory it was last asked for
     size_t context_smem[3] = {};
-    int heads_ctas = 0;             // and for the kernel of the latest positions
-    size_t heads_smem = 0;
     bool sam_coop = true;               // warp-cooperative tour / pass 2 when the stream fits shared memory
     bool sam_coop_ready = false;
     bool sam_lanes_fixed = false;       // ULLIS_CUDA_SAM_LANES was given: no per-launch choice in pass 1

@@ -43,7 +43,8 @@ __global__ void __launch_bounds__(128)
 rosa_classify_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restrict__ k_sw,
                      const uint32_t* __restrict__ v_sw, uint32_t* __restrict__ idx_sw, size_t streams, uint32_t T,
                      size_t wps, uint32_t* __restrict__ list, uint32_t* __restrict__ count,
-                     uint32_t* __restrict__ cq_list, uint32_t* __restrict__ cq_count, uint32_t* __restrict__ given_up) {
+                     uint32_t* __restrict__ cq_list, uint32_t* __restrict__ cq_count, uint32_t* __restrict__ given_up,
+                     bool clear_listed) {
     chain_entry();
     constexpr uint32_t G = CLASSIFY_LANES;
     const size_t s = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
@@ -116,9 +117,13 @@ rosa_classify_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restri
                 out[w] = word;
             }
         }
-    } else if (sub == 0) {
-        if (constant(2, &c)) cq_list[atomicAdd(cq_count, 1u)] = (uint32_t)s;   // constant q: a long scan, its own kernel
-        else list[atomicAdd(count, 1u)] = (uint32_t)s;
+    } else {
+        if (clear_listed)   // rosa_context_kernel puts the words of a stream together from several CTAs
+            for (uint32_t w = sub; w <= last; w += G) out[w] = 0u;
+        if (sub == 0) {
+            if (constant(2, &c)) cq_list[atomicAdd(cq_count, 1u)] = (uint32_t)s;   // constant q: a long scan, its own kernel
+            else list[atomicAdd(count, 1u)] = (uint32_t)s;
+        }
     }
 }
 
@@ -349,10 +354,14 @@ struct ContextLimits {
     uint32_t deep_by_bits, deep_by_runs;
 };
 
+// Where less than half of the CTAs would have a stream, two or more take one: each sorts all of its keys and answers its share of the
+// steps (one sequence of the default model with gain N(0, 0.02), 64 of 512 streams listed, 148 CTAs: the slowest stream 130 000 cycles,
+// 22 000 of them for the sort).
+constexpr uint32_t MAX_PARTS = 4, PARTS_MAX_STREAMS = 8;
 constexpr uint32_t CONTEXT_LARGE = 48;   // positions before a step in its buckets from which on the whole warp looks through them
 
 struct ContextLayout {   // bytes of shared memory
-    uint32_t hist, start, q, k, q_ends, k_ends, in_word, before, out, entries, steps, total;   // for up to c bits
+    uint32_t hist, start, q, k, v, q_ends, k_ends, in_word, before, out, entries, steps, total;   // for up to c bits
     __host__ __device__ ContextLayout(uint32_t T, uint32_t c, uint32_t warps) {
         const uint32_t C = 1u << c, words = (T + 31u) / 32u + 1u;
         entries = 0;                           // Entry [T]
@@ -360,7 +369,8 @@ struct ContextLayout {   // bytes of shared memory
         start = hist + (warps + 1u) * C * 2u;  // u16 [C + 2]
         q = start + (C + 2u) * 2u;
         k = q + words * 4u;
-        before = k + words * 4u;               // u32 [2][words]
+        v = k + words * 4u;
+        before = v + words * 4u;               // u32 [2][words]
         out = before + words * 8u;
         in_word = out + words * 4u;             // u16 [2][words]
         q_ends = in_word + words * 4u;         // u16 [words]
@@ -373,17 +383,140 @@ struct ContextLayout {   // bytes of shared memory
 // Bits of the longest contexts of a shape.
 __host__ __device__ inline uint32_t context_bits(uint32_t T, bool together) { return together ? context::bits_for_uneven(T) : context::bits_for(T); }
 
+// The streams whose keys are spread evenly (rosa_heads.cuh).  A stream is cut into `pieces`, a warp takes one: it puts the keys
+// of the rows before into tables of its own and goes on from there.  The other streams go to `left`, once: a stream is given up
+// as soon as the walks of a piece, the longest of each row, have come to more than `base` + `per_row` positions per row so far, 32
+// steps beyond the first window counted as a position.  given_up: a word per stream, zero before.
+struct HeadsLayout {   // bytes of shared memory of a warp
+    uint32_t latest_7, latest_3, link, q, k, v, total;   // latest_11 is at 0
+    __host__ __device__ explicit HeadsLayout(uint32_t T) {
+        const uint32_t words = (T + 31u) / 32u;
+        latest_7 = heads::LATEST_11 * 2u;
+        latest_3 = latest_7 + heads::LATEST_7 * 4u;
+        link = latest_3 + heads::LATEST_3 * 4u;   // u16 [32 * words + 2]: by position + 1, the latest one before it with its context
+        q = link + (32u * words + 2u) * 2u;       // u32 [words + 1]
+        k = q + (words + 1u) * 4u;
+        v = k + (words + 1u) * 4u;                // u32 [words]
+        total = (v + words * 4u + 15u) & ~15u;
+    }
+};
+
+struct HeadsCall {
+    uint32_t warps;   // of a CTA that take pieces: as many as have room in its shared memory
+    uint32_t pieces, base, per_row;
+    uint32_t *next, *left, *left_count, *given_up;
+};
+
+// Bound by the integer pipe: per row of 32 steps of the model's streams (2048 steps) about 350 warp instructions, 215 of them on
+// that pipe, which takes one every second cycle - the refinement of the masks 100, the look-ups 70, the walk over the
+// chains 70, the keys 40.  rosa_context_kernel sorts each stream first and compares what lies in a bucket: 750 per row.  Both kernels
+// in all layers, gain 1 + N(0, 0.02), contexts alone before: default model 64 times 2048 steps 21.5 -> 12.8 ms, 16 5.8 -> 4.3, 8 3.2 -> 2.6,
+// 64 times 512 6.5 -> 2.7, 16 times 700 2.4 -> 1.3.
+__device__ __forceinline__ void heads_streams(const uint32_t* __restrict__ q_sw, const uint32_t* __restrict__ k_sw, const uint32_t* __restrict__ v_sw,
+                                              uint32_t* __restrict__ idx_sw, const uint32_t* __restrict__ list, uint32_t total, uint32_t T, size_t wps,
+                                              uint8_t* __restrict__ heads_mem, const HeadsCall& call) {
+    constexpr uint32_t ALL = 0xFFFFFFFFu;
+    const uint32_t words = (T + 31u) / 32u, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const HeadsLayout L(T);
+    uint8_t* mem = heads_mem + warp * L.total;
+    uint16_t* latest_11 = reinterpret_cast<uint16_t*>(mem);
+    uint32_t* latest_7 = reinterpret_cast<uint32_t*>(mem + L.latest_7);
+    uint32_t* latest_3 = reinterpret_cast<uint32_t*>(mem + L.latest_3);
+    uint16_t* link = reinterpret_cast<uint16_t*>(mem + L.link);
+    uint32_t* Q = reinterpret_cast<uint32_t*>(mem + L.q);
+    uint32_t* K = reinterpret_cast<uint32_t*>(mem + L.k);
+    uint32_t* V = reinterpret_cast<uint32_t*>(mem + L.v);
+    if (warp >= call.warps) return;
+    const uint32_t pieces = call.pieces, warps = gridDim.x * call.warps, above = ALL << lane << 1, below = (1u << lane) - 1u;
+    const uint32_t piece_rows = (words + pieces - 1u) / pieces;
+    auto keys_in = [&](uint32_t row, uint32_t wk) {
+        const uint32_t r1 = 32u * row + lane + 1u, ctx = wk >> 21;
+        uint32_t before = latest_11[ctx];
+        atomicMax(&latest_7[wk >> 25], r1);
+        atomicMax(&latest_3[wk >> 29], r1);
+        __syncwarp();   // the tables have been read
+        latest_11[ctx] = (uint16_t)r1;
+        __syncwarp();
+        if (__any_sync(ALL, latest_11[ctx] != (uint16_t)r1)) {   // a context twice in the row: its last lane counts
+            const uint32_t same = __match_any_sync(ALL, ctx);
+            if (!(same & above)) latest_11[ctx] = (uint16_t)r1;
+            if (same & below) before = heads::latest(row, same & below);
+        }
+        link[r1] = (uint16_t)before;
+        __syncwarp();
+    };
+    // The last pieces first, which have the most keys to put in.
+    for (uint32_t item = warp * gridDim.x + blockIdx.x; item < total * pieces;
+         item = warps + __shfl_sync(ALL, lane == 0u ? atomicAdd(call.next, 1u) : 0u, 0)) {
+        const uint32_t piece = pieces - 1u - item / total;
+        const size_t s = list[item % total], at = s * wps;
+        const uint32_t row0 = min(piece * piece_rows, words), row1 = min(row0 + piece_rows, words);
+        __syncwarp();
+        for (uint32_t w = lane; w < row1; w += 32u) {
+            Q[w + 1u] = q_sw[at + w];
+            K[w + 1u] = k_sw[at + w];
+            V[w] = v_sw[at + w];
+        }
+        if (lane == 0u) Q[0] = K[0] = 0u;
+        for (uint32_t i = lane; i < L.link / 16u; i += 32u) reinterpret_cast<uint4*>(mem)[i] = uint4{0u, 0u, 0u, 0u};
+        __syncwarp();
+        uint32_t k0 = 0u, q0 = Q[row0], work = 0;
+        for (uint32_t row = 0; row < row0; ++row) {
+            const uint32_t k1 = K[row + 1u];
+            keys_in(row, __funnelshift_l(k0, k1, 31u - lane));
+            k0 = k1;
+        }
+        bool gone = false;
+        for (uint32_t row = row0; row < row1 && !gone; ++row) {
+            const uint32_t k1 = K[row + 1u], q1 = Q[row + 1u], t = 32u * row + lane;
+            const uint32_t wk = __funnelshift_l(k0, k1, 31u - lane), wq = __funnelshift_l(q0, q1, 31u - lane);
+            uint32_t found = heads::probe_11(latest_11, wq);
+            if (!found) found = heads::probe(latest_7, wq, 7u);
+            if (!found) found = heads::probe(latest_3, wq, 3u);
+            const uint32_t in_row = row ? heads::agreeing<false>(k0, k1, below, wq) : heads::agreeing<true>(k0, k1, below, wq);
+            k0 = k1;
+            q0 = q1;
+            __syncwarp();
+            keys_in(row, wk);
+            // the latest lane of those that agree longest, and in how many bits
+            const uint32_t near = heads::latest(row, in_row), near_key = __shfl_sync(ALL, wk, (near - 1u) & 31u);
+            const uint32_t near_bits = min(min(context::leading(wq ^ near_key), heads::DEPTH), near);
+            if (in_row && near_bits >= found >> 16) found = near_bits << 16 | near;
+            const uint32_t most = call.base + call.per_row * (row - row0) - work;   // not below 0: the stream would be gone
+            uint32_t r1 = found & 0xFFFFu, best = 0, walked = 0, p = found >> 16 == heads::DEPTH && t < T ? r1 : 0u;
+            while (p && walked <= most) {
+                uint32_t n = min(context::leading(wq ^ heads::window_before(K, p)), p);
+                if (n == 32u) n = context::agreement(Q, K, t, p - 1u, 0u, walked);
+                if (n > best) {
+                    best = n;
+                    r1 = p;
+                }
+                p = link[p];
+                ++walked;
+            }
+            walked = __reduce_max_sync(ALL, walked);
+            work += walked;
+            gone = walked > most;
+            const uint32_t word = __ballot_sync(ALL, r1 && t < T && (V[r1 >> 5] >> (r1 & 31u) & 1u));
+            if (lane == 0u) idx_sw[at + row] = word;
+        }
+        if (gone && lane == 0u && atomicExch(&call.given_up[s], 1u) == 0u) call.left[atomicAdd(call.left_count, 1u)] = (uint32_t)s;
+    }
+}
+
 // TOGETHER: large buckets by a whole warp, one step after the other, and one bit more for the streams that are not easy (a stream
 // at a time: default model with gain N(0, 0.02), contexts of 64 sequences 7.49 -> 6.97 ms, of one at 1000 steps 0.65 -> 0.54; with
 // the bit for every stream of a launch even ones paid, 148 of 2048 steps 26 -> 34 us, of 4096 41 -> 55).  Runs where the
-// number of listed streams is in [from, to); with `left` for that list where there are more.
-template <int NT, bool TOGETHER>
+// number of listed streams is in [from, to).
+// FORM: IN_PARTS costs the other calls 3 % of the kernel.  LATEST_TOO, where more streams are listed, answers them by the latest positions
+// in the same launch: as a launch before this one, which leaves at once where few are listed, it took those calls 6 us per layer.
+enum ContextForm { PLAIN, IN_PARTS, LATEST_TOO };
+template <int NT, bool TOGETHER, int FORM = PLAIN>
 __global__ void __launch_bounds__(NT, NT > 512 ? 1 : NT > 256 ? 2 : 5)
 rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restrict__ k_sw, const uint32_t* __restrict__ v_sw,
                     uint32_t* __restrict__ idx_sw, const uint32_t* __restrict__ list, const uint32_t* __restrict__ count,
-                    const uint32_t* __restrict__ left, const uint32_t* __restrict__ left_count, uint32_t* __restrict__ next,
-                    uint32_t* __restrict__ hard, uint32_t* __restrict__ hard_count, uint32_t T, size_t wps, uint32_t easy_bits,
-                    ContextLimits limits, uint32_t from, uint32_t to) {
+                    uint32_t* __restrict__ next, uint32_t* __restrict__ hard, uint32_t* __restrict__ hard_count, uint32_t T,
+                    size_t wps, uint32_t easy_bits, ContextLimits limits, uint32_t from, uint32_t to, HeadsCall heads_call) {
     chain_entry();
     constexpr uint32_t NW = NT / 32, BRUTE = context::BRUTE;
     extern __shared__ __align__(16) uint8_t context_mem[];
@@ -396,6 +529,7 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
     uint32_t* start2 = reinterpret_cast<uint32_t*>(context_mem + L.start);
     uint32_t* Q = reinterpret_cast<uint32_t*>(context_mem + L.q);
     uint32_t* K = reinterpret_cast<uint32_t*>(context_mem + L.k);
+    uint32_t* V = reinterpret_cast<uint32_t*>(context_mem + L.v);
     uint16_t* q_ends = reinterpret_cast<uint16_t*>(context_mem + L.q_ends);
     uint16_t* k_ends = reinterpret_cast<uint16_t*>(context_mem + L.k_ends);
     uint16_t* in_word = reinterpret_cast<uint16_t*>(context_mem + L.in_word);
@@ -406,13 +540,13 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
     uint16_t* large_steps = hist;   // after the sort; NW * C > T entries for the 16 warps of TOGETHER
     const context::Runs runs{k_ends, in_word, before_word};
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    uint32_t total = *count;
-    if (left && total >= to) {
-        list = left;
-        total = *left_count;
-    } else if (total < from || total >= to) {
+    const uint32_t total = *count;
+    if (FORM == LATEST_TOO && total >= to) {
+        heads_streams(q_sw, k_sw, v_sw, idx_sw, list, total, T, wps, context_mem, heads_call);
         return;
     }
+    if (total < from || total >= to) return;
+    const uint32_t parts = FORM == IN_PARTS && total ? min(max(gridDim.x / total, 1u), MAX_PARTS) : 1u;
     const uint32_t rows_per_warp = (words + NW - 1u) / NW;
     const uint32_t row0 = min(warp * rows_per_warp, words), row1 = min(row0 + rows_per_warp, words);   // a warp's keys
     for (;;) {
@@ -423,11 +557,15 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
             sh_large = 0u;
         }
         __syncthreads();
-        if (sh_item >= total) return;
-        const size_t s = list[sh_item];
+        if (sh_item >= total * parts) return;
+        // Every parts-th row of 32 steps is this part's own: it sorts for itself, in an order of its own within a bucket.
+        const uint32_t part = FORM == IN_PARTS ? sh_item / total : 0u;
+        const auto own_row = [&](uint32_t row) { return parts == 1u || row % parts == part; };
+        const size_t s = list[FORM == IN_PARTS ? sh_item % total : sh_item];
         for (uint32_t w = threadIdx.x; w < words; w += NT) {
             Q[w + 1u] = q_sw[s * wps + w];
             K[w + 1u] = k_sw[s * wps + w];
+            if (TOGETHER) V[w] = v_sw[s * wps + w];
             out_s[w] = 0u;
         }
         if (threadIdx.x == 0) Q[0] = K[0] = 0u;
@@ -455,7 +593,7 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
                 if (r < T) {
                     const uint32_t ck = key_of_key(r);
                     atomicAdd(&hist2[warp * pair_words + (ck >> 1)], 1u << ((ck & 1u) * 16u));
-                    if (r >= BRUTE) {
+                    if (r >= BRUTE && own_row(row)) {
                         const uint32_t cq = key_of_step(r);
                         atomicAdd(&nq2[cq >> 1], 1u << ((cq & 1u) * 16u));
                     }
@@ -493,6 +631,7 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
                 if (w < warp) run += sh_sums[w];
                 pairs += sh_pairs[w];
             }
+            pairs *= parts;   // about what all of them have
             // By bits when that is easy; otherwise by whichever of the two ways has fewer pairs, if those are few enough.
             if (attempt == 0) {
                 taken = pairs <= limits.easy * T;
@@ -535,8 +674,11 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
                 }
             }
         }
+        const auto leave = [&] {   // to rosa_match_kernel, by the first part that does
+            if (parts == 1u || atomicExch(&heads_call.given_up[s], 1u) == 0u) hard[atomicAdd(hard_count, 1u)] = (uint32_t)s;
+        };
         if (!taken) {
-            if (threadIdx.x == 0) hard[atomicAdd(hard_count, 1u)] = (uint32_t)s;
+            if (threadIdx.x == 0) leave();
             continue;
         }
         __syncthreads();
@@ -550,7 +692,7 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
             if (r < T) {
                 at = hist[warp * C + ck];
                 entries[at + rank] = context::Entry{context::window(K, r), r};
-                if (sorted && r >= BRUTE) {   // in any order within a bucket
+                if (sorted && r >= BRUTE && own_row(row)) {   // in any order within a bucket
                     const uint32_t cq = key_of_step(r), sh = (cq & 1u) * 16u;
                     steps[(atomicAdd(&nq2[cq >> 1], 1u << sh) >> sh) & 0xFFFFu] = (uint16_t)r;
                 }
@@ -589,7 +731,9 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
         __syncthreads();
         // Easy streams step by step.  On the others the number of positions to look at differs a lot from bucket to bucket:
         // their steps are taken bucket by bucket, so that the lanes of a warp look through the same ones.
-        const uint32_t* v = v_sw + s * wps;
+        // Many streams side by side hide the way to L1 and pay for the copy (four sequences 1.96 ms, with it 1.98); of few the slowest
+        // stream is what lasts (one 0.88, with it 0.85).
+        const uint32_t* v = TOGETHER ? V : v_sw + s * wps;
         uint32_t* out = idx_sw + s * wps;
         uint32_t deep = 0;
         const uint32_t most_deep = by_runs ? limits.deep_by_runs : limits.deep_by_bits;
@@ -628,7 +772,7 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
             return true;
         };
         if (TOGETHER) {   // the steps below BRUTE by a warp each
-            for (uint32_t t = warp; t < min(BRUTE, T); t += NW) {
+            for (uint32_t t = part * NW + warp; t < min(BRUTE, T); t += parts * NW) {
                 const uint32_t wq = context::window(Q, t);
                 uint32_t best = 0;
                 for (uint32_t r = lane; r < t; r += 32u) {
@@ -641,14 +785,24 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
         }
         // The last rows first: they have the most keys to agree with, so a stream that has to be given up is at once.
         const uint32_t first_row = min(TOGETHER ? BRUTE / 32u : 0u, words);
-        const uint32_t next_row = sorted ? NW : 0u - NW;
-        for (uint32_t row = sorted ? first_row + warp : words - 1u - warp; row - first_row < words - first_row; row += next_row) {
-            const uint32_t i = row * 32u + lane, t = sorted && i >= BRUTE && i < T ? steps[i - BRUTE] : i;
+        // The rows of this part (each may sort or not, by its own count of pairs), the sorted steps of which are in `steps`.
+        const int32_t last_own = (int32_t)(words - 1u) - (int32_t)((words - 1u + parts - part) % parts);
+        uint32_t n_rows = last_own >= (int32_t)first_row ? ((uint32_t)last_own - first_row) / parts + 1u : 0u, own_steps = 0;
+        if (sorted) {
+            if (last_own >= (int32_t)(BRUTE / 32u)) {
+                own_steps = (((uint32_t)last_own - BRUTE / 32u) / parts + 1u) * 32u;
+                if ((uint32_t)last_own == words - 1u) own_steps -= 32u * words - T;
+            }
+            n_rows = min(BRUTE / 32u, words) - first_row + (own_steps + 31u) / 32u;
+        }
+        for (uint32_t j = warp; j < n_rows; j += NW) {
+            const uint32_t row = sorted ? first_row + j : (uint32_t)last_own - j * parts;
+            const uint32_t i = row * 32u + lane, t = !sorted || i < BRUTE ? i : i - BRUTE < own_steps ? steps[i - BRUTE] : T;
             uint32_t r1 = 0;
             bool large = false;
             if (row * 32u < BRUTE) {
-                if (i < T) r1 = context::find_brute(Q, K, t, deep);
-            } else if (i < T) {
+                if (t < T) r1 = context::find_brute(Q, K, t, deep);
+            } else if (t < T) {
                 const Step x = find_bucket(t);
                 large = TOGETHER && (x.e - x.b) * t > CONTEXT_LARGE * T;   // about so many of them lie before t
                 if (!large) {
@@ -704,136 +858,13 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
         }
         __syncthreads();
         if (sh_gone) {
-            if (threadIdx.x == 0) hard[atomicAdd(hard_count, 1u)] = (uint32_t)s;
+            if (threadIdx.x == 0) leave();
+        } else if (parts > 1u) {
+            for (uint32_t w = threadIdx.x; w < words; w += NT)
+                if (out_s[w]) atomicOr(&out[w], out_s[w]);
         } else if (sorted || TOGETHER) {
             for (uint32_t w = threadIdx.x; w < words; w += NT) out[w] = out_s[w];
         }
-    }
-}
-
-// The streams whose keys are spread evenly (rosa_heads.cuh).  A stream is cut into `pieces`, a warp takes one: it puts the keys
-// of the rows before into tables of its own and goes on from there.  The other streams go to `left`, once: a stream is given up
-// as soon as the walks of a piece, the longest of each row, have come to more than `base` + `per_row` positions per row so far, 32
-// steps beyond the first window counted as a position.  given_up: a word per stream, zero before.
-// Warps per CTA: they have nothing to do with one another, but at 2048 steps two CTAs of 12 leave less shared memory idle than five of
-// four (20 warps per SM, not 24: 16 sequences in all layers 3.85 / 3.56 ms; 8 times 300 steps 0.39 / 0.42).
-constexpr int HEAD_WARPS = 12;
-
-struct HeadsLayout {   // bytes of shared memory of a warp
-    uint32_t latest_7, latest_3, link, q, k, v, total;   // latest_11 is at 0
-    __host__ __device__ explicit HeadsLayout(uint32_t T) {
-        const uint32_t words = (T + 31u) / 32u;
-        latest_7 = heads::LATEST_11 * 2u;
-        latest_3 = latest_7 + heads::LATEST_7 * 4u;
-        link = latest_3 + heads::LATEST_3 * 4u;   // u16 [32 * words + 2]: by position + 1, the latest one before it with its context
-        q = link + (32u * words + 2u) * 2u;       // u32 [words + 1]
-        k = q + (words + 1u) * 4u;
-        v = k + (words + 1u) * 4u;                // u32 [words]
-        total = (v + words * 4u + 15u) & ~15u;
-    }
-};
-
-struct HeadsLimits {
-    uint32_t base, per_row;
-};
-
-// Bound by the integer pipe: per row of 32 steps of the model's streams (2048 steps) about 350 warp instructions, 215 of them on
-// that pipe, which takes one every second cycle - the refinement of the masks 100, the look-ups 70, the walk over the
-// chains 70, the keys 40.  rosa_context_kernel sorts each stream first and compares what lies in a bucket: 750 per row.  Both kernels
-// in all layers, gain 1 + N(0, 0.02), contexts alone before: default model 64 times 2048 steps 21.5 -> 12.8 ms, 16 5.8 -> 4.3, 8 3.2 -> 2.6,
-// 64 times 512 6.5 -> 2.7, 16 times 700 2.4 -> 1.3.
-__global__ void __launch_bounds__(32 * HEAD_WARPS)
-rosa_heads_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restrict__ k_sw, const uint32_t* __restrict__ v_sw,
-                  uint32_t* __restrict__ idx_sw, const uint32_t* __restrict__ list, const uint32_t* __restrict__ count,
-                  uint32_t* __restrict__ next, uint32_t* __restrict__ left, uint32_t* __restrict__ left_count,
-                  uint32_t* __restrict__ given_up, uint32_t T, size_t wps, uint32_t pieces, uint32_t from, HeadsLimits limits) {
-    chain_entry();
-    constexpr uint32_t ALL = 0xFFFFFFFFu;
-    extern __shared__ __align__(16) uint8_t heads_mem[];
-    const uint32_t words = (T + 31u) / 32u, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const HeadsLayout L(T);
-    uint8_t* mem = heads_mem + warp * L.total;
-    uint16_t* latest_11 = reinterpret_cast<uint16_t*>(mem);
-    uint32_t* latest_7 = reinterpret_cast<uint32_t*>(mem + L.latest_7);
-    uint32_t* latest_3 = reinterpret_cast<uint32_t*>(mem + L.latest_3);
-    uint16_t* link = reinterpret_cast<uint16_t*>(mem + L.link);
-    uint32_t* Q = reinterpret_cast<uint32_t*>(mem + L.q);
-    uint32_t* K = reinterpret_cast<uint32_t*>(mem + L.k);
-    uint32_t* V = reinterpret_cast<uint32_t*>(mem + L.v);
-    const uint32_t total = *count >= from ? *count : 0u, warps = gridDim.x * HEAD_WARPS, above = ALL << lane << 1, below = (1u << lane) - 1u;
-    const uint32_t piece_rows = (words + pieces - 1u) / pieces;
-    auto keys_in = [&](uint32_t row, uint32_t wk) {
-        const uint32_t r1 = 32u * row + lane + 1u, ctx = wk >> 21;
-        uint32_t before = latest_11[ctx];
-        atomicMax(&latest_7[wk >> 25], r1);
-        atomicMax(&latest_3[wk >> 29], r1);
-        __syncwarp();   // the tables have been read
-        latest_11[ctx] = (uint16_t)r1;
-        __syncwarp();
-        if (__any_sync(ALL, latest_11[ctx] != (uint16_t)r1)) {   // a context twice in the row: its last lane counts
-            const uint32_t same = __match_any_sync(ALL, ctx);
-            if (!(same & above)) latest_11[ctx] = (uint16_t)r1;
-            if (same & below) before = heads::latest(row, same & below);
-        }
-        link[r1] = (uint16_t)before;
-        __syncwarp();
-    };
-    // The last pieces first, which have the most keys to put in.
-    for (uint32_t item = warp * gridDim.x + blockIdx.x; item < total * pieces;
-         item = warps + __shfl_sync(ALL, lane == 0u ? atomicAdd(next, 1u) : 0u, 0)) {
-        const uint32_t piece = pieces - 1u - item / total;
-        const size_t s = list[item % total], at = s * wps;
-        const uint32_t row0 = min(piece * piece_rows, words), row1 = min(row0 + piece_rows, words);
-        __syncwarp();
-        for (uint32_t w = lane; w < row1; w += 32u) {
-            Q[w + 1u] = q_sw[at + w];
-            K[w + 1u] = k_sw[at + w];
-            V[w] = v_sw[at + w];
-        }
-        if (lane == 0u) Q[0] = K[0] = 0u;
-        for (uint32_t i = lane; i < L.link / 16u; i += 32u) reinterpret_cast<uint4*>(mem)[i] = uint4{0u, 0u, 0u, 0u};
-        __syncwarp();
-        uint32_t k0 = 0u, q0 = Q[row0], work = 0;
-        for (uint32_t row = 0; row < row0; ++row) {
-            const uint32_t k1 = K[row + 1u];
-            keys_in(row, __funnelshift_l(k0, k1, 31u - lane));
-            k0 = k1;
-        }
-        bool gone = false;
-        for (uint32_t row = row0; row < row1 && !gone; ++row) {
-            const uint32_t k1 = K[row + 1u], q1 = Q[row + 1u], t = 32u * row + lane;
-            const uint32_t wk = __funnelshift_l(k0, k1, 31u - lane), wq = __funnelshift_l(q0, q1, 31u - lane);
-            uint32_t found = heads::probe_11(latest_11, wq);
-            if (!found) found = heads::probe(latest_7, wq, 7u);
-            if (!found) found = heads::probe(latest_3, wq, 3u);
-            const uint32_t in_row = row ? heads::agreeing<false>(k0, k1, below, wq) : heads::agreeing<true>(k0, k1, below, wq);
-            k0 = k1;
-            q0 = q1;
-            __syncwarp();
-            keys_in(row, wk);
-            // the latest lane of those that agree longest, and in how many bits
-            const uint32_t near = heads::latest(row, in_row), near_key = __shfl_sync(ALL, wk, (near - 1u) & 31u);
-            const uint32_t near_bits = min(min(context::leading(wq ^ near_key), heads::DEPTH), near);
-            if (in_row && near_bits >= found >> 16) found = near_bits << 16 | near;
-            const uint32_t most = limits.base + limits.per_row * (row - row0) - work;   // not below 0: the stream would be gone
-            uint32_t r1 = found & 0xFFFFu, best = 0, walked = 0, p = found >> 16 == heads::DEPTH && t < T ? r1 : 0u;
-            while (p && walked <= most) {
-                uint32_t n = min(context::leading(wq ^ heads::window_before(K, p)), p);
-                if (n == 32u) n = context::agreement(Q, K, t, p - 1u, 0u, walked);
-                if (n > best) {
-                    best = n;
-                    r1 = p;
-                }
-                p = link[p];
-                ++walked;
-            }
-            walked = __reduce_max_sync(ALL, walked);
-            work += walked;
-            gone = walked > most;
-            const uint32_t word = __ballot_sync(ALL, r1 && t < T && (V[r1 >> 5] >> (r1 & 31u) & 1u));
-            if (lane == 0u) idx_sw[at + row] = word;
-        }
-        if (gone && lane == 0u && atomicExch(&given_up[s], 1u) == 0u) left[atomicAdd(left_count, 1u)] = (uint32_t)s;
     }
 }
 
@@ -926,6 +957,7 @@ rosa_match_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restrict_
 
 constexpr size_t MATCH_MAX_TIME = 8192;   // 256 words of lags, eight per lane
 constexpr uint32_t HEADS_MAX_TIME = 2048;
+constexpr size_t SM_SMEM = 228 * 1024, CTA_SMEM = 1536;   // of an SM; what a CTA needs beside its dynamic part, reserved and static
 
 struct MatchCall {   // the buffers of one call
     const uint32_t *q, *k, *v;
@@ -935,6 +967,7 @@ struct MatchCall {   // the buffers of one call
     uint32_t *counts, *clear;
     size_t streams, wps;
     uint32_t T;
+    ContextForm form;
 };
 
 // The shapes of the context kernel: threads per stream, and whether a warp takes a large bucket together.
@@ -947,6 +980,9 @@ void prepare_context(ullis_cuda_runtime* rt, uint32_t T, int shape) {
     if (!rt->context_smem[shape]) {   // the attribute belongs to the function, not to this runtime: always the same value
         const size_t most = ContextLayout((uint32_t)MATCH_MAX_TIME, context::bits_for((uint32_t)MATCH_MAX_TIME), NT / 32).total;
         ULLIS_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+        if constexpr (TOGETHER)
+            ULLIS_CUDA_CHECK(cudaFuncSetAttribute(rosa_context_kernel<NT, TOGETHER, IN_PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+        ULLIS_CUDA_CHECK(cudaFuncSetAttribute(rosa_context_kernel<NT, TOGETHER, LATEST_TOO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SM_SMEM - CTA_SMEM)));
     }
     if (rt->context_smem[shape] != smem) {
         int per_sm = 0;
@@ -957,7 +993,8 @@ void prepare_context(ullis_cuda_runtime* rt, uint32_t T, int shape) {
 }
 
 template <int NT, bool TOGETHER>
-void launch_context(ullis_cuda_runtime* rt, const MatchCall& m, int shape, const uint32_t* left, uint32_t from, uint32_t to, const char* what) {
+void launch_context(ullis_cuda_runtime* rt, const MatchCall& m, int shape, ContextForm form, const uint32_t* list, const uint32_t* count, uint32_t from,
+                    uint32_t to, const char* what) {
     const unsigned grid = (unsigned)std::min<size_t>(rt->context_ctas[shape], m.streams);
     // A match kernel step costs about as much as 100 positions here; up to 24 the lanes are even enough without sorting
     // the steps.  What a thread has compared when its stream turns out to repeat itself is thrown away: by bits 64 long
@@ -965,38 +1002,32 @@ void launch_context(ullis_cuda_runtime* rt, const MatchCall& m, int shape, const
     // 256, now 0.13 / 0.67), by runs 256 (with 64, 64 sequences of the default model 33.3 ms, not 29.8: streams that hardly
     // ever change went to the match kernel).
     const ContextLimits limits{24u, 96u, 160u, 64u, 256u};
-    rt->chain(rosa_context_kernel<NT, TOGETHER>, grid, NT, rt->context_smem[shape], m.q, m.k, m.v, m.idx, m.list, m.counts,
-              left, m.counts + 5, m.counts + 3, m.hard, m.counts + 2, m.T, m.wps, context::bits_for(m.T), limits, from, to);
+    size_t smem = rt->context_smem[shape];
+    HeadsCall heads{0u, 1u, 128u, 24u, m.counts + 6, m.left, m.counts + 5, m.given_up};
+    auto kernel = rosa_context_kernel<NT, TOGETHER>;
+    if (form == LATEST_TOO) {
+        kernel = rosa_context_kernel<NT, TOGETHER, LATEST_TOO>;
+        // As many warps as have room beside each other with the CTAs that an SM holds anyway (2048 steps: 23 with 1024 threads, 22 with 512, 20
+        // with 256).
+        const size_t per_sm = (size_t)rt->context_ctas[shape] / rt->sm_count, each = HeadsLayout(m.T).total;
+        heads.warps = (uint32_t)std::min<size_t>(NT / 32, (SM_SMEM / per_sm - CTA_SMEM) / each);
+        smem = std::max(smem, heads.warps * each);
+        // More pieces make a launch of few streams shorter and one of many longer, since their warps put in the same keys again.  Below
+        // 1024 steps a piece costs more than it saves unless warps would be idle (gain 1 + N(0, 0.02), ROSA kernels in all layers with 20
+        // warps per SM, 1 / 2 / 4 pieces: 16 times 700 steps of the default model 1.51 / 1.66 / 1.81 ms, 3 times 333 of the small one 0.255 /
+        // 0.235 / 0.236; 2048 steps of the default model: 4 sequences 2.90 / 2.45 / 2.10, 8 3.71 / 3.11 / 2.99, 16 5.09 / 4.75 / 4.97, 64 14.0 /
+        // 14.4 / 16.7).
+        const size_t warps = (size_t)rt->context_ctas[shape] * heads.warps;
+        heads.pieces = m.T < 1024u ? (m.streams * 4u <= warps ? 4u : 1u) : m.streams * 2u < 3u * warps ? 4u : m.streams < 8u * warps ? 2u : 1u;
+        // heads.base, heads.per_row: a row whose walks are 29 positions long takes as many instructions as by contexts.  Less than 16 leaves
+        // them streams that are cheaper here (8 times 2048 steps 12 / 16 / 24 / 32 per row 3.12 / 3.03 / 2.94 / 2.95 ms, 16 times 1100 2.43 /
+        // 2.46 / 2.44 / 2.41), and a base too small all that are short (twice 700 steps, base 32 / 64 / 128: 0.75 / 0.62 / 0.61).
+    } else if constexpr (TOGETHER) {
+        if (form == IN_PARTS) kernel = rosa_context_kernel<NT, TOGETHER, IN_PARTS>;
+    }
+    rt->chain(kernel, grid, NT, smem, m.q, m.k, m.v, m.idx, list, count, m.counts + 3, m.hard, m.counts + 2, m.T, m.wps, context::bits_for(m.T), limits,
+              from, to, heads);
     rt->launched(what);
-}
-
-// Where at least `from` streams are listed.
-void launch_heads(ullis_cuda_runtime* rt, const MatchCall& m, uint32_t from) {
-    const size_t smem = (size_t)HeadsLayout(m.T).total * HEAD_WARPS;
-    if (!rt->heads_smem) {
-        const size_t most = (size_t)HeadsLayout(HEADS_MAX_TIME).total * HEAD_WARPS;
-        ULLIS_CUDA_CHECK(cudaFuncSetAttribute(rosa_heads_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
-    }
-    if (rt->heads_smem != smem) {
-        int per_sm = 0;
-        ULLIS_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rosa_heads_kernel, 32 * HEAD_WARPS, smem));
-        rt->heads_ctas = std::max(1, per_sm) * rt->sm_count;
-        rt->heads_smem = smem;
-    }
-    const size_t warps = (size_t)rt->heads_ctas * HEAD_WARPS;
-    // More pieces make a launch of few streams shorter and one of many longer, since their warps put in the same keys again.  Below
-    // 1024 steps a piece costs more than it saves unless warps would be idle (gain 1 + N(0, 0.02), ROSA kernels in all layers with four
-    // warps per CTA, 1 / 2 / 4 pieces: 16 times 700 steps of the default model 1.51 / 1.66 / 1.81 ms, 3 times 333 of the small one 0.255 / 0.235 /
-    // 0.236; 2048 steps of the default model: 4 sequences 2.90 / 2.45 / 2.10, 8 3.71 / 3.11 / 2.99, 16 5.09 / 4.75 / 4.97, 64 14.0 / 14.4 / 16.7).
-    const uint32_t pieces = m.T < 1024u ? (m.streams * 4u <= warps ? 4u : 1u) : m.streams * 2u < 3u * warps ? 4u : m.streams < 8u * warps ? 2u : 1u;
-    const unsigned grid = (unsigned)std::min<size_t>(rt->heads_ctas, (m.streams * pieces + HEAD_WARPS - 1) / HEAD_WARPS);
-    // A row whose walks are 29 positions long takes as many instructions as in rosa_context_kernel.  Less than 16 leaves it streams that
-    // are cheaper here (8 times 2048 steps 12 / 16 / 24 / 32 per row 3.12 / 3.03 / 2.94 / 2.95 ms, 16 times 1100 2.43 / 2.46 / 2.44 / 2.41),
-    // and a base too small all that are short (twice 700 steps, base 32 / 64 / 128: 0.75 / 0.62 / 0.61).
-    const HeadsLimits limits{128u, 24u};
-    rt->chain(rosa_heads_kernel, grid, 32 * HEAD_WARPS, smem, m.q, m.k, m.v, m.idx, m.list, m.counts, m.counts + 6, m.left, m.counts + 5,
-              m.given_up, m.T, m.wps, pieces, from, limits);
-    rt->launched("rosa_heads");
 }
 
 template <int NW>
@@ -1080,22 +1111,32 @@ void contexts(ullis_cuda_runtime* rt, const MatchCall& m) {
         uneven = std::max<int>(many, m.T >= 1024u && m.streams * 50u <= m.T * sms ? CONTEXT_1024 : CONTEXT_512);
         rest = std::max<int>(many, m.streams <= (m.T < 1024u ? 7u : 6u) * sms ? CONTEXT_512 : CONTEXT_256);
     }
+    const uint32_t all = ~0u, half = uneven == rest && m.form != LATEST_TOO ? all : (uint32_t)(m.streams / 2) + 1u;
+    auto launch = [&](int shape, ContextForm form, const uint32_t* list, const uint32_t* count, uint32_t from, uint32_t to, const char* what) {
+        if (shape == CONTEXT_256) launch_context<256, false>(rt, m, shape, form, list, count, from, to, what);
+        else if (shape == CONTEXT_512) launch_context<512, true>(rt, m, shape, form, list, count, from, to, what);
+        else launch_context<1024, true>(rt, m, shape, form, list, count, from, to, what);
+    };
+    if (m.form == LATEST_TOO) {
+        launch(uneven, m.form, m.list, m.counts, 0u, half, "rosa_heads");
+        launch(uneven, PLAIN, m.left, m.counts + 5, 1u, all, "rosa_context");
+        return;
+    }
+    launch(uneven, m.form, m.list, m.counts, 0u, half, "rosa_context");
+    if (half != all) launch(rest, PLAIN, m.list, m.counts, half, all, "rosa_context_even");
+}
+
+// How the listed streams of a call are to be answered.
+ContextForm context_form(const ullis_cuda_runtime* rt, size_t streams, uint32_t T) {
+    const size_t sms = (size_t)rt->sm_count;
     // The latest positions, where most streams are listed: one warp per stream or piece, so there have to be enough of them (all layers,
     // gain 1 + N(0, 0.02), contexts / latest positions, ms; 2048 steps: two sequences of the default model 1.57 / 1.73, three 1.83 / 1.93, four
     // 2.18 / 2.05, eight 3.49 / 2.82, 64 21.7 / 13.1; 1100 steps: two 1.01 / 1.06, four 1.39 / 1.25; 700: one 0.58 / 0.69, two 0.81 / 0.62, 16 2.57 / 1.49;
     // 300: two 0.51 / 0.45, 64 5.88 / 1.98).  Where few are listed those are uneven, and their chains long: 64 times 2048 steps with gain
     // N(0, 0.02) 7.7 / 9.3.  Beyond 2048 steps chains and tables grow (8192 steps of bits of probability 0.25 to 0.6: 1.09 / 1.63).
-    const bool by_heads = m.T <= HEADS_MAX_TIME && m.streams > (m.T < 512u ? 4u : m.T < 1024u ? 5u : 12u) * sms;
-    const uint32_t all = ~0u, half = uneven == rest && !by_heads ? all : (uint32_t)(m.streams / 2) + 1u;
-    auto launch = [&](int shape, uint32_t from, uint32_t to, const char* what) {
-        const uint32_t* left = by_heads ? m.left : nullptr;
-        if (shape == CONTEXT_256) launch_context<256, false>(rt, m, shape, left, from, to, what);
-        else if (shape == CONTEXT_512) launch_context<512, true>(rt, m, shape, left, from, to, what);
-        else launch_context<1024, true>(rt, m, shape, left, from, to, what);
-    };
-    if (by_heads) launch_heads(rt, m, half);
-    launch(uneven, 0u, half, "rosa_context");
-    if (!by_heads && half != all) launch(rest, half, all, "rosa_context_even");
+    if (T <= HEADS_MAX_TIME && streams > (T < 512u ? 4u : T < 1024u ? 5u : 14u) * sms) return LATEST_TOO;
+    // Only a call of few streams can list less than half as many as there are CTAs.
+    return streams <= PARTS_MAX_STREAMS * sms ? IN_PARTS : PLAIN;
 }
 
 // The whole call without an automaton: classification, the listed streams by contexts, and by sets of lags those that
@@ -1110,12 +1151,13 @@ void rosa_match(ullis_cuda_runtime* rt, const uint32_t* q_sw, const uint32_t* k_
     m.hard = m.cq_list + streams;
     m.left = m.hard + streams;
     m.given_up = m.left + streams;
+    m.form = context_form(rt, streams, T);
     rt->counters(rt->match_counters, MATCH_COUNTS, &m.counts, &m.clear);
     rt->sam_last_counts = m.counts;
     rt->sam_last_streams = streams;
     if (!rt->parent) rt->lanes_last = 1;
     rt->chain(rosa_classify_kernel, (unsigned)((streams * CLASSIFY_LANES + 127) / 128), 128, 0, q_sw, k_sw, v_sw, idx_sw,
-              streams, T, m.wps, m.list, m.counts, m.cq_list, m.counts + 1, m.given_up);
+              streams, T, m.wps, m.list, m.counts, m.cq_list, m.counts + 1, m.given_up, m.form == IN_PARTS);
     rt->launched("rosa_classify");
     contexts(rt, m);
     if (T <= 1024u) launch_match<1>(rt, m, 0, 1024);
@@ -1195,7 +1237,7 @@ void rosa_sam(ullis_cuda_runtime* rt, const uint32_t* q_sw, const uint32_t* k_sw
         rt->zero(count, 8);   // both counters
         const unsigned classify_grid = (unsigned)((streams * CLASSIFY_LANES + 127) / 128);
         rt->chain(rosa_classify_kernel, classify_grid, 128, 0, q_sw, k_sw, v_sw, idx_sw, streams, (uint32_t)time, wps, list,
-                                                             count, cq_list, cq_count, nullptr);
+                                                             count, cq_list, cq_count, nullptr, false);
         rt->launched("rosa_classify");
         // The constant-q scan is a long serial loop for a few thousand threads; it depends on nothing but the
         // classification and writes idx words no other kernel of this call touches, so it runs on the side stream
