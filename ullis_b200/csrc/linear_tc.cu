@@ -33,12 +33,12 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
     return fn;
 }
 
-// [rows, K] 16-bit row-major matrix, 64 x 128 boxes, 128-byte swizzle, zero fill
-CUtensorMap make_map(const void* ptr, size_t rows, size_t K, bool bf16) {
+// [rows, K] 16-bit row-major matrix, boxes of 64 columns x 128 rows (or fewer), 128-byte swizzle, zero fill
+CUtensorMap make_map(const void* ptr, size_t rows, size_t K, bool bf16, uint32_t box_rows = BM) {
     CUtensorMap m;
     cuuint64_t dims[2] = {K, rows};
     cuuint64_t strides[1] = {K * 2};
-    cuuint32_t box[2] = {BK, BM};
+    cuuint32_t box[2] = {BK, box_rows};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = encode_fn()(&m, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
                              const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -673,6 +673,16 @@ bool usable(ullis_cuda_runtime* rt) {
             ULLIS_SET_SMEM(EPI_RESIDUAL, true);
             ULLIS_SET_SMEM(EPI_RESIDUAL, false);
             ULLIS_SET_SMEM(EPI_RELU2, true);
+#define ULLIS_SET_SMEM_NARROW(EPI, PACKED)                                                                                      \
+    ULLIS_CUDA_CHECK(cudaFuncSetAttribute(gemm_kernel<EPI, PACKED, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));    \
+    ULLIS_CUDA_CHECK(cudaFuncSetAttribute(gemm_kernel<EPI, PACKED, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem))
+            ULLIS_SET_SMEM_NARROW(EPI_STORE, true);
+            ULLIS_SET_SMEM_NARROW(EPI_STORE, false);
+            ULLIS_SET_SMEM_NARROW(EPI_RESIDUAL, true);
+            ULLIS_SET_SMEM_NARROW(EPI_RESIDUAL, false);
+            ULLIS_SET_SMEM_NARROW(EPI_RELU2, true);
+            ULLIS_SET_SMEM_NARROW(EPI_SIGNBITS, true);
+#undef ULLIS_SET_SMEM_NARROW
             ULLIS_SET_SMEM(EPI_SIGNBITS, true);
             ULLIS_SET_SMEM(EPI_CE, true);
 #undef ULLIS_SET_SMEM
@@ -771,7 +781,7 @@ uint32_t stages_for(const ullis_cuda_runtime* rt, const GemmParams& p, size_t ct
     const size_t per_sm = (ctas + rt->sm_count - 1) / rt->sm_count;
     if (per_sm > 2) return p.stages;
     const size_t room = WS_SMEM_LIMIT / per_sm - 1024 * (per_sm - 1), fixed = gemm_smem_bytes(p.n_a, 0);
-    const uint32_t fit = (uint32_t)((room - fixed) / ((p.n_a + 1) * TILE_BYTES));
+    const uint32_t fit = (uint32_t)((room - fixed) / gemm_stage_bytes(p.n_a, p.columns));
     return std::max(p.stages, std::min({fit, (uint32_t)MAX_STAGES, p.K / BK}));
 }
 
@@ -786,11 +796,35 @@ bool takes_ws2_dense(const ullis_cuda_runtime* rt, const GemmParams& p, unsigned
            ws2_shape(p.K, p.n_a, EPI, false).stages >= 2;
 }
 
+// Columns of gemm_kernel's tiles for M x N outputs: as few as still leave no SM two tiles.  Narrow tiles read the activations more
+// often, from L2, but a launch of few rows lasts as long as one CTA: what it brings in (32 KB per k-block with 128 columns, 20 with 32),
+// its products and its epilogue.  us of a launch, with the brackets of events: 512 rows, value (K = 1024, 256 columns) 18 -> 14, O (K = 256)
+// 14 -> 10, key (1024 columns) 13 -> 10; 2048 rows of 512, value (K = 2048) 25 -> 21, O 17.5 -> 14.  Default model, one sequence 1975 ->
+// 1902 us, small model 546 -> 475.
+uint32_t tile_columns(const ullis_cuda_runtime* rt, size_t M, size_t N, size_t n_prob = 1) {
+    const auto tiles = [&](size_t columns) { return n_prob * ((M + BM - 1) / BM) * ((N + columns - 1) / columns); };
+    for (uint32_t columns : {32u, 64u})
+        if (tiles(columns) <= (size_t)rt->sm_count) return columns;
+    return BN;
+}
+
 template <int EPI, bool PACKED>
 void launch(ullis_cuda_runtime* rt, const GemmMaps& maps, const GemmParams& p, unsigned n_prob, const char* what) {
     if (PACKED && takes_ws2(rt, EPI, p.M, p.K, p.N, p.n_a)) {
         launch_ws2<EPI, true>(rt, maps, p, n_prob, rt->tc_ws2_clusters[EPI], what);
         return;
+    }
+    if constexpr (EPI != EPI_CE) {   // its partials are those of 128 columns
+        if (p.columns < BN) {
+            GemmParams q = p;
+            const dim3 grid((p.N + p.columns - 1) / p.columns, (p.M + BM - 1) / BM, n_prob);
+            q.stages = stages_for(rt, p, (size_t)grid.x * grid.y * grid.z);
+            const size_t smem = gemm_smem_bytes(q.n_a, q.stages, q.columns);
+            if (p.columns == 64) rt->chain(gemm_kernel<EPI, PACKED, 64>, grid, GEMM_THREADS, smem, maps, q);
+            else rt->chain(gemm_kernel<EPI, PACKED, 32>, grid, GEMM_THREADS, smem, maps, q);
+            rt->launched(what);
+            return;
+        }
     }
     if (PACKED && takes_ws(rt, p.K, p.n_a)) {
         // one (problem, column tile) pair per CTA, the CTAs of a pair share the row tiles
@@ -842,6 +876,7 @@ GemmParams base_params(ullis_cuda_runtime* rt, size_t M, size_t N, size_t K) {
     p.K = (uint32_t)K;
     p.n_a = 1;
     p.stages = rt->tc_stages;   // shallow pipeline, several CTAs per SM: one CTA's epilogue runs under another's MMAs
+    p.columns = BN;
     p.status = rt->dev_status;
     return p;
 }
@@ -918,6 +953,7 @@ bool binary_linear(ullis_cuda_runtime* rt, const float* x, const uint32_t* bits,
     maps.a[0][0] = make_map(a, rows, in_features, false);
     GemmParams p = base_params(rt, rows, out_features, in_features);
     p.prob[0] = GemmProblem{bits, scale, bias, y, nullptr, nullptr};
+    p.columns = tile_columns(rt, rows, out_features);
     launch<EPI_STORE, true>(rt, maps, p, 1, "gemm_packed_store");
     return true;
 }
@@ -932,8 +968,9 @@ bool fp16_linear(ullis_cuda_runtime* rt, const float* x, const uint16_t* w, floa
     GemmMaps maps;
     memset(&maps, 0, sizeof(maps));
     maps.a[0][0] = make_map(a, rows, in_features, false);
-    maps.b[0] = make_map(w, out_features, in_features, false);
     GemmParams p = base_params(rt, rows, out_features, in_features);
+    p.columns = tile_columns(rt, rows, out_features);
+    maps.b[0] = make_map(w, out_features, in_features, false, p.columns);
     p.prob[0] = GemmProblem{nullptr, nullptr, nullptr, y, nullptr, nullptr};
     launch<EPI_STORE, false>(rt, maps, p, 1, "gemm_dense_store");
     return true;
@@ -1064,6 +1101,8 @@ bool rosa_qkv_bits(ullis_cuda_runtime* rt, const float* ln3_out, const LayerWeig
     uint32_t* outs[3] = {q_sw, k_sw, v_sw};
     for (int z = 0; z < 3; ++z)
         p.prob[z] = GemmProblem{W[z]->bits, W[z]->scale, W[z]->bias, outs[z], flags + z * sw, s1 + z * prows};
+    // 64 columns no better than the kernel that keeps its weights (small model, 3 times 333 steps 457 us, so 444)
+    p.columns = tile_columns(rt, prows, d, 3) == 32 ? 32 : BN;
     launch<EPI_SIGNBITS, true>(rt, maps, p, 3, "gemm_qkv_signbits");
     // rows < 2^30, so both grids fit
     if (rt->tc_fix_blocks && fix_block_threads(d) <= FIXB_MAX_THREADS) {   // d % 64 == 0 (shape_ok)
@@ -1099,6 +1138,7 @@ bool rosa_out_residual(ullis_cuda_runtime* rt, const uint32_t* idx_sw, const Lay
     maps.a[0][0] = make_map(y16, rows, d, false);
     GemmParams p = base_params(rt, rows, d, d);
     p.prob[0] = GemmProblem{L.o.bits, L.o.scale, L.o.bias, x, nullptr, nullptr};
+    p.columns = tile_columns(rt, rows, d);
     launch<EPI_RESIDUAL, true>(rt, maps, p, 1, "gemm_o_residual");
     return true;
 }
@@ -1123,11 +1163,13 @@ bool cmix_residual(ullis_cuda_runtime* rt, const LayerWeights& L, float* x, size
     GemmParams p = base_params(rt, rows, ffn, d);
     p.out_fmt = 0;  // FP16: three more significant bits than bf16; the epilogue reports values past 65504
     p.prob[0] = GemmProblem{L.key.bits, L.key.scale, nullptr, k16, nullptr, nullptr};
+    p.columns = tile_columns(rt, rows, ffn);
     launch<EPI_RELU2, true>(rt, maps, p, 1, "gemm_key_relu2");
     memset(&maps, 0, sizeof(maps));
     maps.a[0][0] = make_map(k16, rows, ffn, false);
-    maps.b[0] = make_map(L.value, d, ffn, false);   // the FP16 weights as stored
     GemmParams pv = base_params(rt, rows, d, ffn);
+    pv.columns = tile_columns(rt, rows, d);
+    maps.b[0] = make_map(L.value, d, ffn, false, pv.columns);   // the FP16 weights as stored
     pv.prob[0] = GemmProblem{nullptr, nullptr, nullptr, x, nullptr, nullptr};
     launch<EPI_RESIDUAL, false>(rt, maps, pv, 1, "gemm_value_residual");
     return true;

@@ -8,7 +8,7 @@
 //    words into FP16 +/-1.0 rows written straight into the swizzled layout the
 //    MMA reads (reference weight order: bit o*K+i, LSB first, 1 => +1,
 //    src/model.rs:146-148) - or a dense FP16 [N,K] matrix loaded by TMA.
-//  * One CTA computes one 128x128 tile: warp 0 issues TMA, warp 1 owns TMEM and
+//  * One CTA computes one tile of 128 rows and 128 columns, or 64 or 32 of them: warp 0 issues TMA, warp 1 owns TMEM and
 //    issues the MMAs, warps 2-5 expand weight bits during the main loop and
 //    then run the epilogue, one TMEM lane (= output row) per thread.
 //  * Pipeline: STAGES shared-memory stages guarded by full/empty mbarriers;
@@ -78,12 +78,14 @@ struct GemmParams {
     const uint32_t* labels;  // EPI_CE
     uint32_t ignore_id;      // EPI_CE
     uint32_t n_tiles;        // EPI_CE: (max, sum exp) partials per row: one per vocabulary tile and epilogue warp group
+    uint32_t columns;        // of a tile of gemm_kernel: BN, or 64 or 32 (not EPI_CE)
     uint32_t split_k;        // > 1 (dense weights, one problem): a share of the grid owns a K range and writes its own [M,N] partial
     uint32_t* status;
 };
 
-inline size_t gemm_smem_bytes(uint32_t n_a, uint32_t stages) {
-    return 1024 /*alignment slack*/ + (size_t)stages * (n_a + 1) * TILE_BYTES + 256 * 16 /*LUT*/ + 2 * BN * 4 + 256;
+inline size_t gemm_stage_bytes(uint32_t n_a, uint32_t columns) { return (size_t)n_a * TILE_BYTES + columns * BK * 2; }
+inline size_t gemm_smem_bytes(uint32_t n_a, uint32_t stages, uint32_t columns = BN) {
+    return 1024 /*alignment slack*/ + stages * gemm_stage_bytes(n_a, columns) + 256 * 16 /*LUT*/ + 2 * BN * 4 + 256;
 }
 
 __device__ __forceinline__ float h2f_bits(uint16_t b) { return __half2float(__ushort_as_half(b)); }
@@ -395,12 +397,15 @@ __device__ __forceinline__ void epilogue(const GemmParams& p, const GemmProblem&
         static_cast<float2*>(pr.out)[(size_t)m * p.n_tiles + part] = make_float2(run_max, run_sum);
 }
 
-template <int EPI, bool PACKED>
+// COLUMNS: of the tile.  With few rows 128 leave most SMs idle, and a CTA is bound by what it brings in and by its epilogue; an
+// output's terms are added up in the same order whatever the tile.
+template <int EPI, bool PACKED, int COLUMNS = BN>
 __global__ void __launch_bounds__(GEMM_THREADS, 3)
 gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const uint32_t stage_bytes = (p.n_a + 1) * TILE_BYTES;
+    constexpr uint32_t B_BYTES = COLUMNS * BK * 2;
+    const uint32_t stage_bytes = p.n_a * TILE_BYTES + B_BYTES;
     const uint32_t STAGES = p.stages;
     uint8_t* tiles = smem;
     uint4* lut = reinterpret_cast<uint4*>(smem + STAGES * stage_bytes);
@@ -417,7 +422,7 @@ gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t z = p.split_k > 1 ? 0u : blockIdx.z;
     GemmProblem pr = p.prob[z];
-    const uint32_t n0 = blockIdx.x * BN, m0 = blockIdx.y * BM;
+    const uint32_t n0 = blockIdx.x * COLUMNS, m0 = blockIdx.y * BM;
     uint32_t KB = p.K / BK, kb0 = 0;
     if (p.split_k > 1) {   // the host sizes the grid so that every split owns at least one k-block
         const uint32_t per = (KB + p.split_k - 1) / p.split_k;
@@ -452,13 +457,13 @@ gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p) {
         }
     }
     if (warp >= 2) {
-        const int c = threadIdx.x - 64;  // 0..127: column of the tile
+        const int c = (threadIdx.x - 64) % COLUMNS;  // column of the tile
         const uint32_t n = n0 + c;
         s_scale[c] = (pr.scale && n < p.N) ? h2f_bits(pr.scale[n]) : 1.0f;
         s_bias[c] = (pr.bias && n < p.N) ? h2f_bits(pr.bias[n]) : 0.0f;
     }
     if (warp == 1) {
-        ptx::tmem_alloc(tmem_slot, 128);
+        ptx::tmem_alloc(tmem_slot, COLUMNS);
         ptx::tmem_relinquish();
     }
     chain_entry();   // scale and bias are weights, which the kernel directly before never writes
@@ -470,7 +475,7 @@ gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p) {
     if (warp == 0) {
         // ------------------------------------------------------ TMA producer
         if (ptx::elect_one()) {
-            const uint32_t tx = (p.n_a + (PACKED ? 0 : 1)) * TILE_BYTES;
+            const uint32_t tx = p.n_a * TILE_BYTES + (PACKED ? 0 : B_BYTES);
             uint32_t issued = 0;
             for (uint32_t kb = 0; kb < KB; ++kb, ++issued) {
                 const uint32_t s = kb % STAGES;
@@ -491,7 +496,7 @@ gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p) {
     } else if (warp == 1) {
         // -------------------------------------------------------- MMA issuer
         if (ptx::elect_one()) {
-            const uint32_t idesc = ptx::idesc_f16(p.a_fmt, p.b_fmt, BM, BN);
+            const uint32_t idesc = ptx::idesc_f16(p.a_fmt, p.b_fmt, BM, COLUMNS);
             bool ok = true;
             for (uint32_t kb = 0; kb < KB && ok; ++kb) {
                 const uint32_t s = kb % STAGES, ph = (kb / STAGES) & 1u;
@@ -514,20 +519,24 @@ gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p) {
         }
     } else {
         // ------------------------------------- weight expansion, then epilogue
-        const int r = threadIdx.x - 64;  // tile row of W (0..127) now, output row later
+        const int r = threadIdx.x - 64;
         if (PACKED) {
-            const uint32_t n = n0 + r;
+            // (The first stages expanded before chain_entry, under the end of the kernel before: small model, one sequence 475 -> 488 us.)
+            constexpr int SHARE = 8 * COLUMNS / 128;   // 16-byte pieces of a row of W for a thread
+            const int row = r % COLUMNS, first = r / COLUMNS * SHARE;
+            const uint32_t n = n0 + row;
             const uint32_t* wrow = pr.bits + ((size_t)n * p.K >> 5);
             for (uint32_t kb = 0; kb < KB; ++kb) {
                 const uint32_t s = kb % STAGES;
                 if (kb >= STAGES && !ptx::mbar_wait(&empty[s], ((kb / STAGES) & 1u) ^ 1u)) { atomicExch(s_error, 3u); break; }
                 uint32_t w0 = 0, w1 = 0;
                 if (n < p.N) { w0 = wrow[kb * 2]; w1 = wrow[kb * 2 + 1]; }
-                uint8_t* dst = tiles + s * stage_bytes + p.n_a * TILE_BYTES + r * 128;
+                uint8_t* dst = tiles + s * stage_bytes + p.n_a * TILE_BYTES + row * 128;
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
+                for (int i = 0; i < SHARE; ++i) {
+                    const int j = first + i;
                     const uint32_t byte = ((j < 4 ? w0 : w1) >> (8 * (j & 3))) & 0xFFu;
-                    *reinterpret_cast<uint4*>(dst + ((j ^ (r & 7)) << 4)) = lut[byte];
+                    *reinterpret_cast<uint4*>(dst + ((j ^ (row & 7)) << 4)) = lut[byte];
                 }
                 ptx::fence_proxy_async_smem();  // generic-proxy stores -> visible to the MMA's async reads
                 ptx::mbar_arrive(&full_b[s]);
@@ -543,7 +552,7 @@ gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p) {
         if (waited && *s_error == 0) {
             const uint32_t taddr = tmem_base + ((quarter * 32) << 16);
             // the pipeline stages are dead once the accumulator is complete: their space stages the stores
-            epilogue<EPI>(p, pr, taddr, m, n0, s_scale, s_bias, lane, blockIdx.x, 0, BN / 32,
+            epilogue<EPI>(p, pr, taddr, m, n0, s_scale, s_bias, lane, blockIdx.x, 0, COLUMNS / 32,
                           reinterpret_cast<float*>(tiles + (warp - 2) * STAGE_BYTES));
         }
     }
@@ -551,7 +560,7 @@ gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p) {
     __syncthreads();
     if (warp == 1) {
         ptx::tc_fence_after_sync();
-        ptx::tmem_dealloc(tmem_base, 128);
+        ptx::tmem_dealloc(tmem_base, COLUMNS);
     }
     if (threadIdx.x == 0 && *s_error) {
         if (atomicCAS(p.status, ULLIS_DEV_OK, ULLIS_DEV_WAIT_TIMEOUT) == ULLIS_DEV_OK) p.status[1] = *s_error;
