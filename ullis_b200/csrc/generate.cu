@@ -197,9 +197,15 @@ void ullis_cuda_generate_state::prepare_one_kernel() {
     ullis_cuda_model* m = model;
     ullis_cuda_runtime* rt = m->rt;
     if (getenv("ULLIS_CUDA_GEN_UNFUSED") || getenv("ULLIS_CUDA_NO_GRAPH") || m->d % 32 || m->ffn % gen::PIECE || rt->cc_major < 9) return;
-    auto kernel_for = [](uint32_t g) {
-        return g == 1 ? reinterpret_cast<const void*>(gen::gen_step_kernel<1>)
-               : g == 2 ? reinterpret_cast<const void*>(gen::gen_step_kernel<2>) : reinterpret_cast<const void*>(gen::gen_step_kernel<4>);
+    auto kernel_for = [](uint32_t g, uint32_t own) {
+        const gen::StepShape shape = gen::step_shape(g, own);
+        if (g == 1) return reinterpret_cast<const void*>(gen::gen_step_kernel<1, gen::PLAIN>);
+#define ULLIS_STEP_OF(G)                                                                                     \
+    (shape == gen::BY_ROW ? reinterpret_cast<const void*>(gen::gen_step_kernel<G, gen::BY_ROW>)              \
+     : shape == gen::WIDE ? reinterpret_cast<const void*>(gen::gen_step_kernel<G, gen::WIDE>)                \
+                          : reinterpret_cast<const void*>(gen::gen_step_kernel<G, gen::PLAIN>))
+        return g == 2 ? ULLIS_STEP_OF(2) : ULLIS_STEP_OF(4);
+#undef ULLIS_STEP_OF
     };
     // One round of clusters if there is a way, with as many CTAs per cluster as have 32 channels each (a CTA's share of the
     // sums is shortest then) and as few sequences per cluster as the clusters that the device holds at once allow.
@@ -217,7 +223,7 @@ void ullis_cuda_generate_state::prepare_one_kernel() {
             }
             const size_t smem = gen::Layout(g, (uint32_t)m->d, (uint32_t)m->ffn, c, stages, staged).total, want = (batch + g - 1) / g;
             if (smem > MOST_SMEM || stages > gen::MAX_STAGES) break;
-            const void* kernel = kernel_for(g);
+            const void* kernel = kernel_for(g, (uint32_t)m->d / c);
             ULLIS_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MOST_SMEM));
             ULLIS_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
             cudaLaunchAttribute attr;

@@ -34,6 +34,8 @@
 #include <cuda_fp16.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "common.hpp"
 #include "gen_push.cuh"
 #include "tc_ptx.cuh"
@@ -584,8 +586,16 @@ __device__ __forceinline__ void value_piece(float (&sum)[N], const uint8_t* piec
     }
 }
 
-// G: sequences of a cluster.
-template <int G>
+// G: sequences of a cluster.  The shape follows from G and the channels of a CTA; it is the kernel's, since code that one shape does not
+// need costs it instruction cache (32 sequences: 579 us per step, 590 with the others' in between).
+//   BY_ROW: D has a warp per row and tile of outputs where that leaves no scheduler two of them, rather than two rows at once (16 sequences,
+//     four rows of 32 outputs: 25 000 cycles, now 19 900; with eight warps, 64 sequences, 24 200 and 27 900)
+//   WIDE: q, k and v of a channel are shared by two threads
+enum StepShape { BY_ROW, PLAIN, WIDE };
+__host__ __device__ constexpr StepShape step_shape(uint32_t group, uint32_t own) {
+    return group == 1u ? PLAIN : own >= THREADS / 2u ? WIDE : group * (own / VALUE_OUT) <= WARPS / 2u ? BY_ROW : PLAIN;
+}
+template <int G, StepShape SHAPE>
 __global__ void __launch_bounds__(THREADS, 1)
 gen_step_kernel(const Step p) {
     extern __shared__ __align__(16) uint8_t step_smem[];
@@ -605,7 +615,7 @@ gen_step_kernel(const Step p) {
     float* products = reinterpret_cast<float*>(base + at.products);
     float* x = reinterpret_cast<float*>(base + at.rows);   // [G][d]
     float* in0 = x + G * d;                                     // [d][G]
-    float* act = in0 + G * d;                                   // [ffn][G] in C and D
+    float* act = in0 + G * d;                                   // [ffn][G] in C and D, or [G][ffn] (act_by_row)
     float* in1 = act;                                           // [d][G], and the third input behind it, in A
     float* y = act + 2u * G * d;                                // [d][G] in A and B
     uint8_t* bits = base + at.bits;                             // [3][G][own]
@@ -690,7 +700,8 @@ gen_step_kernel(const Step p) {
             return push::begin(p.push, stream, live, p.time);
         };
         push::Ahead ahead = push_begin(0u);
-        const uint32_t sums = (n + N - 1u) / N * tiles, passes = (sums + WARPS - 1u) / WARPS, items = passes * pieces;   // of D
+        constexpr bool act_by_row = SHAPE == BY_ROW;
+        const uint32_t sums = act_by_row ? n * tiles : (n + N - 1u) / N * tiles, passes = (sums + WARPS - 1u) / WARPS, items = passes * pieces;   // of D
 #pragma unroll 1
         for (uint32_t l = 0; l < p.n_layers; ++l) {
             const Layer& L = layers[l & 1u];   // everybody's since a barrier ago
@@ -710,28 +721,36 @@ gen_step_kernel(const Step p) {
                         x[r * d + o0 + o] = __fadd_rn(x[r * d + o0 + o], v);
                     } else {
                         const float m = fmaxf(v, 0.0f);           // src/model.rs:999
-                        act[(f0 + o) * G + r] = __fmul_rn(m, m);
+                        act[act_by_row ? r * ffn + f0 + o : (f0 + o) * G + r] = __fmul_rn(m, m);
                     }
                 };
-                // As many outputs per thread as leave a warp for every scheduler.
-                if (G > 1 && stage == 0u && staged && own >= THREADS / 2u) {   // q, k and v of a channel
+                // Q, K and V of this CTA's channels from matrix z0 on, J of them and all rows per thread.
+                auto qkv_of_channels = [&](auto matrices, uint32_t z0, uint32_t thread, uint32_t threads) {
+                    constexpr int J = decltype(matrices)::value;
 #pragma unroll 1
-                    for (uint32_t c = threadIdx.x; c < own; c += THREADS) {
-                        uint32_t scale[3], bias[3];
+                    for (uint32_t c = thread; c < own; c += threads) {
+                        uint32_t scale[J], bias[J];
 #pragma unroll
-                        for (int z = 0; z < 3; ++z) {
-                            scale[z] = load_half_ahead(L.qkv[z].scale + o0 + c);
-                            bias[z] = load_half_ahead(L.qkv[z].bias + o0 + c);
+                        for (int z = 0; z < J; ++z) {
+                            scale[z] = load_half_ahead(L.qkv[z0 + z].scale + o0 + c);
+                            bias[z] = load_half_ahead(L.qkv[z0 + z].bias + o0 + c);
                         }
-                        float sum[3][G];
-                        packed_sums<G, 3, true>(in0, G * d, w_wide + c * words, own * words, d, sum);
+                        float sum[J][G];
+                        packed_sums<G, J, true>(in0 + z0 * (G * d), G * d, w_wide + (z0 * own + c) * words, own * words, d, sum);
 #pragma unroll
-                        for (int z = 0; z < 3; ++z)
+                        for (int z = 0; z < J; ++z)
 #pragma unroll
                             for (int r = 0; r < G; ++r)
-                                if (r < n) emit(z * own + c, r, __fadd_rn(low_half(bias[z]), __fmul_rn(low_half(scale[z]), sum[z][r])));
+                                if (r < n) emit((z0 + z) * own + c, r, __fadd_rn(low_half(bias[z]), __fmul_rn(low_half(scale[z]), sum[z][r])));
                     }
-                } else if (stage == 2u && n_out >= 2u * THREADS) {
+                };
+                // As many outputs per thread as leave two warps for every scheduler, since one by itself issues every other cycle at best
+                // (64 sequences, 128 channels and 512 hidden units of a CTA: q, k and v of a channel by one thread 12 400 cycles, q and k beside v
+                // 11 400; four hidden units per thread 14 000, two 12 700).
+                if (SHAPE == WIDE && stage == 0u && staged) {
+                    if (threadIdx.x < THREADS / 2u) qkv_of_channels(std::integral_constant<int, 2>{}, 0u, threadIdx.x, THREADS / 2u);
+                    else qkv_of_channels(std::integral_constant<int, 1>{}, 2u, threadIdx.x - THREADS / 2u, THREADS / 2u);
+                } else if (stage == 2u && n_out >= 4u * THREADS) {
                     packed_outputs<G, 4>(L.key, staged ? w_wide : L.key.bits + (size_t)f0 * words, in0, n, d, f0, n_out, emit);
                 } else if (stage == 2u && n_out >= THREADS && n_out % 2u == 0u) {
                     packed_outputs<G, 2>(L.key, staged ? w_wide : L.key.bits + (size_t)f0 * words, in0, n, d, f0, n_out, emit);
@@ -765,8 +784,10 @@ gen_step_kernel(const Step p) {
                     }
                     __syncthreads();
                 }
-                const float* shared_out = stage == 0u ? y + o0 * G : stage == 1u ? x + o0 : act + f0 * G;
-                const bool sent = send_to_cluster(shared_out, stage == 1u ? n : 1u, d, stage == 0u ? own * G : stage == 1u ? own : f_own * G, copies, copies.exchange(stage));
+                const bool in_rows = stage == 1u || (stage == 2u && act_by_row);
+                const float* shared_out = stage == 0u ? y + o0 * G : stage == 1u ? x + o0 : act + (act_by_row ? f0 : f0 * G);
+                const bool sent = send_to_cluster(shared_out, in_rows ? n : 1u, stage == 1u ? d : ffn, (stage == 2u ? f_own : own) * (in_rows ? 1u : G), copies,
+                                                  copies.exchange(stage));
                 if (sent) exchange_odd ^= 1u << stage;
                 if (stage == 0u) {
                     // the key weights, in place of Q, K and V, and the first pieces of D
@@ -806,7 +827,16 @@ gen_step_kernel(const Step p) {
                             fetch_piece(l, i + stages - 1u);
                         }
                         copies_wait(copies, copies.ring + slot, lap, p, 0x604u);
-                        if (mine < sums) value_piece<G, N>(sum, ring + slot * stage_bytes, tiles, tile, act + k * PIECE * G + pair * N, p.minus_zero);
+                        if (mine < sums) {
+                            const uint8_t* piece = ring + slot * stage_bytes;
+                            if constexpr (act_by_row) {
+                                float one[1] = {sum[0]};
+                                value_piece<1, 1>(one, piece, tiles, tile, act + pair * ffn + k * PIECE, p.minus_zero);
+                                sum[0] = one[0];
+                            } else {
+                                value_piece<G, N>(sum, piece, tiles, tile, act + k * PIECE * G + pair * N, p.minus_zero);
+                            }
+                        }
                         __syncwarp();
                         if (lane == 0u) ptx::mbar_arrive(copies.empty() + slot);
                         if (++slot == stages) { slot = 0; ++lap; }
@@ -814,8 +844,8 @@ gen_step_kernel(const Step p) {
                     if (mine < sums) {
 #pragma unroll
                         for (int r = 0; r < N; ++r)
-                            if (pair * N + r < n) {
-                                float* to = x + (pair * N + r) * d + o0 + tile * VALUE_OUT + lane;
+                            if (act_by_row ? r == 0 : pair * N + r < n) {
+                                float* to = x + (act_by_row ? pair : pair * N + r) * d + o0 + tile * VALUE_OUT + lane;
                                 *to = __fadd_rn(*to, sum[r]);
                             }
                     }
