@@ -3,8 +3,9 @@
 // rosa_match.cuh says what a push computes: the position r < i whose key history agrees with the query history of
 // step i over the most steps, the latest of equals, and the v bit after it.  While the lag of the step before still
 // matches it stays the answer (the matches of step i are those of step i - 1 that go on), which is one bit to look at;
-// otherwise a warp compares the last 32 query bits with the 32 key bits before every position, 32 positions per
-// handful of instructions, and counts on beyond 32 steps only where all of them agree.  A stream is its three bit
+// otherwise the positions of a key word that agree with the query history are a bit mask, refined by one step of the
+// histories after the other - a word per lane where a warp searches for one stream, word after word where each lane has
+// a stream of its own - and only where 32 steps agree are they counted on one by one.  A stream is its three bit
 // histories and a lag: 3 * T / 8 + 16 bytes (at T = 2048 784 instead of the 28.7 KB of an automaton with its
 // chain), and the cost of a step grows with i / 32 and not with the runs of the keys.
 #pragma once
@@ -90,6 +91,33 @@ __device__ __forceinline__ uint32_t search_runs(const uint32_t* q, const uint32_
     return i - __reduce_max_sync(0xFFFFFFFFu, longest == top ? position : 0u);
 }
 
+// Of the positions `valid` of a word of keys those whose histories agree with the query history wq over the most steps, up to 32; `before`:
+// the word before.  MAYBE_FIRST: position r of the first word (others = 0; ~0 in any other) has only r + 1 steps behind it.
+// (A position at a time - window, difference, leading zeros - took four instructions for each of 32 positions; a word takes 32 for
+// the first eight steps, and few words have positions beyond.)
+struct Agreeing {
+    uint32_t steps, positions;
+};
+template <bool MAYBE_FIRST>
+__device__ __forceinline__ Agreeing agreeing(uint32_t before, uint32_t word, uint32_t valid, uint32_t wq, uint32_t others) {
+    Agreeing z{0u, 0u};
+    uint32_t at = valid;
+#pragma unroll
+    for (uint32_t d = 1; d <= 8u; ++d) {
+        at &= ~(__funnelshift_l(before, word, d - 1u) ^ (uint32_t)((int32_t)(wq << (d - 1u)) >> 31));
+        const uint32_t full = MAYBE_FIRST ? at & (0xFFFFFFFFu << (d - 1u) | others) : at;
+        if (full) z = Agreeing{d, full};
+    }
+#pragma unroll 1
+    for (uint32_t d = 9; at && d <= 32u; ++d) {
+        at &= ~(__funnelshift_l(before, word, d - 1u) ^ (uint32_t)((int32_t)(wq << (d - 1u)) >> 31));
+        const uint32_t full = MAYBE_FIRST ? at & (0xFFFFFFFFu << (d - 1u) | others) : at;
+        if (full) z = Agreeing{d, full};
+    }
+    return z;
+}
+__device__ __forceinline__ uint32_t top_bit(uint32_t x) { return 31u - (uint32_t)__clz((int)x); }
+
 // The lag of step i for one stream, by the whole warp; wq: the query bits up to i, k_word: the keys before i.
 __device__ __forceinline__ uint32_t search(const uint32_t* q, const uint32_t* k, uint32_t i, uint32_t wq, uint32_t k_word) {
     const uint32_t lane = threadIdx.x & 31u, last = i >> 5, q_word = wq >> (31u - (i & 31u));
@@ -97,26 +125,24 @@ __device__ __forceinline__ uint32_t search(const uint32_t* q, const uint32_t* k,
         const uint32_t lag = search_runs(q, k, i, wq, k_word);
         if (lag) return lag;
     }
-    uint32_t best = 0, before = 0;      // agreement << 26 | word of the position, the bit within the word is the lane
+    uint32_t best = 0, bit = 0, carry = 0;      // agreement << 26 | word of the position; the bit within the word
 #pragma unroll 1
     for (uint32_t w0 = 0; w0 <= last; w0 += 32u) {
-        const uint32_t mine = w0 + lane < last ? k[w0 + lane] : w0 + lane == last ? k_word : 0u;
-        const uint32_t n_words = min(32u, last + 1u - w0);
-#pragma unroll 2
-        for (uint32_t j = 0; j < n_words; ++j) {
-            const uint32_t w = w0 + j, word = __shfl_sync(0xFFFFFFFFu, mine, (int)j);
-            uint32_t n = (uint32_t)__clz((int)(wq ^ __funnelshift_l(before, word, 31u - lane)));
-            if (w == 0u) n = min(n, lane + 1u);                  // a history has position + 1 steps
-            if (w == last && lane >= (i & 31u)) n = 0u;          // not a key yet
-            best = max(best, n ? n << 26 | w : 0u);
-            before = word;
+        const uint32_t w = w0 + lane, mine = w < last ? k[w] : w == last ? k_word : 0u;
+        const uint32_t below = __shfl_up_sync(0xFFFFFFFFu, mine, 1);
+        const uint32_t valid = w < last ? ~0u : w == last ? (1u << (i & 31u)) - 1u : 0u;   // not a key yet
+        const Agreeing z = agreeing<true>(lane ? below : carry, mine, valid, wq, w ? ~0u : 0u);
+        if (z.steps && (z.steps << 26 | w) >= best) {
+            best = z.steps << 26 | w;
+            bit = top_bit(z.positions);
         }
+        carry = __shfl_sync(0xFFFFFFFFu, mine, 31);
     }
     const uint32_t most = __reduce_max_sync(0xFFFFFFFFu, best);
     if (most >> 26 < 32u) {
-        if (most == 0u) return 0u;
-        const uint32_t at = 31u - (uint32_t)__clz((int)__ballot_sync(0xFFFFFFFFu, best == most));
-        return i - (32u * (most & 0x3FFFFFFu) + at);
+        const uint32_t w = most & 0x3FFFFFFu;
+        bit = __shfl_sync(0xFFFFFFFFu, bit, (int)(w & 31u));   // of the lane that has this word
+        return most ? i - (32u * w + bit) : 0u;
     }
     // whole windows agree: count on from there
     uint32_t longest = 0, position = 0;
@@ -130,26 +156,24 @@ __device__ __forceinline__ uint32_t search(const uint32_t* q, const uint32_t* k,
     return i - __reduce_max_sync(0xFFFFFFFFu, longest == top ? position : 0u);
 }
 
-// The same for one stream per lane (open lanes only); DEEP where whole windows agree, which is left to search().  The
-// position is found at once, so it has to fit 26 bits.
+// The same for one stream per lane (open lanes only); DEEP where whole windows agree, which is left to search().
 constexpr uint32_t DEEP = ~0u;
 __device__ __forceinline__ uint32_t search_alone(const uint32_t* k, uint32_t i, uint32_t wq, uint32_t k_word) {
     const uint32_t last = i >> 5;
-    uint32_t best = 0, before = 0, next = last ? k[0] : k_word;
+    uint32_t steps = 0, position = 0, word = k_word, valid = (1u << (i & 31u)) - 1u;
 #pragma unroll 1
-    for (uint32_t w = 0; w <= last; ++w) {
-        const uint32_t word = next, n_bits = w == last ? i & 31u : 32u;
-        next = w + 1u < last ? k[w + 1u] : k_word;
-#pragma unroll 8
-        for (uint32_t b = 0; b < n_bits; ++b) {
-            uint32_t n = (uint32_t)__clz((int)(wq ^ __funnelshift_l(before, word, 31u - b)));
-            if (w == 0u) n = min(n, b + 1u);
-            best = max(best, (n << 26) + 32u * w + b);
+    for (uint32_t w = last; steps < 32u; --w) {   // from the latest word on: of equals the first one found counts
+        const uint32_t before = w ? k[w - 1u] : 0u;
+        const Agreeing z = w ? agreeing<false>(before, word, valid, wq, ~0u) : agreeing<true>(before, word, valid, wq, 0u);
+        if (z.steps > steps) {
+            steps = z.steps;
+            position = 32u * w + top_bit(z.positions);
         }
-        before = word;
+        if (w == 0u) break;
+        word = before;
+        valid = ~0u;
     }
-    const uint32_t most = best >> 26;
-    return most == 32u ? DEEP : most ? i - (best & 0x3FFFFFFu) : 0u;
+    return steps == 32u ? DEEP : steps ? i - position : 0u;
 }
 
 // What step i of 32 streams (first + lane; a lane with live = false has none) can know before its bits: whether the lag of
@@ -183,7 +207,7 @@ __device__ __forceinline__ bool step(const Histories& H, size_t first, bool live
     const bool known = !live || goes_on;
     uint32_t open = __ballot_sync(0xFFFFFFFFu, !known);
     // One after the other by the whole warp, or side by side with a lane each: by the instructions either takes.
-    if ((uint32_t)__popc(open) * (6u * last + 150u) > 6u * i + 100u && i < (1u << 26)) {
+    if ((uint32_t)__popc(open) * (60u * (last / 32u + 1u) + 110u) > 48u * (last + 1u) + 60u) {
         if (!known) c.lag = search_alone(H.of(s, 1), i, c.q, c.k);
         open = __ballot_sync(0xFFFFFFFFu, !known && c.lag == DEEP);
     }

@@ -282,11 +282,14 @@ __device__ __forceinline__ void mixed_inputs(const Step& p, const Layer& L, uint
     if (c < d) ask(c);
     __syncthreads();
     if (rows_statistics(x, in, n, d, stats) && !half) {
-        // the keys of this CTA's streams, for a search
+        // the keys of this CTA's streams, for a search, and the v bits it leads to
         const uint32_t threads = THREADS - n * 32u;
 #pragma unroll 1
-        for (uint32_t i = threadIdx.x - n * 32u; i < n * own; i += threads)
-            warm(p.push.of(((size_t)layer * p.rows + row + i / own) * d + o0 + i % own, 1), (p.time / 32u + 1u) * 4u);
+        for (uint32_t i = threadIdx.x - n * 32u; i < n * own; i += threads) {
+            const size_t stream = ((size_t)layer * p.rows + row + i / own) * d + o0 + i % own;
+            warm(p.push.of(stream, 1), (p.time / 32u + 1u) * 4u);
+            warm(p.push.of(stream, 2), (p.time / 32u + 1u) * 4u);
+        }
     }
     __syncthreads();
 #pragma unroll 1
