@@ -43,8 +43,7 @@ __global__ void __launch_bounds__(128)
 rosa_classify_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restrict__ k_sw,
                      const uint32_t* __restrict__ v_sw, uint32_t* __restrict__ idx_sw, size_t streams, uint32_t T,
                      size_t wps, uint32_t* __restrict__ list, uint32_t* __restrict__ count,
-                     uint32_t* __restrict__ cq_list, uint32_t* __restrict__ cq_count, uint32_t* __restrict__ given_up,
-                     bool clear_listed) {
+                     uint32_t* __restrict__ cq_list, uint32_t* __restrict__ cq_count, uint32_t* __restrict__ given_up) {
     chain_entry();
     constexpr uint32_t G = CLASSIFY_LANES;
     const size_t s = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
@@ -117,13 +116,9 @@ rosa_classify_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restri
                 out[w] = word;
             }
         }
-    } else {
-        if (clear_listed)   // rosa_context_kernel puts the words of a stream together from several CTAs
-            for (uint32_t w = sub; w <= last; w += G) out[w] = 0u;
-        if (sub == 0) {
-            if (constant(2, &c)) cq_list[atomicAdd(cq_count, 1u)] = (uint32_t)s;   // constant q: a long scan, its own kernel
-            else list[atomicAdd(count, 1u)] = (uint32_t)s;
-        }
+    } else if (sub == 0) {
+        if (constant(2, &c)) cq_list[atomicAdd(cq_count, 1u)] = (uint32_t)s;   // constant q: a long scan, its own kernel
+        else list[atomicAdd(count, 1u)] = (uint32_t)s;
     }
 }
 
@@ -386,7 +381,7 @@ __host__ __device__ inline uint32_t context_bits(uint32_t T, bool together) { re
 // The streams whose keys are spread evenly (rosa_heads.cuh).  A stream is cut into `pieces`, a warp takes one: it puts the keys
 // of the rows before into tables of its own and goes on from there.  The other streams go to `left`, once: a stream is given up
 // as soon as the walks of a piece, the longest of each row, have come to more than `base` + `per_row` positions per row so far, 32
-// steps beyond the first window counted as a position.  given_up: a word per stream, zero before.
+// steps beyond the first window counted as a position.  given_up: a word per stream, zero before (2: to rosa_match_kernel).
 struct HeadsLayout {   // bytes of shared memory of a warp
     uint32_t latest_7, latest_3, link, q, k, v, total;   // latest_11 is at 0
     __host__ __device__ explicit HeadsLayout(uint32_t T) {
@@ -675,7 +670,7 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
             }
         }
         const auto leave = [&] {   // to rosa_match_kernel, by the first part that does
-            if (parts == 1u || atomicExch(&heads_call.given_up[s], 1u) == 0u) hard[atomicAdd(hard_count, 1u)] = (uint32_t)s;
+            if (parts == 1u || atomicExch(&heads_call.given_up[s], 2u) != 2u) hard[atomicAdd(hard_count, 1u)] = (uint32_t)s;
         };
         if (!taken) {
             if (threadIdx.x == 0) leave();
@@ -772,7 +767,8 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
             return true;
         };
         if (TOGETHER) {   // the steps below BRUTE by a warp each
-            for (uint32_t t = part * NW + warp; t < min(BRUTE, T); t += parts * NW) {
+            for (uint32_t t = warp; t < min(BRUTE, T); t += NW) {
+                if (!own_row(t >> 5)) continue;
                 const uint32_t wq = context::window(Q, t);
                 uint32_t best = 0;
                 for (uint32_t r = lane; r < t; r += 32u) {
@@ -859,11 +855,9 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
         __syncthreads();
         if (sh_gone) {
             if (threadIdx.x == 0) leave();
-        } else if (parts > 1u) {
-            for (uint32_t w = threadIdx.x; w < words; w += NT)
-                if (out_s[w]) atomicOr(&out[w], out_s[w]);
         } else if (sorted || TOGETHER) {
-            for (uint32_t w = threadIdx.x; w < words; w += NT) out[w] = out_s[w];
+            for (uint32_t w = threadIdx.x; w < words; w += NT)
+                if (own_row(w)) out[w] = out_s[w];
         }
     }
 }
@@ -1119,7 +1113,7 @@ void contexts(ullis_cuda_runtime* rt, const MatchCall& m) {
     };
     if (m.form == LATEST_TOO) {
         launch(uneven, m.form, m.list, m.counts, 0u, half, "rosa_heads");
-        launch(uneven, PLAIN, m.left, m.counts + 5, 1u, all, "rosa_context");
+        launch(uneven, IN_PARTS, m.left, m.counts + 5, 1u, all, "rosa_context");
         return;
     }
     launch(uneven, m.form, m.list, m.counts, 0u, half, "rosa_context");
@@ -1157,7 +1151,7 @@ void rosa_match(ullis_cuda_runtime* rt, const uint32_t* q_sw, const uint32_t* k_
     rt->sam_last_streams = streams;
     if (!rt->parent) rt->lanes_last = 1;
     rt->chain(rosa_classify_kernel, (unsigned)((streams * CLASSIFY_LANES + 127) / 128), 128, 0, q_sw, k_sw, v_sw, idx_sw,
-              streams, T, m.wps, m.list, m.counts, m.cq_list, m.counts + 1, m.given_up, m.form == IN_PARTS);
+              streams, T, m.wps, m.list, m.counts, m.cq_list, m.counts + 1, m.given_up);
     rt->launched("rosa_classify");
     contexts(rt, m);
     if (T <= 1024u) launch_match<1>(rt, m, 0, 1024);
@@ -1237,7 +1231,7 @@ void rosa_sam(ullis_cuda_runtime* rt, const uint32_t* q_sw, const uint32_t* k_sw
         rt->zero(count, 8);   // both counters
         const unsigned classify_grid = (unsigned)((streams * CLASSIFY_LANES + 127) / 128);
         rt->chain(rosa_classify_kernel, classify_grid, 128, 0, q_sw, k_sw, v_sw, idx_sw, streams, (uint32_t)time, wps, list,
-                                                             count, cq_list, cq_count, nullptr, false);
+                                                             count, cq_list, cq_count, nullptr);
         rt->launched("rosa_classify");
         // The constant-q scan is a long serial loop for a few thousand threads; it depends on nothing but the
         // classification and writes idx words no other kernel of this call touches, so it runs on the side stream
