@@ -177,13 +177,21 @@ void in_shares(ullis_cuda_runtime* rt, size_t shares, bool results_locked, In co
     ULLIS_CUDA_CHECK(cudaEventRecord(rt->copies_done, rt->copy_out));
     ULLIS_CUDA_CHECK(cudaStreamWaitEvent(rt->stream, rt->copies_done, 0));
 }
-// Shares of a call: each with results of 4 MiB at least (about 80 us on the link, where a share costs its launches) and `least` of
-// the `items` that it is cut by.  A call whose kernels are timed goes in one piece: a bracket of events around a share's kernel
-// would hold the wait for its input, and the copies beside it.
-size_t shares_for(const ullis_cuda_runtime* rt, size_t result_bytes, size_t items, size_t least) {
-    if (rt->kernel_timing) return 1;
-    return std::max<size_t>(1, std::min({ullis_cuda_runtime::MAX_SHARES, result_bytes >> 22, items / std::max<size_t>(least, 1)}));
-}
+// Shares of a call: up to four, each with results of 4 MiB at least (about 80 us on the link, where a share costs its launches) and `least`
+// of the `items` that it is cut by; the first one in two halves, where they have as much, since nothing comes back before it is computed.
+// A call whose kernels are timed goes in one piece: a bracket of events around a share's kernel would hold the wait for its input, and the
+// copies beside it.
+struct Shares {
+    size_t n, items, whole;   // whole: as many as there would be without the halves
+    Shares(const ullis_cuda_runtime* rt, size_t result_bytes, size_t items_, size_t least) : items(items_) {
+        least = std::max<size_t>(least, 1);
+        whole = rt->kernel_timing ? 1 : std::max<size_t>(1, std::min({ullis_cuda_runtime::MAX_SHARES - 1, result_bytes >> 22, items / least}));
+        n = whole > 1 && items / (2 * whole) >= std::max<size_t>(least / 2, 1) ? whole + 1 : whole;
+    }
+    size_t first(size_t s) const {   // 0 <= s <= n
+        return n == whole ? items * s / n : items * (s <= 1 ? s : 2 * (s - 1)) / (2 * whole);
+    }
+};
 bool page_locked(const void* p) {
     cudaPointerAttributes attr;
     if (p && cudaPointerGetAttributes(&attr, p) == cudaSuccess) return attr.type == cudaMemoryTypeHost;
@@ -1045,7 +1053,8 @@ int32_t ullis_cuda_binary_linear(ullis_cuda_runtime* rt, const float* x, const u
         if (rows == 0) return;
         need_ptr(x, "x"); need_ptr(bits, "bits"); need_ptr(scale, "scale"); need_ptr(y, "y");
         // whole 256-row tiles in every share but the last
-        const size_t shares = shares_for(rt, ny * 4, rows, 256), share_rows = ((rows + shares - 1) / shares + 255) / 256 * 256;
+        const Shares split(rt, ny * 4, (rows + 255) / 256, 2);
+        const size_t shares = split.n;
         Inputs in(rt);
         float* dx = shares > 1 ? rt->pool[0].as<float>(nx) : in.add(0, x, nx);
         uint32_t* dbits = in.add(1, bits, words);
@@ -1054,7 +1063,7 @@ int32_t ullis_cuda_binary_linear(ullis_cuda_runtime* rt, const float* x, const u
         float* dy = rt->pool[4].as<float>(ny);
         in.send();
         rt->clear_status();
-        const auto first = [&](size_t s) { return std::min(rows, s * share_rows); };
+        const auto first = [&](size_t s) { return std::min(rows, split.first(s) * 256); };
         const auto count = [&](size_t s) { return first(s + 1) - first(s); };
         in_shares(rt, shares, shares > 1 && page_locked(y),
             [&](size_t s, cudaStream_t stream) {
@@ -1143,7 +1152,9 @@ int32_t ullis_cuda_rosa_qkv_1bit_fwd(ullis_cuda_runtime* rt, const uint32_t* q_b
         // Shares of whole sequences, whose planes begin on a word; 1 024 streams keep the device busy (not in the automaton, whose
         // launches last as long as a stream).
         const size_t result_bytes = (idx ? n : 0) + (out ? n * 4 : 0);
-        const size_t shares = time * channels % 32 || !k::rosa_without_automaton(rt, batch * channels, time) ? 1 : shares_for(rt, result_bytes, batch, (1023 + channels) / channels);
+        const bool whole = time * channels % 32 || !k::rosa_without_automaton(rt, batch * channels, time);
+        const Shares split(rt, whole ? 0 : result_bytes, batch, (1023 + channels) / channels);
+        const size_t shares = split.n;
         Inputs in(rt);
         uint32_t* planes[3];
         const uint32_t* const host[3] = {q_bits, k_bits, v_bits};
@@ -1157,7 +1168,7 @@ int32_t ullis_cuda_rosa_qkv_1bit_fwd(ullis_cuda_runtime* rt, const uint32_t* q_b
         uint32_t* counts = shares > 1 ? rt->sam_share_counts.as<uint32_t>(2 * ullis_cuda_runtime::MAX_SHARES) : nullptr;
         in.send();
         rt->clear_status();
-        const auto first = [&](size_t s) { return batch * s / shares; };
+        const auto first = [&](size_t s) { return split.first(s); };
         in_shares(rt, shares, shares > 1 && page_locked(out ? static_cast<const void*>(out) : idx),
             [&](size_t s, cudaStream_t stream) {
                 const size_t w0 = first(s) * time * channels / 32, w1 = first(s + 1) * time * channels / 32;

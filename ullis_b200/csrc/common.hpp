@@ -151,7 +151,7 @@ struct ullis_cuda_runtime {
     const uint32_t* sam_last_counts = nullptr;   // ... and its counters: listed, constant q
     // Copies beside kernels: an op-level call with large results runs in shares, whose inputs and results travel on streams of
     // their own while `stream` computes.  Created on first use; idle whenever no call is running.
-    static constexpr size_t MAX_SHARES = 4;
+    static constexpr size_t MAX_SHARES = 5;
     cudaStream_t copy_in = nullptr, copy_out = nullptr;
     cudaEvent_t share_in[MAX_SHARES] = {}, share_out[MAX_SHARES] = {}, copies_done = nullptr;
     void copy_streams();

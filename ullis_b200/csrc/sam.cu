@@ -997,7 +997,7 @@ void launch_context(ullis_cuda_runtime* rt, const MatchCall& m, int shape, Conte
     // ever change went to the match kernel).
     const ContextLimits limits{24u, 96u, 160u, 64u, 256u};
     size_t smem = rt->context_smem[shape];
-    HeadsCall heads{0u, 1u, 128u, 24u, m.counts + 6, m.left, m.counts + 5, m.given_up};
+    HeadsCall heads{0u, 1u, 128u, 40u, m.counts + 6, m.left, m.counts + 5, m.given_up};
     auto kernel = rosa_context_kernel<NT, TOGETHER>;
     if (form == LATEST_TOO) {
         kernel = rosa_context_kernel<NT, TOGETHER, LATEST_TOO>;
@@ -1013,9 +1013,9 @@ void launch_context(ullis_cuda_runtime* rt, const MatchCall& m, int shape, Conte
         // 14.4 / 16.7).
         const size_t warps = (size_t)rt->context_ctas[shape] * heads.warps;
         heads.pieces = m.T < 1024u ? (m.streams * 4u <= warps ? 4u : 1u) : m.streams * 2u < 3u * warps ? 4u : m.streams < 8u * warps ? 2u : 1u;
-        // heads.base, heads.per_row: a row whose walks are 29 positions long takes as many instructions as by contexts.  Less than 16 leaves
-        // them streams that are cheaper here (8 times 2048 steps 12 / 16 / 24 / 32 per row 3.12 / 3.03 / 2.94 / 2.95 ms, 16 times 1100 2.43 /
-        // 2.46 / 2.44 / 2.41), and a base too small all that are short (twice 700 steps, base 32 / 64 / 128: 0.75 / 0.62 / 0.61).
+        // heads.base, heads.per_row: less leaves the contexts streams that are cheaper here (whole calls with 12 / 16 / 24 / 40 per row, ms:
+        // 16 times 2048 steps 9.70 / 9.61 / 9.57 / 9.46, 16 times 1100 5.37 / 5.35 / 5.25 / 5.13, 5 times 1531 3.38 / 3.36 / 3.36 / 3.31), and a base
+        // too small all that are short (ROSA kernels of twice 700 steps, base 32 / 64 / 128: 0.75 / 0.62 / 0.61).
     } else if constexpr (TOGETHER) {
         if (form == IN_PARTS) kernel = rosa_context_kernel<NT, TOGETHER, IN_PARTS>;
     }
