@@ -868,44 +868,47 @@ constexpr int MATCH_WARPS = 4;
 constexpr uint32_t MATCH_COUNTS = 7;   // of MatchCall
 
 // A stream whose query bits are all c: idx follows the longest run of c among the keys so far, the latest of equals
-// (sam_core.cuh run_constant_q), a running maximum over (run length, position).  T <= 65535.
+// (sam_core.cuh run_constant_q), a running maximum over (run length, position).  A lane has a word: the run that comes in from the words
+// before follows from the full ones among them, the longest run so far from a scan over the words' maxima, and the v bit that a
+// run leads to lies in the word or the one after it.  T <= 8192.  (With a lane per step and a scan per word, 64 words one after the other:
+// one sequence of the default model, 2048 steps, 18 us a layer for this kernel, now 13.5; an empty launch between events takes 6.)
 __device__ __forceinline__ void constant_q_warp(uint32_t c, const uint32_t* __restrict__ k, const uint32_t* __restrict__ v,
                                                 uint32_t* __restrict__ out, uint32_t T) {
+    constexpr uint32_t ALL = 0xFFFFFFFFu;
     const uint32_t lane = threadIdx.x & 31u, words = (T + 31u) / 32u;
-    uint32_t run_before = 0, best = 0;   // run length << 16 | position + 1
-    for (uint32_t row0 = 0; row0 < words; row0 += 32u) {
-        const uint32_t keys = row0 + lane < words ? k[row0 + lane] : 0u;
-        for (uint32_t row4 = row0; row4 < min(row0 + 32u, words); row4 += 4u) {   // four words, their v bits in flight together
-            uint32_t mine[4], bit[4];
+    uint32_t run_before = 0, best = 0;   // run length << 15 | (position + 1) << 1 | v bit of the step after the position
+    for (uint32_t w0 = 0; w0 < words; w0 += 32u) {
+        const uint32_t w = w0 + lane, key = w < words ? k[w] : 0u, same = w < words ? c ? key : ~key : 0u;
+        const uint32_t after = __funnelshift_r(w < words ? v[w] : 0u, w + 1u < words ? v[w + 1u] : 0u, 1u);   // bit b: v of step b + 1
+        const uint32_t full = __ballot_sync(ALL, same == ALL), upper = (uint32_t)__clz((int)~same);
+        const uint32_t z = lane ? min((uint32_t)__clz((int)~(full << (32u - lane))), lane) : 0u;   // full words right below
+        const uint32_t there = __shfl_sync(ALL, upper, (int)(z < lane ? lane - 1u - z : 0u));
+        const uint32_t run0 = 32u * z + (z < lane ? there : run_before);
+        // the longest run that ends at a position of the word from `cur` on; bit b of the answer: what is known before position b
+        const auto walk = [&](uint32_t cur, uint32_t& answer) {
+            uint32_t run = run0;
 #pragma unroll
-            for (uint32_t u = 0; u < 4u; ++u) {
-                const uint32_t row = row4 + u, t = row * 32u + lane, word = __shfl_sync(0xFFFFFFFFu, keys, (int)(row - row0));
-                const uint32_t same = c ? word : ~word;
-                const uint32_t n = min((uint32_t)__clz((int)~(same << (31u - lane))), lane + 1u);
-                const uint32_t run = n == lane + 1u ? n + run_before : n;
-                uint32_t key = run ? run << 16 | (t + 1u) : 0u;
-#pragma unroll
-                for (uint32_t o = 1; o < 32u; o <<= 1) {
-                    const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, key, o);
-                    if (lane >= o) key = max(key, x);
-                }
-                mine[u] = __shfl_up_sync(0xFFFFFFFFu, key, 1);   // the positions before t
-                mine[u] = lane == 0u ? best : max(mine[u], best);
-                if (t >= T) mine[u] = 0u;
-                run_before = __shfl_sync(0xFFFFFFFFu, run, 31);
-                best = max(best, __shfl_sync(0xFFFFFFFFu, key, 31));
+            for (uint32_t b = 0; b < 32u; ++b) {
+                answer |= (cur & 1u) << b;
+                const bool is = same >> b & 1u;
+                run = is ? run + 1u : 0u;
+                const uint32_t x = run << 15 | (32u * w + b + 1u) << 1 | (after >> b & 1u);
+                cur = is && x > cur ? x : cur;
             }
+            return cur;
+        };
+        uint32_t unused = 0, word = 0, longest = walk(0u, unused);
 #pragma unroll
-            for (uint32_t u = 0; u < 4u; ++u) {
-                const uint32_t p = mine[u] & 0xFFFFu;
-                bit[u] = mine[u] ? (v[p >> 5] >> (p & 31u)) & 1u : 0u;
-            }
-#pragma unroll
-            for (uint32_t u = 0; u < 4u; ++u) {
-                const uint32_t word = __ballot_sync(0xFFFFFFFFu, bit[u] != 0u);
-                if (lane == 0 && row4 + u < words) out[row4 + u] = word;
-            }
+        for (uint32_t o = 1; o < 32u; o <<= 1) {
+            const uint32_t x = __shfl_up_sync(ALL, longest, o);
+            if (lane >= o) longest = max(longest, x);
         }
+        const uint32_t below = __shfl_up_sync(ALL, longest, 1);
+        walk(lane ? max(best, below) : best, word);
+        if (w + 1u == words && (T & 31u)) word &= (1u << (T & 31u)) - 1u;
+        if (w < words) out[w] = word;
+        best = max(best, __shfl_sync(ALL, longest, 31));
+        run_before = __shfl_sync(ALL, same == ALL ? run0 + 32u : upper, 31);
     }
 }
 
