@@ -335,9 +335,27 @@ col_partial_kernel(const float* __restrict__ a, const void* __restrict__ b, cons
     if (c < C && warp < (MODE == COL_LN ? 2u : 1u)) part[((size_t)warp * gridDim.y + blockIdx.y) * C + c] = acc;
 }
 
-// out[y, c] = sum over the chunks of part[y, chunk, c]
+// Fp16Storage::apply_clipped_sgd (src/precision.rs:106-113) on g * gmul
+__device__ __forceinline__ void clipped_step(uint16_t& w, float& residual, float g, float lr) {
+    const float current = h2f(w);
+    const float update = __fmul_rn(lr, fminf(fmaxf(g, -1.0f), 1.0f));
+    const float desired = __fadd_rn(__fsub_rn(current, update), residual);
+    const uint16_t rounded = __half_as_ushort(__float2half_rn(desired));
+    residual = __fsub_rn(desired, h2f(rounded));
+    w = rounded;
+}
+
+// FP16 parameters that a column sum (or two) is the gradient of; null: the sums themselves are wanted.
+struct ColStep {
+    uint16_t* w[2];
+    float* residual[2];
+    float gmul, lr;
+};
+
+// out[y, c] = sum over the chunks of part[y, chunk, c]; or the step that it is the gradient for, at once (as a launch of its own each of
+// these vectors of 512 took a training step 2.5 us, 62 of them).
 __global__ void __launch_bounds__(64)
-col_final_kernel(const float* __restrict__ part, float* __restrict__ out, size_t chunks, size_t C) {
+col_final_kernel(const float* __restrict__ part, float* __restrict__ out, size_t chunks, size_t C, const ColStep step) {
     chain_entry();
     const size_t c = (size_t)blockIdx.x * 64 + threadIdx.x;
     if (c >= C) return;
@@ -352,7 +370,8 @@ col_final_kernel(const float* __restrict__ part, float* __restrict__ out, size_t
         for (int i = 0; i < 16; ++i) acc += v[i];
     }
     for (; k < chunks; ++k) acc += part[k * C];
-    out[blockIdx.y * C + c] = acc;
+    if (step.w[0]) clipped_step(step.w[blockIdx.y][c], step.residual[blockIdx.y][c], __fmul_rn(acc, step.gmul), step.lr);
+    else out[blockIdx.y * C + c] = acc;
 }
 
 // ------------------------------------------------------------ LayerNorm backward
@@ -511,16 +530,6 @@ __global__ void emit_transposed_kernel(const uint32_t* __restrict__ idx_sw, cons
 }
 
 // ------------------------------------------------------------ optimiser
-// Fp16Storage::apply_clipped_sgd (src/precision.rs:106-113) on g * gmul
-__device__ __forceinline__ void clipped_step(uint16_t& w, float& residual, float g, float lr) {
-    const float current = h2f(w);
-    const float update = __fmul_rn(lr, fminf(fmaxf(g, -1.0f), 1.0f));
-    const float desired = __fadd_rn(__fsub_rn(current, update), residual);
-    const uint16_t rounded = __half_as_ushort(__float2half_rn(desired));
-    residual = __fsub_rn(desired, h2f(rounded));
-    w = rounded;
-}
-
 // A CTA has 1024 elements, four per thread, their loads in flight together.  The gradient is the sum of `sums` arrays of n
 // elements, in their order (the shares of a split product).
 __global__ void __launch_bounds__(256)
@@ -778,12 +787,10 @@ __global__ void init_latent_kernel(const uint32_t* __restrict__ bits, uint16_t* 
     latent[i] = (bits[i >> 5] >> (i & 31)) & 1u ? LATENT_PLUS : (uint16_t)(LATENT_PLUS | 0x8000u);
 }
 
-// out [C] (COL_LN: two of them)
-void col_reduce_launch(ullis_cuda_runtime* rt, const float* a, const void* b, float* out, size_t R, size_t C, ColMode mode,
-                       DeviceBuffer& scratch, size_t time = 0, const float2* stats = nullptr) {
+// The sums over chunks of rows, left in `part`.
+void col_partial_launch(ullis_cuda_runtime* rt, const float* a, const void* b, float* part, size_t R, size_t C, ColMode mode, size_t time,
+                        const float2* stats) {
     const size_t chunks = (R + COL_ROWS - 1) / COL_ROWS;
-    const unsigned outs = mode == COL_LN ? 2 : 1;
-    float* part = scratch.as<float>(outs * chunks * C);
     const dim3 grid(blocks_for(C, 32), (unsigned)chunks);
     const auto run = [&](auto kernel) {
         rt->chain(kernel, grid, 256, 0, a, b, stats, part, (uint32_t)R, (uint32_t)C, (uint32_t)time);
@@ -796,8 +803,19 @@ void col_reduce_launch(ullis_cuda_runtime* rt, const float* a, const void* b, fl
         case COL_BITS: run(col_partial_kernel<COL_BITS>); break;
     }
     rt->launched("col_partial");
-    rt->chain(col_final_kernel, dim3(blocks_for(C, 64), outs), 64, 0, part, out, chunks, C);
+}
+// out [outs, C], or the steps
+void col_final_launch(ullis_cuda_runtime* rt, const float* part, float* out, size_t R, size_t C, unsigned outs, const ColStep& step) {
+    rt->chain(col_final_kernel, dim3(blocks_for(C, 64), outs), 64, 0, part, out, (R + COL_ROWS - 1) / COL_ROWS, C, step);
     rt->launched("col_final");
+}
+// out [C] (COL_LN: two of them)
+void col_reduce_launch(ullis_cuda_runtime* rt, const float* a, const void* b, float* out, size_t R, size_t C, ColMode mode,
+                       DeviceBuffer& scratch, size_t time = 0, const float2* stats = nullptr) {
+    const unsigned outs = mode == COL_LN ? 2 : 1;
+    float* part = scratch.as<float>(outs * ((R + COL_ROWS - 1) / COL_ROWS) * C);
+    col_partial_launch(rt, a, b, part, R, C, mode, time, stats);
+    col_final_launch(rt, part, out, R, C, outs, ColStep{});
 }
 
 // ------------------------------------------------------------ host helpers
@@ -833,9 +851,13 @@ struct Step {
         rt->chain(unpack_transpose_kernel, blocks_for(in_f * outp, 256), 256, 0, bits, out, out_f, in_f, outp);
         rt->launched("unpack_transpose");
     }
-    // out[c] = sum_r f(a[r,c], b[r,c])
-    void col_reduce(const float* a, const void* b, float* out, size_t R, size_t C, ColMode mode, size_t time = 0) {
-        col_reduce_launch(rt, a, b, out, R, C, mode, st->part, time);
+    // The gradient g[c] = sum_r f(a[r,c], b[r,c]) of a vector, and (after the last use of the vector, before the next gradient) its step.
+    void col_gradient(const float* a, const void* b, size_t R, size_t C, ColMode mode, size_t time = 0, const float2* stats = nullptr) {
+        col_partial_launch(rt, a, b, st->part.as<float>((mode == COL_LN ? 2 : 1) * ((R + COL_ROWS - 1) / COL_ROWS) * C), R, C, mode, time, stats);
+    }
+    void col_step(const Fp16Param& p, size_t R, float rate, const Fp16Param* second = nullptr) {
+        col_final_launch(rt, st->part.as<float>(1), nullptr, R, p.n, second ? 2 : 1,
+                         ColStep{{p.w, second ? second->w : nullptr}, {p.residual, second ? second->residual : nullptr}, gmul, rate});
     }
     void sgd(const Fp16Param& p, const float* g, float rate, uint32_t sums = 1) {
         rt->chain(clipped_sgd_kernel, blocks_for(p.n, 1024), 256, 0, p.w, p.residual, g, sums, gmul, rate, p.n);
@@ -843,17 +865,15 @@ struct Step {
     }
     // gx_out (+)= LN backward of (x, gy); steps the LayerNorm's weight and bias
     void ln_backward(const float* x, const float* gy, const Fp16Param& w, const Fp16Param& b, float* gx_out,
-                     bool accumulate, float* small, size_t rows, size_t d) {
+                     bool accumulate, size_t rows, size_t d) {
         float2* stats = st->ln_stats.as<float2>(rows);
         ln_backward_launch(rt, x, gy, w.w, gx_out, stats, rows, d, accumulate ? 1 : 0);
-        col_reduce_launch(rt, gy, x, small, rows, d, COL_LN, st->part, 0, stats);   // g_weight, then g_bias
-        sgd(w, small, lr);
-        sgd(b, small + d, lr);
+        col_gradient(gy, x, rows, d, COL_LN, 0, stats);   // g_weight, then g_bias
+        col_step(w, rows, lr, &b);
     }
-    // Packed matrix: G = gy^T . x (unscaled by the row scale), then scale / bias / latent steps.
-    // gy16t: FP16(gy)^T [out, rows_p]; x16t: FP16(x)^T [in, rows_p].  g_bias (or null) is already reduced.
-    void packed_update(PackedParam& p, const uint16_t* gy16t, const uint16_t* x16t, size_t rows_p, const float* g_bias,
-                       float bias_lr, unsigned long long* flips, float* small) {
+    // Packed matrix: G = gy^T . x (unscaled by the row scale), then scale / latent steps.
+    // gy16t: FP16(gy)^T [out, rows_p]; x16t: FP16(x)^T [in, rows_p].
+    void packed_update(PackedParam& p, const uint16_t* gy16t, const uint16_t* x16t, size_t rows_p, unsigned long long* flips, float* small) {
         const size_t out_f = p.weights->out, in_f = p.weights->in;
         float* G = st->gmat.as<float>(out_f * in_f);
         uint32_t* bits = const_cast<uint32_t*>(p.weights->bits);
@@ -872,7 +892,6 @@ struct Step {
             rt->launched("latent_sgd");
             sgd(p.scale, small, lr);
         }
-        if (p.bias.w && g_bias) sgd(p.bias, g_bias, bias_lr);
     }
 };
 
@@ -1117,15 +1136,18 @@ void ullis_cuda_train_state::step(const uint32_t* tokens, const uint32_t* labels
     k::ce_reduce(rt, RL, lab, ignore_id, rows, time, reinterpret_cast<double*>(res),
                  reinterpret_cast<unsigned long long*>(res + 8));
     m->have_result = true;
-    s.col_reduce(LG, nullptr, SM + 2 * vocab, rows, vocab, COL_SUM);                // g_bias
+    if (head.bias.w) {   // not used again in this step
+        s.col_gradient(LG, nullptr, rows, vocab, COL_SUM);
+        s.col_step(head.bias, rows, learning_rate * HEAD_BIAS_LR_MULT);
+    }
     s.operands(LG, m->head.scale, A16, T16, rows, vocab, rows_p);                   // (gy*scale) [rows, V], gy^T [V, rows]
     s.unpack_transpose(m->head.bits, B16, vocab, d, vocab_p);                       // S^T [d, V]
     s.gemm(A16, B16, GX, rows, vocab_p, d);                                         // g_hidden
     s.operands(H, nullptr, nullptr, B16, rows, d, rows_p);                          // hidden^T [d, rows]
-    s.packed_update(head, T16, B16, rows_p, SM + 2 * vocab, learning_rate * HEAD_BIAS_LR_MULT, CNT + 0, SM);
+    s.packed_update(head, T16, B16, rows_p, CNT + 0, SM);
 
     // ---- ln_out
-    s.ln_backward(X, GX, ln_out_w, ln_out_b, T1, false, SM, rows, d);
+    s.ln_backward(X, GX, ln_out_w, ln_out_b, T1, false, rows, d);
     std::swap(GX, T1);
 
     for (size_t li = m->layers; li-- > 0;) {
@@ -1159,34 +1181,37 @@ void ullis_cuda_train_state::step(const uint32_t* tokens, const uint32_t* labels
         s.unpack_transpose(L.key.bits, B16, f, d, f_p);
         s.gemm(KEY16, B16, T3, rows, f_p, d);                                                         // g_shifted
         s.operands(T2, nullptr, nullptr, B16, rows, d, rows_p);
-        s.packed_update(T.key, key_t, B16, rows_p, nullptr, 0.0f, CNT + 1, SM);
+        s.packed_update(T.key, key_t, B16, rows_p, CNT + 1, SM);
         // time-shift mix (src/model.rs:1164-1176)
-        s.col_reduce(T3, T1, SM, rows, d, COL_SHIFT, time);                                                     // g_mix
+        s.col_gradient(T3, T1, rows, d, COL_SHIFT, time);                                                       // g_mix
         if (d % 4 == 0)
             rt->chain(lerp_bwd_kernel<4>, blocks_for(n / 4, 256), 256, 0, T3, L.ffn_x_k, T1, (uint32_t)rows, (uint32_t)time,
                       (uint32_t)d);
         else
             rt->chain(lerp_bwd_kernel<1>, blocks_for(n, 256), 256, 0, T3, L.ffn_x_k, T1, (uint32_t)rows, (uint32_t)time, (uint32_t)d);
         rt->launched("lerp_bwd");
-        s.sgd(T.x_k, SM, learning_rate);                                                              // after its last use
-        s.ln_backward(AR, T1, T.ln2_w, T.ln2_b, GX, true, SM, rows, d);
+        s.col_step(T.x_k, rows, learning_rate);                                                       // after its last use
+        s.ln_backward(AR, T1, T.ln2_w, T.ln2_b, GX, true, rows, d);
 
         // ---- ROSA: gradients stop at the q/k/v bits (src/model.rs:1494-1521)
         const uint32_t* idx = m->tape_idx[li].as<uint32_t>(1);
-        s.col_reduce(GX, nullptr, SM + 2 * d, rows, d, COL_SUM);                                      // g_bias
+        if (T.o.bias.w) {   // not used again in this step
+            s.col_gradient(GX, nullptr, rows, d, COL_SUM);
+            s.col_step(T.o.bias, rows, learning_rate);
+        }
         s.operands(GX, L.o.scale, A16, T16, rows, d, rows_p);
         s.unpack_transpose(L.o.bits, B16, d, d, d_p);
         s.gemm(A16, B16, T2, rows, d_p, d);                                                           // g_y
-        s.col_reduce(T2, idx, SM + 3 * d, rows, d, COL_BITS, time);                                   // g_e
+        s.col_gradient(T2, idx, rows, d, COL_BITS, time);                                             // g_e
         rt->chain(emit_transposed_kernel, dim3(blocks_for(rows_p, 8 * 128), (unsigned)d), 128, 0, idx, L.e, B16, (uint32_t)rows,
                   (uint32_t)d, (uint32_t)rows_p, (uint32_t)time);                                      // y = +/-e
         rt->launched("emit_transposed");
-        s.packed_update(T.o, T16, B16, rows_p, SM + 2 * d, learning_rate, CNT + 2, SM);
-        s.sgd(T.e, SM + 3 * d, learning_rate);
+        s.col_step(T.e, rows, learning_rate);                                                         // after its last use
+        s.packed_update(T.o, T16, B16, rows_p, CNT + 2, SM);
 
         if (li == 0) {   // ln0 replaced x on layer 0: its input is the embedded rows (src/model.rs:2972-2977)
             k::embed(rt, m->ids.as<uint32_t>(rows), m->embedding, T1, rows, d, vocab);
-            s.ln_backward(T1, GX, T.ln0_w, T.ln0_b, T2, false, SM, rows, d);
+            s.ln_backward(T1, GX, T.ln0_w, T.ln0_b, T2, false, rows, d);
             std::swap(GX, T2);
         }
     }
