@@ -245,10 +245,9 @@ ce_grad_kernel(float* __restrict__ logits, const uint32_t* __restrict__ labels, 
 //   COL_SHIFT  a * (b of the row before - b), 0 before the first row of a sequence
 //   COL_SIGN   b ? a : -a                                   b u8 [R, C]
 //   COL_BITS   the same, b stream-major bits
-// The sum of a column is a serial chain, but its terms are not: a CTA of eight warps brings 128 rows of 32 columns to shared
-// memory, 16 rows per warp with all their loads in flight, and one warp adds them up, a column per lane.  As one thread per
-// column that also did the loads, one per addition, 16 384 rows of 512 took 44 us, with the loads of 64 rows ahead of
-// their additions 12 (COL_SUM) to 54; so 10 to 23.
+// Bound by bringing the rows in: a warp has 16 rows of 32 columns on their way at a time, a column per lane, and adds up its own; the
+// eight sums of a CTA meet in shared memory.  (With the rows in shared memory and one warp that adds up 128 of them the chain was
+// what lasted: the 102 sums of two steps of 8 x 2048 tokens 2.23 ms between events, now 2.07.)
 enum ColMode { COL_SUM, COL_LN, COL_SHIFT, COL_SIGN, COL_BITS };
 constexpr int COL_ROWS = 256, COL_STEP = 128, COL_WARP_ROWS = COL_STEP / 8;
 template <ColMode MODE>
@@ -257,11 +256,11 @@ col_partial_kernel(const float* __restrict__ a, const void* __restrict__ b, cons
                    float* __restrict__ part, uint32_t R, uint32_t C, uint32_t time) {
     chain_entry();
     constexpr bool PRODUCT = MODE == COL_LN || MODE == COL_SHIFT;
-    __shared__ float sa[COL_STEP][32], sb[PRODUCT ? COL_STEP : 1][32];
+    __shared__ float sums[2][8][32];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, c = blockIdx.x * 32u + lane;
     const uint32_t r0 = blockIdx.y * COL_ROWS, r1 = min(r0 + COL_ROWS, R);
     const float* b32 = static_cast<const float*>(b);
-    float acc = 0.0f;
+    float acc = 0.0f, plain = 0.0f;
     for (uint32_t h = r0; h < r1; h += COL_STEP) {
         const uint32_t rw = h + warp * COL_WARP_ROWS;
         float av[COL_WARP_ROWS] = {}, bv[COL_WARP_ROWS] = {};
@@ -312,27 +311,22 @@ col_partial_kernel(const float* __restrict__ a, const void* __restrict__ b, cons
                 }
             }
         }
-        if (h != r0) __syncthreads();                        // the rows before have been added up
 #pragma unroll
-        for (int i = 0; i < COL_WARP_ROWS; ++i) {
-            const bool negative = (MODE == COL_SIGN || MODE == COL_BITS) && bv[i] == 0.0f;
-            sa[warp * COL_WARP_ROWS + i][lane] = negative ? -av[i] : av[i];
-            if (PRODUCT) sb[PRODUCT ? warp * COL_WARP_ROWS + i : 0][lane] = bv[i];
-        }
-        __syncthreads();
-        const uint32_t n = min((uint32_t)COL_STEP, r1 - h);
-        if (warp == 0) {
-#pragma unroll 16
-            for (uint32_t j = 0; j < n; ++j) {
-                if (PRODUCT) acc += sa[j][lane] * sb[PRODUCT ? j : 0][lane];
-                else acc += sa[j][lane];
-            }
-        } else if (MODE == COL_LN && warp == 1) {
-#pragma unroll 16
-            for (uint32_t j = 0; j < n; ++j) acc += sa[j][lane];
+        for (int i = 0; i < COL_WARP_ROWS; ++i) {   // rows past the last are zeros
+            if (PRODUCT) acc += av[i] * bv[i];
+            else acc += (MODE == COL_SIGN || MODE == COL_BITS) && bv[i] == 0.0f ? -av[i] : av[i];
+            if (MODE == COL_LN) plain += av[i];
         }
     }
-    if (c < C && warp < (MODE == COL_LN ? 2u : 1u)) part[((size_t)warp * gridDim.y + blockIdx.y) * C + c] = acc;
+    sums[0][warp][lane] = acc;
+    if (MODE == COL_LN) sums[1][warp][lane] = plain;
+    __syncthreads();
+    if (c < C && warp < (MODE == COL_LN ? 2u : 1u)) {
+        float all = 0.0f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) all += sums[warp][w][lane];
+        part[((size_t)warp * gridDim.y + blockIdx.y) * C + c] = all;
+    }
 }
 
 // Fp16Storage::apply_clipped_sgd (src/precision.rs:106-113) on g * gmul
