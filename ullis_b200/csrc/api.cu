@@ -178,18 +178,18 @@ void in_shares(ullis_cuda_runtime* rt, size_t shares, bool results_locked, In co
     ULLIS_CUDA_CHECK(cudaStreamWaitEvent(rt->stream, rt->copies_done, 0));
 }
 // Shares of a call: up to four, each with results of 4 MiB at least (about 80 us on the link, where a share costs its launches) and `least`
-// of the `items` that it is cut by; the first one in two halves, where they have as much, since nothing comes back before it is computed.
+// of the `items` that it is cut by; a half one at either end, where it has `least` too, since nothing comes back before the first one is
+// computed and nothing goes out beside the results of the last.
 // A call whose kernels are timed goes in one piece: a bracket of events around a share's kernel would hold the wait for its input, and the
 // copies beside it.
 struct Shares {
     size_t n, items, whole;   // whole: as many as there would be without the halves
     Shares(const ullis_cuda_runtime* rt, size_t result_bytes, size_t items_, size_t least) : items(items_) {
-        least = std::max<size_t>(least, 1);
         whole = rt->kernel_timing ? 1 : std::max<size_t>(1, std::min({ullis_cuda_runtime::MAX_SHARES - 1, result_bytes >> 22, items / least}));
-        n = whole > 1 && items / (2 * whole) >= std::max<size_t>(least / 2, 1) ? whole + 1 : whole;
+        n = whole > 1 && items / (2 * whole) >= least ? whole + 1 : whole;
     }
     size_t first(size_t s) const {   // 0 <= s <= n
-        return n == whole ? items * s / n : items * (s <= 1 ? s : 2 * (s - 1)) / (2 * whole);
+        return n == whole ? items * s / n : s == 0 ? 0 : s == n ? items : items * (2 * s - 1) / (2 * whole);
     }
 };
 bool page_locked(const void* p) {
@@ -1053,7 +1053,7 @@ int32_t ullis_cuda_binary_linear(ullis_cuda_runtime* rt, const float* x, const u
         if (rows == 0) return;
         need_ptr(x, "x"); need_ptr(bits, "bits"); need_ptr(scale, "scale"); need_ptr(y, "y");
         // whole 256-row tiles in every share but the last
-        const Shares split(rt, ny * 4, (rows + 255) / 256, 2);
+        const Shares split(rt, ny * 4, (rows + 255) / 256, 1);
         const size_t shares = split.n;
         Inputs in(rt);
         float* dx = shares > 1 ? rt->pool[0].as<float>(nx) : in.add(0, x, nx);
