@@ -1,4 +1,4 @@
-"""The latest positions of contexts (rosa_heads_kernel) against the oracle's pushes: rows that are not whole, streams in one, two and
+"""The latest positions of contexts (the first launch of the contexts) against the oracle's pushes: rows that are not whole, streams in one, two and
 four pieces, pieces that end past the last row, and streams that have to be given up beside even ones."""
 import numpy as np
 import pytest
@@ -27,5 +27,5 @@ def test_even_streams_beside_others(cuda_rt, oracle, T, B, C, odd):
     idx, _ = cuda_rt.rosa_qkv_1bit_fwd(q, k, v, np.zeros(C, np.uint16), B, T, C)
     ran = cuda_rt.kernel_times()
     cuda_rt.kernel_timing(False)
-    assert "rosa_heads" in ran
+    assert "rosa_context_left" in ran
     assert np.array_equal(idx, oracle.rosa_qkv_batch_packed(q, k, v, B, T, C))

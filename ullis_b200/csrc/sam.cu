@@ -1115,8 +1115,8 @@ void contexts(ullis_cuda_runtime* rt, const MatchCall& m) {
         else launch_context<1024, true>(rt, m, shape, form, list, count, from, to, what);
     };
     if (m.form == LATEST_TOO) {
-        launch(uneven, m.form, m.list, m.counts, 0u, half, "rosa_heads");
-        launch(uneven, IN_PARTS, m.left, m.counts + 5, 1u, all, "rosa_context");
+        launch(uneven, m.form, m.list, m.counts, 0u, half, "rosa_context");
+        launch(uneven, IN_PARTS, m.left, m.counts + 5, 1u, all, "rosa_context_left");
         return;
     }
     launch(uneven, m.form, m.list, m.counts, 0u, half, "rosa_context");
