@@ -210,6 +210,14 @@ void ullis_cuda_generate_state::prepare_one_kernel() {
     // One round of clusters if there is a way, with as many CTAs per cluster as have 32 channels each (a CTA's share of the
     // sums is shortest then) and as few sequences per cluster as the clusters that the device holds at once allow.
     constexpr size_t MOST_SMEM = 224 * 1024;
+    const auto prepare = [&](const void* kernel) {
+        ULLIS_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MOST_SMEM));
+        ULLIS_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    };
+    // All forms have an SM to themselves by their registers, so one of them tells how many clusters there is room for (a form that is asked
+    // for is loaded, 3 ms each).
+    const void* any_form = kernel_for(1, 32);
+    prepare(any_form);
     size_t best_rounds = SIZE_MAX;
     for (uint32_t c = gen::MAX_CLUSTER; c >= 1 && best_rounds > 1; c /= 2) {
         if (m->d % (c * 32) || m->ffn % (c * 4)) continue;
@@ -223,22 +231,21 @@ void ullis_cuda_generate_state::prepare_one_kernel() {
             }
             const size_t smem = gen::Layout(g, (uint32_t)m->d, (uint32_t)m->ffn, c, stages, staged).total, want = (batch + g - 1) / g;
             if (smem > MOST_SMEM || stages > gen::MAX_STAGES) break;
-            const void* kernel = kernel_for(g, (uint32_t)m->d / c);
-            ULLIS_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MOST_SMEM));
-            ULLIS_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
             cudaLaunchAttribute attr;
             const cudaLaunchConfig_t cfg = step_config(&attr, c, c, smem);
             int clusters = 0;
-            ULLIS_CUDA_CHECK(cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg));
+            ULLIS_CUDA_CHECK(cudaOccupancyMaxActiveClusters(&clusters, any_form, &cfg));
             if (clusters < 1) break;
             const size_t rounds = (want + clusters - 1) / clusters;
             if (rounds >= best_rounds) continue;
             best_rounds = rounds;
-            cluster = c; group = g; step_stages = stages; step_staged = staged; step_kernel = kernel; step_smem = smem;
+            cluster = c; group = g; step_stages = stages; step_staged = staged; step_smem = smem;
             step_grid = (unsigned)(std::min<size_t>(want, (size_t)clusters) * c);
         }
     }
     if (!step_grid) return;
+    step_kernel = kernel_for(group, (uint32_t)m->d / cluster);
+    prepare(step_kernel);
     std::vector<gen::Layer> layers(m->layers);
     for (size_t l = 0; l < m->layers; ++l) {
         const LayerWeights& L = m->blocks[l];

@@ -352,7 +352,7 @@ struct ContextLimits {
 // Where less than half of the CTAs would have a stream, two or more take one: each sorts all of its keys and answers its share of the
 // steps (one sequence of the default model with gain N(0, 0.02), 64 of 512 streams listed, 148 CTAs: the slowest stream 130 000 cycles,
 // 22 000 of them for the sort).
-constexpr uint32_t MAX_PARTS = 4, PARTS_MAX_STREAMS = 8;
+constexpr uint32_t MAX_PARTS = 4, PARTS_MAX_STREAMS = 4;   // per SM: of more hardly ever so few are listed, and the form costs the others 3 %
 constexpr uint32_t CONTEXT_LARGE = 48;   // positions before a step in its buckets from which on the whole warp looks through them
 
 struct ContextLayout {   // bytes of shared memory
