@@ -347,6 +347,8 @@ __device__ __forceinline__ bool exact_mixed_sign(const float* __restrict__ xr, b
 // listed the entries, one that read both rows of each anew for its warp, 4 KB per entry through L2, and one that left at once 179,
 // so 110.  The whole call: 64 sequences 26 860 -> 26 080, 16 in training 11 540 -> 11 370, 5 x 1531 3 697 -> 3 607, one
 // 2 215 -> 2 183.
+// Whole rows at once where a CTA has few steps, without the waits in between, took the kernel from 12.7 to 11.4 us a layer by itself and one
+// sequence from 1 817 to 1 844 us.
 // Any number of flags: what the queue does not hold waits in its finder's registers.
 constexpr uint32_t FIXB_COLS = 64, FIXB_PITCH = FIXB_COLS + 4, FIXB_ROWS = 33, FIXB_QUEUE = 512, FIXB_WORDS = 8, FIXB_MAX_THREADS = 160;
 // Threads per CTA: a third more than there are entries on average, so that hardly a block needs a second round; at most
