@@ -5,10 +5,9 @@
 #include <cstdio>
 #include <cstring>
 #include <exception>
-#include <map>
-#include <mutex>
 #include <new>
 
+#include "host_blocks.hpp"
 #include "kernels.hpp"
 #include "linear_tc.hpp"
 #include "generate.hpp"
@@ -103,17 +102,6 @@ struct Inputs {
     }
 };
 
-// The blocks of ullis_cuda_host_alloc: what lies in one can be written by kernels of any device.
-struct HostBlocks {
-    std::mutex lock;
-    std::map<uintptr_t, size_t> sizes;
-    bool hold(const void* p, size_t bytes) {
-        std::lock_guard<std::mutex> held(lock);
-        const uintptr_t at = reinterpret_cast<uintptr_t>(p);
-        auto it = sizes.upper_bound(at);
-        return it != sizes.begin() && (--it, at - it->first + bytes <= it->second);
-    }
-};
 HostBlocks& host_blocks() {
     static HostBlocks* blocks = new HostBlocks;   // never gone: blocks may be freed while the process ends
     return *blocks;
@@ -627,17 +615,17 @@ int32_t ullis_cuda_host_alloc(ullis_cuda_runtime* rt, size_t bytes, void** out) 
             *out = nullptr;
             fail(ULLIS_CUDA_ERR_NOMEM, "page-locked host allocation failed");
         }
-        std::lock_guard<std::mutex> held(host_blocks().lock);
-        host_blocks().sizes[reinterpret_cast<uintptr_t>(*out)] = bytes ? bytes : 1;
+        if (!host_blocks().add(*out, bytes ? bytes : 1)) {
+            cudaFreeHost(*out);
+            *out = nullptr;
+            fail(ULLIS_CUDA_ERR_NOMEM, "no memory for the entry of a page-locked block");
+        }
     });
 }
 
 void ullis_cuda_host_free(void* block) {
     if (!block) return;
-    {
-        std::lock_guard<std::mutex> held(host_blocks().lock);
-        host_blocks().sizes.erase(reinterpret_cast<uintptr_t>(block));
-    }
+    host_blocks().remove(block);
     cudaFreeHost(block);
 }
 
