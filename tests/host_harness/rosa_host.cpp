@@ -173,3 +173,13 @@ extern "C" int rosa_host_batch(uint32_t way, const uint32_t* q, const uint32_t* 
     }
     return 0;
 }
+
+// The rows of each of the pieces that a stream of T steps is cut into where `wanted` are; returns how many there are.
+extern "C" uint32_t rosa_host_pieces(uint32_t T, uint32_t wanted, uint32_t* row0, uint32_t* row1) {
+    const uint32_t words = (T + 31u) / 32u, pieces = heads::pieces_with_rows(words, wanted), rows = heads::rows_of_piece(words, pieces);
+    for (uint32_t i = 0; i < pieces; ++i) {
+        row0[i] = i * rows < words ? i * rows : words;
+        row1[i] = row0[i] + rows < words ? row0[i] + rows : words;
+    }
+    return pieces;
+}

@@ -121,5 +121,10 @@ RC_HD uint32_t window_before(const uint32_t* W, uint32_t r1) {
 #endif
 }
 
+// A stream of `words` rows in pieces of equal length, the last one shorter; of the pieces that are wanted as many as have a row
+// (a piece without any would put in all keys of the stream and answer nothing: 33 steps in four pieces have two such).
+constexpr uint32_t rows_of_piece(uint32_t words, uint32_t pieces) { return (words + pieces - 1u) / pieces; }
+constexpr uint32_t pieces_with_rows(uint32_t words, uint32_t wanted) { return rows_of_piece(words, rows_of_piece(words, wanted)); }
+
 }  // namespace heads
 }  // namespace ullis

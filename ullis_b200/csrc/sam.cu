@@ -423,7 +423,7 @@ __device__ __forceinline__ void heads_streams(const uint32_t* __restrict__ q_sw,
     uint32_t* V = reinterpret_cast<uint32_t*>(mem + L.v);
     if (warp >= call.warps) return;
     const uint32_t pieces = call.pieces, warps = gridDim.x * call.warps, above = ALL << lane << 1, below = (1u << lane) - 1u;
-    const uint32_t piece_rows = (words + pieces - 1u) / pieces;
+    const uint32_t piece_rows = heads::rows_of_piece(words, pieces);
     auto keys_in = [&](uint32_t row, uint32_t wk) {
         const uint32_t r1 = 32u * row + lane + 1u, ctx = wk >> 21;
         uint32_t before = latest_11[ctx];
@@ -1015,7 +1015,8 @@ void launch_context(ullis_cuda_runtime* rt, const MatchCall& m, int shape, Conte
         // 0.235 / 0.236; 2048 steps of the default model: 4 sequences 2.90 / 2.45 / 2.10, 8 3.71 / 3.11 / 2.99, 16 5.09 / 4.75 / 4.97, 64 14.0 /
         // 14.4 / 16.7).
         const size_t warps = (size_t)rt->context_ctas[shape] * heads.warps;
-        heads.pieces = m.T < 1024u ? (m.streams * 4u <= warps ? 4u : 1u) : m.streams * 2u < 3u * warps ? 4u : m.streams < 8u * warps ? 2u : 1u;
+        const uint32_t wanted = m.T < 1024u ? (m.streams * 4u <= warps ? 4u : 1u) : m.streams * 2u < 3u * warps ? 4u : m.streams < 8u * warps ? 2u : 1u;
+        heads.pieces = heads::pieces_with_rows((m.T + 31u) / 32u, wanted);
         // heads.base, heads.per_row: less leaves the contexts streams that are cheaper here (whole calls with 12 / 16 / 24 / 40 per row, ms:
         // 16 times 2048 steps 9.70 / 9.61 / 9.57 / 9.46, 16 times 1100 5.37 / 5.35 / 5.25 / 5.13, 5 times 1531 3.38 / 3.36 / 3.36 / 3.31), and a base
         // too small all that are short (ROSA kernels of twice 700 steps, base 32 / 64 / 128: 0.75 / 0.62 / 0.61).
