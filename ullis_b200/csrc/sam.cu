@@ -952,6 +952,7 @@ rosa_match_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restrict_
     }
 }
 
+constexpr uint32_t LEFT_PER_SM = 6;   // streams, beyond which they are many (`contexts`)
 constexpr size_t MATCH_MAX_TIME = 8192;   // 256 words of lags, eight per lane
 constexpr uint32_t HEADS_MAX_TIME = 2048;
 constexpr size_t SM_SMEM = 228 * 1024, CTA_SMEM = 1536;   // of an SM; what a CTA needs beside its dynamic part, reserved and static
@@ -1116,8 +1117,13 @@ void contexts(ullis_cuda_runtime* rt, const MatchCall& m) {
         else launch_context<1024, true>(rt, m, shape, form, list, count, from, to, what);
     };
     if (m.form == LATEST_TOO) {
+        // What the latest positions leave: few streams in parts, many of them in the shape of many, from where `rest` has that one.  In one launch,
+        // in parts, many took twice the time (all of 2560 streams of 2048 steps left, bits of probability 0.9 1208 / 704 us, of clean periods
+        // 928 / 254, 8192 of them 3281 / 2093 and 1315 / 670); a launch that leaves at once costs 1.5 us a layer.
+        const uint32_t many_left = rest == uneven ? all : LEFT_PER_SM * (uint32_t)sms + 1u;
         launch(uneven, m.form, m.list, m.counts, 0u, half, "rosa_context");
-        launch(uneven, IN_PARTS, m.left, m.counts + 5, 1u, all, "rosa_context_left");
+        launch(uneven, IN_PARTS, m.left, m.counts + 5, 1u, many_left, "rosa_context_left");
+        if (many_left != all) launch(rest, PLAIN, m.left, m.counts + 5, many_left, all, "rosa_context_left_many");
         return;
     }
     launch(uneven, m.form, m.list, m.counts, 0u, half, "rosa_context");
