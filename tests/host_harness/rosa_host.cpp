@@ -183,3 +183,14 @@ extern "C" uint32_t rosa_host_pieces(uint32_t T, uint32_t wanted, uint32_t* row0
     }
     return pieces;
 }
+
+// What the warp of a piece asks before it puts any key in: whether the runs of the first `rows` rows alone make its walks too long.
+extern "C" int rosa_host_runs_too_long(const uint32_t* q, const uint32_t* k, uint32_t rows, uint32_t most) {
+    uint32_t keys[2] = {0, 0}, in[2] = {0, 0};
+    for (uint32_t w = 0; w < rows; ++w)
+        for (uint32_t z = 0; z < 2u; ++z) {
+            keys[z] += (uint32_t)__builtin_popcount(heads::ends_of_runs(z ? ~k[w] : k[w]));
+            in[z] += heads::ends_of_runs(z ? ~q[w] : q[w]) != 0u;
+        }
+    return heads::walks_too_long(keys[0], in[0], most) || heads::walks_too_long(keys[1], in[1], most);
+}

@@ -121,6 +121,17 @@ RC_HD uint32_t window_before(const uint32_t* W, uint32_t r1) {
 #endif
 }
 
+// The positions of a word that end a run of DEPTH ones inside it.
+RC_HD uint32_t ends_of_runs(uint32_t x) {
+    x &= x << 1;
+    x &= x << 2;
+    x &= x << 4;
+    return x & x << 3;   // 8 and 3
+}
+// Whether the walks of rows with queries in the one context of such a run, `rows` of them, come to more than `most` positions if
+// `keys` positions are in it: on average half of those lie before a row.
+RC_HD bool walks_too_long(uint32_t keys, uint32_t rows, uint32_t most) { return keys * rows > 2u * most; }
+
 // A stream of `words` rows in pieces of equal length, the last one shorter; of the pieces that are wanted as many as have a row
 // (a piece without any would put in all keys of the stream and answer nothing: 33 steps in four pieces have two such).
 constexpr uint32_t rows_of_piece(uint32_t words, uint32_t pieces) { return (words + pieces - 1u) / pieces; }

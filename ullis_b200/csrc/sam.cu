@@ -402,6 +402,14 @@ struct HeadsCall {
     uint32_t *next, *left, *left_count, *given_up;
 };
 
+// A piece is left out, or its walk broken off, when another one has given the stream up; and a stream whose runs alone make its walks too long,
+// `base` + RUNS_PER_ROW positions per row, is given up before its keys are put in.  (Without either every piece of an uneven stream spent its
+// own `base` and more.  us of the ROSA kernels, contexts alone / before / now: 16 x 2048 steps x 512 channels, bits of probability 0.9 2112 / 2340 /
+// 2135, of slow changes 1099 / 1302 / 1127, of clean periods 1343 / 1650 / 1509; 5 x 2048 725 / 877 / 741, 401 / 553 / 418, 492 / 661 / 612; 4 x 700
+// 171 / 286 / 180, 139 / 232 / 150, 260 / 277 / 279.  Whole calls in training: 16 x 2048 9.43 / 9.46 ms, 5 x 1531 3.25 / 3.25, 16 x 700 3.88 / 3.91.  With
+// 12 per row more of those are given up, 24 leaves 4 x 700 of probability 0.9 at 277.)
+constexpr uint32_t RUNS_PER_ROW = 16;
+
 // Bound by the integer pipe: per row of 32 steps of the model's streams (2048 steps) about 350 warp instructions, 215 of them on
 // that pipe, which takes one every second cycle - the refinement of the masks 100, the look-ups 70, the walk over the
 // chains 70, the keys 40.  rosa_context_kernel sorts each stream first and compares what lies in a bucket: 750 per row.  Both kernels
@@ -440,19 +448,41 @@ __device__ __forceinline__ void heads_streams(const uint32_t* __restrict__ q_sw,
         link[r1] = (uint16_t)before;
         __syncwarp();
     };
+    auto give_up = [&](size_t s) {
+        if (lane == 0u && atomicExch(&call.given_up[s], 1u) == 0u) call.left[atomicAdd(call.left_count, 1u)] = (uint32_t)s;
+    };
     // The last pieces first, which have the most keys to put in.
     for (uint32_t item = warp * gridDim.x + blockIdx.x; item < total * pieces;
          item = warps + __shfl_sync(ALL, lane == 0u ? atomicAdd(call.next, 1u) : 0u, 0)) {
         const uint32_t piece = pieces - 1u - item / total;
         const size_t s = list[item % total], at = s * wps;
         const uint32_t row0 = min(piece * piece_rows, words), row1 = min(row0 + piece_rows, words);
+        const uint32_t by_other = pieces > 1u && lane == 0u ? __ldcg(&call.given_up[s]) : 0u;
+        const uint32_t most_along_runs = call.base + RUNS_PER_ROW * row1;
+        uint32_t keys = 0;   // positions in runs of ones, and of zeros << 16
         __syncwarp();
         for (uint32_t w = lane; w < row1; w += 32u) {
+            const uint32_t key = k_sw[at + w];
             Q[w + 1u] = q_sw[at + w];
-            K[w + 1u] = k_sw[at + w];
+            K[w + 1u] = key;
             V[w] = v_sw[at + w];
+            keys += (uint32_t)__popc(heads::ends_of_runs(key)) + ((uint32_t)__popc(heads::ends_of_runs(~key)) << 16);
         }
         if (lane == 0u) Q[0] = K[0] = 0u;
+        if (__any_sync(ALL, by_other)) continue;
+        keys = __reduce_add_sync(ALL, keys);
+        if (__any_sync(ALL, heads::walks_too_long(max(keys & 0xFFFFu, keys >> 16), row1, most_along_runs))) {
+            uint32_t rows = 0;   // with a query in a run of ones, and of zeros << 16
+            for (uint32_t w = lane; w < row1; w += 32u) {
+                const uint32_t query = Q[w + 1u];
+                rows += (heads::ends_of_runs(query) ? 1u : 0u) + (heads::ends_of_runs(~query) ? 0x10000u : 0u);
+            }
+            rows = __reduce_add_sync(ALL, rows);
+            if (__any_sync(ALL, heads::walks_too_long(keys & 0xFFFFu, rows & 0xFFFFu, most_along_runs) || heads::walks_too_long(keys >> 16, rows >> 16, most_along_runs))) {
+                give_up(s);
+                continue;
+            }
+        }
         for (uint32_t i = lane; i < L.link / 16u; i += 32u) reinterpret_cast<uint4*>(mem)[i] = uint4{0u, 0u, 0u, 0u};
         __syncwarp();
         uint32_t k0 = 0u, q0 = Q[row0], work = 0;
@@ -492,10 +522,11 @@ __device__ __forceinline__ void heads_streams(const uint32_t* __restrict__ q_sw,
             walked = __reduce_max_sync(ALL, walked);
             work += walked;
             gone = walked > most;
+            if (walked > call.per_row && pieces > 1u) gone |= __any_sync(ALL, lane == 0u && __ldcg(&call.given_up[s]));
             const uint32_t word = __ballot_sync(ALL, r1 && t < T && (V[r1 >> 5] >> (r1 & 31u) & 1u));
             if (lane == 0u) idx_sw[at + row] = word;
         }
-        if (gone && lane == 0u && atomicExch(&call.given_up[s], 1u) == 0u) call.left[atomicAdd(call.left_count, 1u)] = (uint32_t)s;
+        if (gone) give_up(s);
     }
 }
 
