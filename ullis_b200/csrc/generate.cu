@@ -23,6 +23,7 @@
 #include <string>
 #include <vector>
 
+#include "generate_plan.hpp"
 #include "generate_step.cuh"
 #include "kernels.hpp"
 #include "linear_tc.hpp"
@@ -207,45 +208,42 @@ void ullis_cuda_generate_state::prepare_one_kernel() {
         return g == 2 ? ULLIS_STEP_OF(2) : ULLIS_STEP_OF(4);
 #undef ULLIS_STEP_OF
     };
-    // One round of clusters if there is a way, with as many CTAs per cluster as have 32 channels each (a CTA's share of the
-    // sums is shortest then) and as few sequences per cluster as the clusters that the device holds at once allow.
     constexpr size_t MOST_SMEM = 224 * 1024;
     const auto prepare = [&](const void* kernel) {
         ULLIS_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MOST_SMEM));
         ULLIS_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     };
-    // All forms have an SM to themselves by their registers, so one of them tells how many clusters there is room for (a form that is asked
-    // for is loaded, 3 ms each).
+    const auto room = [&](const void* kernel, const gen::StepPlan& p) {
+        cudaLaunchAttribute attr;
+        const cudaLaunchConfig_t cfg = step_config(&attr, p.cluster, p.cluster, p.smem);
+        int clusters = 0;
+        ULLIS_CUDA_CHECK(cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg));
+        return clusters;
+    };
+    const uint32_t d = (uint32_t)m->d, ffn = (uint32_t)m->ffn;
+    const auto fit = [&](gen::StepPlan& p) {   // packed weights stay where they are if there is no room for them beside the ring
+        for (const bool staged : {true, false}) {
+            p.staged = staged;
+            p.stages = gen::ring_stages(p.group, d, ffn, p.cluster, staged, MOST_SMEM);
+            p.smem = gen::Layout(p.group, d, ffn, p.cluster, p.stages, staged).total;
+            if (p.smem <= MOST_SMEM) break;
+        }
+        return p.smem <= MOST_SMEM && p.stages <= gen::MAX_STAGES;
+    };
+    // All forms have an SM to themselves by their registers, so any of them tells how much room there is (a form is loaded when it is asked for, 3 ms
+    // each); the one that is taken is asked too.
     const void* any_form = kernel_for(1, 32);
     prepare(any_form);
-    size_t best_rounds = SIZE_MAX;
-    for (uint32_t c = gen::MAX_CLUSTER; c >= 1 && best_rounds > 1; c /= 2) {
-        if (m->d % (c * 32) || m->ffn % (c * 4)) continue;
-        for (uint32_t g = 1; g <= gen::MAX_GROUP && best_rounds > 1; g *= 2) {
-            // packed weights stay where they are if there is no room for them beside the ring
-            bool staged = true;
-            uint32_t stages = gen::ring_stages(g, (uint32_t)m->d, (uint32_t)m->ffn, c, true, MOST_SMEM);
-            if (gen::Layout(g, (uint32_t)m->d, (uint32_t)m->ffn, c, stages, true).total > MOST_SMEM) {
-                staged = false;
-                stages = gen::ring_stages(g, (uint32_t)m->d, (uint32_t)m->ffn, c, false, MOST_SMEM);
-            }
-            const size_t smem = gen::Layout(g, (uint32_t)m->d, (uint32_t)m->ffn, c, stages, staged).total, want = (batch + g - 1) / g;
-            if (smem > MOST_SMEM || stages > gen::MAX_STAGES) break;
-            cudaLaunchAttribute attr;
-            const cudaLaunchConfig_t cfg = step_config(&attr, c, c, smem);
-            int clusters = 0;
-            ULLIS_CUDA_CHECK(cudaOccupancyMaxActiveClusters(&clusters, any_form, &cfg));
-            if (clusters < 1) break;
-            const size_t rounds = (want + clusters - 1) / clusters;
-            if (rounds >= best_rounds) continue;
-            best_rounds = rounds;
-            cluster = c; group = g; step_stages = stages; step_staged = staged; step_smem = smem;
-            step_grid = (unsigned)(std::min<size_t>(want, (size_t)clusters) * c);
-        }
-    }
-    if (!step_grid) return;
-    step_kernel = kernel_for(group, (uint32_t)m->d / cluster);
-    prepare(step_kernel);
+    const gen::StepPlan plan = gen::plan_step(
+        batch, gen::MAX_CLUSTER, gen::MAX_GROUP, [&](uint32_t c) { return d % (c * 32) == 0 && ffn % (c * 4) == 0; }, fit,
+        [&](const gen::StepPlan& p) { return room(any_form, p); },
+        [&](const gen::StepPlan& p) {
+            step_kernel = kernel_for(p.group, d / p.cluster);
+            prepare(step_kernel);
+            return room(step_kernel, p);
+        });
+    if (!plan.grid) return;
+    cluster = plan.cluster; group = plan.group; step_stages = plan.stages; step_staged = plan.staged; step_smem = plan.smem; step_grid = plan.grid;
     std::vector<gen::Layer> layers(m->layers);
     for (size_t l = 0; l < m->layers; ++l) {
         const LayerWeights& L = m->blocks[l];
