@@ -683,7 +683,7 @@ bool usable(ullis_cuda_runtime* rt) {
             ULLIS_SET_SMEM_NARROW(EPI_RESIDUAL, true);
             ULLIS_SET_SMEM_NARROW(EPI_RESIDUAL, false);
             ULLIS_SET_SMEM_NARROW(EPI_RELU2, true);
-            ULLIS_SET_SMEM_NARROW(EPI_SIGNBITS, true);
+            ULLIS_CUDA_CHECK(cudaFuncSetAttribute(gemm_kernel<EPI_SIGNBITS, true, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
 #undef ULLIS_SET_SMEM_NARROW
             ULLIS_SET_SMEM(EPI_SIGNBITS, true);
             ULLIS_SET_SMEM(EPI_CE, true);
@@ -822,8 +822,10 @@ void launch(ullis_cuda_runtime* rt, const GemmMaps& maps, const GemmParams& p, u
             const dim3 grid((p.N + p.columns - 1) / p.columns, (p.M + BM - 1) / BM, n_prob);
             q.stages = stages_for(rt, p, (size_t)grid.x * grid.y * grid.z);
             const size_t smem = gemm_smem_bytes(q.n_a, q.stages, q.columns);
-            if (p.columns == 64) rt->chain(gemm_kernel<EPI, PACKED, 64>, grid, GEMM_THREADS, smem, maps, q);
-            else rt->chain(gemm_kernel<EPI, PACKED, 32>, grid, GEMM_THREADS, smem, maps, q);
+            auto kernel = gemm_kernel<EPI, PACKED, 32>;
+            if constexpr (EPI != EPI_SIGNBITS)   // 128 or 32 (rosa_qkv_bits)
+                if (p.columns == 64) kernel = gemm_kernel<EPI, PACKED, 64>;
+            rt->chain(kernel, grid, GEMM_THREADS, smem, maps, q);
             rt->launched(what);
             return;
         }
