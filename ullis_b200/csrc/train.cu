@@ -1112,7 +1112,7 @@ void ullis_cuda_train_state::step(const uint32_t* tokens, const uint32_t* labels
     uint16_t* A16 = a16.as<uint16_t>(rows * widest);
     uint16_t* B16 = b16.as<uint16_t>(std::max(d * rows_p, widest * std::max(f, d)));
     uint16_t* T16 = t16.as<uint16_t>(std::max(vocab, d + 2 * f) * rows_p);
-    float* SM = small.as<float>(4 * std::max({f, vocab, d}));
+    float* SM = small.as<float>(std::max({f, vocab, d}));   // gradients of a packed matrix's scales
     unsigned long long* CNT = counters.as<unsigned long long>(3);
     const uint32_t* lab = m->labels.as<uint32_t>(rows);
     float* RL = m->row_loss.as<float>(rows);
