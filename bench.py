@@ -85,11 +85,11 @@ def measured_peak_gbs():
         return 6650.0, "fallback"
 
 
-def profiled_traffic(kernel: str):
-    """DRAM bytes per launch of `kernel` from the committed ncu summary, if any."""
+def profiled_traffic(kernel: str, weights: str):
+    """DRAM bytes per launch of `kernel` with these weights from the committed ncu summary, if any."""
     try:
         with open(os.path.join(ROOT, "profiles", "roofline_traffic.json")) as f:
-            return json.load(f).get(kernel)
+            return json.load(f).get(weights, {}).get(kernel)
     except Exception:  # noqa: BLE001
         return None
 
@@ -510,7 +510,7 @@ def run_cuda(args):
             "gpu_launches": int(launches),
             "clocks": clocks,
             "roofline": {"kernel": dominant, "bound": "hbm", "achieved": achieved, "peak": peak,
-                         "unit": "GB/s", "frac": achieved / peak, "traffic": profiled_traffic(dominant),
+                         "unit": "GB/s", "frac": achieved / peak, "traffic": profiled_traffic(dominant, "gain_one" if args.ln_gain_one else "gain_0.02"),
                          "peak_source": peak_kind, "launch_ms": dom_ms, "leading_kernel": leader,
                          "algorithmic_bytes_per_launch": alg_bytes,
                          "rosa_kernels_ms_per_layer": rosa_ms,
