@@ -230,8 +230,13 @@ void ullis_cuda_generate_state::prepare_one_kernel() {
         }
         return p.smem <= MOST_SMEM && p.stages <= gen::MAX_STAGES;
     };
-    // All forms have an SM to themselves by their registers, so any of them tells how much room there is (a form is loaded when it is asked for, 3 ms
-    // each); the one that is taken is asked too.
+    // An SM holds one CTA of any form, by its registers, so any of them tells how much room there is (a form is loaded when it is asked for, 3 ms
+    // each, and the question takes 0.1 ms more); the one that is taken is asked where that does not hold.
+    const auto alone = [&](const void* kernel) {
+        cudaFuncAttributes attr;
+        ULLIS_CUDA_CHECK(cudaFuncGetAttributes(&attr, kernel));
+        return (size_t)attr.numRegs * gen::THREADS * 2 > 64 * 1024;
+    };
     const void* any_form = kernel_for(1, 32);
     prepare(any_form);
     const gen::StepPlan plan = gen::plan_step(
@@ -240,7 +245,7 @@ void ullis_cuda_generate_state::prepare_one_kernel() {
         [&](const gen::StepPlan& p) {
             step_kernel = kernel_for(p.group, d / p.cluster);
             prepare(step_kernel);
-            return room(step_kernel, p);
+            return alone(any_form) && alone(step_kernel) ? p.clusters : room(step_kernel, p);
         });
     if (!plan.grid) return;
     cluster = plan.cluster; group = plan.group; step_stages = plan.stages; step_staged = plan.staged; step_smem = plan.smem; step_grid = plan.grid;

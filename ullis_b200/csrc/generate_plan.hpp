@@ -11,6 +11,7 @@ struct StepPlan {
     uint32_t cluster = 0, group = 1, stages = 0;   // CTAs of a cluster, its sequences, pieces of the value weights in flight
     bool staged = false;                           // packed weights through shared memory
     size_t smem = 0;
+    int clusters = 0;                              // the device holds at once
     unsigned grid = 0;                             // 0: the step does not run as one kernel
 };
 
@@ -19,7 +20,8 @@ struct StepPlan {
 //   divides(cluster): whether channels and hidden units come out even
 //   fit(plan): sets stages, staged and smem for its cluster and group; false: no room
 //   room(plan): clusters the device holds at once, by any form of the kernel that is at hand
-//   room_of(plan): the same by the form that the plan takes; asked once, since a form that is asked for is loaded
+//   room_of(plan): the same by the form that the plan takes, whose `clusters` are those of `room`; asked once, since a form that is asked for
+//     is loaded
 template <typename Divides, typename Fit, typename Room, typename RoomOf>
 StepPlan plan_step(size_t batch, uint32_t max_cluster, uint32_t max_group, Divides divides, Fit fit, Room room, RoomOf room_of) {
     StepPlan best;
@@ -31,9 +33,9 @@ StepPlan plan_step(size_t batch, uint32_t max_cluster, uint32_t max_group, Divid
             p.cluster = c;
             p.group = g;
             if (!fit(p)) break;
-            const int clusters = room(p);
-            if (clusters < 1) break;
-            const size_t rounds = ((batch + g - 1) / g + clusters - 1) / clusters;
+            p.clusters = room(p);
+            if (p.clusters < 1) break;
+            const size_t rounds = ((batch + g - 1) / g + p.clusters - 1) / p.clusters;
             if (rounds >= best_rounds) continue;
             best_rounds = rounds;
             best = p;
@@ -41,8 +43,8 @@ StepPlan plan_step(size_t batch, uint32_t max_cluster, uint32_t max_group, Divid
     }
     if (!best.cluster) return best;
     // The forms differ in registers: a grid of more clusters than this one has room for would run its last ones alone.
-    const int clusters = room_of(best);
-    if (clusters >= 1) best.grid = (unsigned)(std::min<size_t>((batch + best.group - 1) / best.group, (size_t)clusters) * best.cluster);
+    best.clusters = room_of(best);
+    if (best.clusters >= 1) best.grid = (unsigned)(std::min<size_t>((batch + best.group - 1) / best.group, (size_t)best.clusters) * best.cluster);
     return best;
 }
 
