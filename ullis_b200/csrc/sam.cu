@@ -5,9 +5,9 @@
 // Up to 8192 steps a stream needs no automaton (rosa_match below): every step
 // is looked up by itself (rosa_heads.cuh, rosa_context.cuh) or in sets of lags
 // (rosa_match.cuh), so no launch lasts as long as a stream's chain of steps.
-// 64 sequences x 512 channels x 2048 steps: 1.5 ms on evenly spread bits where
-// the automaton took 11.3, 0.79 against 2.10 per layer of the benchmark model;
-// 1 sequence 0.105 against 0.62.
+// 64 sequences x 512 channels x 2048 steps: 0.85 ms on evenly spread bits where
+// the automaton took 11.3, 0.60 against 2.10 per layer of the benchmark model;
+// 1 sequence 0.07 against 0.62.
 //
 // Longer streams, and calls that ask for one of its forms, run the suffix
 // automaton: one thread per (sequence, channel) stream, automaton state in a
@@ -1122,6 +1122,9 @@ size_t stride_for(int algo, size_t T) {
 // threads: T = 1024, 2048 streams 47 / 49, 4096 68 / 70, 8192 100 / 121; T = 1531, 4096 112 / 109, 6144 129 / 144; T = 2048,
 // 4096 152 / 137, 6144 199 / 190, 8192 233 / 238; T = 4096, 8192 539 / 451.  Layers of the default model with gain N(0, 0.02),
 // 2048 steps: one sequence 1.20 / 0.79 ms, 4 1.41 / 1.00, 8 1.63 / 1.48, 12 1.99 / 1.96, 16 2.33 / 2.43, 64 6.94 / 8.31.
+//
+// (Where the latest positions take the calls with most streams listed - context_form - the columns of so many streams are those of what
+// they leave.)
 void contexts(ullis_cuda_runtime* rt, const MatchCall& m) {
     prepare_context<256, false>(rt, m.T, CONTEXT_256);
     prepare_context<512, true>(rt, m.T, CONTEXT_512);
@@ -1168,7 +1171,9 @@ ContextForm context_form(const ullis_cuda_runtime* rt, size_t streams, uint32_t 
     // gain 1 + N(0, 0.02), contexts / latest positions, ms; 2048 steps: two sequences of the default model 1.57 / 1.73, three 1.83 / 1.93, four
     // 2.18 / 2.05, eight 3.49 / 2.82, 64 21.7 / 13.1; 1100 steps: two 1.01 / 1.06, four 1.39 / 1.25; 700: one 0.58 / 0.69, two 0.81 / 0.62, 16 2.57 / 1.49;
     // 300: two 0.51 / 0.45, 64 5.88 / 1.98).  Where few are listed those are uneven, and their chains long: 64 times 2048 steps with gain
-    // N(0, 0.02) 7.7 / 9.3.  Beyond 2048 steps chains and tables grow (8192 steps of bits of probability 0.25 to 0.6: 1.09 / 1.63).
+    // N(0, 0.02) 7.7 / 9.3.  How uneven the listed ones are is not known here: a call of nothing but uneven streams takes 1 to 1.2 times as long as by
+    // contexts alone from 1024 steps on, 5 x 2048 of clean periods 608 / 496 us, and up to 1.9 times with few streams of few steps (4 x 300 slow
+    // changes 141 / 74, bits of probability 0.9 123 / 77).  Beyond 2048 steps chains and tables grow (8192 steps of bits of probability 0.25 to 0.6: 1.09 / 1.63).
     if (T <= HEADS_MAX_TIME && streams > (T < 512u ? 4u : T < 1024u ? 5u : 14u) * sms) return LATEST_TOO;
     // Only a call of few streams can list less than half as many as there are CTAs.
     return streams <= PARTS_MAX_STREAMS * sms ? IN_PARTS : PLAIN;
