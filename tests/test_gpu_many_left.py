@@ -37,3 +37,12 @@ def test_streams_that_are_left(cuda_rt, oracle, T, B, C, kind, share):
     assert 2 * cuda_rt.sam_counts()["automaton"] > B * C   # the listed streams: most, so the latest positions have run
     assert "rosa_context_left" in ran and ("rosa_context_left_many" in ran) == (T >= 700)
     assert np.array_equal(idx, oracle.rosa_qkv_batch_packed(*planes, B, T, C))
+
+
+@pytest.mark.parametrize("T,B,C", [(127, 4, 512), (128, 2, 320), (300, 4, 512), (511, 8, 512)])
+@pytest.mark.parametrize("kind,share", [("biased", 1.0), ("slow", 0.5), ("slow", 0.03)])
+def test_few_short_streams_of_which_some_are_uneven(cuda_rt, oracle, T, B, C, kind, share):
+    """More or fewer of them than the share from which on all streams go by contexts, and a length where they are not counted; two calls, since
+    the count of one must not be the next one's."""
+    test_streams_that_are_left(cuda_rt, oracle, T, B, C, kind, share)
+    test_streams_that_are_left(cuda_rt, oracle, T, B, C, "even", 0.0)

@@ -39,11 +39,16 @@ namespace {
 // consecutive bytes per request), the group combines by shuffle, and the closed forms - all of them word by
 // word - are written the same way.  One thread per stream spent its time in 3 x 64 dependent strided loads.
 constexpr int CLASSIFY_LANES = 8;
+// COUNT_UNEVEN: how many of the listed streams have walks of more than UNEVEN_PER_ROW positions per row along their runs alone
+// (rosa_heads.cuh; T <= 2048).
+constexpr uint32_t UNEVEN_PER_ROW = 10, UNEVEN_SHARE = 16;
+template <bool COUNT_UNEVEN>
 __global__ void __launch_bounds__(128)
 rosa_classify_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restrict__ k_sw,
                      const uint32_t* __restrict__ v_sw, uint32_t* __restrict__ idx_sw, size_t streams, uint32_t T,
                      size_t wps, uint32_t* __restrict__ list, uint32_t* __restrict__ count,
-                     uint32_t* __restrict__ cq_list, uint32_t* __restrict__ cq_count, uint32_t* __restrict__ given_up) {
+                     uint32_t* __restrict__ cq_list, uint32_t* __restrict__ cq_count, uint32_t* __restrict__ given_up,
+                     uint32_t* __restrict__ uneven_count) {
     chain_entry();
     constexpr uint32_t G = CLASSIFY_LANES;
     const size_t s = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
@@ -59,6 +64,7 @@ rosa_classify_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restri
     const uint32_t tail = (T & 31u) ? ((1u << (T & 31u)) - 1u) : 0xFFFFFFFFu;
     // AND and OR of the three streams over steps 0 .. T-1 (the bits past T in the last word count for neither)
     uint32_t all[3] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, any[3] = {0u, 0u, 0u};
+    uint32_t keys = 0, rows = 0;   // in runs of ones, and of zeros << 16: positions of keys, and words with a query
     for (uint32_t w = sub; w <= last; w += G) {
         const uint32_t m = w == last ? tail : 0xFFFFFFFFu;
         const uint32_t x[3] = {kw[w], vw[w], qw[w]};
@@ -67,6 +73,20 @@ rosa_classify_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restri
             all[a] &= x[a] | ~m;
             any[a] |= x[a] & m;
         }
+        if (COUNT_UNEVEN) {
+            keys += (uint32_t)__popc(heads::ends_of_runs(x[0] & m)) + ((uint32_t)__popc(heads::ends_of_runs(~x[0] & m)) << 16);
+            rows += (heads::ends_of_runs(x[2] & m) ? 1u : 0u) + (heads::ends_of_runs(~x[2] & m) ? 0x10000u : 0u);
+        }
+    }
+    bool uneven = false;
+    if (COUNT_UNEVEN) {
+#pragma unroll
+        for (uint32_t o = 1; o < G; o <<= 1) {
+            keys += __shfl_xor_sync(group, keys, o);
+            rows += __shfl_xor_sync(group, rows, o);
+        }
+        const uint32_t most = UNEVEN_PER_ROW * (last + 1u);
+        uneven = heads::walks_too_long(keys & 0xFFFFu, rows & 0xFFFFu, most) || heads::walks_too_long(keys >> 16, rows >> 16, most);
     }
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
@@ -118,7 +138,10 @@ rosa_classify_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restri
         }
     } else if (sub == 0) {
         if (constant(2, &c)) cq_list[atomicAdd(cq_count, 1u)] = (uint32_t)s;   // constant q: a long scan, its own kernel
-        else list[atomicAdd(count, 1u)] = (uint32_t)s;
+        else {
+            list[atomicAdd(count, 1u)] = (uint32_t)s;
+            if (COUNT_UNEVEN && uneven) atomicAdd(uneven_count, 1u);
+        }
     }
 }
 
@@ -400,6 +423,7 @@ struct HeadsCall {
     uint32_t warps;   // of a CTA that take pieces: as many as have room in its shared memory
     uint32_t pieces, base, per_row;
     uint32_t *next, *left, *left_count, *given_up;
+    const uint32_t* uneven_count;
 };
 
 // A piece is left out, or its walk broken off, when another one has given the stream up; and a stream whose runs alone make its walks too long,
@@ -567,11 +591,12 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
     const context::Runs runs{k_ends, in_word, before_word};
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t total = *count;
-    if (FORM == LATEST_TOO && total >= to) {
+    const bool contexts_for_all = FORM == LATEST_TOO && *heads_call.uneven_count * UNEVEN_SHARE > total;   // 0 where they were not counted
+    if (FORM == LATEST_TOO && total >= to && !contexts_for_all) {
         heads_streams(q_sw, k_sw, v_sw, idx_sw, list, total, T, wps, context_mem, heads_call);
         return;
     }
-    if (total < from || total >= to) return;
+    if (total < from || (total >= to && !contexts_for_all)) return;
     const uint32_t parts = FORM == IN_PARTS && total ? min(max(gridDim.x / total, 1u), MAX_PARTS) : 1u;
     const uint32_t rows_per_warp = (words + NW - 1u) / NW;
     const uint32_t row0 = min(warp * rows_per_warp, words), row1 = min(row0 + rows_per_warp, words);   // a warp's keys
@@ -896,7 +921,7 @@ rosa_context_kernel(const uint32_t* __restrict__ q_sw, const uint32_t* __restric
 // The remaining streams by sets of lags (rosa_match.cuh).  A work item is a piece of one stream, a warp takes items
 // from a counter until they run out; the warps of a CTA have nothing to do with one another.
 constexpr int MATCH_WARPS = 4;
-constexpr uint32_t MATCH_COUNTS = 7;   // of MatchCall
+constexpr uint32_t MATCH_COUNTS = 8;   // of MatchCall
 
 // A stream whose query bits are all c: idx follows the longest run of c among the keys so far, the latest of equals
 // (sam_core.cuh run_constant_q), a running maximum over (run length, position).  A lane has a word: the run that comes in from the words
@@ -991,8 +1016,8 @@ constexpr size_t SM_SMEM = 228 * 1024, CTA_SMEM = 1536;   // of an SM; what a CT
 struct MatchCall {   // the buffers of one call
     const uint32_t *q, *k, *v;
     uint32_t *idx, *list, *cq_list, *hard, *left, *given_up;
-    // listed, constant q, hard, next of the contexts, next of the matches, left by the latest positions, their next; those of the
-    // next call
+    // listed, constant q, hard, next of the contexts, next of the matches, left by the latest positions, their next, listed and uneven; those
+    // of the next call
     uint32_t *counts, *clear;
     size_t streams, wps;
     uint32_t T;
@@ -1032,7 +1057,7 @@ void launch_context(ullis_cuda_runtime* rt, const MatchCall& m, int shape, Conte
     // ever change went to the match kernel).
     const ContextLimits limits{24u, 96u, 160u, 64u, 256u};
     size_t smem = rt->context_smem[shape];
-    HeadsCall heads{0u, 1u, 128u, 40u, m.counts + 6, m.left, m.counts + 5, m.given_up};
+    HeadsCall heads{0u, 1u, 128u, 40u, m.counts + 6, m.left, m.counts + 5, m.given_up, m.counts + 7};
     auto kernel = rosa_context_kernel<NT, TOGETHER>;
     if (form == LATEST_TOO) {
         kernel = rosa_context_kernel<NT, TOGETHER, LATEST_TOO>;
@@ -1172,8 +1197,7 @@ ContextForm context_form(const ullis_cuda_runtime* rt, size_t streams, uint32_t 
     // 2.18 / 2.05, eight 3.49 / 2.82, 64 21.7 / 13.1; 1100 steps: two 1.01 / 1.06, four 1.39 / 1.25; 700: one 0.58 / 0.69, two 0.81 / 0.62, 16 2.57 / 1.49;
     // 300: two 0.51 / 0.45, 64 5.88 / 1.98).  Where few are listed those are uneven, and their chains long: 64 times 2048 steps with gain
     // N(0, 0.02) 7.7 / 9.3.  How uneven the listed ones are is not known here: a call of nothing but uneven streams takes 1 to 1.2 times as long as by
-    // contexts alone from 1024 steps on, 5 x 2048 of clean periods 608 / 496 us, and up to 1.9 times with few streams of few steps (4 x 300 slow
-    // changes 141 / 74, bits of probability 0.9 123 / 77).  Beyond 2048 steps chains and tables grow (8192 steps of bits of probability 0.25 to 0.6: 1.09 / 1.63).
+    // contexts alone, 5 x 2048 of clean periods 608 / 496 us, at worst 1.5 times (4 x 700 of all probabilities 209 / 141).  Beyond 2048 steps chains and tables grow (8192 steps of bits of probability 0.25 to 0.6: 1.09 / 1.63).
     if (T <= HEADS_MAX_TIME && streams > (T < 512u ? 4u : T < 1024u ? 5u : 14u) * sms) return LATEST_TOO;
     // Only a call of few streams can list less than half as many as there are CTAs.
     return streams <= PARTS_MAX_STREAMS * sms ? IN_PARTS : PLAIN;
@@ -1196,8 +1220,14 @@ void rosa_match(ullis_cuda_runtime* rt, const uint32_t* q_sw, const uint32_t* k_
     rt->sam_last_counts = m.counts;
     rt->sam_last_streams = streams;
     if (!rt->parent) rt->lanes_last = 1;
-    rt->chain(rosa_classify_kernel, (unsigned)((streams * CLASSIFY_LANES + 127) / 128), 128, 0, q_sw, k_sw, v_sw, idx_sw,
-              streams, T, m.wps, m.list, m.counts, m.cq_list, m.counts + 1, m.given_up);
+    // Few short streams by the latest positions last as long as the longest walk, and what is given up as long again.  If more than one listed
+    // stream in UNEVEN_SHARE is uneven all are answered by contexts.  us of the ROSA kernels, without / with the count: 4 x 300 x 512 bits of
+    // probability 0.9 121 / 84, of slow changes 139 / 82, one half of those 120 / 74, even ones 39 / 41; 4 x 128 72 / 63, 86 / 68, 78 / 63, 31 / 32; 4 x 500 211 /
+    // 133, 199 / 119, 160 / 95, 45 / 47; 8 x 400 238 / 177, 239 / 158, 173 / 127, 53 / 53.  Not at 16 x 600 (522 / 570, 456 / 449, 268 / 355), nor at 8 x 64 (43 / 73,
+    // 45 / 70, 43 / 73).  No model in training has so many of them.
+    const bool count_uneven = m.form == LATEST_TOO && T >= 128u && T < 512u && streams <= 28u * (size_t)rt->sm_count;
+    rt->chain(count_uneven ? rosa_classify_kernel<true> : rosa_classify_kernel<false>, (unsigned)((streams * CLASSIFY_LANES + 127) / 128), 128, 0, q_sw, k_sw,
+              v_sw, idx_sw, streams, T, m.wps, m.list, m.counts, m.cq_list, m.counts + 1, m.given_up, m.counts + 7);
     rt->launched("rosa_classify");
     contexts(rt, m);
     if (T <= 1024u) launch_match<1>(rt, m, 0, 1024);
@@ -1276,8 +1306,8 @@ void rosa_sam(ullis_cuda_runtime* rt, const uint32_t* q_sw, const uint32_t* k_sw
     } else {
         rt->zero(count, 8);   // both counters
         const unsigned classify_grid = (unsigned)((streams * CLASSIFY_LANES + 127) / 128);
-        rt->chain(rosa_classify_kernel, classify_grid, 128, 0, q_sw, k_sw, v_sw, idx_sw, streams, (uint32_t)time, wps, list,
-                                                             count, cq_list, cq_count, nullptr);
+        rt->chain(rosa_classify_kernel<false>, classify_grid, 128, 0, q_sw, k_sw, v_sw, idx_sw, streams, (uint32_t)time, wps, list,
+                                                             count, cq_list, cq_count, nullptr, nullptr);
         rt->launched("rosa_classify");
         // The constant-q scan is a long serial loop for a few thousand threads; it depends on nothing but the
         // classification and writes idx words no other kernel of this call touches, so it runs on the side stream
